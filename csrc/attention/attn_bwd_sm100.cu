@@ -1,25 +1,28 @@
 // Variable-length causal GQA attention backward for sm_100a.  Three kernels:
 //
 //   delta   : delta[h, i] = sum_d O[i, h, d] * dO[i, h, d]                                  (memory bound)
-//   dq      : one CTA per (128-query tile, query head), loops over 64-key blocks:
-//               S = Q K^T, dP = dO V^T on tcgen05 -> P = exp2(S*c - lse), dS = P*(dP - delta)*scale in registers
-//               -> dS (bf16) to shared memory -> dQ += dS K accumulated in TMEM
-//   dk/dv   : one CTA per (128-key tile, kv head), loops over the query heads of the group and 64-query blocks:
+//   dq      : one CTA per (128-query tile, query head), loops over 128-key blocks:
+//               S = Q K^T, dP = dO V^T on tcgen05 -> P = exp2(S*c - lse), dS = P*(dP - delta) in registers
+//               -> dS (bf16) to TMEM -> dQ += dS K accumulated in TMEM
+//   dk/dv   : one CTA per (128-key tile, kv head), loops over the query heads of the group and 128-query blocks:
 //               S^T = K Q^T, dP^T = V dO^T -> P^T, dS^T -> dV += P^T dO, dK += dS^T Q accumulated in TMEM
 //
-// All operand layouts are the ones the forward kernel uses (row-major [tokens, heads*d] tiles fetched by TMA with
-// the 128-byte swizzle, consumed K-major or MN-major), P is recomputed from the forward's log-sum-exp so nothing
-// but O and lse is kept from the forward.  The mask is the forward's: a per-query inclusive key range
-// [k_lo[i], k_hi[i]] (k_hi null = the query's own index, i.e. packed causal self-attention); queries and keys may be
-// different token sets.  The dK/dV kernel additionally takes, per key, bounds [q_lo[n], q_hi[n]] on the queries that
-// can see it (null = derived from the causal structure), which only limit its loop: visibility itself is always
-// decided by the per-query ranges.
+// The softmax scale multiplies dQ and dK once, when they are written.  All operand tiles are the ones the forward kernel
+// uses (row-major [tokens, heads*d] tiles fetched by TMA with the 128-byte swizzle, consumed K-major or MN-major); the
+// probabilities and dS go to the second product as its A operand through TMEM, never through shared memory, and P is
+// recomputed from the forward's log-sum-exp so nothing but O and lse is kept from the forward.  The mask is the
+// forward's: a per-query inclusive key range [k_lo[i], k_hi[i]] (k_hi null = the query's own index, i.e. packed causal
+// self-attention); queries and keys may be different token sets.  The dK/dV kernel additionally takes, per key, bounds
+// [q_lo[n], q_hi[n]] on the queries that can see it (null = derived from the causal structure), which only limit its
+// loop: visibility itself is always decided by the per-query ranges.
 //
-// Warp roles in dq and dk/dv (320 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2..9
-// element-wise in two groups of four (thread = TMEM lane = query row in dq, key row in dk/dv); group g takes the
-// blocks j = g, g+2, ... and owns TMEM / shared-memory buffer g, so every scheduler has two element-wise warps to
-// interleave and the exponentials of one block overlap the TMEM reads of the next.  Every wait is bounded and
-// reports through the status buffer.
+// Warp roles (384 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warp 2 (dk/dv) stages the per-query
+// values of the next blocks, warps 4..11 element-wise: thread = TMEM lane = query row in dq, key row in dk/dv; warps
+// 4..7 take columns 0..63 of every block, warps 8..11 columns 64..127, so that a block's latency is half a block's
+// arithmetic.  The tensor core is kept busy by the order of the products, not by second buffers (see each kernel).
+// Every wait is bounded and reports through the status buffer.  Measured, 32 query / 8 kv heads of 128, causal: 8192 tokens
+// in four segments 0.58 ms = 597 TFLOP/s, one 16384-token segment 7.35 ms = 748 TFLOP/s; with 64-row blocks and P / dS
+// through shared memory the latter ran at 411 TFLOP/s.
 #include <climits>
 
 #include "../common/host_utils.cuh"
@@ -30,10 +33,13 @@ using namespace mcb;
 
 namespace {
 
-constexpr int TM = 128;   // rows of the CTA's resident tile (TMEM lanes)
-constexpr int BLK = 64;   // rows of the streamed blocks (MMA N for the score GEMMs, K for the gradient GEMMs)
-constexpr int BWD_THREADS = 320;
+constexpr int TM = 128;   // rows of the CTA's resident tile (TMEM lanes) and of the streamed blocks
+constexpr int BWD_THREADS = 384;
+constexpr int HALF = TM / 2;   // columns of a block that one element-wise warp handles
 constexpr float LOG2E = 1.4426950408889634f;
+// 384 threads x 168 registers at launch: 128 x (104 + 200 + 200) = 64512
+#define MCB_REGS_CONTROL() asm volatile("setmaxnreg.dec.sync.aligned.u32 104;")
+#define MCB_REGS_MATH() asm volatile("setmaxnreg.inc.sync.aligned.u32 200;")
 
 struct BwdParams {
   int T, Tk, nq, nkv, d;    // T queries, Tk keys
@@ -66,24 +72,9 @@ __host__ __device__ constexpr uint32_t idesc(int m, int n, bool b_mn) {
          (uint32_t(m >> 4) << 24);
 }
 
-// writes 32 consecutive bf16 of row r (columns c..c+31 of a [128 x 64] K-major swizzled tile)
-__device__ __forceinline__ void store_row_chunk(uint8_t* tile, int r, int c, const float* x) {
-  uint8_t* row = tile + r * 128;
-#pragma unroll
-  for (int e = 0; e < 32; e += 8) {
-    uint4 o;
-    o.x = pack_bf16x2(x[e], x[e + 1]);
-    o.y = pack_bf16x2(x[e + 2], x[e + 3]);
-    o.z = pack_bf16x2(x[e + 4], x[e + 5]);
-    o.w = pack_bf16x2(x[e + 6], x[e + 7]);
-    const int chunk = (c + e) >> 3;
-    *reinterpret_cast<uint4*>(row + ((chunk ^ (r & 7)) << 4)) = o;
-  }
-}
-
 // one TMEM lane's D accumulator columns -> a bf16 row in global memory
 template <int COLS>
-__device__ __forceinline__ void store_acc_row(uint32_t taddr, __nv_bfloat16* dst, bool ok) {
+__device__ __forceinline__ void store_acc_row(uint32_t taddr, __nv_bfloat16* dst, float f, bool ok) {
 #pragma unroll 1
   for (int c = 0; c < COLS; c += 32) {
     uint32_t v[32];
@@ -93,10 +84,10 @@ __device__ __forceinline__ void store_acc_row(uint32_t taddr, __nv_bfloat16* dst
 #pragma unroll
       for (int e = 0; e < 32; e += 8) {
         uint4 o;
-        o.x = pack_bf16x2(__uint_as_float(v[e]), __uint_as_float(v[e + 1]));
-        o.y = pack_bf16x2(__uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]));
-        o.z = pack_bf16x2(__uint_as_float(v[e + 4]), __uint_as_float(v[e + 5]));
-        o.w = pack_bf16x2(__uint_as_float(v[e + 6]), __uint_as_float(v[e + 7]));
+        o.x = pack_bf16x2(__uint_as_float(v[e]) * f, __uint_as_float(v[e + 1]) * f);
+        o.y = pack_bf16x2(__uint_as_float(v[e + 2]) * f, __uint_as_float(v[e + 3]) * f);
+        o.z = pack_bf16x2(__uint_as_float(v[e + 4]) * f, __uint_as_float(v[e + 5]) * f);
+        o.w = pack_bf16x2(__uint_as_float(v[e + 6]) * f, __uint_as_float(v[e + 7]) * f);
         *reinterpret_cast<uint4*>(dst + c + e) = o;
       }
     }
@@ -105,7 +96,7 @@ __device__ __forceinline__ void store_acc_row(uint32_t taddr, __nv_bfloat16* dst
 
 // one TMEM lane's accumulator columns -> an fp32 row in global memory
 template <int COLS>
-__device__ __forceinline__ void store_acc_row_f32(uint32_t taddr, float* dst, bool ok) {
+__device__ __forceinline__ void store_acc_row_f32(uint32_t taddr, float* dst, float f, bool ok) {
 #pragma unroll 1
   for (int c = 0; c < COLS; c += 32) {
     uint32_t v[32];
@@ -114,50 +105,67 @@ __device__ __forceinline__ void store_acc_row_f32(uint32_t taddr, float* dst, bo
     if (ok) {
 #pragma unroll
       for (int e = 0; e < 32; e += 4)
-        *reinterpret_cast<uint4*>(dst + c + e) = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+        *reinterpret_cast<float4*>(dst + c + e) =
+            make_float4(__uint_as_float(v[e]) * f, __uint_as_float(v[e + 1]) * f, __uint_as_float(v[e + 2]) * f,
+                        __uint_as_float(v[e + 3]) * f);
     }
   }
 }
 
-__device__ __forceinline__ void drain(uint64_t* bar, uint32_t it) {
+__device__ __forceinline__ void drain(uint64_t* bar, uint32_t parity) {
   uint64_t t0 = globaltimer_ns();
-  while (!mbar_try_wait(smem_u32(bar), (it >> 1) & 1))
+  while (!mbar_try_wait(smem_u32(bar), parity))
     if (globaltimer_ns() - t0 > 200000000ull) break;
 }
 
 // ---------------------------------------------------------------------------------------------------- delta
+// D / 8 lanes per (token, head) row, 16-byte loads, 4 rows per lane group in flight: bound by reading O and dO once.
 template <int D>
-__global__ void attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                                      float* __restrict__ delta, int T, int nq) {
-  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= (long long)T * nq) return;
-  const int i = int(w / nq), h = int(w % nq);
-  const __nv_bfloat16* po = o + w * D;
-  const __nv_bfloat16* pd = dout + w * D;
-  float acc = 0.f;
-  for (int c = lane * 2; c < D; c += 64) {
-    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(po + c);
-    const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(pd + c);
-    acc += __bfloat162float(a.x) * __bfloat162float(b.x) + __bfloat162float(a.y) * __bfloat162float(b.y);
+__global__ void __launch_bounds__(256)
+attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
+                      float* __restrict__ delta, int T, int nq) {
+  constexpr int LANES = D / 8, ROWS = 256 / LANES, UNROLL = 4;
+  const long long rows = (long long)T * nq;
+  const long long base = (long long)blockIdx.x * ROWS * UNROLL + threadIdx.x / LANES;
+  const int c = (threadIdx.x % LANES) * 8;
+  uint4 a[UNROLL], b[UNROLL];
+#pragma unroll
+  for (int u = 0; u < UNROLL; ++u) {
+    const long long w = base + u * ROWS;
+    const bool in = w < rows;
+    a[u] = in ? *reinterpret_cast<const uint4*>(o + w * D + c) : make_uint4(0, 0, 0, 0);
+    b[u] = in ? *reinterpret_cast<const uint4*>(dout + w * D + c) : make_uint4(0, 0, 0, 0);
   }
 #pragma unroll
-  for (int s = 16; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (lane == 0) delta[(long long)h * T + i] = acc;
+  for (int u = 0; u < UNROLL; ++u) {
+    const long long w = base + u * ROWS;
+    const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&a[u]);
+    const __nv_bfloat162* y = reinterpret_cast<const __nv_bfloat162*>(&b[u]);
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __bfloat1622float2(x[e]), g = __bfloat1622float2(y[e]);
+      acc += f.x * g.x + f.y * g.y;
+    }
+#pragma unroll
+    for (int s = LANES / 2; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (c == 0 && w < rows) delta[(w % nq) * T + w / nq] = acc;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------- dQ
+// Order of the products:  S0 dP0 S1 | dP(j+1) dQ(j) S(j+2) | ...  Two score buffers, one dP buffer: dP(j+1) starts as soon
+// as the element-wise warps hold dP(j) in registers and runs under their arithmetic; dS(j) overwrites the scores it came
+// from, so dQ(j) frees the buffer S(j+2) goes to.  K(j) is needed from S(j) to dQ(j): three stages of K, two of V.
+// Bound: 3 x 512 tensor cycles and 1024 MUFU cycles per 128 x 128 block.
 template <int D>
 struct DqSmem {
   static constexpr int TILE = TM * D * 2;
-  static constexpr int BLOCK = BLK * D * 2;
-  static constexpr int DS = TM * BLK * 2;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_DO = TILE;
-  static constexpr int OFF_K = 2 * TILE;               // 2 stages
-  static constexpr int OFF_V = OFF_K + 2 * BLOCK;      // 2 stages
-  static constexpr int OFF_DS = OFF_V + 2 * BLOCK;     // 2 buffers
-  static constexpr int OFF_BAR = OFF_DS + 2 * DS;
+  static constexpr int OFF_K = 2 * TILE;               // 3 stages
+  static constexpr int OFF_V = OFF_K + 3 * TILE;       // 2 stages
+  static constexpr int OFF_BAR = OFF_V + 2 * TILE;
   static constexpr int TOTAL = OFF_BAR + 1024 + 1024;
 };
 
@@ -169,24 +177,26 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   using L = DqSmem<D>;
   constexpr int NBOX = D / 64;
   constexpr uint32_t TMEM_COLS = 512;
-  constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DQ = 256;
+  constexpr uint32_t COL_S = 0, COL_DP = 256, COL_DQ = 384;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
   uint64_t* q_full = bars;             // 1
-  uint64_t* kv_full = bars + 1;        // 2
-  uint64_t* kv_empty = bars + 3;       // 2
-  uint64_t* s_full = bars + 5;         // 2
-  uint64_t* s_empty = bars + 7;        // 2
-  uint64_t* ds_full = bars + 9;        // 2
-  uint64_t* ds_empty = bars + 11;      // 2
-  uint64_t* dq_full = bars + 13;       // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* k_full = bars + 1;         // 3
+  uint64_t* k_empty = bars + 4;        // 3
+  uint64_t* v_full = bars + 7;         // 2
+  uint64_t* v_empty = bars + 9;        // 2
+  uint64_t* s_full = bars + 11;        // 2
+  uint64_t* dp_full = bars + 13;       // 1
+  uint64_t* dp_empty = bars + 14;      // 1
+  uint64_t* ds_full = bars + 15;       // 1
+  uint64_t* dq_full = bars + 16;       // 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tile = gridDim.x - 1 - blockIdx.x;
-  const int head = blockIdx.y;
+  const int m_tile = (gridDim.x - 1 - blockIdx.x) / p.nq;      // long tiles of every head first
+  const int head = blockIdx.x % p.nq;
   const int kvh = head / (p.nq / p.nkv);
   const int m0 = m_tile * TM;
   __shared__ int s_rng[8];
@@ -195,14 +205,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     mbar_init(smem_u32(q_full), 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&kv_full[i]), 1);
-      mbar_init(smem_u32(&kv_empty[i]), 1);
-      mbar_init(smem_u32(&s_full[i]), 1);
-      mbar_init(smem_u32(&s_empty[i]), 4);
-      mbar_init(smem_u32(&ds_full[i]), 128);
-      mbar_init(smem_u32(&ds_empty[i]), 1);
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(smem_u32(&k_full[i]), 1);
+      mbar_init(smem_u32(&k_empty[i]), 1);
     }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&v_full[i]), 1);
+      mbar_init(smem_u32(&v_empty[i]), 1);
+      mbar_init(smem_u32(&s_full[i]), 1);
+    }
+    mbar_init(smem_u32(dp_full), 1);
+    mbar_init(smem_u32(dp_empty), 8);
+    mbar_init(smem_u32(ds_full), 8);
     mbar_init(smem_u32(dq_full), 1);
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -220,143 +234,163 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const int kmin = tile_range_min(s_rng), kmax = tile_range_max(s_rng);
-  const int kb0 = kmin / BLK;
-  const int nblk = kmax >= kmin ? kmax / BLK - kb0 + 1 : 0;
+  const int kb0 = kmin / TM;
+  const int nblk = kmax >= kmin ? kmax / TM - kb0 + 1 : 0;
 
-  if (nblk <= 0) {
-    // no row of this tile sees any key: its queries get a zero gradient
-    if (warp >= 2) {
-      const int grp = (warp - 2) >> 2;
-      const int i = m0 + (warp & 3) * 32 + lane;
-      if (i < p.T) {
-        uint4* row = reinterpret_cast<uint4*>(p.dq + ((long long)i * p.nq + head) * D + grp * (D / 2));
-#pragma unroll
-        for (int c = 0; c < D / 16; ++c) row[c] = make_uint4(0, 0, 0, 0);
-      }
-    }
-  } else if (warp == 0) {
-    if (lane == 0) {
+  if (warp < 4) {
+    MCB_REGS_CONTROL();
+    if (warp == 0 && lane == 0 && nblk > 0) {
+      // ---------------------------------------------------------------- TMA producer
       mbar_expect_tx(smem_u32(q_full), 2 * L::TILE);
 #pragma unroll
       for (int b = 0; b < NBOX; ++b) {
         tma_load_2d(smem_u32(smem + L::OFF_Q + b * TM * 128), &tm_q, head * D + b * 64, m0, smem_u32(q_full));
         tma_load_2d(smem_u32(smem + L::OFF_DO + b * TM * 128), &tm_do, head * D + b * 64, m0, smem_u32(q_full));
       }
-      int j = 0;
-      for (; j < nblk; ++j) {
-        const uint32_t st = j & 1, ph = (j >> 1) & 1;
-        const int n0 = (kb0 + j) * BLK;
-        if (!mbar_wait(smem_u32(&kv_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
-        mbar_expect_tx(smem_u32(&kv_full[st]), 2 * L::BLOCK);
+      int nk = 0, nv = 0;
+      for (int j = 0; j < nblk; ++j) {
+        const uint32_t ks = j % 3, kp = (j / 3) & 1, vs = j & 1, vp = (j >> 1) & 1;
+        const int n0 = (kb0 + j) * TM;
+        if (!mbar_wait(smem_u32(&k_empty[ks]), kp ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_expect_tx(smem_u32(&k_full[ks]), L::TILE);
 #pragma unroll
-        for (int b = 0; b < NBOX; ++b) {
-          tma_load_2d(smem_u32(smem + L::OFF_K + st * L::BLOCK + b * BLK * 128), &tm_k, kvh * D + b * 64, n0,
-                      smem_u32(&kv_full[st]));
-          tma_load_2d(smem_u32(smem + L::OFF_V + st * L::BLOCK + b * BLK * 128), &tm_v, kvh * D + b * 64, n0,
-                      smem_u32(&kv_full[st]));
-        }
+        for (int b = 0; b < NBOX; ++b)
+          tma_load_2d(smem_u32(smem + L::OFF_K + ks * L::TILE + b * TM * 128), &tm_k, kvh * D + b * 64, n0,
+                      smem_u32(&k_full[ks]));
+        ++nk;
+        if (!mbar_wait(smem_u32(&v_empty[vs]), vp ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_expect_tx(smem_u32(&v_full[vs]), L::TILE);
+#pragma unroll
+        for (int b = 0; b < NBOX; ++b)
+          tma_load_2d(smem_u32(smem + L::OFF_V + vs * L::TILE + b * TM * 128), &tm_v, kvh * D + b * 64, n0,
+                      smem_u32(&v_full[vs]));
+        ++nv;
       }
-      for (int i = (j > 2 ? j - 2 : 0); i < j; ++i) drain(&kv_full[i & 1], i);   // loads land before the CTA exits
+      // the last loads land before the CTA exits
+      for (int i = (nk > 3 ? nk - 3 : 0); i < nk; ++i) drain(&k_full[i % 3], (i / 3) & 1);
+      for (int i = (nv > 2 ? nv - 2 : 0); i < nv; ++i) drain(&v_full[i & 1], (i >> 1) & 1);
       drain(q_full, 0);
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = idesc(TM, BLK, false);
+    } else if (warp == 1 && lane == 0 && nblk > 0) {
+      // ---------------------------------------------------------------- MMA issuer
+      constexpr uint32_t idesc_s = idesc(TM, TM, false);
       constexpr uint32_t idesc_dq = idesc(TM, D, true);
       const uint32_t sq = smem_u32(smem + L::OFF_Q), sdo = smem_u32(smem + L::OFF_DO);
-      bool ok = mbar_wait(smem_u32(q_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
-      auto issue_sdp = [&](int j) -> bool {
-        const uint32_t st = j & 1, ph = (j >> 1) & 1;
-        if (!mbar_wait(smem_u32(&kv_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
-        if (!mbar_wait(smem_u32(&s_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
+      auto issue_s = [&](int j) -> bool {
+        const uint32_t ks = j % 3, kp = (j / 3) & 1;
+        if (!mbar_wait(smem_u32(&k_full[ks]), kp, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        const uint32_t sk = smem_u32(smem + L::OFF_K + st * L::BLOCK);
-        const uint32_t sv = smem_u32(smem + L::OFF_V + st * L::BLOCK);
+        const uint32_t sk = smem_u32(smem + L::OFF_K + ks * L::TILE);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_S + st * BLK, kdesc(sq, kk, TM), kdesc(sk, kk, BLK), idesc_s, kk ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_DP + st * BLK, kdesc(sdo, kk, TM), kdesc(sv, kk, BLK), idesc_s, kk ? 1u : 0u);
-        umma_commit(smem_u32(&s_full[st]));
+          umma_f16(tmem + COL_S + (j & 1) * TM, kdesc(sq, kk, TM), kdesc(sk, kk, TM), idesc_s, kk ? 1u : 0u);
+        umma_commit(smem_u32(&s_full[j & 1]));
         return true;
       };
-      if (ok) ok = issue_sdp(0);
-      for (int j = 0; j < nblk && ok; ++j) {
-        if (j + 1 < nblk) {
-          ok = issue_sdp(j + 1);
-          if (!ok) break;
-        }
-        const uint32_t st = j & 1, ph = (j >> 1) & 1;
-        if (!mbar_wait(smem_u32(&ds_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+      auto issue_dp = [&](int j) -> bool {
+        const uint32_t vs = j & 1, vp = (j >> 1) & 1;
+        if (!mbar_wait(smem_u32(&v_full[vs]), vp, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
+        if (j > 0 && !mbar_wait(smem_u32(dp_empty), (j & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
         tc_fence_after();
-        const uint32_t sds = smem_u32(smem + L::OFF_DS + st * L::DS);
-        const uint32_t sk = smem_u32(smem + L::OFF_K + st * L::BLOCK);
+        const uint32_t sv = smem_u32(smem + L::OFF_V + vs * L::TILE);
 #pragma unroll
-        for (int kk = 0; kk < BLK / 16; ++kk)
-          umma_f16(tmem + COL_DQ, kdesc(sds, kk, TM), mndesc(sk, kk, BLK), idesc_dq, (j | kk) ? 1u : 0u);
-        umma_commit(smem_u32(&ds_empty[st]));
-        umma_commit(smem_u32(&kv_empty[st]));
+        for (int kk = 0; kk < D / 16; ++kk)
+          umma_f16(tmem + COL_DP, kdesc(sdo, kk, TM), kdesc(sv, kk, TM), idesc_s, kk ? 1u : 0u);
+        umma_commit(smem_u32(dp_full));
+        umma_commit(smem_u32(&v_empty[vs]));
+        return true;
+      };
+      bool ok = mbar_wait(smem_u32(q_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
+      if (ok) ok = issue_s(0);
+      if (ok) ok = issue_dp(0);
+      if (ok && nblk > 1) ok = issue_s(1);
+      for (int j = 0; j < nblk && ok; ++j) {
+        if (j + 1 < nblk && !issue_dp(j + 1)) { ok = false; break; }
+        if (!mbar_wait(smem_u32(ds_full), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sk = smem_u32(smem + L::OFF_K + (j % 3) * L::TILE);
+        const uint32_t ads = tmem + COL_S + (j & 1) * TM;
+#pragma unroll
+        for (int kk = 0; kk < TM / 16; ++kk)     // dS: 32 packed columns at the start of each 64-column half
+          umma_f16_ts(tmem + COL_DQ, ads + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sk, kk, TM), idesc_dq,
+                      (j | kk) ? 1u : 0u);
+        umma_commit(smem_u32(&k_empty[j % 3]));
+        if (j + 2 < nblk) ok = issue_s(j + 2);
       }
       if (ok) umma_commit(smem_u32(dq_full));
     }
   } else {
+    MCB_REGS_MATH();
     const int q = warp & 3;
-    const int grp = (warp - 2) >> 2;
+    const int grp = (warp - 4) >> 2;
     const int r = q * 32 + lane;
     const int i = m0 + r;
     const bool row_ok = i < p.T;
     int lo, hi;
     attn_row_range(p.k_lo, p.k_hi, i, p.T, lo, hi);
-    // a query that sees nothing has lse = -inf; its masked probabilities are zeroed below, keep the arithmetic finite
+    if (lo > hi) lo = hi = 0x40000000;            // sees nothing: a range no key index reaches
+    const unsigned span = (unsigned)(hi - lo);    // key k is visible iff (unsigned)(k - lo) <= span
+    // a query that sees nothing has lse = -inf; its probabilities are masked below, keep the arithmetic finite
     const float lse_i = row_ok ? p.lse[(long long)head * p.T + i] : 0.f;
     const float lse2 = (lse_i == -INFINITY) ? 0.f : lse_i * LOG2E;
     const float dl = row_ok ? p.delta[(long long)head * p.T + i] : 0.f;
+    const uint64_t cc = f32x2(p.scale_log2, p.scale_log2), nl = f32x2(-lse2, -lse2), nd = f32x2(-dl, -dl);
     const uint32_t lane_addr = uint32_t(q * 32) << 16;
-    const uint32_t st = grp;
     bool ok = true;
-    for (int j = grp; j < nblk && ok; j += 2) {
-      const uint32_t ph = (j >> 1) & 1;
-      if (!mbar_wait(smem_u32(&s_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-      if (!mbar_wait(smem_u32(&ds_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
+    for (int j = 0; j < nblk && ok; ++j) {
+      const uint32_t ts = tmem + lane_addr + COL_S + (j & 1) * TM + grp * HALF;
+      const uint32_t td = tmem + lane_addr + COL_DP + grp * HALF;
+      const int n0 = (kb0 + j) * TM + grp * HALF;
+      const bool full = __all_sync(0xffffffffu, lo <= n0 && n0 + HALF - 1 <= hi);
+      uint32_t pr[HALF];
+      if (!mbar_wait(smem_u32(&s_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      const int n0 = (kb0 + j) * BLK;
-      const bool full = (lo <= n0) && (n0 + BLK - 1 <= hi);
-      uint8_t* tile = smem + L::OFF_DS + st * L::DS;
-#pragma unroll 1
-      for (int c = 0; c < BLK; c += 32) {
-        uint32_t s[32], dp[32];
-        tmem_ld_32x32(tmem + lane_addr + COL_S + st * BLK + c, s);
-        tmem_ld_32x32(tmem + lane_addr + COL_DP + st * BLK + c, dp);
-        tmem_ld_wait();
-        float ds[32];
-        if (full) {
+      tmem_ld_32x32_x64(ts, pr);
+      tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const float pr = exp2f(__uint_as_float(s[e]) * p.scale_log2 - lse2);
-            ds[e] = pr * (__uint_as_float(dp[e]) - dl) * p.scale;
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int key = n0 + c + e;
-            const float pr = exp2f(__uint_as_float(s[e]) * p.scale_log2 - lse2);
-            ds[e] = (key >= lo && key <= hi) ? pr * (__uint_as_float(dp[e]) - dl) * p.scale : 0.f;
-          }
-        }
-        store_row_chunk(tile, r, c, ds);
+      for (int e = 0; e < HALF; e += 2) {
+        const float2 x = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1])), cc, nl));
+        pr[e] = __float_as_uint(ex2_ftz(x.x));
+        pr[e + 1] = __float_as_uint(ex2_ftz(x.y));
       }
+      if (!full) {
+#pragma unroll
+        for (int e = 0; e < HALF; ++e) pr[e] = (unsigned)(n0 + e - lo) <= span ? pr[e] : 0u;
+      }
+      if (!mbar_wait(smem_u32(dp_full), j & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t dp[HALF];
+      tmem_ld_32x32_x64(td, dp);
+      tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_empty[st]));
-      fence_proxy_async_smem();
-      mbar_arrive(smem_u32(&ds_full[st]));
+      if (lane == 0) mbar_arrive(smem_u32(dp_empty));   // dP is in registers: the next dO V^T may start
+      uint32_t pk[HALF / 2];
+#pragma unroll
+      for (int e = 0; e < HALF; e += 2) {
+        const uint64_t d2 = add_f32x2(f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1])), nd);
+        float2 x = f32x2_split(mul_f32x2(d2, f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1]))));
+        if (!full) {                              // a masked pair contributes zero whatever its dP is
+          x.x = (unsigned)(n0 + e - lo) <= span ? x.x : 0.f;
+          x.y = (unsigned)(n0 + e + 1 - lo) <= span ? x.y : 0.f;
+        }
+        pk[e >> 1] = pack_bf16x2(x.x, x.y);
+      }
+      tmem_st_32x32(ts, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(ds_full));
     }
-    if (ok && mbar_wait(smem_u32(dq_full), 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
+    __nv_bfloat16* row = p.dq + ((long long)i * p.nq + head) * D + grp * (D / 2);   // each group writes half of the row
+    if (nblk <= 0) {
+      // no row of this tile sees any key: its queries get a zero gradient
+      if (row_ok) {
+#pragma unroll
+        for (int c = 0; c < D / 16; ++c) reinterpret_cast<uint4*>(row)[c] = make_uint4(0, 0, 0, 0);
+      }
+    } else if (ok && mbar_wait(smem_u32(dq_full), 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
-      // each group writes half of the row
-      store_acc_row<D / 2>(tmem + lane_addr + COL_DQ + grp * (D / 2),
-                           p.dq + ((long long)i * p.nq + head) * D + grp * (D / 2), row_ok);
+      store_acc_row<D / 2>(tmem + lane_addr + COL_DQ + grp * (D / 2), row, p.scale, row_ok);
     }
   }
   tc_fence_before();
@@ -368,21 +402,22 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 }
 
 // ---------------------------------------------------------------------------------------------------- dK / dV
+// The accumulators take half of TMEM, one S^T and one dP^T block the other half.  Order of the products:
+//   S0 | dP(j) dV(j) S(j+1) dK(j) | dP(j+1) ...
+// P(j) overwrites S(j) and dS(j) overwrites dP(j); the exponentials of block j+1 run under dK(j) and dP(j+1), the dS
+// arithmetic of block j under dV(j) and S(j+1), so the tensor core has work while either is computed.
+// Bound: 4 x 512 tensor cycles per 128 x 128 block.
 template <int D>
 struct DkvSmem {
   static constexpr int TILE = TM * D * 2;
-  static constexpr int BLOCK = BLK * D * 2;
-  static constexpr int PT = TM * BLK * 2;
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = TILE;
   static constexpr int OFF_Q = 2 * TILE;                // 2 stages
-  static constexpr int OFF_DO = OFF_Q + 2 * BLOCK;      // 2 stages
-  static constexpr int OFF_P = OFF_DO + 2 * BLOCK;      // 2 buffers
-  static constexpr int OFF_DS = OFF_P + 2 * PT;         // 2 buffers
-  static constexpr int OFF_COL = OFF_DS + 2 * PT;       // per-column lse / delta / k_lo / k_hi + 4 ints of block
-                                                        // bounds, 2 buffers per group
-  static constexpr int COL_BYTES = 4 * BLK * 4 + 16;
-  static constexpr int OFF_BAR = OFF_COL + 4 * COL_BYTES;
+  static constexpr int OFF_DO = OFF_Q + 2 * TILE;       // 2 stages
+  static constexpr int OFF_COL = OFF_DO + 2 * TILE;     // 2 buffers: per-query lse / delta / k_lo / k_hi, then the
+                                                        // largest k_lo and the smallest k_hi of the block
+  static constexpr int COL_BYTES = 4 * TM * 4 + 16;
+  static constexpr int OFF_BAR = OFF_COL + 2 * COL_BYTES;
   static constexpr int TOTAL = OFF_BAR + 1024 + 1024;
 };
 
@@ -394,41 +429,47 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   using L = DkvSmem<D>;
   constexpr int NBOX = D / 64;
   constexpr uint32_t TMEM_COLS = 512;
-  constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + D;
+  constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 384;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
   uint64_t* kv_full = bars;            // 1
-  uint64_t* qdo_full = bars + 1;       // 2
-  uint64_t* qdo_empty = bars + 3;      // 2
-  uint64_t* s_full = bars + 5;         // 2
-  uint64_t* s_empty = bars + 7;        // 2
-  uint64_t* pds_full = bars + 9;       // 2
-  uint64_t* pds_empty = bars + 11;     // 2
+  uint64_t* q_full = bars + 1;         // 2
+  uint64_t* q_empty = bars + 3;        // 2
+  uint64_t* do_full = bars + 5;        // 2
+  uint64_t* do_empty = bars + 7;       // 2
+  uint64_t* s_full = bars + 9;         // 1
+  uint64_t* p_full = bars + 10;        // 1
+  uint64_t* dp_full = bars + 11;       // 1
+  uint64_t* ds_full = bars + 12;       // 1
   uint64_t* out_full = bars + 13;      // 1
-  uint64_t* col_full = bars + 14;      // 4
+  uint64_t* col_full = bars + 14;      // 2
+  uint64_t* col_empty = bars + 16;     // 2
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* i_end_slot = reinterpret_cast<int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.y;
+  const int group_cta = blockIdx.x % (p.nkv * p.splits);         // key tiles ascend slowest: long ones first when causal
+  const int kvh = group_cta / p.splits, split = group_cta % p.splits;
   const int qpg = p.nq / p.nkv;
-  const int n0 = blockIdx.x * TM;
+  const int n0 = blockIdx.x / (p.nkv * p.splits) * TM;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     mbar_init(smem_u32(kv_full), 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&qdo_full[i]), 1);
-      mbar_init(smem_u32(&qdo_empty[i]), 1);
-      mbar_init(smem_u32(&s_full[i]), 1);
-      mbar_init(smem_u32(&s_empty[i]), 4);
-      mbar_init(smem_u32(&pds_full[i]), 128);
-      mbar_init(smem_u32(&pds_empty[i]), 1);
-      mbar_init(smem_u32(&col_full[i]), 128);
-      mbar_init(smem_u32(&col_full[2 + i]), 128);
+      mbar_init(smem_u32(&q_full[i]), 1);
+      mbar_init(smem_u32(&q_empty[i]), 1);
+      mbar_init(smem_u32(&do_full[i]), 1);
+      mbar_init(smem_u32(&do_empty[i]), 1);
+      mbar_init(smem_u32(&col_full[i]), 32);
+      mbar_init(smem_u32(&col_empty[i]), 8);
     }
+    mbar_init(smem_u32(s_full), 1);
+    mbar_init(smem_u32(p_full), 8);
+    mbar_init(smem_u32(dp_full), 1);
+    mbar_init(smem_u32(ds_full), 8);
     mbar_init(smem_u32(out_full), 1);
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -461,207 +502,244 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   const uint32_t tmem = *tmem_slot;
   const int i_first = p.q_lo ? tile_range_min(s_rng) : i_end_slot[0];
   const int i_last = p.q_lo ? min(tile_range_max(s_rng), p.T - 1) : i_end_slot[1];
-  const int qb0 = i_first / BLK;
-  const int nqb = i_last >= i_first ? i_last / BLK - qb0 + 1 : 0;   // 0: no query sees a key of this tile
+  const int qb0 = i_first / TM;
+  const int nqb = i_last >= i_first ? i_last / TM - qb0 + 1 : 0;    // 0: no query sees a key of this tile
   const int hps = qpg / p.splits;                 // query heads handled by this CTA
-  const int h_first = kvh * qpg + blockIdx.z * hps;
+  const int h_first = kvh * qpg + split * hps;
   const int iters = hps * nqb;
 
-  if (warp == 0) {
-    if (lane == 0) {
+  if (warp < 4) {
+    MCB_REGS_CONTROL();
+    if (warp == 0 && lane == 0 && iters > 0) {
+      // ---------------------------------------------------------------- TMA producer
       mbar_expect_tx(smem_u32(kv_full), 2 * L::TILE);
 #pragma unroll
       for (int b = 0; b < NBOX; ++b) {
         tma_load_2d(smem_u32(smem + L::OFF_K + b * TM * 128), &tm_k, kvh * D + b * 64, n0, smem_u32(kv_full));
         tma_load_2d(smem_u32(smem + L::OFF_V + b * TM * 128), &tm_v, kvh * D + b * 64, n0, smem_u32(kv_full));
       }
-      int it = 0;
-      for (; it < iters; ++it) {
+      int nQ = 0, nD = 0, h = h_first, qb = 0;
+      for (int it = 0; it < iters; ++it) {
         const uint32_t st = it & 1, ph = (it >> 1) & 1;
-        const int h = h_first + it / nqb;
-        const int i0 = (qb0 + it % nqb) * BLK;
-        if (!mbar_wait(smem_u32(&qdo_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
-        mbar_expect_tx(smem_u32(&qdo_full[st]), 2 * L::BLOCK);
+        const int i0 = (qb0 + qb) * TM;
+        if (!mbar_wait(smem_u32(&q_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_expect_tx(smem_u32(&q_full[st]), L::TILE);
 #pragma unroll
-        for (int b = 0; b < NBOX; ++b) {
-          tma_load_2d(smem_u32(smem + L::OFF_Q + st * L::BLOCK + b * BLK * 128), &tm_q, h * D + b * 64, i0,
-                      smem_u32(&qdo_full[st]));
-          tma_load_2d(smem_u32(smem + L::OFF_DO + st * L::BLOCK + b * BLK * 128), &tm_do, h * D + b * 64, i0,
-                      smem_u32(&qdo_full[st]));
-        }
+        for (int b = 0; b < NBOX; ++b)
+          tma_load_2d(smem_u32(smem + L::OFF_Q + st * L::TILE + b * TM * 128), &tm_q, h * D + b * 64, i0,
+                      smem_u32(&q_full[st]));
+        ++nQ;
+        if (!mbar_wait(smem_u32(&do_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_expect_tx(smem_u32(&do_full[st]), L::TILE);
+#pragma unroll
+        for (int b = 0; b < NBOX; ++b)
+          tma_load_2d(smem_u32(smem + L::OFF_DO + st * L::TILE + b * TM * 128), &tm_do, h * D + b * 64, i0,
+                      smem_u32(&do_full[st]));
+        ++nD;
+        if (++qb == nqb) { qb = 0; ++h; }
       }
-      for (int i = (it > 2 ? it - 2 : 0); i < it; ++i) drain(&qdo_full[i & 1], i);
+      for (int i = (nQ > 2 ? nQ - 2 : 0); i < nQ; ++i) drain(&q_full[i & 1], (i >> 1) & 1);
+      for (int i = (nD > 2 ? nD - 2 : 0); i < nD; ++i) drain(&do_full[i & 1], (i >> 1) & 1);
       drain(kv_full, 0);
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = idesc(TM, BLK, false);
+    } else if (warp == 1 && lane == 0 && iters > 0) {
+      // ---------------------------------------------------------------- MMA issuer
+      constexpr uint32_t idesc_s = idesc(TM, TM, false);
       constexpr uint32_t idesc_o = idesc(TM, D, true);
       const uint32_t sk = smem_u32(smem + L::OFF_K), sv = smem_u32(smem + L::OFF_V);
-      bool ok = mbar_wait(smem_u32(kv_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
-      auto issue_sdp = [&](int it) -> bool {
-        const uint32_t st = it & 1, ph = (it >> 1) & 1;
-        if (!mbar_wait(smem_u32(&qdo_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
-        if (!mbar_wait(smem_u32(&s_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
+      auto issue_s = [&](int it) -> bool {
+        if (!mbar_wait(smem_u32(&q_full[it & 1]), (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        const uint32_t sq = smem_u32(smem + L::OFF_Q + st * L::BLOCK);
-        const uint32_t sdo = smem_u32(smem + L::OFF_DO + st * L::BLOCK);
+        const uint32_t sq = smem_u32(smem + L::OFF_Q + (it & 1) * L::TILE);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_S + st * BLK, kdesc(sk, kk, TM), kdesc(sq, kk, BLK), idesc_s, kk ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_DP + st * BLK, kdesc(sv, kk, TM), kdesc(sdo, kk, BLK), idesc_s, kk ? 1u : 0u);
-        umma_commit(smem_u32(&s_full[st]));
+          umma_f16(tmem + COL_S, kdesc(sk, kk, TM), kdesc(sq, kk, TM), idesc_s, kk ? 1u : 0u);
+        umma_commit(smem_u32(s_full));
         return true;
       };
-      if (ok && iters > 0) ok = issue_sdp(0);
+      bool ok = mbar_wait(smem_u32(kv_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
+      if (ok) ok = issue_s(0);
       for (int it = 0; it < iters && ok; ++it) {
-        if (it + 1 < iters) {
-          ok = issue_sdp(it + 1);
-          if (!ok) break;
-        }
         const uint32_t st = it & 1, ph = (it >> 1) & 1;
-        if (!mbar_wait(smem_u32(&pds_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+        const uint32_t sq = smem_u32(smem + L::OFF_Q + st * L::TILE);
+        const uint32_t sdo = smem_u32(smem + L::OFF_DO + st * L::TILE);
+        if (!mbar_wait(smem_u32(&do_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t sp = smem_u32(smem + L::OFF_P + st * L::PT);
-        const uint32_t sds = smem_u32(smem + L::OFF_DS + st * L::PT);
-        const uint32_t sq = smem_u32(smem + L::OFF_Q + st * L::BLOCK);
-        const uint32_t sdo = smem_u32(smem + L::OFF_DO + st * L::BLOCK);
 #pragma unroll
-        for (int kk = 0; kk < BLK / 16; ++kk)
-          umma_f16(tmem + COL_DV, kdesc(sp, kk, TM), mndesc(sdo, kk, BLK), idesc_o, (it | kk) ? 1u : 0u);
+        for (int kk = 0; kk < D / 16; ++kk)
+          umma_f16(tmem + COL_DP, kdesc(sv, kk, TM), kdesc(sdo, kk, TM), idesc_s, kk ? 1u : 0u);
+        umma_commit(smem_u32(dp_full));
+        if (!mbar_wait(smem_u32(p_full), it & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+        tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < BLK / 16; ++kk)
-          umma_f16(tmem + COL_DK, kdesc(sds, kk, TM), mndesc(sq, kk, BLK), idesc_o, (it | kk) ? 1u : 0u);
-        umma_commit(smem_u32(&pds_empty[st]));
-        umma_commit(smem_u32(&qdo_empty[st]));
+        for (int kk = 0; kk < TM / 16; ++kk)     // P, dS: 32 packed columns at the start of each 64-column half
+          umma_f16_ts(tmem + COL_DV, tmem + COL_S + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sdo, kk, TM), idesc_o,
+                      (it | kk) ? 1u : 0u);
+        umma_commit(smem_u32(&do_empty[st]));
+        if (it + 1 < iters && !issue_s(it + 1)) { ok = false; break; }
+        if (!mbar_wait(smem_u32(ds_full), it & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+        tc_fence_after();
+#pragma unroll
+        for (int kk = 0; kk < TM / 16; ++kk)
+          umma_f16_ts(tmem + COL_DK, tmem + COL_DP + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sq, kk, TM), idesc_o,
+                      (it | kk) ? 1u : 0u);
+        umma_commit(smem_u32(&q_empty[st]));
       }
       if (ok) umma_commit(smem_u32(out_full));
+    } else if (warp == 2) {
+      // ---------------------------------------------------------------- per-query values of the coming blocks
+      int h = h_first, qb = 0;
+      for (int it = 0; it < iters; ++it) {
+        const uint32_t b = it & 1, ph = (it >> 1) & 1;
+        float* c_lse = reinterpret_cast<float*>(smem + L::OFF_COL + b * L::COL_BYTES);
+        float* c_delta = c_lse + TM;
+        int* c_lo = reinterpret_cast<int*>(c_delta + TM);
+        int* c_hi = c_lo + TM;
+        const int i0 = (qb0 + qb) * TM;
+        float lse[4], dl[4];
+        int klo[4], khi[4], mxlo = 0, mnhi = INT_MAX;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * 32 + lane;
+          lse[u] = i < p.T ? p.lse[(long long)h * p.T + i] : 0.f;
+          dl[u] = i < p.T ? p.delta[(long long)h * p.T + i] : 0.f;
+          attn_row_range(p.k_lo, p.k_hi, i, p.T, klo[u], khi[u]);
+          mxlo = max(mxlo, klo[u]);
+          mnhi = min(mnhi, khi[u]);
+        }
+#pragma unroll
+        for (int s = 16; s; s >>= 1) {
+          mxlo = max(mxlo, __shfl_xor_sync(0xffffffffu, mxlo, s));
+          mnhi = min(mnhi, __shfl_xor_sync(0xffffffffu, mnhi, s));
+        }
+        if (!mbar_wait(smem_u32(&col_empty[b]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = u * 32 + lane;
+          c_lse[c] = (lse[u] == -INFINITY) ? 0.f : -lse[u] * LOG2E;    // -inf: such a query sees nothing, masked below
+          c_delta[c] = -dl[u];
+          c_lo[c] = klo[u];
+          c_hi[c] = khi[u];
+        }
+        if (lane == 0) {
+          c_hi[TM] = mxlo;
+          c_hi[TM + 1] = mnhi;
+        }
+        mbar_arrive(smem_u32(&col_full[b]));
+        if (++qb == nqb) { qb = 0; ++h; }
+      }
     }
   } else {
+    MCB_REGS_MATH();
     const int q = warp & 3;
-    const int grp = (warp - 2) >> 2;
+    const int grp = (warp - 4) >> 2;
     const int r = q * 32 + lane;            // key row of this thread
     const int n = n0 + r;
     const bool row_ok = n < p.Tk;
-    const int t = (threadIdx.x - 64) & 127; // 0..127 inside the group
     const uint32_t lane_addr = uint32_t(q * 32) << 16;
-    const uint32_t st = grp;
+    const uint32_t ts = tmem + lane_addr + COL_S + grp * HALF, td = tmem + lane_addr + COL_DP + grp * HALF;
+    const uint64_t cc = f32x2(p.scale_log2, p.scale_log2);
     bool ok = true;
-    for (int it = grp; it < iters && ok; it += 2) {
-      const uint32_t ph = (it >> 1) & 1;
-      const int h = h_first + it / nqb;
-      const int i0 = (qb0 + it % nqb) * BLK;
-      // per-column values of this query block; two buffers per group: a thread can run at most one of the group's
-      // iterations ahead of the slowest reader, because passing col_full needs every thread's arrival
-      const uint32_t cb = st * 2 + ph;
-      float* col_lse = reinterpret_cast<float*>(smem + L::OFF_COL + cb * L::COL_BYTES);
-      float* col_delta = col_lse + BLK;
-      int* col_lo = reinterpret_cast<int*>(col_delta + BLK);
-      int* col_hi = col_lo + BLK;
-      int* col_meta = col_hi + BLK;            // [0..1] largest k_lo, [2..3] smallest k_hi of each half of the block
-      {
-        const int c = t & (BLK - 1);
-        const int i = i0 + c;
-        if (t < BLK) {
-          int klo, khi;
-          attn_row_range(p.k_lo, p.k_hi, i, p.T, klo, khi);
-          col_lo[c] = klo;
-          col_hi[c] = khi;
-          int mxlo = klo, mnhi = khi;
-#pragma unroll
-          for (int sft = 16; sft; sft >>= 1) {
-            mxlo = max(mxlo, __shfl_xor_sync(0xffffffffu, mxlo, sft));
-            mnhi = min(mnhi, __shfl_xor_sync(0xffffffffu, mnhi, sft));
-          }
-          if ((t & 31) == 0) {
-            col_meta[t >> 5] = mxlo;
-            col_meta[2 + (t >> 5)] = mnhi;
-          }
-        } else {
-          const float l = i < p.T ? p.lse[(long long)h * p.T + i] : 0.f;
-          col_lse[c] = (l == -INFINITY) ? 0.f : l * LOG2E;    // such a query sees nothing: masked below
-          col_delta[c] = i < p.T ? p.delta[(long long)h * p.T + i] : 0.f;
-        }
-      }
-      mbar_arrive(smem_u32(&col_full[cb]));
-      if (!mbar_wait(smem_u32(&col_full[cb]), (it >> 2) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-      if (!mbar_wait(smem_u32(&s_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-      if (!mbar_wait(smem_u32(&pds_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-      tc_fence_after();
+    for (int it = 0; it < iters && ok; ++it) {
+      const uint32_t b = it & 1;
+      const float* c_lse = reinterpret_cast<const float*>(smem + L::OFF_COL + b * L::COL_BYTES) + grp * HALF;
+      const float* c_delta = c_lse + TM;
+      const int* c_lo = reinterpret_cast<const int*>(c_delta + TM);
+      const int* c_hi = c_lo + TM;
+      const int* c_meta = c_hi + TM - grp * HALF;
+      if (!mbar_wait(smem_u32(&col_full[b]), (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
       // every query of the block sees this key: largest lower bound <= n <= smallest upper bound
-      const bool full = row_ok && max(col_meta[0], col_meta[1]) <= n && n <= min(col_meta[2], col_meta[3]);
-      uint8_t* tile_p = smem + L::OFF_P + st * L::PT;
-      uint8_t* tile_ds = smem + L::OFF_DS + st * L::PT;
-#pragma unroll 1
-      for (int c = 0; c < BLK; c += 32) {
-        uint32_t s[32], dp[32];
-        tmem_ld_32x32(tmem + lane_addr + COL_S + st * BLK + c, s);
-        tmem_ld_32x32(tmem + lane_addr + COL_DP + st * BLK + c, dp);
-        tmem_ld_wait();
-        float pr[32], ds[32];
+      const bool full = __all_sync(0xffffffffu, row_ok && c_meta[0] <= n && n <= c_meta[1]);
+      if (!mbar_wait(smem_u32(s_full), it & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t pr[HALF];
+      tmem_ld_32x32_x64(ts, pr);
+      tmem_ld_wait();
+      uint32_t seen[2] = {0xffffffffu, 0xffffffffu};   // bit e: this key is visible to query e of the half block
+      if (!full) {
+        seen[0] = seen[1] = 0u;
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(col_lse + c + e);
-          const float4 d4 = *reinterpret_cast<const float4*>(col_delta + c + e);
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, dd[4] = {d4.x, d4.y, d4.z, d4.w};
-          if (full) {
+        for (int e = 0; e < HALF; e += 4) {
+          const int4 a = *reinterpret_cast<const int4*>(c_lo + e), z = *reinterpret_cast<const int4*>(c_hi + e);
+          const int aa[4] = {a.x, a.y, a.z, a.w}, zz[4] = {z.x, z.y, z.z, z.w};
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const float x = exp2f(__uint_as_float(s[e + u]) * p.scale_log2 - ls[u]);
-              pr[e + u] = x;
-              ds[e + u] = x * (__uint_as_float(dp[e + u]) - dd[u]) * p.scale;
-            }
-          } else {
-            const int4 s4 = *reinterpret_cast<const int4*>(col_lo + c + e);
-            const int4 h4 = *reinterpret_cast<const int4*>(col_hi + c + e);
-            const int ss[4] = {s4.x, s4.y, s4.z, s4.w}, hh[4] = {h4.x, h4.y, h4.z, h4.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const bool vis = row_ok && ss[u] <= n && n <= hh[u];
-              const float x = exp2f(__uint_as_float(s[e + u]) * p.scale_log2 - ls[u]);
-              pr[e + u] = vis ? x : 0.f;
-              ds[e + u] = vis ? x * (__uint_as_float(dp[e + u]) - dd[u]) * p.scale : 0.f;
-            }
-          }
+          for (int u = 0; u < 4; ++u)
+            seen[e >> 5] |= (row_ok && aa[u] <= n && n <= zz[u]) ? 1u << ((e + u) & 31) : 0u;
         }
-        store_row_chunk(tile_p, r, c, pr);
-        store_row_chunk(tile_ds, r, c, ds);
       }
+      uint32_t pk[HALF / 2];
+#pragma unroll
+      for (int e = 0; e < HALF; e += 4) {
+        const float4 l4 = *reinterpret_cast<const float4*>(c_lse + e);
+        const float2 x = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1])), cc, f32x2(l4.x, l4.y)));
+        const float2 y = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e + 2]), __uint_as_float(pr[e + 3])), cc, f32x2(l4.z, l4.w)));
+        float v[4] = {ex2_ftz(x.x), ex2_ftz(x.y), ex2_ftz(y.x), ex2_ftz(y.y)};
+        if (!full) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) v[u] = (seen[e >> 5] >> ((e + u) & 31)) & 1u ? v[u] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) pr[e + u] = __float_as_uint(v[u]);
+        pk[e >> 1] = pack_bf16x2(v[0], v[1]);
+        pk[(e >> 1) + 1] = pack_bf16x2(v[2], v[3]);
+      }
+      tmem_st_32x32(ts, pk);
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_empty[st]));
-      fence_proxy_async_smem();
-      mbar_arrive(smem_u32(&pds_full[st]));
+      if (lane == 0) mbar_arrive(smem_u32(p_full));
+      if (!mbar_wait(smem_u32(dp_full), it & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t dp[HALF];
+      tmem_ld_32x32_x64(td, dp);
+      tmem_ld_wait();
+#pragma unroll
+      for (int e = 0; e < HALF; e += 4) {
+        const float4 d4 = *reinterpret_cast<const float4*>(c_delta + e);
+        float2 x = f32x2_split(mul_f32x2(add_f32x2(f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1])), f32x2(d4.x, d4.y)),
+                                         f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1]))));
+        float2 y = f32x2_split(mul_f32x2(add_f32x2(f32x2(__uint_as_float(dp[e + 2]), __uint_as_float(dp[e + 3])), f32x2(d4.z, d4.w)),
+                                         f32x2(__uint_as_float(pr[e + 2]), __uint_as_float(pr[e + 3]))));
+        if (!full) {                              // a masked pair contributes zero whatever its dP is
+          const uint32_t m = seen[e >> 5] >> (e & 31);
+          x.x = m & 1u ? x.x : 0.f;
+          x.y = m & 2u ? x.y : 0.f;
+          y.x = m & 4u ? y.x : 0.f;
+          y.y = m & 8u ? y.y : 0.f;
+        }
+        pk[e >> 1] = pack_bf16x2(x.x, x.y);
+        pk[(e >> 1) + 1] = pack_bf16x2(y.x, y.y);
+      }
+      tmem_st_32x32(td, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(smem_u32(ds_full));
+        mbar_arrive(smem_u32(&col_empty[b]));
+      }
     }
+    // group 0 writes dV, group 1 writes dK
+    const long long row_off = ((long long)n * p.nkv + kvh) * D;
+    const long long plane = (long long)p.Tk * p.nkv * D;
     if (iters == 0) {
       // no query sees this tile's keys: zero gradients (the accumulators were never written)
-      const long long row_off = ((long long)n * p.nkv + kvh) * D;
       if (row_ok) {
         if (p.partial == nullptr) {
           uint4* dst = reinterpret_cast<uint4*>((grp == 0 ? p.dv : p.dk) + row_off);
 #pragma unroll 1
           for (int c = 0; c < D / 8; ++c) dst[c] = make_uint4(0, 0, 0, 0);
         } else {
-          const long long plane = (long long)p.Tk * p.nkv * D;
-          uint4* dst = reinterpret_cast<uint4*>(p.partial + ((long long)grp * p.splits + blockIdx.z) * plane + row_off);
+          uint4* dst = reinterpret_cast<uint4*>(p.partial + ((long long)grp * p.splits + split) * plane + row_off);
 #pragma unroll 1
           for (int c = 0; c < D / 4; ++c) dst[c] = make_uint4(0, 0, 0, 0);
         }
       }
     } else if (ok && mbar_wait(smem_u32(out_full), 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
-      // group 0 writes dV, group 1 writes dK
-      const long long row_off = ((long long)n * p.nkv + kvh) * D;
-      if (p.partial == nullptr) {
-        if (grp == 0) store_acc_row<D>(tmem + lane_addr + COL_DV, p.dv + row_off, row_ok);
-        else store_acc_row<D>(tmem + lane_addr + COL_DK, p.dk + row_off, row_ok);
-      } else {
-        const long long plane = (long long)p.Tk * p.nkv * D;
-        float* dst = p.partial + ((long long)grp * p.splits + blockIdx.z) * plane + row_off;
-        store_acc_row_f32<D>(tmem + lane_addr + (grp == 0 ? COL_DV : COL_DK), dst, row_ok);
-      }
+      const uint32_t acc = tmem + lane_addr + (grp == 0 ? COL_DV : COL_DK);
+      const float f = grp == 0 ? 1.f : p.scale;
+      if (p.partial == nullptr) store_acc_row<D>(acc, (grp == 0 ? p.dv : p.dk) + row_off, f, row_ok);
+      else store_acc_row_f32<D>(acc, p.partial + ((long long)grp * p.splits + split) * plane + row_off, f, row_ok);
     }
   }
   tc_fence_before();
@@ -701,22 +779,19 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* o, const
   const long long rows = (long long)p.T * p.nq;
   cudaError_t e = cudaSuccess;
   if (!delta_given) {
-    attn_bwd_delta_kernel<D><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(
+    constexpr int PER = 4 * 256 / (D / 8);      // rows of a block
+    attn_bwd_delta_kernel<D><<<(unsigned)((rows + PER - 1) / PER), 256, 0, stream>>>(
         (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, p.T, p.nq);
     e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
   }
-  CUtensorMap tq128, tdo128, tk64, tv64, tk128, tv128, tq64, tdo64;
+  CUtensorMap tq, tdo, tk, tv;
   const long long wq = (long long)p.nq * D, wk = (long long)p.nkv * D;
   int rc = 0;
-  if ((rc = make_tmap_2d_bf16(&tq128, q, wq, p.T, wq, 64, TM))) return rc;
-  if ((rc = make_tmap_2d_bf16(&tdo128, dout, wq, p.T, wq, 64, TM))) return rc;
-  if ((rc = make_tmap_2d_bf16(&tk64, k, wk, p.Tk, wk, 64, BLK))) return rc;
-  if ((rc = make_tmap_2d_bf16(&tv64, v, wk, p.Tk, wk, 64, BLK))) return rc;
-  if ((rc = make_tmap_2d_bf16(&tk128, k, wk, p.Tk, wk, 64, TM))) return rc;
-  if ((rc = make_tmap_2d_bf16(&tv128, v, wk, p.Tk, wk, 64, TM))) return rc;
-  if ((rc = make_tmap_2d_bf16(&tq64, q, wq, p.T, wq, 64, BLK))) return rc;
-  if ((rc = make_tmap_2d_bf16(&tdo64, dout, wq, p.T, wq, 64, BLK))) return rc;
+  if ((rc = make_tmap_2d_bf16(&tq, q, wq, p.T, wq, 64, TM))) return rc;
+  if ((rc = make_tmap_2d_bf16(&tdo, dout, wq, p.T, wq, 64, TM))) return rc;
+  if ((rc = make_tmap_2d_bf16(&tk, k, wk, p.Tk, wk, 64, TM))) return rc;
+  if ((rc = make_tmap_2d_bf16(&tv, v, wk, p.Tk, wk, 64, TM))) return rc;
   static bool cfg = false;
   if (!cfg) {
     e = cudaFuncSetAttribute(attn_bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem<D>::TOTAL);
@@ -726,11 +801,10 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* o, const
     cfg = true;
   }
   const int tiles = (p.T + TM - 1) / TM, ktiles = (p.Tk + TM - 1) / TM;
-  attn_bwd_dq_kernel<D><<<dim3(tiles, p.nq), BWD_THREADS, DqSmem<D>::TOTAL, stream>>>(tq128, tdo128, tk64, tv64, p);
+  attn_bwd_dq_kernel<D><<<(unsigned)tiles * p.nq, BWD_THREADS, DqSmem<D>::TOTAL, stream>>>(tq, tdo, tk, tv, p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
-  attn_bwd_dkv_kernel<D><<<dim3(ktiles, p.nkv, p.splits), BWD_THREADS, DkvSmem<D>::TOTAL, stream>>>(tk128, tv128, tq64,
-                                                                                                     tdo64, p);
+  attn_bwd_dkv_kernel<D><<<(unsigned)ktiles * p.nkv * p.splits, BWD_THREADS, DkvSmem<D>::TOTAL, stream>>>(tk, tv, tq, tdo, p);
   e = cudaGetLastError();
   if (e != cudaSuccess || p.partial == nullptr) return (int)e;
   const long long plane = (long long)p.Tk * p.nkv * D;

@@ -1,21 +1,26 @@
 // Variable-length causal GQA attention forward for sm_100a: S = Q K^T and O += P V on tcgen05 with accumulators in
-// TMEM, operands staged by TMA, softmax in registers.
+// TMEM, operands staged by TMA, softmax in registers, P handed to the second product through TMEM.
 //
-// One CTA per (128-query tile, query head).  The mask is a per-query inclusive key range [k_lo[i], k_hi[i]] (see
-// attn_common.cuh): packed causal self-attention is k_lo = first token of the query's sequence, k_hi = the query
-// itself, so tiles may straddle sequence boundaries and nothing is synchronised with the host; queries and keys may
-// also be different token sets (the steps of context-parallel ring attention, non-causal attention).
+// The mask is a per-query inclusive key range [k_lo[i], k_hi[i]] (see attn_common.cuh): packed causal self-attention is
+// k_lo = first token of the query's sequence, k_hi = the query itself, so tiles may straddle sequence boundaries and
+// nothing is synchronised with the host; queries and keys may also be different token sets (the steps of
+// context-parallel ring attention, non-causal attention).
 //
-// Two passes over the key blocks instead of online rescaling: pass 1 computes only the row maxima (Q K^T + max),
-// pass 2 recomputes S, forms P = exp2(S - max) and accumulates O += P V directly in TMEM with no correction step.
-// The extra Q K^T is cheap next to the exponentials, which bound attention on this architecture, and the kernel
-// needs no accumulator rescaling traffic.
+// One CTA works on two 128-query tiles at once and walks the key blocks either of them can see.  The exponentials of one
+// tile run while the tensor core multiplies for the other, and one K / V load serves both.  Online softmax with a lazy
+// reference: a row's accumulator is rescaled only when its maximum has grown by more than 2^8 over the reference in use
+// (P then stays below 256, where bf16 and fp32 have the same relative precision as below 1), which happens in the first
+// blocks of a row and hardly ever after them.
 //
-// Warp roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2..9 softmax in two groups of
-// four (thread = query row).  Group g owns score buffer g in TMEM, i.e. every other key block of both passes, so each
-// scheduler has two softmax warps to interleave (exponentials of one block overlap the TMEM reads of the next); the
-// groups exchange their partial row maxima after pass 1 and their partial row sums after pass 2 through shared memory.
-#include <type_traits>
+// Warp roles (384 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4..7 softmax of tile 0, warps 8..11
+// of tile 1 (thread = query row, a whole 128-column score row in registers: the control warps give registers up).  TMEM: S0 | S1 (128 columns each, P overwrites the scores it came from as packed bf16)
+// | O0 | O1.  The issuer's order is  PV_t(j), QK_t(j + 1)  for t = 0, 1: the score buffer of a tile is reused as soon as
+// its P has been multiplied, and MMAs of one thread complete in order.
+//
+// Bound: per 128 x 128 block the two products take 1024 tensor cycles and the 16384 exponentials 1024 MUFU cycles of an
+// SM, so both pipes are the floor; the two tiles in flight overlap them.  Measured, 32 query / 8 kv heads of 128, causal:
+// 16384 tokens 2.02 ms = 1090 TFLOP/s; the form before it (maxima in a first pass over Q K^T, one tile per CTA, P through
+// shared memory) took 3.35 ms.
 #include "../common/host_utils.cuh"
 #include "../common/ptx.cuh"
 #include "attn_common.cuh"
@@ -26,7 +31,7 @@ namespace {
 
 constexpr int BM = 128;  // queries per CTA
 constexpr int BNK = 128; // keys per block
-constexpr int ATT_THREADS = 320;
+constexpr int ATT_THREADS = 384;
 
 struct AttnParams {
   int T, Tk, nq, nkv, d;  // T queries, Tk keys
@@ -37,17 +42,22 @@ struct AttnParams {
   __nv_bfloat16* o;       // [T, nq, d]
   float* lse;             // [nq, T] natural log of sum exp(scaled scores); -inf for a query that sees no key
   int* status;
+  int pairing, per_row;   // how a CTA's two tiles are chosen; CTAs per row of tiles (set by the launcher)
 };
+
+// How the two tiles of a CTA are chosen.  PAIR_HEADS: two query heads of one kv group, same queries (the ranges are then
+// equal and no block is loaded for one tile only).  PAIR_ROWS: adjacent query tiles of one head (odd GQA ratios).
+// SOLO: one tile; taken when all tiles fit the GPU at once, where sharing an SM only makes each of them longer (and up to
+// half of the SMs would get nothing).
+enum { PAIR_HEADS = 0, PAIR_ROWS = 1, SOLO = 2 };
 
 template <int D>
 struct AttnSmem {
   static constexpr int TILE = BM * D * 2;            // one 128-row operand tile
-  static constexpr int P_BYTES = BM * BNK * 2;
-  static constexpr int OFF_Q = 0;
-  static constexpr int OFF_K = TILE;                  // 2 stages
+  static constexpr int OFF_Q = 0;                     // 2 tiles
+  static constexpr int OFF_K = 2 * TILE;              // 2 stages
   static constexpr int OFF_V = OFF_K + 2 * TILE;      // 2 stages
-  static constexpr int OFF_P = OFF_V + 2 * TILE;      // 2 buffers
-  static constexpr int OFF_BAR = OFF_P + 2 * P_BYTES;
+  static constexpr int OFF_BAR = OFF_V + 2 * TILE;
   static constexpr int TOTAL = OFF_BAR + 1024 + 1024;
 };
 
@@ -62,6 +72,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, bool b_mn) {
          (uint32_t(m >> 4) << 24);
 }
 
+// Largest growth of a row's maximum (log2 units) that is absorbed without rescaling the accumulator.
+constexpr float LAZY_LOG2 = 8.f;
+
 template <int D>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -73,44 +86,51 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
-  uint64_t* q_full = bars;            // 1
-  uint64_t* k_full = bars + 1;        // 2
-  uint64_t* k_empty = bars + 3;       // 2
-  uint64_t* v_full = bars + 5;        // 2
-  uint64_t* v_empty = bars + 7;       // 2
-  uint64_t* s_full = bars + 9;        // 2
-  uint64_t* s_empty = bars + 11;      // 2
-  uint64_t* p_full = bars + 13;       // 2
-  uint64_t* p_empty = bars + 15;      // 2
-  uint64_t* o_full = bars + 17;       // 1
-  uint64_t* xchg = bars + 18;         // 2: row maxima / row sums exchanged between the softmax groups
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  uint64_t* q_full = bars;            // 2, per tile
+  uint64_t* k_full = bars + 2;        // 2 stages
+  uint64_t* k_empty = bars + 4;       // 2
+  uint64_t* v_full = bars + 6;        // 2
+  uint64_t* v_empty = bars + 8;       // 2
+  uint64_t* s_full = bars + 10;       // 2, per tile
+  uint64_t* p_full = bars + 12;       // 2, per tile
+  uint64_t* o_done = bars + 14;       // 2, per tile: a P V product has completed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tile = gridDim.x - 1 - blockIdx.x;  // long tiles first
-  const int head = blockIdx.y;
-  const int kvh = head / (p.nq / p.nkv);
-  const int m0 = m_tile * BM;
-  __shared__ int s_rng[8];
-  tile_range_partial(p.k_lo, p.k_hi, m0, p.T, s_rng);
+  const int bx = blockIdx.x % p.per_row;
+  const int mt = (gridDim.x - 1 - blockIdx.x) / p.per_row;   // long tiles of every head first: the tail gets short ones
+  int head0, head1, m00, m01;
+  if (p.pairing == PAIR_HEADS) {
+    head0 = 2 * bx;
+    head1 = head0 + 1;
+    m00 = m01 = mt * BM;
+  } else if (p.pairing == PAIR_ROWS) {
+    head0 = head1 = bx;
+    m00 = 2 * mt * BM;
+    m01 = m00 + BM;
+  } else {
+    head0 = head1 = bx;
+    m00 = mt * BM;
+    m01 = p.T;                                    // past the end: an empty tile
+  }
+  const int kvh = head0 / (p.nq / p.nkv);
+  __shared__ int s_rng[2][8];
+  tile_range_partial(p.k_lo, p.k_hi, m00, p.T, s_rng[0]);
+  tile_range_partial(p.k_lo, p.k_hi, m01, p.T, s_rng[1]);
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    mbar_init(smem_u32(q_full), 1);
     for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&q_full[i]), 1);
       mbar_init(smem_u32(&k_full[i]), 1);
       mbar_init(smem_u32(&k_empty[i]), 1);
       mbar_init(smem_u32(&v_full[i]), 1);
       mbar_init(smem_u32(&v_empty[i]), 1);
       mbar_init(smem_u32(&s_full[i]), 1);
-      mbar_init(smem_u32(&s_empty[i]), 4);
-      mbar_init(smem_u32(&p_full[i]), 128);
-      mbar_init(smem_u32(&p_empty[i]), 1);
+      mbar_init(smem_u32(&p_full[i]), 4);
+      mbar_init(smem_u32(&o_done[i]), 1);
     }
-    mbar_init(smem_u32(o_full), 1);
-    mbar_init(smem_u32(&xchg[0]), 256);
-    mbar_init(smem_u32(&xchg[1]), 256);
     fence_barrier_init();
     fence_proxy_async_smem();
     prefetch_tensormap(&tm_q);
@@ -125,240 +145,229 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const int kmin = tile_range_min(s_rng), kmax = tile_range_max(s_rng);
-  const int kb0 = kmin / BNK;                      // first key block any row of this tile can see
-  const int nblk = kmax >= kmin ? kmax / BNK - kb0 + 1 : 0;
+  // key blocks [b0, b1) of each tile, and their union [jb, je)
+  int b0[2], b1[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int kmin = tile_range_min(s_rng[t]), kmax = tile_range_max(s_rng[t]);
+    b0[t] = kmax >= kmin ? kmin / BNK : 0;
+    b1[t] = kmax >= kmin ? kmax / BNK + 1 : 0;
+  }
+  const bool any0 = b1[0] > b0[0], any1 = b1[1] > b0[1];
+  const int jb = any0 ? (any1 ? min(b0[0], b0[1]) : b0[0]) : b0[1];
+  const int je = max(b1[0], b1[1]);
 
-  if (nblk <= 0) {
-    // no row of this tile sees any key: the output is zero and the log-sum-exp -inf
-    if (warp >= 2) {
-      const int grp = (warp - 2) >> 2;
-      const int i = m0 + (warp & 3) * 32 + lane;
-      if (i < p.T) {
-        uint4* orow = reinterpret_cast<uint4*>(p.o + ((long long)i * p.nq + head) * D + grp * (D / 2));
-#pragma unroll
-        for (int c = 0; c < D / 16; ++c) orow[c] = make_uint4(0, 0, 0, 0);
-        if (grp == 0) p.lse[(long long)head * p.T + i] = p.sinks ? p.sinks[head] : -INFINITY;
-      }
-    }
-  } else if (warp == 0) {
+  // 384 threads x 168 registers at launch: 128 x (104 + 200 + 200) = 64512
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+  if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      mbar_expect_tx(smem_u32(q_full), L::TILE);
+    if (lane == 0 && je > jb) {
 #pragma unroll
-      for (int b = 0; b < NBOX; ++b)
-        tma_load_2d(smem_u32(smem + L::OFF_Q + b * BM * 128), &tm_q, head * D + b * 64, m0, smem_u32(q_full));
-      uint32_t kit = 0;
-      bool ok = true;
-      for (int pass = 0; pass < 2 && ok; ++pass) {
-        for (int j = 0; j < nblk && ok; ++j, ++kit) {
-          const int n0 = (kb0 + j) * BNK;
-          const uint32_t st = kit & 1, ph = (kit >> 1) & 1;
-          if (!mbar_wait(smem_u32(&k_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-          mbar_expect_tx(smem_u32(&k_full[st]), L::TILE);
+      for (int t = 0; t < 2; ++t) {
+        if (!(t ? any1 : any0)) continue;
+        mbar_expect_tx(smem_u32(&q_full[t]), L::TILE);
 #pragma unroll
-          for (int b = 0; b < NBOX; ++b)
-            tma_load_2d(smem_u32(smem + L::OFF_K + st * L::TILE + b * BM * 128), &tm_k, kvh * D + b * 64, n0,
-                        smem_u32(&k_full[st]));
-          if (pass == 1) {
-            const uint32_t vst = j & 1, vph = (j >> 1) & 1;
-            if (!mbar_wait(smem_u32(&v_empty[vst]), vph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-            mbar_expect_tx(smem_u32(&v_full[vst]), L::TILE);
+        for (int b = 0; b < NBOX; ++b)
+          tma_load_2d(smem_u32(smem + L::OFF_Q + t * L::TILE + b * BM * 128), &tm_q, (t ? head1 : head0) * D + b * 64,
+                      t ? m01 : m00, smem_u32(&q_full[t]));
+      }
+      int n = 0, nv = 0;
+      for (int j = jb; j < je; ++j, ++n) {
+        const uint32_t st = n & 1, ph = (n >> 1) & 1;
+        if (!mbar_wait(smem_u32(&k_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_expect_tx(smem_u32(&k_full[st]), L::TILE);
 #pragma unroll
-            for (int b = 0; b < NBOX; ++b)
-              tma_load_2d(smem_u32(smem + L::OFF_V + vst * L::TILE + b * BM * 128), &tm_v, kvh * D + b * 64, n0,
-                          smem_u32(&v_full[vst]));
-          }
-        }
+        for (int b = 0; b < NBOX; ++b)
+          tma_load_2d(smem_u32(smem + L::OFF_K + st * L::TILE + b * BM * 128), &tm_k, kvh * D + b * 64, j * BNK,
+                      smem_u32(&k_full[st]));
+        if (!mbar_wait(smem_u32(&v_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ++n; break; }
+        mbar_expect_tx(smem_u32(&v_full[st]), L::TILE);
+#pragma unroll
+        for (int b = 0; b < NBOX; ++b)
+          tma_load_2d(smem_u32(smem + L::OFF_V + st * L::TILE + b * BM * 128), &tm_v, kvh * D + b * 64, j * BNK,
+                      smem_u32(&v_full[st]));
+        ++nv;
       }
       // drain: the last loads must land before the CTA exits
-      for (uint32_t i = (kit > 2 ? kit - 2 : 0); i < kit; ++i) {
+      auto drain = [](uint64_t* bar, uint32_t parity) {
         uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(smem_u32(&k_full[i & 1]), (i >> 1) & 1))
+        while (!mbar_try_wait(smem_u32(bar), parity))
           if (globaltimer_ns() - t0 > 200000000ull) break;
-      }
-      for (int j = (nblk > 2 ? nblk - 2 : 0); j < nblk; ++j) {
-        uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(smem_u32(&v_full[j & 1]), (j >> 1) & 1))
-          if (globaltimer_ns() - t0 > 200000000ull) break;
-      }
+      };
+      for (int i = (n > 2 ? n - 2 : 0); i < n; ++i) drain(&k_full[i & 1], (i >> 1) & 1);
+      for (int i = (nv > 2 ? nv - 2 : 0); i < nv; ++i) drain(&v_full[i & 1], (i >> 1) & 1);
+      if (any0) drain(&q_full[0], 0);
+      if (any1) drain(&q_full[1], 0);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (lane == 0 && je > jb) {
       constexpr uint32_t idesc_s = idesc_bf16(BM, BNK, false);
       constexpr uint32_t idesc_o = idesc_bf16(BM, D, true);
-      const uint32_t sq = smem_u32(smem + L::OFF_Q);
-      bool ok = mbar_wait(smem_u32(q_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
-      uint32_t kit = 0, sit = 0;
-      auto issue_s = [&](uint32_t kit_, uint32_t sit_) -> bool {
-        const uint32_t st = kit_ & 1, ph = (kit_ >> 1) & 1, sb = sit_ & 1, sph = (sit_ >> 1) & 1;
-        if (!mbar_wait(smem_u32(&k_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
-        if (!mbar_wait(smem_u32(&s_empty[sb]), sph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
-        tc_fence_after();
-        const uint32_t sk = smem_u32(smem + L::OFF_K + st * L::TILE);
+      bool ok = true;
+      for (int j = jb - 1; j < je && ok; ++j) {
+        const uint32_t st = (j - jb) & 1, ph = ((j - jb) >> 1) & 1;          // V stage of block j
+        const uint32_t kst = (j + 1 - jb) & 1, kph = ((j + 1 - jb) >> 1) & 1;  // K stage of block j + 1
+        bool v_seen = false, k_seen = false;
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_S + sb * BNK, kmajor_desc<D>(sq, kk), kmajor_desc<D>(sk, kk), idesc_s, kk ? 1u : 0u);
-        umma_commit(smem_u32(&k_empty[st]));
-        umma_commit(smem_u32(&s_full[sb]));
-        return true;
-      };
-      // pass 1: row maxima
-      for (int j = 0; j < nblk && ok; ++j, ++kit, ++sit) ok = issue_s(kit, sit);
-      // pass 2: S again, then O += P V one block behind
-      if (ok) ok = issue_s(kit, sit);
-      ++kit; ++sit;
-      for (int j = 0; j < nblk && ok; ++j) {
-        if (j + 1 < nblk) {
-          ok = issue_s(kit, sit);
-          ++kit; ++sit;
-          if (!ok) break;
-        }
-        const uint32_t pb = j & 1, pph = (j >> 1) & 1;
-        if (!mbar_wait(smem_u32(&p_full[pb]), pph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-        if (!mbar_wait(smem_u32(&v_full[pb]), pph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t sp = smem_u32(smem + L::OFF_P + pb * L::P_BYTES);
-        const uint32_t sv = smem_u32(smem + L::OFF_V + pb * L::TILE);
+        for (int t = 0; t < 2; ++t) {
+          if (j >= b0[t] && j < b1[t]) {
+            const uint32_t n = j - b0[t];
+            if (!v_seen) {
+              if (!mbar_wait(smem_u32(&v_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+              v_seen = true;
+            }
+            if (!mbar_wait(smem_u32(&p_full[t]), n & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t sv = smem_u32(smem + L::OFF_V + st * L::TILE);
 #pragma unroll
-        for (int kk = 0; kk < BNK / 16; ++kk) {
-          const uint64_t ad = make_smem_desc_sw128(sp + (kk >> 2) * (BM * 128) + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc_sw128(sv + kk * 2048, BM * 128, 1024);
-          umma_f16(tmem + COL_O, ad, bd, idesc_o, (j | kk) ? 1u : 0u);
+            for (int kk = 0; kk < BNK / 16; ++kk)
+              umma_f16_ts(tmem + COL_O + t * 128, tmem + COL_S + t * BNK + kk * 8,
+                          make_smem_desc_sw128(sv + kk * 2048, BM * 128, 1024), idesc_o, (n | kk) ? 1u : 0u);
+            umma_commit(smem_u32(&o_done[t]));
+          }
+          if (j + 1 >= b0[t] && j + 1 < b1[t]) {
+            if (!k_seen) {
+              if (!mbar_wait(smem_u32(&k_full[kst]), kph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+              k_seen = true;
+            }
+            if (j + 1 == b0[t] &&
+                !mbar_wait(smem_u32(&q_full[t]), 0, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t sq = smem_u32(smem + L::OFF_Q + t * L::TILE);
+            const uint32_t sk = smem_u32(smem + L::OFF_K + kst * L::TILE);
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk)
+              umma_f16(tmem + COL_S + t * BNK, kmajor_desc<D>(sq, kk), kmajor_desc<D>(sk, kk), idesc_s, kk ? 1u : 0u);
+            umma_commit(smem_u32(&s_full[t]));
+          }
         }
-        umma_commit(smem_u32(&p_empty[pb]));
-        umma_commit(smem_u32(&v_empty[pb]));
+        // a block neither tile needs (ranges with a gap between them) must have landed too before its stage is reused
+        if (ok && j >= jb && !v_seen) ok = mbar_wait(smem_u32(&v_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL);
+        if (ok && j + 1 < je && !k_seen) ok = mbar_wait(smem_u32(&k_full[kst]), kph, abort_flag, p.status, ST_TIMEOUT_FULL);
+        if (!ok) break;
+        if (j >= jb) umma_commit(smem_u32(&v_empty[st]));
+        if (j + 1 < je) umma_commit(smem_u32(&k_empty[kst]));
       }
-      if (ok) umma_commit(smem_u32(o_full));
     }
+  }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
     // ------------------------------------------------------------------ softmax warps: thread = query row
     const int q = warp & 3;
-    const int grp = (warp - 2) >> 2;
+    const int t = (warp - 4) >> 2;
     const int r = q * 32 + lane;
-    const int i = m0 + r;
+    const int head = t ? head1 : head0;
+    const int i = (t ? m01 : m00) + r;
+    const int jfirst = t ? b0[1] : b0[0], jlast = t ? b1[1] : b1[0];
     const bool row_ok = i < p.T;
+    const uint32_t lane_addr = uint32_t(q * 32) << 16;
+    const uint32_t ts = tmem + lane_addr + COL_S + t * BNK, to = tmem + lane_addr + COL_O + t * 128;
     int lo, hi;
     attn_row_range(p.k_lo, p.k_hi, i, p.T, lo, hi);
-    const uint32_t lane_addr = uint32_t(q * 32) << 16;
-    const uint32_t sb = grp;                         // this group's score buffer
-    float mx = -INFINITY;
+    if (lo > hi) lo = hi = 0x40000000;            // sees nothing: a range no key index reaches
+    const unsigned span = (unsigned)(hi - lo);    // key k is visible iff (unsigned)(k - lo) <= span
+    float mref = -INFINITY;                       // reference maximum, log2 units
+    uint64_t sum2 = 0;                            // two fp32 partial row sums
     bool ok = true;
-    // pass 1: score iterations sit = j (this group takes sit & 1 == grp)
-    for (int j = grp; j < nblk && ok; j += 2) {
-      const uint32_t sph = (uint32_t(j) >> 1) & 1;
-      if (!mbar_wait(smem_u32(&s_full[sb]), sph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+    for (int j = jfirst; j < jlast && ok; ++j) {
+      const uint32_t n = j - jfirst;
+      if (!mbar_wait(smem_u32(&s_full[t]), n & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      const int n0 = (kb0 + j) * BNK;
-      const bool full = (lo <= n0) && (n0 + BNK - 1 <= hi);
-      // the whole 128-column row in one TMEM round trip; the score buffer is released as soon as the values are in
-      // registers, so the next QK^T of this group overlaps the arithmetic below
-      uint32_t v0[64], v1[64];
-      tmem_ld_32x32_x64(tmem + lane_addr + COL_S + sb * BNK, v0);
-      tmem_ld_32x32_x64(tmem + lane_addr + COL_S + sb * BNK + 64, v1);
+      uint32_t v[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + 32 * c, v[c]);
       tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_empty[sb]));
-      if (full) {
+      const int n0 = j * BNK;
+      const bool full = __all_sync(0xffffffffu, lo <= n0 && n0 + BNK - 1 <= hi) && p.scale_log2 > 0.f;
+      float mx, mul = p.scale_log2;               // mul: what the scores in registers still have to be multiplied by
+      if (!full) {
 #pragma unroll
-        for (int e = 0; e < 64; ++e) mx = fmaxf(mx, fmaxf(__uint_as_float(v0[e]), __uint_as_float(v1[e])));
-      } else {
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int e = 0; e < 64; ++e) {
-          const int key = n0 + e;
-          if (key >= lo && key <= hi) mx = fmaxf(mx, __uint_as_float(v0[e]));
-          if (key + 64 >= lo && key + 64 <= hi) mx = fmaxf(mx, __uint_as_float(v1[e]));
+          for (int e = 0; e < 32; ++e)
+            v[c][e] = (unsigned)(n0 + 32 * c + e - lo) <= span ? __float_as_uint(__uint_as_float(v[c][e]) * mul)
+                                                               : 0xff800000u;
+        mul = 1.f;
+      }
+      {
+        float m4[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          m4[c] = __uint_as_float(v[c][0]);
+#pragma unroll
+          for (int e = 1; e < 32; ++e) m4[c] = fmaxf(m4[c], __uint_as_float(v[c][e]));
+        }
+        mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * mul;
+      }
+      if (mref == -INFINITY) {
+        mref = mx;                                // nothing accumulated yet (sum and accumulator are zero)
+      }
+      const bool grow = mx > mref + LAZY_LOG2;
+      if (__any_sync(0xffffffffu, grow)) {
+        // the accumulator must hold every product issued so far; P of this block has not been handed over yet
+        if (!mbar_wait(smem_u32(&o_done[t]), (n & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        tc_fence_after();
+        const float f = grow ? ex2_ftz(mref - mx) : 1.f;
+        if (grow) mref = mx;
+        sum2 = mul_f32x2(sum2, f32x2(f, f));
+#pragma unroll 1
+        for (int c = 0; c < D; c += 32) {
+          uint32_t o[32];
+          tmem_ld_32x32(to + c, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+          tmem_st_32x32(to + c, o);
         }
       }
+      const float m2 = mref == -INFINITY ? 0.f : mref;
+      const uint64_t cc = f32x2(mul, mul), mm = f32x2(-m2, -m2);
+#pragma unroll
+      for (int c = 0; c < 4; c += 2) {
+        uint32_t pk[32];
+#pragma unroll
+        for (int e = 0; e < 64; e += 2) {
+          const float2 x = f32x2_split(fma_f32x2(
+              f32x2(__uint_as_float(v[c + (e >> 5)][e & 31]), __uint_as_float(v[c + (e >> 5)][(e & 31) + 1])), cc, mm));
+          const float e0 = ex2_ftz(x.x), e1 = ex2_ftz(x.y);
+          sum2 = add_f32x2(sum2, f32x2(e0, e1));
+          pk[e >> 1] = pack_bf16x2(e0, e1);
+        }
+        tmem_st_32x32(ts + 16 * c, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&p_full[t]));
     }
-    // The row maximum is over both groups' blocks.  The partial maxima travel through the P buffers, which nothing
-    // has written yet: a group leaves its value in the buffer the *other* group owns in pass 2, so the value is
-    // overwritten only by its reader, after it has been read.
-    {
-      const int pb_mine = (grp + nblk) & 1;
-      reinterpret_cast<float*>(smem + L::OFF_P + (pb_mine ^ 1) * L::P_BYTES)[r] = mx;
-      mbar_arrive(smem_u32(&xchg[0]));
-      if (ok && !mbar_wait(smem_u32(&xchg[0]), 0, abort_flag, p.status, ST_TIMEOUT_FULL)) ok = false;
-      if (ok) mx = fmaxf(mx, reinterpret_cast<const float*>(smem + L::OFF_P + pb_mine * L::P_BYTES)[r]);
-    }
+    const float2 sp = f32x2_split(sum2);
+    float sum = sp.x + sp.y;
+    const bool seen = jlast > jfirst;
     // learnable softmax sink: an extra logit (already in softmax units, no scale) in the row's maximum and sum
     const float sink2 = p.sinks ? p.sinks[head] * 1.4426950408889634f : -INFINITY;
-    const float m_tot = fmaxf((mx == -INFINITY) ? -INFINITY : mx * p.scale_log2, sink2);
-    const float m2 = (m_tot == -INFINITY) ? 0.f : m_tot;
-    float sum = (p.sinks && grp == 0) ? exp2f(sink2 - m2) : 0.f;
-    // pass 2: score iterations sit = nblk + j; this group takes the j with (nblk + j) & 1 == grp, which all share
-    // one P buffer
-    const int j0 = (grp + nblk) & 1;
-    for (int j = j0; j < nblk && ok; j += 2) {
-      const uint32_t sit = uint32_t(nblk + j);
-      const uint32_t sph = (sit >> 1) & 1, pb = j & 1, pph = (uint32_t(j) >> 1) & 1;
-      if (!mbar_wait(smem_u32(&s_full[sb]), sph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t v0[64], v1[64];
-      tmem_ld_32x32_x64(tmem + lane_addr + COL_S + sb * BNK, v0);
-      tmem_ld_32x32_x64(tmem + lane_addr + COL_S + sb * BNK + 64, v1);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_empty[sb]));   // scores are in registers: the next QK^T may start
-      if (!mbar_wait(smem_u32(&p_empty[pb]), pph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-      const int n0 = (kb0 + j) * BNK;
-      const bool full = (lo <= n0) && (n0 + BNK - 1 <= hi);
-      uint8_t* prow = smem + L::OFF_P + pb * L::P_BYTES + r * 128;
-      auto half = [&](const uint32_t (&v)[64], int c0, auto fullc) {
-        constexpr bool FULL = decltype(fullc)::value;
-        uint8_t* box = prow + (c0 >> 6) * (BM * 128);
+    const float mtot = fmaxf(mref, sink2);
+    const float fold = mref == -INFINITY ? 0.f : ex2_ftz(mref - mtot);
+    sum = sum * fold + (p.sinks ? ex2_ftz(sink2 - mtot) : 0.f);
+    const float inv = sum > 0.f ? fold / sum : 0.f;
+    __nv_bfloat16* orow = p.o + ((long long)i * p.nq + head) * D;
+    if (!seen) {
+      // no row of this tile sees any key: the output is zero
+      if (row_ok) {
 #pragma unroll
-        for (int e = 0; e < 64; e += 8) {
-          float pv[8];
-#pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const float x = exp2f(__uint_as_float(v[e + t]) * p.scale_log2 - m2);
-            const int key = n0 + c0 + e + t;
-            pv[t] = (FULL || (key >= lo && key <= hi)) ? x : 0.f;
-            sum += pv[t];
-          }
-          uint4 o;
-          o.x = pack_bf16x2(pv[0], pv[1]);
-          o.y = pack_bf16x2(pv[2], pv[3]);
-          o.z = pack_bf16x2(pv[4], pv[5]);
-          o.w = pack_bf16x2(pv[6], pv[7]);
-          *reinterpret_cast<uint4*>(box + (((e >> 3) ^ (r & 7)) << 4)) = o;
-        }
-      };
-      if (full) {
-        half(v0, 0, std::true_type{});
-        half(v1, 64, std::true_type{});
-      } else {
-        half(v0, 0, std::false_type{});
-        half(v1, 64, std::false_type{});
+        for (int c = 0; c < D / 8; ++c) reinterpret_cast<uint4*>(orow)[c] = make_uint4(0, 0, 0, 0);
       }
-      fence_proxy_async_smem();   // P stores -> visible to the tensor core's shared-memory reads
-      mbar_arrive(smem_u32(&p_full[pb]));
-    }
-    // once every MMA has completed the Q tile is free: the partial row sums are exchanged through it
-    const bool done = ok && mbar_wait(smem_u32(o_full), 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
-    float* sbuf = reinterpret_cast<float*>(smem + L::OFF_Q);
-    if (done) sbuf[grp * BM + r] = sum;
-    mbar_arrive(smem_u32(&xchg[1]));
-    if (done && mbar_wait(smem_u32(&xchg[1]), 0, abort_flag, p.status, ST_TIMEOUT_FULL)) {
-      sum += sbuf[(grp ^ 1) * BM + r];
+    } else if (ok && mbar_wait(smem_u32(&o_done[t]), (jlast - jfirst - 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
-      const float inv = sum > 0.f ? 1.f / sum : 0.f;
-      // each group writes half of the head dimension
-      __nv_bfloat16* orow = p.o + ((long long)i * p.nq + head) * D + grp * (D / 2);
-      constexpr int OW = (D / 2 >= 64) ? 64 : 32;   // columns per TMEM load
 #pragma unroll 1
-      for (int c = 0; c < D / 2; c += OW) {
-        uint32_t v[OW];
-        if constexpr (OW == 64) tmem_ld_32x32_x64(tmem + lane_addr + COL_O + grp * (D / 2) + c, v);
-        else tmem_ld_32x32(tmem + lane_addr + COL_O + grp * (D / 2) + c, v);
+      for (int c = 0; c < D; c += 64) {
+        uint32_t v[64];
+        tmem_ld_32x32_x64(to + c, v);
         tmem_ld_wait();
         if (row_ok) {
 #pragma unroll
-          for (int e = 0; e < OW; e += 8) {
+          for (int e = 0; e < 64; e += 8) {
             uint4 o;
             o.x = pack_bf16x2(__uint_as_float(v[e]) * inv, __uint_as_float(v[e + 1]) * inv);
             o.y = pack_bf16x2(__uint_as_float(v[e + 2]) * inv, __uint_as_float(v[e + 3]) * inv);
@@ -368,9 +377,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
       }
-      if (row_ok && grp == 0)
-        p.lse[(long long)head * p.T + i] = (sum > 0.f) ? (m2 + log2f(sum)) * 0.6931471805599453f : -INFINITY;
     }
+    if (row_ok && ok)
+      p.lse[(long long)head * p.T + i] = sum > 0.f ? (mtot + log2f(sum)) * 0.6931471805599453f : -INFINITY;
   }
   tc_fence_before();
   __syncthreads();
@@ -381,7 +390,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 }
 
 template <int D>
-int launch_fwd(const void* q, const void* k, const void* v, const AttnParams& p, cudaStream_t stream) {
+int launch_fwd(const void* q, const void* k, const void* v, AttnParams p, cudaStream_t stream) {
   CUtensorMap tq, tk, tv;
   int rc = make_tmap_2d_bf16(&tq, q, (long long)p.nq * D, p.T, (long long)p.nq * D, 64, BM);
   if (rc) return rc;
@@ -395,7 +404,10 @@ int launch_fwd(const void* q, const void* k, const void* v, const AttnParams& p,
     if (e != cudaSuccess) return (int)e;
     cfg = true;
   }
-  dim3 grid((p.T + BM - 1) / BM, p.nq);
+  const int tiles = (p.T + BM - 1) / BM, qpg = p.nq / p.nkv;
+  p.pairing = tiles * p.nq <= device_sm_count() ? SOLO : (qpg % 2 == 0 ? PAIR_HEADS : PAIR_ROWS);
+  p.per_row = p.pairing == PAIR_HEADS ? p.nq / 2 : p.nq;
+  const unsigned grid = (unsigned)p.per_row * (p.pairing == PAIR_ROWS ? (tiles + 1) / 2 : tiles);
   attn_fwd_kernel<D><<<grid, ATT_THREADS, AttnSmem<D>::TOTAL, stream>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
@@ -412,7 +424,7 @@ int mcb_attn_fwd_ranges(const void* q, const void* k, const void* v, const int* 
                         int* status, void* stream_) {
   if (T == 0) return 0;
   if (nq % nkv || Tk <= 0 || (k_hi == nullptr && Tk < T)) return -2;
-  AttnParams p{T, Tk, nq, nkv, d, scale * 1.4426950408889634f, k_lo, k_hi, sinks, (__nv_bfloat16*)o, lse, status};
+  AttnParams p{T, Tk, nq, nkv, d, scale * 1.4426950408889634f, k_lo, k_hi, sinks, (__nv_bfloat16*)o, lse, status, SOLO, nq};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
   if (d == 128) return launch_fwd<128>(q, k, v, p, s);
   if (d == 64) return launch_fwd<64>(q, k, v, p, s);

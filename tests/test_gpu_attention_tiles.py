@@ -1,0 +1,82 @@
+"""Attention kernels at the edges of their tiles: one to a few 128-row query tiles and key blocks, every way the forward
+kernel pairs tiles (two heads of a group, two row tiles, alone), windows, sinks and ranges with gaps, against fp64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = 'cuda'
+
+CASES = [   # queries, keys, query heads, kv heads, head size, mask
+    (1, 1, 1, 1, 64, 'causal'), (127, 127, 4, 2, 64, 'packed'), (128, 128, 3, 1, 128, 'causal'),
+    (129, 129, 6, 2, 128, 'packed'), (1100, 1100, 32, 8, 128, 'packed'),       # paired heads
+    (1300, 1300, 24, 8, 64, 'window'),                                         # paired rows (odd group size)
+    (2100, 2100, 9, 3, 128, 'window'), (2000, 2000, 64, 8, 64, 'sinks'),
+    (700, 1300, 32, 4, 128, 'ranges'), (1300, 700, 30, 10, 64, 'ranges'), (900, 2000, 24, 8, 128, 'gaps'),
+]
+
+
+def _mask(T, Tk, kind, gen):
+    """Per-query inclusive key ranges (lo, hi or None = own index) and, for general ranges, per-key query bounds."""
+    i = torch.arange(T, device=DEV, dtype=torch.int32)
+    lo, hi, ql, qh = torch.zeros_like(i), None, None, None
+    if kind in ('packed', 'window', 'sinks'):
+        from mcore_bridge_b200.ops.attention_cuda import seq_start_from_cu
+        cu = torch.tensor(sorted({0, T // 7, T // 3, T // 3 + 5, T}), dtype=torch.int32, device=DEV)
+        lo = seq_start_from_cu(cu, T, DEV)
+    if kind in ('window', 'sinks'):
+        lo = torch.maximum(lo, i - 100)
+    if kind == 'ranges':        # arbitrary, some empty
+        lo = torch.randint(0, Tk, (T,), generator=gen, device=DEV, dtype=torch.int32)
+        hi = (lo + torch.randint(-20, Tk // 2, (T,), generator=gen, device=DEV, dtype=torch.int32)).clamp(max=Tk - 1)
+    if kind == 'gaps':          # tiles of one CTA see key blocks far apart
+        lo = torch.where(i % 300 < 150, 0, Tk - 200).int()
+        hi = lo + 150
+    keys = torch.arange(Tk, device=DEV)
+    vis = (keys[None] >= lo[:, None]) & (keys[None] <= (i if hi is None else hi)[:, None])
+    if hi is not None:
+        seen = vis.any(0)
+        ql = torch.where(seen, vis.int().argmax(0), 1).int()
+        qh = torch.where(seen, T - 1 - vis.flip(0).int().argmax(0), 0).int()
+    return lo.contiguous(), hi, ql, qh, vis
+
+
+@pytest.mark.parametrize('sharp', [1.0, 6.0])       # 6: row maxima grow past the lazy-rescale threshold
+@pytest.mark.parametrize('T,Tk,nq,nkv,d,kind', CASES)
+def test_tile_edges_match_fp64(T, Tk, nq, nkv, d, kind, sharp):
+    from mcore_bridge_b200.ops import _lib
+    from mcore_bridge_b200.ops.attention_cuda import attention_ranges
+    gen = torch.Generator(device=DEV).manual_seed(3)
+
+    def rand(*shape):
+        return torch.randn(*shape, generator=gen, device=DEV)
+
+    q, k, v = (rand(T, nq, d) * sharp).bfloat16(), rand(Tk, nkv, d).bfloat16(), rand(Tk, nkv, d).bfloat16()
+    sinks = rand(nq) * 3 if kind == 'sinks' else None
+    leaves = [t.requires_grad_() for t in ([q, k, v] + ([sinks] if sinks is not None else []))]
+    lo, hi, ql, qh, vis = _mask(T, Tk, kind, gen)
+    o, lse = attention_ranges(q, k, v, lo, hi, ql, qh, d ** -0.5, sinks)
+    dy = rand(T, nq, d).bfloat16()
+    grads = torch.autograd.grad(o, leaves, dy)
+    _lib.check_status()
+
+    wide = [t.detach().double().requires_grad_() for t in leaves]
+    qw, kw, vw = (t.transpose(0, 1) for t in wide[:3])
+    kw, vw = (t.repeat_interleave(nq // nkv, 0) for t in (kw, vw))
+    s = (qw @ kw.transpose(1, 2) * d ** -0.5).masked_fill(~vis[None], -1e30)
+    if sinks is not None:
+        s = torch.cat([s, wide[3].view(nq, 1, 1).expand(nq, T, 1)], -1)
+    p = torch.softmax(s, -1)[..., :Tk] * vis[None]
+    ref = (p @ vw).transpose(0, 1)
+    want = torch.autograd.grad(ref, wide, dy.double())
+
+    def rel(a, b):
+        return ((a.double() - b).norm() / b.norm().clamp(min=1e-30)).item()
+
+    # bf16 probabilities and a bf16 result: at most 2^-9 relative each; the gradients add bf16 dS, dO sums and results
+    assert rel(o, ref) < 2 ** -8
+    for a, b in zip(grads, want):
+        assert rel(a, b) < 2 ** -7
+    some = vis.any(1) if sinks is None else torch.ones(T, dtype=torch.bool, device=DEV)
+    exact = torch.logsumexp(s, -1)
+    assert (lse[:, some].double() - exact[:, some]).abs().max() < 1e-4      # fp32 sums of up to 2100 terms, |lse| < 100
+    assert torch.isneginf(lse[:, ~some]).all() and (o[~some] == 0).all()
