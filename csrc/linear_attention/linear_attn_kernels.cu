@@ -2,8 +2,7 @@
 //
 //   causal depthwise conv1d (+SiLU) forward / backward over packed sequences          (memory bound)
 //   gated RMSNorm  y = rmsnorm(x) * w * silu(z)  forward / backward                  (memory bound)
-//   simple gated linear attention with a constant per-head decay, forward / backward (recurrent, fp32 state in
-//   registers):   S_t = exp(g_h) S_{t-1} + k_t v_t^T,   o_t = scale * S_t^T q_t
+//   (simple gated linear attention: simple_gla.cu)
 //
 // Packed sequences are described by `seq_start[t]` (index of the first token of t's sequence), as in the attention
 // kernels: no host synchronisation, histories never cross a sequence boundary.
@@ -252,119 +251,6 @@ __global__ void gated_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, co
   for (int i = threadIdx.x; i < D; i += blockDim.x) atomicAdd(&dw[i], dws[i]);
 }
 
-// ------------------------------------------------------------------------------------------ simple GLA (recurrent)
-// q, k [T, H, DK], v, o [T, H, DV] bf16; decay[h] = g_h <= 0 (log-decay per step); one CTA of DV threads per
-// (sequence, head): thread j keeps column j of the state S [DK x DV] in registers.  q and k of the current token are
-// staged in shared memory (double buffered) so every thread reads them as broadcasts.
-template <int DK, int DV>
-__global__ void __launch_bounds__(DV)
-simple_gla_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                      const __nv_bfloat16* __restrict__ v, const float* __restrict__ decay,
-                      const int* __restrict__ cu_seqlens, __nv_bfloat16* __restrict__ o, int H, float scale) {
-  __shared__ float qs[2][DK], ks[2][DK];
-  const int seq = blockIdx.x, h = blockIdx.y, j = threadIdx.x;
-  const int t0 = cu_seqlens[seq], t1 = cu_seqlens[seq + 1];
-  const float a = __expf(decay[h]);
-  float S[DK];
-#pragma unroll
-  for (int i = 0; i < DK; ++i) S[i] = 0.f;
-  auto stage = [&](int t, int b) {
-    for (int i = j; i < DK; i += DV) {
-      qs[b][i] = __bfloat162float(q[((long long)t * H + h) * DK + i]) * scale;
-      ks[b][i] = __bfloat162float(k[((long long)t * H + h) * DK + i]);
-    }
-  };
-  if (t0 < t1) stage(t0, 0);
-  __syncthreads();
-  for (int t = t0; t < t1; ++t) {
-    const int b = (t - t0) & 1;
-    if (t + 1 < t1) stage(t + 1, b ^ 1);
-    const float vj = __bfloat162float(v[((long long)t * H + h) * DV + j]);
-    float acc = 0.f;
-#pragma unroll
-    for (int i = 0; i < DK; ++i) {
-      S[i] = fmaf(S[i], a, ks[b][i] * vj);
-      acc = fmaf(S[i], qs[b][i], acc);
-    }
-    o[((long long)t * H + h) * DV + j] = __float2bfloat16(acc);
-    __syncthreads();
-  }
-}
-
-// Backward in three sweeps with no stored states (DK == DV == number of threads).
-//   forward sweep, thread = row i of S_t :      dq_t[i] = scale * sum_c S_t[i, c] do_t[c]
-//   reverse sweep, thread = row i of R_t :      R_t = a R_{t+1} + scale * q_t do_t^T,   dk_t[i] = sum_c R_t[i, c] v_t[c]
-//   reverse sweep, thread = column c of R_t :   dv_t[c] = sum_i R_t[i, c] k_t[i]
-// Owning rows for dq / dk and columns for dv keeps every reduction inside a thread.
-template <int DK, int DV>
-__global__ void __launch_bounds__(DK)
-simple_gla_bwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                      const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ dout,
-                      const float* __restrict__ decay, const int* __restrict__ cu_seqlens,
-                      __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-                      int H, float scale) {
-  static_assert(DK == DV, "square state only");
-  __shared__ float sa[DV], sb[DV];
-  const int seq = blockIdx.x, h = blockIdx.y, i = threadIdx.x;
-  const int t0 = cu_seqlens[seq], t1 = cu_seqlens[seq + 1];
-  const float a = __expf(decay[h]);
-  float M[DV];
-  // ---- forward sweep: dq (row i of S)
-#pragma unroll
-  for (int c = 0; c < DV; ++c) M[c] = 0.f;
-  for (int t = t0; t < t1; ++t) {
-    const long long base = (long long)t * H + h;
-    sa[i] = __bfloat162float(v[base * DV + i]);
-    sb[i] = __bfloat162float(dout[base * DV + i]);
-    __syncthreads();
-    const float ki = __bfloat162float(k[base * DK + i]);
-    float acc = 0.f;
-#pragma unroll
-    for (int c = 0; c < DV; ++c) {
-      M[c] = fmaf(M[c], a, ki * sa[c]);
-      acc = fmaf(M[c], sb[c], acc);
-    }
-    dq[base * DK + i] = __float2bfloat16(acc * scale);
-    __syncthreads();
-  }
-  // ---- reverse sweep: dk (row i of R)
-#pragma unroll
-  for (int c = 0; c < DV; ++c) M[c] = 0.f;
-  for (int t = t1 - 1; t >= t0; --t) {
-    const long long base = (long long)t * H + h;
-    sa[i] = __bfloat162float(v[base * DV + i]);
-    sb[i] = __bfloat162float(dout[base * DV + i]);
-    __syncthreads();
-    const float qi = __bfloat162float(q[base * DK + i]) * scale;
-    float acc = 0.f;
-#pragma unroll
-    for (int c = 0; c < DV; ++c) {
-      M[c] = fmaf(M[c], a, qi * sb[c]);
-      acc = fmaf(M[c], sa[c], acc);
-    }
-    dk[base * DK + i] = __float2bfloat16(acc);
-    __syncthreads();
-  }
-  // ---- reverse sweep: dv (column i of R)
-#pragma unroll
-  for (int c = 0; c < DK; ++c) M[c] = 0.f;
-  for (int t = t1 - 1; t >= t0; --t) {
-    const long long base = (long long)t * H + h;
-    sa[i] = __bfloat162float(q[base * DK + i]) * scale;
-    sb[i] = __bfloat162float(k[base * DK + i]);
-    __syncthreads();
-    const float gi = __bfloat162float(dout[base * DV + i]);
-    float acc = 0.f;
-#pragma unroll
-    for (int r = 0; r < DK; ++r) {
-      M[r] = fmaf(M[r], a, sa[r] * gi);
-      acc = fmaf(M[r], sb[r], acc);
-    }
-    dv[base * DV + i] = __float2bfloat16(acc);
-    __syncthreads();
-  }
-}
-
 }  // namespace
 
 extern "C" {
@@ -441,44 +327,6 @@ int mcb_gated_rmsnorm_bwd(const void* x, const void* z, const void* w, const voi
   else if (D == 256) MCB_GN_BWD(256);
   else return -3;
 #undef MCB_GN_BWD
-  return (int)cudaGetLastError();
-}
-
-// q, k [T, H, DK]; v, o [T, H, DV]; decay [H] fp32 (log-decay per step, <= 0); cu_seqlens [n_seq + 1] int32
-int mcb_simple_gla_fwd(const void* q, const void* k, const void* v, const float* decay, const int* cu_seqlens, void* o,
-                       int n_seq, int H, int DK, int DV, float scale, void* stream_) {
-  if (n_seq == 0) return 0;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  dim3 grid(n_seq, H);
-  if (DK == 128 && DV == 128)
-    simple_gla_fwd_kernel<128, 128><<<grid, 128, 0, s>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
-                                                         (const __nv_bfloat16*)v, decay, cu_seqlens, (__nv_bfloat16*)o,
-                                                         H, scale);
-  else if (DK == 64 && DV == 64)
-    simple_gla_fwd_kernel<64, 64><<<grid, 64, 0, s>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
-                                                      (const __nv_bfloat16*)v, decay, cu_seqlens, (__nv_bfloat16*)o, H,
-                                                      scale);
-  else
-    return -3;
-  return (int)cudaGetLastError();
-}
-
-int mcb_simple_gla_bwd(const void* q, const void* k, const void* v, const void* dout, const float* decay,
-                       const int* cu_seqlens, void* dq, void* dk, void* dv, int n_seq, int H, int DK, int DV,
-                       float scale, void* stream_) {
-  if (n_seq == 0) return 0;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  dim3 grid(n_seq, H);
-  if (DK == 128 && DV == 128)
-    simple_gla_bwd_kernel<128, 128><<<grid, 128, 0, s>>>(
-        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (const __nv_bfloat16*)dout, decay,
-        cu_seqlens, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, H, scale);
-  else if (DK == 64 && DV == 64)
-    simple_gla_bwd_kernel<64, 64><<<grid, 64, 0, s>>>(
-        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (const __nv_bfloat16*)dout, decay,
-        cu_seqlens, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, H, scale);
-  else
-    return -3;
   return (int)cudaGetLastError();
 }
 

@@ -1,0 +1,141 @@
+// Warp-level bf16 tensor-core products on swizzled shared-memory tiles, for the chunked linear-attention kernels.
+//
+// Those kernels multiply fp32 quantities (states, decayed weights) with bf16 inputs.  An fp32 operand is fed to the
+// tensor core as two bf16 terms (value rounded to bf16 + the rounding error), i.e. with 16 mantissa bits, accumulated in
+// fp32; the terms are formed in registers, which is why these products use warp-level MMAs: their operands come straight
+// from the accumulators of the product before, and each is far too small to fill the tcgen05 pipe.
+//
+// A tile is [rows][D] bf16 with 16-byte chunks swizzled by the row: chunk c of row r is stored at chunk c ^ (r & 7), in
+// tiles of 32 columns (4 chunks) at c ^ ((r / 2) & 3); eight consecutive rows of one column then lie in distinct banks.
+#pragma once
+#include "../common/ptx.cuh"
+
+namespace mcb {
+
+template <int D>
+__device__ __forceinline__ uint32_t tile_addr(uint32_t base, int row, int col) {   // col: multiple of 8
+  if constexpr (D == 32) return base + row * 64 + (((col >> 3) ^ ((row >> 1) & 3)) << 4);
+  return base + row * (D * 2) + (((col >> 3) ^ (row & 7)) << 4);
+}
+
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// four 8 x 8 blocks of packed accumulators, each stored transposed: the lane addresses name rows of the stored blocks
+__device__ __forceinline__ void stsm4_t(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c),
+               "r"(d) : "memory");
+}
+// acc (16 x 8 fp32) += a (16 x 16 bf16, row) * b (16 x 8 bf16, col)
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// A operand: rows r0 .. r0+15, contraction columns k0 .. k0+15 of a row-major tile
+template <int D>
+__device__ __forceinline__ void load_a(uint32_t tile, int r0, int k0, int lane, uint32_t (&a)[4]) {
+  ldsm4(tile_addr<D>(tile, r0 + (lane & 15), k0 + ((lane >> 4) << 3)), a);
+}
+// A operand taken transposed: rows = tile columns m0 .. m0+15, contraction = tile rows k0 .. k0+15
+template <int D>
+__device__ __forceinline__ void load_a_t(uint32_t tile, int m0, int k0, int lane, uint32_t (&a)[4]) {
+  ldsm4_t(tile_addr<D>(tile, k0 + ((lane >> 4) << 3) + (lane & 7), m0 + (((lane >> 3) & 1) << 3)), a);
+}
+// B operand of X Y^T: two 8-wide column blocks n0, n0+8 = tile rows, contraction = tile columns k0 .. k0+15;
+// b[0], b[1] belong to n0, b[2], b[3] to n0 + 8
+template <int D>
+__device__ __forceinline__ void load_b_nt(uint32_t tile, int n0, int k0, int lane, uint32_t (&b)[4]) {
+  ldsm4(tile_addr<D>(tile, n0 + ((lane >> 4) << 3) + (lane & 7), k0 + (((lane >> 3) & 1) << 3)), b);
+}
+// B operand of X Y: contraction = tile rows k0 .. k0+15, two column blocks n0, n0+8 = tile columns
+template <int D>
+__device__ __forceinline__ void load_b_nn(uint32_t tile, int k0, int n0, int lane, uint32_t (&b)[4]) {
+  ldsm4_t(tile_addr<D>(tile, k0 + (((lane >> 3) & 1) << 3) + (lane & 7), n0 + ((lane >> 4) << 3)), b);
+}
+
+// two fp32 values -> packed bf16 pair and the packed pair of rounding errors
+__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const float2 f = __bfloat1622float2(h);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = pack_bf16x2(x - f.x, y - f.y);
+}
+// accumulators of two neighbouring 16 x 8 blocks -> the A operand of the next product, as two terms
+__device__ __forceinline__ void acc_to_a(const float (&c0)[4], const float (&c1)[4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+  split2(c0[0], c0[1], hi[0], lo[0]);
+  split2(c0[2], c0[3], hi[1], lo[1]);
+  split2(c1[0], c1[1], hi[2], lo[2]);
+  split2(c1[2], c1[3], hi[3], lo[3]);
+}
+
+// 16-byte asynchronous copy; `bytes` 0 writes zeros instead of reading
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// ROWS x D tile from rows `src + r * stride`; rows at or past `valid` become zero
+template <int D, int ROWS, int THREADS>
+__device__ __forceinline__ void load_tile(uint32_t tile, const __nv_bfloat16* src, long long stride, int valid) {
+  constexpr int CH = D / 8;
+  for (int id = threadIdx.x; id < ROWS * CH; id += THREADS) {
+    const int r = id / CH, c = (id % CH) * 8;
+    const bool in = r < valid;
+    cp_async16(tile_addr<D>(tile, r, c), in ? src + r * stride + c : src, in ? 16 : 0);
+  }
+}
+
+// One entry of the chunk list of a packed batch: sequence `s` contributes ceil(len / C) chunks and, between them,
+// ceil(len / C) - 1 boundaries.  Called by one warp; finds the sequence that holds item `id` of the list of chunks
+// (BOUNDARY = false) or of boundaries (true).  `seq` is -1 past the end.
+struct ChunkPos {
+  int seq, index, t0, t1, boundary0;   // index inside the sequence; token bounds of the sequence; its first boundary
+};
+template <int C, bool BOUNDARY>
+__device__ __forceinline__ ChunkPos find_chunk(const int* __restrict__ cu, int n_seq, int id, int lane) {
+  ChunkPos p{-1, 0, 0, 0, 0};
+  int done = 0, bdone = 0;
+  for (int s0 = 0; s0 < n_seq; s0 += 32) {
+    const int s = s0 + lane;
+    const int a = s < n_seq ? cu[s] : 0, b = s < n_seq ? cu[s + 1] : 0;
+    const int nc = b > a ? (b - a + C - 1) / C : 0, nb = nc > 0 ? nc - 1 : 0;
+    const int mine = BOUNDARY ? nb : nc;
+    int incl = mine, bincl = nb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl, o), y = __shfl_up_sync(0xffffffffu, bincl, o);
+      if (lane >= o) {
+        incl += x;
+        bincl += y;
+      }
+    }
+    const bool here = id >= done + incl - mine && id < done + incl;
+    const unsigned m = __ballot_sync(0xffffffffu, here);
+    if (m) {
+      const int w = __ffs(m) - 1;
+      p.seq = s0 + w;
+      p.index = id - (done + __shfl_sync(0xffffffffu, incl - mine, w));
+      p.t0 = __shfl_sync(0xffffffffu, a, w);
+      p.t1 = __shfl_sync(0xffffffffu, b, w);
+      p.boundary0 = bdone + __shfl_sync(0xffffffffu, bincl - nb, w);
+      return p;
+    }
+    done += __shfl_sync(0xffffffffu, incl, 31);
+    bdone += __shfl_sync(0xffffffffu, bincl, 31);
+  }
+  return p;
+}
+
+}  // namespace mcb

@@ -317,9 +317,11 @@ class _SimpleGlaFn(torch.autograd.Function):
         decay = decay.float().contiguous()
         o = torch.empty_like(v)
         n_seq = cu_seqlens.numel() - 1
-        rc = _lib.lib().mcb_simple_gla_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(decay), _lib.ptr(cu_seqlens),
-                                           _lib.ptr(o), ctypes.c_int(n_seq), ctypes.c_int(h), ctypes.c_int(dk),
-                                           ctypes.c_int(dv), ctypes.c_float(scale), _lib.stream_ptr())
+        lib = _lib.lib()
+        states = torch.empty((lib.mcb_simple_gla_boundaries(T), h, dk, dv), dtype=torch.float32, device=q.device)
+        rc = lib.mcb_simple_gla_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(decay), _lib.ptr(cu_seqlens),
+                                    _lib.ptr(o), _lib.ptr(states), ctypes.c_int(T), ctypes.c_int(n_seq),
+                                    ctypes.c_int(h), ctypes.c_int(dk), ctypes.c_float(scale), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_simple_gla_fwd')
         ctx.save_for_backward(q, k, v, decay, cu_seqlens)
         ctx.scale = scale
@@ -332,19 +334,21 @@ class _SimpleGlaFn(torch.autograd.Function):
         from . import _lib
         q, k, v, decay, cu = ctx.saved_tensors
         T, h, dk = q.shape
-        dv_ = v.shape[-1]
         do = do.contiguous()
         dq, dk_, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        rc = _lib.lib().mcb_simple_gla_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(do), _lib.ptr(decay),
-                                           _lib.ptr(cu), _lib.ptr(dq), _lib.ptr(dk_), _lib.ptr(dv),
-                                           ctypes.c_int(cu.numel() - 1), ctypes.c_int(h), ctypes.c_int(dk),
-                                           ctypes.c_int(dv_), ctypes.c_float(ctx.scale), _lib.stream_ptr())
+        lib = _lib.lib()
+        # the forward's states are formed again: keeping them would add half of the layer's q / k / v / o
+        states = torch.empty((2, lib.mcb_simple_gla_boundaries(T), h, dk, dk), dtype=torch.float32, device=q.device)
+        rc = lib.mcb_simple_gla_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(do), _lib.ptr(decay), _lib.ptr(cu),
+                                    _lib.ptr(dq), _lib.ptr(dk_), _lib.ptr(dv), _lib.ptr(states), ctypes.c_int(T),
+                                    ctypes.c_int(cu.numel() - 1), ctypes.c_int(h), ctypes.c_int(dk),
+                                    ctypes.c_float(ctx.scale), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_simple_gla_bwd')
         return dq, dk_, dv, None, None, None
 
 
 def simple_gla(q, k, v, decay, cu_seqlens=None, scale: Optional[float] = None) -> torch.Tensor:
-    """Dispatches to the recurrent CUDA kernels (bf16, square 64 / 128 state) or the torch restatement."""
+    """Dispatches to the chunked CUDA kernels (bf16, square 64 / 128 state) or the torch restatement."""
     T, h, dk = q.shape
     scale = dk**-0.5 if scale is None else scale
     if _cuda_ok(q, k, v) and dk == v.shape[-1] and dk in (64, 128):
