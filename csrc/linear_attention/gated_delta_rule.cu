@@ -1,0 +1,988 @@
+// Gated delta rule in chunks of 64 tokens over packed sequences, forward and backward (d = 64 or 128, dk = dv).
+//
+//   S <- exp(g_t) S;   S <- S + beta_t k_t (v_t - S^T k_t)^T;   o_t = scale * S^T q_t
+//
+// With G the running sum of g inside a chunk, D_ij = exp(G_i - G_j), A_ij = beta_i (k_i . k_j) D_ij below the diagonal,
+// M = (I + A)^-1 (the WY form), P = scale (q k^T) D on and below the diagonal, and S the state the chunk starts from:
+//
+//   R = v - exp(G) (k S)      V = M (beta R)      o = scale exp(G) (q S) + P V      S' = exp(G_last) S + (exp(G_last - G) k)^T V
+//
+// and backward, dS' given, dV = P^T do + exp(G_last - G) (k dS'),  Y = M^T dV:
+//
+//   dv = beta Y     dS = exp(G_last) dS' + (scale exp(G) q)^T do - (exp(G) k)^T (beta Y)     dA = -(Y V^T)     dP = do V^T
+//
+// with dq, dk, dg, dbeta following from these products (gdr_grad_kernel).  Launches: `prep` forms M and P of every chunk
+// independently; `scan` walks the chunks of a (sequence, head, 64 columns of v) in order; backward, `scan` runs again and
+// keeps S and V, `scan_bwd` walks in reverse and keeps dS' and Y, `grad` finishes every chunk independently.
+//
+// Precision: the state, M, P, V and every accumulation are fp32.  Operands of a product that are not bf16 inputs enter the
+// tensor core as two bf16 terms (16 mantissa bits, warp_mma.cuh); a product of two such operands takes three MMAs.
+//
+// In the scans a warp owns 16 columns of v and keeps S^T (16 x d) in its accumulators: the accumulators of every product
+// are the first operand of the next one, so the warps of a CTA share the loaded tiles and never exchange values.  Bound:
+// the chain of ~500 MMAs per chunk; the next chunk's tiles are copied meanwhile.  Measured, 4096 tokens in three sequences,
+// 32 heads of 128: forward 0.27 ms (prep 0.07, scan 0.19), backward 0.92 ms (prep, scan, scan_bwd 0.26, grad 0.39); the
+// batched torch evaluation of the rule was most of a 29.5 ms block.
+#include "../common/host_utils.cuh"
+#include "warp_mma.cuh"
+
+using namespace mcb;
+
+namespace {
+
+constexpr int C = 64;           // tokens of a chunk
+constexpr int THREADS = 128;    // 4 warps, 16 rows (tokens, or columns of v) each
+constexpr int CC = C * C;       // elements of a chunk's square matrices
+constexpr int SQ = CC * 2;      // bytes of one of their bf16 terms
+constexpr float L2E = 1.4426950408889634f;
+
+struct GdrParams {
+  const __nv_bfloat16 *q, *k, *v, *dout;   // [T, H, D]
+  const float *g, *beta;                   // [T, H]
+  const int* cu;                           // [n_seq + 1]
+  __nv_bfloat16 *o, *dq, *dk, *dv;
+  float *dg, *dbeta;                       // [T, H]
+  // per chunk and head, chunks numbered through the packed batch:
+  __nv_bfloat16* mp;                       // [4, 64, 64]: M and P, two terms each
+  float* gb;                               // [2, 64]: G * log2(e) and beta (0 past the end of the sequence)
+  __nv_bfloat16 *S, *dS;                   // [2, D, D]: S^T and dS'^T, two terms
+  __nv_bfloat16 *V, *Y;                    // [2, D, 64]: V^T and Y^T, two terms
+  int n_seq, H;
+  float scale;
+};
+
+__device__ __forceinline__ ChunkPos locate(const GdrParams& p, ChunkPos* slot) {
+  ChunkPos mine{-1, 0, 0, 0, 0};
+  if (threadIdx.x < 32) mine = find_chunk<C, false>(p.cu, p.n_seq, blockIdx.x, threadIdx.x);
+  if (threadIdx.x == 0) *slot = mine;
+  __syncthreads();
+  return *slot;
+}
+
+// 64 x 64 bf16 matrix (contiguous) -> tile
+__device__ __forceinline__ void load_square(uint32_t tile, const __nv_bfloat16* src) {
+  for (int id = threadIdx.x; id < C * 8; id += THREADS) cp_async16(tile_addr<64>(tile, id >> 3, (id & 7) * 8), src + id * 8, 16);
+}
+
+// ---------------------------------------------------------------------------------------------------- prep
+template <int D>
+constexpr int PREP_TILES = 2 * C * D * 2 > 2 * C * 72 * 2 ? 2 * C * D * 2 : 2 * C * 72 * 2;   // q and k, later M's two terms
+
+template <int D>
+__global__ void __launch_bounds__(THREADS)
+gdr_prep_kernel(const GdrParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ ChunkPos slot;
+  __shared__ float s_g[C], s_b[C];
+  constexpr int LDA = C + 4;
+  const uint32_t sq = (smem_u32(smem_raw) + 127) & ~127u, sk = sq + C * D * 2;
+  float* sA = reinterpret_cast<float*>(smem_raw + (sq + PREP_TILES<D> - smem_u32(smem_raw)));  // [64][LDA]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y;
+  const ChunkPos pos = locate(p, &slot);
+  if (pos.seq < 0) return;
+  const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
+  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
+  const long long ch = (long long)blockIdx.x * p.H + h;
+  load_tile<D, C, THREADS>(sq, p.q + off, stride, len);
+  load_tile<D, C, THREADS>(sk, p.k + off, stride, len);
+  cp_async_commit();
+  if (warp == 0) {                              // running sum of g: two tokens a lane
+    const long long a = (long long)(t + 2 * lane) * p.H + h;
+    const bool in0 = 2 * lane < len, in1 = 2 * lane + 1 < len;
+    const float g0 = in0 ? p.g[a] * L2E : 0.f, g1 = in1 ? p.g[a + p.H] * L2E : 0.f;
+    float run = g0 + g1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float x = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += x;
+    }
+    const float before = run - (g0 + g1);
+    const float2 gg = make_float2(before + g0, run), bb = make_float2(in0 ? p.beta[a] : 0.f, in1 ? p.beta[a + p.H] : 0.f);
+    reinterpret_cast<float2*>(s_g)[lane] = gg;
+    reinterpret_cast<float2*>(s_b)[lane] = bb;
+    reinterpret_cast<float2*>(p.gb + ch * 2 * C)[lane] = gg;
+    reinterpret_cast<float2*>(p.gb + ch * 2 * C + C)[lane] = bb;
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  const int r0 = warp * 16, i = r0 + (lane >> 2);
+  __nv_bfloat16* mp = p.mp + ch * 4 * CC;
+  const float gi[2] = {s_g[i], s_g[i + 8]}, bi[2] = {s_b[i], s_b[i + 8]};
+  for (int jb = 0; jb < 4; ++jb) {
+    float kk2[2][4] = {}, qk2[2][4] = {};
+    if (jb <= warp) {
+#pragma unroll
+      for (int kk = 0; kk < D; kk += 16) {
+        uint32_t a[4], c[4], b[4];
+        load_a<D>(sk, r0, kk, lane, a);
+        load_a<D>(sq, r0, kk, lane, c);
+        load_b_nt<D>(sk, jb * 16, kk, lane, b);
+        mma16816(kk2[0], a, b[0], b[1]);
+        mma16816(kk2[1], a, b[2], b[3]);
+        mma16816(qk2[0], c, b[0], b[1]);
+        mma16816(qk2[1], c, b[2], b[3]);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const int j = jb * 16 + n * 8 + (lane & 3) * 2;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float pv[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int ii = i + 8 * r, jj = j + u;
+          const float d = jj <= ii ? exp2f(gi[r] - s_g[jj]) : 0.f;
+          sA[ii * LDA + jj] = jj < ii ? bi[r] * kk2[n][2 * r + u] * d : 0.f;
+          pv[u] = jj <= ii ? p.scale * qk2[n][2 * r + u] * d : 0.f;
+        }
+        uint32_t hi, lo;
+        split2(pv[0], pv[1], hi, lo);
+        *reinterpret_cast<uint32_t*>(mp + 2 * CC + (i + 8 * r) * C + j) = hi;
+        *reinterpret_cast<uint32_t*>(mp + 3 * CC + (i + 8 * r) * C + j) = lo;
+      }
+    }
+  }
+  __syncthreads();
+  // M = (I + A)^-1, one column a thread by forward substitution (A rows are shared-memory broadcasts); the columns meet as
+  // bf16 terms in the q / k tiles, which nothing reads any more
+  __nv_bfloat16* sm = reinterpret_cast<__nv_bfloat16*>(smem_raw + (sq - smem_u32(smem_raw)));  // [2][64][72]
+  if (threadIdx.x < C) {
+    const int j = threadIdx.x;
+    float x[C];
+#pragma unroll
+    for (int r = 0; r < C; ++r) {
+      float s0 = r == j ? 1.f : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+      for (int c = 0; c < r; c += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(sA + r * LDA + c);
+        s0 = fmaf(-a.x, x[c], s0);
+        if (c + 1 < r) s1 = fmaf(-a.y, x[c + 1], s1);
+        if (c + 2 < r) s2 = fmaf(-a.z, x[c + 2], s2);
+        if (c + 3 < r) s3 = fmaf(-a.w, x[c + 3], s3);
+      }
+      x[r] = (s0 + s1) + (s2 + s3);
+      const __nv_bfloat16 hi = __float2bfloat16(x[r]);
+      sm[r * 72 + j] = hi;
+      sm[C * 72 + r * 72 + j] = __float2bfloat16(x[r] - __bfloat162float(hi));
+    }
+  }
+  __syncthreads();
+  for (int id = threadIdx.x; id < 2 * C * 8; id += THREADS) {
+    const int m = id >> 9, r = (id >> 3) & 63, c = (id & 7) * 8;
+    *reinterpret_cast<uint4*>(mp + m * CC + r * C + c) = *reinterpret_cast<const uint4*>(sm + m * C * 72 + r * 72 + c);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------- scans
+// shared-memory stage of a scan: k, q (or, backward, both needed too), a 64-column slice of v / do, M, P, G and beta
+template <int D>
+struct ScanSmem {
+  static constexpr int K = 0, Q = C * D * 2, X = 2 * C * D * 2, M = X + SQ, P = M + 2 * SQ, G = P + 2 * SQ;
+  static constexpr int STAGE = G + 2 * C * 4;
+  static constexpr int TOTAL = 2 * STAGE + 128;
+};
+
+template <int D, bool WITH_Q>
+__device__ __forceinline__ void load_stage(uint32_t st, const GdrParams& p, const __nv_bfloat16* x, int t, int len, int h, int col0,
+                                           long long ch) {
+  using L = ScanSmem<D>;
+  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
+  load_tile<D, C, THREADS>(st + L::K, p.k + off, stride, len);
+  if (WITH_Q) load_tile<D, C, THREADS>(st + L::Q, p.q + off, stride, len);
+  load_tile<64, C, THREADS>(st + L::X, x + off + col0, stride, len);
+  load_square(st + L::M, p.mp + ch * 4 * CC);
+  load_square(st + L::M + SQ, p.mp + ch * 4 * CC + CC);
+  if (WITH_Q) {
+    load_square(st + L::P, p.mp + ch * 4 * CC + 2 * CC);
+    load_square(st + L::P + SQ, p.mp + ch * 4 * CC + 3 * CC);
+  }
+  if (threadIdx.x < 32) cp_async16(st + L::G + threadIdx.x * 16, p.gb + ch * 2 * C + threadIdx.x * 4, 16);
+  cp_async_commit();
+}
+
+struct ScanPos {
+  int t0, len, chunk0, n, h, col0;   // the sequence; its first chunk and their number; head; first column of v
+};
+template <int D>
+__device__ __forceinline__ ScanPos scan_pos(const GdrParams& p, int* slot) {
+  constexpr int SL = D / 64;
+  ScanPos s;
+  const int seq = blockIdx.x / (p.H * SL), rest = blockIdx.x % (p.H * SL);
+  s.h = rest / SL;
+  s.col0 = (rest % SL) * 64;
+  s.t0 = p.cu[seq];
+  s.len = p.cu[seq + 1] - s.t0;
+  s.n = s.len > 0 ? (s.len + C - 1) / C : 0;
+  if (threadIdx.x < 32) {
+    int n = 0;
+    for (int i = threadIdx.x; i < seq; i += 32) {
+      const int l = p.cu[i + 1] - p.cu[i];
+      if (l > 0) n += (l + C - 1) / C;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if (threadIdx.x == 0) *slot = n;
+  }
+  __syncthreads();
+  s.chunk0 = *slot;
+  return s;
+}
+
+__device__ __forceinline__ float2 lds2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float lds1(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+// accumulators (16 rows x 8 N columns) -> two bf16 planes with `ld` columns
+template <int N>
+__device__ __forceinline__ void store_terms(const float (&a)[N][4], __nv_bfloat16* dst, long long plane, int ld, int row, int lane) {
+  const int col = (lane & 3) * 2;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      uint32_t hi, lo;
+      split2(a[n][2 * r], a[n][2 * r + 1], hi, lo);
+      __nv_bfloat16* at = dst + (long long)(row + 8 * r) * ld + n * 8 + col;
+      *reinterpret_cast<uint32_t*>(at) = hi;
+      *reinterpret_cast<uint32_t*>(at + plane) = lo;
+    }
+  }
+}
+
+// x [8][4] holds (16 columns of v) x (64 tokens): written as bf16 rows of tokens through the warp's columns of `tile`
+__device__ __forceinline__ void store_transposed(const float (&x)[8][4], uint32_t tile, __nv_bfloat16* dst, long long stride, int len,
+                                                 int warp, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int n = 0; n < 8; n += 2) {
+    const int tok = n * 8 + ((lane >> 4) << 3) + (lane & 7), col = warp * 16 + (((lane >> 3) & 1) << 3);
+    stsm4_t(tile_addr<64>(tile, tok, col), pack_bf16x2(x[n][0], x[n][1]), pack_bf16x2(x[n][2], x[n][3]),
+            pack_bf16x2(x[n + 1][0], x[n + 1][1]), pack_bf16x2(x[n + 1][2], x[n + 1][3]));
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int tok = u * 16 + (lane >> 1), col = warp * 16 + (lane & 1) * 8;
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(tile_addr<64>(tile, tok, col)) : "memory");
+    if (tok < len) *reinterpret_cast<uint4*>(dst + (long long)tok * stride + col) = v;
+  }
+}
+
+// SAVE: keep S and V of every chunk for the backward pass instead of forming the outputs
+template <int D, bool SAVE>
+__global__ void __launch_bounds__(THREADS)
+gdr_scan_kernel(const GdrParams p) {
+  using L = ScanSmem<D>;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ int slot;
+  const uint32_t base = (smem_u32(smem_raw) + 127) & ~127u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const ScanPos s = scan_pos<D>(p, &slot);
+  if (s.n == 0) return;
+  const long long stride = (long long)p.H * D;
+  float St[D / 8][4];
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n) St[n][0] = St[n][1] = St[n][2] = St[n][3] = 0.f;
+  load_stage<D, !SAVE>(base, p, p.v, s.t0, min(C, s.len), s.h, s.col0, (long long)s.chunk0 * p.H + s.h);
+  for (int c = 0; c < s.n; ++c) {
+    const uint32_t st = base + (c & 1) * L::STAGE;
+    const int t = s.t0 + c * C, len = min(C, s.len - c * C);
+    const long long ch = (long long)(s.chunk0 + c) * p.H + s.h;
+    if (c + 1 < s.n) {
+      load_stage<D, !SAVE>(base + ((c + 1) & 1) * L::STAGE, p, p.v, t + C, min(C, s.len - (c + 1) * C), s.h, s.col0, ch + p.H);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    if (SAVE) store_terms<D / 8>(St, p.S + ch * 2 * D * D, (long long)D * D, D, s.col0 + warp * 16 + (lane >> 2), lane);
+    float X[8][4] = {}, O[8][4] = {};
+    if (c > 0) {                                // the state is zero before the first chunk
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        uint32_t hi[4], lo[4];
+        acc_to_a(St[2 * kk], St[2 * kk + 1], hi, lo);
+#pragma unroll
+        for (int n = 0; n < 8; n += 2) {
+          uint32_t b[4];
+          load_b_nt<D>(st + L::K, n * 8, kk * 16, lane, b);
+          mma16816(X[n], hi, b[0], b[1]);
+          mma16816(X[n + 1], hi, b[2], b[3]);
+          mma16816(X[n], lo, b[0], b[1]);
+          mma16816(X[n + 1], lo, b[2], b[3]);
+          if (!SAVE) {
+            load_b_nt<D>(st + L::Q, n * 8, kk * 16, lane, b);
+            mma16816(O[n], hi, b[0], b[1]);
+            mma16816(O[n + 1], hi, b[2], b[3]);
+            mma16816(O[n], lo, b[0], b[1]);
+            mma16816(O[n + 1], lo, b[2], b[3]);
+          }
+        }
+      }
+    }
+    // beta (v - exp(G) k S), columns = tokens
+    const uint32_t sg = st + L::G + (lane & 3) * 8, sb = sg + C * 4;
+    const float glast = lds1(st + L::G + (C - 1) * 4);
+#pragma unroll
+    for (int n = 0; n < 8; n += 2) {
+      uint32_t a[4];
+      load_a_t<64>(st + L::X, warp * 16, n * 8, lane, a);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float2 g = lds2(sg + (n + u) * 32), b = lds2(sb + (n + u) * 32);
+        const float e0 = exp2f(g.x), e1 = exp2f(g.y);
+        const float2 v0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u]));
+        const float2 v1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u + 1]));
+        float (&x)[4] = X[n + u];
+        x[0] = b.x * (v0.x - e0 * x[0]);
+        x[1] = b.y * (v0.y - e1 * x[1]);
+        x[2] = b.x * (v1.x - e0 * x[2]);
+        x[3] = b.y * (v1.y - e1 * x[3]);
+        if (!SAVE) {
+          O[n + u][0] *= p.scale * e0;
+          O[n + u][1] *= p.scale * e1;
+          O[n + u][2] *= p.scale * e0;
+          O[n + u][3] *= p.scale * e1;
+        }
+      }
+    }
+    float V[8][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      uint32_t hi[4], lo[4];
+      acc_to_a(X[2 * kk], X[2 * kk + 1], hi, lo);
+#pragma unroll
+      for (int n = 2 * kk; n < 8; n += 2) {     // M is lower triangular
+        uint32_t b[4], d[4];
+        load_b_nt<64>(st + L::M, n * 8, kk * 16, lane, b);
+        load_b_nt<64>(st + L::M + SQ, n * 8, kk * 16, lane, d);
+        mma16816(V[n], hi, b[0], b[1]);
+        mma16816(V[n + 1], hi, b[2], b[3]);
+        mma16816(V[n], lo, b[0], b[1]);
+        mma16816(V[n + 1], lo, b[2], b[3]);
+        mma16816(V[n], hi, d[0], d[1]);
+        mma16816(V[n + 1], hi, d[2], d[3]);
+      }
+    }
+    if (SAVE) {
+      store_terms<8>(V, p.V + ch * 2 * D * C, (long long)D * C, C, s.col0 + warp * 16 + (lane >> 2), lane);
+    } else {
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t hi[4], lo[4];
+        acc_to_a(V[2 * kk], V[2 * kk + 1], hi, lo);
+#pragma unroll
+        for (int n = 2 * kk; n < 8; n += 2) {   // P is lower triangular
+          uint32_t b[4], d[4];
+          load_b_nt<64>(st + L::P, n * 8, kk * 16, lane, b);
+          load_b_nt<64>(st + L::P + SQ, n * 8, kk * 16, lane, d);
+          mma16816(O[n], hi, b[0], b[1]);
+          mma16816(O[n + 1], hi, b[2], b[3]);
+          mma16816(O[n], lo, b[0], b[1]);
+          mma16816(O[n + 1], lo, b[2], b[3]);
+          mma16816(O[n], hi, d[0], d[1]);
+          mma16816(O[n + 1], hi, d[2], d[3]);
+        }
+      }
+      store_transposed(O, st + L::X, p.o + ((long long)t * p.H + s.h) * D + s.col0, stride, len, warp, lane);
+    }
+    if (c + 1 < s.n) {
+      const float el = exp2f(glast);
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n) {
+        St[n][0] *= el;
+        St[n][1] *= el;
+        St[n][2] *= el;
+        St[n][3] *= el;
+      }
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const float2 g = lds2(sg + n * 32);
+        const float w0 = exp2f(glast - g.x), w1 = exp2f(glast - g.y);
+        V[n][0] *= w0;
+        V[n][1] *= w1;
+        V[n][2] *= w0;
+        V[n][3] *= w1;
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t hi[4], lo[4];
+        acc_to_a(V[2 * kk], V[2 * kk + 1], hi, lo);
+#pragma unroll
+        for (int n = 0; n < D / 8; n += 2) {
+          uint32_t b[4];
+          load_b_nn<D>(st + L::K, kk * 16, n * 8, lane, b);
+          mma16816(St[n], hi, b[0], b[1]);
+          mma16816(St[n + 1], hi, b[2], b[3]);
+          mma16816(St[n], lo, b[0], b[1]);
+          mma16816(St[n + 1], lo, b[2], b[3]);
+        }
+      }
+    }
+    __syncthreads();                            // the stage is free for the copies of the chunk after the next
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(THREADS)
+gdr_scan_bwd_kernel(const GdrParams p) {
+  using L = ScanSmem<D>;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ int slot;
+  const uint32_t base = (smem_u32(smem_raw) + 127) & ~127u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const ScanPos s = scan_pos<D>(p, &slot);
+  if (s.n == 0) return;
+  const long long stride = (long long)p.H * D;
+  float dSt[D / 8][4];
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n) dSt[n][0] = dSt[n][1] = dSt[n][2] = dSt[n][3] = 0.f;
+  const int lastc = s.n - 1;
+  load_stage<D, true>(base, p, p.dout, s.t0 + lastc * C, s.len - lastc * C, s.h, s.col0, (long long)(s.chunk0 + lastc) * p.H + s.h);
+  for (int it = 0; it < s.n; ++it) {
+    const int c = lastc - it;
+    const uint32_t st = base + (it & 1) * L::STAGE;
+    const int t = s.t0 + c * C, len = min(C, s.len - c * C);
+    const long long ch = (long long)(s.chunk0 + c) * p.H + s.h;
+    if (c > 0) {
+      load_stage<D, true>(base + ((it + 1) & 1) * L::STAGE, p, p.dout, t - C, C, s.h, s.col0, ch - p.H);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    const int row = s.col0 + warp * 16 + (lane >> 2);
+    store_terms<D / 8>(dSt, p.dS + ch * 2 * D * D, (long long)D * D, D, row, lane);
+    const uint32_t sg = st + L::G + (lane & 3) * 8, sb = sg + C * 4;
+    const float glast = lds1(st + L::G + (C - 1) * 4);
+    float dV[8][4] = {};
+    if (it > 0) {                               // nothing flows into the sequence's last state
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        uint32_t hi[4], lo[4];
+        acc_to_a(dSt[2 * kk], dSt[2 * kk + 1], hi, lo);
+#pragma unroll
+        for (int n = 0; n < 8; n += 2) {
+          uint32_t b[4];
+          load_b_nt<D>(st + L::K, n * 8, kk * 16, lane, b);
+          mma16816(dV[n], hi, b[0], b[1]);
+          mma16816(dV[n + 1], hi, b[2], b[3]);
+          mma16816(dV[n], lo, b[0], b[1]);
+          mma16816(dV[n + 1], lo, b[2], b[3]);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const float2 g = lds2(sg + n * 32);
+        const float w0 = exp2f(glast - g.x), w1 = exp2f(glast - g.y);
+        dV[n][0] *= w0;
+        dV[n][1] *= w1;
+        dV[n][2] *= w0;
+        dV[n][3] *= w1;
+      }
+    }
+    uint32_t da[4][4];                          // do^T: rows = columns of v, contraction = tokens
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      load_a_t<64>(st + L::X, warp * 16, kk * 16, lane, da[kk]);
+#pragma unroll
+      for (int n = 0; n <= 2 * kk; n += 2) {    // rows i of P from column block j <= i
+        uint32_t b[4], d[4];
+        load_b_nn<64>(st + L::P, kk * 16, n * 8, lane, b);
+        load_b_nn<64>(st + L::P + SQ, kk * 16, n * 8, lane, d);
+        mma16816(dV[n], da[kk], b[0], b[1]);
+        mma16816(dV[n + 1], da[kk], b[2], b[3]);
+        mma16816(dV[n], da[kk], d[0], d[1]);
+        mma16816(dV[n + 1], da[kk], d[2], d[3]);
+      }
+    }
+    float Y[8][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      uint32_t hi[4], lo[4];
+      acc_to_a(dV[2 * kk], dV[2 * kk + 1], hi, lo);
+#pragma unroll
+      for (int n = 0; n <= 2 * kk; n += 2) {
+        uint32_t b[4], d[4];
+        load_b_nn<64>(st + L::M, kk * 16, n * 8, lane, b);
+        load_b_nn<64>(st + L::M + SQ, kk * 16, n * 8, lane, d);
+        mma16816(Y[n], hi, b[0], b[1]);
+        mma16816(Y[n + 1], hi, b[2], b[3]);
+        mma16816(Y[n], lo, b[0], b[1]);
+        mma16816(Y[n + 1], lo, b[2], b[3]);
+        mma16816(Y[n], hi, d[0], d[1]);
+        mma16816(Y[n + 1], hi, d[2], d[3]);
+      }
+    }
+    store_terms<8>(Y, p.Y + ch * 2 * D * C, (long long)D * C, C, row, lane);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      const float2 b = lds2(sb + n * 32);
+      Y[n][0] *= b.x;
+      Y[n][1] *= b.y;
+      Y[n][2] *= b.x;
+      Y[n][3] *= b.y;
+    }
+    store_transposed(Y, st + L::X, p.dv + ((long long)t * p.H + s.h) * D + s.col0, stride, len, warp, lane);
+    if (c > 0) {
+      const float el = exp2f(glast);
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n) {
+        dSt[n][0] *= el;
+        dSt[n][1] *= el;
+        dSt[n][2] *= el;
+        dSt[n][3] *= el;
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t hi[4], lo[4], yh[4], yl[4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {           // registers 2u, 2u + 1: tokens of the lower / upper half of the slice
+          const float2 g = lds2(sg + (2 * kk + u) * 32);
+          const float e0 = exp2f(g.x), e1 = exp2f(g.y);
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&da[kk][2 * u + r]));
+            split2(x.x * (p.scale * e0), x.y * (p.scale * e1), hi[2 * u + r], lo[2 * u + r]);
+            split2(-e0 * Y[2 * kk + u][2 * r], -e1 * Y[2 * kk + u][2 * r + 1], yh[2 * u + r], yl[2 * u + r]);
+          }
+        }
+#pragma unroll
+        for (int n = 0; n < D / 8; n += 2) {
+          uint32_t b[4], d[4];
+          load_b_nn<D>(st + L::Q, kk * 16, n * 8, lane, b);
+          load_b_nn<D>(st + L::K, kk * 16, n * 8, lane, d);
+          mma16816(dSt[n], hi, b[0], b[1]);
+          mma16816(dSt[n + 1], hi, b[2], b[3]);
+          mma16816(dSt[n], lo, b[0], b[1]);
+          mma16816(dSt[n + 1], lo, b[2], b[3]);
+          mma16816(dSt[n], yh, d[0], d[1]);
+          mma16816(dSt[n + 1], yh, d[2], d[3]);
+          mma16816(dSt[n], yl, d[0], d[1]);
+          mma16816(dSt[n + 1], yl, d[2], d[3]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------- grad
+// dq, dk, dg, dbeta of one chunk.  Rows = tokens, 16 a warp.  S^T and dS'^T stream through shared memory 32 columns at a
+// time (two stages); everything else the chunk needs is resident.
+template <int D>
+struct GradSmem {
+  static constexpr int TILE = C * D * 2;
+  static constexpr int Q = 0, K = TILE, V = 2 * TILE, DO = 3 * TILE;        // token tiles
+  static constexpr int VT = 4 * TILE, YT = 6 * TILE;                        // V^T, Y^T: two terms of [D][64] each
+  static constexpr int ST = 8 * TILE;                                       // 2 stages of S^T, dS'^T: two terms of [D][32]
+  static constexpr int STRIP = D * 32 * 2;
+  static constexpr int TOTAL = ST + 2 * 4 * STRIP + 128;
+};
+
+template <int D>
+__device__ __forceinline__ void load_strips(uint32_t st, const __nv_bfloat16* S, const __nv_bfloat16* dS, int col0) {
+  for (int id = threadIdx.x; id < 4 * D * 4; id += THREADS) {
+    const int m = id / (D * 4), r = (id / 4) % D, c = (id & 3) * 8;
+    const __nv_bfloat16* src = (m < 2 ? S : dS) + (m & 1) * D * D + r * D + col0 + c;
+    cp_async16(tile_addr<32>(st + m * GradSmem<D>::STRIP, r, c), src, 16);
+  }
+  cp_async_commit();
+}
+
+__device__ __forceinline__ float quad_sum(float x) {   // over the four lanes that share an accumulator row
+  x += __shfl_xor_sync(0xffffffffu, x, 1);
+  return x + __shfl_xor_sync(0xffffffffu, x, 2);
+}
+template <int D>
+__device__ __forceinline__ float2 tile_pair(uint32_t tile, int row, int col) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(tile_addr<D>(tile, row, col & ~7) + (col & 7) * 2) : "memory");
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
+}
+
+template <int D>
+__global__ void __launch_bounds__(THREADS)
+gdr_grad_kernel(const GdrParams p) {
+  using L = GradSmem<D>;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ ChunkPos slot;
+  __shared__ float s_g[C], s_b[C], s_dg[C], s_red[4];
+  const uint32_t base = (smem_u32(smem_raw) + 127) & ~127u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y;
+  const ChunkPos pos = locate(p, &slot);
+  if (pos.seq < 0) return;
+  const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
+  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
+  const long long ch = (long long)blockIdx.x * p.H + h;
+  load_tile<D, C, THREADS>(base + L::Q, p.q + off, stride, len);
+  load_tile<D, C, THREADS>(base + L::K, p.k + off, stride, len);
+  load_tile<D, C, THREADS>(base + L::V, p.v + off, stride, len);
+  load_tile<D, C, THREADS>(base + L::DO, p.dout + off, stride, len);
+  for (int id = threadIdx.x; id < 4 * D * 8; id += THREADS) {
+    const int m = id / (D * 8), r = (id / 8) % D, c = (id & 7) * 8;
+    const __nv_bfloat16* src = (m < 2 ? p.V : p.Y) + ch * 2 * D * C + (m & 1) * D * C + r * C + c;
+    cp_async16(tile_addr<64>(base + L::VT + m * L::TILE, r, c), src, 16);
+  }
+  cp_async_commit();
+  const __nv_bfloat16 *S = p.S + ch * 2 * D * D, *dS = p.dS + ch * 2 * D * D;
+  load_strips<D>(base + L::ST, S, dS, 0);
+  if (threadIdx.x < C) {
+    s_g[threadIdx.x] = p.gb[ch * 2 * C + threadIdx.x];
+    s_b[threadIdx.x] = p.gb[ch * 2 * C + C + threadIdx.x];
+  }
+  const int r0 = warp * 16, i = r0 + (lane >> 2), c2 = (lane & 3) * 2;
+  float dq[D / 8][4], dk[D / 8][4];
+  float qf[2] = {0.f, 0.f}, kh[2] = {0.f, 0.f}, ke[2] = {0.f, 0.f}, sdot = 0.f;
+  float eg[2], el[2], bi[2], gi[2];
+#pragma unroll
+  for (int w = 0; w < D / 32; ++w) {
+    if (w + 1 < D / 32) {
+      load_strips<D>(base + L::ST + ((w + 1) & 1) * 4 * L::STRIP, S, dS, (w + 1) * 32);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    if (w == 0) {
+      const float gl = s_g[C - 1];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        gi[r] = s_g[i + 8 * r];
+        bi[r] = s_b[i + 8 * r];
+        eg[r] = exp2f(gi[r]);
+        el[r] = exp2f(gl - gi[r]);
+      }
+    }
+    const uint32_t st = base + L::ST + (w & 1) * 4 * L::STRIP;
+    float F[4][4] = {}, E[4][4] = {}, Hh[4][4] = {};
+#pragma unroll 1
+    for (int kk = 0; kk < D; kk += 16) {        // contraction over the columns of v
+      uint32_t a[4], yh[4], yl[4], vh[4], vl[4];
+      load_a<D>(base + L::DO, r0, kk, lane, a);
+      load_a_t<64>(base + L::YT, r0, kk, lane, yh);
+      load_a_t<64>(base + L::YT + L::TILE, r0, kk, lane, yl);
+      load_a_t<64>(base + L::VT, r0, kk, lane, vh);
+      load_a_t<64>(base + L::VT + L::TILE, r0, kk, lane, vl);
+#pragma unroll
+      for (int n = 0; n < 4; n += 2) {
+        uint32_t b[4], d[4];
+        load_b_nn<32>(st, kk, n * 8, lane, b);
+        load_b_nn<32>(st + L::STRIP, kk, n * 8, lane, d);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          mma16816(F[n + u], a, b[2 * u], b[2 * u + 1]);
+          mma16816(E[n + u], yh, b[2 * u], b[2 * u + 1]);
+          mma16816(F[n + u], a, d[2 * u], d[2 * u + 1]);
+          mma16816(E[n + u], yl, b[2 * u], b[2 * u + 1]);
+          mma16816(E[n + u], yh, d[2 * u], d[2 * u + 1]);
+        }
+        load_b_nn<32>(st + 2 * L::STRIP, kk, n * 8, lane, b);
+        load_b_nn<32>(st + 3 * L::STRIP, kk, n * 8, lane, d);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          mma16816(Hh[n + u], vh, b[2 * u], b[2 * u + 1]);
+          mma16816(Hh[n + u], vl, b[2 * u], b[2 * u + 1]);
+          mma16816(Hh[n + u], vh, d[2 * u], d[2 * u + 1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int col = w * 32 + n * 8 + c2;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float2 qq = tile_pair<D>(base + L::Q, i + 8 * r, col), kq = tile_pair<D>(base + L::K, i + 8 * r, col);
+        const float f0 = p.scale * eg[r] * F[n][2 * r], f1 = p.scale * eg[r] * F[n][2 * r + 1];
+        const float h0 = el[r] * Hh[n][2 * r], h1 = el[r] * Hh[n][2 * r + 1];
+        const float e0 = eg[r] * E[n][2 * r], e1 = eg[r] * E[n][2 * r + 1];
+        qf[r] += qq.x * f0 + qq.y * f1;
+        kh[r] += kq.x * h0 + kq.y * h1;
+        ke[r] += kq.x * e0 + kq.y * e1;
+        dq[w * 4 + n][2 * r] = f0;
+        dq[w * 4 + n][2 * r + 1] = f1;
+        dk[w * 4 + n][2 * r] = h0 - bi[r] * e0;
+        dk[w * 4 + n][2 * r + 1] = h1 - bi[r] * e1;
+      }
+    }
+    for (int id = threadIdx.x; id < D * 16; id += THREADS) {       // <S, dS'>
+      const int r = id >> 4, c = (id & 15) * 2;
+      const float2 a = tile_pair<32>(st, r, c), b = tile_pair<32>(st + L::STRIP, r, c);
+      const float2 d = tile_pair<32>(st + 2 * L::STRIP, r, c), e = tile_pair<32>(st + 3 * L::STRIP, r, c);
+      sdot += (a.x + b.x) * (d.x + e.x) + (a.y + b.y) * (d.y + e.y);
+    }
+    __syncthreads();
+  }
+  float yv[2] = {0.f, 0.f};                      // Y_i . v_i: the diagonal of a 16 x 16 product
+  {
+    float s[2][4] = {};
+#pragma unroll 1
+    for (int kk = 0; kk < D; kk += 16) {
+      uint32_t yh[4], yl[4], b[4];
+      load_a_t<64>(base + L::YT, r0, kk, lane, yh);
+      load_a_t<64>(base + L::YT + L::TILE, r0, kk, lane, yl);
+      load_b_nt<D>(base + L::V, r0, kk, lane, b);
+      mma16816(s[0], yh, b[0], b[1]);
+      mma16816(s[1], yh, b[2], b[3]);
+      mma16816(s[0], yl, b[0], b[1]);
+      mma16816(s[1], yl, b[2], b[3]);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (c2 + u == (lane >> 2)) {
+        yv[0] = s[0][u];
+        yv[1] = s[1][2 + u];
+      }
+    }
+  }
+  float dgc[2], db[2], xs = 0.f;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    dgc[r] = qf[r] - kh[r] - bi[r] * ke[r];
+    db[r] = yv[r] - ke[r];
+    xs += kh[r];
+  }
+  // rows i, columns j <= i
+#pragma unroll 1
+  for (int jb = 0; jb <= warp; ++jb) {
+    float dP[2][4] = {}, dA[2][4] = {}, qk[2][4] = {}, kk2[2][4] = {};
+#pragma unroll 1
+    for (int kk = 0; kk < D; kk += 16) {
+      uint32_t a[4], yh[4], yl[4], b[4], d[4];
+      load_a<D>(base + L::DO, r0, kk, lane, a);
+      load_a_t<64>(base + L::YT, r0, kk, lane, yh);
+      load_a_t<64>(base + L::YT + L::TILE, r0, kk, lane, yl);
+      load_b_nn<64>(base + L::VT, kk, jb * 16, lane, b);
+      load_b_nn<64>(base + L::VT + L::TILE, kk, jb * 16, lane, d);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(dP[u], a, b[2 * u], b[2 * u + 1]);
+        mma16816(dA[u], yh, b[2 * u], b[2 * u + 1]);
+        mma16816(dP[u], a, d[2 * u], d[2 * u + 1]);
+        mma16816(dA[u], yl, b[2 * u], b[2 * u + 1]);
+        mma16816(dA[u], yh, d[2 * u], d[2 * u + 1]);
+      }
+      load_a<D>(base + L::Q, r0, kk, lane, a);
+      load_a<D>(base + L::K, r0, kk, lane, yh);
+      load_b_nt<D>(base + L::K, jb * 16, kk, lane, b);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(qk[u], a, b[2 * u], b[2 * u + 1]);
+        mma16816(kk2[u], yh, b[2 * u], b[2 * u + 1]);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = e >> 1, ii = i + 8 * r, jj = jb * 16 + n * 8 + c2 + (e & 1);
+        const float D_ = jj <= ii ? exp2f(gi[r] - s_g[jj]) : 0.f;
+        const float x = dP[n][e] * p.scale * D_;                    // d(q k^T)_ij
+        const float y = jj < ii ? -dA[n][e] * D_ : 0.f;             // dA_ij D_ij
+        dgc[r] += x * qk[n][e] + y * bi[r] * kk2[n][e];
+        db[r] += y * kk2[n][e];
+        dP[n][e] = x;
+        dA[n][e] = y * bi[r];
+      }
+    uint32_t xh[4], xl[4], yh[4], yl[4];
+    acc_to_a(dP[0], dP[1], xh, xl);
+    acc_to_a(dA[0], dA[1], yh, yl);
+#pragma unroll
+    for (int n = 0; n < D / 8; n += 2) {
+      uint32_t b[4];
+      load_b_nn<D>(base + L::K, jb * 16, n * 8, lane, b);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(dq[n + u], xh, b[2 * u], b[2 * u + 1]);
+        mma16816(dk[n + u], yh, b[2 * u], b[2 * u + 1]);
+        mma16816(dq[n + u], xl, b[2 * u], b[2 * u + 1]);
+        mma16816(dk[n + u], yl, b[2 * u], b[2 * u + 1]);
+      }
+    }
+  }
+  // the same pairs seen from their column: rows j (this warp's tokens), columns i >= j
+#pragma unroll 1
+  for (int ib = warp; ib < 4; ++ib) {
+    float dP[2][4] = {}, dA[2][4] = {}, qk[2][4] = {}, kk2[2][4] = {};
+#pragma unroll 1
+    for (int kk = 0; kk < D; kk += 16) {
+      uint32_t vh[4], vl[4], b[4], d[4];
+      load_a_t<64>(base + L::VT, r0, kk, lane, vh);
+      load_a_t<64>(base + L::VT + L::TILE, r0, kk, lane, vl);
+      load_b_nt<D>(base + L::DO, ib * 16, kk, lane, b);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(dP[u], vh, b[2 * u], b[2 * u + 1]);
+        mma16816(dP[u], vl, b[2 * u], b[2 * u + 1]);
+      }
+      load_b_nn<64>(base + L::YT, kk, ib * 16, lane, b);
+      load_b_nn<64>(base + L::YT + L::TILE, kk, ib * 16, lane, d);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(dA[u], vh, b[2 * u], b[2 * u + 1]);
+        mma16816(dA[u], vl, b[2 * u], b[2 * u + 1]);
+        mma16816(dA[u], vh, d[2 * u], d[2 * u + 1]);
+      }
+      load_a<D>(base + L::K, r0, kk, lane, vh);
+      load_b_nt<D>(base + L::Q, ib * 16, kk, lane, b);
+      load_b_nt<D>(base + L::K, ib * 16, kk, lane, d);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(qk[u], vh, b[2 * u], b[2 * u + 1]);
+        mma16816(kk2[u], vh, d[2 * u], d[2 * u + 1]);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = e >> 1, jj = i + 8 * r, ii = ib * 16 + n * 8 + c2 + (e & 1);
+        const float D_ = jj <= ii ? exp2f(s_g[ii] - gi[r]) : 0.f;
+        const float x = dP[n][e] * p.scale * D_;
+        const float y = jj < ii ? -dA[n][e] * D_ * s_b[ii] : 0.f;
+        dgc[r] -= x * qk[n][e] + y * kk2[n][e];
+        dP[n][e] = x;
+        dA[n][e] = y;
+      }
+    uint32_t xh[4], xl[4], yh[4], yl[4];
+    acc_to_a(dP[0], dP[1], xh, xl);
+    acc_to_a(dA[0], dA[1], yh, yl);
+#pragma unroll
+    for (int n = 0; n < D / 8; n += 2) {
+      uint32_t b[4], d[4];
+      load_b_nn<D>(base + L::Q, ib * 16, n * 8, lane, b);
+      load_b_nn<D>(base + L::K, ib * 16, n * 8, lane, d);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(dk[n + u], xh, b[2 * u], b[2 * u + 1]);
+        mma16816(dk[n + u], xl, b[2 * u], b[2 * u + 1]);
+        mma16816(dk[n + u], yh, d[2 * u], d[2 * u + 1]);
+        mma16816(dk[n + u], yl, d[2 * u], d[2 * u + 1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      if (i + 8 * r < len) {
+        const long long at = off + (i + 8 * r) * stride + n * 8 + c2;
+        *reinterpret_cast<uint32_t*>(p.dq + at) = pack_bf16x2(dq[n][2 * r], dq[n][2 * r + 1]);
+        *reinterpret_cast<uint32_t*>(p.dk + at) = pack_bf16x2(dk[n][2 * r], dk[n][2 * r + 1]);
+      }
+  // gradient of G -> gradient of g (suffix sums); G_last collects the decays of the state
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const float a = quad_sum(dgc[r]), b = quad_sum(db[r]);
+    if ((lane & 3) == 0) {
+      s_dg[i + 8 * r] = a;
+      if (i + 8 * r < len) p.dbeta[(long long)(t + i + 8 * r) * p.H + h] = b;
+    }
+  }
+  float tot = xs + exp2f(s_g[C - 1]) * sdot;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+  if (lane == 0) s_red[warp] = tot;
+  __syncthreads();
+  if (warp == 0) {
+    const float last = (s_red[0] + s_red[1]) + (s_red[2] + s_red[3]);
+    const float x0 = s_dg[2 * lane], x1 = s_dg[2 * lane + 1] + (lane == 31 ? last : 0.f);
+    float run = x0 + x1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float y = __shfl_down_sync(0xffffffffu, run, o);
+      if (lane + o < 32) run += y;
+    }
+    const long long at = (long long)(t + 2 * lane) * p.H + h;
+    if (2 * lane < len) p.dg[at] = run;
+    if (2 * lane + 1 < len) p.dg[at + p.H] = run - x0;
+  }
+}
+
+template <int D>
+int launch_gdr(const GdrParams& p, int T, bool grad, cudaStream_t s) {
+  constexpr int PREP = PREP_TILES<D> + C * (C + 4) * 4 + 128;
+  static bool cfg = false;
+  cudaError_t e;
+  if (!cfg) {
+    if ((e = cudaFuncSetAttribute(gdr_prep_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, PREP)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gdr_scan_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ScanSmem<D>::TOTAL)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gdr_scan_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ScanSmem<D>::TOTAL)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gdr_scan_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, ScanSmem<D>::TOTAL)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gdr_grad_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, GradSmem<D>::TOTAL)) != cudaSuccess)
+      return (int)e;
+    cfg = true;
+  }
+  const dim3 chunks(T / C + p.n_seq, p.H);       // at least the number of chunks of any packing of T tokens
+  const unsigned scans = (unsigned)p.n_seq * p.H * (D / 64);
+  gdr_prep_kernel<D><<<chunks, THREADS, PREP, s>>>(p);
+  if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+  if (!grad) {
+    gdr_scan_kernel<D, false><<<scans, THREADS, ScanSmem<D>::TOTAL, s>>>(p);
+    return (int)cudaGetLastError();
+  }
+  gdr_scan_kernel<D, true><<<scans, THREADS, ScanSmem<D>::TOTAL, s>>>(p);
+  if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+  gdr_scan_bwd_kernel<D><<<scans, THREADS, ScanSmem<D>::TOTAL, s>>>(p);
+  if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+  gdr_grad_kernel<D><<<chunks, THREADS, GradSmem<D>::TOTAL, s>>>(p);
+  return (int)cudaGetLastError();
+}
+
+int run_gdr(const GdrParams& p, int T, int D, bool grad, cudaStream_t s) {
+  if (D == 128) return launch_gdr<128>(p, T, grad, s);
+  if (D == 64) return launch_gdr<64>(p, T, grad, s);
+  return -3;
+}
+
+GdrParams common(const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu, void* mp, float* gb,
+                 int n_seq, int H, float scale) {
+  GdrParams p{};
+  p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
+  p.g = g; p.beta = beta; p.cu = cu; p.mp = (__nv_bfloat16*)mp; p.gb = gb; p.n_seq = n_seq; p.H = H; p.scale = scale;
+  return p;
+}
+
+}  // namespace
+
+extern "C" {
+
+// Chunks a packed batch of T tokens in n_seq sequences can have at most: rows of the workspaces.
+int mcb_gdr_chunks(int T, int n_seq) { return T / C + n_seq; }
+
+// q, k, v, o [T, H, D] bf16; g, beta [T, H] fp32; cu_seqlens [n_seq + 1] int32 from 0 to T.  Workspaces, per chunk and
+// head: mp [4, 64, 64] bf16, gb [2, 64] fp32.
+int mcb_gdr_fwd(const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu_seqlens, void* o,
+                void* mp, float* gb, int T, int n_seq, int H, int D, float scale, void* stream_) {
+  if (n_seq <= 0 || T <= 0) return 0;
+  GdrParams p = common(q, k, v, g, beta, cu_seqlens, mp, gb, n_seq, H, scale);
+  p.o = (__nv_bfloat16*)o;
+  return run_gdr(p, T, D, false, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+// Further workspaces, per chunk and head: states [2, 2, D, D] bf16 (all S first, then all dS), values [2, 2, D, 64] bf16
+// (all V, then all Y).
+int mcb_gdr_bwd(const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu_seqlens,
+                const void* dout, void* dq, void* dk, void* dv, float* dg, float* dbeta, void* mp, float* gb, void* states,
+                void* values, int T, int n_seq, int H, int D, float scale, void* stream_) {
+  if (n_seq <= 0 || T <= 0) return 0;
+  GdrParams p = common(q, k, v, g, beta, cu_seqlens, mp, gb, n_seq, H, scale);
+  const long long n = (long long)mcb_gdr_chunks(T, n_seq) * H;
+  p.dout = (const __nv_bfloat16*)dout;
+  p.dq = (__nv_bfloat16*)dq; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.dg = dg; p.dbeta = dbeta;
+  p.S = (__nv_bfloat16*)states; p.dS = p.S + n * 2 * D * D;
+  p.V = (__nv_bfloat16*)values; p.Y = p.V + n * 2 * D * C;
+  return run_gdr(p, T, D, true, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+}  // extern "C"

@@ -347,6 +347,77 @@ class _SimpleGlaFn(torch.autograd.Function):
         return dq, dk_, dv, None, None, None
 
 
+class _GatedDeltaRuleFn(torch.autograd.Function):
+    """``csrc/linear_attention/gated_delta_rule.cu``; the inputs are all that is kept for the backward pass."""
+
+    @staticmethod
+    def _workspaces(lib, T, h, n_seq, device):
+        n = lib.mcb_gdr_chunks(T, n_seq) * h
+        return (torch.empty((n, 4, 64, 64), dtype=torch.bfloat16, device=device),
+                torch.empty((n, 2, 64), dtype=torch.float32, device=device), n)
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, beta, cu, scale, covered):
+        import ctypes
+
+        from . import _lib
+        lib = _lib.lib()
+        T, h, d = q.shape
+        q, k, v, g, beta = (t.contiguous() for t in (q, k, v, g, beta))
+        n_seq = cu.numel() - 1
+        o = torch.empty_like(v) if covered else torch.zeros_like(v)
+        mp, gb, _ = _GatedDeltaRuleFn._workspaces(lib, T, h, n_seq, q.device)
+        rc = lib.mcb_gdr_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(g), _lib.ptr(beta), _lib.ptr(cu),
+                             _lib.ptr(o), _lib.ptr(mp), _lib.ptr(gb), ctypes.c_int(T), ctypes.c_int(n_seq),
+                             ctypes.c_int(h), ctypes.c_int(d), ctypes.c_float(scale), _lib.stream_ptr())
+        _lib.check_rc(rc, 'mcb_gdr_fwd')
+        ctx.save_for_backward(q, k, v, g, beta, cu)
+        ctx.scale, ctx.covered = scale, covered
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        import ctypes
+
+        from . import _lib
+        lib = _lib.lib()
+        q, k, v, g, beta, cu = ctx.saved_tensors
+        T, h, d = q.shape
+        n_seq = cu.numel() - 1
+        do = do.contiguous()
+        alloc = torch.empty_like if ctx.covered else torch.zeros_like
+        dq, dk, dv, dg, dbeta = (alloc(t) for t in (q, k, v, g, beta))
+        mp, gb, n = _GatedDeltaRuleFn._workspaces(lib, T, h, n_seq, q.device)
+        states = torch.empty((2, n, 2, d, d), dtype=torch.bfloat16, device=q.device)
+        values = torch.empty((2, n, 2, d, 64), dtype=torch.bfloat16, device=q.device)
+        rc = lib.mcb_gdr_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(g), _lib.ptr(beta), _lib.ptr(cu),
+                             _lib.ptr(do), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(dg), _lib.ptr(dbeta),
+                             _lib.ptr(mp), _lib.ptr(gb), _lib.ptr(states), _lib.ptr(values), ctypes.c_int(T),
+                             ctypes.c_int(n_seq), ctypes.c_int(h), ctypes.c_int(d), ctypes.c_float(ctx.scale),
+                             _lib.stream_ptr())
+        _lib.check_rc(rc, 'mcb_gdr_bwd')
+        return dq, dk, dv, dg, dbeta, None, None, None
+
+
+_chunk_gated_delta_rule_torch = chunk_gated_delta_rule
+
+
+def chunk_gated_delta_rule(q, k, v, g, beta, cu_seqlens=None, scale: Optional[float] = None,  # noqa: F811
+                           chunk: int = 64):
+    """Dispatches to the CUDA kernels (bf16 q / k / v with square heads of 64 or 128) or the torch evaluation."""
+    T, h, d = q.shape
+    if _cuda_ok(q, k, v) and d in (64, 128) and k.shape == q.shape and v.shape == q.shape and T > 0 \
+            and g.is_floating_point() and beta.is_floating_point() and g.shape == beta.shape == (T, h):
+        host = (0, T) if cu_seqlens is None else getattr(cu_seqlens, '_host_list', None)
+        # tokens outside every sequence read as zero: only boundaries known to span the batch spare the zero fill
+        covered = host is not None and host[0] == 0 and host[-1] == T
+        cu = torch.tensor([0, T], dtype=torch.int32, device=q.device) if cu_seqlens is None else \
+            cu_seqlens.to(device=q.device, dtype=torch.int32)
+        return _GatedDeltaRuleFn.apply(q, k, v, g.float(), beta.float(), cu,
+                                       float(d**-0.5 if scale is None else scale), covered)
+    return _chunk_gated_delta_rule_torch(q, k, v, g, beta, cu_seqlens, scale, chunk)
+
+
 def simple_gla(q, k, v, decay, cu_seqlens=None, scale: Optional[float] = None) -> torch.Tensor:
     """Dispatches to the chunked CUDA kernels (bf16, square 64 / 128 state) or the torch restatement."""
     T, h, dk = q.shape

@@ -42,3 +42,44 @@ def test_simple_gla_chunk_edges(T, h, d, cuts):
     # fp32 products and states (16-bit-mantissa terms): what remains is the rounding of the result to bf16, 2^-9
     for a, b in zip([o, *grads], [ref, *torch.autograd.grad(ref, wide, dy.double())]):
         assert _rel(a, b) < 2 ** -8
+
+
+def _delta_rule(q, k, v, g, beta, spans):
+    out = []
+    for s, e in spans:
+        S = torch.zeros(q.shape[1], q.shape[2], q.shape[2], dtype=torch.float64, device=DEV)
+        for t in range(s, e):
+            S = S * g[t].exp()[:, None, None]
+            write = (v[t] - torch.einsum('hkv,hk->hv', S, k[t])) * beta[t][:, None]
+            S = S + k[t][:, :, None] * write[:, None, :]
+            out.append(torch.einsum('hkv,hk->hv', S, q[t]) * q.shape[2] ** -0.5)
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize('T,h,d,cuts', [(1, 1, 64, []), (5, 2, 128, [2, 2]), (63, 2, 64, []), (64, 3, 128, []),
+                                        (65, 2, 128, [1]), (300, 4, 64, [3, 130, 131]), (270, 2, 128, [128])])
+def test_gated_delta_rule_chunk_edges(T, h, d, cuts):
+    from mcore_bridge_b200.ops.gdn import chunk_gated_delta_rule, l2norm
+    (q, k, v, dy), gen = _inputs(T, h, d, 2)
+    q, k = l2norm(q), l2norm(k)
+    g = -torch.rand(T, h, generator=gen, device=DEV) * torch.tensor([0.05, 8.0, 0.5, 0.001], device=DEV)[:h]
+    beta = torch.rand(T, h, generator=gen, device=DEV)
+    cu = torch.tensor([0] + cuts + [T], dtype=torch.int32, device=DEV)
+    leaves = [t.requires_grad_() for t in (q, k, v, g, beta)]
+    o = chunk_gated_delta_rule(*leaves, cu)
+    grads = torch.autograd.grad(o, leaves, dy)
+    wide = [t.detach().double().requires_grad_() for t in leaves]
+    ref = _delta_rule(*wide, _spans(T, cuts))
+    # fp32 throughout (operands with 16 mantissa bits): bf16 results are rounded once, g and beta gradients not at all
+    for a, b in zip([o, *grads], [ref, *torch.autograd.grad(ref, wide, dy.double())]):
+        assert _rel(a, b) < (2 ** -8 if a.dtype == torch.bfloat16 else 2 ** -12)
+
+
+def test_gated_delta_rule_outside_every_sequence_is_zero():
+    from mcore_bridge_b200.ops.gdn import chunk_gated_delta_rule
+    (q, k, v, dy), _ = _inputs(100, 2, 64, 3)
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    g, beta = -torch.rand(100, 2, device=DEV), torch.rand(100, 2, device=DEV)
+    o = chunk_gated_delta_rule(*leaves, g, beta, torch.tensor([0, 70], dtype=torch.int32, device=DEV))
+    grads = torch.autograd.grad(o, leaves, dy)
+    assert all((t[70:] == 0).all() and (t[:70] != 0).any() for t in (o, *grads))
