@@ -403,8 +403,9 @@ int mcb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, void* y, v
 }
 
 static int rmsnorm_bwd_launch(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                              float* dw, float* partials, long long rows, int H, long long ldx, float eps,
+                              void* dw_any, int dw_bf16, float* partials, long long rows, int H, long long ldx, float eps,
                               int zero_centered, cudaStream_t s) {
+  float* dw = dw_bf16 ? nullptr : reinterpret_cast<float*>(dw_any);
   if (rows == 0) return 0;
   if (H % 8 || ldx % 8) return -1;
   // the two-rows-per-iteration kernel needs up to ~160 registers: blocks stay at <= 256 threads
@@ -415,7 +416,8 @@ static int rmsnorm_bwd_launch(const void* dy, const void* x, const void* w, cons
   long long cap = (long long)device_sm_count() * (vpt <= 2 ? 2 : 1);
   long long pairs = (rows + 1) / 2;
   long long grid = pairs < cap ? pairs : cap;
-  if (!dw) partials = nullptr;
+  if (!dw_any) partials = nullptr;
+  if (dw_bf16 && !partials) return -3;
 #define LAUNCH(V)                                                                                                    \
   rmsnorm_bwd_kernel<V><<<(int)grid, threads, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,              \
                                                       (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,      \
@@ -427,7 +429,10 @@ static int rmsnorm_bwd_launch(const void* dy, const void* x, const void* w, cons
   else if (vpt <= 8) LAUNCH(8);
   else return -2;
 #undef LAUNCH
-  if (partials) launch_reduce_partials(partials, (int)grid, H, dw, nullptr, H, s);
+  if (partials && dw_bf16)
+    launch_reduce_partials<__nv_bfloat16>(partials, (int)grid, H, reinterpret_cast<__nv_bfloat16*>(dw_any), nullptr, H, s);
+  else if (partials)
+    launch_reduce_partials<float>(partials, (int)grid, H, dw, nullptr, H, s);
   return (int)cudaGetLastError();
 }
 
@@ -435,7 +440,7 @@ static int rmsnorm_bwd_launch(const void* dy, const void* x, const void* w, cons
 // dres (optional) is added to dx (residual branch).
 int mcb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                     float* dw, long long rows, int H, long long ldx, float eps, int zero_centered, void* stream_) {
-  return rmsnorm_bwd_launch(dy, x, w, rstd, dres, dx, dw, nullptr, rows, H, ldx, eps, zero_centered,
+  return rmsnorm_bwd_launch(dy, x, w, rstd, dres, dx, dw, 0, nullptr, rows, H, ldx, eps, zero_centered,
                             reinterpret_cast<cudaStream_t>(stream_));
 }
 
@@ -450,11 +455,12 @@ int mcb_rmsnorm_bwd_partial_rows(long long rows, int H) {
 }
 
 // Same as mcb_rmsnorm_bwd, but the weight gradient is summed in a fixed order through `partials`
-// ([mcb_rmsnorm_bwd_partial_rows(rows, H), H] fp32 scratch), so it repeats bit for bit.
+// ([mcb_rmsnorm_bwd_partial_rows(rows, H), H] fp32 scratch), so it repeats bit for bit.  dw [H]: fp32, added to, or, with
+// dw_bf16, bf16 and overwritten.
 int mcb_rmsnorm_bwd_det(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                        float* dw, float* partials, long long rows, int H, long long ldx, float eps, int zero_centered,
-                        void* stream_) {
-  return rmsnorm_bwd_launch(dy, x, w, rstd, dres, dx, dw, partials, rows, H, ldx, eps, zero_centered,
+                        void* dw, int dw_bf16, float* partials, long long rows, int H, long long ldx, float eps,
+                        int zero_centered, void* stream_) {
+  return rmsnorm_bwd_launch(dy, x, w, rstd, dres, dx, dw, dw_bf16, partials, rows, H, ldx, eps, zero_centered,
                             reinterpret_cast<cudaStream_t>(stream_));
 }
 

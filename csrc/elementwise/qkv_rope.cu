@@ -448,11 +448,12 @@ int mcb_qkv_bwd_partial_rows(long long T) {
   return (int)(T < cap ? T : cap);
 }
 
-// dwq / dwk: fp32 [d], accumulated into (caller zeroes or carries them across micro-batches).  With `partials` the
-// norm-weight gradients are summed in a fixed order (bit-reproducible); without, with atomics.
+// dwq / dwk: fp32 [d], accumulated into (caller zeroes or carries them across micro-batches), or, with `dw_bf16` (needs
+// `partials`), bf16 [d] and overwritten.  With `partials` the norm-weight gradients are summed in a fixed order
+// (bit-reproducible); without, with atomics.
 int mcb_qkv_split_norm_rope_bwd(const void* qkv, const void* wq, const void* wk, const float* cosb, const float* sinb,
                                 const void* dq, const void* dk, const void* dv, const void* dgate, void* dqkv,
-                                float* dwq, float* dwk, float* partials, long long T, int ng, int qpg, int d, int has_gate,
+                                void* dwq_any, void* dwk_any, int dw_bf16, float* partials, long long T, int ng, int qpg, int d, int has_gate,
                                 int rot, int interleaved, int norm, int zero_centered, float eps, long long ld,
                                 void* stream_) {
   if (T == 0) return 0;
@@ -461,6 +462,9 @@ int mcb_qkv_split_norm_rope_bwd(const void* qkv, const void* wq, const void* wk,
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
   const int grid = mcb_qkv_bwd_partial_rows(T);
   if (!norm) partials = nullptr;
+  if (norm && dw_bf16 && !partials) return -3;
+  float* dwq = dw_bf16 ? nullptr : reinterpret_cast<float*>(dwq_any);
+  float* dwk = dw_bf16 ? nullptr : reinterpret_cast<float*>(dwk_any);
   if (d == 128 && rot == 128 && !interleaved) {
     qkv_bwd_fast_kernel<<<grid, WARPS * 32, 0, s>>>(
         (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, cosb, sinb,
@@ -472,7 +476,11 @@ int mcb_qkv_split_norm_rope_bwd(const void* qkv, const void* wq, const void* wk,
         (const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, (const __nv_bfloat16*)dgate,
         (__nv_bfloat16*)dqkv, dwq, dwk, partials, T, L);
   }
-  if (partials) launch_reduce_partials(partials, grid, 2 * d, dwq, dwk, d, s);   // rows are [dwq | dwk]
+  if (partials && dw_bf16)                                                       // rows are [dwq | dwk]
+    launch_reduce_partials<__nv_bfloat16>(partials, grid, 2 * d, reinterpret_cast<__nv_bfloat16*>(dwq_any),
+                                          reinterpret_cast<__nv_bfloat16*>(dwk_any), d, s);
+  else if (partials)
+    launch_reduce_partials<float>(partials, grid, 2 * d, dwq, dwk, d, s);
   return (int)cudaGetLastError();
 }
 

@@ -51,14 +51,14 @@ class _RMSNormCuda(torch.autograd.Function):
         dw = part = None
         if ctx.needs_input_grad[1]:
             # per-CTA partial rows summed in a fixed order: the weight gradient repeats bit for bit
-            dw = torch.zeros(H, dtype=torch.float32, device=x2.device)
+            dw = (torch.empty if rows else torch.zeros)(H, dtype=w.dtype, device=x2.device)
             part = torch.empty((_lib.lib().mcb_rmsnorm_bwd_partial_rows(_ll(rows), _int(H)), H), dtype=torch.float32,
                                device=x2.device)
         rc = _lib.lib().mcb_rmsnorm_bwd_det(_lib.ptr(dy2), _lib.ptr(x2), _lib.ptr(w), _lib.ptr(rstd), None,
-                                            _lib.ptr(dx), _lib.ptr(dw), _lib.ptr(part), _ll(rows), _int(H),
+                                            _lib.ptr(dx), _lib.ptr(dw), _int(1), _lib.ptr(part), _ll(rows), _int(H),
                                             _ll(x2.stride(0)), _f(ctx.eps), _int(int(ctx.zc)), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_rmsnorm_bwd_det')
-        return dx.view(ctx.shape), (dw.to(w.dtype) if dw is not None else None), None, None
+        return dx.view(ctx.shape), dw, None, None
 
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, zero_centered: bool = False) -> torch.Tensor:

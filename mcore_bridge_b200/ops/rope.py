@@ -110,19 +110,20 @@ class _QkvCuda(torch.autograd.Function):
         if has_gate:
             dgate = _c(dgate, (T, nq, d))
         dqkv = torch.empty_like(qkv)
-        dwq = torch.zeros(d, dtype=torch.float32, device=dev) if norm else None
-        dwk = torch.zeros(d, dtype=torch.float32, device=dev) if norm else None
+        # bf16 weights (the only ones this path takes): the reduction below writes them rounded
+        alloc = torch.empty if T else torch.zeros
+        dwq, dwk = alloc((2, d), dtype=wq.dtype, device=dev).unbind(0) if norm else (None, None)
         # per-CTA partial sums of the norm-weight gradients, added in a fixed order (bit-reproducible)
         part = torch.empty((_lib.lib().mcb_qkv_bwd_partial_rows(_ll(T)), 2, d), dtype=torch.float32,
                            device=dev) if norm else None
         rc = _lib.lib().mcb_qkv_split_norm_rope_bwd(
             _lib.ptr(qkv), _lib.ptr(wq), _lib.ptr(wk), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(dq), _lib.ptr(dk),
             _lib.ptr(dv), _lib.ptr(dgate if has_gate else None), _lib.ptr(dqkv), _lib.ptr(dwq), _lib.ptr(dwk),
-            _lib.ptr(part), _ll(T),
+            _int(1), _lib.ptr(part), _ll(T),
             _int(ng), _int(qpg), _int(d), _int(int(has_gate)), _int(rot), _int(int(interleaved)), _int(int(norm)),
             _int(int(zc)), _f(eps), _ll(qkv.stride(0)), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_qkv_split_norm_rope_bwd')
-        return (dqkv, dwq.to(wq.dtype) if norm else None, dwk.to(wk.dtype) if norm else None, None, None, None, None,
+        return (dqkv, dwq, dwk, None, None, None, None,
                 None, None, None, None, None)
 
 
