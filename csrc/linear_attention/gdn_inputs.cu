@@ -1,0 +1,390 @@
+// Everything between the input projection of a gated-DeltaNet block and its delta rule, one pass each way.
+//
+// The projection row of a token holds, per key-head group, [q (d) | k (d) | v (R d) | z (R d) | b (R) | a (R)].  Forward:
+// causal depthwise conv (4 taps) + SiLU over q | k | v, L2 normalisation of q and k, q and k repeated for the R value heads
+// of the group, z copied out, beta = sigmoid(b), g = -exp(A_log) softplus(a + dt_bias).  Backward: the gradient of the
+// whole projection row, of the taps and of the two per-head vectors; everything in between is recomputed from the
+// projection, which is all that is kept.
+//
+// A warp owns one group and walks consecutive tokens with the last rows in registers, so every projection element is read
+// once (plus 3 rows of overlap per walk) instead of once per slice, copy, norm and tap.  Bound: memory.
+//
+// Values are rounded to bf16 where the separate operators store them (convolution output, normalised q / k).
+#include "../common/host_utils.cuh"
+#include "../common/partials.cuh"
+#include "../common/ptx.cuh"
+
+using namespace mcb;
+
+namespace {
+
+constexpr int KW = 4;            // taps
+constexpr int WARPS = 4;
+constexpr int TOK_F = 16;        // tokens a warp walks, forward / backward: enough warps at a few thousand tokens
+constexpr int TOK_B = 16;
+
+struct InParams {
+  const __nv_bfloat16* proj;               // [T, ld]
+  const __nv_bfloat16 *w, *A_log, *dt;     // [G * (2 + R) d, 4], [G * R], [G * R]
+  const int* seq_start;                    // [T]
+  __nv_bfloat16 *q, *k, *v, *z;            // [T, G * R, d]
+  float *g, *beta;                         // [T, G * R]
+  const __nv_bfloat16 *dq, *dk, *dv, *dz;
+  const float *dg, *dbeta;
+  __nv_bfloat16* dproj;                    // [T, ld_d]
+  float* wpart;                            // [blocks along T, G * (2 + R) d * 4]
+  float* hpart;                            // [blocks along T, 2 * G * R]: dA_log, ddt_bias
+  long long ld, ld_d;
+  int T, G;
+};
+
+__device__ __forceinline__ float wsum(float x) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+__device__ __forceinline__ float sigmoid_(float x) { return 1.f / (1.f + __expf(-x)); }
+__device__ __forceinline__ float bf_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
+
+// exp with the rounding error of x * log2(e) carried along: the decays are sums of hundreds of these
+__device__ __forceinline__ float exp_full(float x) {
+  const float t = x * 1.44269504f;
+  const float r = fmaf(x, 1.44269504f, -t) + x * 1.92596299e-8f;
+  return exp2f(t) * fmaf(r, 0.693147181f, 1.f);
+}
+__device__ __forceinline__ float softplus_(float x) { return x > 20.f ? x : log1pf(exp_full(x)); }
+
+// N consecutive bf16 (N even) at a 4-byte aligned address
+template <int N>
+__device__ __forceinline__ void ldn(const __nv_bfloat16* p, float (&f)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + i));
+    f[i] = t.x;
+    f[i + 1] = t.y;
+  }
+}
+template <int N>
+__device__ __forceinline__ void stn(__nv_bfloat16* p, const float (&f)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) *reinterpret_cast<uint32_t*>(p + i) = pack_bf16x2(f[i], f[i + 1]);
+}
+
+// S = 2 + R slices of d channels (q, k, R times v); a lane owns PER = d / 32 consecutive channels of each
+template <int D, int R>
+__global__ void __launch_bounds__(WARPS * 32)
+gdn_inputs_fwd_kernel(const InParams p) {
+  constexpr int PER = D / 32, S = 2 + R;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = blockIdx.y;
+  const int t0 = (blockIdx.x * WARPS + warp) * TOK_F, t1 = min(t0 + TOK_F, p.T);
+  if (t0 >= p.T) return;
+  const __nv_bfloat16* src = p.proj + (long long)grp * (2 * D + 2 * R * D + 2 * R) + lane * PER;
+  float w[S][PER][KW];
+#pragma unroll
+  for (int s = 0; s < S; ++s)
+#pragma unroll
+    for (int c = 0; c < PER; ++c)
+#pragma unroll
+      for (int j = 0; j < KW; ++j)
+        w[s][c][j] = __bfloat162float(p.w[((long long)grp * S * D + s * D + lane * PER + c) * KW + j]);
+  const int hv = lane < R ? grp * R + lane : 0;
+  const float neg_a = lane < R ? -exp_full(__bfloat162float(p.A_log[hv])) : 0.f;
+  const float dtb = lane < R ? __bfloat162float(p.dt[hv]) : 0.f;
+  float x[KW][S][PER];                           // row t is slot t & 3
+#pragma unroll
+  for (int u = 0; u < KW; ++u)
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+#pragma unroll
+      for (int c = 0; c < PER; ++c) x[u][s][c] = 0.f;
+#pragma unroll
+  for (int b = 1; b < KW; ++b) {
+    const int t = t0 - b;
+    if (t >= 0) {
+#pragma unroll
+      for (int s = 0; s < S; ++s) ldn<PER>(src + t * p.ld + s * D, x[KW - b][s]);    // t0 is a multiple of 4
+    }
+  }
+  for (int tb = t0; tb < t1; tb += KW) {
+#pragma unroll
+    for (int u = 0; u < KW; ++u) {
+      const int t = tb + u;
+      if (t >= t1) break;
+#pragma unroll
+      for (int s = 0; s < S; ++s) ldn<PER>(src + t * p.ld + s * D, x[u][s]);
+      const int back = t - p.seq_start[t];       // rows of the same sequence before this one
+      float y[S][PER];
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+#pragma unroll
+        for (int c = 0; c < PER; ++c) {
+          float a = 0.f;
+#pragma unroll
+          for (int j = 0; j < KW; ++j)
+            a = fmaf(w[s][c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][s][c] : 0.f, a);
+          y[s][c] = bf_round(a * sigmoid_(a));
+        }
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        float ss = 0.f;
+#pragma unroll
+        for (int c = 0; c < PER; ++c) ss += y[s][c] * y[s][c];
+        const float r = rsqrtf(wsum(ss) + 1e-6f);
+#pragma unroll
+        for (int c = 0; c < PER; ++c) y[s][c] *= r;
+      }
+      const long long row = ((long long)t * p.G + grp) * R * D + lane * PER;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        stn<PER>(p.q + row + r * D, y[0]);
+        stn<PER>(p.k + row + r * D, y[1]);
+        stn<PER>(p.v + row + r * D, y[2 + r]);
+        float zz[PER];
+        ldn<PER>(src + t * p.ld + (S + r) * D, zz);
+        stn<PER>(p.z + row + r * D, zz);
+      }
+      if (lane < R) {
+        const __nv_bfloat16* ba = src - lane * PER + t * p.ld + (S + R) * D + lane;
+        const long long at = (long long)t * p.G * R + hv;
+        p.beta[at] = 1.f / (1.f + exp_full(-__bfloat162float(ba[0])));
+        p.g[at] = neg_a * softplus_(__bfloat162float(ba[R]) + dtb);
+      }
+    }
+  }
+}
+
+template <int D, int R>
+__global__ void __launch_bounds__(WARPS * 32)
+gdn_inputs_bwd_kernel(const InParams p) {
+  constexpr int PER = D / 32, S = 2 + R;
+  __shared__ float s_w[WARPS][32 * PER * KW];
+  __shared__ float s_h[WARPS][2][R];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = blockIdx.y;
+  const int t0 = (blockIdx.x * WARPS + warp) * TOK_B, t1 = min(t0 + TOK_B, p.T);
+  const int width = 2 * D + 2 * R * D + 2 * R;
+  const __nv_bfloat16* src = p.proj + (long long)grp * width + lane * PER;
+  __nv_bfloat16* dst = p.dproj + (long long)grp * width + lane * PER;
+  float dw[S][PER][KW];
+#pragma unroll
+  for (int s = 0; s < S; ++s)
+#pragma unroll
+    for (int c = 0; c < PER; ++c)
+#pragma unroll
+      for (int j = 0; j < KW; ++j) dw[s][c][j] = 0.f;
+  float dA = 0.f, ddt = 0.f;
+  if (t0 < t1) {
+    // slices are walked one after the other: the rows in flight of one slice are what fits the registers
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      float w[PER][KW], x[KW][PER], dp[KW][PER];     // row t and its dpre in slot t & 3
+#pragma unroll
+      for (int c = 0; c < PER; ++c)
+#pragma unroll
+        for (int j = 0; j < KW; ++j)
+          w[c][j] = __bfloat162float(p.w[((long long)grp * S * D + s * D + lane * PER + c) * KW + j]);
+#pragma unroll
+      for (int u = 0; u < KW; ++u)
+#pragma unroll
+        for (int c = 0; c < PER; ++c) x[u][c] = dp[u][c] = 0.f;
+#pragma unroll
+      for (int b = 1; b < KW; ++b)
+        if (t0 - b >= 0) ldn<PER>(src + (t0 - b) * p.ld + s * D, x[KW - b]);
+      const int te = min(t1 + KW - 1, p.T);          // dpre of the KW - 1 tokens behind the walk reaches into it
+      for (int tb = t0; tb < t1 + KW - 1; tb += KW) {
+#pragma unroll
+        for (int u = 0; u < KW; ++u) {
+          const int t = tb + u;
+          if (t >= t1 + KW - 1) break;
+          int first = 0x7fffffff;                    // first token of t's sequence; none past the end of the batch
+          if (t < te) {
+            first = p.seq_start[t];
+            ldn<PER>(src + t * p.ld + s * D, x[u]);
+            const long long row = ((long long)t * p.G + grp) * R * D + lane * PER;
+            float d[PER];
+            if (s < 2) {
+              const __nv_bfloat16* dn = (s == 0 ? p.dq : p.dk) + row;
+              ldn<PER>(dn, d);
+#pragma unroll
+              for (int r = 1; r < R; ++r) {
+                float e[PER];
+                ldn<PER>(dn + r * D, e);
+#pragma unroll
+                for (int c = 0; c < PER; ++c) d[c] += e[c];
+              }
+            } else {
+              ldn<PER>(p.dv + row + (s - 2) * D, d);
+            }
+            const int back = t - first;
+            float pre[PER], sg[PER], y[PER];
+#pragma unroll
+            for (int c = 0; c < PER; ++c) {
+              float a = 0.f;
+#pragma unroll
+              for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
+              pre[c] = a;
+              sg[c] = sigmoid_(a);
+              y[c] = bf_round(a * sg[c]);
+            }
+            if (s < 2) {                             // through y * rsqrt(sum y^2 + eps)
+              float ss = 0.f, dot = 0.f;
+#pragma unroll
+              for (int c = 0; c < PER; ++c) {
+                ss += y[c] * y[c];
+                dot += y[c] * d[c];
+              }
+              const float r = rsqrtf(wsum(ss) + 1e-6f);
+              dot = wsum(dot) * r * r;
+#pragma unroll
+              for (int c = 0; c < PER; ++c) d[c] = r * (d[c] - y[c] * dot);
+            }
+#pragma unroll
+            for (int c = 0; c < PER; ++c) {
+              dp[u][c] = d[c] * sg[c] * (1.f + pre[c] * (1.f - sg[c]));
+              if (t < t1) {                          // every token's tap gradients are added once, by its own walk
+#pragma unroll
+                for (int j = 0; j < KW; ++j)
+                  dw[s][c][j] = fmaf(dp[u][c], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, dw[s][c][j]);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < PER; ++c) dp[u][c] = 0.f;
+          }
+          // dpre of the rows t-3 .. t is complete for the projection row t - 3, as far as they share its sequence
+          const int tr = t - (KW - 1);
+          if (tr >= t0 && tr < t1) {
+            float dx[PER];
+#pragma unroll
+            for (int c = 0; c < PER; ++c) dx[c] = 0.f;
+#pragma unroll
+            for (int j = 0; j < KW; ++j) {           // tap j of row tr + (KW - 1 - j)
+              const int tt = tr + (KW - 1 - j);
+              const int f = tt == t ? first : (tt < p.T ? p.seq_start[tt] : 0x7fffffff);
+              if (f <= tr) {
+#pragma unroll
+                for (int c = 0; c < PER; ++c) dx[c] = fmaf(w[c][j], dp[(u + 4 - j) & 3][c], dx[c]);
+              }
+            }
+            stn<PER>(dst + tr * p.ld_d + s * D, dx);
+          }
+        }
+      }
+    }
+    const int hv = lane < R ? grp * R + lane : 0;
+    const float neg_a = lane < R ? -exp_full(__bfloat162float(p.A_log[hv])) : 0.f;
+    const float dtb = lane < R ? __bfloat162float(p.dt[hv]) : 0.f;
+    for (int t = t0; t < t1; ++t) {
+      const long long row = ((long long)t * p.G + grp) * R * D + lane * PER;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float zz[PER];
+        ldn<PER>(p.dz + row + r * D, zz);
+        stn<PER>(dst + t * p.ld_d + (S + r) * D, zz);
+      }
+      if (lane < R) {
+        const __nv_bfloat16* ba = src - lane * PER + t * p.ld + (S + R) * D + lane;
+        __nv_bfloat16* dba = dst - lane * PER + t * p.ld_d + (S + R) * D + lane;
+        const long long at = (long long)t * p.G * R + hv;
+        const float beta = 1.f / (1.f + exp_full(-__bfloat162float(ba[0])));
+        dba[0] = __float2bfloat16(p.dbeta[at] * beta * (1.f - beta));
+        const float xx = __bfloat162float(ba[R]) + dtb, dg = p.dg[at];
+        const float da = dg * neg_a * (1.f / (1.f + exp_full(-xx)));
+        dba[R] = __float2bfloat16(da);
+        dA += dg * neg_a * softplus_(xx);
+        ddt += da;
+      }
+    }
+  }
+  // the block's sums, in a fixed order
+  const long long wcols = (long long)p.G * S * D * KW;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+#pragma unroll
+    for (int c = 0; c < PER; ++c)
+#pragma unroll
+      for (int j = 0; j < KW; ++j) s_w[warp][(lane * PER + c) * KW + j] = dw[s][c][j];
+    __syncthreads();
+    for (int id = threadIdx.x; id < D * KW; id += WARPS * 32)
+      p.wpart[blockIdx.x * wcols + ((long long)grp * S + s) * D * KW + id] =
+          (s_w[0][id] + s_w[1][id]) + (s_w[2][id] + s_w[3][id]);
+    __syncthreads();
+  }
+  if (lane < R) {
+    s_h[warp][0][lane] = dA;
+    s_h[warp][1][lane] = ddt;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * R) {
+    const int which = threadIdx.x / R, r = threadIdx.x % R;
+    p.hpart[(long long)blockIdx.x * 2 * p.G * R + which * p.G * R + grp * R + r] =
+        (s_h[0][which][r] + s_h[1][which][r]) + (s_h[2][which][r] + s_h[3][which][r]);
+  }
+}
+
+int blocks_t(int T, int tok) { return (T + WARPS * tok - 1) / (WARPS * tok); }
+
+template <int D, int R>
+int launch_inputs(const InParams& p, bool grad, float* dw, float* dA, float* ddt, cudaStream_t s) {
+  if (!grad) {
+    gdn_inputs_fwd_kernel<D, R><<<dim3(blocks_t(p.T, TOK_F), p.G), WARPS * 32, 0, s>>>(p);
+    return (int)cudaGetLastError();
+  }
+  const int nb = blocks_t(p.T, TOK_B);
+  gdn_inputs_bwd_kernel<D, R><<<dim3(nb, p.G), WARPS * 32, 0, s>>>(p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return (int)e;
+  launch_reduce_partials<float>(p.wpart, nb, p.G * (2 + R) * D * KW, dw, nullptr, p.G * (2 + R) * D * KW, s);
+  if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+  launch_reduce_partials<float>(p.hpart, nb, 2 * p.G * R, dA, ddt, p.G * R, s);
+  return (int)cudaGetLastError();
+}
+
+int run_inputs(const InParams& p, int D, int R, bool grad, float* dw, float* dA, float* ddt, cudaStream_t s) {
+  if ((p.ld & 1) || (p.ld_d & 1)) return -2;     // rows start on 4-byte boundaries
+  if (D == 128 && R == 1) return launch_inputs<128, 1>(p, grad, dw, dA, ddt, s);
+  if (D == 128 && R == 2) return launch_inputs<128, 2>(p, grad, dw, dA, ddt, s);
+  if (D == 128 && R == 4) return launch_inputs<128, 4>(p, grad, dw, dA, ddt, s);
+  if (D == 64 && R == 1) return launch_inputs<64, 1>(p, grad, dw, dA, ddt, s);
+  if (D == 64 && R == 2) return launch_inputs<64, 2>(p, grad, dw, dA, ddt, s);
+  if (D == 64 && R == 4) return launch_inputs<64, 4>(p, grad, dw, dA, ddt, s);
+  return -3;
+}
+
+}  // namespace
+
+extern "C" {
+
+// Rows of the two partial-sum workspaces of the backward pass.
+int mcb_gdn_inputs_partials(int T) { return blocks_t(T, TOK_B); }
+
+// proj [T, ld] bf16 with G groups of [q d | k d | v R d | z R d | b R | a R]; w [G (2 + R) d, 4]; A_log, dt_bias [G R] bf16;
+// seq_start [T] int32.  Out: q, k, v, z [T, G R, d] bf16, g, beta [T, G R] fp32.
+int mcb_gdn_inputs_fwd(const void* proj, long long ld, const void* w, const void* A_log, const void* dt, const int* seq_start,
+                       void* q, void* k, void* v, void* z, float* g, float* beta, int T, int G, int R, int D, void* stream_) {
+  if (T <= 0) return 0;
+  InParams p{};
+  p.proj = (const __nv_bfloat16*)proj; p.ld = ld; p.w = (const __nv_bfloat16*)w; p.A_log = (const __nv_bfloat16*)A_log;
+  p.dt = (const __nv_bfloat16*)dt; p.seq_start = seq_start;
+  p.q = (__nv_bfloat16*)q; p.k = (__nv_bfloat16*)k; p.v = (__nv_bfloat16*)v; p.z = (__nv_bfloat16*)z; p.g = g; p.beta = beta;
+  p.T = T; p.G = G;
+  return run_inputs(p, D, R, false, nullptr, nullptr, nullptr, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+// dproj [T, G (2 d + 2 R d + 2 R)] contiguous; dw, dA, ddt fp32, zero on entry; wpart [partials, G (2 + R) d 4],
+// hpart [partials, 2 G R] fp32 workspaces.
+int mcb_gdn_inputs_bwd(const void* proj, long long ld, const void* w, const void* A_log, const void* dt, const int* seq_start,
+                       const void* dq, const void* dk, const void* dv, const void* dz, const float* dg, const float* dbeta,
+                       void* dproj, float* dw, float* dA, float* ddt, float* wpart, float* hpart, int T, int G, int R, int D,
+                       void* stream_) {
+  if (T <= 0) return 0;
+  InParams p{};
+  p.proj = (const __nv_bfloat16*)proj; p.ld = ld; p.w = (const __nv_bfloat16*)w; p.A_log = (const __nv_bfloat16*)A_log;
+  p.dt = (const __nv_bfloat16*)dt; p.seq_start = seq_start;
+  p.dq = (const __nv_bfloat16*)dq; p.dk = (const __nv_bfloat16*)dk; p.dv = (const __nv_bfloat16*)dv;
+  p.dz = (const __nv_bfloat16*)dz; p.dg = dg; p.dbeta = dbeta;
+  p.dproj = (__nv_bfloat16*)dproj; p.ld_d = (long long)G * (2 * D + 2 * R * D + 2 * R);
+  p.wpart = wpart; p.hpart = hpart; p.T = T; p.G = G;
+  return run_inputs(p, D, R, true, dw, dA, ddt, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+}  // extern "C"

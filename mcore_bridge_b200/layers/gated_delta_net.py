@@ -78,26 +78,32 @@ class GatedDeltaNet(nn.Module):
         T = proj.shape[0]
         nk = self.nk_local // cp
         nvh = nk * self.ratio
-        g = proj.view(T, nk, self.group_all)
-        qkv = g[..., :self.group_conv].reshape(T, nk * self.group_conv)
-        z = g[..., self.group_conv:self.group_qkvz].reshape(T, nvh, self.dv)
-        b = g[..., self.group_qkvz:self.group_qkvz + self.ratio].reshape(T, nvh)
-        a = g[..., self.group_qkvz + self.ratio:].reshape(T, nvh)
         w = self._cp_slice(self.conv1d.weight.squeeze(1), self.group_conv)
-        with nvtx_range('conv1d'):
-            qkv = G.causal_conv1d_silu(qkv.contiguous(), w, None, cu)
-        qkv = qkv.view(T, nk, self.group_conv)
-        q = qkv[..., :self.dk]
-        k = qkv[..., self.dk:2 * self.dk]
-        v = qkv[..., 2 * self.dk:].reshape(T, nvh, self.dv)
-        q, k = G.l2norm(q), G.l2norm(k)
-        if self.ratio > 1:
-            q = q.repeat_interleave(self.ratio, dim=1)
-            k = k.repeat_interleave(self.ratio, dim=1)
         A_log, dt_bias = self._cp_slice(self.A_log, 1), self._cp_slice(self.dt_bias, 1)
-        with nvtx_range('g_and_beta'):
-            gdecay = -A_log.float().exp() * F.softplus(a.float() + dt_bias.float())
-            beta = torch.sigmoid(b.float())
+        if G.gdn_inputs_supported(proj, w, A_log, dt_bias, self.ratio, self.dk, self.dv):
+            # one pass over the projection instead of its slices, copies, convolution, norms and gates one by one
+            seq_start = ctx.seq_start if cp == 1 and ctx.seq_start is not None else G._seq_start(cu, T, proj.device)
+            with nvtx_range('conv1d'):
+                q, k, v, z, gdecay, beta = G.gdn_inputs(proj, w, A_log, dt_bias, seq_start, nk, self.ratio, self.dk)
+        else:
+            g = proj.view(T, nk, self.group_all)
+            qkv = g[..., :self.group_conv].reshape(T, nk * self.group_conv)
+            z = g[..., self.group_conv:self.group_qkvz].reshape(T, nvh, self.dv)
+            b = g[..., self.group_qkvz:self.group_qkvz + self.ratio].reshape(T, nvh)
+            a = g[..., self.group_qkvz + self.ratio:].reshape(T, nvh)
+            with nvtx_range('conv1d'):
+                qkv = G.causal_conv1d_silu(qkv.contiguous(), w, None, cu)
+            qkv = qkv.view(T, nk, self.group_conv)
+            q = qkv[..., :self.dk]
+            k = qkv[..., self.dk:2 * self.dk]
+            v = qkv[..., 2 * self.dk:].reshape(T, nvh, self.dv)
+            q, k = G.l2norm(q), G.l2norm(k)
+            if self.ratio > 1:
+                q = q.repeat_interleave(self.ratio, dim=1)
+                k = k.repeat_interleave(self.ratio, dim=1)
+            with nvtx_range('g_and_beta'):
+                gdecay = -A_log.float().exp() * F.softplus(a.float() + dt_bias.float())
+                beta = torch.sigmoid(b.float())
         with nvtx_range('gated_delta_rule'):
             o = G.chunk_gated_delta_rule(q.contiguous(), k.contiguous(), v.contiguous(), gdecay, beta, cu)
         with nvtx_range('gated_norm'):

@@ -399,6 +399,70 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
         return dq, dk, dv, dg, dbeta, None, None, None
 
 
+class _GdnInputsFn(torch.autograd.Function):
+    """``csrc/linear_attention/gdn_inputs.cu``: projection rows -> q, k, v, z, g, beta; keeps the projection only."""
+
+    @staticmethod
+    def forward(ctx, proj, weight, A_log, dt_bias, seq_start, groups, ratio, d):
+        import ctypes
+
+        from . import _lib
+        T = proj.shape[0]
+        proj, w, A_log, dt_bias = proj.contiguous(), weight.contiguous(), A_log.contiguous(), dt_bias.contiguous()
+        h = groups * ratio
+        q, k, v, z = (torch.empty((T, h, d), dtype=proj.dtype, device=proj.device) for _ in range(4))
+        g, beta = (torch.empty((T, h), dtype=torch.float32, device=proj.device) for _ in range(2))
+        rc = _lib.lib().mcb_gdn_inputs_fwd(_lib.ptr(proj), ctypes.c_longlong(proj.stride(0)), _lib.ptr(w),
+                                           _lib.ptr(A_log), _lib.ptr(dt_bias), _lib.ptr(seq_start), _lib.ptr(q),
+                                           _lib.ptr(k), _lib.ptr(v), _lib.ptr(z), _lib.ptr(g), _lib.ptr(beta),
+                                           ctypes.c_int(T), ctypes.c_int(groups), ctypes.c_int(ratio), ctypes.c_int(d),
+                                           _lib.stream_ptr())
+        _lib.check_rc(rc, 'mcb_gdn_inputs_fwd')
+        ctx.save_for_backward(proj, w, A_log, dt_bias, seq_start)
+        ctx.meta = (groups, ratio, d)
+        return q, k, v, z, g, beta
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv, dz, dg, dbeta):
+        import ctypes
+
+        from . import _lib
+        lib = _lib.lib()
+        proj, w, A_log, dt_bias, seq_start = ctx.saved_tensors
+        groups, ratio, d = ctx.meta
+        T, h, dev = proj.shape[0], groups * ratio, proj.device
+
+        def full(t, shape, dtype):
+            return torch.zeros(shape, dtype=dtype, device=dev) if t is None else t.to(dtype).contiguous()
+
+        dq, dk, dv, dz = (full(t, (T, h, d), proj.dtype) for t in (dq, dk, dv, dz))
+        dg, dbeta = (full(t, (T, h), torch.float32) for t in (dg, dbeta))
+        dproj = torch.empty_like(proj)
+        dw, dA, ddt = (torch.zeros(t.shape, dtype=torch.float32, device=dev) for t in (w, A_log, dt_bias))
+        parts = lib.mcb_gdn_inputs_partials(T)
+        wpart = torch.empty((parts, w.numel()), dtype=torch.float32, device=dev)
+        hpart = torch.empty((parts, 2 * h), dtype=torch.float32, device=dev)
+        rc = lib.mcb_gdn_inputs_bwd(_lib.ptr(proj), ctypes.c_longlong(proj.stride(0)), _lib.ptr(w), _lib.ptr(A_log),
+                                    _lib.ptr(dt_bias), _lib.ptr(seq_start), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv),
+                                    _lib.ptr(dz), _lib.ptr(dg), _lib.ptr(dbeta), _lib.ptr(dproj), _lib.ptr(dw),
+                                    _lib.ptr(dA), _lib.ptr(ddt), _lib.ptr(wpart), _lib.ptr(hpart), ctypes.c_int(T),
+                                    ctypes.c_int(groups), ctypes.c_int(ratio), ctypes.c_int(d), _lib.stream_ptr())
+        _lib.check_rc(rc, 'mcb_gdn_inputs_bwd')
+        return dproj, dw.to(w.dtype), dA.to(A_log.dtype), ddt.to(dt_bias.dtype), None, None, None, None
+
+
+def gdn_inputs_supported(proj, weight, A_log, dt_bias, ratio: int, dk: int, dv: int) -> bool:
+    return (_cuda_ok(proj, weight, A_log, dt_bias) and dk == dv and dk in (64, 128) and ratio in (1, 2, 4)
+            and weight.shape[-1] == 4 and proj.shape[0] > 0)
+
+
+def gdn_inputs(proj, weight, A_log, dt_bias, seq_start, groups: int, ratio: int, d: int):
+    """Projection rows ``[T, groups * (2 d + 2 ratio d + 2 ratio)]``, per group ``[q | k | v | z | b | a]``, to the
+    inputs of the delta rule in one pass: ``q, k, v, z [T, groups * ratio, d]`` (convolved, q and k normalised and
+    repeated) and ``g, beta [T, groups * ratio]`` fp32.  ``weight [groups * (2 + ratio) * d, 4]``."""
+    return _GdnInputsFn.apply(proj, weight, A_log, dt_bias, seq_start, groups, ratio, d)
+
+
 _chunk_gated_delta_rule_torch = chunk_gated_delta_rule
 
 

@@ -83,3 +83,43 @@ def test_gated_delta_rule_outside_every_sequence_is_zero():
     o = chunk_gated_delta_rule(*leaves, g, beta, torch.tensor([0, 70], dtype=torch.int32, device=DEV))
     grads = torch.autograd.grad(o, leaves, dy)
     assert all((t[70:] == 0).all() and (t[:70] != 0).any() for t in (o, *grads))
+
+
+@pytest.mark.parametrize('T,groups,ratio,d,cuts', [(1, 1, 1, 64, []), (3, 2, 2, 128, [1]), (16, 1, 4, 64, [13, 15]),
+                                                   (65, 3, 2, 128, [62, 64]), (130, 2, 4, 128, []), (257, 2, 1, 64, [1, 2, 3])])
+def test_gdn_inputs_walk_edges(T, groups, ratio, d, cuts):
+    """Projection -> inputs of the delta rule in one pass, at the edges of a warp's walk (16 tokens) and of sequences."""
+    import torch.nn.functional as F
+    from mcore_bridge_b200.ops.attention_cuda import seq_start_from_cu
+    from mcore_bridge_b200.ops.gdn import gdn_inputs
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    S, h = 2 + ratio, groups * ratio
+
+    def rand(*shape):
+        return torch.randn(*shape, generator=gen, device=DEV).bfloat16()
+
+    proj, w = rand(T, groups * (2 * d + 2 * ratio * d + 2 * ratio)), rand(groups * S * d, 4) * 0.5
+    A_log, dt = rand(h), rand(h)
+    cu = torch.tensor([0] + cuts + [T], dtype=torch.int32, device=DEV)
+    leaves = [t.requires_grad_() for t in (proj, w, A_log, dt)]
+    out = gdn_inputs(*leaves, seq_start_from_cu(cu, T, DEV), groups, ratio, d)
+    cot = [rand(*t.shape).to(t.dtype) for t in out]
+    grads = torch.autograd.grad(out, leaves, cot)
+
+    wide = [t.detach().double().requires_grad_() for t in leaves]
+    qkv, z, b, a = wide[0].view(T, groups, -1).split([S * d, ratio * d, ratio, ratio], dim=-1)
+    qkv, pieces = qkv.reshape(T, -1), []
+    for s, e in _spans(T, cuts):
+        xs = F.pad(qkv[s:e], (0, 0, 3, 0))
+        pieces.append(sum(xs[j:j + e - s] * wide[1][:, j] for j in range(4)))
+    q, k, v = F.silu(torch.cat(pieces)).view(T, groups, -1).split([d, d, ratio * d], dim=-1)
+    q, k = (t * torch.rsqrt(t.pow(2).sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+    q, k = (t.repeat_interleave(ratio, dim=1) for t in (q, k))
+    ref = [q, k, v.reshape(T, h, d), z.reshape(T, h, d),
+           -wide[2].exp() * F.softplus(a.reshape(T, h) + wide[3]), torch.sigmoid(b.reshape(T, h))]
+    want = torch.autograd.grad(ref, wide, [c.double() for c in cot])
+    # bf16 results, q and k rounded once more before their norm: 2^-9 each; g and beta are fp32
+    for x, y in zip(out, ref):
+        assert _rel(x, y) < (2 ** -8 if x.dtype == torch.bfloat16 else 1e-5)
+    for x, y in zip(grads, want):
+        assert _rel(x, y) < 2 ** -7
