@@ -31,9 +31,15 @@ class KernelError(RuntimeError):
     pass
 
 
+_device_present = None  # whether the process has a GPU cannot change; asking the driver on every op costs more than the op
+
+
 def cuda_enabled() -> bool:
     """True when the hand-written kernels should be used (a CUDA device is present and not disabled)."""
-    return torch.cuda.is_available() and os.environ.get('MCB200_DISABLE_CUDA_KERNELS', '0') != '1'
+    global _device_present
+    if _device_present is None:
+        _device_present = torch.cuda.is_available()
+    return _device_present and os.environ.get('MCB200_DISABLE_CUDA_KERNELS', '0') != '1'
 
 
 def lib() -> ctypes.CDLL:
@@ -59,7 +65,8 @@ def available() -> bool:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the current stream's handle without building a Stream object around it
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def ptr(t) -> ctypes.c_void_p:
