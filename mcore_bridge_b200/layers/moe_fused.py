@@ -466,7 +466,7 @@ def _sum_slots(b: ExchangeBuffers, par: int, sent: torch.Tensor) -> torch.Tensor
 
 def pull_gemm_supported(experts, config, El: int, H: int) -> bool:
     """The fused dispatch + expert GEMM applies to plain stacked bf16 expert weights without biases, probabilities
-    applied after the first layer and at most 64 local experts."""
+    applied after the first layer and at most 256 local experts."""
     from .moe import GroupedLinear, GroupedMLP
     if os.environ.get('MCB200_MOE_FUSED_GEMM', '1') == '0':
         return False
@@ -476,7 +476,7 @@ def pull_gemm_supported(experts, config, El: int, H: int) -> bool:
         if type(lin) is not GroupedLinear or lin.bias is not None or lin.weight.dtype != torch.bfloat16:
             return False
     f = experts.linear_fc2.weight.shape[2]
-    return El <= 64 and H % 64 == 0 and f % 64 == 0 and experts.linear_fc1.weight.shape[1] % 8 == 0
+    return El <= 256 and H % 64 == 0 and f % 64 == 0 and experts.linear_fc1.weight.shape[1] % 8 == 0
 
 
 class _DispatchFc1Fn(torch.autograd.Function):
