@@ -32,9 +32,9 @@ cudaError_t launch_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUte
   return launch<BN, true, false>(ta, tb, p, grid, s);
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int EPI = EPI_NONE>
 cudaError_t launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
-  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN>;
+  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, EPI>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
@@ -158,16 +158,24 @@ int mcb_gemm_ce_bf16(const void* A, long long lda, const void* B, long long ldb,
     return -2;
   constexpr int BN = 256;
   const int sms = device_sm_count();
+  // same tile width either way, so `part` has the same layout
+  const bool pair = use_pair(M, N, K, GEMM_DENSE, sms);
   CUtensorMap ta, tb;
   int rc = make_tmap_2d_bf16(&ta, A, K, M, lda, GEMM_BK, GEMM_BM);
   if (rc) return rc;
-  rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, GEMM_BK, BN);
+  rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, GEMM_BK, pair ? PAIR_HALF_N : BN);
   if (rc) return rc;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.alpha = 1.f; p.mode = GEMM_DENSE;
   p.epilogue = grad ? EPI_CE_GRAD : EPI_CE_STATS;
   p.ce_labels = labels; p.ce_col0 = col0; p.ce_part = part; p.ce_tgt = tgt; p.ce_lse = lse; p.ce_g = g;
   p.status = status;
+  if (pair) {
+    const long long ptiles = (long long)((M + PAIR_BM - 1) / PAIR_BM) * ((N + PAIR_BN - 1) / PAIR_BN);
+    const int grid = 2 * (int)(ptiles < sms / 2 ? ptiles : sms / 2);
+    return (int)(grad ? launch_pair<false, false, EPI_CE_GRAD>(ta, tb, p, grid, stream)
+                      : launch_pair<false, false, EPI_CE_STATS>(ta, tb, p, grid, stream));
+  }
   const long long tiles = (long long)((M + GEMM_BM - 1) / GEMM_BM) * ((N + BN - 1) / BN);
   const int grid = (int)(tiles < sms ? tiles : sms);
   static bool cfg[2] = {false, false};

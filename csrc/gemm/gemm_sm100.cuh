@@ -108,6 +108,74 @@ __device__ __forceinline__ void epilogue_accumulate_fp32(uint32_t tmem_row, floa
   }
 }
 
+// Epilogue of the fused language-model head for one row of a BN-column tile (one thread owns the row): running soft-max
+// statistics of the row's logits and the label's logit (EPI_CE_STATS), or the logits' gradient as bf16 (EPI_CE_GRAD).
+template <int BN, int EPI>
+__device__ __forceinline__ void epilogue_ce(const GemmParams& p, uint32_t tmem_row, int row, bool row_ok, int n0, int tiles_n) {
+  constexpr float LOG2E = 1.4426950408889634f;
+  const bool vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
+  const int label_col = row_ok ? (int)(p.ce_labels[row] - p.ce_col0) - n0 : -1;   // column inside this tile
+  float run_m = -INFINITY, run_s = 0.f, tgt = 0.f;
+  const float lse2 = (EPI == EPI_CE_GRAD && row_ok) ? p.ce_lse[row] * LOG2E : 0.f;
+  const float g = (EPI == EPI_CE_GRAD && row_ok) ? p.ce_g[row] : 0.f;
+#pragma unroll 1
+  for (int cc = 0; cc < BN; cc += 32) {
+    if (n0 + cc >= p.N) break;
+    uint32_t r[32];
+    tmem_ld_32x32(tmem_row + cc, r);
+    tmem_ld_wait();
+    if (!row_ok) continue;
+    const int valid = min(32, p.N - (n0 + cc));
+    if constexpr (EPI == EPI_CE_STATS) {
+      float cm = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < valid) cm = fmaxf(cm, __uint_as_float(r[j]) * p.alpha);
+      const float nm = fmaxf(run_m, cm);
+      float add = 0.f;
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < valid) add += exp2f((__uint_as_float(r[j]) * p.alpha - nm) * LOG2E);
+      run_s = run_s * exp2f((run_m - nm) * LOG2E) + add;
+      run_m = nm;
+      const int lj = label_col - cc;
+      if (lj >= 0 && lj < valid) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (j == lj) tgt = __uint_as_float(r[j]) * p.alpha;
+      }
+    } else {
+      const int lj = label_col - cc;
+      float v[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        v[j] = (exp2f(__uint_as_float(r[j]) * p.alpha * LOG2E - lse2) - (j == lj ? 1.f : 0.f)) * g;
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)row * p.ldc + n0 + cc;
+      if (vec_ok && valid == 32) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          uint4 o;
+          o.x = pack_bf16x2(v[j], v[j + 1]);
+          o.y = pack_bf16x2(v[j + 2], v[j + 3]);
+          o.z = pack_bf16x2(v[j + 4], v[j + 5]);
+          o.w = pack_bf16x2(v[j + 6], v[j + 7]);
+          *reinterpret_cast<uint4*>(dst + j) = o;
+        }
+      } else {
+        for (int j = 0; j < valid; ++j) dst[j] = __float2bfloat16(v[j]);
+      }
+    }
+  }
+  if constexpr (EPI == EPI_CE_STATS) {
+    if (row_ok) {
+      float* part = p.ce_part + ((long long)row * tiles_n + n0 / BN) * 2;
+      part[0] = run_m;
+      part[1] = run_s;
+      if (label_col >= 0 && label_col < BN && n0 + label_col < p.N) p.ce_tgt[row] = tgt;
+    }
+  }
+}
+
 struct TileCoord {
   int m0, n0;        // output tile origin (row within C / group output)
   int k_begin, k_end;  // contraction range in elements
@@ -335,68 +403,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                  : nullptr;
       const bool vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
       if constexpr (EPI == EPI_CE_STATS || EPI == EPI_CE_GRAD) {
-        // fused language-model head: one thread owns one row of the tile
-        constexpr float LOG2E = 1.4426950408889634f;
-        const int label_col = row_ok ? (int)(p.ce_labels[row] - p.ce_col0) - c.n0 : -1;   // column inside this tile
-        float run_m = -INFINITY, run_s = 0.f, tgt = 0.f;
-        const float lse2 = (EPI == EPI_CE_GRAD && row_ok) ? p.ce_lse[row] * LOG2E : 0.f;
-        const float g = (EPI == EPI_CE_GRAD && row_ok) ? p.ce_g[row] : 0.f;
-#pragma unroll 1
-        for (int cc = 0; cc < BN; cc += 32) {
-          if (c.n0 + cc >= p.N) break;
-          uint32_t r[32];
-          tmem_ld_32x32(tmem_base + (uint32_t(q * 32) << 16) + acc * BN + cc, r);
-          tmem_ld_wait();
-          if (!row_ok) continue;
-          const int valid = min(32, p.N - (c.n0 + cc));
-          if constexpr (EPI == EPI_CE_STATS) {
-            float cm = -INFINITY;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (j < valid) cm = fmaxf(cm, __uint_as_float(r[j]) * p.alpha);
-            const float nm = fmaxf(run_m, cm);
-            float add = 0.f;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (j < valid) add += exp2f((__uint_as_float(r[j]) * p.alpha - nm) * LOG2E);
-            run_s = run_s * exp2f((run_m - nm) * LOG2E) + add;
-            run_m = nm;
-            const int lj = label_col - cc;
-            if (lj >= 0 && lj < valid) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (j == lj) tgt = __uint_as_float(r[j]) * p.alpha;
-            }
-          } else {
-            const int lj = label_col - cc;
-            float v[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              v[j] = (exp2f(__uint_as_float(r[j]) * p.alpha * LOG2E - lse2) - (j == lj ? 1.f : 0.f)) * g;
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)row * p.ldc + c.n0 + cc;
-            if (vec_ok && valid == 32) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint4 o;
-                o.x = pack_bf16x2(v[j], v[j + 1]);
-                o.y = pack_bf16x2(v[j + 2], v[j + 3]);
-                o.z = pack_bf16x2(v[j + 4], v[j + 5]);
-                o.w = pack_bf16x2(v[j + 6], v[j + 7]);
-                *reinterpret_cast<uint4*>(dst + j) = o;
-              }
-            } else {
-              for (int j = 0; j < valid; ++j) dst[j] = __float2bfloat16(v[j]);
-            }
-          }
-        }
-        if constexpr (EPI == EPI_CE_STATS) {
-          if (row_ok) {
-            float* part = p.ce_part + ((long long)row * sched.tiles_n + c.n0 / BN) * 2;
-            part[0] = run_m;
-            part[1] = run_s;
-            if (label_col >= 0 && label_col < BN && c.n0 + label_col < p.N) p.ce_tgt[row] = tgt;
-          }
-        }
+        epilogue_ce<BN, EPI>(p, tmem_base + (uint32_t(q * 32) << 16) + acc * BN, row, row_ok, c.n0, sched.tiles_n);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

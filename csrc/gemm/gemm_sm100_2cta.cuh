@@ -28,7 +28,7 @@ constexpr int PAIR_B_BYTES = PAIR_HALF_N * GEMM_BK * 2;   // 16 KiB
 constexpr int PAIR_STAGE_BYTES = PAIR_A_BYTES + PAIR_B_BYTES;
 constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 1024;
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int EPI = EPI_NONE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const GemmParams p) {
@@ -189,6 +189,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const int row = tm * PAIR_BM + (int)cta * GEMM_BM + q * 32 + lane;
       const bool row_ok = row < p.M;
       const int n0 = tn * PAIR_BN;
+      if constexpr (EPI == EPI_CE_STATS || EPI == EPI_CE_GRAD) {
+        epilogue_ce<PAIR_BN, EPI>(p, tmem_base + (uint32_t(q * 32) << 16) + acc * PAIR_BN, row, row_ok, n0, tiles_n);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc ? tempty_leader1 : tempty_leader0);
+        continue;
+      }
       const long long cbase = (long long)row * p.ldc;
       const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
       const bool vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);

@@ -231,10 +231,14 @@ class _FusedLinearCE(torch.autograd.Function):
         mg = getattr(weight, 'main_grad', None)
         dw = None
         need_dw = ctx.needs_input_grad[1]
-        if need_dw and mg is None:
-            dw = torch.zeros(weight.shape, dtype=torch.float32, device=weight.device)
         ddt = h2.dtype if h2.dtype == torch.bfloat16 else torch.float32
         fused = _head_kernel_ok(h2, weight)
+        # without `main_grad` the chunks' products are summed in fp32 and rounded once; a single chunk needs no such
+        # buffer (at 151936 x 4096 it costs 2.5 GB of zero fill, accumulation and conversion), its GEMM rounds itself
+        one_chunk = 0 < T <= chunk and mg is None and weight.dtype in (torch.bfloat16, torch.float32)
+        if need_dw and mg is None and not one_chunk:
+            alloc = torch.empty if T > 0 else torch.zeros
+            dw = alloc(weight.shape, dtype=torch.float32, device=weight.device)
         for s0 in range(0, T, chunk):
             s1 = min(T, s0 + chunk)
             if fused:
@@ -244,8 +248,10 @@ class _FusedLinearCE(torch.autograd.Function):
                 d = _dlogits(logits, lab[s0:s1], vstart, lse[s0:s1], g[s0:s1], ddt)
                 del logits
             gemm.mm_nn(d, weight, out=dh[s0:s1])
-            if need_dw:
-                gemm.mm_tn(d, h2[s0:s1], out=mg if mg is not None else dw, accumulate=True)
+            if need_dw and one_chunk:
+                dw = gemm.mm_tn(d, h2, out_dtype=weight.dtype)
+            elif need_dw:
+                gemm.mm_tn(d, h2[s0:s1], out=mg if mg is not None else dw, accumulate=mg is not None or s0 > 0)
             del d
         # dh is this vocab shard's partial gradient: the caller's input mapping (copy-to-region or
         # sequence-parallel gather) sums it over the tensor-parallel group in its own backward.
