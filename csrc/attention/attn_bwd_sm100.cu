@@ -439,13 +439,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   uint64_t* do_full = bars + 5;        // 2
   uint64_t* do_empty = bars + 7;       // 2
   uint64_t* s_full = bars + 9;         // 1
-  uint64_t* p_full = bars + 10;        // 1
-  uint64_t* dp_full = bars + 11;       // 1
-  uint64_t* ds_full = bars + 12;       // 1
-  uint64_t* out_full = bars + 13;      // 1
-  uint64_t* col_full = bars + 14;      // 2
-  uint64_t* col_empty = bars + 16;     // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+  uint64_t* p_full = bars + 10;        // 2: the first and the second 32 queries of each 64-query half
+  uint64_t* dp_full = bars + 12;       // 1
+  uint64_t* ds_full = bars + 13;       // 2
+  uint64_t* out_full = bars + 15;      // 1
+  uint64_t* col_full = bars + 16;      // 2
+  uint64_t* col_empty = bars + 18;     // 2
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* i_end_slot = reinterpret_cast<int*>(tmem_slot + 2);
 
@@ -465,11 +465,11 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       mbar_init(smem_u32(&do_empty[i]), 1);
       mbar_init(smem_u32(&col_full[i]), 32);
       mbar_init(smem_u32(&col_empty[i]), 8);
+      mbar_init(smem_u32(&p_full[i]), 8);
+      mbar_init(smem_u32(&ds_full[i]), 8);
     }
     mbar_init(smem_u32(s_full), 1);
-    mbar_init(smem_u32(p_full), 8);
     mbar_init(smem_u32(dp_full), 1);
-    mbar_init(smem_u32(ds_full), 8);
     mbar_init(smem_u32(out_full), 1);
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -568,20 +568,24 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         for (int kk = 0; kk < D / 16; ++kk)
           umma_f16(tmem + COL_DP, kdesc(sv, kk, TM), kdesc(sdo, kk, TM), idesc_s, kk ? 1u : 0u);
         umma_commit(smem_u32(dp_full));
-        if (!mbar_wait(smem_u32(p_full), it & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-        tc_fence_after();
+        // P, dS: 32 packed columns at the start of each 64-column half; part u of them is ready first in both halves
+        auto product = [&](uint32_t col_d, uint32_t col_a, uint32_t sb, uint64_t* full) -> bool {
+          for (int u = 0; u < 2; ++u) {
+            if (!mbar_wait(smem_u32(&full[u]), it & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
+            tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < TM / 16; ++kk)     // P, dS: 32 packed columns at the start of each 64-column half
-          umma_f16_ts(tmem + COL_DV, tmem + COL_S + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sdo, kk, TM), idesc_o,
-                      (it | kk) ? 1u : 0u);
+            for (int v = 0; v < 4; ++v) {
+              const int kk = (v >> 1) * 4 + u * 2 + (v & 1);
+              umma_f16_ts(tmem + col_d, tmem + col_a + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sb, kk, TM), idesc_o,
+                          (it | u | v) ? 1u : 0u);
+            }
+          }
+          return true;
+        };
+        if (!product(COL_DV, COL_S, sdo, p_full)) { ok = false; break; }
         umma_commit(smem_u32(&do_empty[st]));
         if (it + 1 < iters && !issue_s(it + 1)) { ok = false; break; }
-        if (!mbar_wait(smem_u32(ds_full), it & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < TM / 16; ++kk)
-          umma_f16_ts(tmem + COL_DK, tmem + COL_DP + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sq, kk, TM), idesc_o,
-                      (it | kk) ? 1u : 0u);
+        if (!product(COL_DK, COL_DP, sq, ds_full)) { ok = false; break; }
         umma_commit(smem_u32(&q_empty[st]));
       }
       if (ok) umma_commit(smem_u32(out_full));
@@ -666,57 +670,62 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             seen[e >> 5] |= (row_ok && aa[u] <= n && n <= zz[u]) ? 1u << ((e + u) & 31) : 0u;
         }
       }
-      uint32_t pk[HALF / 2];
 #pragma unroll
-      for (int e = 0; e < HALF; e += 4) {
-        const float4 l4 = *reinterpret_cast<const float4*>(c_lse + e);
-        const float2 x = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1])), cc, f32x2(l4.x, l4.y)));
-        const float2 y = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e + 2]), __uint_as_float(pr[e + 3])), cc, f32x2(l4.z, l4.w)));
-        float v[4] = {ex2_ftz(x.x), ex2_ftz(x.y), ex2_ftz(y.x), ex2_ftz(y.y)};
-        if (!full) {
+      for (int u2 = 0; u2 < 2; ++u2) {
+        uint32_t pk[16];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) v[u] = (seen[e >> 5] >> ((e + u) & 31)) & 1u ? v[u] : 0.f;
+        for (int e = u2 * 32; e < u2 * 32 + 32; e += 4) {
+          const float4 l4 = *reinterpret_cast<const float4*>(c_lse + e);
+          const float2 x = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1])), cc, f32x2(l4.x, l4.y)));
+          const float2 y = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e + 2]), __uint_as_float(pr[e + 3])), cc, f32x2(l4.z, l4.w)));
+          float v[4] = {ex2_ftz(x.x), ex2_ftz(x.y), ex2_ftz(y.x), ex2_ftz(y.y)};
+          if (!full) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = (seen[e >> 5] >> ((e + u) & 31)) & 1u ? v[u] : 0.f;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) pr[e + u] = __float_as_uint(v[u]);
+          pk[(e & 31) >> 1] = pack_bf16x2(v[0], v[1]);
+          pk[((e & 31) >> 1) + 1] = pack_bf16x2(v[2], v[3]);
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) pr[e + u] = __float_as_uint(v[u]);
-        pk[e >> 1] = pack_bf16x2(v[0], v[1]);
-        pk[(e >> 1) + 1] = pack_bf16x2(v[2], v[3]);
+        tmem_st_32x16(ts + u2 * 16, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&p_full[u2]));
       }
-      tmem_st_32x32(ts, pk);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(p_full));
       if (!mbar_wait(smem_u32(dp_full), it & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       uint32_t dp[HALF];
       tmem_ld_32x32_x64(td, dp);
       tmem_ld_wait();
 #pragma unroll
-      for (int e = 0; e < HALF; e += 4) {
-        const float4 d4 = *reinterpret_cast<const float4*>(c_delta + e);
-        float2 x = f32x2_split(mul_f32x2(add_f32x2(f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1])), f32x2(d4.x, d4.y)),
-                                         f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1]))));
-        float2 y = f32x2_split(mul_f32x2(add_f32x2(f32x2(__uint_as_float(dp[e + 2]), __uint_as_float(dp[e + 3])), f32x2(d4.z, d4.w)),
-                                         f32x2(__uint_as_float(pr[e + 2]), __uint_as_float(pr[e + 3]))));
-        if (!full) {                              // a masked pair contributes zero whatever its dP is
-          const uint32_t m = seen[e >> 5] >> (e & 31);
-          x.x = m & 1u ? x.x : 0.f;
-          x.y = m & 2u ? x.y : 0.f;
-          y.x = m & 4u ? y.x : 0.f;
-          y.y = m & 8u ? y.y : 0.f;
+      for (int u2 = 0; u2 < 2; ++u2) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int e = u2 * 32; e < u2 * 32 + 32; e += 4) {
+          const float4 d4 = *reinterpret_cast<const float4*>(c_delta + e);
+          float2 x = f32x2_split(mul_f32x2(add_f32x2(f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1])), f32x2(d4.x, d4.y)),
+                                           f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1]))));
+          float2 y = f32x2_split(mul_f32x2(add_f32x2(f32x2(__uint_as_float(dp[e + 2]), __uint_as_float(dp[e + 3])), f32x2(d4.z, d4.w)),
+                                           f32x2(__uint_as_float(pr[e + 2]), __uint_as_float(pr[e + 3]))));
+          if (!full) {                              // a masked pair contributes zero whatever its dP is
+            const uint32_t m = seen[e >> 5] >> (e & 31);
+            x.x = m & 1u ? x.x : 0.f;
+            x.y = m & 2u ? x.y : 0.f;
+            y.x = m & 4u ? y.x : 0.f;
+            y.y = m & 8u ? y.y : 0.f;
+          }
+          pk[(e & 31) >> 1] = pack_bf16x2(x.x, x.y);
+          pk[((e & 31) >> 1) + 1] = pack_bf16x2(y.x, y.y);
         }
-        pk[e >> 1] = pack_bf16x2(x.x, x.y);
-        pk[(e >> 1) + 1] = pack_bf16x2(y.x, y.y);
+        tmem_st_32x16(td + u2 * 16, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ds_full[u2]));
       }
-      tmem_st_32x32(td, pk);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(smem_u32(ds_full));
-        mbar_arrive(smem_u32(&col_empty[b]));
-      }
+      if (lane == 0) mbar_arrive(smem_u32(&col_empty[b]));
     }
     // group 0 writes dV, group 1 writes dK
     const long long row_off = ((long long)n * p.nkv + kvh) * D;

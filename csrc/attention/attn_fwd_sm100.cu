@@ -19,7 +19,8 @@
 //
 // Bound: per 128 x 128 block the two products take 1024 tensor cycles and the 16384 exponentials 1024 MUFU cycles of an
 // SM, so both pipes are the floor; the two tiles in flight overlap them.  Measured, 32 query / 8 kv heads of 128, causal:
-// 16384 tokens 2.02 ms = 1090 TFLOP/s; the form before it (maxima in a first pass over Q K^T, one tile per CTA, P through
+// 16384 tokens 2.0 ms = 1090 TFLOP/s (tensor pipe 43 %, MUFU 43 %: the chain load - maximum - exponentials - product - scores
+// of a tile sets the pace, which is why P is handed over in halves); the form before it (maxima in a first pass over Q K^T, one tile per CTA, P through
 // shared memory) took 3.35 ms.
 #include "../common/host_utils.cuh"
 #include "../common/ptx.cuh"
@@ -92,9 +93,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint64_t* v_full = bars + 6;        // 2
   uint64_t* v_empty = bars + 8;       // 2
   uint64_t* s_full = bars + 10;       // 2, per tile
-  uint64_t* p_full = bars + 12;       // 2, per tile
-  uint64_t* o_done = bars + 14;       // 2, per tile: a P V product has completed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* p_full = bars + 12;       // 2 x 2: halves of P (64 keys each), per tile
+  uint64_t* o_done = bars + 16;       // 2, per tile: a P V product has completed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -128,7 +129,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_init(smem_u32(&v_full[i]), 1);
       mbar_init(smem_u32(&v_empty[i]), 1);
       mbar_init(smem_u32(&s_full[i]), 1);
-      mbar_init(smem_u32(&p_full[i]), 4);
+      mbar_init(smem_u32(&p_full[2 * i]), 4);
+      mbar_init(smem_u32(&p_full[2 * i + 1]), 4);
       mbar_init(smem_u32(&o_done[i]), 1);
     }
     fence_barrier_init();
@@ -218,13 +220,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               if (!mbar_wait(smem_u32(&v_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
               v_seen = true;
             }
-            if (!mbar_wait(smem_u32(&p_full[t]), n & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-            tc_fence_after();
             const uint32_t sv = smem_u32(smem + L::OFF_V + st * L::TILE);
+            for (int h = 0; h < 2; ++h) {        // the second half of the exponentials runs under the first half's product
+              if (!mbar_wait(smem_u32(&p_full[2 * t + h]), n & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+              tc_fence_after();
 #pragma unroll
-            for (int kk = 0; kk < BNK / 16; ++kk)
-              umma_f16_ts(tmem + COL_O + t * 128, tmem + COL_S + t * BNK + kk * 8,
-                          make_smem_desc_sw128(sv + kk * 2048, BM * 128, 1024), idesc_o, (n | kk) ? 1u : 0u);
+              for (int k4 = 0; k4 < BNK / 32; ++k4) {
+                const int kk = h * (BNK / 32) + k4;
+                umma_f16_ts(tmem + COL_O + t * 128, tmem + COL_S + t * BNK + kk * 8,
+                            make_smem_desc_sw128(sv + kk * 2048, BM * 128, 1024), idesc_o, (n | kk) ? 1u : 0u);
+              }
+            }
+            if (!ok) break;
             umma_commit(smem_u32(&o_done[t]));
           }
           if (j + 1 >= b0[t] && j + 1 < b1[t]) {
@@ -336,11 +343,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           pk[e >> 1] = pack_bf16x2(e0, e1);
         }
         tmem_st_32x32(ts + 16 * c, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&p_full[2 * t + (c >> 1)]));
       }
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&p_full[t]));
     }
     const float2 sp = f32x2_split(sum2);
     float sum = sp.x + sp.y;
