@@ -15,11 +15,11 @@ cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParam
   auto kern = gemm_bf16_sm100_kernel<BN, A_MN, B_MN>;
   static bool configured = false;  // per template instantiation
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (GemmSmem<BN>::TOTAL + EPI_STAGE_BYTES));
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(ta, tb, p);
+  kern<<<grid, GEMM_THREADS, (GemmSmem<BN>::TOTAL + EPI_STAGE_BYTES), stream>>>(ta, tb, p);
   return cudaGetLastError();
 }
 
@@ -183,19 +183,19 @@ int mcb_gemm_ce_bf16(const void* A, long long lda, const void* B, long long ldb,
   if (grad) {
     auto kern = gemm_bf16_sm100_kernel<BN, false, false, EPI_CE_GRAD>;
     if (!cfg[1]) {
-      if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL)) != cudaSuccess)
+      if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (GemmSmem<BN>::TOTAL + EPI_STAGE_BYTES))) != cudaSuccess)
         return (int)e;
       cfg[1] = true;
     }
-    kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(ta, tb, p);
+    kern<<<grid, GEMM_THREADS, (GemmSmem<BN>::TOTAL + EPI_STAGE_BYTES), stream>>>(ta, tb, p);
   } else {
     auto kern = gemm_bf16_sm100_kernel<BN, false, false, EPI_CE_STATS>;
     if (!cfg[0]) {
-      if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL)) != cudaSuccess)
+      if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (GemmSmem<BN>::TOTAL + EPI_STAGE_BYTES))) != cudaSuccess)
         return (int)e;
       cfg[0] = true;
     }
-    kern<<<grid, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(ta, tb, p);
+    kern<<<grid, GEMM_THREADS, (GemmSmem<BN>::TOTAL + EPI_STAGE_BYTES), stream>>>(ta, tb, p);
   }
   return (int)cudaGetLastError();
 }

@@ -108,6 +108,54 @@ __device__ __forceinline__ void epilogue_accumulate_fp32(uint32_t tmem_row, floa
   }
 }
 
+// Per-warp staging area of the bf16 epilogue: 32 rows x 64 columns.
+constexpr int EPI_STAGE_WARP = 32 * 128;
+constexpr int EPI_STAGE_BYTES = 4 * EPI_STAGE_WARP;
+
+// C[row0 .. row0 + 32, n0 .. n0 + BN) = alpha * accumulators (+ bias) as bf16, for C rows on 16-byte boundaries and N a
+// multiple of 8.  A thread holds one row; stored from there every 16-byte store instruction of a warp touches 32 rows, i.e.
+// 32 memory transactions for 512 bytes.  Through shared memory (16-byte chunks swizzled by the row) eight lanes write 128
+// contiguous bytes of a row, four rows per instruction: an eighth of the transactions.  Short contractions (expert weight
+// gradients: 4 to 6 k-blocks per tile) were bound by the former: 128 experts x (1536 + 768) x 2048, 256 rows each,
+// 757 -> 466 us.
+template <int BN>
+__device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* stage, __nv_bfloat16* C, long long ldc, int row0,
+                                                    int m_limit, int n0, int N, float alpha, const __nv_bfloat16* bias) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int cc = 0; cc < BN; cc += 64) {
+    if (n0 + cc >= N) break;
+    uint32_t r[64];
+    tmem_ld_32x32_x64(tmem_row + cc, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]) * alpha;
+      if (bias && n0 + cc + 8 * j < N) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] += __bfloat162float(bias[n0 + cc + 8 * j + e]);
+      }
+      uint4 o;
+      o.x = pack_bf16x2(v[0], v[1]);
+      o.y = pack_bf16x2(v[2], v[3]);
+      o.z = pack_bf16x2(v[4], v[5]);
+      o.w = pack_bf16x2(v[6], v[7]);
+      *reinterpret_cast<uint4*>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) = o;
+    }
+    __syncwarp();
+    const int j = lane & 7, col = n0 + cc + 8 * j;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int rr = it * 4 + (lane >> 3);
+      const uint4 o = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((j ^ (rr & 7)) << 4));
+      if (row0 + rr < m_limit && col < N) *reinterpret_cast<uint4*>(C + (long long)(row0 + rr) * ldc + col) = o;
+    }
+    __syncwarp();
+  }
+}
+
 // Epilogue of the fused language-model head for one row of a BN-column tile (one thread owns the row): running soft-max
 // statistics of the row's logits and the label's logit (EPI_CE_STATS), or the logits' gradient as bf16 (EPI_CE_GRAD).
 template <int BN, int EPI>
@@ -414,6 +462,18 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       if (p.accumulate == 2 && p.c_fp32 && vec_ok && has_acc && !bias && cols_valid % 32 == 0) {
         epilogue_accumulate_fp32<BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * BN,
                                      reinterpret_cast<float*>(p.C) + cbase + c.n0, cols_valid / 32, row_ok, p.alpha);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
+        ++lt;
+        continue;
+      }
+      if (!p.c_fp32 && !p.accumulate && vec_ok && has_acc && p.N % 8 == 0) {
+        const long long gbase = p.mode == GEMM_GROUPED_K ? (long long)c.group * p.c_group_stride : 0ll;
+        epilogue_store_bf16<BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * BN,
+                                smem + STAGES * L::STAGE_BYTES + L::BAR_BYTES + q * EPI_STAGE_WARP,
+                                reinterpret_cast<__nv_bfloat16*>(p.C) + gbase, p.ldc, c.m0 + q * 32, c.m_limit, c.n0, p.N,
+                                p.alpha, bias);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

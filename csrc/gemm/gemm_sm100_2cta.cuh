@@ -26,7 +26,7 @@ constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_A_BYTES = GEMM_BM * GEMM_BK * 2;       // 16 KiB
 constexpr int PAIR_B_BYTES = PAIR_HALF_N * GEMM_BK * 2;   // 16 KiB
 constexpr int PAIR_STAGE_BYTES = PAIR_A_BYTES + PAIR_B_BYTES;
-constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 1024;
+constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 1024 + EPI_STAGE_BYTES;
 
 template <bool A_MN, bool B_MN, int EPI = EPI_NONE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
@@ -199,6 +199,15 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const long long cbase = (long long)row * p.ldc;
       const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
       const bool vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
+      if (!p.c_fp32 && !p.accumulate && vec_ok && p.N % 8 == 0) {
+        epilogue_store_bf16<PAIR_BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * PAIR_BN,
+                                     smem + STAGES * PAIR_STAGE_BYTES + 1024 + q * EPI_STAGE_WARP,
+                                     reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, row - lane, p.M, n0, p.N, p.alpha, bias);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc ? tempty_leader1 : tempty_leader0);
+        continue;
+      }
 #pragma unroll 1
       for (int cc = 0; cc < PAIR_BN; cc += 32) {
         if (n0 + cc >= p.N) break;  // whole chunk out of range (uniform across the warp)
