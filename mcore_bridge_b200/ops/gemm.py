@@ -27,15 +27,28 @@ def _use_cuda(*ts) -> bool:
     return all(t is None or t.is_cuda for t in ts) and ts[0].dtype == torch.bfloat16 and _lib.available()
 
 
+_entry = None
+
+
+def _gemm_entry():
+    """The C entry point with its argument types declared once: plain integers then pass through, where wrapping each of
+    the 28 arguments of every call was a large part of a small GEMM's time on the host."""
+    global _entry
+    if _entry is None:
+        f = _lib.lib().mcb_gemm_bf16
+        p, ll, i, fl = ctypes.c_void_p, _c_ll, _c_int, ctypes.c_float
+        f.argtypes = [p, ll, ll, ll, i, p, ll, ll, ll, i, p, ll, ll, i, i, i, i, i, fl, p, i, i, p, i, p, i, i, p]
+        _entry = f
+    return _entry
+
+
 def _launch(a, a_inner, a_outer, lda, a_mn, b, b_inner, b_outer, ldb, b_mn, c, ldc, c_group_stride, M, N, K, alpha,
             bias, accumulate, mode=DENSE, num_groups=0, offsets=None, b_group_rows=0, max_sms=0, force_bn=0):
-    rc = _lib.lib().mcb_gemm_bf16(
-        _lib.ptr(a), _c_ll(a_inner), _c_ll(a_outer), _c_ll(lda), _c_int(int(a_mn)),
-        _lib.ptr(b), _c_ll(b_inner), _c_ll(b_outer), _c_ll(ldb), _c_int(int(b_mn)),
-        _lib.ptr(c), _c_ll(ldc), _c_ll(c_group_stride), _c_int(int(c.dtype == torch.float32)), _c_int(int(accumulate)),
-        _c_int(M), _c_int(N), _c_int(K), ctypes.c_float(alpha), _lib.ptr(bias),
-        _c_int(mode), _c_int(num_groups), _lib.ptr(offsets), _c_int(b_group_rows),
-        _lib.ptr(_lib.status_word(a.device)), _c_int(max_sms), _c_int(force_bn), _lib.stream_ptr())
+    rc = _gemm_entry()(
+        a.data_ptr(), a_inner, a_outer, lda, int(a_mn), b.data_ptr(), b_inner, b_outer, ldb, int(b_mn),
+        c.data_ptr(), ldc, c_group_stride, int(c.dtype == torch.float32), int(accumulate), M, N, K, alpha,
+        None if bias is None else bias.data_ptr(), mode, num_groups, None if offsets is None else offsets.data_ptr(),
+        b_group_rows, _lib.status_word(a.device).data_ptr(), max_sms, force_bn, _lib.stream_ptr())
     _lib.check_rc(rc, 'mcb_gemm_bf16')
 
 
