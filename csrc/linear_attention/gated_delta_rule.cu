@@ -21,7 +21,7 @@
 // In the scans a warp owns 16 columns of v and keeps S^T (16 x d) in its accumulators: the accumulators of every product
 // are the first operand of the next one, so the warps of a CTA share the loaded tiles and never exchange values.  Bound:
 // the chain of ~500 MMAs per chunk; the next chunk's tiles are copied meanwhile.  Measured, 4096 tokens in three sequences,
-// 32 heads of 128: forward 0.27 ms (prep 0.07, scan 0.19), backward 0.92 ms (prep, scan, scan_bwd 0.26, grad 0.39); the
+// 32 heads of 128: forward 0.22 ms (prep 0.07, scan 0.15), backward 0.81 ms (prep, scan, scan_bwd 0.20, grad 0.39); the
 // batched torch evaluation of the rule was most of a 29.5 ms block.
 #include "../common/host_utils.cuh"
 #include "warp_mma.cuh"
@@ -208,7 +208,25 @@ template <int D>
 __device__ __forceinline__ ScanPos scan_pos(const GdrParams& p, int* slot) {
   constexpr int SL = D / 64;
   ScanPos s;
-  const int seq = blockIdx.x / (p.H * SL), rest = blockIdx.x % (p.H * SL);
+  int seq = blockIdx.x / (p.H * SL);
+  const int rest = blockIdx.x % (p.H * SL);
+  // Few sequences: the longest ones are walked first, or the last to start would set the time (sequences of 1463, 585 and
+  // 2048 tokens, 64 walks each: 194 -> 151 us).  With more than 32 of them one walk is a small share of the launch and the
+  // order of the batch does.
+  if (p.n_seq <= 32) {
+    if (threadIdx.x < 32) {
+      const int i = threadIdx.x, len = i < p.n_seq ? p.cu[i + 1] - p.cu[i] : -1;
+      int rank = 0;
+      for (int j = 0; j < p.n_seq; ++j) {
+        const int other = __shfl_sync(0xffffffffu, len, j);
+        rank += other > len || (other == len && j < i);
+      }
+      if (i < p.n_seq && rank == seq) *slot = i;
+    }
+    __syncthreads();
+    seq = *slot;
+    __syncthreads();
+  }
   s.h = rest / SL;
   s.col0 = (rest % SL) * 64;
   s.t0 = p.cu[seq];

@@ -70,84 +70,86 @@ __device__ __forceinline__ void stn(__nv_bfloat16* p, const float (&f)[N]) {
   for (int i = 0; i < N; i += 2) *reinterpret_cast<uint32_t*>(p + i) = pack_bf16x2(f[i], f[i + 1]);
 }
 
-// S = 2 + R slices of d channels (q, k, R times v); a lane owns PER = d / 32 consecutive channels of each
+// The projection row of a group has S = 2 + R convolved slices of d channels (q, k, R times v), then z and the gates.  A
+// block's z index names one slice, or (index S) z and the gates; a lane owns PER = d / 32 consecutive channels.
 template <int D, int R>
 __global__ void __launch_bounds__(WARPS * 32)
 gdn_inputs_fwd_kernel(const InParams p) {
   constexpr int PER = D / 32, S = 2 + R;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = blockIdx.y, s = blockIdx.z;
   const int t0 = (blockIdx.x * WARPS + warp) * TOK_F, t1 = min(t0 + TOK_F, p.T);
   if (t0 >= p.T) return;
-  const __nv_bfloat16* src = p.proj + (long long)grp * (2 * D + 2 * R * D + 2 * R) + lane * PER;
-  float w[S][PER][KW];
+  const __nv_bfloat16* src = p.proj + (long long)grp * (2 * D + 2 * R * D + 2 * R) + s * D + lane * PER;
+  auto out_row = [&](int t) { return ((long long)t * p.G + grp) * R * D + lane * PER; };
+  if (s == S) {                                  // z and the gates
+    const int hv = lane < R ? grp * R + lane : 0;
+    const float neg_a = lane < R ? -exp_full(__bfloat162float(p.A_log[hv])) : 0.f;
+    const float dtb = lane < R ? __bfloat162float(p.dt[hv]) : 0.f;
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) {
 #pragma unroll
-  for (int s = 0; s < S; ++s)
+      for (int r = 0; r < R; ++r) {
+        float zz[PER];
+        ldn<PER>(src + t * p.ld + r * D, zz);
+        stn<PER>(p.z + out_row(t) + r * D, zz);
+      }
+      if (lane < R) {
+        const __nv_bfloat16* ba = src - lane * PER + t * p.ld + R * D + lane;
+        const long long at = (long long)t * p.G * R + hv;
+        p.beta[at] = 1.f / (1.f + exp_full(-__bfloat162float(ba[0])));
+        p.g[at] = neg_a * softplus_(__bfloat162float(ba[R]) + dtb);
+      }
+    }
+    return;
+  }
+  float w[PER][KW], x[KW][PER];                  // row t is slot t & 3
 #pragma unroll
-    for (int c = 0; c < PER; ++c)
+  for (int c = 0; c < PER; ++c)
 #pragma unroll
-      for (int j = 0; j < KW; ++j)
-        w[s][c][j] = __bfloat162float(p.w[((long long)grp * S * D + s * D + lane * PER + c) * KW + j]);
-  const int hv = lane < R ? grp * R + lane : 0;
-  const float neg_a = lane < R ? -exp_full(__bfloat162float(p.A_log[hv])) : 0.f;
-  const float dtb = lane < R ? __bfloat162float(p.dt[hv]) : 0.f;
-  float x[KW][S][PER];                           // row t is slot t & 3
+    for (int j = 0; j < KW; ++j)
+      w[c][j] = __bfloat162float(p.w[(((long long)grp * S + s) * D + lane * PER + c) * KW + j]);
 #pragma unroll
   for (int u = 0; u < KW; ++u)
 #pragma unroll
-    for (int s = 0; s < S; ++s)
+    for (int c = 0; c < PER; ++c) x[u][c] = 0.f;
 #pragma unroll
-      for (int c = 0; c < PER; ++c) x[u][s][c] = 0.f;
-#pragma unroll
-  for (int b = 1; b < KW; ++b) {
-    const int t = t0 - b;
-    if (t >= 0) {
-#pragma unroll
-      for (int s = 0; s < S; ++s) ldn<PER>(src + t * p.ld + s * D, x[KW - b][s]);    // t0 is a multiple of 4
-    }
-  }
+  for (int b = 1; b < KW; ++b)
+    if (t0 - b >= 0) ldn<PER>(src + (t0 - b) * p.ld, x[KW - b]);    // t0 is a multiple of 4
   for (int tb = t0; tb < t1; tb += KW) {
+    float nx[KW][PER];                           // four rows in flight
+    int first[KW];
+#pragma unroll
+    for (int u = 0; u < KW; ++u)
+      if (tb + u < t1) {
+        ldn<PER>(src + (tb + u) * p.ld, nx[u]);
+        first[u] = p.seq_start[tb + u];
+      }
 #pragma unroll
     for (int u = 0; u < KW; ++u) {
       const int t = tb + u;
       if (t >= t1) break;
 #pragma unroll
-      for (int s = 0; s < S; ++s) ldn<PER>(src + t * p.ld + s * D, x[u][s]);
-      const int back = t - p.seq_start[t];       // rows of the same sequence before this one
-      float y[S][PER];
+      for (int c = 0; c < PER; ++c) x[u][c] = nx[u][c];
+      const int back = t - first[u];             // rows of the same sequence before this one
+      float y[PER];
 #pragma unroll
-      for (int s = 0; s < S; ++s)
+      for (int c = 0; c < PER; ++c) {
+        float a = 0.f;
 #pragma unroll
-        for (int c = 0; c < PER; ++c) {
-          float a = 0.f;
-#pragma unroll
-          for (int j = 0; j < KW; ++j)
-            a = fmaf(w[s][c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][s][c] : 0.f, a);
-          y[s][c] = bf_round(a * sigmoid_(a));
-        }
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
+        for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
+        y[c] = bf_round(a * sigmoid_(a));
+      }
+      if (s >= 2) {
+        stn<PER>(p.v + out_row(t) + (s - 2) * D, y);
+      } else {
         float ss = 0.f;
 #pragma unroll
-        for (int c = 0; c < PER; ++c) ss += y[s][c] * y[s][c];
+        for (int c = 0; c < PER; ++c) ss += y[c] * y[c];
         const float r = rsqrtf(wsum(ss) + 1e-6f);
 #pragma unroll
-        for (int c = 0; c < PER; ++c) y[s][c] *= r;
-      }
-      const long long row = ((long long)t * p.G + grp) * R * D + lane * PER;
+        for (int c = 0; c < PER; ++c) y[c] *= r;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        stn<PER>(p.q + row + r * D, y[0]);
-        stn<PER>(p.k + row + r * D, y[1]);
-        stn<PER>(p.v + row + r * D, y[2 + r]);
-        float zz[PER];
-        ldn<PER>(src + t * p.ld + (S + r) * D, zz);
-        stn<PER>(p.z + row + r * D, zz);
-      }
-      if (lane < R) {
-        const __nv_bfloat16* ba = src - lane * PER + t * p.ld + (S + R) * D + lane;
-        const long long at = (long long)t * p.G * R + hv;
-        p.beta[at] = 1.f / (1.f + exp_full(-__bfloat162float(ba[0])));
-        p.g[at] = neg_a * softplus_(__bfloat162float(ba[R]) + dtb);
+        for (int rr = 0; rr < R; ++rr) stn<PER>((s == 0 ? p.q : p.k) + out_row(t) + rr * D, y);
       }
     }
   }
@@ -157,133 +159,30 @@ template <int D, int R>
 __global__ void __launch_bounds__(WARPS * 32)
 gdn_inputs_bwd_kernel(const InParams p) {
   constexpr int PER = D / 32, S = 2 + R;
-  __shared__ float s_w[WARPS][32 * PER * KW];
+  __shared__ float s_w[WARPS][D * KW];
   __shared__ float s_h[WARPS][2][R];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = blockIdx.y, s = blockIdx.z;
   const int t0 = (blockIdx.x * WARPS + warp) * TOK_B, t1 = min(t0 + TOK_B, p.T);
   const int width = 2 * D + 2 * R * D + 2 * R;
-  const __nv_bfloat16* src = p.proj + (long long)grp * width + lane * PER;
-  __nv_bfloat16* dst = p.dproj + (long long)grp * width + lane * PER;
-  float dw[S][PER][KW];
-#pragma unroll
-  for (int s = 0; s < S; ++s)
-#pragma unroll
-    for (int c = 0; c < PER; ++c)
-#pragma unroll
-      for (int j = 0; j < KW; ++j) dw[s][c][j] = 0.f;
-  float dA = 0.f, ddt = 0.f;
-  if (t0 < t1) {
-    // slices are walked one after the other: the rows in flight of one slice are what fits the registers
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      float w[PER][KW], x[KW][PER], dp[KW][PER];     // row t and its dpre in slot t & 3
-#pragma unroll
-      for (int c = 0; c < PER; ++c)
-#pragma unroll
-        for (int j = 0; j < KW; ++j)
-          w[c][j] = __bfloat162float(p.w[((long long)grp * S * D + s * D + lane * PER + c) * KW + j]);
-#pragma unroll
-      for (int u = 0; u < KW; ++u)
-#pragma unroll
-        for (int c = 0; c < PER; ++c) x[u][c] = dp[u][c] = 0.f;
-#pragma unroll
-      for (int b = 1; b < KW; ++b)
-        if (t0 - b >= 0) ldn<PER>(src + (t0 - b) * p.ld + s * D, x[KW - b]);
-      const int te = min(t1 + KW - 1, p.T);          // dpre of the KW - 1 tokens behind the walk reaches into it
-      for (int tb = t0; tb < t1 + KW - 1; tb += KW) {
-#pragma unroll
-        for (int u = 0; u < KW; ++u) {
-          const int t = tb + u;
-          if (t >= t1 + KW - 1) break;
-          int first = 0x7fffffff;                    // first token of t's sequence; none past the end of the batch
-          if (t < te) {
-            first = p.seq_start[t];
-            ldn<PER>(src + t * p.ld + s * D, x[u]);
-            const long long row = ((long long)t * p.G + grp) * R * D + lane * PER;
-            float d[PER];
-            if (s < 2) {
-              const __nv_bfloat16* dn = (s == 0 ? p.dq : p.dk) + row;
-              ldn<PER>(dn, d);
-#pragma unroll
-              for (int r = 1; r < R; ++r) {
-                float e[PER];
-                ldn<PER>(dn + r * D, e);
-#pragma unroll
-                for (int c = 0; c < PER; ++c) d[c] += e[c];
-              }
-            } else {
-              ldn<PER>(p.dv + row + (s - 2) * D, d);
-            }
-            const int back = t - first;
-            float pre[PER], sg[PER], y[PER];
-#pragma unroll
-            for (int c = 0; c < PER; ++c) {
-              float a = 0.f;
-#pragma unroll
-              for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
-              pre[c] = a;
-              sg[c] = sigmoid_(a);
-              y[c] = bf_round(a * sg[c]);
-            }
-            if (s < 2) {                             // through y * rsqrt(sum y^2 + eps)
-              float ss = 0.f, dot = 0.f;
-#pragma unroll
-              for (int c = 0; c < PER; ++c) {
-                ss += y[c] * y[c];
-                dot += y[c] * d[c];
-              }
-              const float r = rsqrtf(wsum(ss) + 1e-6f);
-              dot = wsum(dot) * r * r;
-#pragma unroll
-              for (int c = 0; c < PER; ++c) d[c] = r * (d[c] - y[c] * dot);
-            }
-#pragma unroll
-            for (int c = 0; c < PER; ++c) {
-              dp[u][c] = d[c] * sg[c] * (1.f + pre[c] * (1.f - sg[c]));
-              if (t < t1) {                          // every token's tap gradients are added once, by its own walk
-#pragma unroll
-                for (int j = 0; j < KW; ++j)
-                  dw[s][c][j] = fmaf(dp[u][c], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, dw[s][c][j]);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < PER; ++c) dp[u][c] = 0.f;
-          }
-          // dpre of the rows t-3 .. t is complete for the projection row t - 3, as far as they share its sequence
-          const int tr = t - (KW - 1);
-          if (tr >= t0 && tr < t1) {
-            float dx[PER];
-#pragma unroll
-            for (int c = 0; c < PER; ++c) dx[c] = 0.f;
-#pragma unroll
-            for (int j = 0; j < KW; ++j) {           // tap j of row tr + (KW - 1 - j)
-              const int tt = tr + (KW - 1 - j);
-              const int f = tt == t ? first : (tt < p.T ? p.seq_start[tt] : 0x7fffffff);
-              if (f <= tr) {
-#pragma unroll
-                for (int c = 0; c < PER; ++c) dx[c] = fmaf(w[c][j], dp[(u + 4 - j) & 3][c], dx[c]);
-              }
-            }
-            stn<PER>(dst + tr * p.ld_d + s * D, dx);
-          }
-        }
-      }
-    }
+  const __nv_bfloat16* src = p.proj + (long long)grp * width + s * D + lane * PER;
+  __nv_bfloat16* dst = p.dproj + (long long)grp * width + s * D + lane * PER;
+  auto grad_row = [&](int t) { return ((long long)t * p.G + grp) * R * D + lane * PER; };
+  if (s == S) {                                  // z and the gates
     const int hv = lane < R ? grp * R + lane : 0;
     const float neg_a = lane < R ? -exp_full(__bfloat162float(p.A_log[hv])) : 0.f;
     const float dtb = lane < R ? __bfloat162float(p.dt[hv]) : 0.f;
+    float dA = 0.f, ddt = 0.f;
+#pragma unroll 4
     for (int t = t0; t < t1; ++t) {
-      const long long row = ((long long)t * p.G + grp) * R * D + lane * PER;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         float zz[PER];
-        ldn<PER>(p.dz + row + r * D, zz);
-        stn<PER>(dst + t * p.ld_d + (S + r) * D, zz);
+        ldn<PER>(p.dz + grad_row(t) + r * D, zz);
+        stn<PER>(dst + t * p.ld_d + r * D, zz);
       }
       if (lane < R) {
-        const __nv_bfloat16* ba = src - lane * PER + t * p.ld + (S + R) * D + lane;
-        __nv_bfloat16* dba = dst - lane * PER + t * p.ld_d + (S + R) * D + lane;
+        const __nv_bfloat16* ba = src - lane * PER + t * p.ld + R * D + lane;
+        __nv_bfloat16* dba = dst - lane * PER + t * p.ld_d + R * D + lane;
         const long long at = (long long)t * p.G * R + hv;
         const float beta = 1.f / (1.f + exp_full(-__bfloat162float(ba[0])));
         dba[0] = __float2bfloat16(p.dbeta[at] * beta * (1.f - beta));
@@ -294,31 +193,138 @@ gdn_inputs_bwd_kernel(const InParams p) {
         ddt += da;
       }
     }
+    if (lane < R) {
+      s_h[warp][0][lane] = dA;
+      s_h[warp][1][lane] = ddt;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * R) {                   // the block's sums, in a fixed order
+      const int which = threadIdx.x / R, r = threadIdx.x % R;
+      p.hpart[(long long)blockIdx.x * 2 * p.G * R + which * p.G * R + grp * R + r] =
+          (s_h[0][which][r] + s_h[1][which][r]) + (s_h[2][which][r] + s_h[3][which][r]);
+    }
+    return;
   }
-  // the block's sums, in a fixed order
-  const long long wcols = (long long)p.G * S * D * KW;
+  float dw[PER][KW];
 #pragma unroll
-  for (int s = 0; s < S; ++s) {
+  for (int c = 0; c < PER; ++c)
+#pragma unroll
+    for (int j = 0; j < KW; ++j) dw[c][j] = 0.f;
+  if (t0 < t1) {
+    float w[PER][KW], x[KW][PER], dp[KW][PER];   // row t and its dpre in slot t & 3
 #pragma unroll
     for (int c = 0; c < PER; ++c)
 #pragma unroll
-      for (int j = 0; j < KW; ++j) s_w[warp][(lane * PER + c) * KW + j] = dw[s][c][j];
-    __syncthreads();
-    for (int id = threadIdx.x; id < D * KW; id += WARPS * 32)
-      p.wpart[blockIdx.x * wcols + ((long long)grp * S + s) * D * KW + id] =
-          (s_w[0][id] + s_w[1][id]) + (s_w[2][id] + s_w[3][id]);
-    __syncthreads();
+      for (int j = 0; j < KW; ++j)
+        w[c][j] = __bfloat162float(p.w[(((long long)grp * S + s) * D + lane * PER + c) * KW + j]);
+#pragma unroll
+    for (int u = 0; u < KW; ++u)
+#pragma unroll
+      for (int c = 0; c < PER; ++c) x[u][c] = dp[u][c] = 0.f;
+    int start[KW];                               // first token of the sequence of row t, in slot t & 3
+#pragma unroll
+    for (int u = 0; u < KW; ++u) start[u] = 0x7fffffff;
+#pragma unroll
+    for (int b = 1; b < KW; ++b)
+      if (t0 - b >= 0) ldn<PER>(src + (t0 - b) * p.ld, x[KW - b]);
+    const int last = t1 + KW - 1;                // dpre of the KW - 1 tokens behind the walk reaches into it
+    const int te = min(last, p.T);
+    for (int tb = t0; tb < last; tb += KW) {
+      float nx[KW][PER], nd[KW][PER];            // four rows and their gradients in flight
+      int nf[KW];
+#pragma unroll
+      for (int u = 0; u < KW; ++u) {
+        const int t = tb + u;
+        nf[u] = 0x7fffffff;                      // past the end of the batch: in no sequence
+        if (t < te) {
+          nf[u] = p.seq_start[t];
+          ldn<PER>(src + t * p.ld, nx[u]);
+          const __nv_bfloat16* dn = (s == 0 ? p.dq : s == 1 ? p.dk : p.dv) + grad_row(t) + (s < 2 ? 0 : s - 2) * D;
+          ldn<PER>(dn, nd[u]);
+          if (s < 2) {
+#pragma unroll
+            for (int r = 1; r < R; ++r) {
+              float e[PER];
+              ldn<PER>(dn + r * D, e);
+#pragma unroll
+              for (int c = 0; c < PER; ++c) nd[u][c] += e[c];
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < KW; ++u) {
+        const int t = tb + u;
+        if (t >= last) break;
+        start[u] = nf[u];
+#pragma unroll
+        for (int c = 0; c < PER; ++c) dp[u][c] = 0.f;
+        if (t < te) {
+          const int back = t - nf[u];
+          float pre[PER], sg[PER], y[PER], d[PER];
+#pragma unroll
+          for (int c = 0; c < PER; ++c) {
+            x[u][c] = nx[u][c];
+            d[c] = nd[u][c];
+          }
+#pragma unroll
+          for (int c = 0; c < PER; ++c) {
+            float a = 0.f;
+#pragma unroll
+            for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
+            pre[c] = a;
+            sg[c] = sigmoid_(a);
+            y[c] = bf_round(a * sg[c]);
+          }
+          if (s < 2) {                           // through y * rsqrt(sum y^2 + eps)
+            float ss = 0.f, dot = 0.f;
+#pragma unroll
+            for (int c = 0; c < PER; ++c) {
+              ss += y[c] * y[c];
+              dot += y[c] * d[c];
+            }
+            const float r = rsqrtf(wsum(ss) + 1e-6f);
+            dot = wsum(dot) * r * r;
+#pragma unroll
+            for (int c = 0; c < PER; ++c) d[c] = r * (d[c] - y[c] * dot);
+          }
+#pragma unroll
+          for (int c = 0; c < PER; ++c) {
+            dp[u][c] = d[c] * sg[c] * (1.f + pre[c] * (1.f - sg[c]));
+            if (t < t1) {                        // every token's tap gradients are added once, by its own walk
+#pragma unroll
+              for (int j = 0; j < KW; ++j)
+                dw[c][j] = fmaf(dp[u][c], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, dw[c][j]);
+            }
+          }
+        }
+        // dpre of the rows t-3 .. t is complete for the projection row t - 3, as far as they share its sequence
+        const int tr = t - (KW - 1);
+        if (tr >= t0 && tr < t1) {
+          float dx[PER];
+#pragma unroll
+          for (int c = 0; c < PER; ++c) dx[c] = 0.f;
+#pragma unroll
+          for (int j = 0; j < KW; ++j) {         // tap j of row t - j
+            if (start[(u + 4 - j) & 3] <= tr) {
+#pragma unroll
+              for (int c = 0; c < PER; ++c) dx[c] = fmaf(w[c][j], dp[(u + 4 - j) & 3][c], dx[c]);
+            }
+          }
+          stn<PER>(dst + tr * p.ld_d, dx);
+        }
+      }
+    }
   }
-  if (lane < R) {
-    s_h[warp][0][lane] = dA;
-    s_h[warp][1][lane] = ddt;
-  }
+  // the block's sums, in a fixed order
+#pragma unroll
+  for (int c = 0; c < PER; ++c)
+#pragma unroll
+    for (int j = 0; j < KW; ++j) s_w[warp][(lane * PER + c) * KW + j] = dw[c][j];
   __syncthreads();
-  if (threadIdx.x < 2 * R) {
-    const int which = threadIdx.x / R, r = threadIdx.x % R;
-    p.hpart[(long long)blockIdx.x * 2 * p.G * R + which * p.G * R + grp * R + r] =
-        (s_h[0][which][r] + s_h[1][which][r]) + (s_h[2][which][r] + s_h[3][which][r]);
-  }
+  for (int id = threadIdx.x; id < D * KW; id += WARPS * 32)
+    p.wpart[((long long)blockIdx.x * p.G * S + (long long)grp * S + s) * D * KW + id] =
+        (s_w[0][id] + s_w[1][id]) + (s_w[2][id] + s_w[3][id]);
 }
 
 int blocks_t(int T, int tok) { return (T + WARPS * tok - 1) / (WARPS * tok); }
@@ -326,11 +332,11 @@ int blocks_t(int T, int tok) { return (T + WARPS * tok - 1) / (WARPS * tok); }
 template <int D, int R>
 int launch_inputs(const InParams& p, bool grad, float* dw, float* dA, float* ddt, cudaStream_t s) {
   if (!grad) {
-    gdn_inputs_fwd_kernel<D, R><<<dim3(blocks_t(p.T, TOK_F), p.G), WARPS * 32, 0, s>>>(p);
+    gdn_inputs_fwd_kernel<D, R><<<dim3(blocks_t(p.T, TOK_F), p.G, 3 + R), WARPS * 32, 0, s>>>(p);
     return (int)cudaGetLastError();
   }
   const int nb = blocks_t(p.T, TOK_B);
-  gdn_inputs_bwd_kernel<D, R><<<dim3(nb, p.G), WARPS * 32, 0, s>>>(p);
+  gdn_inputs_bwd_kernel<D, R><<<dim3(nb, p.G, 3 + R), WARPS * 32, 0, s>>>(p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   launch_reduce_partials<float>(p.wpart, nb, p.G * (2 + R) * D * KW, dw, nullptr, p.G * (2 + R) * D * KW, s);
