@@ -363,7 +363,6 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
         from . import _lib
         lib = _lib.lib()
         T, h, d = q.shape
-        q, k, v, g, beta = (t.contiguous() for t in (q, k, v, g, beta))
         n_seq = cu.numel() - 1
         o = torch.empty_like(v) if covered else torch.zeros_like(v)
         mp, gb, _ = _GatedDeltaRuleFn._workspaces(lib, T, h, n_seq, q.device)
@@ -382,6 +381,12 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
         from . import _lib
         lib = _lib.lib()
         q, k, v, g, beta, cu = ctx.saved_tensors
+        if torch.is_grad_enabled():     # create_graph: the torch evaluation, whose gradient can be differentiated again
+            leaves = (q, k, v, g, beta)
+            o = _chunk_gated_delta_rule_torch(*leaves, cu, ctx.scale)
+            need = [t for t, n in zip(leaves, ctx.needs_input_grad) if n]
+            grads = iter(torch.autograd.grad(o, need, do, create_graph=True))
+            return tuple(next(grads) if n else None for n in ctx.needs_input_grad[:5]) + (None, None, None)
         T, h, d = q.shape
         n_seq = cu.numel() - 1
         do = do.contiguous()
@@ -470,15 +475,19 @@ def chunk_gated_delta_rule(q, k, v, g, beta, cu_seqlens=None, scale: Optional[fl
                            chunk: int = 64):
     """Dispatches to the CUDA kernels (bf16 q / k / v with square heads of 64 or 128) or the torch evaluation."""
     T, h, d = q.shape
-    if _cuda_ok(q, k, v) and d in (64, 128) and k.shape == q.shape and v.shape == q.shape and T > 0 \
+    # function transforms and forward-mode derivatives go through the torch evaluation, which composes with them
+    plain = not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+    if plain and _cuda_ok(q, k, v) and d in (64, 128) and k.shape == q.shape and v.shape == q.shape and T > 0 \
             and g.is_floating_point() and beta.is_floating_point() and g.shape == beta.shape == (T, h):
         host = (0, T) if cu_seqlens is None else getattr(cu_seqlens, '_host_list', None)
         # tokens outside every sequence read as zero: only boundaries known to span the batch spare the zero fill
         covered = host is not None and host[0] == 0 and host[-1] == T
         cu = torch.tensor([0, T], dtype=torch.int32, device=q.device) if cu_seqlens is None else \
             cu_seqlens.to(device=q.device, dtype=torch.int32)
-        return _GatedDeltaRuleFn.apply(q, k, v, g.float(), beta.float(), cu,
-                                       float(d**-0.5 if scale is None else scale), covered)
+        # contiguous outside of the function: what it saves are its inputs, which keeps them differentiable again
+        q, k, v, g, beta = (t.contiguous() for t in (q, k, v, g.float(), beta.float()))
+        return _GatedDeltaRuleFn.apply(q, k, v, g, beta, cu, float(d**-0.5 if scale is None else scale),
+                                       covered)
     return _chunk_gated_delta_rule_torch(q, k, v, g, beta, cu_seqlens, scale, chunk)
 
 

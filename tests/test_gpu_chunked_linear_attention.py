@@ -85,6 +85,21 @@ def test_gated_delta_rule_outside_every_sequence_is_zero():
     assert all((t[70:] == 0).all() and (t[:70] != 0).any() for t in (o, *grads))
 
 
+def test_gated_delta_rule_differentiates_twice():
+    """With ``create_graph`` the gradient comes from the torch evaluation: same values, and differentiable again."""
+    from mcore_bridge_b200.ops.gdn import chunk_gated_delta_rule, l2norm
+    (q, k, v, dy), _ = _inputs(80, 2, 64, 5)
+    q, k = l2norm(q), l2norm(k)
+    g, beta = -torch.rand(80, 2, device=DEV), torch.rand(80, 2, device=DEV)
+    leaves = [t.requires_grad_() for t in (q, k, v, g, beta)]
+    first = torch.autograd.grad(chunk_gated_delta_rule(*leaves), leaves, dy)
+    again = torch.autograd.grad(chunk_gated_delta_rule(*leaves), leaves, dy, create_graph=True)
+    for a, b in zip(first, again):
+        assert _rel(a, b.double()) < 2 ** -8
+    second = torch.autograd.grad(again[2].float().square().sum(), beta)[0]
+    assert torch.isfinite(second).all() and (second != 0).any()
+
+
 @pytest.mark.parametrize('T,groups,ratio,d,cuts', [(1, 1, 1, 64, []), (3, 2, 2, 128, [1]), (16, 1, 4, 64, [13, 15]),
                                                    (65, 3, 2, 128, [62, 64]), (130, 2, 4, 128, []), (257, 2, 1, 64, [1, 2, 3])])
 def test_gdn_inputs_walk_edges(T, groups, ratio, d, cuts):
