@@ -12,8 +12,8 @@
 //   dv = beta Y     dS = exp(G_last) dS' + (scale exp(G) q)^T do - (exp(G) k)^T (beta Y)     dA = -(Y V^T)     dP = do V^T
 //
 // with dq, dk, dg, dbeta following from these products (gdr_grad_kernel).  Launches: `prep` forms M and P of every chunk
-// independently; `scan` walks the chunks of a (sequence, head, 64 columns of v) in order; backward, `scan` runs again and
-// keeps S and V, `scan_bwd` walks in reverse and keeps dS' and Y, `grad` finishes every chunk independently.
+// independently (kept for the backward pass); `scan` walks the chunks of a (sequence, head, 64 columns of v) in order; backward,
+// `scan` runs again and keeps S and V, `scan_bwd` walks in reverse and keeps dS' and Y, `grad` finishes every chunk independently.
 //
 // Precision: the state, M, P, V and every accumulation are fp32.  Operands of a product that are not bf16 inputs enter the
 // tensor core as two bf16 terms (16 mantissa bits, warp_mma.cuh); a product of two such operands takes three MMAs.
@@ -21,7 +21,7 @@
 // In the scans a warp owns 16 columns of v and keeps S^T (16 x d) in its accumulators: the accumulators of every product
 // are the first operand of the next one, so the warps of a CTA share the loaded tiles and never exchange values.  Bound:
 // the chain of ~500 MMAs per chunk; the next chunk's tiles are copied meanwhile.  Measured, 4096 tokens in three sequences,
-// 32 heads of 128: forward 0.22 ms (prep 0.07, scan 0.15), backward 0.81 ms (prep, scan, scan_bwd 0.20, grad 0.39); the
+// 32 heads of 128: forward 0.22 ms (prep 0.07, scan 0.15), backward 0.72 ms (scan, scan_bwd 0.21, grad 0.36); the
 // batched torch evaluation of the rule was most of a 29.5 ms block.
 #include "../common/host_utils.cuh"
 #include "warp_mma.cuh"
@@ -596,26 +596,30 @@ gdr_scan_bwd_kernel(const GdrParams p) {
 }
 
 // ---------------------------------------------------------------------------------------------------- grad
-// dq, dk, dg, dbeta of one chunk.  Rows = tokens, 16 a warp.  S^T and dS'^T stream through shared memory 32 columns at a
-// time (two stages); everything else the chunk needs is resident.
+// dq, dk, dg, dbeta of one chunk.  Rows = tokens; two warps share 16 of them, each with half of the d columns of dq and dk
+// (both form the 16 x 16 blocks of dP and dA: a fifth more MMAs, yet 387 -> 363 us against one warp per 16 rows, whose
+// chains waited for themselves; what bounds it now is the rate of the warp-level MMAs and the unoverlapped load of 256 KB a
+// chunk).  S^T and dS'^T pass through shared memory 32 columns per half at a time;
+// everything else the chunk needs is resident.
+constexpr int GT = 256;
+
 template <int D>
 struct GradSmem {
   static constexpr int TILE = C * D * 2;
   static constexpr int Q = 0, K = TILE, V = 2 * TILE, DO = 3 * TILE;        // token tiles
   static constexpr int VT = 4 * TILE, YT = 6 * TILE;                        // V^T, Y^T: two terms of [D][64] each
-  static constexpr int ST = 8 * TILE;                                       // 2 stages of S^T, dS'^T: two terms of [D][32]
+  static constexpr int ST = 8 * TILE;                                       // per half: S^T, dS'^T, two terms of [D][32] each
   static constexpr int STRIP = D * 32 * 2;
   static constexpr int TOTAL = ST + 2 * 4 * STRIP + 128;
 };
 
 template <int D>
 __device__ __forceinline__ void load_strips(uint32_t st, const __nv_bfloat16* S, const __nv_bfloat16* dS, int col0) {
-  for (int id = threadIdx.x; id < 4 * D * 4; id += THREADS) {
+  for (int id = threadIdx.x; id < 4 * D * 4; id += GT) {
     const int m = id / (D * 4), r = (id / 4) % D, c = (id & 3) * 8;
     const __nv_bfloat16* src = (m < 2 ? S : dS) + (m & 1) * D * D + r * D + col0 + c;
     cp_async16(tile_addr<32>(st + m * GradSmem<D>::STRIP, r, c), src, 16);
   }
-  cp_async_commit();
 }
 
 __device__ __forceinline__ float quad_sum(float x) {   // over the four lanes that share an accumulator row
@@ -630,47 +634,46 @@ __device__ __forceinline__ float2 tile_pair(uint32_t tile, int row, int col) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(GT)
 gdr_grad_kernel(const GdrParams p) {
   using L = GradSmem<D>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ ChunkPos slot;
-  __shared__ float s_g[C], s_b[C], s_dg[C], s_red[4];
+  __shared__ float s_g[C], s_b[C], s_dg[2][C], s_db[2][C], s_red[8];
+  constexpr int NW = D / 64, NT = D / 16;      // strips and 8-column blocks of a half
   const uint32_t base = (smem_u32(smem_raw) + 127) & ~127u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y;
+  const int warp = (threadIdx.x >> 5) & 3, half = threadIdx.x >> 7, lane = threadIdx.x & 31, h = blockIdx.y;
   const ChunkPos pos = locate(p, &slot);
   if (pos.seq < 0) return;
   const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
   const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
   const long long ch = (long long)blockIdx.x * p.H + h;
-  load_tile<D, C, THREADS>(base + L::Q, p.q + off, stride, len);
-  load_tile<D, C, THREADS>(base + L::K, p.k + off, stride, len);
-  load_tile<D, C, THREADS>(base + L::V, p.v + off, stride, len);
-  load_tile<D, C, THREADS>(base + L::DO, p.dout + off, stride, len);
-  for (int id = threadIdx.x; id < 4 * D * 8; id += THREADS) {
+  load_tile<D, C, GT>(base + L::Q, p.q + off, stride, len);
+  load_tile<D, C, GT>(base + L::K, p.k + off, stride, len);
+  load_tile<D, C, GT>(base + L::V, p.v + off, stride, len);
+  load_tile<D, C, GT>(base + L::DO, p.dout + off, stride, len);
+  for (int id = threadIdx.x; id < 4 * D * 8; id += GT) {
     const int m = id / (D * 8), r = (id / 8) % D, c = (id & 7) * 8;
     const __nv_bfloat16* src = (m < 2 ? p.V : p.Y) + ch * 2 * D * C + (m & 1) * D * C + r * C + c;
     cp_async16(tile_addr<64>(base + L::VT + m * L::TILE, r, c), src, 16);
   }
-  cp_async_commit();
   const __nv_bfloat16 *S = p.S + ch * 2 * D * D, *dS = p.dS + ch * 2 * D * D;
-  load_strips<D>(base + L::ST, S, dS, 0);
+  const int c0 = half * (D / 2);               // first column of this warp's half
+  const uint32_t st = base + L::ST + half * 4 * L::STRIP;
   if (threadIdx.x < C) {
     s_g[threadIdx.x] = p.gb[ch * 2 * C + threadIdx.x];
     s_b[threadIdx.x] = p.gb[ch * 2 * C + C + threadIdx.x];
   }
   const int r0 = warp * 16, i = r0 + (lane >> 2), c2 = (lane & 3) * 2;
-  float dq[D / 8][4], dk[D / 8][4];
+  float dq[NT][4], dk[NT][4];
   float qf[2] = {0.f, 0.f}, kh[2] = {0.f, 0.f}, ke[2] = {0.f, 0.f}, sdot = 0.f;
   float eg[2], el[2], bi[2], gi[2];
 #pragma unroll
-  for (int w = 0; w < D / 32; ++w) {
-    if (w + 1 < D / 32) {
-      load_strips<D>(base + L::ST + ((w + 1) & 1) * 4 * L::STRIP, S, dS, (w + 1) * 32);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+  for (int w = 0; w < NW; ++w) {
+    load_strips<D>(base + L::ST, S, dS, w * 32);
+    load_strips<D>(base + L::ST + 4 * L::STRIP, S, dS, D / 2 + w * 32);
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
     if (w == 0) {
       const float gl = s_g[C - 1];
@@ -682,7 +685,6 @@ gdr_grad_kernel(const GdrParams p) {
         el[r] = exp2f(gl - gi[r]);
       }
     }
-    const uint32_t st = base + L::ST + (w & 1) * 4 * L::STRIP;
     float F[4][4] = {}, E[4][4] = {}, Hh[4][4] = {};
 #pragma unroll 1
     for (int kk = 0; kk < D; kk += 16) {        // contraction over the columns of v
@@ -717,7 +719,7 @@ gdr_grad_kernel(const GdrParams p) {
     }
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
-      const int col = w * 32 + n * 8 + c2;
+      const int col = c0 + w * 32 + n * 8 + c2;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const float2 qq = tile_pair<D>(base + L::Q, i + 8 * r, col), kq = tile_pair<D>(base + L::K, i + 8 * r, col);
@@ -733,7 +735,7 @@ gdr_grad_kernel(const GdrParams p) {
         dk[w * 4 + n][2 * r + 1] = h1 - bi[r] * e1;
       }
     }
-    for (int id = threadIdx.x; id < D * 16; id += THREADS) {       // <S, dS'>
+    for (int id = threadIdx.x & 127; id < D * 16; id += 128) {     // <S, dS'>, this half's columns
       const int r = id >> 4, c = (id & 15) * 2;
       const float2 a = tile_pair<32>(st, r, c), b = tile_pair<32>(st + L::STRIP, r, c);
       const float2 d = tile_pair<32>(st + 2 * L::STRIP, r, c), e = tile_pair<32>(st + 3 * L::STRIP, r, c);
@@ -742,7 +744,7 @@ gdr_grad_kernel(const GdrParams p) {
     __syncthreads();
   }
   float yv[2] = {0.f, 0.f};                      // Y_i . v_i: the diagonal of a 16 x 16 product
-  {
+  if (half == 0) {
     float s[2][4] = {};
 #pragma unroll 1
     for (int kk = 0; kk < D; kk += 16) {
@@ -807,8 +809,10 @@ gdr_grad_kernel(const GdrParams p) {
         const float D_ = jj <= ii ? exp2f(gi[r] - s_g[jj]) : 0.f;
         const float x = dP[n][e] * p.scale * D_;                    // d(q k^T)_ij
         const float y = jj < ii ? -dA[n][e] * D_ : 0.f;             // dA_ij D_ij
-        dgc[r] += x * qk[n][e] + y * bi[r] * kk2[n][e];
-        db[r] += y * kk2[n][e];
+        if (half == 0) {
+          dgc[r] += x * qk[n][e] + y * bi[r] * kk2[n][e];
+          db[r] += y * kk2[n][e];
+        }
         dP[n][e] = x;
         dA[n][e] = y * bi[r];
       }
@@ -816,9 +820,9 @@ gdr_grad_kernel(const GdrParams p) {
     acc_to_a(dP[0], dP[1], xh, xl);
     acc_to_a(dA[0], dA[1], yh, yl);
 #pragma unroll
-    for (int n = 0; n < D / 8; n += 2) {
+    for (int n = 0; n < NT; n += 2) {
       uint32_t b[4];
-      load_b_nn<D>(base + L::K, jb * 16, n * 8, lane, b);
+      load_b_nn<D>(base + L::K, jb * 16, c0 + n * 8, lane, b);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         mma16816(dq[n + u], xh, b[2 * u], b[2 * u + 1]);
@@ -868,7 +872,7 @@ gdr_grad_kernel(const GdrParams p) {
         const float D_ = jj <= ii ? exp2f(s_g[ii] - gi[r]) : 0.f;
         const float x = dP[n][e] * p.scale * D_;
         const float y = jj < ii ? -dA[n][e] * D_ * s_b[ii] : 0.f;
-        dgc[r] -= x * qk[n][e] + y * kk2[n][e];
+        if (half == 0) dgc[r] -= x * qk[n][e] + y * kk2[n][e];
         dP[n][e] = x;
         dA[n][e] = y;
       }
@@ -876,10 +880,10 @@ gdr_grad_kernel(const GdrParams p) {
     acc_to_a(dP[0], dP[1], xh, xl);
     acc_to_a(dA[0], dA[1], yh, yl);
 #pragma unroll
-    for (int n = 0; n < D / 8; n += 2) {
+    for (int n = 0; n < NT; n += 2) {
       uint32_t b[4], d[4];
-      load_b_nn<D>(base + L::Q, ib * 16, n * 8, lane, b);
-      load_b_nn<D>(base + L::K, ib * 16, n * 8, lane, d);
+      load_b_nn<D>(base + L::Q, ib * 16, c0 + n * 8, lane, b);
+      load_b_nn<D>(base + L::K, ib * 16, c0 + n * 8, lane, d);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         mma16816(dk[n + u], xh, b[2 * u], b[2 * u + 1]);
@@ -890,11 +894,11 @@ gdr_grad_kernel(const GdrParams p) {
     }
   }
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n)
+  for (int n = 0; n < NT; ++n)
 #pragma unroll
     for (int r = 0; r < 2; ++r)
       if (i + 8 * r < len) {
-        const long long at = off + (i + 8 * r) * stride + n * 8 + c2;
+        const long long at = off + (i + 8 * r) * stride + c0 + n * 8 + c2;
         *reinterpret_cast<uint32_t*>(p.dq + at) = pack_bf16x2(dq[n][2 * r], dq[n][2 * r + 1]);
         *reinterpret_cast<uint32_t*>(p.dk + at) = pack_bf16x2(dk[n][2 * r], dk[n][2 * r + 1]);
       }
@@ -903,18 +907,25 @@ gdr_grad_kernel(const GdrParams p) {
   for (int r = 0; r < 2; ++r) {
     const float a = quad_sum(dgc[r]), b = quad_sum(db[r]);
     if ((lane & 3) == 0) {
-      s_dg[i + 8 * r] = a;
-      if (i + 8 * r < len) p.dbeta[(long long)(t + i + 8 * r) * p.H + h] = b;
+      s_dg[half][i + 8 * r] = a;
+      s_db[half][i + 8 * r] = b;
     }
   }
   float tot = xs + exp2f(s_g[C - 1]) * sdot;
 #pragma unroll
   for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-  if (lane == 0) s_red[warp] = tot;
+  if (lane == 0) s_red[threadIdx.x >> 5] = tot;
   __syncthreads();
-  if (warp == 0) {
-    const float last = (s_red[0] + s_red[1]) + (s_red[2] + s_red[3]);
-    const float x0 = s_dg[2 * lane], x1 = s_dg[2 * lane + 1] + (lane == 31 ? last : 0.f);
+  if (threadIdx.x >= 32 && threadIdx.x < 32 + C) {
+    const int r = threadIdx.x - 32;
+    if (r < len) p.dbeta[(long long)(t + r) * p.H + h] = s_db[0][r] + s_db[1][r];
+  }
+  if (threadIdx.x < 32) {
+    float last = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) last += s_red[r];
+    const float x0 = s_dg[0][2 * lane] + s_dg[1][2 * lane];
+    const float x1 = s_dg[0][2 * lane + 1] + s_dg[1][2 * lane + 1] + (lane == 31 ? last : 0.f);
     float run = x0 + x1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -943,9 +954,9 @@ int launch_gdr(const GdrParams& p, int T, bool grad, cudaStream_t s) {
   }
   const dim3 chunks(T / C + p.n_seq, p.H);       // at least the number of chunks of any packing of T tokens
   const unsigned scans = (unsigned)p.n_seq * p.H * (D / 64);
-  gdr_prep_kernel<D><<<chunks, THREADS, PREP, s>>>(p);
-  if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
   if (!grad) {
+    gdr_prep_kernel<D><<<chunks, THREADS, PREP, s>>>(p);
+    if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
     gdr_scan_kernel<D, false><<<scans, THREADS, ScanSmem<D>::TOTAL, s>>>(p);
     return (int)cudaGetLastError();
   }
@@ -953,7 +964,7 @@ int launch_gdr(const GdrParams& p, int T, bool grad, cudaStream_t s) {
   if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
   gdr_scan_bwd_kernel<D><<<scans, THREADS, ScanSmem<D>::TOTAL, s>>>(p);
   if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-  gdr_grad_kernel<D><<<chunks, THREADS, GradSmem<D>::TOTAL, s>>>(p);
+  gdr_grad_kernel<D><<<chunks, GT, GradSmem<D>::TOTAL, s>>>(p);
   return (int)cudaGetLastError();
 }
 
@@ -979,7 +990,7 @@ extern "C" {
 int mcb_gdr_chunks(int T, int n_seq) { return T / C + n_seq; }
 
 // q, k, v, o [T, H, D] bf16; g, beta [T, H] fp32; cu_seqlens [n_seq + 1] int32 from 0 to T.  Workspaces, per chunk and
-// head: mp [4, 64, 64] bf16, gb [2, 64] fp32.
+// head: mp [4, 64, 64] bf16, gb [2, 64] fp32; the backward pass reads them again.
 int mcb_gdr_fwd(const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu_seqlens, void* o,
                 void* mp, float* gb, int T, int n_seq, int H, int D, float scale, void* stream_) {
   if (n_seq <= 0 || T <= 0) return 0;
@@ -988,7 +999,7 @@ int mcb_gdr_fwd(const void* q, const void* k, const void* v, const float* g, con
   return run_gdr(p, T, D, false, reinterpret_cast<cudaStream_t>(stream_));
 }
 
-// Further workspaces, per chunk and head: states [2, 2, D, D] bf16 (all S first, then all dS), values [2, 2, D, 64] bf16
+// mp and gb as the forward pass left them.  Further workspaces, per chunk and head: states [2, 2, D, D] bf16 (all S first, then all dS), values [2, 2, D, 64] bf16
 // (all V, then all Y).
 int mcb_gdr_bwd(const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu_seqlens,
                 const void* dout, void* dq, void* dk, void* dv, float* dg, float* dbeta, void* mp, float* gb, void* states,

@@ -9,6 +9,9 @@
 // A warp owns one group and walks consecutive tokens with the last rows in registers, so every projection element is read
 // once (plus 3 rows of overlap per walk) instead of once per slice, copy, norm and tap.  Bound: memory.
 //
+// Measured, 4096 tokens, 16 groups, R = 2, d = 128: forward 86 us, backward 241 us (instruction-bound: the taps, SiLU and
+// its derivative are recomputed per element); the copy rate would take 36 and 70 us.
+//
 // Values are rounded to bf16 where the separate operators store them (convolution output, normalised q / k).
 #include "../common/host_utils.cuh"
 #include "../common/partials.cuh"
@@ -20,8 +23,8 @@ namespace {
 
 constexpr int KW = 4;            // taps
 constexpr int WARPS = 4;
-constexpr int TOK_F = 16;        // tokens a warp walks, forward / backward: enough warps at a few thousand tokens
-constexpr int TOK_B = 16;
+constexpr int TOK_F = 16;        // tokens a warp walks, forward / backward (which repeats 3 tokens of the next walk):
+constexpr int TOK_B = 32;        // enough warps at a few thousand tokens
 
 struct InParams {
   const __nv_bfloat16* proj;               // [T, ld]
@@ -135,8 +138,13 @@ gdn_inputs_fwd_kernel(const InParams p) {
 #pragma unroll
       for (int c = 0; c < PER; ++c) {
         float a = 0.f;
+        if (back >= KW - 1) {                    // the whole window lies in the sequence (the same for all lanes)
 #pragma unroll
-        for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
+          for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], x[(u + 1 + j) & 3][c], a);
+        } else {
+#pragma unroll
+          for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
+        }
         y[c] = bf_round(a * sigmoid_(a));
       }
       if (s >= 2) {
@@ -270,8 +278,13 @@ gdn_inputs_bwd_kernel(const InParams p) {
 #pragma unroll
           for (int c = 0; c < PER; ++c) {
             float a = 0.f;
+            if (back >= KW - 1) {
 #pragma unroll
-            for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
+              for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], x[(u + 1 + j) & 3][c], a);
+            } else {
+#pragma unroll
+              for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
+            }
             pre[c] = a;
             sg[c] = sigmoid_(a);
             y[c] = bf_round(a * sg[c]);
@@ -292,9 +305,14 @@ gdn_inputs_bwd_kernel(const InParams p) {
           for (int c = 0; c < PER; ++c) {
             dp[u][c] = d[c] * sg[c] * (1.f + pre[c] * (1.f - sg[c]));
             if (t < t1) {                        // every token's tap gradients are added once, by its own walk
+              if (back >= KW - 1) {
 #pragma unroll
-              for (int j = 0; j < KW; ++j)
-                dw[c][j] = fmaf(dp[u][c], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, dw[c][j]);
+                for (int j = 0; j < KW; ++j) dw[c][j] = fmaf(dp[u][c], x[(u + 1 + j) & 3][c], dw[c][j]);
+              } else {
+#pragma unroll
+                for (int j = 0; j < KW; ++j)
+                  dw[c][j] = fmaf(dp[u][c], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, dw[c][j]);
+              }
             }
           }
         }

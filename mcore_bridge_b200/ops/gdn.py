@@ -348,13 +348,8 @@ class _SimpleGlaFn(torch.autograd.Function):
 
 
 class _GatedDeltaRuleFn(torch.autograd.Function):
-    """``csrc/linear_attention/gated_delta_rule.cu``; the inputs are all that is kept for the backward pass."""
-
-    @staticmethod
-    def _workspaces(lib, T, h, n_seq, device):
-        n = lib.mcb_gdr_chunks(T, n_seq) * h
-        return (torch.empty((n, 4, 64, 64), dtype=torch.bfloat16, device=device),
-                torch.empty((n, 2, 64), dtype=torch.float32, device=device), n)
+    """``csrc/linear_attention/gated_delta_rule.cu``; kept for the backward pass: the inputs and, per chunk and head, the
+    two 64 x 64 matrices ``prep`` forms (as much as q and k together at a head size of 128)."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, cu, scale, covered):
@@ -365,12 +360,14 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
         T, h, d = q.shape
         n_seq = cu.numel() - 1
         o = torch.empty_like(v) if covered else torch.zeros_like(v)
-        mp, gb, _ = _GatedDeltaRuleFn._workspaces(lib, T, h, n_seq, q.device)
+        n = lib.mcb_gdr_chunks(T, n_seq) * h
+        mp = torch.empty((n, 4, 64, 64), dtype=torch.bfloat16, device=q.device)
+        gb = torch.empty((n, 2, 64), dtype=torch.float32, device=q.device)
         rc = lib.mcb_gdr_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(g), _lib.ptr(beta), _lib.ptr(cu),
                              _lib.ptr(o), _lib.ptr(mp), _lib.ptr(gb), ctypes.c_int(T), ctypes.c_int(n_seq),
                              ctypes.c_int(h), ctypes.c_int(d), ctypes.c_float(scale), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_gdr_fwd')
-        ctx.save_for_backward(q, k, v, g, beta, cu)
+        ctx.save_for_backward(q, k, v, g, beta, cu, mp, gb)
         ctx.scale, ctx.covered = scale, covered
         return o
 
@@ -380,7 +377,7 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
 
         from . import _lib
         lib = _lib.lib()
-        q, k, v, g, beta, cu = ctx.saved_tensors
+        q, k, v, g, beta, cu, mp, gb = ctx.saved_tensors
         if torch.is_grad_enabled():     # create_graph: the torch evaluation, whose gradient can be differentiated again
             leaves = (q, k, v, g, beta)
             o = _chunk_gated_delta_rule_torch(*leaves, cu, ctx.scale)
@@ -392,7 +389,7 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
         do = do.contiguous()
         alloc = torch.empty_like if ctx.covered else torch.zeros_like
         dq, dk, dv, dg, dbeta = (alloc(t) for t in (q, k, v, g, beta))
-        mp, gb, n = _GatedDeltaRuleFn._workspaces(lib, T, h, n_seq, q.device)
+        n = mp.shape[0]
         states = torch.empty((2, n, 2, d, d), dtype=torch.bfloat16, device=q.device)
         values = torch.empty((2, n, 2, d, 64), dtype=torch.bfloat16, device=q.device)
         rc = lib.mcb_gdr_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(g), _lib.ptr(beta), _lib.ptr(cu),
