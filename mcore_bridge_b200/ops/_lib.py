@@ -31,7 +31,8 @@ class KernelError(RuntimeError):
     pass
 
 
-_device_present = None  # whether the process has a GPU cannot change; asking the driver on every op costs more than the op
+# whether the process has a GPU cannot change; asking the driver on every op is slow
+_device_present = None
 
 
 def cuda_enabled() -> bool:

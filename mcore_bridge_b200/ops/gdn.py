@@ -348,8 +348,8 @@ class _SimpleGlaFn(torch.autograd.Function):
 
 
 class _GatedDeltaRuleFn(torch.autograd.Function):
-    """``csrc/linear_attention/gated_delta_rule.cu``; kept for the backward pass: the inputs and, per chunk and head, the
-    two 64 x 64 matrices ``prep`` forms (as much as q and k together at a head size of 128)."""
+    """``csrc/linear_attention/gated_delta_rule.cu``; kept for the backward pass: the inputs and,
+    per chunk and head, the two 64 x 64 matrices ``prep`` forms (as much as q and k together at a head size of 128)."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, cu, scale, covered):

@@ -21,7 +21,8 @@ def _inputs(T, h, d, seed):
 
 
 @pytest.mark.parametrize('T,h,d,cuts', [(1, 1, 64, []), (5, 2, 128, [2, 2]), (127, 2, 64, []), (128, 3, 128, []),
-                                        (129, 2, 128, [1]), (700, 4, 64, [3, 130, 131, 600]), (800, 2, 128, [128, 384])])
+                                        (129, 2, 128, [1]), (700, 4, 64, [3, 130, 131, 600]),
+                                        (800, 2, 128, [128, 384])])
 def test_simple_gla_chunk_edges(T, h, d, cuts):
     from mcore_bridge_b200.ops.gdn import simple_gla
     (q, k, v, dy), _ = _inputs(T, h, d, 1)
@@ -101,9 +102,11 @@ def test_gated_delta_rule_differentiates_twice():
 
 
 @pytest.mark.parametrize('T,groups,ratio,d,cuts', [(1, 1, 1, 64, []), (3, 2, 2, 128, [1]), (16, 1, 4, 64, [13, 15]),
-                                                   (65, 3, 2, 128, [62, 64]), (130, 2, 4, 128, []), (257, 2, 1, 64, [1, 2, 3])])
+                                                   (65, 3, 2, 128, [62, 64]), (130, 2, 4, 128, []),
+                                                   (257, 2, 1, 64, [1, 2, 3])])
 def test_gdn_inputs_walk_edges(T, groups, ratio, d, cuts):
-    """Projection -> inputs of the delta rule in one pass, at the edges of a warp's walk (16 tokens) and of sequences."""
+    """Projection -> inputs of the delta rule in one pass, at the edges of a warp's walk (16 / 32 tokens) and of
+    sequences."""
     import torch.nn.functional as F
     from mcore_bridge_b200.ops.attention_cuda import seq_start_from_cu
     from mcore_bridge_b200.ops.gdn import gdn_inputs
