@@ -12,19 +12,23 @@
 // grows.  FlashAttention-4 waits until it has grown by 2^8, which spares most of the rescales, but then the row's largest
 // probabilities lie anywhere between two powers of two instead of just below 1, where the spacing of bf16 is finest
 // relative to them: off from fp64 by 0.00223 instead of 0.00213 (12363 tokens; 0.00215 with the final maximum as the
-// reference).  The rescales cost 4 % of this kernel at 4096 and 16384 tokens.
+// reference).
 //
-// Warp roles (384 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4..7 softmax of tile 0, warps 8..11
-// of tile 1 (thread = query row, a whole 128-column score row in registers: the control warps give registers up).  TMEM:
-// S0 | S1 (128 columns each, P overwrites the scores it came from as packed bf16) | O0 | O1.  The issuer's order is
-// PV_t(j), QK_t(j + 1)  for t = 0, 1: the score buffer of a tile is reused as soon as its P has been multiplied, and MMAs
-// of one thread complete in order.
+// Warp roles (512 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4..7 softmax of tile 0, warps 8..11
+// of tile 1 (thread = query row, a whole 128-column score row in registers: the other warps give registers up), warps
+// 12..15 rescale the accumulators of both tiles.  TMEM: S0 | S1 (128 columns each, P overwrites the scores it came from as
+// packed bf16) | O0 | O1.  The issuer's order is  PV_t(j), QK_t(j + 1)  for t = 0, 1: the score buffer of a tile is reused
+// as soon as its P has been multiplied, MMAs of one thread complete in order, and the two tiles stay out of phase.
 //
 // Bound: per 128 x 128 block the two products take 1024 tensor cycles and the 16384 exponentials 1024 MUFU cycles of an
-// SM, so both pipes are the floor; the two tiles in flight overlap them.  Measured, 32 query / 8 kv heads of 128, causal:
-// 16384 tokens 2.24 ms = 980 TFLOP/s; the form before it (maxima in a first pass over Q K^T, one tile per CTA, P through
-// shared memory) took 3.35 ms.  Neither pipe is full (43 % each in a capture at 4096 tokens, there at 880 TFLOP/s): the chain
-// load - maximum - exponentials - product - scores of a tile sets the pace, which is why P is handed over in halves.
+// SM; what sets the pace is the chain of a tile, load - maximum - exponentials - product - next scores.  Clock stamps of the
+// form with the rescale in the softmax warps and an issuer inside `if (lane == 0)`, cycles a block and tile: wait for the
+// scores 1360, load 86, maximum 430, rescale 770 (some row of 32 grows in nearly every block), exponentials 1540.  The rescale
+// now runs beside the exponentials and the issuer's whole warp stays converged (umma_f16_warp).  Measured, 32 query / 8 kv
+// heads of 128: 16384 tokens causal 2.19 -> 2.02 ms (1090 TFLOP/s, at the power cap: sustained, 4.28 -> 3.65 Mcycles at 1792 and
+// 1717 MHz), 8192 tokens in five sequences 200 -> 183 us, 2048 tokens 58 -> 52.  Taken back: the exponentials in four parts
+// instead of two (2.49 ms), a quarter of them by polynomial on the FMA pipe (2.17), two issuers (tiles drift into phase: 2.20;
+// with turns for the exponentials 2.03), four softmax warps a scheduler with half a row a thread (2.22).
 #include "../common/host_utils.cuh"
 #include "../common/ptx.cuh"
 #include "attn_common.cuh"
@@ -35,7 +39,7 @@ namespace {
 
 constexpr int BM = 128;  // queries per CTA
 constexpr int BNK = 128; // keys per block
-constexpr int ATT_THREADS = 384;
+constexpr int ATT_THREADS = 512;
 
 struct AttnParams {
   int T, Tk, nq, nkv, d;  // T queries, Tk keys
@@ -90,17 +94,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
   uint64_t* q_full = bars;            // 2, per tile
-  uint64_t* k_full = bars + 2;        // 2 stages
-  uint64_t* k_empty = bars + 4;       // 2
-  uint64_t* v_full = bars + 6;        // 2
-  uint64_t* v_empty = bars + 8;       // 2
-  uint64_t* s_full = bars + 10;       // 2, per tile
-  uint64_t* p_full = bars + 12;       // 2 x 2: halves of P (64 keys each), per tile
-  uint64_t* o_done = bars + 16;       // 2, per tile: a P V product has completed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+  uint64_t* kv_full = bars + 2;       // 2 stages: V of block j and K of block j + ahead
+  uint64_t* kv_empty = bars + 4;      // 2
+  uint64_t* s_full = bars + 6;        // 2, per tile
+  uint64_t* p_full = bars + 8;        // 2 x 2, per tile: halves of P (64 keys), the first with the accumulator rescaled
+  uint64_t* o_done = bars + 12;       // 2, per tile: all products have completed
+  uint64_t* f_full = bars + 14;       // 2 x 4, per tile and quarter of rows: the factors of a block's rescale are in s_fac
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int bx = blockIdx.x % p.per_row;
   const int mt = (gridDim.x - 1 - blockIdx.x) / p.per_row;   // long tiles of every head first: the tail gets short ones
   int head0, head1, m00, m01;
@@ -119,6 +122,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const bool split = p.pairing == SPLIT_KEYS;
   const int kvh = head0 / (p.nq / p.nkv);
   __shared__ int s_rng[2][8];
+  __shared__ float s_fac[2][BM];                // per tile and row: what its accumulator has to be multiplied by
   __shared__ float s_part[2][2][BM];            // SPLIT_KEYS: maxima and sums of the two groups
   tile_range_partial(p.k_lo, p.k_hi, m00, p.T, s_rng[0]);
   tile_range_partial(p.k_lo, p.k_hi, m01, p.T, s_rng[1]);
@@ -127,14 +131,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     *abort_flag = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&q_full[i]), 1);
-      mbar_init(smem_u32(&k_full[i]), 1);
-      mbar_init(smem_u32(&k_empty[i]), 1);
-      mbar_init(smem_u32(&v_full[i]), 1);
-      mbar_init(smem_u32(&v_empty[i]), 1);
+      mbar_init(smem_u32(&kv_full[i]), 1);
+      mbar_init(smem_u32(&kv_empty[i]), 1);
       mbar_init(smem_u32(&s_full[i]), 1);
-      mbar_init(smem_u32(&p_full[2 * i]), 4);
+      mbar_init(smem_u32(&p_full[2 * i]), 8);     // softmax and correction warps
       mbar_init(smem_u32(&p_full[2 * i + 1]), 4);
       mbar_init(smem_u32(&o_done[i]), 1);
+      for (int w = 0; w < 4; ++w) mbar_init(smem_u32(&f_full[4 * i + w]), 1);
     }
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -149,22 +152,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = warp_uniform(*tmem_slot);
   // key blocks [b0, b1) of each tile, and their union [jb, je)
   int b0[2], b1[2];
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
     const int kmin = tile_range_min(s_rng[t]), kmax = tile_range_max(s_rng[t]);
-    b0[t] = kmax >= kmin ? kmin / BNK : 0;
-    b1[t] = kmax >= kmin ? kmax / BNK + 1 : 0;
+    b0[t] = warp_uniform(kmax >= kmin ? kmin / BNK : 0);
+    b1[t] = warp_uniform(kmax >= kmin ? kmax / BNK + 1 : 0);
   }
   const bool any0 = b1[0] > b0[0], any1 = b1[1] > b0[1];
   const int jb = any0 ? (any1 ? min(b0[0], b0[1]) : b0[0]) : b0[1];
   const int je = max(b1[0], b1[1]);
+  // the scores of a group's next block replace the P of its previous one: one block on, in split mode two
+  const int ahead = split ? 2 : 1;
+  // in the key range of tile t, and in split mode its turn
+  auto takes = [&](int t, int j) {
+    return j >= b0[t] && j < b1[t] && (!split || ((j - jb) & 1) == t);
+  };
 
-  // 384 threads x 168 registers at launch: 128 x (104 + 200 + 200) = 64512
+  // 512 threads x 128 registers at launch = 128 x (64 + 192 + 192 + 64)
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0 && je > jb) {
@@ -177,22 +186,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           tma_load_2d(smem_u32(smem + L::OFF_Q + t * L::TILE + b * BM * 128), &tm_q, (t ? head1 : head0) * D + b * 64,
                       t ? m01 : m00, smem_u32(&q_full[t]));
       }
-      int n = 0, nv = 0;
-      for (int j = jb; j < je; ++j, ++n) {
+      int n = 0;
+      for (int j = jb - ahead; j < je; ++j, ++n) {
         const uint32_t st = n & 1, ph = (n >> 1) & 1;
-        if (!mbar_wait(smem_u32(&k_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
-        mbar_expect_tx(smem_u32(&k_full[st]), L::TILE);
+        if (!mbar_wait(smem_u32(&kv_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+        const bool has_v = j >= jb, has_k = j + ahead < je;
+        mbar_expect_tx(smem_u32(&kv_full[st]), (has_v + has_k) * L::TILE);
 #pragma unroll
         for (int b = 0; b < NBOX; ++b)
-          tma_load_2d(smem_u32(smem + L::OFF_K + st * L::TILE + b * BM * 128), &tm_k, kvh * D + b * 64, j * BNK,
-                      smem_u32(&k_full[st]));
-        if (!mbar_wait(smem_u32(&v_empty[st]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ++n; break; }
-        mbar_expect_tx(smem_u32(&v_full[st]), L::TILE);
+          if (has_v)
+            tma_load_2d(smem_u32(smem + L::OFF_V + st * L::TILE + b * BM * 128), &tm_v, kvh * D + b * 64, j * BNK,
+                        smem_u32(&kv_full[st]));
 #pragma unroll
         for (int b = 0; b < NBOX; ++b)
-          tma_load_2d(smem_u32(smem + L::OFF_V + st * L::TILE + b * BM * 128), &tm_v, kvh * D + b * 64, j * BNK,
-                      smem_u32(&v_full[st]));
-        ++nv;
+          if (has_k)
+            tma_load_2d(smem_u32(smem + L::OFF_K + st * L::TILE + b * BM * 128), &tm_k, kvh * D + b * 64,
+                        (j + ahead) * BNK, smem_u32(&kv_full[st]));
       }
       // drain: the last loads must land before the CTA exits
       auto drain = [](uint64_t* bar, uint32_t parity) {
@@ -200,94 +209,97 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         while (!mbar_try_wait(smem_u32(bar), parity))
           if (globaltimer_ns() - t0 > 200000000ull) break;
       };
-      for (int i = (n > 2 ? n - 2 : 0); i < n; ++i) drain(&k_full[i & 1], (i >> 1) & 1);
-      for (int i = (nv > 2 ? nv - 2 : 0); i < nv; ++i) drain(&v_full[i & 1], (i >> 1) & 1);
+      for (int i = (n > 2 ? n - 2 : 0); i < n; ++i) drain(&kv_full[i & 1], (i >> 1) & 1);
       if (any0) drain(&q_full[0], 0);
       if (any1 && !split) drain(&q_full[1], 0);
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && je > jb) {
+    // ------------------------------------------------------------------ MMA issuer: a whole warp, see umma_f16_warp
+    // Per stage and tile: P V of block j, then the scores of block j + ahead.
+    if (je > jb) {
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = idesc_bf16(BM, BNK, false);
       constexpr uint32_t idesc_o = idesc_bf16(BM, D, true);
-      auto product_qk = [&](uint32_t t, uint32_t qt, uint32_t st) {        // S_t = Q_qt K^T
-        tc_fence_after();
-        const uint32_t sq = smem_u32(smem + L::OFF_Q + qt * L::TILE);
-        const uint32_t sk = smem_u32(smem + L::OFF_K + st * L::TILE);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_S + t * BNK, kmajor_desc<D>(sq, kk), kmajor_desc<D>(sk, kk), idesc_s, kk ? 1u : 0u);
-      };
-      auto product_pv = [&](uint32_t t, uint32_t n, uint32_t st) -> bool {  // O_t += P_t V, its n-th
-        const uint32_t sv = smem_u32(smem + L::OFF_V + st * L::TILE);
-        for (int h = 0; h < 2; ++h) {            // the second half of the exponentials runs under the first half's product
-          if (!mbar_wait(smem_u32(&p_full[2 * t + h]), n & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
-          tc_fence_after();
-#pragma unroll
-          for (int k4 = 0; k4 < BNK / 32; ++k4) {
-            const int kk = h * (BNK / 32) + k4;
-            umma_f16_ts(tmem + COL_O + t * 128, tmem + COL_S + t * BNK + kk * 8,
-                        make_smem_desc_sw128(sv + kk * 2048, BM * 128, 1024), idesc_o, (n | kk) ? 1u : 0u);
-          }
-        }
-        return true;
-      };
       bool ok = true;
-      // order of a tile whose blocks go to both groups:  PV_t(j), QK_t(j + 2)  with t = j mod 2
-      for (int u = -2; split && u < je - jb; ++u) {
-        if (u >= 0) {
-          const uint32_t t = u & 1, n = u >> 1;
-          if (!mbar_wait(smem_u32(&v_full[t]), n & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) break;
-          if (!product_pv(t, n, t)) break;
-          umma_commit(smem_u32(&o_done[t]));
-          umma_commit(smem_u32(&v_empty[t]));
-        }
-        if (u + 2 < je - jb) {
-          const uint32_t t = u & 1, n = (u + 2) >> 1;
-          if (!mbar_wait(smem_u32(&k_full[t]), n & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) break;
-          if (u == -2 && !mbar_wait(smem_u32(&q_full[0]), 0, abort_flag, p.status, ST_TIMEOUT_FULL)) break;
-          product_qk(t, 0, t);
-          umma_commit(smem_u32(&s_full[t]));
-          umma_commit(smem_u32(&k_empty[t]));
-        }
-      }
-      for (int j = jb - 1; !split && j < je && ok; ++j) {
-        const uint32_t st = (j - jb) & 1, ph = ((j - jb) >> 1) & 1;          // V stage of block j
-        const uint32_t kst = (j + 1 - jb) & 1, kph = ((j + 1 - jb) >> 1) & 1;  // K stage of block j + 1
-        bool v_seen = false, k_seen = false;
+      if (any0) ok = mbar_wait_warp(smem_u32(&q_full[0]), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
+      if (any1 && !split) ok = ok && mbar_wait_warp(smem_u32(&q_full[1]), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
+      uint32_t np[2] = {0, 0};         // products P V issued, per tile
+#pragma unroll 1
+      for (int j = jb - ahead; j < je && ok; ++j) {
+        const uint32_t i = j - (jb - ahead), st = i & 1;
+        const uint32_t sv = smem_u32(smem + L::OFF_V + st * L::TILE), sk = smem_u32(smem + L::OFF_K + st * L::TILE);
+        ok = mbar_wait_warp(smem_u32(&kv_full[st]), (i >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          if (j >= b0[t] && j < b1[t]) {
-            const uint32_t n = j - b0[t];
-            if (!v_seen) {
-              if (!mbar_wait(smem_u32(&v_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-              v_seen = true;
+          const uint32_t ds = tmem + COL_S + t * BNK, dpv = tmem + COL_O + t * 128;
+          if (ok && takes(t, j)) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              ok = ok && mbar_wait_warp(smem_u32(&p_full[2 * t + h]), np[t] & 1, abort_flag, p.status, ST_TIMEOUT_FULL);
+              tc_fence_after();
+              if (ok) {
+#pragma unroll
+                for (int kk = 4 * h; kk < 4 * h + 4; ++kk)
+                  umma_f16_ts_warp(leader, dpv, ds + kk * 8, make_smem_desc_sw128(sv + kk * 2048, BM * 128, 1024), idesc_o,
+                                   (np[t] | kk) ? 1u : 0u);
+              }
             }
-            if (!product_pv(t, n, st)) { ok = false; break; }
-            umma_commit(smem_u32(&o_done[t]));
+            ++np[t];
           }
-          if (j + 1 >= b0[t] && j + 1 < b1[t]) {
-            if (!k_seen) {
-              if (!mbar_wait(smem_u32(&k_full[kst]), kph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-              k_seen = true;
-            }
-            if (j + 1 == b0[t] &&
-                !mbar_wait(smem_u32(&q_full[t]), 0, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-            product_qk(t, t, kst);
-            umma_commit(smem_u32(&s_full[t]));
+          if (ok && takes(t, j + ahead)) {
+            tc_fence_after();
+            const uint32_t sq = smem_u32(smem + L::OFF_Q + (split ? 0 : t) * L::TILE);
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk)
+              umma_f16_warp(leader, ds, kmajor_desc<D>(sq, kk), kmajor_desc<D>(sk, kk), idesc_s, kk ? 1u : 0u);
+            umma_commit_warp(leader, smem_u32(&s_full[t]));
           }
         }
-        // a block neither tile needs (ranges with a gap between them) must have landed too before its stage is reused
-        if (ok && j >= jb && !v_seen) ok = mbar_wait(smem_u32(&v_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL);
-        if (ok && j + 1 < je && !k_seen) ok = mbar_wait(smem_u32(&k_full[kst]), kph, abort_flag, p.status, ST_TIMEOUT_FULL);
-        if (!ok) break;
-        if (j >= jb) umma_commit(smem_u32(&v_empty[st]));
-        if (j + 1 < je) umma_commit(smem_u32(&k_empty[kst]));
+        umma_commit_warp(leader, smem_u32(&kv_empty[st]));
       }
+      umma_commit_warp(leader, smem_u32(&o_done[0]));
+      umma_commit_warp(leader, smem_u32(&o_done[1]));
     }
   }
+  } else if (warp >= 12) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    // ------------------------------------------------------------------ correction warps: thread = query row of both tiles
+    // The scores of block n exist, so every product issued before them for the tile, P V of block n - 1 included, has
+    // completed; P V of block n waits for the arrival here.  Blocks are taken in the issuer's order.
+    const int q = warp & 3, r = q * 32 + lane;
+    const uint32_t lane_addr = uint32_t(q * 32) << 16;
+    bool ok = true;
+    int np[2] = {0, 0};
+    for (int j = jb; j < je && ok; ++j) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (!takes(t, j)) continue;
+        if (np[t] && ok) {
+          ok = mbar_wait_warp(smem_u32(&f_full[4 * t + q]), (np[t] & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+          const float f = s_fac[t][r];
+          if (ok && __any_sync(0xffffffffu, f != 1.f)) {
+            const uint32_t to = tmem + lane_addr + COL_O + t * 128;
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < D; c += 32) {
+              uint32_t o[32];
+              tmem_ld_32x32(to + c, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+              tmem_st_32x32(to + c, o);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+          }
+        }
+        ++np[t];
+        __syncwarp();
+        if (lane == 0 && ok) mbar_arrive(smem_u32(&p_full[2 * t]));
+      }
+    }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
     // ------------------------------------------------------------------ softmax warps: thread = query row
     const int q = warp & 3;
     const int t = (warp - 4) >> 2;
@@ -306,26 +318,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     float mref = -INFINITY;                       // reference maximum, log2 units
     uint64_t sum2 = 0;                            // two fp32 partial row sums
     bool ok = true;
+#pragma unroll 1
     for (int n = 0; n < blocks && ok; ++n) {
-      const int j = jfirst + n * jstep;
-      if (!mbar_wait(smem_u32(&s_full[t]), n & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      const int n0 = (jfirst + n * jstep) * BNK;
+      const bool full = __all_sync(0xffffffffu, lo <= n0 && n0 + BNK - 1 <= hi) && p.scale_log2 > 0.f;
+      const float mul = full ? p.scale_log2 : 1.f;  // what the scores in registers still have to be multiplied by
+      if (!mbar_wait_warp(smem_u32(&s_full[t]), n & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       uint32_t v[4][32];
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + 32 * c, v[c]);
       tmem_ld_wait();
-      const int n0 = j * BNK;
-      const bool full = __all_sync(0xffffffffu, lo <= n0 && n0 + BNK - 1 <= hi) && p.scale_log2 > 0.f;
-      float mx, mul = p.scale_log2;               // mul: what the scores in registers still have to be multiplied by
       if (!full) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int e = 0; e < 32; ++e)
-            v[c][e] = (unsigned)(n0 + 32 * c + e - lo) <= span ? __float_as_uint(__uint_as_float(v[c][e]) * mul)
-                                                               : 0xff800000u;
-        mul = 1.f;
+            v[c][e] = (unsigned)(n0 + 32 * c + e - lo) <= span
+                          ? __float_as_uint(__uint_as_float(v[c][e]) * p.scale_log2) : 0xff800000u;
       }
+      float mx;
       {
         float m4[4];
 #pragma unroll
@@ -336,46 +348,44 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * mul;
       }
-      if (mref == -INFINITY) {
-        mref = mx;                                // nothing accumulated yet (sum and accumulator are zero)
-      }
-      const bool grow = mx > mref;
-      if (__any_sync(0xffffffffu, grow)) {
-        // the accumulator must hold every product issued so far; P of this block has not been handed over yet
-        if (!mbar_wait(smem_u32(&o_done[t]), (n & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-        tc_fence_after();
-        const float f = grow ? ex2_ftz(mref - mx) : 1.f;
-        if (grow) mref = mx;
-        sum2 = mul_f32x2(sum2, f32x2(f, f));
-#pragma unroll 1
-        for (int c = 0; c < D; c += 32) {
-          uint32_t o[32];
-          tmem_ld_32x32(to + c, o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-          tmem_st_32x32(to + c, o);
-        }
-      }
+      const float mold = mref == -INFINITY ? mx : mref;   // nothing accumulated yet: sum and accumulator are zero
+      mref = fmaxf(mold, mx);
       const float m2 = mref == -INFINITY ? 0.f : mref;
       const uint64_t cc = f32x2(mul, mul), mm = f32x2(-m2, -m2);
+      uint64_t add2 = 0;
 #pragma unroll
-      for (int c = 0; c < 4; c += 2) {
-        uint32_t pk[32];
+      for (int c = 0; c < 4; ++c) {
+        uint32_t pk[16];
 #pragma unroll
-        for (int e = 0; e < 64; e += 2) {
-          const float2 x = f32x2_split(fma_f32x2(
-              f32x2(__uint_as_float(v[c + (e >> 5)][e & 31]), __uint_as_float(v[c + (e >> 5)][(e & 31) + 1])), cc, mm));
+        for (int e = 0; e < 32; e += 2) {
+          const uint64_t x2 = fma_f32x2(f32x2(__uint_as_float(v[c][e]), __uint_as_float(v[c][e + 1])), cc, mm);
+          const float2 x = f32x2_split(x2);
           const float e0 = ex2_ftz(x.x), e1 = ex2_ftz(x.y);
-          sum2 = add_f32x2(sum2, f32x2(e0, e1));
+          add2 = add_f32x2(add2, f32x2(e0, e1));
           pk[e >> 1] = pack_bf16x2(e0, e1);
         }
-        tmem_st_32x32(ts + 16 * c, pk);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&p_full[2 * t + (c >> 1)]));
+        if (c == 2) {                             // the first half's stores have had the time of a quarter of the block
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&p_full[2 * t]));
+        }
+        tmem_st_32x16(ts + 16 * c, pk);
+        if (c == 0) {                             // after the first exponentials: the correction warps have time
+          const float f = mold == mref ? 1.f : ex2_ftz(mold - mref);
+          if (n) {
+            s_fac[t][r] = f;                      // read before P V of this block, which the next scores wait for
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&f_full[4 * t + q]));
+          }
+          sum2 = mul_f32x2(sum2, f32x2(f, f));
+        }
       }
+      sum2 = add_f32x2(sum2, add2);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&p_full[2 * t + 1]));
     }
     const float2 sp = f32x2_split(sum2);
     float sum = sp.x + sp.y, fold = 1.f, fold2 = 0.f;       // what this group's accumulator, and the other's, counts for
@@ -409,9 +419,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int c = c0; c < c1; c += 8) *reinterpret_cast<uint4*>(orow + c) = make_uint4(0, 0, 0, 0);
       }
     } else {
-      if (blocks > 0 && ok) ok = mbar_wait(smem_u32(&o_done[t]), (blocks - 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
-      if (blocks2 > 0 && ok)
-        ok = mbar_wait(smem_u32(&o_done[t ^ 1]), (blocks2 - 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+      if (blocks > 0 && ok) ok = mbar_wait(smem_u32(&o_done[t]), 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+      if (blocks2 > 0 && ok) ok = mbar_wait(smem_u32(&o_done[t ^ 1]), 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
       const uint32_t to2 = tmem + lane_addr + COL_O + (t ^ 1) * 128;

@@ -83,6 +83,7 @@ __device__ __forceinline__ uint64_t wait_limit_ns(const int* status) {
 // shared by every role of the CTA; `status` is the kernel's global status word.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
                                           int code) {
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;  // keeps the loop below out of the callers' way
   uint64_t t0 = 0;
   for (uint32_t it = 0; it < 0x7fffffffu; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -91,6 +92,42 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
       uint64_t now = globaltimer_ns();
       if (t0 == 0) t0 = now;
       if (now - t0 > wait_limit_ns(status)) break;
+    }
+  }
+  *abort_flag = 1;
+  if (status) atomicCAS(status, 0, code);
+  return false;
+}
+
+// ---------------------------------------------------------------- issuing with a whole warp
+// A tcgen05 instruction takes its descriptors and addresses from uniform registers.  Inside `if (lane == 0)` they are
+// computed per thread and moved over one by one, about 85 cycles for each MMA where the tensor core needs 64 for
+// 128 x 128 x 16; in a warp that stays converged they are computed there, and one elected lane issues by predicate.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(e));
+  return e;
+}
+// A value all lanes hold, in a form that is uniform for the compiler too.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+// mbar_wait by all lanes of a converged warp; the result is the same in all of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                               int code) {
+  if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
+  uint64_t t0 = 0;
+  for (uint32_t it = 0; it < 0x7fffffffu; ++it) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((it & 0x3ffu) == 0x3ffu) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      if (__any_sync(0xffffffffu, now - t0 > wait_limit_ns(status))) break;
     }
   }
   *abort_flag = 1;
@@ -158,6 +195,19 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// as umma_f16, by a converged warp: the lane with `leader` set issues
+__device__ __forceinline__ void umma_f16_warp(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                              uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
 // fp8 (e4m3/e5m2) inputs, fp32 accumulate
 __device__ __forceinline__ void umma_f8f6f4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
@@ -173,6 +223,16 @@ __device__ __forceinline__ void umma_f8f6f4(uint32_t d_tmem, uint64_t adesc, uin
 // Arrive on an mbarrier once every tcgen05.mma issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void umma_commit_warp(uint32_t leader, uint32_t bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %1, 0;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar), "r"(leader)
+      : "memory");
 }
 
 // 32 lanes x 32 consecutive fp32 columns: thread t of the warp gets lane (base_lane + t).
@@ -224,6 +284,18 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
       "}\n" ::"r"(d_tmem),
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_ts_warp(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
+                                                 uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 
