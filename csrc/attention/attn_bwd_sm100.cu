@@ -20,9 +20,10 @@
 // values of the next blocks, warps 4..11 element-wise: thread = TMEM lane = query row in dq, key row in dk/dv; warps
 // 4..7 take columns 0..63 of every block, warps 8..11 columns 64..127, so that a block's latency is half a block's
 // arithmetic.  The tensor core is kept busy by the order of the products, not by second buffers (see each kernel).
-// Every wait is bounded and reports through the status buffer.  Measured, 32 query / 8 kv heads of 128, causal: 8192 tokens
-// in four segments 0.58 ms = 597 TFLOP/s, one 16384-token segment 7.35 ms = 748 TFLOP/s; with 64-row blocks and P / dS
-// through shared memory the latter ran at 411 TFLOP/s.
+// Every wait is bounded and reports through the status buffer.  The issuer is a whole converged warp (umma_f16_warp): a block's
+// 24 (dq) or 32 (dk/dv) MMAs issued by `if (lane == 0)` took longer than the tensor core needs for them.  Measured, delta to
+// dK/dV, 32 query / 8 kv heads of 128, causal: one 16384-token segment 7.19 -> 6.38 ms (861 TFLOP/s counting five products), 8192
+// tokens in five segments 621 -> 559 us; 3000 tokens, 9 / 3 heads 262 -> 216.
 #include <climits>
 
 #include "../common/host_utils.cuh"
@@ -193,7 +194,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int m_tile = (gridDim.x - 1 - blockIdx.x) / p.nq;      // long tiles of every head first
   const int head = blockIdx.x % p.nq;
   const int kvh = head / (p.nq / p.nkv);
@@ -231,8 +232,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-  const int kmin = tile_range_min(s_rng), kmax = tile_range_max(s_rng);
+  const uint32_t tmem = warp_uniform(*tmem_slot);
+  const int kmin = warp_uniform(tile_range_min(s_rng)), kmax = warp_uniform(tile_range_max(s_rng));
   const int kb0 = kmin / TM;
   const int nblk = kmax >= kmin ? kmax / TM - kb0 + 1 : 0;
 
@@ -269,53 +270,54 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       for (int i = (nk > 3 ? nk - 3 : 0); i < nk; ++i) drain(&k_full[i % 3], (i / 3) & 1);
       for (int i = (nv > 2 ? nv - 2 : 0); i < nv; ++i) drain(&v_full[i & 1], (i >> 1) & 1);
       drain(q_full, 0);
-    } else if (warp == 1 && lane == 0 && nblk > 0) {
-      // ---------------------------------------------------------------- MMA issuer
+    } else if (warp == 1 && nblk > 0) {
+      // ---------------------------------------------------------------- MMA issuer: a whole warp, see umma_f16_warp
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = idesc(TM, TM, false);
       constexpr uint32_t idesc_dq = idesc(TM, D, true);
       const uint32_t sq = smem_u32(smem + L::OFF_Q), sdo = smem_u32(smem + L::OFF_DO);
       auto issue_s = [&](int j) -> bool {
         const uint32_t ks = j % 3, kp = (j / 3) & 1;
-        if (!mbar_wait(smem_u32(&k_full[ks]), kp, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
+        if (!mbar_wait_warp(smem_u32(&k_full[ks]), kp, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
         const uint32_t sk = smem_u32(smem + L::OFF_K + ks * L::TILE);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_S + (j & 1) * TM, kdesc(sq, kk, TM), kdesc(sk, kk, TM), idesc_s, kk ? 1u : 0u);
-        umma_commit(smem_u32(&s_full[j & 1]));
+          umma_f16_warp(leader, tmem + COL_S + (j & 1) * TM, kdesc(sq, kk, TM), kdesc(sk, kk, TM), idesc_s, kk ? 1u : 0u);
+        umma_commit_warp(leader, smem_u32(&s_full[j & 1]));
         return true;
       };
       auto issue_dp = [&](int j) -> bool {
         const uint32_t vs = j & 1, vp = (j >> 1) & 1;
-        if (!mbar_wait(smem_u32(&v_full[vs]), vp, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
-        if (j > 0 && !mbar_wait(smem_u32(dp_empty), (j & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
+        if (!mbar_wait_warp(smem_u32(&v_full[vs]), vp, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
+        if (j > 0 && !mbar_wait_warp(smem_u32(dp_empty), (j & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
         tc_fence_after();
         const uint32_t sv = smem_u32(smem + L::OFF_V + vs * L::TILE);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_DP, kdesc(sdo, kk, TM), kdesc(sv, kk, TM), idesc_s, kk ? 1u : 0u);
-        umma_commit(smem_u32(dp_full));
-        umma_commit(smem_u32(&v_empty[vs]));
+          umma_f16_warp(leader, tmem + COL_DP, kdesc(sdo, kk, TM), kdesc(sv, kk, TM), idesc_s, kk ? 1u : 0u);
+        umma_commit_warp(leader, smem_u32(dp_full));
+        umma_commit_warp(leader, smem_u32(&v_empty[vs]));
         return true;
       };
-      bool ok = mbar_wait(smem_u32(q_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
+      bool ok = mbar_wait_warp(smem_u32(q_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
       if (ok) ok = issue_s(0);
       if (ok) ok = issue_dp(0);
       if (ok && nblk > 1) ok = issue_s(1);
       for (int j = 0; j < nblk && ok; ++j) {
         if (j + 1 < nblk && !issue_dp(j + 1)) { ok = false; break; }
-        if (!mbar_wait(smem_u32(ds_full), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(smem_u32(ds_full), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sk = smem_u32(smem + L::OFF_K + (j % 3) * L::TILE);
         const uint32_t ads = tmem + COL_S + (j & 1) * TM;
 #pragma unroll
         for (int kk = 0; kk < TM / 16; ++kk)     // dS: 32 packed columns at the start of each 64-column half
-          umma_f16_ts(tmem + COL_DQ, ads + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sk, kk, TM), idesc_dq,
+          umma_f16_ts_warp(leader, tmem + COL_DQ, ads + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sk, kk, TM), idesc_dq,
                       (j | kk) ? 1u : 0u);
-        umma_commit(smem_u32(&k_empty[j % 3]));
+        umma_commit_warp(leader, smem_u32(&k_empty[j % 3]));
         if (j + 2 < nblk) ok = issue_s(j + 2);
       }
-      if (ok) umma_commit(smem_u32(dq_full));
+      if (ok) umma_commit_warp(leader, smem_u32(dq_full));
     }
   } else {
     MCB_REGS_MATH();
@@ -449,7 +451,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* i_end_slot = reinterpret_cast<int*>(tmem_slot + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int group_cta = blockIdx.x % (p.nkv * p.splits);         // key tiles ascend slowest: long ones first when causal
   const int kvh = group_cta / p.splits, split = group_cta % p.splits;
   const int qpg = p.nq / p.nkv;
@@ -499,9 +501,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-  const int i_first = p.q_lo ? tile_range_min(s_rng) : i_end_slot[0];
-  const int i_last = p.q_lo ? min(tile_range_max(s_rng), p.T - 1) : i_end_slot[1];
+  const uint32_t tmem = warp_uniform(*tmem_slot);
+  const int i_first = warp_uniform(p.q_lo ? tile_range_min(s_rng) : i_end_slot[0]);
+  const int i_last = warp_uniform(p.q_lo ? min(tile_range_max(s_rng), p.T - 1) : i_end_slot[1]);
   const int qb0 = i_first / TM;
   const int nqb = i_last >= i_first ? i_last / TM - qb0 + 1 : 0;    // 0: no query sees a key of this tile
   const int hps = qpg / p.splits;                 // query heads handled by this CTA
@@ -541,54 +543,55 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       for (int i = (nQ > 2 ? nQ - 2 : 0); i < nQ; ++i) drain(&q_full[i & 1], (i >> 1) & 1);
       for (int i = (nD > 2 ? nD - 2 : 0); i < nD; ++i) drain(&do_full[i & 1], (i >> 1) & 1);
       drain(kv_full, 0);
-    } else if (warp == 1 && lane == 0 && iters > 0) {
-      // ---------------------------------------------------------------- MMA issuer
+    } else if (warp == 1 && iters > 0) {
+      // ---------------------------------------------------------------- MMA issuer: a whole warp, see umma_f16_warp
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = idesc(TM, TM, false);
       constexpr uint32_t idesc_o = idesc(TM, D, true);
       const uint32_t sk = smem_u32(smem + L::OFF_K), sv = smem_u32(smem + L::OFF_V);
       auto issue_s = [&](int it) -> bool {
-        if (!mbar_wait(smem_u32(&q_full[it & 1]), (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
+        if (!mbar_wait_warp(smem_u32(&q_full[it & 1]), (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
         const uint32_t sq = smem_u32(smem + L::OFF_Q + (it & 1) * L::TILE);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_S, kdesc(sk, kk, TM), kdesc(sq, kk, TM), idesc_s, kk ? 1u : 0u);
-        umma_commit(smem_u32(s_full));
+          umma_f16_warp(leader, tmem + COL_S, kdesc(sk, kk, TM), kdesc(sq, kk, TM), idesc_s, kk ? 1u : 0u);
+        umma_commit_warp(leader, smem_u32(s_full));
         return true;
       };
-      bool ok = mbar_wait(smem_u32(kv_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
+      bool ok = mbar_wait_warp(smem_u32(kv_full), 0, abort_flag, p.status, ST_TIMEOUT_FULL);
       if (ok) ok = issue_s(0);
       for (int it = 0; it < iters && ok; ++it) {
         const uint32_t st = it & 1, ph = (it >> 1) & 1;
         const uint32_t sq = smem_u32(smem + L::OFF_Q + st * L::TILE);
         const uint32_t sdo = smem_u32(smem + L::OFF_DO + st * L::TILE);
-        if (!mbar_wait(smem_u32(&do_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(smem_u32(&do_full[st]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tmem + COL_DP, kdesc(sv, kk, TM), kdesc(sdo, kk, TM), idesc_s, kk ? 1u : 0u);
-        umma_commit(smem_u32(dp_full));
+          umma_f16_warp(leader, tmem + COL_DP, kdesc(sv, kk, TM), kdesc(sdo, kk, TM), idesc_s, kk ? 1u : 0u);
+        umma_commit_warp(leader, smem_u32(dp_full));
         // P, dS: 32 packed columns at the start of each 64-column half; part u of them is ready first in both halves
         auto product = [&](uint32_t col_d, uint32_t col_a, uint32_t sb, uint64_t* full) -> bool {
           for (int u = 0; u < 2; ++u) {
-            if (!mbar_wait(smem_u32(&full[u]), it & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
+            if (!mbar_wait_warp(smem_u32(&full[u]), it & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
             tc_fence_after();
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
               const int kk = (v >> 1) * 4 + u * 2 + (v & 1);
-              umma_f16_ts(tmem + col_d, tmem + col_a + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sb, kk, TM), idesc_o,
+              umma_f16_ts_warp(leader, tmem + col_d, tmem + col_a + (kk >> 2) * HALF + (kk & 3) * 8, mndesc(sb, kk, TM), idesc_o,
                           (it | u | v) ? 1u : 0u);
             }
           }
           return true;
         };
         if (!product(COL_DV, COL_S, sdo, p_full)) { ok = false; break; }
-        umma_commit(smem_u32(&do_empty[st]));
+        umma_commit_warp(leader, smem_u32(&do_empty[st]));
         if (it + 1 < iters && !issue_s(it + 1)) { ok = false; break; }
         if (!product(COL_DK, COL_DP, sq, ds_full)) { ok = false; break; }
-        umma_commit(smem_u32(&q_empty[st]));
+        umma_commit_warp(leader, smem_u32(&q_empty[st]));
       }
-      if (ok) umma_commit(smem_u32(out_full));
+      if (ok) umma_commit_warp(leader, smem_u32(out_full));
     } else if (warp == 2) {
       // ---------------------------------------------------------------- per-query values of the coming blocks
       int h = h_first, qb = 0;
