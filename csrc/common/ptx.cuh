@@ -350,6 +350,28 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t adesc, u
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// as umma_f16_pair, by a converged warp of the leader CTA: the lane with `leader` set issues
+__device__ __forceinline__ void umma_f16_pair_warp(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                                   uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair_warp(uint32_t leader, uint32_t bar_cluster_addr) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %1, 0;\n"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar_cluster_addr), "r"(leader)
+      : "memory");
+}
 // Arrive on one mbarrier (shared::cluster address, possibly in the peer CTA) once every pair MMA issued so far by this
 // thread has completed.
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {

@@ -53,7 +53,7 @@ cudaError_t launch_pair_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const
   return launch_pair<true, false>(ta, tb, p, grid, s);
 }
 
-// CTA pairs (256 x 256 tiles) pay off once there are enough tiles to fill the 74 clusters a few times over; small or
+// CTA pairs (256 x 256 tiles; 8192 x 4096 x 4096 171 us against 183 of the 256-wide single-CTA tiles) pay off once there are enough tiles to fill the 74 clusters a few times over; small or
 // skinny problems keep the single-CTA tiles, whose narrower variants quantise better.
 bool use_pair(int M, int N, int K, int mode, int sms) {
   if (mode != GEMM_DENSE || M < 512 || N < 256 || K < 128) return false;
@@ -61,9 +61,13 @@ bool use_pair(int M, int N, int K, int mode, int sms) {
   return tiles >= (sms / 2);
 }
 
-int pick_bn(int M, int N, int groups, int sms) {
+// Tile width that finishes first: waves x width x the time of a column against that of the 256-wide tile, which is the shared
+// memory a narrower tile reads per product.  Measured at 8192 x 4096 x 4096, us at 256 / 128 / 64: both operands K-major 183 /
+// 225 / 429, B MN-major 185 / 270 / 452, both MN-major 200 / 315 / 534.
+int pick_bn(int M, int N, int groups, int mn_major, int sms) {
   const int cand[3] = {256, 128, 64};
-  const float penalty[3] = {1.0f, 1.8f, 3.0f};  // measured: 128-wide tiles reach ~55% of the 256-wide rate
+  constexpr float kPenalty[3][3] = {{1.0f, 1.25f, 2.35f}, {1.0f, 1.45f, 2.45f}, {1.0f, 1.6f, 2.7f}};
+  const float* penalty = kPenalty[mn_major];
   int best = 256;
   float best_cost = 1e30f;
   for (int i = 0; i < 3; ++i) {
@@ -103,7 +107,7 @@ int mcb_gemm_bf16(const void* A, long long a_inner, long long a_outer, long long
   // force_bn: 0 = choose; 64 / 128 / 256 = single-CTA tile width; 512 = CTA pairs (256 x 256 per cluster)
   const bool pair = force_bn == 512 || (force_bn == 0 && use_pair(M, N, K, mode, sms));
   if (pair && mode != GEMM_DENSE) return -4;
-  int bn = pair ? PAIR_HALF_N : (force_bn > 0 ? force_bn : pick_bn(M, N, groups, sms));
+  int bn = pair ? PAIR_HALF_N : (force_bn > 0 ? force_bn : pick_bn(M, N, groups, (a_mn != 0) + (b_mn != 0), sms));
   if (bn != 256 && bn != 128 && bn != 64) return -4;
 
   CUtensorMap ta, tb;

@@ -13,6 +13,10 @@
 //
 // Warp roles (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner,
 // warps 2..5 = epilogue (each owns the 32 TMEM lanes its warp id % 4 selects).
+//
+// The issuer is a whole converged warp (umma_f16_warp).  One thread under `if (lane == 0)` took about 85 cycles for an MMA, more
+// than a 128-wide tile (64 cycles) or a 64-wide one leaves it and close to the 128 of the widest: us before and after, 8192 x
+// 4096 x 4096 128-wide 309 / 225, 64-wide 528 / 429, CTA pairs 185 / 171; 773 x 2048 x 12288 63 / 46; 64 x 4096 x 4096 25 / 19.
 #pragma once
 #include "../common/ptx.cuh"
 
@@ -311,7 +315,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   __shared__ int s_off[GEMM_MAX_GROUPS + 1];
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   if (p.mode != GEMM_DENSE) {
@@ -339,7 +343,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   TileScheduler sched(p, s_off, BN);
 
@@ -390,22 +394,24 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // ------------------------------------------------------------ MMA issuer: a whole warp, see umma_f16_warp
+    {
       constexpr uint32_t idesc = make_idesc_bf16(GEMM_BM, BN, A_MN, B_MN);
+      const uint32_t leader = elect_one();
       uint32_t it = 0, lt = 0;
       bool ok = true;
+#pragma unroll 1
       for (int t = blockIdx.x; t < sched.total && ok; t += gridDim.x) {
-        TileCoord c = sched.get(t);
-        if (!c.valid || c.k_end <= c.k_begin) continue;
+        const TileCoord c = sched.get(t);
+        const int k_blocks = warp_uniform(c.valid && c.k_end > c.k_begin ? (c.k_end - c.k_begin + GEMM_BK - 1) / GEMM_BK : 0);
+        if (k_blocks == 0) continue;
         const uint32_t acc = lt & 1, aph = (lt >> 1) & 1;
-        if (!mbar_wait(smem_u32(&tempty_bar[acc]), aph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
+        if (!mbar_wait_warp(smem_u32(&tempty_bar[acc]), aph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
         const uint32_t d_tmem = tmem_base + acc * BN;
-        bool first = true;
-        for (int k = c.k_begin; k < c.k_end; k += GEMM_BK, ++it) {
+#pragma unroll 1
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) {
+          if (!mbar_wait_warp(smem_u32(&full_bar[s]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) {
             ok = false;
             break;
           }
@@ -415,16 +421,15 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 #pragma unroll
           for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
             // K-major: 16 bf16 = 32 B inside the swizzle row.  MN-major: 16 k-rows = 2048 B.
-            uint64_t ad = A_MN ? make_smem_desc_sw128(sa + kk * 2048, 8192, 1024)
-                               : make_smem_desc_sw128(sa + kk * 32, 16, 1024);
-            uint64_t bd = B_MN ? make_smem_desc_sw128(sb + kk * 2048, 8192, 1024)
-                               : make_smem_desc_sw128(sb + kk * 32, 16, 1024);
-            umma_f16(d_tmem, ad, bd, idesc, first ? 0u : 1u);
-            first = false;
+            const uint64_t ad = A_MN ? make_smem_desc_sw128(sa + kk * 2048, 8192, 1024)
+                                     : make_smem_desc_sw128(sa + kk * 32, 16, 1024);
+            const uint64_t bd = B_MN ? make_smem_desc_sw128(sb + kk * 2048, 8192, 1024)
+                                     : make_smem_desc_sw128(sb + kk * 32, 16, 1024);
+            umma_f16_warp(leader, d_tmem, ad, bd, idesc, (kb | kk) ? 1u : 0u);
           }
-          umma_commit(smem_u32(&empty_bar[s]));  // frees the smem stage when these MMAs retire
+          umma_commit_warp(leader, smem_u32(&empty_bar[s]));  // frees the smem stage when these MMAs retire
         }
-        if (ok) umma_commit(smem_u32(&tfull_bar[acc]));
+        if (ok) umma_commit_warp(leader, smem_u32(&tfull_bar[acc]));
         ++lt;
       }
     }

@@ -44,7 +44,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();       // 0 = leader
   const uint32_t peer = cta ^ 1u;
   const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
@@ -72,7 +72,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   __syncthreads();
   cluster_sync_all();      // the peer's barriers exist before anything of this CTA can signal them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   const int tiles_m = (p.M + PAIR_BM - 1) / PAIR_BM;
   const int tiles_n = (p.N + PAIR_BN - 1) / PAIR_BN;
@@ -135,20 +135,22 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && cta == 0) {
+    // ------------------------------------------------------------ MMA issuer: a whole warp of the leader CTA
+    if (cta == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(PAIR_BM, PAIR_BN, A_MN, B_MN);
+      const uint32_t leader = elect_one();
       uint32_t it = 0, lt = 0;
       bool ok = true;
+#pragma unroll 1
       for (int t = cluster_id; t < total && ok; t += num_clusters, ++lt) {
         const uint32_t acc = lt & 1, aph = (lt >> 1) & 1;
-        if (!mbar_wait(smem_u32(&tempty_bar[acc]), aph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
+        if (!mbar_wait_warp(smem_u32(&tempty_bar[acc]), aph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * PAIR_BN;
-        bool first = true;
+#pragma unroll 1
         for (int k = 0; k < p.K; k += GEMM_BK, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) {
+          if (!mbar_wait_warp(smem_u32(&full_bar[s]), ph, abort_flag, p.status, ST_TIMEOUT_FULL)) {
             ok = false;
             break;
           }
@@ -161,16 +163,15 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                                      : make_smem_desc_sw128(sa + kk * 32, 16, 1024);
             const uint64_t bd = B_MN ? make_smem_desc_sw128(sb + kk * 2048, 8192, 1024)
                                      : make_smem_desc_sw128(sb + kk * 32, 16, 1024);
-            umma_f16_pair(d_tmem, ad, bd, idesc, first ? 0u : 1u);
-            first = false;
+            umma_f16_pair_warp(leader, d_tmem, ad, bd, idesc, (k | kk) ? 1u : 0u);
           }
           // the stage is free in both CTAs once these MMAs retire
-          umma_commit_pair(smem_u32(&empty_bar[s]));
-          umma_commit_pair(mapa_shared(smem_u32(&empty_bar[s]), peer));
+          umma_commit_pair_warp(leader, smem_u32(&empty_bar[s]));
+          umma_commit_pair_warp(leader, mapa_shared(smem_u32(&empty_bar[s]), peer));
         }
         if (ok) {
-          umma_commit_pair(smem_u32(&tfull_bar[acc]));
-          umma_commit_pair(mapa_shared(smem_u32(&tfull_bar[acc]), peer));
+          umma_commit_pair_warp(leader, smem_u32(&tfull_bar[acc]));
+          umma_commit_pair_warp(leader, mapa_shared(smem_u32(&tfull_bar[acc]), peer));
         }
       }
     }
