@@ -53,7 +53,8 @@ cudaError_t launch_pair_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const
   return launch_pair<true, false>(ta, tb, p, grid, s);
 }
 
-// CTA pairs (256 x 256 tiles; 8192 x 4096 x 4096 171 us against 183 of the 256-wide single-CTA tiles) pay off once there are enough tiles to fill the 74 clusters a few times over; small or
+// CTA pairs (256 x 256 tiles; 8192 x 4096 x 4096 171 us against 183 of the 256-wide single-CTA tiles) pay off once there
+// are enough tiles to fill the 74 clusters a few times over; small or
 // skinny problems keep the single-CTA tiles, whose narrower variants quantise better.
 bool use_pair(int M, int N, int K, int mode, int sms) {
   if (mode != GEMM_DENSE || M < 512 || N < 256 || K < 128) return false;
@@ -148,9 +149,10 @@ int mcb_gemm_bf16(const void* A, long long a_inner, long long a_outer, long long
 }
 
 // Fused language-model head on the GEMM engine: logits = A[M,K] . B[N,K]^T (both K-major) are consumed by the
-// epilogue and never stored.
+// epilogue.
 //   grad == 0: `part` [M, ceil(N/256), 2] receives per row and 256-column tile (max, sum exp(logit - max)); `tgt` [M]
-//              the logit of the row's label when its column is in [col0, col0 + N) (untouched otherwise: zero it first)
+//              the logit of the row's label when its column is in [col0, col0 + N) (untouched otherwise: zero it first);
+//              C null, or [M, N] fp32 for the logits (N and ldc multiples of 4, C on a 16-byte boundary)
 //   grad != 0: C [M, N] bf16 = (exp(logit - lse[row]) - [col0 + column == label]) * g[row]
 int mcb_gemm_ce_bf16(const void* A, long long lda, const void* B, long long ldb, int M, int N, int K,
                      const long long* labels, int col0, float* part, float* tgt, const float* lse, const float* g,
@@ -160,6 +162,7 @@ int mcb_gemm_ce_bf16(const void* A, long long lda, const void* B, long long ldb,
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
   if (labels == nullptr || (grad ? (C == nullptr || lse == nullptr || g == nullptr) : (part == nullptr || tgt == nullptr)))
     return -2;
+  if (!grad && C != nullptr && (N % 4 || ldc % 4 || (reinterpret_cast<uintptr_t>(C) & 15))) return -5;
   constexpr int BN = 256;
   const int sms = device_sm_count();
   // The gradient epilogue only: 4096 rows, 32000 columns, us, pairs and single CTAs, at K = 256 200 / 198, 512 219 / 222, 1024

@@ -28,9 +28,10 @@ constexpr int GEMM_THREADS = 192;
 constexpr int GEMM_MAX_GROUPS = 512;
 
 enum GemmMode : int { GEMM_DENSE = 0, GEMM_GROUPED_M = 1, GEMM_GROUPED_K = 2 };
-// Epilogues.  The cross-entropy ones belong to the fused language-model head (logits = h . W^T are never stored):
+// Epilogues.  The cross-entropy ones belong to the fused language-model head (logits = h . W^T):
 //   EPI_CE_STATS  per row and column tile, the running maximum and sum of exp(logit - max) over the tile's columns go
-//                 to `ce_part`, and the logit of the row's label (when its column lies in the tile) to `ce_tgt`
+//                 to `ce_part`, and the logit of the row's label (when its column lies in the tile) to `ce_tgt`; with C
+//                 the logits themselves go there in fp32
 //   EPI_CE_GRAD   C = (exp(logit - lse[row]) - [column == label]) * g[row] in bf16: the gradient w.r.t. the logits
 enum GemmEpilogue : int { EPI_NONE = 0, EPI_CE_STATS = 2, EPI_CE_GRAD = 3 };
 
@@ -162,8 +163,11 @@ __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* 
 
 // Epilogue of the fused language-model head for one row of a BN-column tile (one thread owns the row): running soft-max
 // statistics of the row's logits and the label's logit (EPI_CE_STATS), or the logits' gradient as bf16 (EPI_CE_GRAD).
+// With p.C the statistics epilogue also keeps the logits, fp32 and rounded nowhere, for a backward pass that then needs no second
+// product; they leave through `stage` (4 KiB a warp) as 128-byte rows, see epilogue_store_bf16.
 template <int BN, int EPI>
-__device__ __forceinline__ void epilogue_ce(const GemmParams& p, uint32_t tmem_row, int row, bool row_ok, int n0, int tiles_n) {
+__device__ __forceinline__ void epilogue_ce(const GemmParams& p, uint32_t tmem_row, int row, bool row_ok, int n0, int tiles_n,
+                                            uint8_t* stage) {
   constexpr float LOG2E = 1.4426950408889634f;
   const bool vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
   const int label_col = row_ok ? (int)(p.ce_labels[row] - p.ce_col0) - n0 : -1;   // column inside this tile
@@ -176,6 +180,25 @@ __device__ __forceinline__ void epilogue_ce(const GemmParams& p, uint32_t tmem_r
     uint32_t r[32];
     tmem_ld_32x32(tmem_row + cc, r);
     tmem_ld_wait();
+    if constexpr (EPI == EPI_CE_STATS) {
+      if (p.C) {                                   // N and ldc are multiples of 4 then
+        const int lane = threadIdx.x & 31, row0 = row - lane;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<uint4*>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+              make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        __syncwarp();
+        const int j = lane & 7, col = n0 + cc + 4 * j;
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const int rr = it * 4 + (lane >> 3);
+          const uint4 o = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((j ^ (rr & 7)) << 4));
+          if (row0 + rr < p.M && col < p.N)
+            *reinterpret_cast<uint4*>(reinterpret_cast<float*>(p.C) + (long long)(row0 + rr) * p.ldc + col) = o;
+        }
+        __syncwarp();
+      }
+    }
     if (!row_ok) continue;
     const int valid = min(32, p.N - (n0 + cc));
     if constexpr (EPI == EPI_CE_STATS) {
@@ -456,7 +479,8 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                  : nullptr;
       const bool vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
       if constexpr (EPI == EPI_CE_STATS || EPI == EPI_CE_GRAD) {
-        epilogue_ce<BN, EPI>(p, tmem_base + (uint32_t(q * 32) << 16) + acc * BN, row, row_ok, c.n0, sched.tiles_n);
+        epilogue_ce<BN, EPI>(p, tmem_base + (uint32_t(q * 32) << 16) + acc * BN, row, row_ok, c.n0, sched.tiles_n,
+                             smem + STAGES * L::STAGE_BYTES + L::BAR_BYTES + q * EPI_STAGE_WARP);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

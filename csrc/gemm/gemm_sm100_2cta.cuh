@@ -191,7 +191,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const bool row_ok = row < p.M;
       const int n0 = tn * PAIR_BN;
       if constexpr (EPI == EPI_CE_GRAD) {
-        epilogue_ce<PAIR_BN, EPI>(p, tmem_base + (uint32_t(q * 32) << 16) + acc * PAIR_BN, row, row_ok, n0, tiles_n);
+        epilogue_ce<PAIR_BN, EPI>(p, tmem_base + (uint32_t(q * 32) << 16) + acc * PAIR_BN, row, row_ok, n0, tiles_n,
+                                   nullptr);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(acc ? tempty_leader1 : tempty_leader0);

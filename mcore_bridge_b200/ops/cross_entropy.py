@@ -3,13 +3,14 @@
 * :func:`vocab_parallel_cross_entropy` — logits sharded on the vocab dim; max / sum-exp / target-logit
   reduced over the tensor-parallel group (parity: the ``compute_language_model_loss`` call at reference
   ``src/mcore_bridge/model/gpt_model.py:577``).
-* :func:`fused_linear_cross_entropy` — never materialises the logits.  On a GPU the head GEMM's epilogue reduces
+* :func:`fused_linear_cross_entropy` — the head and the loss in one.  On a GPU the head GEMM's epilogue reduces
   every 128 x 256 accumulator tile to per-row (max, sum-exp) partials and picks out the label's logit
   (``csrc/gemm``, ``EPI_CE_STATS``); the partials of a row are combined, the tensor-parallel ranks exchange their
   ``[T]`` statistics through peer memory (``parallel/dp_comm.py`` all-gather kernel; ``torch.distributed`` elsewhere)
-  and the loss follows.  Backward runs the head GEMM again per token chunk with an epilogue that writes the
-  gradient of the logits directly in bf16 (``EPI_CE_GRAD``) and feeds it to the two gradient GEMMs.  Only ``[T]``
-  statistics are kept between forward and backward.  On CPU the same chunked algorithm runs on torch ops.
+  and the loss follows.  Backward turns the logits, which the forward pass keeps in fp32 while memory is plentiful, into
+  their gradient per token chunk and feeds it to the two gradient GEMMs; otherwise only ``[T]`` statistics are kept and
+  the head GEMM runs again with an epilogue that writes that gradient directly in bf16 (``EPI_CE_GRAD``).  On CPU the
+  same chunked algorithm runs on torch ops.
 
 Both return the per-token loss ``[T]`` in fp32 (the caller masks and averages).
 """
@@ -132,8 +133,33 @@ def _head_kernel_ok(h2, weight) -> bool:
             and h2.shape[1] % 8 == 0 and weight.is_contiguous())
 
 
-def _head_stats(h2, weight, lab, vocab_start):
-    """(max, sum exp, label logit) of every row over the local vocabulary shard, from the GEMM epilogue."""
+_KEEP_MIN_HIDDEN = 1024
+
+
+def _logits_to_keep(T, vl, H, device):
+    """A ``[T, vl]`` fp32 buffer that saves the backward pass the second head product, or ``None``.
+
+    A kept logit costs 8 bytes of traffic and 4 of memory until the backward pass, a recomputed one ``2 H`` operations: at
+    6.5 TB/s and 1.4 PFLOP/s the two are even near ``H`` = 860.  Forward + backward, us, recomputed and kept: 4096 x 151936
+    at ``H`` 4096 14808 / 12990, 2048 7173 / 6743, 1024 4420 / 3941; 64 x 151936 at 4096 1347 / 1165.  Buffers above 256 MB
+    are kept only where the device has four times as much to spare, so that what fits into memory does not depend on it."""
+    if T == 0 or vl % 8 or H < _KEEP_MIN_HIDDEN:
+        return None
+    need = 4 * T * vl
+    if need > 1 << 28:
+        stats = torch.cuda.memory_stats_as_nested_dict(device)
+        cached = stats['reserved_bytes']['all']['current'] - stats['allocated_bytes']['all']['current']
+        if torch.cuda.mem_get_info(device)[0] + cached < 4 * need:
+            return None
+    try:
+        return torch.empty((T, vl), dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:       # free, but in pieces
+        return None
+
+
+def _head_stats(h2, weight, lab, vocab_start, logits=None):
+    """(max, sum exp, label logit) of every row over the local vocabulary shard, from the GEMM epilogue; the logits go to
+    ``logits`` when that is given."""
     T, H = h2.shape
     vl = weight.shape[0]
     tiles_n = (vl + 255) // 256
@@ -141,8 +167,8 @@ def _head_stats(h2, weight, lab, vocab_start):
     tgt = torch.zeros(T, dtype=torch.float32, device=h2.device)
     rc = _lib.lib().mcb_gemm_ce_bf16(_lib.ptr(h2), _ll(h2.stride(0)), _lib.ptr(weight), _ll(weight.stride(0)), _int(T),
                                      _int(vl), _int(H), _lib.ptr(lab), _int(vocab_start), _lib.ptr(part), _lib.ptr(tgt),
-                                     None, None, None, _ll(0), _int(0), _lib.ptr(_lib.status_word(h2.device)),
-                                     _lib.stream_ptr())
+                                     None, None, _lib.ptr(logits), _ll(vl), _int(0),
+                                     _lib.ptr(_lib.status_word(h2.device)), _lib.stream_ptr())
     _lib.check_rc(rc, 'mcb_gemm_ce_bf16')
     m_t, s_t = part[..., 0], part[..., 1]
     m = m_t.max(dim=1).values
@@ -200,7 +226,9 @@ class _FusedLinearCE(torch.autograd.Function):
         if h2.stride(1) != 1 or h2.stride(0) % 8:
             h2 = h2.contiguous()
         if _head_kernel_ok(h2, weight):
-            m, s, tgt = _head_stats(h2, weight, lab, r * vl)
+            # not a saved tensor: hooks that move those to the host would move far more than the product costs
+            ctx.logits = _logits_to_keep(T, vl, H, h2.device) if any(ctx.needs_input_grad) else None
+            m, s, tgt = _head_stats(h2, weight, lab, r * vl, ctx.logits)
             lse_all, tgt = _combine(m, s, tgt, group_name, group)
             ctx.save_for_backward(h2, weight, lab, lse_all)
             ctx.meta = (group_name, chunk, r * vl, h.shape, labels.shape)
@@ -233,6 +261,7 @@ class _FusedLinearCE(torch.autograd.Function):
         need_dw = ctx.needs_input_grad[1]
         ddt = h2.dtype if h2.dtype == torch.bfloat16 else torch.float32
         fused = _head_kernel_ok(h2, weight)
+        kept, ctx.logits = getattr(ctx, 'logits', None), None   # a second pass over the graph forms them again
         # without `main_grad` the chunks' products are summed in fp32 and rounded once; a single chunk needs no such
         # buffer (at 151936 x 4096 it costs 2.5 GB of zero fill, accumulation and conversion), its GEMM rounds itself
         one_chunk = 0 < T <= chunk and mg is None and weight.dtype in (torch.bfloat16, torch.float32)
@@ -241,7 +270,9 @@ class _FusedLinearCE(torch.autograd.Function):
             dw = alloc(weight.shape, dtype=torch.float32, device=weight.device)
         for s0 in range(0, T, chunk):
             s1 = min(T, s0 + chunk)
-            if fused:
+            if kept is not None:
+                d = _dlogits(kept[s0:s1], lab[s0:s1], vstart, lse[s0:s1], g[s0:s1], h2.dtype)
+            elif fused:
                 d = _head_dlogits(h2[s0:s1], weight, lab[s0:s1], vstart, lse[s0:s1], g[s0:s1])
             else:
                 logits = gemm.mm_nt(h2[s0:s1], weight, out_dtype=torch.float32)
@@ -253,6 +284,7 @@ class _FusedLinearCE(torch.autograd.Function):
             elif need_dw:
                 gemm.mm_tn(d, h2[s0:s1], out=mg if mg is not None else dw, accumulate=mg is not None or s0 > 0)
             del d
+        del kept
         # dh is this vocab shard's partial gradient: the caller's input mapping (copy-to-region or
         # sequence-parallel gather) sums it over the tensor-parallel group in its own backward.
         if need_dw and mg is not None:

@@ -1,0 +1,70 @@
+"""Results that a backward pass forms again or finds kept, tile widths of the GEMM, growing maxima in attention: at the sizes
+where they can go wrong, against 64-bit references."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = 'cuda'
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp(min=1e-30)).item()
+
+
+@pytest.mark.parametrize('T,V,H,chunk', [(515, 4104, 1024, 4096),      # ragged rows, a last column tile with 8 columns
+                                         (1, 264, 1032, 4096),
+                                         (1030, 2056, 1024, 600)])     # two chunks of kept logits
+def test_head_loss_with_kept_logits(T, V, H, chunk):
+    from mcore_bridge_b200.ops import cross_entropy as ce
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    h = torch.randn(T, H, generator=gen, device=DEV).bfloat16().requires_grad_()
+    w = (torch.randn(V, H, generator=gen, device=DEV) * 0.05).bfloat16().requires_grad_()
+    lab = torch.randint(0, V, (T,), generator=gen, device=DEV)
+    lab[0] = V - 1
+    g = torch.rand(T, generator=gen, device=DEV)
+    assert ce._logits_to_keep(T, V, H, h.device) is not None
+    loss = ce.fused_linear_cross_entropy(h, w, lab, chunk=chunk)
+    kept = torch.autograd.grad(loss, (h, w), g, retain_graph=True)
+    again = torch.autograd.grad(loss, (h, w), g)                        # the logits are gone: formed a second time
+    hw, ww = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(hw @ ww.t(), lab, reduction='none')
+    want = torch.autograd.grad(ref, (hw, ww), g.double())
+    # logits and their sums are fp32; dlogits and the results are rounded to bf16, 2^-9 each
+    assert (loss.double() - ref).abs().max() < 1e-4
+    for got in (kept, again):
+        assert _rel(got[0], want[0]) < 2 ** -8 and _rel(got[1], want[1]) < 2 ** -8
+
+
+@pytest.mark.parametrize('M,N,K', [(1, 8, 8), (129, 264, 72), (300, 1000, 64), (520, 2056, 200)])
+def test_gemm_tile_widths_agree(M, N, K):
+    """Every width adds the same products in the same order; operands of both layouts, remainders in all three extents."""
+    from mcore_bridge_b200.ops import gemm
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    x = torch.randn(M, K, generator=gen, device=DEV).bfloat16()
+    w = torch.randn(N, K, generator=gen, device=DEV).bfloat16()
+    dy = torch.randn(M, N, generator=gen, device=DEV).bfloat16()
+    ref = {'nt': x.double() @ w.double().t(), 'nn': dy.double() @ w.double(), 'tn': dy.double().t() @ x.double()}
+    for bn in (0, 64, 128, 256, 512):
+        got = {'nt': gemm.mm_nt(x, w, force_bn=bn), 'nn': gemm.mm_nn(dy, w, force_bn=bn),
+               'tn': gemm.mm_tn(dy, x, force_bn=bn)}
+        for k, r in ref.items():
+            # fp32 sums of at most 2056 products (1e-5 of their size), rounded to bf16
+            assert ((got[k].double() - r).abs() <= 2 ** -8 * r.abs() + 1e-3).all(), (k, bn)
+
+
+@pytest.mark.parametrize('T,nq,nkv,d', [(300, 2, 1, 64), (2500, 3, 1, 128), (3000, 32, 8, 128)])
+def test_attention_maxima_that_grow_with_every_block(T, nq, nkv, d):
+    """Every block raises the maxima of its rows, which rescales every accumulator every time; split tiles, pairs of heads."""
+    from mcore_bridge_b200.ops.attention import attention
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    q = torch.rand(T, nq, d, generator=gen, device=DEV).bfloat16() + 0.5
+    ramp = torch.linspace(0.1, 2.0, T, device=DEV)[:, None, None]
+    k = (torch.rand(T, nkv, d, generator=gen, device=DEV) * ramp).bfloat16()
+    v = torch.randn(T, nkv, d, generator=gen, device=DEV).bfloat16()
+    o = attention(q, k, v)
+    kk, vv = (t.double().repeat_interleave(nq // nkv, dim=1).transpose(0, 1) for t in (k, v))
+    mask = torch.ones(T, T, dtype=torch.bool, device=DEV).triu(1)
+    for h in range(nq):
+        s = (q[:, h].double() @ kk[h].t() * d ** -0.5).masked_fill(mask, float('-inf'))
+        # probabilities and the result are rounded to bf16, 2^-9 each
+        assert _rel(o[:, h], torch.softmax(s, dim=-1) @ vv[h]) < 2 ** -8
