@@ -1,13 +1,13 @@
 """Activation-lean fused blocks for the single-rank (no tensor parallel) dense path.
 
 ``norm_linear``:  ``y = rmsnorm(x) @ W^T`` that keeps ``x`` and the per-row ``rstd`` for backward instead of the
-normalised activation, and re-runs the (memory-bound, ~30 us) norm in backward for the weight gradient.
-``glu_linear``:   ``y = glu(h) @ W^T`` that keeps ``h`` only and re-runs the gated activation in backward.
+normalised activation, which the norm's backward kernel forms again for the weight gradient.
+``glu_linear``:   ``y = glu(h) @ W^T`` that keeps ``h`` only; the gated activation comes out of its backward kernel.
 
 Per Qwen3-8B layer and 8192 tokens this drops 2 x 67 MB (normalised inputs of QKV and FC1) and 201 MB (SwiGLU output)
 from what autograd holds, about 30 % of a layer's activations, which is what lets a single 180 GB GPU keep almost all
 layers' activations instead of recomputing a third of the forward pass.  Results are bit-identical to the unfused
-sequence (the recomputed tensors come from the same kernels on the same inputs).
+sequence (the recomputed tensors are the same expressions of the same inputs, written over the gradient they follow).
 """
 from __future__ import annotations
 
@@ -21,11 +21,10 @@ from .linear import _weight_grad
 _ll, _int, _f = ctypes.c_longlong, ctypes.c_int, ctypes.c_float
 
 
-def _rmsnorm_raw(x2, w, eps, zc, rstd=None):
+def _rmsnorm_raw(x2, w, eps, zc):
     rows, H = x2.shape
     y = torch.empty((rows, H), dtype=x2.dtype, device=x2.device)
-    if rstd is None:
-        rstd = torch.empty(rows, dtype=torch.float32, device=x2.device)
+    rstd = torch.empty(rows, dtype=torch.float32, device=x2.device)
     rc = _lib.lib().mcb_rmsnorm_fwd(_lib.ptr(x2), None, _lib.ptr(w), _lib.ptr(y), None, _lib.ptr(rstd), _ll(rows),
                                     _int(H), _ll(x2.stride(0)), _f(eps), _int(int(zc)), _lib.stream_ptr())
     _lib.check_rc(rc, 'mcb_rmsnorm_fwd')
@@ -62,20 +61,17 @@ class _NormLinearFn(torch.autograd.Function):
         dy2 = dy.reshape(rows, weight.shape[0])
         if dy2.stride(-1) != 1:
             dy2 = dy2.contiguous()
-        dw = None
-        if ctx.needs_input_grad[2]:
-            xn, _ = _rmsnorm_raw(x2, ln_w, ctx.eps, ctx.zc, rstd)
-            dw = _weight_grad(weight, dy2, xn)
-            del xn
         dxn = gemm.mm_nn(dy2, weight)
         dx = torch.empty((rows, H), dtype=x2.dtype, device=x2.device)
         dlw = (torch.empty if rows else torch.zeros)(H, dtype=ln_w.dtype, device=x2.device)
         part = torch.empty((_lib.lib().mcb_rmsnorm_bwd_partial_rows(_ll(rows), _int(H)), H), dtype=torch.float32,
                            device=x2.device)
-        rc = _lib.lib().mcb_rmsnorm_bwd_det(_lib.ptr(dxn), _lib.ptr(x2), _lib.ptr(ln_w), _lib.ptr(rstd), None,
-                                            _lib.ptr(dx), _lib.ptr(dlw), _int(1), _lib.ptr(part), _ll(rows), _int(H),
-                                            _ll(x2.stride(0)), _f(ctx.eps), _int(int(ctx.zc)), _lib.stream_ptr())
+        need_dw = ctx.needs_input_grad[2]
+        fn = _lib.lib().mcb_rmsnorm_bwd_det_y if need_dw else _lib.lib().mcb_rmsnorm_bwd_det
+        rc = fn(_lib.ptr(dxn), _lib.ptr(x2), _lib.ptr(ln_w), _lib.ptr(rstd), None, _lib.ptr(dx), _lib.ptr(dlw), _int(1),
+                _lib.ptr(part), _ll(rows), _int(H), _ll(x2.stride(0)), _f(ctx.eps), _int(int(ctx.zc)), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_rmsnorm_bwd_det')
+        dw = _weight_grad(weight, dy2, dxn) if need_dw else None   # dxn is the normalised input by now
         return dx.view(ctx.shape), dlw, dw, None, None
 
 
@@ -101,16 +97,14 @@ class _GluLinearFn(torch.autograd.Function):
         dy2 = dy.reshape(rows, weight.shape[0])
         if dy2.stride(-1) != 1:
             dy2 = dy2.contiguous()
-        dw = None
-        if ctx.needs_input_grad[1]:
-            a = _glu_raw(h2, kind, clamp, offset)
-            dw = _weight_grad(weight, dy2, a)
-            del a
         da = gemm.mm_nn(dy2, weight)
         dh = torch.empty((rows, F2), dtype=h2.dtype, device=h2.device)
-        rc = _lib.lib().mcb_glu_bwd(_lib.ptr(h2), None, _lib.ptr(da), _lib.ptr(dh), None, _ll(rows), _int(F2 // 2),
-                                    _ll(h2.stride(0)), _int(kind), _f(clamp), _f(offset), _lib.stream_ptr())
+        need_dw = ctx.needs_input_grad[1]
+        fn = _lib.lib().mcb_glu_bwd_act if need_dw else _lib.lib().mcb_glu_bwd
+        rc = fn(_lib.ptr(h2), None, _lib.ptr(da), _lib.ptr(dh), None, _ll(rows), _int(F2 // 2), _ll(h2.stride(0)),
+                _int(kind), _f(clamp), _f(offset), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_glu_bwd')
+        dw = _weight_grad(weight, dy2, da) if need_dw else None    # da is the activation by now
         return dh.view(shape), dw, None, None, None
 
 

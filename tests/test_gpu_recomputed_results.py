@@ -35,6 +35,43 @@ def test_head_loss_with_kept_logits(T, V, H, chunk):
         assert _rel(got[0], want[0]) < 2 ** -8 and _rel(got[1], want[1]) < 2 ** -8
 
 
+@pytest.mark.parametrize('rows', [1, 7, 130])
+@pytest.mark.parametrize('H', [264, 1032, 4104])       # one, one and several vectors a thread, the last ones partly idle
+def test_norm_linear_recomputes_the_normalised_input(rows, H):
+    from mcore_bridge_b200.ops import fused_mlp
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    x = torch.randn(rows, H, generator=gen, device=DEV).bfloat16().requires_grad_()
+    lw = (1 + 0.1 * torch.randn(H, generator=gen, device=DEV)).bfloat16().requires_grad_()
+    w = (torch.randn(72, H, generator=gen, device=DEV) * 0.05).bfloat16().requires_grad_()
+    dy = torch.randn(rows, 72, generator=gen, device=DEV).bfloat16()
+    y = fused_mlp.norm_linear(x, lw, w, 1e-6, False)
+    got = [y, *torch.autograd.grad(y, (x, lw, w), dy)]
+    xd, ld, wd = (t.detach().double().requires_grad_() for t in (x, lw, w))
+    ref = (xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * ld) @ wd.t()
+    want = [ref, *torch.autograd.grad(ref, (xd, ld, wd), dy.double())]
+    # at most the normalised input, its gradient and the result are rounded to bf16: 3 x 2^-9
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 2 ** -7
+
+
+@pytest.mark.parametrize('rows', [1, 7, 130])
+@pytest.mark.parametrize('F', [264, 1536])
+def test_glu_linear_recomputes_the_activation(rows, F):
+    from mcore_bridge_b200.ops import fused_mlp
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    h = torch.randn(rows, 2 * F, generator=gen, device=DEV).bfloat16().requires_grad_()
+    w = (torch.randn(72, F, generator=gen, device=DEV) * 0.05).bfloat16().requires_grad_()
+    dy = torch.randn(rows, 72, generator=gen, device=DEV).bfloat16()
+    y = fused_mlp.glu_linear(h, w, 0, 0.0, 0.0)
+    got = [y, *torch.autograd.grad(y, (h, w), dy)]
+    hd, wd = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    gate, up = hd.chunk(2, dim=-1)
+    ref = (torch.nn.functional.silu(gate) * up) @ wd.t()
+    want = [ref, *torch.autograd.grad(ref, (hd, wd), dy.double())]
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 2 ** -7
+
+
 @pytest.mark.parametrize('M,N,K', [(1, 8, 8), (129, 264, 72), (300, 1000, 64), (520, 2056, 200)])
 def test_gemm_tile_widths_agree(M, N, K):
     """Every width adds the same products in the same order; operands of both layouts, remainders in all three extents."""
