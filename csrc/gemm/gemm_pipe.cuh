@@ -64,6 +64,31 @@ __device__ __forceinline__ void issue_mma_tile(Pipe<BN>& P, uint32_t d_tmem, int
   }
 }
 
+// issue_mma_tile by a whole converged warp (see umma_f16_warp); false when a wait gave up
+template <int BN, bool B_MN>
+__device__ __forceinline__ bool issue_mma_tile_warp(uint32_t leader, Pipe<BN>& P, uint32_t d_tmem, int K, uint32_t& it,
+                                                    int* status) {
+  using L = GemmSmem<BN>;
+  constexpr uint32_t idesc = make_idesc_bf16(GEMM_BM, BN, false, B_MN);
+#pragma unroll 1
+  for (int k = 0; k < K; k += GEMM_BK, ++it) {
+    const uint32_t s = it % L::STAGES, ph = (it / L::STAGES) & 1;
+    if (!mbar_wait_warp(smem_u32(&P.full_bar[s]), ph, P.abort_flag, status, ST_TIMEOUT_FULL)) return false;
+    tc_fence_after();
+    const uint32_t sa = smem_u32(P.smem + s * L::STAGE_BYTES);
+    const uint32_t sb = sa + L::A_BYTES;
+#pragma unroll
+    for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
+      const uint64_t ad = make_smem_desc_sw128(sa + kk * 32, 16, 1024);
+      const uint64_t bd = B_MN ? make_smem_desc_sw128(sb + kk * 2048, 8192, 1024)
+                               : make_smem_desc_sw128(sb + kk * 32, 16, 1024);
+      umma_f16_warp(leader, d_tmem, ad, bd, idesc, (k | kk) ? 1u : 0u);
+    }
+    umma_commit_warp(leader, smem_u32(&P.empty_bar[s]));
+  }
+  return true;
+}
+
 template <int BN, bool B_MN>
 __device__ __forceinline__ bool load_tile(Pipe<BN>& P, const CUtensorMap* ta, const CUtensorMap* tb, int a_row, int n0,
                                           int K, uint32_t& it, int* status, int b_k_base = 0) {

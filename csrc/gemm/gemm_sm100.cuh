@@ -123,18 +123,24 @@ constexpr int EPI_STAGE_BYTES = 4 * EPI_STAGE_WARP;
 // contiguous bytes of a row, four rows per instruction: an eighth of the transactions.  Short contractions (expert weight
 // gradients: 4 to 6 k-blocks per tile) were bound by the former: 128 experts x (1536 + 768) x 2048, 256 rows each,
 // 757 -> 466 us.
-template <int BN>
+// WIDE = 64 columns at a time (4 KiB of shared memory per warp) or 32 (2 KiB, 64 contiguous bytes a row).
+template <int BN, int WIDE = 64>
 __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* stage, __nv_bfloat16* C, long long ldc, int row0,
                                                     int m_limit, int n0, int N, float alpha, const __nv_bfloat16* bias) {
   const int lane = threadIdx.x & 31;
+  constexpr int CH = WIDE / 8;                   // 16-byte chunks of a row
+  auto at = [&](int row, int j) {                // chunks of a row are permuted so that neither side has bank conflicts
+    return stage + row * (WIDE * 2) + ((j ^ (WIDE == 64 ? row & 7 : (row >> 1) & 3)) << 4);
+  };
 #pragma unroll 1
-  for (int cc = 0; cc < BN; cc += 64) {
+  for (int cc = 0; cc < BN; cc += WIDE) {
     if (n0 + cc >= N) break;
-    uint32_t r[64];
-    tmem_ld_32x32_x64(tmem_row + cc, r);
+    uint32_t r[WIDE];
+    if constexpr (WIDE == 64) tmem_ld_32x32_x64(tmem_row + cc, r);
+    else tmem_ld_32x32(tmem_row + cc, r);
     tmem_ld_wait();
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < CH; ++j) {
       float v[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]) * alpha;
@@ -147,14 +153,14 @@ __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* 
       o.y = pack_bf16x2(v[2], v[3]);
       o.z = pack_bf16x2(v[4], v[5]);
       o.w = pack_bf16x2(v[6], v[7]);
-      *reinterpret_cast<uint4*>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) = o;
+      *reinterpret_cast<uint4*>(at(lane, j)) = o;
     }
     __syncwarp();
-    const int j = lane & 7, col = n0 + cc + 8 * j;
+    const int j = lane % CH, col = n0 + cc + 8 * j;
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const int rr = it * 4 + (lane >> 3);
-      const uint4 o = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((j ^ (rr & 7)) << 4));
+    for (int it = 0; it < CH; ++it) {
+      const int rr = it * (32 / CH) + lane / CH;
+      const uint4 o = *reinterpret_cast<const uint4*>(at(rr, j));
       if (row0 + rr < m_limit && col < N) *reinterpret_cast<uint4*>(C + (long long)(row0 + rr) * ldc + col) = o;
     }
     __syncwarp();

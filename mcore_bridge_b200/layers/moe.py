@@ -204,7 +204,7 @@ class TopKRouter(nn.Module):
             else:
                 sc = scores if valid is None else scores * valid[:, None]
                 counts = moe_ops.tokens_per_expert(idx, self.num_experts, valid)
-                ntok = torch.tensor(float(scores.shape[0]), device=x.device) if valid is None else valid.sum().float()
+                ntok = torch.full((), float(scores.shape[0]), device=x.device) if valid is None else valid.sum().float()
                 group = 'tp_dp_cp' if lb == 'global_aux_loss' else ('tp_cp' if cfg.sequence_parallel or
                                                                     cfg.context_parallel_size > 1 else None)
                 if group is not None and ps.get_world_size(group) > 1:
@@ -469,7 +469,7 @@ class MoELayer(nn.Module):
                     r.local_tokens_per_expert += counts.float()
             coeff = cfg.moe_aux_loss_coeff
             if self.training and coeff and lb in ('aux_loss', 'global_aux_loss'):
-                ntok = torch.tensor(float(T), device=x.device) if valid is None else valid.sum().float()
+                ntok = torch.full((), float(T), device=x.device) if valid is None else valid.sum().float()
                 cnt = counts.float()
                 group = 'tp_dp_cp' if lb == 'global_aux_loss' else ('tp_cp' if cfg.sequence_parallel or
                                                                     cfg.context_parallel_size > 1 else None)

@@ -105,3 +105,31 @@ def test_attention_maxima_that_grow_with_every_block(T, nq, nkv, d):
         s = (q[:, h].double() @ kk[h].t() * d ** -0.5).masked_fill(mask, float('-inf'))
         # probabilities and the result are rounded to bf16, 2^-9 each
         assert _rel(o[:, h], torch.softmax(s, dim=-1) @ vv[h]) < 2 ** -8
+
+
+@pytest.mark.parametrize('hidden,ffn', [(192, 320), (128, 64)])         # 2.5 and half a column tile
+def test_expert_widths_that_end_inside_a_tile(monkeypatch, hidden, ffn):
+    """Results of the gather + expert GEMM leave through shared memory."""
+    from mcore_bridge_b200.layers.moe import MoELayer
+    from mcore_bridge_b200.ops import _lib
+    from mcore_bridge_b200.train.presets import model_config
+    cfg = model_config('qwen3_moe_tiny', dict(hidden_size=hidden, moe_intermediate_size=ffn, num_experts=8,
+                                              num_experts_per_tok=2), bf16=True)
+    gen = torch.Generator(device=DEV).manual_seed(6)
+    with torch.device(DEV):
+        layer = MoELayer(cfg).train()
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.copy_(torch.randn(p.shape, generator=gen, device=DEV) * 0.1)
+    x = torch.randn(333, hidden, generator=gen, device=DEV).bfloat16()
+    dy = torch.randn(333, hidden, generator=gen, device=DEV).bfloat16()
+    res = {}
+    for fused in ('1', '0'):
+        monkeypatch.setenv('MCB200_FUSED_MOE', fused)
+        xx = x.clone().requires_grad_()
+        y = layer(xx)
+        res[fused] = [y, *torch.autograd.grad(y, [xx, *layer.parameters()], dy)]
+    _lib.check_status()
+    # either path rounds the hidden rows, their activation, the expert outputs and the result to bf16: 4 x 2^-9 each
+    for a, b in zip(res['1'], res['0']):
+        assert _rel(a, b) < 2 ** -6
