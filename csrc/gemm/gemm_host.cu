@@ -63,11 +63,11 @@ bool use_pair(int M, int N, int K, int mode, int sms) {
 }
 
 // Tile width that finishes first: waves x width x the time of a column against that of the 256-wide tile, which is the shared
-// memory a narrower tile reads per product.  Measured at 8192 x 4096 x 4096, us at 256 / 128 / 64: both operands K-major 183 /
-// 225 / 429, B MN-major 185 / 270 / 452, both MN-major 200 / 315 / 534.
+// memory a narrower tile reads per product.  Measured at 8192 x 4096 x 4096, us at 256 / 128 / 64: both operands K-major 181 /
+// 204 / 271, B MN-major 179 / 203 / 278, both MN-major 206 / 232 / 357.
 int pick_bn(int M, int N, int groups, int mn_major, int sms) {
   const int cand[3] = {256, 128, 64};
-  constexpr float kPenalty[3][3] = {{1.0f, 1.25f, 2.35f}, {1.0f, 1.45f, 2.45f}, {1.0f, 1.6f, 2.7f}};
+  constexpr float kPenalty[3][3] = {{1.0f, 1.13f, 1.5f}, {1.0f, 1.13f, 1.55f}, {1.0f, 1.13f, 1.75f}};
   const float* penalty = kPenalty[mn_major];
   int best = 256;
   float best_cost = 1e30f;

@@ -111,6 +111,30 @@ __device__ __forceinline__ bool load_tile(Pipe<BN>& P, const CUtensorMap* ta, co
   return true;
 }
 
+// load_tile by a whole converged warp
+template <int BN, bool B_MN>
+__device__ __forceinline__ bool load_tile_warp(uint32_t leader, Pipe<BN>& P, const CUtensorMap* ta, const CUtensorMap* tb,
+                                               int a_row, int n0, int K, uint32_t& it, int* status, int b_k_base) {
+  using L = GemmSmem<BN>;
+#pragma unroll 1
+  for (int k = 0; k < K; k += GEMM_BK, ++it) {
+    const uint32_t s = it % L::STAGES, ph = (it / L::STAGES) & 1;
+    if (!mbar_wait_warp(smem_u32(&P.empty_bar[s]), ph ^ 1, P.abort_flag, status, ST_TIMEOUT_EMPTY)) return false;
+    const uint32_t fb = smem_u32(&P.full_bar[s]);
+    mbar_expect_tx_warp(leader, fb, L::STAGE_BYTES);
+    const uint32_t sa = smem_u32(P.smem + s * L::STAGE_BYTES);
+    const uint32_t sb = sa + L::A_BYTES;
+    tma_load_2d_warp(leader, sa, ta, k, a_row, fb);
+    if (!B_MN) {
+      tma_load_2d_warp(leader, sb, tb, k, n0, fb);
+    } else {
+#pragma unroll
+      for (int j = 0; j < BN / 64; ++j) tma_load_2d_warp(leader, sb + j * 8192, tb, n0 + j * 64, b_k_base + k, fb);
+    }
+  }
+  return true;
+}
+
 template <int BN>
 __device__ __forceinline__ void drain_loads(Pipe<BN>& P, uint32_t it) {
   using L = GemmSmem<BN>;

@@ -14,9 +14,11 @@
 // Warp roles (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner,
 // warps 2..5 = epilogue (each owns the 32 TMEM lanes its warp id % 4 selects).
 //
-// The issuer is a whole converged warp (umma_f16_warp).  One thread under `if (lane == 0)` took about 85 cycles for an MMA, more
-// than a 128-wide tile (64 cycles) or a 64-wide one leaves it and close to the 128 of the widest: us before and after, 8192 x
-// 4096 x 4096 128-wide 309 / 225, 64-wide 528 / 429, CTA pairs 185 / 171; 773 x 2048 x 12288 63 / 46; 64 x 4096 x 4096 25 / 19.
+// Issuer and producer are whole converged warps (umma_f16_warp).  One thread under `if (lane == 0)` took about 85 cycles for an MMA,
+// more than a 128-wide tile (64 cycles) or a 64-wide one leaves it and close to the 128 of the widest, and as long for each
+// TMA load, of which a k-block needs two to six.  us, one thread each / issuer converged / both: 8192 x 4096 x 4096 128-wide 309 /
+// 225 / 204, 64-wide 528 / 380 / 271, CTA pairs 185 / 171 / 171; 776 x 2048 x 12288 63 / 46 / 42, with B MN-major 63 / 53 / 39;
+// 512 x 512 x 4096 both MN-major 23 / 21 / 13.
 #pragma once
 #include "../common/ptx.cuh"
 
@@ -377,42 +379,46 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   TileScheduler sched(p, s_off, BN);
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // ------------------------------------------------------------ TMA producer: a whole warp, see umma_f16_warp
+    {
+      const uint32_t leader = elect_one();
       uint32_t it = 0;  // global k-block counter -> stage / phase
       bool ok = true;
+#pragma unroll 1
       for (int t = blockIdx.x; t < sched.total && ok; t += gridDim.x) {
-        TileCoord c = sched.get(t);
-        if (!c.valid) continue;
-        for (int k = c.k_begin; k < c.k_end; k += GEMM_BK, ++it) {
+        const TileCoord c = sched.get(t);
+        const int k_end = warp_uniform(c.valid ? c.k_end : c.k_begin), k_begin = warp_uniform(c.k_begin);
+        const int a_row0 = warp_uniform(c.a_row0), n0 = warp_uniform(c.n0);
+        const int b_row0 = warp_uniform(B_MN ? (p.mode == GEMM_GROUPED_M ? c.group * p.b_group_rows : 0) : c.b_row0);
+#pragma unroll 1
+        for (int k = k_begin; k < k_end; k += GEMM_BK, ++it) {
           const uint32_t s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) {
+          if (!mbar_wait_warp(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) {
             ok = false;
             break;
           }
           const uint32_t fb = smem_u32(&full_bar[s]);
-          mbar_expect_tx(fb, L::STAGE_BYTES);
+          mbar_expect_tx_warp(leader, fb, L::STAGE_BYTES);
           const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
           const uint32_t sb = sa + L::A_BYTES;
           if (!A_MN) {
-            tma_load_2d(sa, &tmap_a, k, c.a_row0, fb);
+            tma_load_2d_warp(leader, sa, &tmap_a, k, a_row0, fb);
           } else {
 #pragma unroll
-            for (int j = 0; j < GEMM_BM / 64; ++j) tma_load_2d(sa + j * 8192, &tmap_a, c.a_row0 + j * 64, k, fb);
+            for (int j = 0; j < GEMM_BM / 64; ++j)
+              tma_load_2d_warp(leader, sa + j * 8192, &tmap_a, a_row0 + j * 64, k, fb);
           }
           if (!B_MN) {
-            if (BN <= 256) tma_load_2d(sb, &tmap_b, k, c.b_row0, fb);
+            tma_load_2d_warp(leader, sb, &tmap_b, k, b_row0, fb);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j) {
-              int krow = (p.mode == GEMM_GROUPED_M) ? (c.group * p.b_group_rows + k) : k;
-              tma_load_2d(sb + j * 8192, &tmap_b, c.n0 + j * 64, krow, fb);
-            }
+            for (int j = 0; j < BN / 64; ++j)
+              tma_load_2d_warp(leader, sb + j * 8192, &tmap_b, n0 + j * 64, b_row0 + k, fb);
           }
         }
       }
-      // drain: every load this thread issued must have landed before the CTA may exit
+      // drain: every load this warp issued must have landed before the CTA may exit
       uint32_t first = it > STAGES ? it - STAGES : 0;
       for (uint32_t j = first; j < it; ++j) {
         const uint32_t s = j % STAGES, ph = (j / STAGES) & 1;
@@ -421,6 +427,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           if (globaltimer_ns() - t0 > 200000000ull) break;  // 0.2 s per stage, then give up
         }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer: a whole warp, see umma_f16_warp

@@ -90,37 +90,40 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   };
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    // ------------------------------------------------------------ TMA producer (both CTAs): a whole warp
+    {
+      const uint32_t leader = elect_one();
       uint32_t it = 0;
       bool ok = true;
+#pragma unroll 1
       for (int t = cluster_id; t < total && ok; t += num_clusters) {
         int tm, tn;
         tile_of(t, tm, tn);
         const int a_row0 = tm * PAIR_BM + (int)cta * GEMM_BM;          // this CTA's 128 rows of A / C
         const int b_row0 = tn * PAIR_BN + (int)cta * PAIR_HALF_N;      // this CTA's half of the tile's B rows
+#pragma unroll 1
         for (int k = 0; k < p.K; k += GEMM_BK, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) {
+          if (!mbar_wait_warp(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) {
             ok = false;
             break;
           }
           // bytes of both CTAs are counted on the leader's barrier
           const uint32_t fb = mapa_shared(smem_u32(&full_bar[s]), 0);
-          if (cta == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * PAIR_STAGE_BYTES);
+          if (cta == 0) mbar_expect_tx_warp(leader, smem_u32(&full_bar[s]), 2 * PAIR_STAGE_BYTES);
           const uint32_t sa = smem_u32(smem + s * PAIR_STAGE_BYTES);
           const uint32_t sb = sa + PAIR_A_BYTES;
           if (!A_MN) {
-            tma_load_2d_pair(sa, &tmap_a, k, a_row0, fb);
+            tma_load_2d_pair_warp(leader, sa, &tmap_a, k, a_row0, fb);
           } else {
 #pragma unroll
-            for (int j = 0; j < GEMM_BM / 64; ++j) tma_load_2d_pair(sa + j * 8192, &tmap_a, a_row0 + j * 64, k, fb);
+            for (int j = 0; j < GEMM_BM / 64; ++j) tma_load_2d_pair_warp(leader, sa + j * 8192, &tmap_a, a_row0 + j * 64, k, fb);
           }
           if (!B_MN) {
-            tma_load_2d_pair(sb, &tmap_b, k, b_row0, fb);
+            tma_load_2d_pair_warp(leader, sb, &tmap_b, k, b_row0, fb);
           } else {
 #pragma unroll
-            for (int j = 0; j < PAIR_HALF_N / 64; ++j) tma_load_2d_pair(sb + j * 8192, &tmap_b, b_row0 + j * 64, k, fb);
+            for (int j = 0; j < PAIR_HALF_N / 64; ++j) tma_load_2d_pair_warp(leader, sb + j * 8192, &tmap_b, b_row0 + j * 64, k, fb);
           }
         }
       }
@@ -133,6 +136,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           if (*abort_flag || globaltimer_ns() - t0 > 200000000ull) break;
         }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer: a whole warp of the leader CTA
