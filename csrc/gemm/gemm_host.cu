@@ -87,6 +87,8 @@ int pick_bn(int M, int N, int groups, int mn_major, int sms) {
 
 extern "C" {
 
+int mcb_sm_count() { return device_sm_count(); }
+
 // Returns 0 on success, a negative code for bad arguments, or a positive cudaError_t.
 //   A: K-major  -> [a_outer rows, a_inner = contraction] with leading dimension lda
 //      MN-major -> [a_outer = contraction rows, a_inner = M] with leading dimension lda

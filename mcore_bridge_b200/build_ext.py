@@ -21,6 +21,7 @@ REPO_DIR = PKG_DIR.parent
 CSRC = REPO_DIR / 'csrc'
 LIB_DIR = PKG_DIR / 'lib'
 LIB_NAME = 'libmcb200.so'
+HOST_NAME = '_mcb200_host.so'     # CPython module: the host side of the most frequent calls
 OBJ_DIR = REPO_DIR / 'build' / 'obj'
 
 NVCC_FLAGS = [
@@ -77,15 +78,53 @@ def _compile_one(src: Path, verbose: bool) -> Path:
     return obj
 
 
+def _host_command(out: Path) -> list[str]:
+    import sysconfig
+
+    import torch
+    inc = Path(torch.__file__).resolve().parent / 'include'
+    cuda = Path(_nvcc()).resolve().parent.parent / 'include'
+    dirs = [inc, inc / 'torch' / 'csrc' / 'api' / 'include', Path(sysconfig.get_paths()['include']), cuda]
+    return ['g++', '-O2', '-std=c++17', '-fPIC', '-shared', f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}',
+            *(f'-I{d}' for d in dirs), *map(str, sorted((CSRC / 'host').glob('*.cpp'))), '-o', str(out),
+            f'-L{inc.parent / "lib"}', '-ltorch_python', '-ltorch_cpu', '-lc10', '-lc10_cuda', '-ldl']
+
+
+def build_host(verbose: bool = True, force: bool = False) -> Path:
+    """Compile the CPython module ``lib/_mcb200_host.so`` against this interpreter and its torch. Returns its path."""
+    import torch
+    out, stamp = LIB_DIR / HOST_NAME, OBJ_DIR / 'host.sha1'
+    h = hashlib.sha1(f'{torch.__version__} {sys.version}'.encode())
+    for src in sorted((CSRC / 'host').glob('*.cpp')):
+        h.update(src.read_bytes())
+    if out.exists() and stamp.exists() and stamp.read_text() == h.hexdigest() and not force:
+        return out
+    LIB_DIR.mkdir(parents=True, exist_ok=True)
+    OBJ_DIR.mkdir(parents=True, exist_ok=True)
+    tmp = out.with_name(out.name + f'.tmp{os.getpid()}')
+    res = subprocess.run(_host_command(tmp), capture_output=True, text=True)
+    if res.returncode != 0:
+        tmp.unlink(missing_ok=True)
+        raise RuntimeError(f'g++ failed for csrc/host:\n{res.stdout}\n{res.stderr}')
+    os.replace(tmp, out)
+    stamp.write_text(h.hexdigest())
+    if verbose:
+        sys.stderr.write(f'[build_ext] linked {out}\n')
+    return out
+
+
 def build(verbose: bool = True, force: bool = False) -> Path:
-    """Compile every ``.cu`` under ``csrc/`` and link ``lib/libmcb200.so``. Returns the library path."""
+    """Compile every ``.cu`` under ``csrc/`` and link ``lib/libmcb200.so``, and the host module beside it. Returns the
+    library path."""
     if force and OBJ_DIR.exists():
         shutil.rmtree(OBJ_DIR)
     srcs = sources()
     if not srcs:
         raise RuntimeError(f'no CUDA sources under {CSRC}')
-    with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, len(srcs) + 1)) as ex:
+        host = ex.submit(build_host, verbose, force)
         objs = list(ex.map(lambda s: _compile_one(s, verbose), srcs))
+        host.result()
     LIB_DIR.mkdir(parents=True, exist_ok=True)
     out = LIB_DIR / LIB_NAME
     newest = max(o.stat().st_mtime for o in objs)

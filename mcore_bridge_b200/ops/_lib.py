@@ -7,6 +7,8 @@ library is an error (ops must not fall back silently to PyTorch there); on a CPU
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import threading
 from pathlib import Path
@@ -14,10 +16,19 @@ from pathlib import Path
 import torch
 
 _LIB_PATH = Path(__file__).resolve().parent.parent / 'lib' / 'libmcb200.so'
+_HOST_PATH = _LIB_PATH.with_name('_mcb200_host.so')
 _lib = None
-_lock = threading.Lock()
+_native = None
+_lock = threading.RLock()
 _status_words: dict[int, torch.Tensor] = {}
-LAUNCHES = 0  # kernel launches issued through this library (every op reports exactly one per launch)
+_launches = 0
+
+
+def __getattr__(name):
+    if name == 'LAUNCHES':   # kernel launches issued through this library (every op reports exactly one per launch)
+        return _launches + (_native.launches() if _native is not None else 0)
+    raise AttributeError(name)
+
 
 STATUS_NAMES = {
     0: 'ok', 1: 'timeout waiting for a filled smem stage', 2: 'timeout waiting for a free smem stage',
@@ -41,6 +52,8 @@ def cuda_enabled() -> bool:
     global _device_present
     if not _device_present:
         _device_present = torch.cuda.is_available()
+    if _native is not None:
+        return _device_present and _native.enabled()      # the same variable, read without building a dictionary key
     return _device_present and os.environ.get('MCB200_DISABLE_CUDA_KERNELS', '0') != '1'
 
 
@@ -59,15 +72,42 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+def native():
+    """The module ``csrc/host`` is built into: tensors in, tensors out, one call per operation."""
+    global _native
+    if _native is None:
+        path = str(lib()._name)
+        with _lock:
+            if _native is None:
+                if not _HOST_PATH.exists() and torch.cuda.is_available():
+                    from ..build_ext import build_host
+                    build_host(verbose=False)
+                if not _HOST_PATH.exists():
+                    raise KernelError(f'{_HOST_PATH} is missing: run `python -m mcore_bridge_b200.build_ext`')
+                loader = importlib.machinery.ExtensionFileLoader('_mcb200_host', str(_HOST_PATH))
+                m = importlib.util.module_from_spec(importlib.util.spec_from_loader('_mcb200_host', loader))
+                loader.exec_module(m)
+                m.init(path, KernelError, lambda dev: status_word(torch.device('cuda', dev)).data_ptr())
+                _native = m
+    return _native
+
+
+def native_if_enabled():
+    """:func:`native` where the hand-written kernels are to be used, else ``None``."""
+    return native() if cuda_enabled() else None
+
+
 def available() -> bool:
     if not cuda_enabled():
         return False
-    lib()  # raises loudly on a GPU box without the library
+    native()  # raises loudly on a GPU box without the library
     return True
 
 
 def stream_ptr() -> ctypes.c_void_p:
     # the current stream's handle without building a Stream object around it
+    if _native is not None:
+        return ctypes.c_void_p(_native.raw_stream())
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
@@ -97,7 +137,7 @@ def check_status(device=None, clear: bool = True) -> None:
 
 
 def check_rc(rc: int, what: str) -> None:
-    global LAUNCHES
-    LAUNCHES += 1
+    global _launches
+    _launches += 1
     if rc != 0:
         raise KernelError(f'{what} failed with code {rc}' + (' (CUDA error)' if rc > 0 else ' (bad argument)'))

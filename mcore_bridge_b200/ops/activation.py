@@ -7,7 +7,6 @@ CUDA: ``csrc/elementwise/norm_act.cu``.
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional
 
 import torch
@@ -15,7 +14,6 @@ import torch.nn.functional as F
 
 from . import _lib
 
-_ll, _int, _f = ctypes.c_longlong, ctypes.c_int, ctypes.c_float
 KINDS = {'swiglu': 0, 'quick_geglu': 1, 'geglu_tanh': 2}
 
 
@@ -40,37 +38,18 @@ class _GluCuda(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, probs, kind, clamp, offset):
-        F2 = x.shape[-1]
-        Fh = F2 // 2
-        x2 = x.reshape(-1, F2)
-        if x2.stride(-1) != 1:
-            x2 = x2.contiguous()
-        rows = x2.shape[0]
-        out = torch.empty((rows, Fh), dtype=x.dtype, device=x.device)
         pr = None if probs is None else probs.reshape(-1).float().contiguous()
-        rc = _lib.lib().mcb_glu_fwd(_lib.ptr(x2), _lib.ptr(pr), _lib.ptr(out), _ll(rows), _int(Fh), _ll(x2.stride(0)),
-                                    _int(kind), _f(clamp), _f(offset), _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_glu_fwd')
+        out, x2 = _lib.native().glu_fwd(x, pr, kind, clamp, offset)
         ctx.save_for_backward(x2, pr)
         ctx.args = (kind, clamp, offset, x.shape, None if probs is None else (probs.shape, probs.dtype))
-        return out.view(*x.shape[:-1], Fh)
+        return out if x.dim() == 2 else out.view(*x.shape[:-1], out.shape[-1])
 
     @staticmethod
     def backward(ctx, dout):
         x2, pr = ctx.saved_tensors
         kind, clamp, offset, shape, pmeta = ctx.args
-        rows, F2 = x2.shape
-        Fh = F2 // 2
-        d2 = dout.reshape(rows, Fh).contiguous()
-        din = torch.empty((rows, F2), dtype=x2.dtype, device=x2.device)
-        dpr = torch.empty(rows, dtype=torch.float32, device=x2.device) if pr is not None else None
-        rc = _lib.lib().mcb_glu_bwd(_lib.ptr(x2), _lib.ptr(pr), _lib.ptr(d2), _lib.ptr(din), _lib.ptr(dpr), _ll(rows),
-                                    _int(Fh), _ll(x2.stride(0)), _int(kind), _f(clamp), _f(offset), _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_glu_bwd')
-        dprobs = None
-        if pmeta is not None:
-            dprobs = dpr.view(pmeta[0]).to(pmeta[1])
-        return din.view(shape), dprobs, None, None, None
+        din, dpr = _lib.native().glu_bwd(dout, x2, pr, kind, clamp, offset)
+        return din.view(shape), None if pmeta is None else dpr.view(pmeta[0]).to(pmeta[1]), None, None, None
 
 
 def glu(x: torch.Tensor, kind: str = 'swiglu', probs: Optional[torch.Tensor] = None, clamp: float = 0.0,

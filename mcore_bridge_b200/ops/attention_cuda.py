@@ -70,38 +70,15 @@ class _AttnFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, seq_start, cu_seqlens, max_seqlen, scale):
-        T, nq, d = q.shape
-        nkv = k.shape[1]
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        o = torch.empty_like(q)
-        lse = torch.empty((nq, T), dtype=torch.float32, device=q.device)
-        rc = _lib.lib().mcb_attn_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(seq_start), _lib.ptr(o),
-                                     _lib.ptr(lse), _int(T), _int(nq), _int(nkv), _int(d), _f(scale),
-                                     _lib.ptr(_lib.status_word(q.device)), _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_attn_fwd')
+        o, lse, q, k, v = _lib.native().attn_fwd(q, k, v, seq_start, None, None, scale)
         ctx.save_for_backward(q, k, v, o, lse, seq_start, cu_seqlens)
         ctx.scale, ctx.max_seqlen = scale, max_seqlen
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, o, lse, seq_start, cu = ctx.saved_tensors
-        do = do.contiguous()
-        T, nq, d = q.shape
-        lib = _lib.lib()
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        delta = torch.empty((nq, T), dtype=torch.float32, device=q.device)
-        nkv = k.shape[1]
-        splits = _dkv_splits(T, nq, nkv, q.device)
-        partial = None
-        if splits > 1:
-            partial = torch.empty((2, splits, T, nkv, d), dtype=torch.float32, device=q.device)
-        rc = lib.mcb_attn_bwd_split(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(do),
-                                    _lib.ptr(lse), _lib.ptr(delta), _lib.ptr(seq_start), _lib.ptr(dq),
-                                    _lib.ptr(dk), _lib.ptr(dv), _int(T), _int(nq), _int(nkv), _int(d),
-                                    _f(ctx.scale), _lib.ptr(partial) if partial is not None else None,
-                                    _int(splits), _lib.ptr(_lib.status_word(q.device)), _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_attn_bwd_split')
+        q, k, v, o, lse, seq_start, _cu = ctx.saved_tensors
+        dq, dk, dv, _ = _lib.native().attn_bwd(do, q, k, v, o, lse, seq_start, None, None, None, ctx.scale)
         return dq, dk, dv, None, None, None, None
 
 
@@ -143,17 +120,8 @@ class _AttnRangesFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, k_lo, k_hi, q_lo, q_hi, scale, sinks=None):
-        T, nq, d = q.shape
-        Tk, nkv = k.shape[0], k.shape[1]
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        o = torch.empty_like(q)
-        lse = torch.empty((nq, T), dtype=torch.float32, device=q.device)
         sk = None if sinks is None else sinks.detach().float().contiguous()
-        rc = _lib.lib().mcb_attn_fwd_ranges(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(k_lo), _lib.ptr(k_hi),
-                                            _lib.ptr(sk), _lib.ptr(o), _lib.ptr(lse), _int(T), _int(Tk), _int(nq),
-                                            _int(nkv), _int(d), _f(scale), _lib.ptr(_lib.status_word(q.device)),
-                                            _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_attn_fwd_ranges')
+        o, lse, q, k, v = _lib.native().attn_fwd(q, k, v, k_lo, k_hi, sk, scale)
         ctx.save_for_backward(q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sk)
         ctx.scale = scale
         ctx.sink_dtype = None if sinks is None else sinks.dtype
@@ -163,19 +131,7 @@ class _AttnRangesFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do, _dlse):
         q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sk = ctx.saved_tensors
-        do = do.contiguous()
-        T, nq, d = q.shape
-        Tk, nkv = k.shape[0], k.shape[1]
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        delta = torch.empty((nq, T), dtype=torch.float32, device=q.device)
-        splits = _dkv_splits(Tk, nq, nkv, q.device)
-        partial = torch.empty((2, splits, Tk, nkv, d), dtype=torch.float32, device=q.device) if splits > 1 else None
-        rc = _lib.lib().mcb_attn_bwd_ranges(
-            _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(do), _lib.ptr(lse), _lib.ptr(delta), _int(0),
-            _lib.ptr(k_lo), _lib.ptr(k_hi), _lib.ptr(q_lo), _lib.ptr(q_hi), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv),
-            _int(T), _int(Tk), _int(nq), _int(nkv), _int(d), _f(ctx.scale), _lib.ptr(partial), _int(splits),
-            _lib.ptr(_lib.status_word(q.device)), _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_attn_bwd_ranges')
+        dq, dk, dv, delta = _lib.native().attn_bwd(do, q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, ctx.scale)
         dsinks = None
         if sk is not None:
             # the sink is one more softmax column with a zero value vector: d sink_h = -sum_i p_sink(i, h) * delta(i, h)

@@ -11,106 +11,50 @@ sequence (the recomputed tensors are the same expressions of the same inputs, wr
 """
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
-from . import _lib, gemm
+from . import _lib
 from .linear import _weight_grad
-
-_ll, _int, _f = ctypes.c_longlong, ctypes.c_int, ctypes.c_float
-
-
-def _rmsnorm_raw(x2, w, eps, zc):
-    rows, H = x2.shape
-    y = torch.empty((rows, H), dtype=x2.dtype, device=x2.device)
-    rstd = torch.empty(rows, dtype=torch.float32, device=x2.device)
-    rc = _lib.lib().mcb_rmsnorm_fwd(_lib.ptr(x2), None, _lib.ptr(w), _lib.ptr(y), None, _lib.ptr(rstd), _ll(rows),
-                                    _int(H), _ll(x2.stride(0)), _f(eps), _int(int(zc)), _lib.stream_ptr())
-    _lib.check_rc(rc, 'mcb_rmsnorm_fwd')
-    return y, rstd
-
-
-def _glu_raw(h2, kind, clamp, offset):
-    rows, F2 = h2.shape
-    out = torch.empty((rows, F2 // 2), dtype=h2.dtype, device=h2.device)
-    rc = _lib.lib().mcb_glu_fwd(_lib.ptr(h2), None, _lib.ptr(out), _ll(rows), _int(F2 // 2), _ll(h2.stride(0)),
-                                _int(kind), _f(clamp), _f(offset), _lib.stream_ptr())
-    _lib.check_rc(rc, 'mcb_glu_fwd')
-    return out
 
 
 class _NormLinearFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, ln_w, weight, eps, zc):
-        H = x.shape[-1]
-        x2 = x.reshape(-1, H)
-        if x2.stride(-1) != 1:
-            x2 = x2.contiguous()
-        xn, rstd = _rmsnorm_raw(x2, ln_w, eps, zc)
-        y = gemm.mm_nt(xn, weight)
+        y, x2, rstd = _lib.native().norm_linear_fwd(x, ln_w, weight, eps, zc)
         ctx.save_for_backward(x2, ln_w, rstd, weight)
         ctx.eps, ctx.zc, ctx.shape = eps, zc, x.shape
-        return y.view(*x.shape[:-1], weight.shape[0])
+        return y if x.dim() == 2 else y.view(*x.shape[:-1], weight.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
         x2, ln_w, rstd, weight = ctx.saved_tensors
-        rows, H = x2.shape
-        dy2 = dy.reshape(rows, weight.shape[0])
-        if dy2.stride(-1) != 1:
-            dy2 = dy2.contiguous()
-        dxn = gemm.mm_nn(dy2, weight)
-        dx = torch.empty((rows, H), dtype=x2.dtype, device=x2.device)
-        dlw = (torch.empty if rows else torch.zeros)(H, dtype=ln_w.dtype, device=x2.device)
-        part = torch.empty((_lib.lib().mcb_rmsnorm_bwd_partial_rows(_ll(rows), _int(H)), H), dtype=torch.float32,
-                           device=x2.device)
         need_dw = ctx.needs_input_grad[2]
-        fn = _lib.lib().mcb_rmsnorm_bwd_det_y if need_dw else _lib.lib().mcb_rmsnorm_bwd_det
-        rc = fn(_lib.ptr(dxn), _lib.ptr(x2), _lib.ptr(ln_w), _lib.ptr(rstd), None, _lib.ptr(dx), _lib.ptr(dlw), _int(1),
-                _lib.ptr(part), _ll(rows), _int(H), _ll(x2.stride(0)), _f(ctx.eps), _int(int(ctx.zc)), _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_rmsnorm_bwd_det')
-        dw = _weight_grad(weight, dy2, dxn) if need_dw else None   # dxn is the normalised input by now
-        return dx.view(ctx.shape), dlw, dw, None, None
+        dx, dlw, dy2, xn = _lib.native().norm_linear_bwd(dy, x2, ln_w, rstd, weight, ctx.eps, ctx.zc, need_dw)
+        return dx.view(ctx.shape), dlw, _weight_grad(weight, dy2, xn) if need_dw else None, None, None
 
 
 class _GluLinearFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, h, weight, kind, clamp, offset):
-        F2 = h.shape[-1]
-        h2 = h.reshape(-1, F2)
-        if h2.stride(-1) != 1:
-            h2 = h2.contiguous()
-        a = _glu_raw(h2, kind, clamp, offset)
-        y = gemm.mm_nt(a, weight)
+        y, h2 = _lib.native().glu_linear_fwd(h, weight, kind, clamp, offset)
         ctx.save_for_backward(h2, weight)
         ctx.args = (kind, clamp, offset, h.shape)
-        return y.view(*h.shape[:-1], weight.shape[0])
+        return y if h.dim() == 2 else y.view(*h.shape[:-1], weight.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
         h2, weight = ctx.saved_tensors
         kind, clamp, offset, shape = ctx.args
-        rows, F2 = h2.shape
-        dy2 = dy.reshape(rows, weight.shape[0])
-        if dy2.stride(-1) != 1:
-            dy2 = dy2.contiguous()
-        da = gemm.mm_nn(dy2, weight)
-        dh = torch.empty((rows, F2), dtype=h2.dtype, device=h2.device)
         need_dw = ctx.needs_input_grad[1]
-        fn = _lib.lib().mcb_glu_bwd_act if need_dw else _lib.lib().mcb_glu_bwd
-        rc = fn(_lib.ptr(h2), None, _lib.ptr(da), _lib.ptr(dh), None, _ll(rows), _int(F2 // 2), _ll(h2.stride(0)),
-                _int(kind), _f(clamp), _f(offset), _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_glu_bwd')
-        dw = _weight_grad(weight, dy2, da) if need_dw else None    # da is the activation by now
-        return dh.view(shape), dw, None, None, None
+        dh, dy2, a = _lib.native().glu_linear_bwd(dy, h2, weight, kind, clamp, offset, need_dw)
+        return dh.view(shape), _weight_grad(weight, dy2, a) if need_dw else None, None, None, None
 
 
 def usable(x: torch.Tensor, weight: torch.Tensor) -> bool:
     return (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and _lib.available()
-            and x.shape[-1] % 8 == 0 and torch.is_grad_enabled())
+            and x.shape[-1] % 8 == 0)
 
 
 def norm_linear(x, ln_w, weight, eps, zero_centered):

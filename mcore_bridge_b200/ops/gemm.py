@@ -27,6 +27,17 @@ def _use_cuda(*ts) -> bool:
     return all(t is None or t.is_cuda for t in ts) and ts[0].dtype == torch.bfloat16 and _lib.available()
 
 
+_RESULT_TYPES = (None, torch.bfloat16, torch.float32)
+
+
+def _native(a, b, bias, out_dtype):
+    """The module that forms the product in one call, where the kernels cover the operands."""
+    if a.is_cuda and a.dtype == torch.bfloat16 and b.is_cuda and out_dtype in _RESULT_TYPES \
+            and (bias is None or bias.is_cuda):
+        return _lib.native_if_enabled()
+    return None
+
+
 _entry = None
 
 
@@ -78,88 +89,62 @@ def _out(out, shape, dtype, device, accumulate):
     return out
 
 
+def _deliver(y, x, out, accumulate):
+    """The 2-D result ``y`` of a product with ``x [..., K]``: into ``out`` where that is given."""
+    if out is None:
+        return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
+    if accumulate:
+        out.add_(y.view(out.shape).to(out.dtype))
+    else:
+        out.copy_(y.view(out.shape))
+    return out
+
+
 def mm_nt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
           out_dtype: Optional[torch.dtype] = None, accumulate: bool = False, alpha: float = 1.0,
           max_sms: int = 0, force_bn: int = 0) -> torch.Tensor:
     """``x[..., K] @ w[N, K]^T (+ bias)``."""
-    lead = x.shape[:-1]
-    K = x.shape[-1]
-    N = w.shape[0]
-    assert w.shape[1] == K
-    if not _use_cuda(x, w, bias):
-        y = _lib_mm(x.reshape(-1, K), w.t()) * alpha
-        if bias is not None:
-            y = y + bias.float()
-        y = y.to(out_dtype or x.dtype)
+    nat = _native(x, w, bias, out_dtype)
+    if nat is not None:
+        y = nat.mm(0, x, w, bias, out, out_dtype == torch.float32, accumulate, alpha, max_sms, force_bn)
         if out is not None:
-            if accumulate:
-                out.add_(y.view(out.shape))
-            else:
-                out.copy_(y.view(out.shape))
             return out
-        return y if len(lead) == 1 else y.view(*lead, N)
-    x2, w2 = _row_major_2d(x), _row_major_2d(w)
-    M = x2.shape[0]
-    c = _out(out.view(M, N) if out is not None else None, (M, N), out_dtype or torch.bfloat16, x.device, accumulate)
+        return y if x.dim() == 2 else y.view(*x.shape[:-1], w.shape[0])   # no alias for the common case
+    K = x.shape[-1]
+    assert w.shape[1] == K
+    y = _lib_mm(x.reshape(-1, K), w.t()) * alpha
     if bias is not None:
-        bias = bias.to(torch.bfloat16).contiguous()
-    _launch(x2, K, M, x2.stride(0), False, w2, K, N, w2.stride(0), False, c, c.stride(0), 0, M, N, K, alpha, bias,
-            accumulate, max_sms=max_sms, force_bn=force_bn)
-    if out is not None:
-        return out
-    return c if len(lead) == 1 else c.view(*lead, N)      # no alias for the common 2-D case: callers may add in place
+        y = y + bias.float()
+    return _deliver(y.to(out_dtype or x.dtype), x, out, accumulate)
 
 
 def mm_nn(dy: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
           out_dtype: Optional[torch.dtype] = None, accumulate: bool = False, alpha: float = 1.0,
           max_sms: int = 0, force_bn: int = 0) -> torch.Tensor:
     """``dy[..., N] @ w[N, K]`` -> ``[..., K]``."""
-    lead = dy.shape[:-1]
-    N = dy.shape[-1]
-    K = w.shape[1]
-    assert w.shape[0] == N
-    if not _use_cuda(dy, w):
-        y = (_lib_mm(dy.reshape(-1, N), w) * alpha).to(out_dtype or dy.dtype)
+    nat = _native(dy, w, None, out_dtype)
+    if nat is not None:
+        y = nat.mm(1, dy, w, None, out, out_dtype == torch.float32, accumulate, alpha, max_sms, force_bn)
         if out is not None:
-            if accumulate:
-                out.add_(y.view(out.shape))
-            else:
-                out.copy_(y.view(out.shape))
             return out
-        return y if len(lead) == 1 else y.view(*lead, K)
-    d2, w2 = _row_major_2d(dy), _row_major_2d(w)
-    M = d2.shape[0]
-    c = _out(out.view(M, K) if out is not None else None, (M, K), out_dtype or torch.bfloat16, dy.device, accumulate)
-    # A = dy (K-major over the contraction N); B[k_out, n] = w[n, k_out] is MN-major as stored
-    _launch(d2, N, M, d2.stride(0), False, w2, K, N, w2.stride(0), True, c, c.stride(0), 0, M, K, N, alpha, None,
-            accumulate, max_sms=max_sms, force_bn=force_bn)
-    if out is not None:
-        return out
-    return c if len(lead) == 1 else c.view(*lead, K)
+        return y if dy.dim() == 2 else y.view(*dy.shape[:-1], w.shape[1])
+    N = dy.shape[-1]
+    assert w.shape[0] == N
+    y = (_lib_mm(dy.reshape(-1, N), w) * alpha).to(out_dtype or dy.dtype)
+    return _deliver(y, dy, out, accumulate)
 
 
 def mm_tn(dy: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None,
           out_dtype: Optional[torch.dtype] = None, accumulate: bool = False, alpha: float = 1.0,
           max_sms: int = 0, force_bn: int = 0) -> torch.Tensor:
     """``dy[T, N]^T @ x[T, K]`` -> ``[N, K]`` (weight gradient)."""
-    N = dy.shape[-1]
-    K = x.shape[-1]
-    if not _use_cuda(dy, x):
-        y = (_lib_mm(dy.reshape(-1, N).t(), x.reshape(-1, K)) * alpha)
-        if out is not None:
-            if accumulate:
-                out.add_(y.to(out.dtype))
-            else:
-                out.copy_(y.to(out.dtype))
-            return out
-        return y.to(out_dtype or dy.dtype)
-    d2, x2 = _row_major_2d(dy), _row_major_2d(x)
-    T = d2.shape[0]
-    assert x2.shape[0] == T
-    c = _out(out, (N, K), out_dtype or torch.bfloat16, dy.device, accumulate)
-    _launch(d2, N, T, d2.stride(0), True, x2, K, T, x2.stride(0), True, c, c.stride(0), 0, N, K, T, alpha, None,
-            accumulate, max_sms=max_sms, force_bn=force_bn)
-    return c
+    nat = _native(dy, x, None, out_dtype)
+    if nat is not None:
+        return nat.mm(2, dy, x, None, out, out_dtype == torch.float32, accumulate, alpha, max_sms, force_bn)
+    y = _lib_mm(dy.reshape(-1, dy.shape[-1]).t(), x.reshape(-1, x.shape[-1])) * alpha
+    if out is not None:
+        return _deliver(y, dy, out, accumulate)
+    return y.to(out_dtype or dy.dtype)
 
 
 # ------------------------------------------------------------------ grouped (MoE experts)

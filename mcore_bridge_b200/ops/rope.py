@@ -11,15 +11,12 @@ sections and attention scaling (``mscale`` folded into cos/sin, reference
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional, Tuple
 
 import torch
 
 from . import _lib
 from .norm import rmsnorm_ref
-
-_ll, _int, _f = ctypes.c_longlong, ctypes.c_int, ctypes.c_float
 
 
 def apply_rope_ref(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, interleaved: bool = False) -> torch.Tensor:
@@ -69,62 +66,16 @@ class _QkvCuda(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, wq, wk, cos, sin, ng, qpg, d, has_gate, interleaved, eps, zero_centered):
-        T = qkv.shape[0]
-        if qkv.stride(-1) != 1:
-            qkv = qkv.contiguous()
-        nq = ng * qpg
-        dev, dt = qkv.device, qkv.dtype
-        q = torch.empty((T, nq, d), dtype=dt, device=dev)
-        k = torch.empty((T, ng, d), dtype=dt, device=dev)
-        v = torch.empty((T, ng, d), dtype=dt, device=dev)
-        gate = torch.empty((T, nq, d), dtype=dt, device=dev) if has_gate else None
-        rot = 0 if cos is None else cos.shape[-1] * 2
-        norm = wq is not None
-        rc = _lib.lib().mcb_qkv_split_norm_rope_fwd(
-            _lib.ptr(qkv), _lib.ptr(wq), _lib.ptr(wk), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(q), _lib.ptr(k),
-            _lib.ptr(v), _lib.ptr(gate), _ll(T), _int(ng), _int(qpg), _int(d), _int(int(has_gate)), _int(rot),
-            _int(int(interleaved)), _int(int(norm)), _int(int(zero_centered)), _f(eps), _ll(qkv.stride(0)),
-            _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_qkv_split_norm_rope_fwd')
+        meta = (ng, qpg, d, has_gate, interleaved, eps, zero_centered)
+        q, k, v, gate, qkv = _lib.native().qkv_fwd(qkv, wq, wk, cos, sin, *meta)
         ctx.save_for_backward(qkv, wq, wk, cos, sin)
-        ctx.meta = (ng, qpg, d, has_gate, rot, interleaved, norm, zero_centered, eps)
-        if has_gate:
-            return q, k, v, gate
-        ctx.mark_non_differentiable()
-        return q, k, v, None
+        ctx.meta = meta
+        return q, k, v, gate
 
     @staticmethod
     def backward(ctx, dq, dk, dv, dgate):
-        qkv, wq, wk, cos, sin = ctx.saved_tensors
-        ng, qpg, d, has_gate, rot, interleaved, norm, zc, eps = ctx.meta
-        T = qkv.shape[0]
-        dev = qkv.device
-        nq = ng * qpg
-
-        def _c(t, shape):
-            if t is None:
-                return torch.zeros(shape, dtype=qkv.dtype, device=dev)
-            return t.contiguous()
-
-        dq, dk, dv = _c(dq, (T, nq, d)), _c(dk, (T, ng, d)), _c(dv, (T, ng, d))
-        if has_gate:
-            dgate = _c(dgate, (T, nq, d))
-        dqkv = torch.empty_like(qkv)
-        # bf16 weights (the only ones this path takes): the reduction below writes them rounded
-        alloc = torch.empty if T else torch.zeros
-        dwq, dwk = alloc((2, d), dtype=wq.dtype, device=dev).unbind(0) if norm else (None, None)
-        # per-CTA partial sums of the norm-weight gradients, added in a fixed order (bit-reproducible)
-        part = torch.empty((_lib.lib().mcb_qkv_bwd_partial_rows(_ll(T)), 2, d), dtype=torch.float32,
-                           device=dev) if norm else None
-        rc = _lib.lib().mcb_qkv_split_norm_rope_bwd(
-            _lib.ptr(qkv), _lib.ptr(wq), _lib.ptr(wk), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(dq), _lib.ptr(dk),
-            _lib.ptr(dv), _lib.ptr(dgate if has_gate else None), _lib.ptr(dqkv), _lib.ptr(dwq), _lib.ptr(dwk),
-            _int(1), _lib.ptr(part), _ll(T),
-            _int(ng), _int(qpg), _int(d), _int(int(has_gate)), _int(rot), _int(int(interleaved)), _int(int(norm)),
-            _int(int(zc)), _f(eps), _ll(qkv.stride(0)), _lib.stream_ptr())
-        _lib.check_rc(rc, 'mcb_qkv_split_norm_rope_bwd')
-        return (dqkv, dwq, dwk, None, None, None, None,
-                None, None, None, None, None)
+        dqkv, dwq, dwk = _lib.native().qkv_bwd(dq, dk, dv, dgate, *ctx.saved_tensors, *ctx.meta)
+        return (dqkv, dwq, dwk) + (None,) * 9
 
 
 def qkv_split_norm_rope(qkv: torch.Tensor, wq: Optional[torch.Tensor], wk: Optional[torch.Tensor],

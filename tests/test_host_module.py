@@ -1,0 +1,33 @@
+"""The module behind the most frequent calls: what it refuses, and the switch it reads."""
+import pytest
+import torch
+
+from mcore_bridge_b200.ops import _lib
+
+pytestmark = pytest.mark.skipif(not (_lib._LIB_PATH.exists() and _lib._HOST_PATH.exists()),
+                                reason='the CUDA library and its host module are not built')
+
+
+def test_arguments_are_checked_before_anything_runs():
+    nat = _lib.native()
+    x = torch.zeros(8, 8)
+    before = _lib.LAUNCHES
+    with pytest.raises(TypeError):
+        nat.mm(0, x, x)
+    with pytest.raises(TypeError):
+        nat.mm(0, None, x, None, None, False, False, 1.0, 0, 0)
+    with pytest.raises(AssertionError):
+        nat.mm(0, x, torch.zeros(8, 7), None, None, False, False, 1.0, 0, 0)     # contraction sizes differ
+    with pytest.raises(AssertionError):
+        nat.mm(0, x, x, None, torch.zeros(8, 7), False, False, 1.0, 0, 0)        # output of another shape
+    assert _lib.LAUNCHES == before
+
+
+def test_kernels_are_switched_off_by_the_environment(monkeypatch):
+    nat = _lib.native()
+    monkeypatch.delenv('MCB200_DISABLE_CUDA_KERNELS', raising=False)
+    assert nat.enabled()
+    monkeypatch.setenv('MCB200_DISABLE_CUDA_KERNELS', '1')
+    assert not nat.enabled()
+    monkeypatch.setenv('MCB200_DISABLE_CUDA_KERNELS', '0')
+    assert nat.enabled()
