@@ -1,7 +1,8 @@
 // Variable-length causal GQA attention backward for sm_100a.  Three kernels:
 //
 //   delta   : delta[h, i] = sum_d O[i, h, d] * dO[i, h, d]                                  (memory bound)
-//   dq      : one CTA per (128-query tile, query head), loops over 128-key blocks:
+//   dq      : one CTA per (128-query tile, query head), loops over 128-key blocks (and forms delta itself where that is the
+//             faster way, see launch_bwd):
 //               S = Q K^T, dP = dO V^T on tcgen05 -> P = exp2(S*c - lse), dS = P*(dP - delta)*scale in registers
 //               -> dS (bf16) to TMEM -> dQ += dS K accumulated in TMEM
 //   dk/dv   : one CTA per (128-key tile, kv head), loops over the query heads of the group and 128-query blocks:
@@ -57,6 +58,12 @@ struct BwdParams {
   int* status;
   float* partial;           // head-split mode: [2 (dv, dk), splits, Tk, nkv, d] fp32 partial sums, else null
   int splits;               // CTAs per (key tile, kv head); each takes qpg / splits query heads
+};
+
+// what the dq kernel forms delta from (o null: it is given)
+struct DeltaParams {
+  const __nv_bfloat16 *o, *dout;   // [T, nq, d]
+  float* delta;                    // [nq, T]
 };
 
 // K-major operand: tile of `rows` x D stored as D/64 boxes of [rows x 64]; kk-th 16-wide slice of the reduction dim
@@ -173,7 +180,7 @@ template <int D>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                   const BwdParams p) {
+                   const BwdParams p, const DeltaParams dp_) {
   using L = DqSmem<D>;
   constexpr int NBOX = D / 64;
   constexpr uint32_t TMEM_COLS = 512;
@@ -333,7 +340,34 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     // a query that sees nothing has lse = -inf; its probabilities are masked below, keep the arithmetic finite
     const float lse_i = row_ok ? p.lse[(long long)head * p.T + i] : 0.f;
     const float lse2 = (lse_i == -INFINITY) ? 0.f : lse_i * LOG2E;
-    const float dl = row_ok ? p.delta[(long long)head * p.T + i] : 0.f;
+    // delta of the row: either warp of a row takes half of the channels, read while the first tiles are on their way
+    float dl;
+    if (dp_.o == nullptr) {
+      dl = row_ok ? p.delta[(long long)head * p.T + i] : 0.f;
+    } else {
+      float acc = 0.f;
+      if (row_ok) {
+        const long long at = ((long long)i * p.nq + head) * D + grp * (D / 2);
+        const uint4 *po = reinterpret_cast<const uint4*>(dp_.o + at), *pd = reinterpret_cast<const uint4*>(dp_.dout + at);
+#pragma unroll 2
+        for (int c = 0; c < D / 16; ++c) {
+          const uint4 u = po[c], w = pd[c];
+          const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&u), *y = reinterpret_cast<const __nv_bfloat162*>(&w);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(x[e]), g = __bfloat1622float2(y[e]);
+            acc += f.x * g.x + f.y * g.y;
+          }
+        }
+      }
+      float* s_delta = reinterpret_cast<float*>(smem + L::OFF_BAR + 512);   // [TM], behind the barriers
+      if (grp == 1) s_delta[r] = acc;
+      asm volatile("bar.sync 1, 256;" ::: "memory");       // the eight element-wise warps, before any bounded wait
+      if (grp == 0) s_delta[r] = acc = acc + s_delta[r];
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      dl = grp == 0 ? acc : s_delta[r];
+      if (row_ok && grp == 0) dp_.delta[(long long)head * p.T + i] = dl;
+    }
     const uint64_t cc = f32x2(p.scale_log2, p.scale_log2), nl = f32x2(-lse2, -lse2), nd = f32x2(-dl, -dl);
     const uint64_t sc = f32x2(p.scale, p.scale);
     const uint32_t lane_addr = uint32_t(q * 32) << 16;
@@ -784,10 +818,39 @@ __global__ void attn_bwd_reduce_kernel(const float* __restrict__ partial, __nv_b
   }
 }
 
+// Gradient of the per-head sink logits: one more softmax column with a zero value vector, so
+// d sink_h = -sum_i exp(sink_h - lse(h, i)) delta(h, i).  One CTA per head, sums in a fixed order.
+constexpr int SINK_THREADS = 512;
+__global__ void __launch_bounds__(SINK_THREADS)
+attn_sink_grad_kernel(const float* __restrict__ sinks, const float* __restrict__ lse, const float* __restrict__ delta, int T,
+                      void* __restrict__ out, int out_bf16) {
+  __shared__ float red[SINK_THREADS / 32];
+  const int h = blockIdx.x;
+  const float sink = sinks[h];
+  float acc = 0.f;
+  for (int i = threadIdx.x; i < T; i += SINK_THREADS) {
+    // exp(x) as 2^(x log2 e) with the rounding error of the product put back: ex2's own two ulp remain
+    const float x = sink - lse[(long long)h * T + i], t = x * LOG2E;
+    const float lo = fmaf(x, LOG2E, -t) + x * 1.925963033500e-8f;
+    const float e = ex2_ftz(t);
+    acc += (t > -126.f ? fmaf(e, lo * 0.6931471805599453f, e) : e) * delta[(long long)h * T + i];
+  }
+#pragma unroll
+  for (int s = 16; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float sum = 0.f;
+    for (int w = 0; w < SINK_THREADS / 32; ++w) sum += red[w];
+    if (out_bf16) reinterpret_cast<__nv_bfloat16*>(out)[h] = __float2bfloat16(-sum);
+    else reinterpret_cast<float*>(out)[h] = -sum;
+  }
+}
+
 template <int D>
-int launch_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, float* delta,
-               bool delta_given, const BwdParams& p, cudaStream_t stream) {
-  // the tensor maps first: they refuse operands that are not on a 16-byte boundary, which the delta kernel would fault on
+int launch_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, float* delta, bool delta_given,
+               const BwdParams& p, cudaStream_t stream) {
+  // the tensor maps first: they refuse operands that are not on a 16-byte boundary, which the dq kernel would fault on
   CUtensorMap tq, tdo, tk, tv;
   const long long wq = (long long)p.nq * D, wk = (long long)p.nkv * D;
   int rc = 0;
@@ -795,15 +858,23 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* o, const
   if ((rc = make_tmap_2d_bf16(&tdo, dout, wq, p.T, wq, 64, TM))) return rc;
   if ((rc = make_tmap_2d_bf16(&tk, k, wk, p.Tk, wk, 64, TM))) return rc;
   if ((rc = make_tmap_2d_bf16(&tv, v, wk, p.Tk, wk, 64, TM))) return rc;
-  const long long rows = (long long)p.T * p.nq;
   cudaError_t e = cudaSuccess;
+  DeltaParams dp{nullptr, nullptr, nullptr};
   if (!delta_given) {
-    if (reinterpret_cast<uintptr_t>(o) & 15) return -6;    // read by the delta kernel alone
-    constexpr int PER = 4 * 256 / (D / 8);      // rows of a block
-    attn_bwd_delta_kernel<D><<<(unsigned)((rows + PER - 1) / PER), 256, 0, stream>>>(
-        (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, p.T, p.nq);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
+    if (reinterpret_cast<uintptr_t>(o) & 15) return -6;
+    // The dq kernel reads a row of O and dO per thread, longer for heads of 128; the kernel of its own costs a launch and a
+    // pass.  delta + dq + dk/dv, us, own kernel and in dq: 4095 tokens, 64 heads of 64, window 128 284 / 257, 4096, 24 of 64
+    // 320 / 317, 333, 4 of 64 32 / 29; 3000, 9 of 128 203 / 188, 2048, 32 of 128 194 / 196, 8192, 32 of 128 561 / 573.
+    const long long rows = (long long)p.T * p.nq;
+    if (D == 64 || rows <= 32768) {
+      dp = DeltaParams{(const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta};
+    } else {
+      constexpr int PER = 4 * 256 / (D / 8);    // rows of a block
+      attn_bwd_delta_kernel<D><<<(unsigned)((rows + PER - 1) / PER), 256, 0, stream>>>(
+          (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, p.T, p.nq);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return (int)e;
+    }
   }
   static bool cfg = false;
   if (!cfg) {
@@ -814,7 +885,7 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* o, const
     cfg = true;
   }
   const int tiles = (p.T + TM - 1) / TM, ktiles = (p.Tk + TM - 1) / TM;
-  attn_bwd_dq_kernel<D><<<(unsigned)tiles * p.nq, BWD_THREADS, DqSmem<D>::TOTAL, stream>>>(tq, tdo, tk, tv, p);
+  attn_bwd_dq_kernel<D><<<(unsigned)tiles * p.nq, BWD_THREADS, DqSmem<D>::TOTAL, stream>>>(tq, tdo, tk, tv, p, dp);
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   attn_bwd_dkv_kernel<D><<<(unsigned)ktiles * p.nkv * p.splits, BWD_THREADS, DkvSmem<D>::TOTAL, stream>>>(tk, tv, tq, tdo, p);
@@ -855,6 +926,15 @@ int mcb_attn_bwd_ranges(const void* q, const void* k, const void* v, const void*
   if (d == 128) return launch_bwd<128>(q, k, v, o, dout, delta, delta_given != 0, p, s);
   if (d == 64) return launch_bwd<64>(q, k, v, o, dout, delta, delta_given != 0, p, s);
   return -3;
+}
+
+// d sinks [nq] (fp32, or bf16 with out_bf16) of the forward's sinks [nq] fp32, from lse and delta [nq, T].
+int mcb_attn_sink_grad(const float* sinks, const float* lse, const float* delta, void* out, int out_bf16, int T, int nq,
+                       void* stream_) {
+  if (nq <= 0) return 0;
+  attn_sink_grad_kernel<<<(unsigned)nq, SINK_THREADS, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(sinks, lse, delta, T, out,
+                                                                                                  out_bf16);
+  return (int)cudaGetLastError();
 }
 
 // Packed causal self-attention: seq_start [T] int32 = first token of each token's sequence.

@@ -488,9 +488,22 @@ int launch_fwd(const void* q, const void* k, const void* v, AttnParams p, cudaSt
   return (int)cudaGetLastError();
 }
 
+__global__ void attn_window_starts_kernel(const int* __restrict__ seq_start, int* __restrict__ out, int T, int left) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < T) out[i] = max(seq_start[i], i - left);
+}
+
 }  // namespace
 
 extern "C" {
+
+// First visible key of every token of packed causal self-attention that sees at most `left` predecessors.
+int mcb_attn_window_starts(const int* seq_start, int* out, int T, int left, void* stream_) {
+  if (T <= 0) return 0;
+  attn_window_starts_kernel<<<(unsigned)(T + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(seq_start, out, T,
+                                                                                                           left);
+  return (int)cudaGetLastError();
+}
 
 // General form.  q [T, nq, d], k/v [Tk, nkv, d] bf16 contiguous; k_lo / k_hi [T] int32: query i attends to the keys
 // k_lo[i] .. k_hi[i] (inclusive; k_hi may be null = i, which needs Tk >= T); sinks [nq] fp32 or null; o [T, nq, d];

@@ -46,6 +46,8 @@ typedef long long ll;
   X(mcb_attn_bwd_ranges, int, (const void*, const void*, const void*, const void*, const void*, const float*, float*, int,    \
                                const int*, const int*, const int*, const int*, void*, void*, void*, int, int, int, int, int,  \
                                float, float*, int, int*, void*))                                                        \
+  X(mcb_attn_sink_grad, int, (const float*, const float*, const float*, void*, int, int, int, void*))                   \
+  X(mcb_attn_window_starts, int, (const int*, int*, int, int, void*))                                                   \
   X(mcb_sm_count, int, ())
 
 #define MCB_DECLARE(name, ret, args) ret(*name) args = nullptr;
@@ -410,9 +412,9 @@ PyObject* attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   MCB_END
 }
 
-// do, q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, scale -> dq, dk, dv, delta
+// do, q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sinks, bf16 sinks, scale -> dq, dk, dv, dsinks
 PyObject* attn_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  MCB_BEGIN(11)
+  MCB_BEGIN(13)
   const Tensor dout = tensor(a[0]).contiguous();
   const Tensor &q = tensor(a[1]), &k = tensor(a[2]), &v = tensor(a[3]), &o = tensor(a[4]), &lse = tensor(a[5]),
                &k_lo = tensor(a[6]);
@@ -425,9 +427,28 @@ PyObject* attn_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor partial = splits > 1 ? at::empty({2, splits, Tk, nkv, d}, lse.options()) : Tensor();
   launch("mcb_attn_bwd_ranges", mcb_attn_bwd_ranges, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
          dout.data_ptr(), lse.data_ptr(), delta.data_ptr(), 0, k_lo.data_ptr(), ptr(k_hi), ptr(q_lo), ptr(q_hi),
-         dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), T, Tk, nq, nkv, d, real(a[10]), ptr(partial), splits, status_of(q),
+         dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), T, Tk, nq, nkv, d, real(a[12]), ptr(partial), splits, status_of(q),
          stream());
-  return tuple({dq, dk, dv, delta});
+  Tensor dsinks;
+  if (a[10] != Py_None) {
+    const Tensor& sinks = tensor(a[10]);
+    const bool narrow = truth(a[11]);
+    dsinks = at::empty({nq}, lse.options().dtype(narrow ? at::kBFloat16 : at::kFloat));
+    launch("mcb_attn_sink_grad", mcb_attn_sink_grad, sinks.data_ptr(), lse.data_ptr(), delta.data_ptr(), dsinks.data_ptr(),
+           narrow, T, nq, stream());
+  }
+  return tuple({dq, dk, dv, dsinks});
+  MCB_END
+}
+
+PyObject* attn_window_starts(PyObject*, PyObject* const* a, Py_ssize_t n) {   // seq_start, left -> first visible keys
+  MCB_BEGIN(2)
+  const Tensor start = tensor(a[0]).contiguous();
+  const ll left = integer(a[1]);
+  const Tensor out = at::empty_like(start);
+  launch("mcb_attn_window_starts", mcb_attn_window_starts, start.data_ptr(), out.data_ptr(), start.numel(),
+         left < INT32_MAX ? left : INT32_MAX, stream());
+  return THPVariable_Wrap(out);
   MCB_END
 }
 
@@ -484,6 +505,7 @@ PyMethodDef methods[] = {MCB_FAST(init),
                          MCB_FAST(qkv_bwd),
                          MCB_FAST(attn_fwd),
                          MCB_FAST(attn_bwd),
+                         MCB_FAST(attn_window_starts),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_mcb200_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

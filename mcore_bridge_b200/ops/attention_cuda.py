@@ -78,7 +78,8 @@ class _AttnFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do):
         q, k, v, o, lse, seq_start, _cu = ctx.saved_tensors
-        dq, dk, dv, _ = _lib.native().attn_bwd(do, q, k, v, o, lse, seq_start, None, None, None, ctx.scale)
+        dq, dk, dv, _ = _lib.native().attn_bwd(do, q, k, v, o, lse, seq_start, None, None, None, None, False,
+                                              ctx.scale)
         return dq, dk, dv, None, None, None, None
 
 
@@ -99,7 +100,7 @@ def attention(q, k, v, cu_seqlens, max_seqlen, scale, seq_start: Optional[torch.
     k_lo = seq_start
     if left is not None:
         # still non-decreasing, so the kernels' causal fast paths (k_hi = the query itself) apply unchanged
-        k_lo = torch.maximum(seq_start, (torch.arange(T, device=q.device, dtype=torch.int32) - left))
+        k_lo = _lib.native().attn_window_starts(seq_start, left)
     o, _ = attention_ranges(q, k, v, k_lo.contiguous(), None, None, None, scale, sinks)
     return o
 
@@ -131,11 +132,10 @@ class _AttnRangesFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do, _dlse):
         q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sk = ctx.saved_tensors
-        dq, dk, dv, delta = _lib.native().attn_bwd(do, q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, ctx.scale)
-        dsinks = None
-        if sk is not None:
-            # the sink is one more softmax column with a zero value vector: d sink_h = -sum_i p_sink(i, h) * delta(i, h)
-            dsinks = -(torch.exp(sk[:, None] - lse) * delta).sum(1).to(ctx.sink_dtype)
+        dq, dk, dv, dsinks = _lib.native().attn_bwd(do, q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sk,
+                                                    ctx.sink_dtype == torch.bfloat16, ctx.scale)
+        if dsinks is not None:
+            dsinks = dsinks.to(ctx.sink_dtype)
         return dq, dk, dv, None, None, None, None, None, dsinks
 
 

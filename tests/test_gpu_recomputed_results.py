@@ -133,3 +133,24 @@ def test_expert_widths_that_end_inside_a_tile(monkeypatch, hidden, ffn):
     # either path rounds the hidden rows, their activation, the expert outputs and the result to bf16: 4 x 2^-9 each
     for a, b in zip(res['1'], res['0']):
         assert _rel(a, b) < 2 ** -6
+
+
+@pytest.mark.parametrize('T', [1, 511, 2050])                            # fewer tokens than threads, a remainder, many a thread
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('d', [64, 128])                                  # delta in the dQ kernel; 128: in it for few rows
+def test_sink_and_window_gradients(T, dtype, d):
+    from mcore_bridge_b200.ops.attention import attention, attention_ref
+    gen = torch.Generator(device=DEV).manual_seed(8)
+    nq, nkv = 20, 4
+    q, k, v = (torch.randn(T, n, d, generator=gen, device=DEV).bfloat16().requires_grad_() for n in (nq, nkv, nkv))
+    sinks = torch.randn(nq, generator=gen, device=DEV).to(dtype).requires_grad_()
+    dy = torch.randn(T, nq, d, generator=gen, device=DEV).bfloat16()
+    o = attention(q, k, v, window=(100, 0), sinks=sinks)
+    got = [o, *torch.autograd.grad(o, (q, k, v, sinks), dy)]
+    leaves = [t.detach().float().requires_grad_() for t in (q, k, v, sinks)]
+    ref = attention_ref(*leaves[:3], window=(100, 0), sinks=leaves[3])
+    want = [ref, *torch.autograd.grad(ref, leaves, dy.float())]
+    # probabilities, dS and the results are rounded to bf16, 2^-9 each; a sink's gradient sums T products of such results
+    for a, b, bound in zip(got, want, [2 ** -8] + 3 * [2 ** -6] + [2 ** -6]):
+        if T > 1 or b.abs().max() > 1e-3:          # one token: P = 1 - p_sink, no gradient reaches beyond rounding in places
+            assert _rel(a, b) < bound
