@@ -354,6 +354,58 @@ struct CombineArgs {
 };
 
 // out[t] = sum_k y_owner[row(t,k)]; optionally scalar_out[t,k] = scalar_owner[row(t,k)]
+// 4 to 8 rows a token: all of them are found first, then one 16-byte piece of each is in flight per lane; blockIdx.y takes runs of
+// 32 pieces, which gives few tokens more warps.  Bound: the reads.  Same order of the sums as below.  us, the kernel below / this
+// one: 4096 tokens x 8 rows of 2048 61 / 41 (3.7 TB/s), 1024 x 8 53 / 16, 64 x 8 49 / 8, 1000 x 6 43 / 14, 8192 x 4 of 2880
+// 92 / 74; it has too little in flight with fewer rows: 8192 x 2 of 4096 68 / 74, 16384 x 1 of 5120 80 / 147.  Two pieces a lane
+// measured the same or slower (43, 16, 10, 14, 78).
+__global__ void __launch_bounds__(256)
+moe_combine8_kernel(CombineArgs a, const int* __restrict__ idx, const int* __restrict__ sent_row,
+                    __nv_bfloat16* __restrict__ out, float* __restrict__ scalar_out) {
+  const int lane = threadIdx.x & 31;
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t >= a.T) return;
+  const int nvec = a.H / 8, v = blockIdx.y * 32 + lane;
+  const uint4* src[8];
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) {
+    src[kk] = nullptr;
+    if (kk < a.k) {
+      const int e = idx[t * a.k + kk], row = sent_row[t * a.k + kk];
+      if (row >= 0)
+        src[kk] = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.y_ptrs[e / a.El]) + (long long)row * a.H);
+    }
+  }
+  uint4 raw[8];
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) raw[kk] = src[kk] && v < nvec ? src[kk][v] : make_uint4(0, 0, 0, 0);
+  if (v < nvec) {
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      if (src[kk] == nullptr) continue;
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[kk]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(h[j]);
+        acc[2 * j] += f.x;
+        acc[2 * j + 1] += f.y;
+      }
+    }
+    uint4 o;
+    o.x = pack_bf16x2(acc[0], acc[1]);
+    o.y = pack_bf16x2(acc[2], acc[3]);
+    o.z = pack_bf16x2(acc[4], acc[5]);
+    o.w = pack_bf16x2(acc[6], acc[7]);
+    reinterpret_cast<uint4*>(out + t * a.H)[v] = o;
+  }
+  if (scalar_out && blockIdx.y == 0 && lane < a.k) {
+    const int e = idx[t * a.k + lane];
+    const int row = sent_row[t * a.k + lane];
+    scalar_out[t * a.k + lane] = (row >= 0 && a.scalar_ptrs[e / a.El]) ? a.scalar_ptrs[e / a.El][row] : 0.f;
+  }
+}
+
 __global__ void moe_combine_kernel(CombineArgs a, const int* __restrict__ idx, const int* __restrict__ sent_row,
                                    __nv_bfloat16* __restrict__ out, float* __restrict__ scalar_out) {
   const int lane = threadIdx.x & 31;
@@ -531,7 +583,11 @@ int mcb_moe_combine(const void* const* y_ptrs, const float* const* scalar_ptrs, 
     a.scalar_ptrs[i] = scalar_ptrs ? scalar_ptrs[i] : nullptr;
   }
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  moe_combine_kernel<<<grid_for(T, 256), 256, 0, s>>>(a, idx, sent_row, (__nv_bfloat16*)out, scalar_out);
+  if (k >= 4 && k <= 8)
+    moe_combine8_kernel<<<dim3((unsigned)((T + 7) / 8), (unsigned)((H / 8 + 31) / 32)), 256, 0, s>>>(a, idx, sent_row,
+                                                                                                    (__nv_bfloat16*)out, scalar_out);
+  else
+    moe_combine_kernel<<<grid_for(T, 256), 256, 0, s>>>(a, idx, sent_row, (__nv_bfloat16*)out, scalar_out);
   return (int)cudaGetLastError();
 }
 

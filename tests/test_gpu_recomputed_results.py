@@ -154,3 +154,31 @@ def test_sink_and_window_gradients(T, dtype, d):
     for a, b, bound in zip(got, want, [2 ** -8] + 3 * [2 ** -6] + [2 ** -6]):
         if T > 1 or b.abs().max() > 1e-3:          # one token: P = 1 - p_sink, no gradient reaches beyond rounding in places
             assert _rel(a, b) < bound
+
+
+@pytest.mark.parametrize('T,k,H', [(1, 4, 8), (37, 8, 520), (130, 5, 2048), (9, 8, 1032), (37, 3, 520), (37, 9, 520)])
+def test_expert_rows_are_summed_in_order(T, k, H):
+    """Rows that were not sent count as zero; pieces of 256 columns, the last one ragged; fewer than 4 or more than 8 rows
+    take the other kernel."""
+    import ctypes
+
+    from mcore_bridge_b200.ops import _lib
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    rows, experts = T * k + 3, 4
+    y = torch.randn(rows, H, generator=gen, device=DEV).bfloat16()
+    scalar = torch.rand(rows, generator=gen, device=DEV)
+    idx = torch.randint(0, experts, (T, k), generator=gen, device=DEV, dtype=torch.int32)
+    sent = torch.randperm(rows, generator=gen, device=DEV)[:T * k].view(T, k).int()
+    sent[0, 0] = -1
+    out = torch.empty(T, H, dtype=torch.bfloat16, device=DEV)
+    got = torch.empty(T, k, device=DEV)
+    table, scalars = ((ctypes.c_void_p * 1)(t.data_ptr()) for t in (y, scalar))
+    rc = _lib.lib().mcb_moe_combine(table, scalars, *map(ctypes.c_int, (1, T, k, experts, H)), _lib.ptr(idx), _lib.ptr(sent),
+                                    _lib.ptr(out), _lib.ptr(got), _lib.stream_ptr())
+    _lib.check_rc(rc, 'mcb_moe_combine')
+    hit = (sent >= 0)
+    want = torch.zeros(T, H, device=DEV)
+    for j in range(k):                                  # the kernels' order, in 32 bits: equal bits
+        want += torch.where(hit[:, j, None], y[sent[:, j].clamp(min=0).long()].float(), 0.)
+    assert torch.equal(out, want.bfloat16())
+    assert torch.equal(got, torch.where(hit, scalar[sent.clamp(min=0).long()], 0.))
