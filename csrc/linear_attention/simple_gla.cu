@@ -8,7 +8,7 @@
 // chunk.  Three launches: `boundary` forms what each chunk adds to the state that leaves it, `scan` runs the decayed
 // prefix sum over a sequence's chunk boundaries element by element, `out` computes every chunk independently.  All of
 // them have chunks x heads CTAs, so a single long sequence fills the GPU; token-by-token evaluation has one CTA per
-// (sequence, head).  Measured, 4096 tokens in two sequences, 16 heads of 128: forward 0.10 ms, backward 0.19 ms; token by
+// (sequence, head).  Measured, 4096 tokens in two sequences, 16 heads of 128: forward 0.09 ms, backward 0.17 ms; token by
 // token the two took 10.6 ms.  Batches of sequences of fewer than 16 tokens on average are evaluated token by token.  States
 // are fp32 in memory (64 KB per chunk boundary and head at d = 128; 128-token chunks keep that traffic at half of the
 // inputs') and enter the products as two bf16 terms, see warp_mma.cuh: against fp64 the bf16 results are off by 0.00166, their
@@ -95,8 +95,8 @@ gla_boundary_kernel(const GlaParams p) {
       uint32_t b[4];
       load_b_nn<D>(sy, kk, n, lane, b);
       mma16816(acc[n / 8], hi, b[0], b[1]);
-      mma16816(acc[n / 8], lo, b[0], b[1]);
       mma16816(acc[n / 8 + 1], hi, b[2], b[3]);
+      mma16816(acc[n / 8], lo, b[0], b[1]);
       mma16816(acc[n / 8 + 1], lo, b[2], b[3]);
     }
   }
@@ -162,16 +162,27 @@ gla_scan_kernel(const GlaParams p) {
 // fp32 [D, D] state -> two bf16 tiles
 template <int D>
 __device__ __forceinline__ void load_state(uint32_t hi, uint32_t lo, const float* __restrict__ src) {
-  for (int id = threadIdx.x; id < D * D / 8; id += THREADS) {
-    const int r = id / (D / 8), c = (id % (D / 8)) * 8;
-    const float4 x = *reinterpret_cast<const float4*>(src + r * D + c), y = *reinterpret_cast<const float4*>(src + r * D + c + 4);
-    uint32_t a[4], b[4];
-    split2(x.x, x.y, a[0], b[0]);
-    split2(x.z, x.w, a[1], b[1]);
-    split2(y.x, y.y, a[2], b[2]);
-    split2(y.z, y.w, a[3], b[3]);
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_addr<D>(hi, r, c)), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]) : "memory");
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_addr<D>(lo, r, c)), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]) : "memory");
+  constexpr int AHEAD = D * D / 8 / THREADS < 4 ? D * D / 8 / THREADS : 4;      // loads in flight: 4 x 32 bytes a thread
+#pragma unroll 1
+  for (int id0 = threadIdx.x; id0 < D * D / 8; id0 += AHEAD * THREADS) {
+    float4 x[AHEAD][2];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const float4* at = reinterpret_cast<const float4*>(src) + 2 * (id0 + u * THREADS);
+      x[u][0] = at[0];
+      x[u][1] = at[1];
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int r = (id0 + u * THREADS) / (D / 8), c = ((id0 + u * THREADS) % (D / 8)) * 8;
+      uint32_t a[4], b[4];
+      split2(x[u][0].x, x[u][0].y, a[0], b[0]);
+      split2(x[u][0].z, x[u][0].w, a[1], b[1]);
+      split2(x[u][1].x, x[u][1].y, a[2], b[2]);
+      split2(x[u][1].z, x[u][1].w, a[3], b[3]);
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_addr<D>(hi, r, c)), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]) : "memory");
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_addr<D>(lo, r, c)), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]) : "memory");
+    }
   }
 }
 
@@ -195,8 +206,8 @@ __device__ __forceinline__ void times_state(float (&acc)[D / 8][4], uint32_t x, 
         load_b_nn<D>(mlo, kk, n, lane, c);
       }
       mma16816(acc[n / 8], a, b[0], b[1]);
-      mma16816(acc[n / 8], a, c[0], c[1]);
       mma16816(acc[n / 8 + 1], a, b[2], b[3]);
+      mma16816(acc[n / 8], a, c[0], c[1]);
       mma16816(acc[n / 8 + 1], a, c[2], c[3]);
     }
   }
@@ -244,8 +255,8 @@ __device__ __forceinline__ void inside_chunk(float (&acc)[D / 8][4], uint32_t x,
       uint32_t b[4];
       load_b_nn<D>(z, jb * 16, n, lane, b);
       mma16816(acc[n / 8], hi, b[0], b[1]);
-      mma16816(acc[n / 8], lo, b[0], b[1]);
       mma16816(acc[n / 8 + 1], hi, b[2], b[3]);
+      mma16816(acc[n / 8], lo, b[0], b[1]);
       mma16816(acc[n / 8 + 1], lo, b[2], b[3]);
     }
   }
@@ -359,6 +370,81 @@ gla_grad_kernel(const GlaParams p) {
   store_rows<D>(acc, p.dv + off, stride, r0, len, lane);
 }
 
+// One chunk of one result, from the state M at its edge (S before it or R behind it) and the pairs inside it:
+//   ROLE       out_i = w_i * (X_i . M) + scale * sum_j a^|i-j| (X_i . Y_j) Z_j
+//   O          o  = q S,   (q . k) v       pairs j <= i
+//   DQ         dq = do S^T, (do . v) k     pairs j <= i
+//   DK         dk = v R^T, (v . do) q      pairs j >= i
+//   DV         dv = k R,   (k . q) do      pairs j >= i
+// The state's two terms lie where Y and Z go afterwards, so that three tiles are all a CTA holds and two CTAs share an SM
+// (D = 128: 96 KB each against 160 and 192 above): one computes while the other waits for its tiles.  See `two_per_sm`.
+enum { O, DQ, DK, DV };
+
+template <int D, int ROLE>
+__device__ __forceinline__ void chunk_result(const GlaParams& p, uint32_t sx, const ChunkPos& pos, int h) {
+  constexpr int TILE = C * D * 2;
+  constexpr bool BACK = ROLE >= DK;
+  const uint32_t sy = sx + TILE, sz = sy + TILE;
+  const __nv_bfloat16* X = ROLE == O ? p.q : ROLE == DQ ? p.dout : ROLE == DK ? p.v : p.k;
+  const __nv_bfloat16* Y = ROLE == O ? p.k : ROLE == DQ ? p.v : ROLE == DK ? p.dout : p.q;
+  const __nv_bfloat16* Z = ROLE == O ? p.v : ROLE == DQ ? p.k : ROLE == DK ? p.q : p.dout;
+  __nv_bfloat16* out = ROLE == O ? p.o : ROLE == DQ ? p.dq : ROLE == DK ? p.dk : p.dv;
+  const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
+  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
+  const int bnd = pos.boundary0 + pos.index;
+  // last chunk of a sequence, or (overlapping sequences) no boundary behind it
+  const bool state = BACK ? t + len < pos.t1 && bnd < p.T / C : pos.index > 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = warp * 16, i = r0 + (lane >> 2);
+  const float g2 = decay2(p, h);
+  float acc[D / 8][4];
+  zero_acc<D>(acc);
+  load_tile<D, C, THREADS>(sx, X + off, stride, len);
+  cp_async_commit();
+  if (state) {
+    load_state<D>(sy, sz, (BACK ? p.R : p.S) + ((long long)(BACK ? bnd : bnd - 1) * p.H + h) * D * D);
+    cp_async_wait<0>();
+    __syncthreads();
+    // a chunk that is not its sequence's last one is full: R decays by a^(C - i) to token i
+    const float w0 = BACK ? exp2f(g2 * (C - i)) : p.scale * exp2f(g2 * (i + 1));
+    const float w1 = BACK ? exp2f(g2 * (C - i - 8)) : p.scale * exp2f(g2 * (i + 9));
+    if (r0 < len) times_state<D, ROLE == DQ || ROLE == DK>(acc, sx, sy, sz, r0, lane, w0, w1);
+    __syncthreads();
+  }
+  load_tile<D, C, THREADS>(sy, Y + off, stride, len);
+  load_tile<D, C, THREADS>(sz, Z + off, stride, len);
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (r0 >= len) return;
+  inside_chunk<D, !BACK>(acc, sx, sy, sz, r0, BACK ? warp : 0, BACK ? (len + 15) / 16 : warp + 1, lane, g2, p.scale);
+  store_rows<D>(acc, out + off, stride, r0, len, lane);
+}
+
+// z (gradients): dq, dk, dv
+template <int D, bool GRAD>
+__global__ void __launch_bounds__(THREADS, 2)
+gla_result_kernel(const GlaParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ ChunkPos slot;
+  static_assert(D <= C, "a term of the state fits into a tile");
+  const uint32_t sx = (smem_u32(smem_raw) + 127) & ~127u;
+  const int h = blockIdx.y;
+  ChunkPos mine{-1, 0, 0, 0, 0};
+  if (threadIdx.x < 32) mine = find_chunk<C, false>(p.cu, p.n_seq, p.T, blockIdx.x, threadIdx.x);
+  const ChunkPos pos = broadcast_pos(mine, &slot);
+  if (pos.seq < 0 || pos.boundary0 + pos.index > p.T / C) return;
+  if (!GRAD) {
+    if (h == 0) check_bounds(p.cu, p.n_seq, p.T, p.status);
+    chunk_result<D, O>(p, sx, pos, h);
+  } else if (blockIdx.z == 0) {
+    chunk_result<D, DQ>(p, sx, pos, h);
+  } else if (blockIdx.z == 1) {
+    chunk_result<D, DK>(p, sx, pos, h);
+  } else {
+    chunk_result<D, DV>(p, sx, pos, h);
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------- short sequences
 // Token by token: one CTA of D threads per (sequence, head), thread j keeps column j of the state S [D x D] in registers.  q
 // and k of the current token are staged in shared memory (double buffered) so every thread reads them as broadcasts.
@@ -440,10 +526,25 @@ gla_token_bwd_kernel(const GlaParams p) {
 // A chunk costs about the same however few of its 128 rows a sequence fills, the token kernels cost the same per token.
 // Measured, 8192 tokens, 16 heads, sequences of 8 / 12 / 16 / 32 tokens, us:
 //   heads of 128, forward    chunked 574 / 377 / 283 / 158      token by token 442 / 436 / 430 / 441
+//                            (226 and 134 at 16 and 32 since two CTAs share an SM)
 //                 + backward        1509 / 1004 / 753 / 423                    1520 / 1519 / 1524 / 1571
 //   heads of 64,  forward           183 / 123 / 94 / 57                        93 / 93 / 93 / 95
 //                 + backward        552 / 370 / 283 / 171                      368 / 372 / 375 / 382
 bool by_token(int T, int n_seq) { return (long long)n_seq * 16 > T; }
+
+// One result a CTA and two CTAs an SM, or all results in one CTA.  Heads of 128 only: with 64 several CTAs of either kind share
+// an SM.  There have to be CTAs to share SMs, and the gradients read 9 tiles instead of 4, which pays where the states' products
+// and loads are most of the work, not in sequences of one chunk.  Measured, us, all in one / one a CTA:
+//   heads of 128, 16384 tokens x 32 heads      forward 679 / 548    backward 1482 / 1316
+//   8192 x 16, sequences of 1024                       165 / 144              359 / 332
+//                           200                        157 / 138              331 / 321
+//                           128                         85 / 83               151 / 185
+//                            32                        161 / 134              269 / 327
+//   1000 x 16, one sequence                             34 / 38                58 / 64
+//   heads of 64, 16384 x 32                            241 / 247              505 / 529
+bool two_per_sm(int D, int T, int n_seq, int H, bool grad) {
+  return D == 128 && (long long)(T / C) * H > device_sm_count() && (!grad || (long long)n_seq * C < T);
+}
 
 template <int D>
 int launch_gla(const GlaParams& p, int T, bool grad, cudaStream_t s) {
@@ -453,14 +554,20 @@ int launch_gla(const GlaParams& p, int T, bool grad, cudaStream_t s) {
     else gla_token_fwd_kernel<D><<<seqs, D, 0, s>>>(p);
     return (int)cudaGetLastError();
   }
-  constexpr int B_SMEM = 2 * C * D * 2 + 128, O_SMEM = 3 * C * D * 2 + 2 * D * D * 2 + 128, G_SMEM = O_SMEM + C * D * 2;
+  constexpr int B_SMEM = 2 * C * D * 2 + 128, R_SMEM = 3 * C * D * 2 + 128;
+  constexpr int O_SMEM = R_SMEM + 2 * D * D * 2, G_SMEM = O_SMEM + C * D * 2;
   static bool cfg = false;
   cudaError_t e;
   if (!cfg) {
-    if ((e = cudaFuncSetAttribute(gla_boundary_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, B_SMEM)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(gla_out_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, O_SMEM)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(gla_grad_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, G_SMEM)) != cudaSuccess)
+    constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if ((e = cudaFuncSetAttribute(gla_boundary_kernel<D>, kAttr, B_SMEM)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gla_out_kernel<D>, kAttr, O_SMEM)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gla_grad_kernel<D>, kAttr, G_SMEM)) != cudaSuccess)
       return (int)e;
+    if constexpr (D == 128)
+      if ((e = cudaFuncSetAttribute(gla_result_kernel<D, false>, kAttr, R_SMEM)) != cudaSuccess ||
+          (e = cudaFuncSetAttribute(gla_result_kernel<D, true>, kAttr, R_SMEM)) != cudaSuccess)
+        return (int)e;
     cfg = true;
   }
   const int bounds = T / C;                      // a sequence has at most (len - 1) / C boundaries
@@ -470,7 +577,14 @@ int launch_gla(const GlaParams& p, int T, bool grad, cudaStream_t s) {
     gla_scan_kernel<D><<<dim3(p.n_seq * (D * D / 1024), p.H, grad ? 2 : 1), 256, 0, s>>>(p);
     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
   }
-  const dim3 grid((T + C - 1) / C + p.n_seq, p.H);   // at least the number of chunks of any packing of T tokens
+  dim3 grid((T + C - 1) / C + p.n_seq, p.H);   // at least the number of chunks of any packing of T tokens
+  if constexpr (D == 128)
+    if (two_per_sm(D, T, p.n_seq, p.H, grad)) {
+      grid.z = grad ? 3 : 1;
+      if (grad) gla_result_kernel<D, true><<<grid, THREADS, R_SMEM, s>>>(p);
+      else gla_result_kernel<D, false><<<grid, THREADS, R_SMEM, s>>>(p);
+      return (int)cudaGetLastError();
+    }
   if (grad) gla_grad_kernel<D><<<grid, THREADS, G_SMEM, s>>>(p);
   else gla_out_kernel<D><<<grid, THREADS, O_SMEM, s>>>(p);
   return (int)cudaGetLastError();

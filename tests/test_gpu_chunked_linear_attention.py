@@ -352,3 +352,22 @@ def test_gated_delta_rule_with_hundreds_of_sequences():
     ref = _delta_rule(*wide, _spans(T, ends[:-1].tolist()))
     for a, b in zip([o, *grads], [ref, *torch.autograd.grad(ref, wide, dy.double())]):
         assert _rel(a, b) < (2 ** -8 if a.dtype == torch.bfloat16 else 2 ** -20)
+
+
+@pytest.mark.parametrize('T,h,cuts', [(1300, 16, [1, 130, 130, 700]), (1300, 16, list(range(100, 1300, 100))),
+                                      (130, 150, []), (257, 80, [129])])
+def test_simple_gla_one_result_per_block(T, h, cuts):
+    """More chunks x heads than SMs take kernels with one result a block, half of the heads at a time do not: equal bits."""
+    from mcore_bridge_b200.ops.gdn import simple_gla
+    tensors, gen = _inputs(T, h, 128, 3)
+    decay = -torch.rand(h, generator=gen, device=DEV)
+    cu = torch.tensor([0] + cuts + [T], dtype=torch.int32, device=DEV)
+
+    def run(s):
+        leaves = [t[:, s].contiguous().requires_grad_() for t in tensors[:3]]
+        o = simple_gla(*leaves, decay[s].contiguous(), cu)
+        return [o.detach(), *torch.autograd.grad(o, leaves, tensors[3][:, s].contiguous())]
+
+    parts = [run(slice(0, h // 2)), run(slice(h // 2, h))]
+    for got, *want in zip(run(slice(0, h)), *parts):
+        assert torch.equal(got, torch.cat(want, dim=1))
