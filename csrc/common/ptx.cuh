@@ -296,17 +296,6 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // D[tmem] (+)= A[tmem] * B[smem]: A is K-major bf16, lane = row, two consecutive k per 32-bit column.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void umma_f16_ts_warp(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
                                                  uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -341,13 +330,6 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
 }
 // 2-D tiled load into this CTA's shared memory whose completion bytes are counted on `bar`, a shared::cluster
 // address that may belong to the other CTA of the pair (the one that issues the MMAs).  No multicast.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          dst),
-      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
 __device__ __forceinline__ void tma_load_2d_pair_warp(uint32_t leader, uint32_t dst, const void* tmap, int x, int y,
                                                       uint32_t bar) {
   asm volatile(
@@ -369,20 +351,8 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// One thread of the leader CTA issues; A is read from both CTAs' shared memory (128 rows each), B likewise (N/2 rows
-// each), and each CTA's TMEM receives its own 128 accumulator rows.
-__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// as umma_f16_pair, by a converged warp of the leader CTA: the lane with `leader` set issues
+// One lane of the leader CTA's converged warp (`leader` set) issues; A is read from both CTAs' shared memory (128 rows each),
+// B likewise (N/2 rows each), and each CTA's TMEM receives its own 128 accumulator rows.
 __device__ __forceinline__ void umma_f16_pair_warp(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
                                                    uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -395,6 +365,8 @@ __device__ __forceinline__ void umma_f16_pair_warp(uint32_t leader, uint32_t d_t
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// Arrive on one mbarrier (shared::cluster address, possibly in the peer CTA) once every pair MMA issued so far by the
+// lane with `leader` set has completed.
 __device__ __forceinline__ void umma_commit_pair_warp(uint32_t leader, uint32_t bar_cluster_addr) {
   asm volatile(
       "{\n"
@@ -403,12 +375,6 @@ __device__ __forceinline__ void umma_commit_pair_warp(uint32_t leader, uint32_t 
       "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
       "}\n" ::"r"(bar_cluster_addr), "r"(leader)
       : "memory");
-}
-// Arrive on one mbarrier (shared::cluster address, possibly in the peer CTA) once every pair MMA issued so far by this
-// thread has completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr)
-               : "memory");
 }
 
 // ---------------------------------------------------------------- descriptors

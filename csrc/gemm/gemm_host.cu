@@ -167,9 +167,10 @@ int mcb_gemm_ce_bf16(const void* A, long long lda, const void* B, long long ldb,
   if (!grad && C != nullptr && (N % 4 || ldc % 4 || (reinterpret_cast<uintptr_t>(C) & 15))) return -5;
   constexpr int BN = 256;
   const int sms = device_sm_count();
-  // The gradient epilogue only: 4096 rows, 32000 columns, us, pairs and single CTAs, at K = 256 200 / 198, 512 219 / 222, 1024
-  // 286 / 304, 4096 832 / 860 (151936 columns: 1010 / 1050 at 512, 4040 / 4350 at 4096).  The statistics are slower with pairs
-  // throughout (118 / 105, 133 / 116, 200 / 187, 763 / 738; 595 / 555, 3560 / 3490), for a reason that was not looked into.
+  // CTA pairs for the gradient only.  us, single CTAs / pairs, each alone: gradient, 4096 x 32000 at K = 256 299 / 303, 1024 393 /
+  // 367, 4096 1039 / 875; 4096 x 151936 at 512 1182 / 1147, 4096 4690 / 3976.  Statistics alone, 4096 x 32000, K = 4096, 1024,
+  // 256: 707 / 696, 216 / 241, 148 / 166.  Statistics with the logits kept, 4096 x 151936: at 512 1049 / 1082, at 4096 4473 / 3755,
+  // but the head's forward and backward pass takes 13.88 / 13.83 ms, the power cap, so they stay with single CTAs too.
   const bool pair = grad && K >= 512 && use_pair(M, N, K, GEMM_DENSE, sms);
   CUtensorMap ta, tb;
   int rc = make_tmap_2d_bf16(&ta, A, K, M, lda, GEMM_BK, GEMM_BM);
