@@ -10,8 +10,11 @@
 // rows in registers, so every projection element is read once (plus 3 rows of overlap per walk) instead of once per slice,
 // copy, norm and tap.
 //
-// Measured, 4096 tokens, 16 groups, R = 2, d = 128: forward 87 us, backward 256 us (instruction-bound: the taps, SiLU and
-// its derivative are recomputed per element; 241 us with fast-math gates); the copy rate would take 36 and 70 us.
+// Bound: the latency of the rows.  Four rows are in flight per warp, kept as they lie in memory, and a row's registers are
+// loaded again as soon as it is widened; loading four rows, using them up and loading the next four left the schedulers idle
+// for 68 % of the cycles, half of the stalls waiting for these loads.  Measured, 4096 tokens, 16 groups, R = 2, d = 128, that
+// way / this way: forward 94 / 67 us, backward 280 / 194 (the copy rate would take 36 and 70); 300 tokens 32 / 16 and 83 / 56;
+// R = 1 66 / 52 and 210 / 118; d = 64 66 / 45 and 165 / 106.
 //
 // Values are rounded to bf16 where the separate operators store them (convolution output, normalised q / k).
 #include "../common/host_utils.cuh"
@@ -57,15 +60,31 @@ __device__ __forceinline__ float bf_round(float x) { return __bfloat162float(__f
 __device__ __forceinline__ float gate_sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float softplus_(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
-// N consecutive bf16 (N even) at a 4-byte aligned address
+// N consecutive bf16 (N even) at a 4-byte aligned address: as they are, and as floats
+template <int N>
+__device__ __forceinline__ void ldn(const __nv_bfloat16* p, uint32_t (&x)[N / 2]) {
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) x[i] = reinterpret_cast<const uint32_t*>(p)[i];
+}
+template <int N>
+__device__ __forceinline__ void widen(const uint32_t (&x)[N / 2], float (&f)[N]) {
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[i]));
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
 template <int N>
 __device__ __forceinline__ void ldn(const __nv_bfloat16* p, float (&f)[N]) {
+  uint32_t x[N / 2];
+  ldn<N>(p, x);
+  widen<N>(x, f);
+}
+template <int N>
+__device__ __forceinline__ void stn(__nv_bfloat16* p, const uint32_t (&x)[N / 2]) {
 #pragma unroll
-  for (int i = 0; i < N; i += 2) {
-    const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + i));
-    f[i] = t.x;
-    f[i + 1] = t.y;
-  }
+  for (int i = 0; i < N / 2; ++i) reinterpret_cast<uint32_t*>(p)[i] = x[i];
 }
 template <int N>
 __device__ __forceinline__ void stn(__nv_bfloat16* p, const float (&f)[N]) {
@@ -88,19 +107,31 @@ gdn_inputs_fwd_kernel(const InParams p) {
     const int hv = lane < R ? grp * R + lane : 0;
     const float neg_a = lane < R ? -expf(__bfloat162float(p.A_log[hv])) : 0.f;
     const float dtb = lane < R ? __bfloat162float(p.dt[hv]) : 0.f;
-#pragma unroll 4
-    for (int t = t0; t < t1; ++t) {
+    for (int tb = t0; tb < t1; tb += KW) {
+      uint32_t z[KW][R][PER / 2];                // four rows in flight
+      __nv_bfloat16 b[KW], a[KW];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        float zz[PER];
-        ldn<PER>(src + t * p.ld + r * D, zz);
-        stn<PER>(p.z + out_row(t) + r * D, zz);
+      for (int u = 0; u < KW; ++u) {
+        const __nv_bfloat16* row = src + (tb + u) * p.ld;
+        if (tb + u >= t1) break;
+#pragma unroll
+        for (int r = 0; r < R; ++r) ldn<PER>(row + r * D, z[u][r]);
+        if (lane < R) {
+          b[u] = row[R * D + lane - lane * PER];
+          a[u] = row[R * D + R + lane - lane * PER];
+        }
       }
-      if (lane < R) {
-        const __nv_bfloat16* ba = src - lane * PER + t * p.ld + R * D + lane;
-        const long long at = (long long)t * p.G * R + hv;
-        p.beta[at] = gate_sigmoid(__bfloat162float(ba[0]));
-        p.g[at] = neg_a * softplus_(__bfloat162float(ba[R]) + dtb);
+#pragma unroll
+      for (int u = 0; u < KW; ++u) {
+        const int t = tb + u;
+        if (t >= t1) break;
+#pragma unroll
+        for (int r = 0; r < R; ++r) stn<PER>(p.z + out_row(t) + r * D, z[u][r]);
+        if (lane < R) {
+          const long long at = (long long)t * p.G * R + hv;
+          p.beta[at] = gate_sigmoid(__bfloat162float(b[u]));
+          p.g[at] = neg_a * softplus_(__bfloat162float(a[u]) + dtb);
+        }
       }
     }
     return;
@@ -118,22 +149,24 @@ gdn_inputs_fwd_kernel(const InParams p) {
 #pragma unroll
   for (int b = 1; b < KW; ++b)
     if (t0 - b >= 0) ldn<PER>(src + (t0 - b) * p.ld, x[KW - b]);    // t0 is a multiple of 4
-  for (int tb = t0; tb < t1; tb += KW) {
-    float nx[KW][PER];                           // four rows in flight
-    int first[KW];
+  uint32_t nx[KW][PER / 2];                      // the next four rows, in flight: a row's slot is loaded again once it is read
+  int first[KW];
+  auto fetch = [&](int t, int u) {
+    if (t < t1) {
+      ldn<PER>(src + t * p.ld, nx[u]);
+      first[u] = p.seq_start[t];
+    }
+  };
 #pragma unroll
-    for (int u = 0; u < KW; ++u)
-      if (tb + u < t1) {
-        ldn<PER>(src + (tb + u) * p.ld, nx[u]);
-        first[u] = p.seq_start[tb + u];
-      }
+  for (int u = 0; u < KW; ++u) fetch(t0 + u, u);
+  for (int tb = t0; tb < t1; tb += KW) {
 #pragma unroll
     for (int u = 0; u < KW; ++u) {
       const int t = tb + u;
       if (t >= t1) break;
-#pragma unroll
-      for (int c = 0; c < PER; ++c) x[u][c] = nx[u][c];
+      widen<PER>(nx[u], x[u]);
       const int back = t - first[u];             // rows of the same sequence before this one
+      fetch(t + KW, u);
       float y[PER];
 #pragma unroll
       for (int c = 0; c < PER; ++c) {
@@ -180,25 +213,41 @@ gdn_inputs_bwd_kernel(const InParams p) {
     const float neg_a = lane < R ? -expf(__bfloat162float(p.A_log[hv])) : 0.f;
     const float dtb = lane < R ? __bfloat162float(p.dt[hv]) : 0.f;
     float dA = 0.f, ddt = 0.f;
-#pragma unroll 4
-    for (int t = t0; t < t1; ++t) {
+    for (int tb = t0; tb < t1; tb += KW) {
+      uint32_t z[KW][R][PER / 2];                // four rows in flight
+      __nv_bfloat16 b[KW], a[KW];
+      float db[KW], dgs[KW];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        float zz[PER];
-        ldn<PER>(p.dz + grad_row(t) + r * D, zz);
-        stn<PER>(dst + t * p.ld_d + r * D, zz);
+      for (int u = 0; u < KW; ++u) {
+        const int t = tb + u;
+        if (t >= t1) break;
+#pragma unroll
+        for (int r = 0; r < R; ++r) ldn<PER>(p.dz + grad_row(t) + r * D, z[u][r]);
+        if (lane < R) {
+          const __nv_bfloat16* ba = src - lane * PER + t * p.ld + R * D + lane;
+          const long long at = (long long)t * p.G * R + hv;
+          b[u] = ba[0];
+          a[u] = ba[R];
+          db[u] = p.dbeta[at];
+          dgs[u] = p.dg[at];
+        }
       }
-      if (lane < R) {
-        const __nv_bfloat16* ba = src - lane * PER + t * p.ld + R * D + lane;
-        __nv_bfloat16* dba = dst - lane * PER + t * p.ld_d + R * D + lane;
-        const long long at = (long long)t * p.G * R + hv;
-        const float beta = gate_sigmoid(__bfloat162float(ba[0]));
-        dba[0] = __float2bfloat16(p.dbeta[at] * beta * (1.f - beta));
-        const float xx = __bfloat162float(ba[R]) + dtb, dg = p.dg[at];
-        const float da = dg * neg_a * gate_sigmoid(xx);
-        dba[R] = __float2bfloat16(da);
-        dA += dg * neg_a * softplus_(xx);
-        ddt += da;
+#pragma unroll
+      for (int u = 0; u < KW; ++u) {
+        const int t = tb + u;
+        if (t >= t1) break;
+#pragma unroll
+        for (int r = 0; r < R; ++r) stn<PER>(dst + t * p.ld_d + r * D, z[u][r]);
+        if (lane < R) {
+          __nv_bfloat16* dba = dst - lane * PER + t * p.ld_d + R * D + lane;
+          const float beta = gate_sigmoid(__bfloat162float(b[u]));
+          dba[0] = __float2bfloat16(db[u] * beta * (1.f - beta));
+          const float xx = __bfloat162float(a[u]) + dtb, dg = dgs[u];
+          const float da = dg * neg_a * gate_sigmoid(xx);
+          dba[R] = __float2bfloat16(da);
+          dA += dg * neg_a * softplus_(xx);
+          ddt += da;
+        }
       }
     }
     if (lane < R) {
@@ -237,29 +286,25 @@ gdn_inputs_bwd_kernel(const InParams p) {
       if (t0 - b >= 0) ldn<PER>(src + (t0 - b) * p.ld, x[KW - b]);
     const int last = t1 + KW - 1;                // dpre of the KW - 1 tokens behind the walk reaches into it
     const int te = min(last, p.T);
-    for (int tb = t0; tb < last; tb += KW) {
-      float nx[KW][PER], nd[KW][PER];            // four rows and their gradients in flight
-      int nf[KW];
+    // four rows and their gradients in flight: a row's slot is loaded again once it is read
+    const __nv_bfloat16* dn = (s == 0 ? p.dq : s == 1 ? p.dk : p.dv) + (s < 2 ? 0 : s - 2) * D;
+    uint32_t nx[KW][PER / 2], nd[KW][R][PER / 2];
+    int nf[KW];
+    auto fetch = [&](int t, int u) {
+      nf[u] = 0x7fffffff;                        // past the end of the batch: in no sequence
+      if (t < te) {
+        nf[u] = p.seq_start[t];
+        ldn<PER>(src + t * p.ld, nx[u]);
+        ldn<PER>(dn + grad_row(t), nd[u][0]);
+        if (s < 2) {
 #pragma unroll
-      for (int u = 0; u < KW; ++u) {
-        const int t = tb + u;
-        nf[u] = 0x7fffffff;                      // past the end of the batch: in no sequence
-        if (t < te) {
-          nf[u] = p.seq_start[t];
-          ldn<PER>(src + t * p.ld, nx[u]);
-          const __nv_bfloat16* dn = (s == 0 ? p.dq : s == 1 ? p.dk : p.dv) + grad_row(t) + (s < 2 ? 0 : s - 2) * D;
-          ldn<PER>(dn, nd[u]);
-          if (s < 2) {
-#pragma unroll
-            for (int r = 1; r < R; ++r) {
-              float e[PER];
-              ldn<PER>(dn + r * D, e);
-#pragma unroll
-              for (int c = 0; c < PER; ++c) nd[u][c] += e[c];
-            }
-          }
+          for (int r = 1; r < R; ++r) ldn<PER>(dn + grad_row(t) + r * D, nd[u][r]);
         }
       }
+    };
+#pragma unroll
+    for (int u = 0; u < KW; ++u) fetch(t0 + u, u);
+    for (int tb = t0; tb < last; tb += KW) {
 #pragma unroll
       for (int u = 0; u < KW; ++u) {
         const int t = tb + u;
@@ -270,11 +315,18 @@ gdn_inputs_bwd_kernel(const InParams p) {
         if (t < te) {
           const int back = t - nf[u];
           float pre[PER], sg[PER], y[PER], d[PER];
+          widen<PER>(nx[u], x[u]);
+          widen<PER>(nd[u][0], d);
+          if (s < 2) {
 #pragma unroll
-          for (int c = 0; c < PER; ++c) {
-            x[u][c] = nx[u][c];
-            d[c] = nd[u][c];
+            for (int r = 1; r < R; ++r) {
+              float e[PER];
+              widen<PER>(nd[u][r], e);
+#pragma unroll
+              for (int c = 0; c < PER; ++c) d[c] += e[c];
+            }
           }
+          fetch(t + KW, u);
 #pragma unroll
           for (int c = 0; c < PER; ++c) {
             float a = 0.f;
