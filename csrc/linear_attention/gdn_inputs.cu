@@ -13,13 +13,15 @@
 // Bound: the latency of the rows.  Four rows are in flight per warp, kept as they lie in memory, and a row's registers are
 // loaded again as soon as it is widened; loading four rows, using them up and loading the next four left the schedulers idle
 // for 68 % of the cycles, half of the stalls waiting for these loads.  Measured, 4096 tokens, 16 groups, R = 2, d = 128, that
-// way / this way: forward 94 / 67 us, backward 280 / 194 (the copy rate would take 36 and 70); 300 tokens 32 / 16 and 83 / 56;
-// R = 1 66 / 52 and 210 / 118; d = 64 66 / 45 and 165 / 106.
+// way / this way: forward 94 / 67 us, backward 280 / 146 (the copy rate would take 36 and 70); 300 tokens 32 / 16 and 83 / 36;
+// R = 1 66 / 52 and 210 / 118; d = 64 66 / 45 and 165 / 89.
 //
 // Values are rounded to bf16 where the separate operators store them (convolution output, normalised q / k).
 #include "../common/host_utils.cuh"
 #include "../common/partials.cuh"
 #include "../common/ptx.cuh"
+
+#include <type_traits>
 
 using namespace mcb;
 
@@ -196,8 +198,12 @@ gdn_inputs_fwd_kernel(const InParams p) {
   }
 }
 
+// Backward.  Four rows whose windows lie in one sequence go through straight-line code, in which they overlap.  That takes 154 ..
+// 168 registers at d = 128 (96 at 64) and spills at 128 (80), so three (five) CTAs share an SM instead of four (six).  us, row by
+// row with four (six) / straight with four (six) / straight with three (five), 4096 tokens: d = 128, R = 2, 16 groups 194 / 196 / 146,
+// R = 1 118 / 138 / 118, R = 4, 8 groups 181 / 169 / 118; d = 64, R = 1 97 / 93 / 73, R = 2 105 / 87 / 89, R = 4 97 / 101 / 77.
 template <int D, int R>
-__global__ void __launch_bounds__(WARPS * 32, D == 128 ? 4 : 6)   // 128 registers: with 151, three CTAs per SM, 256 us become 324
+__global__ void __launch_bounds__(WARPS * 32, D == 128 ? 3 : 5)
 gdn_inputs_bwd_kernel(const InParams p) {
   constexpr int PER = D / 32, S = 2 + R;
   __shared__ float s_w[WARPS][D * KW];
@@ -289,100 +295,121 @@ gdn_inputs_bwd_kernel(const InParams p) {
     // four rows and their gradients in flight: a row's slot is loaded again once it is read
     const __nv_bfloat16* dn = (s == 0 ? p.dq : s == 1 ? p.dk : p.dv) + (s < 2 ? 0 : s - 2) * D;
     uint32_t nx[KW][PER / 2], nd[KW][R][PER / 2];
-    int nf[KW];
+    int nf[KW];                                  // of four rows, loaded four rows ahead
     auto fetch = [&](int t, int u) {
-      nf[u] = 0x7fffffff;                        // past the end of the batch: in no sequence
-      if (t < te) {
-        nf[u] = p.seq_start[t];
-        ldn<PER>(src + t * p.ld, nx[u]);
-        ldn<PER>(dn + grad_row(t), nd[u][0]);
-        if (s < 2) {
+      ldn<PER>(src + t * p.ld, nx[u]);
+      ldn<PER>(dn + grad_row(t), nd[u][0]);
+      if (s < 2) {
 #pragma unroll
-          for (int r = 1; r < R; ++r) ldn<PER>(dn + grad_row(t) + r * D, nd[u][r]);
-        }
+        for (int r = 1; r < R; ++r) ldn<PER>(dn + grad_row(t) + r * D, nd[u][r]);
       }
     };
-#pragma unroll
-    for (int u = 0; u < KW; ++u) fetch(t0 + u, u);
-    for (int tb = t0; tb < last; tb += KW) {
-#pragma unroll
-      for (int u = 0; u < KW; ++u) {
-        const int t = tb + u;
-        if (t >= last) break;
-        start[u] = nf[u];
+    auto row = [&](auto whole, int t, int u) {
+      constexpr bool W = decltype(whole)::value;
+      if (!W) {
 #pragma unroll
         for (int c = 0; c < PER; ++c) dp[u][c] = 0.f;
-        if (t < te) {
-          const int back = t - nf[u];
-          float pre[PER], sg[PER], y[PER], d[PER];
-          widen<PER>(nx[u], x[u]);
-          widen<PER>(nd[u][0], d);
-          if (s < 2) {
+      }
+      if (W || t < te) {
+        const int back = t - start[u];
+        float pre[PER], sg[PER], y[PER], d[PER];
+        widen<PER>(nx[u], x[u]);
+        widen<PER>(nd[u][0], d);
+        if (s < 2) {
 #pragma unroll
-            for (int r = 1; r < R; ++r) {
-              float e[PER];
-              widen<PER>(nd[u][r], e);
+          for (int r = 1; r < R; ++r) {
+            float e[PER];
+            widen<PER>(nd[u][r], e);
 #pragma unroll
-              for (int c = 0; c < PER; ++c) d[c] += e[c];
-            }
+            for (int c = 0; c < PER; ++c) d[c] += e[c];
           }
-          fetch(t + KW, u);
+        }
+        if (W || t + KW < te) fetch(t + KW, u);
+#pragma unroll
+        for (int c = 0; c < PER; ++c) {
+          float a = 0.f;
+          if (W || back >= KW - 1) {
+#pragma unroll
+            for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], x[(u + 1 + j) & 3][c], a);
+          } else {
+#pragma unroll
+            for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
+          }
+          pre[c] = a;
+          sg[c] = sigmoid_(a);
+          y[c] = bf_round(a * sg[c]);
+        }
+        if (s < 2) {                             // through y * rsqrt(sum y^2 + eps)
+          float ss = 0.f, dot = 0.f;
 #pragma unroll
           for (int c = 0; c < PER; ++c) {
-            float a = 0.f;
-            if (back >= KW - 1) {
+            ss += y[c] * y[c];
+            dot += y[c] * d[c];
+          }
+          const float r = rsqrtf(wsum(ss) + 1e-6f);
+          dot = wsum(dot) * r * r;
 #pragma unroll
-              for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], x[(u + 1 + j) & 3][c], a);
+          for (int c = 0; c < PER; ++c) d[c] = r * (d[c] - y[c] * dot);
+        }
+#pragma unroll
+        for (int c = 0; c < PER; ++c) {
+          dp[u][c] = d[c] * sg[c] * (1.f + pre[c] * (1.f - sg[c]));
+          if (W || t < t1) {                     // every token's tap gradients are added once, by its own walk
+            if (W || back >= KW - 1) {
+#pragma unroll
+              for (int j = 0; j < KW; ++j) dw[c][j] = fmaf(dp[u][c], x[(u + 1 + j) & 3][c], dw[c][j]);
             } else {
 #pragma unroll
-              for (int j = 0; j < KW; ++j) a = fmaf(w[c][j], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, a);
-            }
-            pre[c] = a;
-            sg[c] = sigmoid_(a);
-            y[c] = bf_round(a * sg[c]);
-          }
-          if (s < 2) {                           // through y * rsqrt(sum y^2 + eps)
-            float ss = 0.f, dot = 0.f;
-#pragma unroll
-            for (int c = 0; c < PER; ++c) {
-              ss += y[c] * y[c];
-              dot += y[c] * d[c];
-            }
-            const float r = rsqrtf(wsum(ss) + 1e-6f);
-            dot = wsum(dot) * r * r;
-#pragma unroll
-            for (int c = 0; c < PER; ++c) d[c] = r * (d[c] - y[c] * dot);
-          }
-#pragma unroll
-          for (int c = 0; c < PER; ++c) {
-            dp[u][c] = d[c] * sg[c] * (1.f + pre[c] * (1.f - sg[c]));
-            if (t < t1) {                        // every token's tap gradients are added once, by its own walk
-              if (back >= KW - 1) {
-#pragma unroll
-                for (int j = 0; j < KW; ++j) dw[c][j] = fmaf(dp[u][c], x[(u + 1 + j) & 3][c], dw[c][j]);
-              } else {
-#pragma unroll
-                for (int j = 0; j < KW; ++j)
-                  dw[c][j] = fmaf(dp[u][c], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, dw[c][j]);
-              }
+              for (int j = 0; j < KW; ++j)
+                dw[c][j] = fmaf(dp[u][c], (KW - 1 - j) <= back ? x[(u + 1 + j) & 3][c] : 0.f, dw[c][j]);
             }
           }
         }
-        // dpre of the rows t-3 .. t is complete for the projection row t - 3, as far as they share its sequence
-        const int tr = t - (KW - 1);
-        if (tr >= t0 && tr < t1) {
-          float dx[PER];
+      }
+      // dpre of the rows t-3 .. t is complete for the projection row t - 3, as far as they share its sequence
+      const int tr = t - (KW - 1);
+      if (W || (tr >= t0 && tr < t1)) {
+        float dx[PER];
 #pragma unroll
-          for (int c = 0; c < PER; ++c) dx[c] = 0.f;
+        for (int c = 0; c < PER; ++c) dx[c] = 0.f;
 #pragma unroll
-          for (int j = 0; j < KW; ++j) {         // tap j of row t - j
-            if (start[(u + 4 - j) & 3] <= tr) {
+        for (int j = 0; j < KW; ++j) {           // tap j of row t - j
+          if (W || start[(u + 4 - j) & 3] <= tr) {
 #pragma unroll
-              for (int c = 0; c < PER; ++c) dx[c] = fmaf(w[c][j], dp[(u + 4 - j) & 3][c], dx[c]);
-            }
+            for (int c = 0; c < PER; ++c) dx[c] = fmaf(w[c][j], dp[(u + 4 - j) & 3][c], dx[c]);
           }
-          stn<PER>(dst + tr * p.ld_d, dx);
         }
+        stn<PER>(dst + tr * p.ld_d, dx);
+      }
+    };
+    auto first_token = [&](int t) { return t < te ? p.seq_start[t] : 0x7fffffff; };   // past the batch: in no sequence
+#pragma unroll
+    for (int u = 0; u < KW; ++u) {
+      nf[u] = first_token(t0 + u);
+      if (t0 + u < te) fetch(t0 + u, u);
+    }
+    for (int tb = t0; tb < last; tb += KW) {
+      // four rows and those loaded meanwhile inside the walk, each row's window inside its sequence: straight-line code, in
+      // which the rows overlap
+      bool whole = tb > t0 && tb + KW <= t1 && tb + 2 * KW <= te;
+#pragma unroll
+      for (int u = 0; u < KW; ++u) whole &= tb + u - nf[u] >= KW - 1;
+      if (whole) {
+#pragma unroll
+        for (int u = 0; u < KW; ++u) {
+          start[u] = nf[u];
+          nf[u] = p.seq_start[tb + KW + u];
+        }
+#pragma unroll
+        for (int u = 0; u < KW; ++u) row(std::true_type{}, tb + u, u);
+        continue;
+      }
+#pragma unroll
+      for (int u = 0; u < KW; ++u) {
+        if (tb + u >= last) break;
+        start[u] = nf[u];
+        nf[u] = first_token(tb + KW + u);
+        row(std::false_type{}, tb + u, u);
       }
     }
   }
