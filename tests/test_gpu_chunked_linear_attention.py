@@ -103,7 +103,9 @@ def test_gated_delta_rule_differentiates_twice():
 
 @pytest.mark.parametrize('T,groups,ratio,d,cuts', [(1, 1, 1, 64, []), (3, 2, 2, 128, [1]), (16, 1, 4, 64, [13, 15]),
                                                    (65, 3, 2, 128, [62, 64]), (130, 2, 4, 128, []),
-                                                   (257, 2, 1, 64, [1, 2, 3])])
+                                                   (257, 2, 1, 64, [1, 2, 3]),
+                                                   # sequences that begin between whole groups of four rows
+                                                   (300, 1, 2, 128, [100, 201, 203, 240]), (299, 2, 1, 128, [74])])
 def test_gdn_inputs_walk_edges(T, groups, ratio, d, cuts):
     """Projection -> inputs of the delta rule in one pass, at the edges of a warp's walk (16 / 32 tokens) and of
     sequences."""
