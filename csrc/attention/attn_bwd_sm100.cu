@@ -126,6 +126,19 @@ __device__ __forceinline__ void drain(uint64_t* bar, uint32_t parity) {
 }
 
 // ---------------------------------------------------------------------------------------------------- delta
+// One row's delta is the sum of D / 8 terms of eight channels, term c + term c + D / 16 first, then a half, a quarter ... of that
+// apart: the kernel below and the dq kernel add them in this order, so the bits do not depend on which of them forms delta.
+__device__ __forceinline__ float delta_term(const uint4& o, const uint4& dout) {
+  const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&o), *y = reinterpret_cast<const __nv_bfloat162*>(&dout);
+  float acc = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __bfloat1622float2(x[e]), g = __bfloat1622float2(y[e]);
+    acc += f.x * g.x + f.y * g.y;
+  }
+  return acc;
+}
+
 // D / 8 lanes per (token, head) row, 16-byte loads, 4 rows per lane group in flight: bound by reading O and dO once.
 template <int D>
 __global__ void __launch_bounds__(256)
@@ -146,14 +159,7 @@ attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* 
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u) {
     const long long w = base + u * ROWS;
-    const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&a[u]);
-    const __nv_bfloat162* y = reinterpret_cast<const __nv_bfloat162*>(&b[u]);
-    float acc = 0.f;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = __bfloat1622float2(x[e]), g = __bfloat1622float2(y[e]);
-      acc += f.x * g.x + f.y * g.y;
-    }
+    float acc = delta_term(a[u], b[u]);
 #pragma unroll
     for (int s = LANES / 2; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
     if (c == 0 && w < rows) delta[(w % nq) * T + w / nq] = acc;
@@ -340,25 +346,24 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     // a query that sees nothing has lse = -inf; its probabilities are masked below, keep the arithmetic finite
     const float lse_i = row_ok ? p.lse[(long long)head * p.T + i] : 0.f;
     const float lse2 = (lse_i == -INFINITY) ? 0.f : lse_i * LOG2E;
-    // delta of the row: either warp of a row takes half of the channels, read while the first tiles are on their way
+    // delta of the row, read while the first tiles are on their way: one warp of a row takes the even terms, the other the
+    // odd ones, which the last addition brings together
     float dl;
     if (dp_.o == nullptr) {
       dl = row_ok ? p.delta[(long long)head * p.T + i] : 0.f;
     } else {
       float acc = 0.f;
       if (row_ok) {
-        const long long at = ((long long)i * p.nq + head) * D + grp * (D / 2);
+        const long long at = ((long long)i * p.nq + head) * D + grp * 8;
         const uint4 *po = reinterpret_cast<const uint4*>(dp_.o + at), *pd = reinterpret_cast<const uint4*>(dp_.dout + at);
-#pragma unroll 2
-        for (int c = 0; c < D / 16; ++c) {
-          const uint4 u = po[c], w = pd[c];
-          const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&u), *y = reinterpret_cast<const __nv_bfloat162*>(&w);
+        float term[D / 16];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 f = __bfloat1622float2(x[e]), g = __bfloat1622float2(y[e]);
-            acc += f.x * g.x + f.y * g.y;
-          }
-        }
+        for (int c = 0; c < D / 16; ++c) term[c] = delta_term(po[2 * c], pd[2 * c]);
+#pragma unroll
+        for (int s = D / 32; s; s >>= 1)
+#pragma unroll
+          for (int c = 0; c < s; ++c) term[c] += term[c + s];
+        acc = term[0];
       }
       float* s_delta = reinterpret_cast<float*>(smem + L::OFF_BAR + 512);   // [TM], behind the barriers
       if (grp == 1) s_delta[r] = acc;

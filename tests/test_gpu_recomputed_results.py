@@ -182,3 +182,32 @@ def test_expert_rows_are_summed_in_order(T, k, H):
         want += torch.where(hit[:, j, None], y[sent[:, j].clamp(min=0).long()].float(), 0.)
     assert torch.equal(out, want.bfloat16())
     assert torch.equal(got, torch.where(hit, scalar[sent.clamp(min=0).long()], 0.))
+
+
+@pytest.mark.parametrize('T,nq,d', [(1, 1, 64), (200, 4, 64), (130, 3, 128),      # delta formed in the dQ kernel
+                                    (3641, 9, 128)])                               # by the kernel of its own: 32769 rows
+def test_attention_delta_has_one_order_of_sums(T, nq, d):
+    """delta of a row has the same bits whichever kernel forms it: eight products of bf16 values, which are exact in fp32, added in
+    pairs, then a tree over the D / 8 sums."""
+    import ctypes
+
+    from mcore_bridge_b200.ops import _lib
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    q, o, do = (torch.randn(T, nq, d, generator=gen, device=DEV).bfloat16() for _ in range(3))
+    k, v = (torch.randn(T, 1, d, generator=gen, device=DEV).bfloat16() for _ in range(2))
+    lse = torch.full((nq, T), 10.0, device=DEV)
+    start = torch.zeros(T, dtype=torch.int32, device=DEV)
+    delta = torch.full((nq, T), float('nan'), device=DEV)
+    dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+    rc = _lib.lib().mcb_attn_bwd_ranges(*map(_lib.ptr, (q, k, v, o, do, lse, delta)), ctypes.c_int(0), _lib.ptr(start), None, None,
+                                        None, _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), *map(ctypes.c_int, (T, T, nq, 1, d)),
+                                        ctypes.c_float(0.1), None, ctypes.c_int(1), _lib.ptr(_lib.status_word(q.device)),
+                                        _lib.stream_ptr())
+    _lib.check_rc(rc, 'mcb_attn_bwd_ranges')
+    pairs = (o.float() * do.float()).view(T, nq, d // 8, 4, 2)
+    pairs = pairs[..., 0] + pairs[..., 1]
+    term = ((pairs[..., 0] + pairs[..., 1]) + pairs[..., 2]) + pairs[..., 3]
+    while term.shape[-1] > 1:
+        half = term.shape[-1] // 2
+        term = term[..., :half] + term[..., half:]
+    assert torch.equal(delta, term[..., 0].t())
