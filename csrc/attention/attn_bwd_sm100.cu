@@ -823,35 +823,6 @@ __global__ void attn_bwd_reduce_kernel(const float* __restrict__ partial, __nv_b
   }
 }
 
-// Gradient of the per-head sink logits: one more softmax column with a zero value vector, so
-// d sink_h = -sum_i exp(sink_h - lse(h, i)) delta(h, i).  One CTA per head, sums in a fixed order.
-constexpr int SINK_THREADS = 512;
-__global__ void __launch_bounds__(SINK_THREADS)
-attn_sink_grad_kernel(const float* __restrict__ sinks, const float* __restrict__ lse, const float* __restrict__ delta, int T,
-                      void* __restrict__ out, int out_bf16) {
-  __shared__ float red[SINK_THREADS / 32];
-  const int h = blockIdx.x;
-  const float sink = sinks[h];
-  float acc = 0.f;
-  for (int i = threadIdx.x; i < T; i += SINK_THREADS) {
-    // exp(x) as 2^(x log2 e) with the rounding error of the product put back: ex2's own two ulp remain
-    const float x = sink - lse[(long long)h * T + i], t = x * LOG2E;
-    const float lo = fmaf(x, LOG2E, -t) + x * 1.925963033500e-8f;
-    const float e = ex2_ftz(t);
-    acc += (t > -126.f ? fmaf(e, lo * 0.6931471805599453f, e) : e) * delta[(long long)h * T + i];
-  }
-#pragma unroll
-  for (int s = 16; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float sum = 0.f;
-    for (int w = 0; w < SINK_THREADS / 32; ++w) sum += red[w];
-    if (out_bf16) reinterpret_cast<__nv_bfloat16*>(out)[h] = __float2bfloat16(-sum);
-    else reinterpret_cast<float*>(out)[h] = -sum;
-  }
-}
-
 template <int D>
 int launch_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, float* delta, bool delta_given,
                const BwdParams& p, cudaStream_t stream) {
@@ -931,15 +902,6 @@ int mcb_attn_bwd_ranges(const void* q, const void* k, const void* v, const void*
   if (d == 128) return launch_bwd<128>(q, k, v, o, dout, delta, delta_given != 0, p, s);
   if (d == 64) return launch_bwd<64>(q, k, v, o, dout, delta, delta_given != 0, p, s);
   return -3;
-}
-
-// d sinks [nq] (fp32, or bf16 with out_bf16) of the forward's sinks [nq] fp32, from lse and delta [nq, T].
-int mcb_attn_sink_grad(const float* sinks, const float* lse, const float* delta, void* out, int out_bf16, int T, int nq,
-                       void* stream_) {
-  if (nq <= 0) return 0;
-  attn_sink_grad_kernel<<<(unsigned)nq, SINK_THREADS, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(sinks, lse, delta, T, out,
-                                                                                                  out_bf16);
-  return (int)cudaGetLastError();
 }
 
 // Packed causal self-attention: seq_start [T] int32 = first token of each token's sequence.

@@ -211,3 +211,25 @@ def test_attention_delta_has_one_order_of_sums(T, nq, d):
         half = term.shape[-1] // 2
         term = term[..., :half] + term[..., half:]
     assert torch.equal(delta, term[..., 0].t())
+
+
+@pytest.mark.parametrize('nq,T', [(4096, 1), (3, 2050), (2, 70001)])    # one term; a few and many terms a thread
+def test_sink_gradient_in_full_fp32_precision(nq, T):
+    import ctypes
+
+    from mcore_bridge_b200.ops import _lib
+    gen = torch.Generator(device=DEV).manual_seed(10)
+    # differences of multiples of 2^-12 below 64 are exact in fp32
+    sinks = torch.randint(-4096 * 8, 4096 * 8, (nq,), generator=gen, device=DEV) / 4096
+    lse = sinks[:, None] + torch.randint(0, 4096 * 16, (nq, T), generator=gen, device=DEV) / 4096
+    delta = torch.randn(nq, T, generator=gen, device=DEV)
+    out = torch.empty(nq, device=DEV)
+    rc = _lib.lib().mcb_attn_sink_grad(*map(_lib.ptr, (sinks, lse, delta, out)), *map(ctypes.c_int, (0, T, nq)),
+                                       _lib.stream_ptr())
+    _lib.check_rc(rc, 'mcb_attn_sink_grad')
+    terms = torch.exp(sinks.double()[:, None] - lse.double()) * delta.double()
+    # expf is within one unit in the last place (2^-23), a product rounds by half of one; then a thread's sums, its warp's
+    # five and the block's sixteen round by half of one of a partial sum each
+    adds = (T + 511) // 512 - 1 + 5 + 16 if T > 1 else 0
+    bound = (1.5 + 0.5 * adds) * 2.0 ** -23 * terms.abs().sum(1)
+    assert ((out.double() + terms.sum(1)).abs() <= bound).all()
