@@ -126,8 +126,8 @@ __device__ __forceinline__ void drain(uint64_t* bar, uint32_t parity) {
 }
 
 // ---------------------------------------------------------------------------------------------------- delta
-// One row's delta is the sum of D / 8 terms of eight channels, term c + term c + D / 16 first, then a half, a quarter ... of that
-// apart: the kernel below and the dq kernel add them in this order, so the bits do not depend on which of them forms delta.
+// One row's delta is the sum of D / 8 terms of eight channels, each held by a lane: the kernel below and the dq kernel form and add
+// them the same way, so the bits do not depend on which of them forms delta.
 __device__ __forceinline__ float delta_term(const uint4& o, const uint4& dout) {
   const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&o), *y = reinterpret_cast<const __nv_bfloat162*>(&dout);
   float acc = 0.f;
@@ -136,6 +136,12 @@ __device__ __forceinline__ float delta_term(const uint4& o, const uint4& dout) {
     const float2 f = __bfloat1622float2(x[e]), g = __bfloat1622float2(y[e]);
     acc += f.x * g.x + f.y * g.y;
   }
+  return acc;
+}
+template <int LANES>
+__device__ __forceinline__ float delta_sum(float acc) {
+#pragma unroll
+  for (int s = LANES / 2; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
   return acc;
 }
 
@@ -159,9 +165,7 @@ attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* 
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u) {
     const long long w = base + u * ROWS;
-    float acc = delta_term(a[u], b[u]);
-#pragma unroll
-    for (int s = LANES / 2; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    const float acc = delta_sum<LANES>(delta_term(a[u], b[u]));
     if (c == 0 && w < rows) delta[(w % nq) * T + w / nq] = acc;
   }
 }
@@ -346,31 +350,28 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     // a query that sees nothing has lse = -inf; its probabilities are masked below, keep the arithmetic finite
     const float lse_i = row_ok ? p.lse[(long long)head * p.T + i] : 0.f;
     const float lse2 = (lse_i == -INFINITY) ? 0.f : lse_i * LOG2E;
-    // delta of the row, read while the first tiles are on their way: one warp of a row takes the even terms, the other the
-    // odd ones, which the last addition brings together
     float dl;
     if (dp_.o == nullptr) {
       dl = row_ok ? p.delta[(long long)head * p.T + i] : 0.f;
     } else {
-      float acc = 0.f;
-      if (row_ok) {
-        const long long at = ((long long)i * p.nq + head) * D + grp * 8;
-        const uint4 *po = reinterpret_cast<const uint4*>(dp_.o + at), *pd = reinterpret_cast<const uint4*>(dp_.dout + at);
-        float term[D / 16];
-#pragma unroll
-        for (int c = 0; c < D / 16; ++c) term[c] = delta_term(po[2 * c], pd[2 * c]);
-#pragma unroll
-        for (int s = D / 32; s; s >>= 1)
-#pragma unroll
-          for (int c = 0; c < s; ++c) term[c] += term[c + s];
-        acc = term[0];
-      }
+      // delta of the tile's rows while the first tiles are on their way, 16 rows a warp, with the lanes of delta's own kernel
+      constexpr int LANES = D / 8, ROWS = 32 / LANES;
       float* s_delta = reinterpret_cast<float*>(smem + L::OFF_BAR + 512);   // [TM], behind the barriers
-      if (grp == 1) s_delta[r] = acc;
+      const int row0 = (warp - 4) * 16 + lane / LANES;
+      uint4 a[16 / ROWS], b[16 / ROWS];
+#pragma unroll
+      for (int u = 0; u < 16 / ROWS; ++u) {
+        const long long at = ((long long)min(m0 + row0 + u * ROWS, p.T - 1) * p.nq + head) * D + lane % LANES * 8;
+        a[u] = *reinterpret_cast<const uint4*>(dp_.o + at);
+        b[u] = *reinterpret_cast<const uint4*>(dp_.dout + at);
+      }
+#pragma unroll
+      for (int u = 0; u < 16 / ROWS; ++u) {
+        const float acc = delta_sum<LANES>(delta_term(a[u], b[u]));
+        if (lane % LANES == 0) s_delta[row0 + u * ROWS] = acc;
+      }
       asm volatile("bar.sync 1, 256;" ::: "memory");       // the eight element-wise warps, before any bounded wait
-      if (grp == 0) s_delta[r] = acc = acc + s_delta[r];
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      dl = grp == 0 ? acc : s_delta[r];
+      dl = row_ok ? s_delta[r] : 0.f;
       if (row_ok && grp == 0) dp_.delta[(long long)head * p.T + i] = dl;
     }
     const uint64_t cc = f32x2(p.scale_log2, p.scale_log2), nl = f32x2(-lse2, -lse2), nd = f32x2(-dl, -dl);
@@ -838,9 +839,9 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* o, const
   DeltaParams dp{nullptr, nullptr, nullptr};
   if (!delta_given) {
     if (reinterpret_cast<uintptr_t>(o) & 15) return -6;
-    // The dq kernel reads a row of O and dO per thread, longer for heads of 128; the kernel of its own costs a launch and a
-    // pass.  delta + dq + dk/dv, us, own kernel and in dq: 4095 tokens, 64 heads of 64, window 128 284 / 257, 4096, 24 of 64
-    // 320 / 317, 333, 4 of 64 32 / 29; 3000, 9 of 128 203 / 188, 2048, 32 of 128 194 / 196, 8192, 32 of 128 561 / 573.
+    // In the dq kernel delta delays the first block, by twice as many rows of loads for heads of 128; the kernel of its own costs a
+    // launch and a pass.  delta + dq + dk/dv, us, own kernel and in dq: 4095 tokens, 64 heads of 64, window 128 284 / 250, 4096,
+    // 24 of 64 320 / 315, 333, 4 of 64 32 / 28; 3000, 9 of 128 203 / 186, 2048, 32 of 128 194 / 196, 8192, 32 of 128 561 / 573.
     const long long rows = (long long)p.T * p.nq;
     if (D == 64 || rows <= 32768) {
       dp = DeltaParams{(const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta};
