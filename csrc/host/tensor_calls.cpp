@@ -159,6 +159,13 @@ PyObject* tuple(std::initializer_list<Tensor> ts) {
   return r;
 }
 
+// What a kernel reads one int32 of per query or key from: at least n of them, beside the operands.
+Tensor per_token(const Tensor& t, ll n, const Tensor& like, const char* what) {
+  if (!t.defined()) return t;
+  require(t.scalar_type() == at::kInt && t.numel() >= n && t.device() == like.device(), what);
+  return t.contiguous();
+}
+
 enum Layout { NT = 0, NN = 1, TN = 2 };
 
 // c = op(a) . op(b): NT a [M, K], b [N, K]; NN a [M, K], b [K, N]; TN a [K, M], b [K, N]
@@ -402,9 +409,11 @@ PyObject* qkv_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   MCB_BEGIN(7)
   const Tensor q = tensor(a[0]).contiguous(), k = tensor(a[1]).contiguous(), v = tensor(a[2]).contiguous();
-  const Tensor &k_lo = tensor(a[3]);
-  const Tensor k_hi = optional(a[4]), sinks = optional(a[5]);
   const ll T = q.size(0), nq = q.size(1), d = q.size(2);
+  const Tensor k_lo = per_token(tensor(a[3]), T, q, "first keys: an int32 for every query, on the queries' device"),
+               k_hi = per_token(optional(a[4]), T, q, "last keys: an int32 for every query, on the queries' device"),
+               sinks = optional(a[5]);
+  require(!sinks.defined() || (sinks.numel() >= nq && sinks.device() == q.device()), "sinks: one for every head");
   const Tensor o = at::empty_like(q), lse = at::empty({nq, T}, q.options().dtype(at::kFloat));
   launch("mcb_attn_fwd_ranges", mcb_attn_fwd_ranges, q.data_ptr(), k.data_ptr(), v.data_ptr(), k_lo.data_ptr(), ptr(k_hi),
          ptr(sinks), o.data_ptr(), lse.data_ptr(), T, k.size(0), nq, k.size(1), d, real(a[6]), status_of(q), stream());
@@ -416,10 +425,12 @@ PyObject* attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* attn_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   MCB_BEGIN(13)
   const Tensor dout = tensor(a[0]).contiguous();
-  const Tensor &q = tensor(a[1]), &k = tensor(a[2]), &v = tensor(a[3]), &o = tensor(a[4]), &lse = tensor(a[5]),
-               &k_lo = tensor(a[6]);
-  const Tensor k_hi = optional(a[7]), q_lo = optional(a[8]), q_hi = optional(a[9]);
+  const Tensor &q = tensor(a[1]), &k = tensor(a[2]), &v = tensor(a[3]), &o = tensor(a[4]), &lse = tensor(a[5]);
   const ll T = q.size(0), Tk = k.size(0), d = q.size(2);
+  const Tensor k_lo = per_token(tensor(a[6]), T, q, "first keys: an int32 for every query, on the queries' device"),
+               k_hi = per_token(optional(a[7]), T, q, "last keys: an int32 for every query, on the queries' device"),
+               q_lo = per_token(optional(a[8]), Tk, q, "first queries: an int32 for every key, on the keys' device"),
+               q_hi = per_token(optional(a[9]), Tk, q, "last queries: an int32 for every key, on the keys' device");
   const int nq = static_cast<int>(q.size(1)), nkv = static_cast<int>(k.size(1));
   const Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
   const Tensor delta = at::empty({nq, T}, lse.options());
@@ -443,7 +454,7 @@ PyObject* attn_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 PyObject* attn_window_starts(PyObject*, PyObject* const* a, Py_ssize_t n) {   // seq_start, left -> first visible keys
   MCB_BEGIN(2)
-  const Tensor start = tensor(a[0]).contiguous();
+  const Tensor start = per_token(tensor(a[0]), 0, tensor(a[0]), "sequence starts: int32");
   const ll left = integer(a[1]);
   const Tensor out = at::empty_like(start);
   launch("mcb_attn_window_starts", mcb_attn_window_starts, start.data_ptr(), out.data_ptr(), start.numel(),

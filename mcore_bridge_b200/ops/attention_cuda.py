@@ -50,6 +50,22 @@ def seq_start_from_cu(cu_seqlens: Optional[torch.Tensor], T: int, device) -> tor
     return cu[:-1][seg.clamp(max=cu.numel() - 2)].to(torch.int32)
 
 
+def _row_starts(seq_start: torch.Tensor, T: int, device, one_each: bool) -> torch.Tensor:
+    """``seq_start`` as the kernels read it: ``T`` int32 on ``device``, one after the other.  A single value counts for every
+    token; more than ``T`` are refused with ``one_each``."""
+    if seq_start.dtype == torch.int32 and seq_start.shape == (T,) and seq_start.device == device:
+        return seq_start.contiguous()
+    n = seq_start.numel()
+    if n != 1 and (n < T or (one_each and n != T)):
+        raise RuntimeError(f'seq_start has {n} elements for {T} tokens')
+    if seq_start.is_floating_point() or seq_start.is_complex():
+        raise RuntimeError(f'seq_start is {seq_start.dtype}: whole numbers are wanted')
+    if seq_start.device != device and seq_start.dim() > 0:
+        raise RuntimeError(f'seq_start is on {seq_start.device}, the queries are on {device}')
+    seq_start = seq_start.to(device=device, dtype=torch.int32).reshape(-1)
+    return (seq_start.expand(T) if n == 1 else seq_start[:T]).contiguous()
+
+
 def _dkv_splits(T: int, nq: int, nkv: int, device) -> int:
     """How many CTAs share one (key tile, kv head) pair in the dK/dV kernel: enough to put at least about three
     CTAs on every SM, limited to divisors of the GQA ratio.  ``MCB200_ATTN_DKV_SPLITS`` overrides it."""
@@ -95,13 +111,14 @@ def attention(q, k, v, cu_seqlens, max_seqlen, scale, seq_start: Optional[torch.
     if max_seqlen is None and cu_seqlens is not None:
         max_seqlen = T
     left = None if window is None or window[0] is None or int(window[0]) < 0 else int(window[0])
+    seq_start = _row_starts(seq_start, T, q.device, left is not None)
     if left is None and sinks is None:
         return _AttnFn.apply(q, k, v, seq_start, cu_seqlens, max_seqlen, float(scale))
     k_lo = seq_start
     if left is not None:
         # still non-decreasing, so the kernels' causal fast paths (k_hi = the query itself) apply unchanged
         k_lo = _lib.native().attn_window_starts(seq_start, left)
-    o, _ = attention_ranges(q, k, v, k_lo.contiguous(), None, None, None, scale, sinks)
+    o, _ = attention_ranges(q, k, v, k_lo, None, None, None, scale, sinks)
     return o
 
 
