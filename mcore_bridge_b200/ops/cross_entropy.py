@@ -217,7 +217,7 @@ def vocab_parallel_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, gro
 class _FusedLinearCE(torch.autograd.Function):
 
     @staticmethod
-    def forward(ctx, h, weight, labels, group_name, chunk):
+    def forward(ctx, h, weight, labels, group_name, chunk, graph):
         n, r, group = _tp_info(group_name)
         vl, H = weight.shape
         h2 = h.reshape(-1, H)
@@ -227,7 +227,7 @@ class _FusedLinearCE(torch.autograd.Function):
             h2 = h2.contiguous()
         if _head_kernel_ok(h2, weight):
             # not a saved tensor: hooks that move those to the host would move far more than the product costs
-            ctx.logits = _logits_to_keep(T, vl, H, h2.device) if any(ctx.needs_input_grad) else None
+            ctx.logits = _logits_to_keep(T, vl, H, h2.device) if graph else None
             m, s, tgt = _head_stats(h2, weight, lab, r * vl, ctx.logits)
             lse_all, tgt = _combine(m, s, tgt, group_name, group)
             ctx.save_for_backward(h2, weight, lab, lse_all)
@@ -291,10 +291,12 @@ class _FusedLinearCE(torch.autograd.Function):
             hook = getattr(weight, 'grad_ready_hook', None)
             if hook is not None:
                 hook()
-        return dh.view(hshape), (dw.to(weight.dtype) if dw is not None else None), None, None, None
+        return dh.view(hshape), (dw.to(weight.dtype) if dw is not None else None), None, None, None, None
 
 
 def fused_linear_cross_entropy(h: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor, group: str = 'tp',
                                chunk: int = 4096) -> torch.Tensor:
     """``h [T, H]`` (full sequence on every TP rank), ``weight [V/tp, H]``, ``labels [T]`` -> loss ``[T]`` fp32."""
-    return _FusedLinearCE.apply(h, weight, labels, group, chunk)
+    # asked here: inside the function grad mode is off, and ``needs_input_grad`` does not depend on it
+    graph = torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad)
+    return _FusedLinearCE.apply(h, weight, labels, group, chunk, graph)
