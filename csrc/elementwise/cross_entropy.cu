@@ -1,7 +1,9 @@
 // Softmax statistics and gradient for (vocab-parallel) cross entropy over one chunk of logits.
 //   mcb_ce_stats   : per row max, sum exp(l - max) and the target logit (0 when the label is in another shard)
 //   mcb_ce_dlogits : (exp(l - lse) - onehot(label)) * g  written as bf16 or fp32
+//   mcb_ce_dlogits_head : the same of the head's own fp32 logits, bit for bit what its GEMM's gradient epilogue writes
 // One block per row, 16-byte loads, a single pass (online max/sum).
+#include "../common/ce_math.cuh"
 #include "../common/host_utils.cuh"
 #include "../common/ptx.cuh"
 
@@ -97,14 +99,14 @@ ce_stats_kernel(const void* __restrict__ logits, long long ld, const long long* 
   }
 }
 
-template <bool FP32_IN, bool FP32_OUT>
+template <bool FP32_IN, bool FP32_OUT, bool HEAD = false>
 __global__ void __launch_bounds__(CE_THREADS)
 ce_dlogits_kernel(const void* __restrict__ logits, long long ld, const long long* __restrict__ labels,
                   const float* __restrict__ lse, const float* __restrict__ g, long long rows, int V, int vocab_start,
                   void* __restrict__ out) {
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const long long base = row * ld, obase = row * (long long)V;
-    const float l = lse[row], gr = g[row];
+    const float l = HEAD ? lse[row] * CE_LOG2E : lse[row], gr = g[row];
     const long long lab = labels[row] - vocab_start;
     const int nvec = V / 8;
     for (int vi = threadIdx.x; vi < nvec; vi += CE_THREADS) {
@@ -112,7 +114,7 @@ ce_dlogits_kernel(const void* __restrict__ logits, long long ld, const long long
       load8<FP32_IN>(logits, base + (long long)vi * 8, f);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        float p = __expf(f[j] - l);
+        float p = HEAD ? ce_prob(f[j], l) : __expf(f[j] - l);
         if ((long long)vi * 8 + j == lab) p -= 1.f;
         f[j] = p * gr;
       }
@@ -130,7 +132,8 @@ ce_dlogits_kernel(const void* __restrict__ logits, long long ld, const long long
       }
     }
     for (int i = nvec * 8 + threadIdx.x; i < V; i += CE_THREADS) {
-      float p = __expf(load1<FP32_IN>(logits, base + i) - l);
+      const float x = load1<FP32_IN>(logits, base + i);
+      float p = HEAD ? ce_prob(x, l) : __expf(x - l);
       if (i == lab) p -= 1.f;
       p *= gr;
       if (FP32_OUT) reinterpret_cast<float*>(out)[obase + i] = p;
@@ -170,6 +173,17 @@ int mcb_ce_dlogits(const void* logits, int fp32_in, long long ld, const long lon
   else if (fp32_out) L(false, true);
   else L(false, false);
 #undef L
+  return (int)cudaGetLastError();
+}
+
+// logits [rows, V] fp32 and out [rows, V] bf16, contiguous, on 16-byte boundaries
+int mcb_ce_dlogits_head(const float* logits, const long long* labels, const float* lse, const float* g, long long rows, int V,
+                        int vocab_start, void* out, void* stream_) {
+  if (rows == 0) return 0;
+  if (V % 8 || (reinterpret_cast<uintptr_t>(logits) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return -1;
+  const long long cap = (long long)device_sm_count() * 4;
+  ce_dlogits_kernel<true, false, true><<<(int)(rows < cap ? rows : cap), CE_THREADS, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(
+      logits, V, labels, lse, g, rows, V, vocab_start, out);
   return (int)cudaGetLastError();
 }
 

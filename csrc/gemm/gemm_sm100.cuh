@@ -20,6 +20,7 @@
 // 225 / 204, 64-wide 528 / 380 / 271, CTA pairs 185 / 171 / 171; 776 x 2048 x 12288 63 / 46 / 42, with B MN-major 63 / 53 / 39;
 // 512 x 512 x 4096 both MN-major 23 / 21 / 13.
 #pragma once
+#include "../common/ce_math.cuh"
 #include "../common/ptx.cuh"
 
 namespace mcb {
@@ -176,7 +177,7 @@ __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* 
 template <int BN, int EPI>
 __device__ __forceinline__ void epilogue_ce(const GemmParams& p, uint32_t tmem_row, int row, bool row_ok, int n0, int tiles_n,
                                             uint8_t* stage) {
-  constexpr float LOG2E = 1.4426950408889634f;
+  constexpr float LOG2E = CE_LOG2E;
   const bool vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
   const int label_col = row_ok ? (int)(p.ce_labels[row] - p.ce_col0) - n0 : -1;   // column inside this tile
   float run_m = -INFINITY, run_s = 0.f, tgt = 0.f;
@@ -232,7 +233,7 @@ __device__ __forceinline__ void epilogue_ce(const GemmParams& p, uint32_t tmem_r
       float v[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        v[j] = (exp2f(__uint_as_float(r[j]) * p.alpha * LOG2E - lse2) - (j == lj ? 1.f : 0.f)) * g;
+        v[j] = (ce_prob(__uint_as_float(r[j]) * p.alpha, lse2) - (j == lj ? 1.f : 0.f)) * g;
       __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)row * p.ldc + n0 + cc;
       if (vec_ok && valid == 32) {
 #pragma unroll

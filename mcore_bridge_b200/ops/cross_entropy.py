@@ -188,6 +188,16 @@ def _head_dlogits(h2, weight, lab, vocab_start, lse, g):
     return d
 
 
+def _kept_dlogits(logits, lab, vocab_start, lse, g):
+    """What :func:`_head_dlogits` forms, from logits that the forward pass kept: the same bits."""
+    rows, vl = logits.shape
+    d = torch.empty((rows, vl), dtype=torch.bfloat16, device=logits.device)
+    rc = _lib.lib().mcb_ce_dlogits_head(_lib.ptr(logits), _lib.ptr(lab), _lib.ptr(lse), _lib.ptr(g), _ll(rows), _int(vl),
+                                        _int(vocab_start), _lib.ptr(d), _lib.stream_ptr())
+    _lib.check_rc(rc, 'mcb_ce_dlogits_head')
+    return d
+
+
 class _VocabParallelCE(torch.autograd.Function):
 
     @staticmethod
@@ -271,7 +281,7 @@ class _FusedLinearCE(torch.autograd.Function):
         for s0 in range(0, T, chunk):
             s1 = min(T, s0 + chunk)
             if kept is not None:
-                d = _dlogits(kept[s0:s1], lab[s0:s1], vstart, lse[s0:s1], g[s0:s1], h2.dtype)
+                d = _kept_dlogits(kept[s0:s1], lab[s0:s1], vstart, lse[s0:s1], g[s0:s1])
             elif fused:
                 d = _head_dlogits(h2[s0:s1], weight, lab[s0:s1], vstart, lse[s0:s1], g[s0:s1])
             else:

@@ -23,6 +23,7 @@ def asked(monkeypatch):
     monkeypatch.setattr(ce, '_head_kernel_ok', lambda h2, weight: True)
     monkeypatch.setattr(ce, '_logits_to_keep', keep)
     monkeypatch.setattr(ce, '_head_stats', stats)
+    monkeypatch.setattr(ce, '_kept_dlogits', lambda *a: ce._dlogits(*a, torch.float32))
     return seen
 
 
@@ -71,3 +72,20 @@ def test_a_loss_without_gradients_allocates_no_logits():
             base = torch.cuda.memory_allocated()
             ce.fused_linear_cross_entropy(h, w, lab)
             assert torch.cuda.max_memory_allocated() - base < 4 * T * V // 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('T,V,H,chunk', [(515, 4104, 1024, 4096),      # a last column tile with 8 columns
+                                         (1, 264, 1032, 4096),
+                                         (1030, 2056, 1024, 600),      # two chunks
+                                         (1100, 8200, 1024, 4096)])    # the gradient epilogue on CTA pairs
+def test_kept_and_repeated_logits_give_the_same_bits(T, V, H, chunk):
+    gen = torch.Generator(device='cuda').manual_seed(4)
+    h = torch.randn(T, H, generator=gen, device='cuda').bfloat16().requires_grad_()
+    w = (torch.randn(V, H, generator=gen, device='cuda') * 0.05).bfloat16().requires_grad_()
+    lab = torch.randint(0, V, (T,), generator=gen, device='cuda')
+    g = torch.rand(T, generator=gen, device='cuda')
+    loss = ce.fused_linear_cross_entropy(h, w, lab, chunk=chunk)
+    kept = torch.autograd.grad(loss, (h, w), g, retain_graph=True)
+    again = torch.autograd.grad(loss, (h, w), g)
+    assert torch.equal(kept[0], again[0]) and torch.equal(kept[1], again[1])
