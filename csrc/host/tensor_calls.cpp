@@ -8,6 +8,7 @@
 #include <dlfcn.h>
 
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -476,6 +477,14 @@ PyObject* raw_stream(PyObject*, PyObject*) {
   END_HANDLE_TH_ERRORS
 }
 
+PyObject* memory(PyObject*, PyObject* const* a, Py_ssize_t n) {   // device -> bytes the caching allocator holds, and has given out
+  MCB_BEGIN(1)
+  const auto s = c10::cuda::CUDACachingAllocator::getDeviceStats(static_cast<c10::DeviceIndex>(integer(a[0])));
+  const size_t all = static_cast<size_t>(c10::CachingAllocator::StatType::AGGREGATE);
+  return Py_BuildValue("LL", static_cast<ll>(s.reserved_bytes[all].current), static_cast<ll>(s.allocated_bytes[all].current));
+  MCB_END
+}
+
 PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t n) {   // path of libmcb200.so, exception class, status callback
   MCB_BEGIN(3)
   const char* path = PyUnicode_AsUTF8(a[0]);
@@ -503,6 +512,7 @@ PyMethodDef methods[] = {MCB_FAST(init),
                          {"enabled", enabled, METH_NOARGS, nullptr},
                          {"launches", launches, METH_NOARGS, nullptr},
                          {"raw_stream", raw_stream, METH_NOARGS, nullptr},
+                         MCB_FAST(memory),
                          MCB_FAST(mm),
                          MCB_FAST(rmsnorm_fwd),
                          MCB_FAST(rmsnorm_bwd),

@@ -23,7 +23,7 @@ from torch import nn
 from ..layers.context import ForwardContext, PackedSeqParams
 from ..layers.embedding import LanguageModelEmbedding
 from ..layers.linear import ColumnParallelLinear, ReplicatedLinear
-from ..ops.cross_entropy import fused_linear_cross_entropy, vocab_parallel_cross_entropy
+from ..ops.cross_entropy import fused_linear_cross_entropy, release_kept_logits, vocab_parallel_cross_entropy
 from ..ops.linear import LinearSpec, linear
 from ..parallel import mappings as M
 from ..parallel import state as ps
@@ -194,6 +194,7 @@ class GPTModel(nn.Module):
             ref = labels if labels is not None else position_ids
             batch, seq = ref.shape[-2], ref.shape[-1]
             device = ref.device
+        release_kept_logits(device)
         ctx = self.build_context(input_ids, position_ids, attention_mask, packed_seq_params, batch, seq, device)
         if extra_block_kwargs:
             ctx.extra.update(extra_block_kwargs)

@@ -17,6 +17,8 @@ Both return the per-token loss ``[T]`` in fp32 (the caller masks and averages).
 from __future__ import annotations
 
 import ctypes
+import threading
+import weakref
 
 import torch
 import torch.distributed as dist
@@ -134,27 +136,88 @@ def _head_kernel_ok(h2, weight) -> bool:
 
 
 _KEEP_MIN_HIDDEN = 1024
+_KEEP_SHARE = 32                 # of a device's memory, all kept logits together
+_KEEP_ASK = 1 << 28              # buffers from here on ask the driver what is free each time
 
 
-def _logits_to_keep(T, vl, H, device):
+class _Kept:
+    """Logits that a graph holds for its backward pass, until that or :func:`release_kept_logits` takes them."""
+
+    def __init__(self, logits):
+        self.logits = logits
+        with _kept_lock:
+            _kept.add(self)
+
+    def take(self):
+        return self.__dict__.pop('logits', None)       # one of several threads gets them
+
+
+_kept: 'weakref.WeakSet[_Kept]' = weakref.WeakSet()
+_kept_lock = threading.Lock()
+_device_bytes: dict = {}         # device -> its memory
+_driver_free: dict = {}          # device -> (bytes the allocator held, bytes the driver had left for it) when last asked
+
+
+def _kept_on(device) -> list:
+    """``(holder, logits)`` of the graphs on ``device`` that hold some."""
+    if not len(_kept):
+        return []
+    with _kept_lock:
+        pairs = [(k, k.__dict__.get('logits')) for k in _kept]
+    return [(k, t) for k, t in pairs if t is not None and t.device == device]
+
+
+def release_kept_logits(device) -> None:
+    """Gives back the logits that graphs still hold: their backward passes form them again, with the same bits.  A model calls
+    this before a forward pass, whose activations had that memory to themselves when no logits were kept."""
+    for holder, _ in _kept_on(device):
+        holder.take()
+
+
+def _memory_left(device, need: int) -> int:
+    """Bytes this process can still allocate: unused ones of its allocator and what the driver has for it.  The driver takes
+    60 to 130 us; a small buffer makes do with its answer of the last time the allocator grew or shrank."""
+    reserved, allocated = _lib.native().memory(device.index)
+    seen = _driver_free.get(device.index)
+    if need > _KEEP_ASK or seen is None or seen[0] != reserved:
+        free, total = torch.cuda.mem_get_info(device)
+        own = int(torch.cuda.get_per_process_memory_fraction(device) * total) - reserved
+        seen = _driver_free[device.index] = (reserved, max(0, min(free, own)))
+    return reserved - allocated + seen[1]
+
+
+def _logits_to_keep(T, vl, H, device, backward: int = 0):
     """A ``[T, vl]`` fp32 buffer that saves the backward pass the second head product, or ``None``.
 
     A kept logit costs 8 bytes of traffic and 4 of memory until the backward pass, a recomputed one ``2 H`` operations: at
     6.5 TB/s and 1.4 PFLOP/s the two are even near ``H`` = 860.  Forward + backward, us, recomputed and kept: 4096 x 151936
-    at ``H`` 4096 14808 / 12990, 2048 7173 / 6743, 1024 4420 / 3941; 64 x 151936 at 4096 1347 / 1165.  Buffers above 256 MB
-    are kept only where the device has four times as much to spare, so that what fits into memory does not depend on it."""
-    if T == 0 or vl % 8 or H < _KEEP_MIN_HIDDEN:
+    at ``H`` 4096 14808 / 12990, 2048 7173 / 6743, 1024 4420 / 3941; 64 x 151936 at 4096 1347 / 1165.
+
+    Memory comes first: a buffer is kept where the device has four times as much to spare beyond the ``backward`` bytes the
+    head's own backward pass allocates, and where all that are kept stay within a 32nd of the device.  In a captured graph a
+    buffer would last as long as the graph, so none is kept there."""
+    if T == 0 or vl % 8 or H < _KEEP_MIN_HIDDEN or torch.cuda.is_current_stream_capturing():
         return None
     need = 4 * T * vl
-    if need > 1 << 28:
-        stats = torch.cuda.memory_stats_as_nested_dict(device)
-        cached = stats['reserved_bytes']['all']['current'] - stats['allocated_bytes']['all']['current']
-        if torch.cuda.mem_get_info(device)[0] + cached < 4 * need:
-            return None
+    held = sum(4 * t.numel() for _, t in _kept_on(device))
+    if device not in _device_bytes:
+        _device_bytes[device] = torch.cuda.get_device_properties(device).total_memory
+    if (held + need) * _KEEP_SHARE > _device_bytes[device]:
+        return None
+    if _memory_left(device, need) < 4 * need + backward:
+        return None
     try:
         return torch.empty((T, vl), dtype=torch.float32, device=device)
     except torch.OutOfMemoryError:       # free, but in pieces
         return None
+
+
+def _backward_bytes(T, chunk, weight, need_dh, need_dw) -> int:
+    """What the head's backward pass allocates beside kept logits: a chunk's gradient of the logits and the results."""
+    vl, H = weight.shape
+    one = T <= chunk
+    dw = 0 if not need_dw or getattr(weight, 'main_grad', None) is not None else (2 if one else 6) * vl * H
+    return 2 * min(T, chunk) * vl + 2 * T * H * need_dh + dw
 
 
 def _head_stats(h2, weight, lab, vocab_start, logits=None):
@@ -236,9 +299,13 @@ class _FusedLinearCE(torch.autograd.Function):
         if h2.stride(1) != 1 or h2.stride(0) % 8:
             h2 = h2.contiguous()
         if _head_kernel_ok(h2, weight):
-            # not a saved tensor: hooks that move those to the host would move far more than the product costs
-            ctx.logits = _logits_to_keep(T, vl, H, h2.device) if graph else None
-            m, s, tgt = _head_stats(h2, weight, lab, r * vl, ctx.logits)
+            logits = None
+            if graph:
+                need = _backward_bytes(T, chunk, weight, *ctx.needs_input_grad[:2])
+                logits = _logits_to_keep(T, vl, H, h2.device, need)
+            if logits is not None:
+                ctx.kept = _Kept(logits)
+            m, s, tgt = _head_stats(h2, weight, lab, r * vl, logits)
             lse_all, tgt = _combine(m, s, tgt, group_name, group)
             ctx.save_for_backward(h2, weight, lab, lse_all)
             ctx.meta = (group_name, chunk, r * vl, h.shape, labels.shape)
@@ -271,7 +338,8 @@ class _FusedLinearCE(torch.autograd.Function):
         need_dw = ctx.needs_input_grad[1]
         ddt = h2.dtype if h2.dtype == torch.bfloat16 else torch.float32
         fused = _head_kernel_ok(h2, weight)
-        kept, ctx.logits = getattr(ctx, 'logits', None), None   # a second pass over the graph forms them again
+        kept = getattr(ctx, 'kept', None)
+        kept = None if kept is None else kept.take()            # a second pass over the graph forms them again
         # without `main_grad` the chunks' products are summed in fp32 and rounded once; a single chunk needs no such
         # buffer (at 151936 x 4096 it costs 2.5 GB of zero fill, accumulation and conversion), its GEMM rounds itself
         one_chunk = 0 < T <= chunk and mg is None and weight.dtype in (torch.bfloat16, torch.float32)
@@ -307,6 +375,8 @@ class _FusedLinearCE(torch.autograd.Function):
 def fused_linear_cross_entropy(h: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor, group: str = 'tp',
                                chunk: int = 4096) -> torch.Tensor:
     """``h [T, H]`` (full sequence on every TP rank), ``weight [V/tp, H]``, ``labels [T]`` -> loss ``[T]`` fp32."""
-    # asked here: inside the function grad mode is off, and ``needs_input_grad`` does not depend on it
-    graph = torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad)
+    # asked here: inside the function grad mode is off, and ``needs_input_grad`` does not depend on it.  Hooks on saved tensors
+    # (checkpointing, offload) spare device memory: logits beside them would undo that.
+    graph = (torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad)
+             and torch._C._autograd._top_saved_tensors_default_hooks(True) is None)
     return _FusedLinearCE.apply(h, weight, labels, group, chunk, graph)
