@@ -1,5 +1,5 @@
 // The host side of the calls a training step makes most: allocation of the results, checks, launch.  A CPython module
-// (mcore_bridge_b200/lib/_mcb200_host.so) that takes and returns tensors; the kernels are reached through the C entry points of
+// (mcore_bridge_b200/lib/_mcb200_host.*.so) that takes and returns tensors; the kernels are reached through the C entry points of
 // libmcb200.so.  The autograd functions themselves stay in Python (ops/*.py), this is what their bodies did one Python
 // call at a time: a GEMM of a small model spent about 24 us in arguments, views and ctypes for 7 us on the device.
 //

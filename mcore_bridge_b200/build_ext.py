@@ -1,8 +1,9 @@
-"""Builds the CUDA sources under ``csrc/`` into one in-tree shared library for sm_100a.
+"""Builds the sources under ``csrc/``, in-tree: one shared library of CUDA kernels for sm_100a and one CPython module.
 
-The kernels expose a plain C ABI and are loaded through ``ctypes`` (see ``ops/_lib.py``), so the
-build is a handful of ``nvcc`` invocations with no dependency on the torch headers: a full
-rebuild takes seconds and works on a machine without a GPU (nvcc cross-compiles).
+The kernels expose a plain C ABI and are loaded through ``ctypes`` (see ``ops/_lib.py``): a handful of ``nvcc`` invocations
+with no dependency on the torch headers, which work on a machine without a GPU (nvcc cross-compiles).  The module
+(``csrc/host``, the host side of the most frequent calls) is compiled against one Python and one torch, which its file
+name carries: after an upgrade of either it is missing rather than stale.
 
 Run as ``python -m mcore_bridge_b200.build_ext`` or call :func:`build`.
 """
@@ -21,7 +22,6 @@ REPO_DIR = PKG_DIR.parent
 CSRC = REPO_DIR / 'csrc'
 LIB_DIR = PKG_DIR / 'lib'
 LIB_NAME = 'libmcb200.so'
-HOST_NAME = '_mcb200_host.so'     # CPython module: the host side of the most frequent calls
 OBJ_DIR = REPO_DIR / 'build' / 'obj'
 
 NVCC_FLAGS = [
@@ -78,6 +78,15 @@ def _compile_one(src: Path, verbose: bool) -> Path:
     return obj
 
 
+def host_name() -> str:
+    """File name of the CPython module for the running Python and torch."""
+    import re
+    import sysconfig
+
+    import torch
+    return f'_mcb200_host.torch-{re.sub("[^0-9A-Za-z.]", "_", torch.__version__)}.{sysconfig.get_config_var("SOABI")}.so'
+
+
 def _host_command(out: Path) -> list[str]:
     import sysconfig
 
@@ -91,10 +100,10 @@ def _host_command(out: Path) -> list[str]:
 
 
 def build_host(verbose: bool = True, force: bool = False) -> Path:
-    """Compile the CPython module ``lib/_mcb200_host.so`` against this interpreter and its torch. Returns its path."""
-    import torch
-    out, stamp = LIB_DIR / HOST_NAME, OBJ_DIR / 'host.sha1'
-    h = hashlib.sha1(f'{torch.__version__} {sys.version}'.encode())
+    """Compile the CPython module ``lib/_mcb200_host.*.so`` against this interpreter and its torch. Returns its path."""
+    out = LIB_DIR / host_name()
+    stamp = OBJ_DIR / f'{out.name}.sha1'
+    h = hashlib.sha1()
     for src in sorted((CSRC / 'host').glob('*.cpp')):
         h.update(src.read_bytes())
     if out.exists() and stamp.exists() and stamp.read_text() == h.hexdigest() and not force:

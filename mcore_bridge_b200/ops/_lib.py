@@ -15,8 +15,10 @@ from pathlib import Path
 
 import torch
 
+from ..build_ext import CSRC, build_host, host_name
+
 _LIB_PATH = Path(__file__).resolve().parent.parent / 'lib' / 'libmcb200.so'
-_HOST_PATH = _LIB_PATH.with_name('_mcb200_host.so')
+_HOST_PATH = _LIB_PATH.with_name(host_name())
 _lib = None
 _native = None
 _lock = threading.RLock()
@@ -79,11 +81,11 @@ def native():
         path = str(lib()._name)
         with _lock:
             if _native is None:
-                if not _HOST_PATH.exists() and torch.cuda.is_available():
-                    from ..build_ext import build_host
+                if not _HOST_PATH.exists() and torch.cuda.is_available() and (CSRC / 'host').is_dir():
                     build_host(verbose=False)
                 if not _HOST_PATH.exists():
-                    raise KernelError(f'{_HOST_PATH} is missing: run `python -m mcore_bridge_b200.build_ext`')
+                    raise KernelError(f'{_HOST_PATH}, the host module for this Python and torch, is missing: run '
+                                      '`python -m mcore_bridge_b200.build_ext`')
                 loader = importlib.machinery.ExtensionFileLoader('_mcb200_host', str(_HOST_PATH))
                 m = importlib.util.module_from_spec(importlib.util.spec_from_loader('_mcb200_host', loader))
                 loader.exec_module(m)
@@ -100,7 +102,7 @@ def native_if_enabled():
 def available() -> bool:
     if not cuda_enabled():
         return False
-    native()  # raises loudly on a GPU box without the library
+    lib()  # raises loudly on a GPU box without the library
     return True
 
 

@@ -31,3 +31,25 @@ def test_kernels_are_switched_off_by_the_environment(monkeypatch):
     assert not nat.enabled()
     monkeypatch.setenv('MCB200_DISABLE_CUDA_KERNELS', '0')
     assert nat.enabled()
+
+
+def test_a_module_for_another_torch_is_not_loaded(monkeypatch, tmp_path):
+    from mcore_bridge_b200 import build_ext
+    mine = build_ext.host_name()
+    assert _lib._HOST_PATH.name == mine
+    monkeypatch.setattr(torch, '__version__', '99.0+other')
+    assert build_ext.host_name() != mine
+    monkeypatch.setattr(_lib, '_native', None)
+    monkeypatch.setattr(_lib, '_HOST_PATH', tmp_path / build_ext.host_name())
+    monkeypatch.setattr(torch.cuda, 'is_available', lambda: False)
+    with pytest.raises(_lib.KernelError, match='build_ext'):
+        _lib.native()
+
+
+def test_kernels_of_the_library_alone_do_without_the_module(monkeypatch):
+    def missing():
+        raise _lib.KernelError('no module')
+
+    monkeypatch.setattr(_lib, 'cuda_enabled', lambda: True)
+    monkeypatch.setattr(_lib, 'native', missing)
+    assert _lib.available()
