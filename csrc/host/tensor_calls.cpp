@@ -3,7 +3,9 @@
 // libmcb200.so.  The autograd functions themselves stay in Python (ops/*.py), this is what their bodies did one Python
 // call at a time: a GEMM of a small model spent about 24 us in arguments, views and ctypes for 7 us on the device.
 //
-// Everything runs with the interpreter's lock held, on the calling thread's current device and stream.
+// Everything runs on the calling thread's current device and stream, with the interpreter's lock held except during a launch.
+// A tensor's type, device and size are checked here against what the kernel reads; the first operand's device and the sizes a
+// kernel supports are the Python callers' and the C entry points' to check.
 #include <Python.h>
 #include <dlfcn.h>
 
@@ -160,11 +162,15 @@ PyObject* tuple(std::initializer_list<Tensor> ts) {
   return r;
 }
 
-// What a kernel reads one int32 of per query or key from: at least n of them, beside the operands.
+// An operand a kernel reads at least n elements of one type from, beside `like`; an undefined one is left out.
+void operand(const Tensor& t, at::ScalarType type, ll n, const Tensor& like, const char* what) {
+  require(!t.defined() || (t.scalar_type() == type && t.numel() >= n && t.device() == like.device()), what);
+}
+
+// What a kernel reads one int32 of per query or key from.
 Tensor per_token(const Tensor& t, ll n, const Tensor& like, const char* what) {
-  if (!t.defined()) return t;
-  require(t.scalar_type() == at::kInt && t.numel() >= n && t.device() == like.device(), what);
-  return t.contiguous();
+  operand(t, at::kInt, n, like, what);
+  return t.defined() ? t.contiguous() : t;
 }
 
 enum Layout { NT = 0, NN = 1, TN = 2 };
@@ -176,9 +182,15 @@ Tensor gemm(int layout, const Tensor& a_, const Tensor& b_, const Tensor& bias_,
   const bool a_mn = layout == TN, b_mn = layout != NT;
   const ll M = a.size(a_mn ? 1 : 0), K = a.size(a_mn ? 0 : 1), N = b.size(b_mn ? 1 : 0);
   require(b.size(b_mn ? 0 : 1) == K, "GEMM operands whose contraction sizes differ");
+  require(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && b.device() == a.device(),
+          "GEMM operands: bf16 on one device");
+  require(!out.defined() || ((out.scalar_type() == at::kFloat || out.scalar_type() == at::kBFloat16) && out.device() == a.device()),
+          "GEMM output: bf16 or fp32 on the operands' device");
+  require(!out.defined() || layout != TN || out.dim() == 2, "GEMM output of another shape");
+  require(!bias_.defined() || (bias_.numel() == N && bias_.device() == a.device()), "GEMM bias: one for every column");
   Tensor c;
   if (out.defined()) {
-    c = out.dim() == 2 ? out : out.view({M, N});
+    c = layout == TN || (out.dim() == 2 && out.size(0) == M && out.size(1) == N) ? out : out.view({M, N});
     require(c.size(0) == M && c.size(1) == N && c.stride(1) == 1, "GEMM output of another shape");
   } else {
     require(!accumulate, "accumulate needs an output tensor");
@@ -194,6 +206,8 @@ Tensor gemm(int layout, const Tensor& a_, const Tensor& b_, const Tensor& bias_,
 
 void norm_fwd(const Tensor& x2, const Tensor& w, float eps, bool zc, Tensor& y, Tensor& rstd) {
   const ll rows = x2.size(0), H = x2.size(1);
+  operand(x2, at::kBFloat16, 0, x2, "norm input: bf16");
+  operand(w, at::kBFloat16, H, x2, "norm weight: bf16, one for every column");
   y = at::empty({rows, H}, x2.options());
   rstd = at::empty({rows}, x2.options().dtype(at::kFloat));
   launch("mcb_rmsnorm_fwd", mcb_rmsnorm_fwd, x2.data_ptr(), nullptr, w.data_ptr(), y.data_ptr(), nullptr, rstd.data_ptr(),
@@ -204,6 +218,9 @@ void norm_fwd(const Tensor& x2, const Tensor& w, float eps, bool zc, Tensor& y, 
 void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor& rstd, float eps, bool zc, bool over,
               bool need_dw, Tensor& dx, Tensor& dw) {
   const ll rows = x2.size(0), H = x2.size(1);
+  operand(dy, at::kBFloat16, rows * H, x2, "norm gradient: bf16 of the input's size");
+  operand(w, at::kBFloat16, H, x2, "norm weight: bf16, one for every column");
+  operand(rstd, at::kFloat, rows, x2, "norm: an fp32 for every row");
   dx = at::empty({rows, H}, x2.options());
   Tensor part;
   if (need_dw) {
@@ -304,6 +321,7 @@ PyObject* glu_linear_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {    // h,
   const Tensor& h = tensor(a[0]);
   const Tensor h2 = rows_of(h, h.size(-1));
   const ll rows = h2.size(0), F = h2.size(1) / 2;
+  operand(h2, at::kBFloat16, 0, h2, "gated activation: bf16");
   const Tensor act = at::empty({rows, F}, h2.options());
   launch("mcb_glu_fwd", mcb_glu_fwd, h2.data_ptr(), nullptr, act.data_ptr(), rows, F, h2.stride(0), integer(a[2]),
          real(a[3]), real(a[4]), stream());
@@ -337,6 +355,8 @@ PyObject* glu_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {           // x,
   const Tensor& x = tensor(a[0]);
   const Tensor x2 = rows_of(x, x.size(-1)), probs = optional(a[1]);
   const ll rows = x2.size(0), F = x2.size(1) / 2;
+  operand(x2, at::kBFloat16, 0, x2, "gated activation: bf16");
+  operand(probs, at::kFloat, rows, x2, "gated activation: an fp32 factor for every row");
   const Tensor y = at::empty({rows, F}, x2.options());
   launch("mcb_glu_fwd", mcb_glu_fwd, x2.data_ptr(), ptr(probs), y.data_ptr(), rows, F, x2.stride(0), integer(a[2]), real(a[3]),
          real(a[4]), stream());
@@ -350,12 +370,25 @@ PyObject* glu_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {           // dy
   const Tensor probs = optional(a[2]);
   const ll rows = x2.size(0), F2 = x2.size(1);
   const Tensor dy = tensor(a[0]).reshape({rows, F2 / 2}).contiguous();
+  operand(dy, at::kBFloat16, 0, x2, "gated activation: bf16");
+  operand(probs, at::kFloat, rows, x2, "gated activation: an fp32 factor for every row");
   const Tensor dx = at::empty({rows, F2}, x2.options());
   const Tensor dp = probs.defined() ? at::empty({rows}, x2.options().dtype(at::kFloat)) : Tensor();
   launch("mcb_glu_bwd", mcb_glu_bwd, x2.data_ptr(), ptr(probs), dy.data_ptr(), dx.data_ptr(), ptr(dp), rows, F2 / 2,
          x2.stride(0), integer(a[3]), real(a[4]), real(a[5]), stream());
   return tuple({dx, dp});
   MCB_END
+}
+
+void check_qkv(const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin, ll ng, ll qpg, ll d,
+               bool gated) {
+  const ll T = qkv.size(0);
+  operand(qkv, at::kBFloat16, T * ng * (qpg * (gated ? 2 : 1) + 2) * d, qkv, "qkv: bf16, every head of every group");
+  require(wq.defined() == wk.defined() && cos.defined() == sin.defined(), "qkv: both weights and both tables, or neither");
+  operand(wq, at::kBFloat16, d, qkv, "query norm weight: bf16, one for every channel");
+  operand(wk, at::kBFloat16, d, qkv, "key norm weight: bf16, one for every channel");
+  operand(cos, at::kFloat, T * (cos.defined() ? cos.size(-1) : 0), qkv, "cosines: fp32, a row for every token");
+  operand(sin, at::kFloat, T * (cos.defined() ? cos.size(-1) : 0), qkv, "sines: fp32, a row for every token");
 }
 
 // qkv, wq, wk, cos, sin, ng, qpg, d, has_gate, interleaved, eps, zc -> q, k, v, gate, qkv
@@ -366,6 +399,7 @@ PyObject* qkv_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor wq = optional(a[1]), wk = optional(a[2]), cos = optional(a[3]), sin = optional(a[4]);
   const ll T = qkv.size(0), ng = integer(a[5]), qpg = integer(a[6]), d = integer(a[7]);
   const bool gated = truth(a[8]);
+  check_qkv(qkv, wq, wk, cos, sin, ng, qpg, d, gated);
   const Tensor q = at::empty({T, ng * qpg, d}, qkv.options()), k = at::empty({T, ng, d}, qkv.options()),
                v = at::empty({T, ng, d}, qkv.options());
   const Tensor gate = gated ? at::empty({T, ng * qpg, d}, qkv.options()) : Tensor();
@@ -383,6 +417,7 @@ PyObject* qkv_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor wq = optional(a[5]), wk = optional(a[6]), cos = optional(a[7]), sin = optional(a[8]);
   const ll T = qkv.size(0), ng = integer(a[9]), qpg = integer(a[10]), d = integer(a[11]);
   const bool gated = truth(a[12]), norm = wq.defined();
+  check_qkv(qkv, wq, wk, cos, sin, ng, qpg, d, gated);
   auto grad = [&](PyObject* o, ll heads) {
     return o == Py_None ? at::zeros({T, heads, d}, qkv.options()) : tensor(o).contiguous();
   };
@@ -411,10 +446,13 @@ PyObject* attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   MCB_BEGIN(7)
   const Tensor q = tensor(a[0]).contiguous(), k = tensor(a[1]).contiguous(), v = tensor(a[2]).contiguous();
   const ll T = q.size(0), nq = q.size(1), d = q.size(2);
+  operand(q, at::kBFloat16, 0, q, "queries: bf16");
+  operand(k, at::kBFloat16, k.size(0) * k.size(1) * d, q, "keys: bf16 with the queries' channels");
+  operand(v, at::kBFloat16, k.numel(), q, "values: bf16, as many as keys");
   const Tensor k_lo = per_token(tensor(a[3]), T, q, "first keys: an int32 for every query, on the queries' device"),
                k_hi = per_token(optional(a[4]), T, q, "last keys: an int32 for every query, on the queries' device"),
                sinks = optional(a[5]);
-  require(!sinks.defined() || (sinks.numel() >= nq && sinks.device() == q.device()), "sinks: one for every head");
+  operand(sinks, at::kFloat, nq, q, "sinks: an fp32 for every head");
   const Tensor o = at::empty_like(q), lse = at::empty({nq, T}, q.options().dtype(at::kFloat));
   launch("mcb_attn_fwd_ranges", mcb_attn_fwd_ranges, q.data_ptr(), k.data_ptr(), v.data_ptr(), k_lo.data_ptr(), ptr(k_hi),
          ptr(sinks), o.data_ptr(), lse.data_ptr(), T, k.size(0), nq, k.size(1), d, real(a[6]), status_of(q), stream());
