@@ -94,7 +94,7 @@ def _deliver(y, x, out, accumulate):
     if out is None:
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
     if accumulate:
-        out.add_(y.view(out.shape).to(out.dtype))
+        out.add_(y.view(out.shape))
     else:
         out.copy_(y.view(out.shape))
     return out
@@ -142,9 +142,9 @@ def mm_tn(dy: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None,
     if nat is not None:
         return nat.mm(2, dy, x, None, out, out_dtype == torch.float32, accumulate, alpha, max_sms, force_bn)
     y = _lib_mm(dy.reshape(-1, dy.shape[-1]).t(), x.reshape(-1, x.shape[-1])) * alpha
-    if out is not None:
-        return _deliver(y, dy, out, accumulate)
-    return y.to(out_dtype or dy.dtype)
+    if out is None:
+        return y.to(out_dtype or dy.dtype)
+    return out.add_(y.to(out.dtype)) if accumulate else out.copy_(y.to(out.dtype))
 
 
 # ------------------------------------------------------------------ grouped (MoE experts)
