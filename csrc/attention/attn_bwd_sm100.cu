@@ -905,19 +905,4 @@ int mcb_attn_bwd_ranges(const void* q, const void* k, const void* v, const void*
   return -3;
 }
 
-// Packed causal self-attention: seq_start [T] int32 = first token of each token's sequence.
-int mcb_attn_bwd_split(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
-                       float* delta, const int* seq_start, void* dq, void* dk, void* dv, int T, int nq, int nkv, int d,
-                       float scale, float* partial, int splits, int* status, void* stream_) {
-  return mcb_attn_bwd_ranges(q, k, v, o, dout, lse, delta, 0, seq_start, nullptr, nullptr, nullptr, dq, dk, dv, T, T, nq,
-                             nkv, d, scale, partial, splits, status, stream_);
-}
-
-int mcb_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
-                 float* delta, const int* seq_start, void* dq, void* dk, void* dv, int T, int nq, int nkv, int d,
-                 float scale, int* status, void* stream_) {
-  return mcb_attn_bwd_split(q, k, v, o, dout, lse, delta, seq_start, dq, dk, dv, T, nq, nkv, d, scale, nullptr, 1,
-                            status, stream_);
-}
-
 }  // extern "C"

@@ -520,10 +520,4 @@ int mcb_attn_fwd_ranges(const void* q, const void* k, const void* v, const int* 
   return -3;
 }
 
-// Packed causal self-attention: seq_start [T] int32 = first token of each token's sequence.
-int mcb_attn_fwd(const void* q, const void* k, const void* v, const int* seq_start, void* o, float* lse, int T, int nq,
-                 int nkv, int d, float scale, int* status, void* stream_) {
-  return mcb_attn_fwd_ranges(q, k, v, seq_start, nullptr, nullptr, o, lse, T, T, nq, nkv, d, scale, status, stream_);
-}
-
 }  // extern "C"

@@ -238,12 +238,17 @@ void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor&
 // How many CTAs share one (key tile, kv head) pair in the dK/dV kernel: enough to put at least about three CTAs on every SM,
 // limited to divisors of the GQA ratio.  MCB200_ATTN_DKV_SPLITS overrides it.
 int dkv_splits(ll T, int nq, int nkv) {
+  require(nkv > 0, "attention without key heads");
   const int qpg = nq / nkv;
-  if (const char* env = std::getenv("MCB200_ATTN_DKV_SPLITS")) {
-    if (*env) {
-      const int s = std::atoi(env);
-      return s >= 1 && qpg % s == 0 ? s : 1;
+  const char* env = std::getenv("MCB200_ATTN_DKV_SPLITS");
+  if (env && *env) {
+    char* end;
+    const long s = std::strtol(env, &end, 10);
+    if (*end) {
+      PyErr_Format(PyExc_ValueError, "MCB200_ATTN_DKV_SPLITS is not a number: %s", env);
+      throw Failed();
     }
+    return s >= 1 && qpg % s == 0 ? static_cast<int>(s) : 1;
   }
   const ll ctas = (T + 127) / 128 * nkv;
   int s = 1;
@@ -502,6 +507,12 @@ PyObject* attn_window_starts(PyObject*, PyObject* const* a, Py_ssize_t n) {   //
   MCB_END
 }
 
+PyObject* attn_dkv_splits(PyObject*, PyObject* const* a, Py_ssize_t n) {      // keys, query heads, kv heads
+  MCB_BEGIN(3)
+  return PyLong_FromLong(dkv_splits(integer(a[0]), static_cast<int>(integer(a[1])), static_cast<int>(integer(a[2]))));
+  MCB_END
+}
+
 PyObject* enabled(PyObject*, PyObject*) {
   const char* e = std::getenv("MCB200_DISABLE_CUDA_KERNELS");
   return PyBool_FromLong(!(e && std::strcmp(e, "1") == 0));
@@ -565,6 +576,7 @@ PyMethodDef methods[] = {MCB_FAST(init),
                          MCB_FAST(attn_fwd),
                          MCB_FAST(attn_bwd),
                          MCB_FAST(attn_window_starts),
+                         MCB_FAST(attn_dkv_splits),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_mcb200_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

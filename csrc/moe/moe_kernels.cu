@@ -353,12 +353,11 @@ struct CombineArgs {
   const float* scalar_ptrs[MAX_WORLD]; // optional per-row scalar on the owner (e.g. d(prob))
 };
 
-// out[t] = sum_k y_owner[row(t,k)]; optionally scalar_out[t,k] = scalar_owner[row(t,k)]
-// 4 to 8 rows a token: all of them are found first, then one 16-byte piece of each is in flight per lane; blockIdx.y takes runs of
-// 32 pieces, which gives few tokens more warps.  Bound: the reads.  Same order of the sums as below.  us, the kernel below / this
-// one: 4096 tokens x 8 rows of 2048 61 / 41 (3.7 TB/s), 1024 x 8 53 / 16, 64 x 8 49 / 8, 1000 x 6 43 / 14, 8192 x 4 of 2880
-// 92 / 74; it has too little in flight with fewer rows: 8192 x 2 of 4096 68 / 74, 16384 x 1 of 5120 80 / 147.  Two pieces a lane
-// measured the same or slower (43, 16, 10, 14, 78).
+// The sums of moe_combine_kernel below, in the same order, for 4 to 8 rows a token: all of them are found first, then one 16-byte piece
+// of each is in flight per lane; blockIdx.y takes runs of 32 pieces, which gives few tokens more warps.  Bound: the reads.  us, the
+// kernel below / this one: 4096 tokens x 8 rows of 2048 61 / 41 (3.7 TB/s), 1024 x 8 53 / 16, 64 x 8 49 / 8, 1000 x 6 43 / 14, 8192 x 4
+// of 2880 92 / 74; it has too little in flight with fewer rows: 8192 x 2 of 4096 68 / 74, 16384 x 1 of 5120 80 / 147.  Two pieces a
+// lane measured the same or slower (43, 16, 10, 14, 78).
 __global__ void __launch_bounds__(256)
 moe_combine8_kernel(CombineArgs a, const int* __restrict__ idx, const int* __restrict__ sent_row,
                     __nv_bfloat16* __restrict__ out, float* __restrict__ scalar_out) {
@@ -406,6 +405,7 @@ moe_combine8_kernel(CombineArgs a, const int* __restrict__ idx, const int* __res
   }
 }
 
+// out[t] = sum_k y_owner[row(t,k)]; optionally scalar_out[t,k] = scalar_owner[row(t,k)]
 __global__ void moe_combine_kernel(CombineArgs a, const int* __restrict__ idx, const int* __restrict__ sent_row,
                                    __nv_bfloat16* __restrict__ out, float* __restrict__ scalar_out) {
   const int lane = threadIdx.x & 31;

@@ -8,7 +8,6 @@ from __future__ import annotations
 
 import ctypes
 import math
-import os
 from typing import Optional
 
 import torch
@@ -66,37 +65,21 @@ def _row_starts(seq_start: torch.Tensor, T: int, device, one_each: bool) -> torc
     return (seq_start.expand(T) if n == 1 else seq_start[:T]).contiguous()
 
 
-def _dkv_splits(T: int, nq: int, nkv: int, device) -> int:
-    """How many CTAs share one (key tile, kv head) pair in the dK/dV kernel: enough to put at least about three
-    CTAs on every SM, limited to divisors of the GQA ratio.  ``MCB200_ATTN_DKV_SPLITS`` overrides it."""
-    env = os.environ.get('MCB200_ATTN_DKV_SPLITS')
-    qpg = nq // nkv
-    if env:
-        s = int(env)
-        return s if s >= 1 and qpg % s == 0 else 1
-    ctas = ((T + 127) // 128) * nkv
-    sms = torch.cuda.get_device_properties(device).multi_processor_count
-    s = 1
-    while ctas * s < 3 * sms and s * 2 <= qpg and qpg % (s * 2) == 0:
-        s *= 2
-    return s
-
-
 class _AttnFn(torch.autograd.Function):
 
     @staticmethod
-    def forward(ctx, q, k, v, seq_start, cu_seqlens, max_seqlen, scale):
+    def forward(ctx, q, k, v, seq_start, scale):
         o, lse, q, k, v = _lib.native().attn_fwd(q, k, v, seq_start, None, None, scale)
-        ctx.save_for_backward(q, k, v, o, lse, seq_start, cu_seqlens)
-        ctx.scale, ctx.max_seqlen = scale, max_seqlen
+        ctx.save_for_backward(q, k, v, o, lse, seq_start)
+        ctx.scale = scale
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, o, lse, seq_start, _cu = ctx.saved_tensors
+        q, k, v, o, lse, seq_start = ctx.saved_tensors
         dq, dk, dv, _ = _lib.native().attn_bwd(do, q, k, v, o, lse, seq_start, None, None, None, None, False,
                                               ctx.scale)
-        return dq, dk, dv, None, None, None, None
+        return dq, dk, dv, None, None
 
 
 def attention(q, k, v, cu_seqlens, max_seqlen, scale, seq_start: Optional[torch.Tensor] = None, window=None,
@@ -108,12 +91,10 @@ def attention(q, k, v, cu_seqlens, max_seqlen, scale, seq_start: Optional[torch.
         scale = 1.0 / math.sqrt(d)
     if seq_start is None:
         seq_start = seq_start_from_cu(cu_seqlens, T, q.device)
-    if max_seqlen is None and cu_seqlens is not None:
-        max_seqlen = T
     left = None if window is None or window[0] is None or int(window[0]) < 0 else int(window[0])
     seq_start = _row_starts(seq_start, T, q.device, left is not None)
     if left is None and sinks is None:
-        return _AttnFn.apply(q, k, v, seq_start, cu_seqlens, max_seqlen, float(scale))
+        return _AttnFn.apply(q, k, v, seq_start, float(scale))
     k_lo = seq_start
     if left is not None:
         # still non-decreasing, so the kernels' causal fast paths (k_hi = the query itself) apply unchanged
@@ -176,7 +157,7 @@ def bwd_ranges_raw(q, k, v, o, do, lse, delta, k_lo, k_hi, q_lo, q_hi, scale: fl
     T, nq, d = q.shape
     Tk, nkv = k.shape[0], k.shape[1]
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    splits = _dkv_splits(Tk, nq, nkv, q.device)
+    splits = _lib.native().attn_dkv_splits(Tk, nq, nkv)
     partial = torch.empty((2, splits, Tk, nkv, d), dtype=torch.float32, device=q.device) if splits > 1 else None
     rc = _lib.lib().mcb_attn_bwd_ranges(
         _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(do), _lib.ptr(lse), _lib.ptr(delta), _int(1),

@@ -241,7 +241,7 @@ def test_attention_kernels(T, nq, nkv, d, segs):
     cu = torch.tensor([0] + list(torch.tensor(segs).cumsum(0)), dtype=torch.int32, device=DEV)
     assert AC.supported(q, k, v, True, None, None, None)
     from mcore_bridge_b200.ops import _lib
-    assert hasattr(_lib.lib(), 'mcb_attn_bwd')
+    assert hasattr(_lib.lib(), 'mcb_attn_bwd_ranges')
     q2, k2, v2 = (t.clone().requires_grad_() for t in (q, k, v))
     o = AC.attention(q2, k2, v2, cu, max(segs), None)
     g = torch.randn_like(o)

@@ -86,3 +86,16 @@ def test_kernels_of_the_library_alone_do_without_the_module(monkeypatch):
     monkeypatch.setattr(_lib, 'cuda_enabled', lambda: True)
     monkeypatch.setattr(_lib, 'native', missing)
     assert _lib.available()
+
+
+def test_split_of_the_key_gradient_kernel(monkeypatch):
+    nat = _lib.native()
+    for text, splits in [('1', 1), ('2', 2), ('4', 4), ('3', 1), ('0', 1), ('-2', 1)]:     # 4 query heads share a kv head
+        monkeypatch.setenv('MCB200_ATTN_DKV_SPLITS', text)
+        assert nat.attn_dkv_splits(1000, 8, 2) == splits
+    monkeypatch.setenv('MCB200_ATTN_DKV_SPLITS', 'many')
+    with pytest.raises(ValueError):
+        nat.attn_dkv_splits(1000, 8, 2)
+    monkeypatch.delenv('MCB200_ATTN_DKV_SPLITS')
+    with pytest.raises(AssertionError):
+        nat.attn_dkv_splits(1000, 8, 0)
