@@ -53,7 +53,7 @@ cudaError_t launch_pair_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const
   return launch_pair<true, false>(ta, tb, p, grid, s);
 }
 
-// CTA pairs (256 x 256 tiles; 8192 x 4096 x 4096 171 us against 183 of the 256-wide single-CTA tiles) pay off once there
+// CTA pairs (256 x 256 tiles; 8192 x 4096 x 4096 171 us against 181 of the 256-wide single-CTA tiles) pay off once there
 // are enough tiles to fill the 74 clusters a few times over; small or
 // skinny problems keep the single-CTA tiles, whose narrower variants quantise better.
 bool use_pair(int M, int N, int K, int mode, int sms) {
