@@ -29,8 +29,9 @@ class MLP(nn.Module):
         cfg = self.config
         h = self.linear_fc1(x)
         fc2 = self.linear_fc2
+        # the fused block does not call fc2 as a module: with hooks on it, which want its input or output, it is called
         if cfg.gated_linear_unit and type(fc2) is RowParallelLinear and fc2.bias is None and not fc2.spec.fp8 \
-                and getattr(cfg, 'lean_activations', True):
+                and getattr(cfg, 'lean_activations', True) and not (fc2._forward_hooks or fc2._forward_pre_hooks):
             from ..parallel import state as ps
             from ..ops import fused_mlp
             if ps.get_world_size(fc2.group) == 1 and fused_mlp.usable(h, fc2.weight) and (h.shape[-1] // 2) % 8 == 0:
