@@ -1,9 +1,9 @@
 """Builds the sources under ``csrc/``, in-tree: one shared library of CUDA kernels for sm_100a and one CPython module.
 
-The kernels expose a plain C ABI and are loaded through ``ctypes`` (see ``ops/_lib.py``): a handful of ``nvcc`` invocations
-with no dependency on the torch headers, which work on a machine without a GPU (nvcc cross-compiles).  The module
-(``csrc/host``, the host side of the most frequent calls) is compiled against one Python and one torch, which its file
-name carries: after an upgrade of either it is missing rather than stale.
+The kernels expose a plain C ABI and are loaded through ``ctypes`` (see ``ops/_lib.py``): a handful of ``nvcc``
+invocations with no dependency on the torch headers, which work on a machine without a GPU (nvcc cross-compiles).  The
+module (``csrc/host``, the host side of the most frequent calls) is compiled against one Python and one torch, which its
+file name carries: after an upgrade of either it is missing rather than stale.
 
 Run as ``python -m mcore_bridge_b200.build_ext`` or call :func:`build`.
 """
@@ -30,7 +30,8 @@ NVCC_FLAGS = [
 ]
 # sources whose fp32 results are computed with the full-precision math functions and divisions (denormals are flushed in
 # them as everywhere else)
-PRECISE_SOURCES = {'attention/attn_sink_grad.cu', 'linear_attention/gdn_inputs.cu', 'linear_attention/gated_delta_rule.cu'}
+PRECISE_SOURCES = {'attention/attn_sink_grad.cu', 'linear_attention/gdn_inputs.cu',
+                   'linear_attention/gated_delta_rule.cu'}
 
 
 def _flags(src: Path) -> list[str]:
@@ -84,7 +85,8 @@ def host_name() -> str:
     import sysconfig
 
     import torch
-    return f'_mcb200_host.torch-{re.sub("[^0-9A-Za-z.]", "_", torch.__version__)}.{sysconfig.get_config_var("SOABI")}.so'
+    version = re.sub('[^0-9A-Za-z.]', '_', torch.__version__)
+    return f'_mcb200_host.torch-{version}.{sysconfig.get_config_var("SOABI")}.so'
 
 
 def _host_command(out: Path) -> list[str]:
@@ -94,7 +96,8 @@ def _host_command(out: Path) -> list[str]:
     inc = Path(torch.__file__).resolve().parent / 'include'
     cuda = Path(_nvcc()).resolve().parent.parent / 'include'
     dirs = [inc, inc / 'torch' / 'csrc' / 'api' / 'include', Path(sysconfig.get_paths()['include']), cuda]
-    return ['g++', '-O2', '-std=c++17', '-fPIC', '-shared', f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}',
+    return ['g++', '-O2', '-std=c++17', '-fPIC', '-shared',
+            f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}',
             *(f'-I{d}' for d in dirs), *map(str, sorted((CSRC / 'host').glob('*.cpp'))), '-o', str(out),
             f'-L{inc.parent / "lib"}', '-ltorch_python', '-ltorch_cpu', '-lc10', '-lc10_cuda', '-ldl']
 

@@ -50,8 +50,8 @@ def seq_start_from_cu(cu_seqlens: Optional[torch.Tensor], T: int, device) -> tor
 
 
 def _row_starts(seq_start: torch.Tensor, T: int, device, one_each: bool) -> torch.Tensor:
-    """``seq_start`` as the kernels read it: ``T`` int32 on ``device``, one after the other.  A single value counts for every
-    token; more than ``T`` are refused with ``one_each``."""
+    """``seq_start`` as the kernels read it: ``T`` int32 on ``device``, one after the other.  A single value counts for
+    every token; more than ``T`` are refused with ``one_each``."""
     if seq_start.dtype == torch.int32 and seq_start.shape == (T,) and seq_start.device == device:
         return seq_start.contiguous()
     n = seq_start.numel()

@@ -155,7 +155,7 @@ class _Kept:
 _kept: 'weakref.WeakSet[_Kept]' = weakref.WeakSet()
 _kept_lock = threading.Lock()
 _device_bytes: dict = {}         # device -> its memory
-_driver_free: dict = {}          # device -> (bytes the allocator held, bytes the driver had left for it) when last asked
+_driver_free: dict = {}          # device -> (bytes the allocator held, bytes the driver had left), when last asked
 
 
 def _kept_on(device) -> list:
@@ -168,15 +168,15 @@ def _kept_on(device) -> list:
 
 
 def release_kept_logits(device) -> None:
-    """Gives back the logits that graphs still hold: their backward passes form them again, with the same bits.  A model calls
-    this before a forward pass, whose activations had that memory to themselves when no logits were kept."""
+    """Gives back the logits that graphs still hold: their backward passes form them again, with the same bits.  A model
+    calls this before a forward pass, whose activations had that memory to themselves when no logits were kept."""
     for holder, _ in _kept_on(device):
         holder.take()
 
 
 def _memory_left(device, need: int) -> int:
-    """Bytes this process can still allocate: unused ones of its allocator and what the driver has for it.  The driver takes
-    60 to 130 us; a small buffer makes do with its answer of the last time the allocator grew or shrank."""
+    """Bytes this process can still allocate: unused ones of its allocator and what the driver has for it.  The driver
+    takes 60 to 130 us; a small buffer makes do with its answer of the last time the allocator grew or shrank."""
     reserved, allocated = _lib.native().memory(device.index)
     seen = _driver_free.get(device.index)
     if need > _KEEP_ASK or seen is None or seen[0] != reserved:
@@ -193,9 +193,9 @@ def _logits_to_keep(T, vl, H, device, backward: int = 0):
     6.5 TB/s and 1.4 PFLOP/s the two are even near ``H`` = 860.  Forward + backward, us, recomputed and kept: 4096 x 151936
     at ``H`` 4096 14808 / 12990, 2048 7173 / 6743, 1024 4420 / 3941; 64 x 151936 at 4096 1347 / 1165.
 
-    Memory comes first: a buffer is kept where the device has four times as much to spare beyond the ``backward`` bytes the
-    head's own backward pass allocates, and where all that are kept stay within a 32nd of the device.  In a captured graph a
-    buffer would last as long as the graph, so none is kept there."""
+    Memory comes first: a buffer is kept where the device has four times as much to spare beyond the ``backward`` bytes
+    the head's own backward pass allocates, and where all that are kept stay within a 32nd of the device.  In a captured
+    graph a buffer would last as long as the graph, so none is kept there."""
     if T == 0 or vl % 8 or H < _KEEP_MIN_HIDDEN or torch.cuda.is_current_stream_capturing():
         return None
     need = 4 * T * vl
@@ -221,8 +221,8 @@ def _backward_bytes(T, chunk, weight, need_dh, need_dw) -> int:
 
 
 def _head_stats(h2, weight, lab, vocab_start, logits=None):
-    """(max, sum exp, label logit) of every row over the local vocabulary shard, from the GEMM epilogue; the logits go to
-    ``logits`` when that is given."""
+    """(max, sum exp, label logit) of every row over the local vocabulary shard, from the GEMM epilogue; the logits go
+    to ``logits`` when that is given."""
     T, H = h2.shape
     vl = weight.shape[0]
     tiles_n = (vl + 255) // 256
@@ -255,8 +255,8 @@ def _kept_dlogits(logits, lab, vocab_start, lse, g):
     """What :func:`_head_dlogits` forms, from logits that the forward pass kept: the same bits."""
     rows, vl = logits.shape
     d = torch.empty((rows, vl), dtype=torch.bfloat16, device=logits.device)
-    rc = _lib.lib().mcb_ce_dlogits_head(_lib.ptr(logits), _lib.ptr(lab), _lib.ptr(lse), _lib.ptr(g), _ll(rows), _int(vl),
-                                        _int(vocab_start), _lib.ptr(d), _lib.stream_ptr())
+    rc = _lib.lib().mcb_ce_dlogits_head(_lib.ptr(logits), _lib.ptr(lab), _lib.ptr(lse), _lib.ptr(g), _ll(rows),
+                                        _int(vl), _int(vocab_start), _lib.ptr(d), _lib.stream_ptr())
     _lib.check_rc(rc, 'mcb_ce_dlogits_head')
     return d
 
@@ -375,8 +375,8 @@ class _FusedLinearCE(torch.autograd.Function):
 def fused_linear_cross_entropy(h: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor, group: str = 'tp',
                                chunk: int = 4096) -> torch.Tensor:
     """``h [T, H]`` (full sequence on every TP rank), ``weight [V/tp, H]``, ``labels [T]`` -> loss ``[T]`` fp32."""
-    # asked here: inside the function grad mode is off, and ``needs_input_grad`` does not depend on it.  Hooks on saved tensors
-    # (checkpointing, offload) spare device memory: logits beside them would undo that.
+    # asked here: inside the function grad mode is off, and ``needs_input_grad`` does not depend on it.  Hooks on saved
+    # tensors (checkpointing, offload) spare device memory: logits beside them would undo that.
     graph = (torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad)
              and torch._C._autograd._top_saved_tensors_default_hooks(True) is None)
     return _FusedLinearCE.apply(h, weight, labels, group, chunk, graph)

@@ -1,7 +1,8 @@
 """``pip install .`` entry point: metadata lives in ``pyproject.toml``; this file only adds the step that compiles
-``csrc/`` for sm_100a into ``mcore_bridge_b200/lib/libmcb200.so``, and its host side into a CPython module for the Python and
-torch that run it, when ``nvcc`` is available (a CPU-only install skips it and the package runs on its PyTorch reference
-paths).  Built in an isolated environment the module fits that environment's torch: use ``--no-build-isolation``."""
+``csrc/`` for sm_100a into ``mcore_bridge_b200/lib/libmcb200.so``, and its host side into a CPython module for the Python
+and torch that run it, when ``nvcc`` is available (a CPU-only install skips it and the package runs on its PyTorch
+reference paths).  Built in an isolated environment the module fits that environment's torch: use
+``--no-build-isolation``."""
 import shutil
 import sys
 
