@@ -74,8 +74,8 @@ struct GdrParams {
 };
 
 __device__ __forceinline__ ChunkPos locate(const GdrParams& p, ChunkPos* slot) {
-  ChunkPos mine{-1, 0, 0, 0, 0};
-  if (threadIdx.x < 32) mine = find_chunk<C, false>(p.cu, p.n_seq, p.T, blockIdx.x, threadIdx.x);
+  ChunkPos mine{-1, 0, 0, 0};
+  if (threadIdx.x < 32) mine = find_chunk<C>(p.cu, p.n_seq, p.T, blockIdx.x, threadIdx.x);
   if (threadIdx.x == 0) *slot = mine;
   __syncthreads();
   return *slot;
@@ -265,13 +265,8 @@ __device__ __forceinline__ ScanPos scan_pos(const GdrParams& p, int* slot) {
   // order of the batch does.
   if (p.n_seq <= 32) {
     if (threadIdx.x < 32) {
-      const int i = threadIdx.x, len = i < p.n_seq ? seq_len(p, i) : -1;
-      int rank = 0;
-      for (int j = 0; j < p.n_seq; ++j) {
-        const int other = __shfl_sync(0xffffffffu, len, j);
-        rank += other > len || (other == len && j < i);
-      }
-      if (i < p.n_seq && rank == seq) *slot = i;
+      const int i = longest_first(p.cu, p.n_seq, p.T, seq, threadIdx.x);
+      if (threadIdx.x == 0) *slot = i;
     }
     __syncthreads();
     seq = *slot;

@@ -4,17 +4,28 @@
 //   S_t = a S_{t-1} + k_t v_t^T,   o_t = scale * S_t^T q_t          R_t = a R_{t+1} + scale * q_t do_t^T
 //   dq_t = scale * S_t do_t,   dk_t = R_t v_t,   dv_t = R_t^T k_t
 //
-// A chunk's outputs need the state at its first token (and, backward, R behind its last one) plus products inside the
-// chunk.  Three launches: `boundary` forms what each chunk adds to the state that leaves it, `scan` runs the decayed
-// prefix sum over a sequence's chunk boundaries element by element, `out` computes every chunk independently.  All of
-// them have chunks x heads CTAs, so a single long sequence fills the GPU; token-by-token evaluation has one CTA per
-// (sequence, head).  Measured, 4096 tokens in two sequences, 16 heads of 128: forward 0.09 ms, backward 0.17 ms; token by
-// token the two took 10.6 ms.  Batches of sequences of fewer than 16 tokens on average are evaluated token by token.  States
-// are fp32 in memory (64 KB per chunk boundary and head at d = 128; 128-token chunks keep that traffic at half of the
-// inputs') and enter the products as two bf16 terms, see warp_mma.cuh: against fp64 the bf16 results are off by 0.00166, their
-// own rounding, as token by token in fp32.
+// Chunks are the tiles of 128 tokens of the packed batch, wherever its sequences begin: a tile's outputs need the state of the
+// sequence that crosses its first edge (backward, R of the one that crosses its last), for the rows of that sequence, and
+// products of tokens of one sequence inside the tile.  So a batch has T / 128 tiles however many sequences it is made of.  Two
+// launches: `walk` forms the states at the edges, `result` computes every tile and result independently.  States are fp32
+// sums, kept as two bf16 terms (64 KB per edge and head at d = 128; 128-token tiles keep that traffic at half of the
+// inputs') and enter the products as these; weights and weighted scores are split the same way: against fp64 the bf16
+// results are off by 0.00166, their own rounding, as token by token in fp32.
 //
-// Packed sequences are described by cu_seqlens on the device; CTAs find their chunk from it, nothing waits for the host.
+// Measured, us, inputs not in the L2, heads of 128 (64): against kernels with warp-level MMAs on chunks of one sequence each (states
+// by one kernel for all chunks and a prefix sum) and token-by-token kernels below 16 tokens a sequence
+//                                          forward before    now         backward before   now
+//   4096 tokens, sequences of 2926 and 1170, 16 heads    87 (48)   52 (42)       183 (79)    83 (56)
+//   16384 in one, 32 heads                              544 (234) 241 (161)     1318 (495)  482 (273)
+//   8192 in sequences of 1024, 16 heads                 144 (62)   79 (46)       331 (130)  130 (85)
+//                        128                             83 (44)   62 (40)       148 (83)   105 (71)
+//                         16                            226 (101)  73 (44)       470 (194)  132 (83)
+//                          8                            457 (115)  71 (44)      1084 (270)  132 (83)
+//   8192 in one, 4 heads (the chain of `walk`)           64 (44)   62 (58)       114 (62)    73 (67)
+//
+// Packed sequences are described by cu_seqlens on the device; nothing waits for the host.
+#include <climits>
+
 #include "../common/host_utils.cuh"
 #include "warp_mma.cuh"
 
@@ -23,7 +34,6 @@ using namespace mcb;
 namespace {
 
 constexpr int C = 128;          // tokens of a chunk
-constexpr int THREADS = 256;    // 8 warps, 16 rows each
 constexpr float L2E = 1.4426950408889634f;
 
 struct GlaParams {
@@ -31,7 +41,7 @@ struct GlaParams {
   __nv_bfloat16 *o, *dq, *dk, *dv;
   const float* decay;                      // [H] log-decay per step
   const int* cu;                           // [n_seq + 1]
-  float *S, *R;                            // [T / C boundaries, H, D, D] fp32
+  __nv_bfloat16 *S, *R;                    // [T / C boundaries, H, 2 terms, D, D]
   int T, n_seq, H;
   float scale;
   int* status;
@@ -44,549 +54,736 @@ __device__ __forceinline__ float decay2(const GlaParams& p, int h) {
   return g2 == -INFINITY ? -1e30f : g2;
 }
 
-__device__ __forceinline__ ChunkPos broadcast_pos(const ChunkPos& mine, ChunkPos* slot) {
-  if (threadIdx.x == 0) *slot = mine;
-  __syncthreads();
-  return *slot;
+// ---------------------------------------------------------------------------------------------------- operand tiles
+// A tile of `rows` x D bf16 lies in shared memory as D / 64 boxes of [rows][64], 128-byte rows with their 16-byte chunks
+// swizzled by the row: what TMA writes and tcgen05 reads.
+__device__ __forceinline__ uint32_t box_addr(uint32_t box, int row, int chunk) {
+  return box + row * 128 + ((chunk ^ (row & 7)) << 4);
 }
-
-// What the chunk before a boundary adds to S (z = 0), what the chunk behind it adds to R (z = 1):
-//   sum_j a^(C-1-j) k_j v_j^T      scale * sum_i a^i q_i do_i^T          rows: warp w owns 16 of D
+__device__ __forceinline__ void sts16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// one whole 32-byte sector
+__device__ __forceinline__ void stg32(void* p, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+// Rows [len, C) of a C-row tile that holds a sequence's last tokens belong to the next sequence, and may be infinite there:
+// they meet weights of zero only as zeros.  Thread = row.
 template <int D>
-__global__ void __launch_bounds__(THREADS)
-gla_boundary_kernel(const GlaParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ ChunkPos slot;
-  const uint32_t sx = (smem_u32(smem_raw) + 127) & ~127u, sy = sx + C * D * 2;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y;
-  ChunkPos mine{-1, 0, 0, 0, 0};
-  if (warp == 0) mine = find_chunk<C, true>(p.cu, p.n_seq, p.T, blockIdx.x, lane);
-  const ChunkPos pos = broadcast_pos(mine, &slot);
-  if (pos.seq < 0) return;
-  const bool rev = blockIdx.z != 0;
-  const int t = pos.t0 + (pos.index + (rev ? 1 : 0)) * C, len = min(C, pos.t1 - t);
-  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
-  load_tile<D, C, THREADS>(sx, (rev ? p.q : p.k) + off, stride, len);
-  load_tile<D, C, THREADS>(sy, (rev ? p.dout : p.v) + off, stride, len);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  if (warp * 16 >= D) return;
-  const float g2 = decay2(p, h), f = rev ? p.scale : 1.f;
-  float acc[D / 8][4];
+__device__ __forceinline__ void zero_row(uint32_t tile, int row) {
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-#pragma unroll 1
-  for (int kk = 0; kk < C; kk += 16) {
-    uint32_t a[4], hi[4], lo[4];
-    load_a_t<D>(sx, warp * 16, kk, lane, a);
+  for (int b = 0; b < D / 64; ++b)
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {               // registers 2u, 2u+1: tokens j, j+1
-      const int j = kk + 8 * u + (lane & 3) * 2;
-      const float w0 = f * exp2f(g2 * (rev ? j : C - 1 - j)), w1 = f * exp2f(g2 * (rev ? j + 1 : C - 2 - j));
+    for (int c = 0; c < 8; ++c) sts16(box_addr(tile + b * C * 128, row, c), 0, 0, 0, 0);
+}
+// `rows` x D tile at row y and column x of a map whose boxes are [rows][64]
+template <int D, int ROWS>
+__device__ __forceinline__ void load_boxes(uint32_t leader, uint32_t tile, const CUtensorMap* map, int x, int y, uint32_t bar) {
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u + r]));
-        split2(x.x * w0, x.y * w1, hi[2 * u + r], lo[2 * u + r]);
-      }
-    }
-#pragma unroll
-    for (int n = 0; n < D; n += 16) {
-      uint32_t b[4];
-      load_b_nn<D>(sy, kk, n, lane, b);
-      mma16816(acc[n / 8], hi, b[0], b[1]);
-      mma16816(acc[n / 8 + 1], hi, b[2], b[3]);
-      mma16816(acc[n / 8], lo, b[0], b[1]);
-      mma16816(acc[n / 8 + 1], lo, b[2], b[3]);
-    }
-  }
-  float* dst = (rev ? p.R : p.S) + ((long long)blockIdx.x * p.H + h) * D * D;
-  const int row = warp * 16 + (lane >> 2), col = (lane & 3) * 2;
-#pragma unroll
-  for (int n = 0; n < D / 8; ++n) {
-    *reinterpret_cast<float2*>(dst + (long long)row * D + n * 8 + col) = make_float2(acc[n][0], acc[n][1]);
-    *reinterpret_cast<float2*>(dst + (long long)(row + 8) * D + n * 8 + col) = make_float2(acc[n][2], acc[n][3]);
-  }
+  for (int b = 0; b < D / 64; ++b) tma_load_2d_warp(leader, tile + b * ROWS * 128, map, x + b * 64, y, bar);
+}
+// the loads that signal `bar` have landed (or 0.2 s have passed): nothing may write into a CTA that is gone
+__device__ __forceinline__ void drain(uint32_t bar, uint32_t parity) {
+  const uint64_t t0 = globaltimer_ns();
+  while (!mbar_try_wait(bar, parity))
+    if (globaltimer_ns() - t0 > 200000000ull) break;
 }
 
-// Decayed prefix sums over the boundaries of a sequence, in place: S forward (z = 0), R backward (z = 1); 4 elements a
-// thread, the next boundaries' contributions are loaded ahead.
+// ---------------------------------------------------------------------------------------------------- states
+// States at the edges between tiles: S behind the tokens before an edge, R of those behind it, of the sequence that crosses it,
+//
+//   S' = a^C S + sum_j a^(C-1-j) k_j v_j^T        R' = a^C R + scale * sum_i a^i q_i do_i^T
+//
+// A walk follows a sequence through its tiles for one head, one of the two and 32 columns of v (do).  Only the sums over tiles
+// are a chain, and they are a multiply-add of 32 registers a thread; everything else runs ahead of it: warp 12 loads the
+// rows of k (q) and the columns of v (do) by TMA; warps 4..11 (thread = token and half of the columns) multiply these by
+// the decays and lay them down as two bf16 terms (columns 0..31 and 32..63 of one operand); warps 13 and 14 multiply k^T with
+// both on tcgen05, tile by tile in turn; warps 0..3 (thread = row of the state) add the two halves to their rows and write
+// them through shared memory and TMA as two bf16 terms, which is how they enter the results' products.  Heads of 64 use the
+// same 128-row product: rows 64..127 are whatever lies behind the tile and are not read.
+//
+// Bound: the chain weights - issue - product - weights of a buffer (2300 cycles, three buffers) and the 600 cycles a warp takes to
+// issue eight products, hence two of them: 64 tiles 50 -> 43 us against two buffers and one issuer.  Columns fetched and states
+// stored by the threads themselves, a row each, kept the load / store unit busy with 32 lines an instruction: 2100 cycles a tile.
+constexpr int WALK_COLS = 32;
+constexpr int WALK_THREADS = 480;
+constexpr int WALK_STAGES = 4;     // tiles loading or in use
+constexpr int WALK_BUFS = 3;       // weighted columns and accumulators
+
 template <int D>
-__global__ void __launch_bounds__(256)
-gla_scan_kernel(const GlaParams p) {
-  constexpr int PER = D * D / (256 * 4);        // blocks per (sequence, head)
-  __shared__ int first;
-  const int seq = blockIdx.x / PER, part = blockIdx.x % PER, h = blockIdx.y;
-  const int2 span = seq_span(p.cu, seq, p.T);
-  int nb = (span.y - span.x + C - 1) / C - 1;
-  if (nb <= 0) return;
-  if (threadIdx.x < 32) {                       // boundaries of the sequences before this one
-    int n = 0;
-    for (int s = threadIdx.x; s < seq; s += 32) {
-      const int2 other = seq_span(p.cu, s, p.T);
-      if (other.y > other.x) n += (other.y - other.x + C - 1) / C - 1;
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    if (threadIdx.x == 0) first = n;
-  }
-  __syncthreads();
-  nb = min(nb, p.T / C - first);                // overlapping sequences: no more boundaries than there is room for
-  if (nb <= 0) return;
-  const bool rev = blockIdx.z != 0;
-  const float full = exp2f(decay2(p, h) * C);   // between two boundaries lies a whole chunk
-  const long long step = (long long)p.H * D * D;
-  float* base = (rev ? p.R : p.S) + ((long long)first * p.H + h) * D * D + (part * 256 + threadIdx.x) * 4;
-  constexpr int AHEAD = 4;
-  float4 buf[AHEAD];
-#pragma unroll
-  for (int i = 0; i < AHEAD; ++i)
-    if (i < nb) buf[i] = *reinterpret_cast<const float4*>(base + (rev ? nb - 1 - i : i) * step);
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int i0 = 0; i0 < nb; i0 += AHEAD) {
-#pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      const int i = i0 + u;
-      if (i >= nb) break;
-      const float4 x = buf[u];
-      if (i + AHEAD < nb) buf[u] = *reinterpret_cast<const float4*>(base + (rev ? nb - 1 - i - AHEAD : i + AHEAD) * step);
-      acc.x = fmaf(acc.x, full, x.x);
-      acc.y = fmaf(acc.y, full, x.y);
-      acc.z = fmaf(acc.z, full, x.z);
-      acc.w = fmaf(acc.w, full, x.w);
-      *reinterpret_cast<float4*>(base + (rev ? nb - 1 - i : i) * step) = acc;
-    }
-  }
-}
+struct WalkSmem {
+  static constexpr int TILE = C * D * 2, W = C * 128, V = C * WALK_COLS * 2, OUT = 2 * 32 * WALK_COLS * 2;
+  static constexpr int OFF_W = WALK_STAGES * TILE;      // also what a 64-wide tile's 128-row product reads behind its last stage
+  static constexpr int OFF_V = OFF_W + WALK_BUFS * W;
+  static constexpr int OFF_OUT = OFF_V + WALK_STAGES * V;     // per warp: 32 rows of both terms
+  static constexpr int OFF_BAR = OFF_OUT + 4 * OUT;
+  static constexpr int TOTAL = OFF_BAR + 256 + 1024;
+};
 
-// fp32 [D, D] state -> two bf16 tiles
+struct WalkMaps {
+  CUtensorMap k, q, v, d, s, r;                 // boxes of 64 x C (k, q), WALK_COLS x C (v, do) and WALK_COLS x 32 (states)
+};
+
+// The sequences that cross an edge, by head, direction and columns, dealt out to the CTAs in turn; every warp goes through the
+// same list.  Up to one sequence a tile they are taken from the list of sequences (the longest first, if there are at most 32),
+// with more of them from the edges: the sequence that crosses one, at the first edge it crosses.
 template <int D>
-__device__ __forceinline__ void load_state(uint32_t hi, uint32_t lo, const float* __restrict__ src) {
-  constexpr int AHEAD = D * D / 8 / THREADS < 4 ? D * D / 8 / THREADS : 4;      // loads in flight: 4 x 32 bytes a thread
-#pragma unroll 1
-  for (int id0 = threadIdx.x; id0 < D * D / 8; id0 += AHEAD * THREADS) {
-    float4 x[AHEAD][2];
-#pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      const float4* at = reinterpret_cast<const float4*>(src) + 2 * (id0 + u * THREADS);
-      x[u][0] = at[0];
-      x[u][1] = at[1];
-    }
-#pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      const int r = (id0 + u * THREADS) / (D / 8), c = ((id0 + u * THREADS) % (D / 8)) * 8;
-      uint32_t a[4], b[4];
-      split2(x[u][0].x, x[u][0].y, a[0], b[0]);
-      split2(x[u][0].z, x[u][0].w, a[1], b[1]);
-      split2(x[u][1].x, x[u][1].y, a[2], b[2]);
-      split2(x[u][1].z, x[u][1].w, a[3], b[3]);
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_addr<D>(hi, r, c)), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]) : "memory");
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_addr<D>(lo, r, c)), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]) : "memory");
-    }
-  }
-}
-
-// acc (16 rows x D) = X[rows r0..] * M with M [D, D] in two terms, taken as M (NT = false) or M^T (true); then every row
-// is multiplied by w0 (rows of the lower half) / w1 (upper half)
-template <int D, bool NT>
-__device__ __forceinline__ void times_state(float (&acc)[D / 8][4], uint32_t x, uint32_t mhi, uint32_t mlo, int r0, int lane,
-                                            float w0, float w1) {
-#pragma unroll 1
-  for (int kk = 0; kk < D; kk += 16) {
-    uint32_t a[4];
-    load_a<D>(x, r0, kk, lane, a);
-#pragma unroll
-    for (int n = 0; n < D; n += 16) {
-      uint32_t b[4], c[4];
-      if (NT) {
-        load_b_nt<D>(mhi, n, kk, lane, b);
-        load_b_nt<D>(mlo, n, kk, lane, c);
+struct Walk {
+  const GlaParams& p;
+  const int lane, dirs, units;
+  int job, nb = 0, h = 0, col0 = 0;             // nb: edges this walk crosses
+  bool rev = false;
+  int2 span = {0, 0};
+  __device__ Walk(const GlaParams& p_, int both, int lane_)
+      : p(p_), lane(lane_), dirs(both ? 2 : 1), units(min(p_.n_seq, (p_.T - 1) / C)), job((int)blockIdx.x - (int)gridDim.x) {}
+  __device__ bool next() {
+    constexpr int SL = D / WALK_COLS;
+    const int jobs = units * dirs * p.H * SL;
+    for (job += gridDim.x; job < jobs; job += gridDim.x) {
+      int id = job;
+      col0 = (id % SL) * WALK_COLS;
+      id /= SL;
+      h = id % p.H;
+      id /= p.H;
+      rev = dirs == 2 && (id & 1);
+      id /= dirs;
+      if (units == p.n_seq) {
+        span = seq_span(p.cu, p.n_seq <= 32 ? longest_first(p.cu, p.n_seq, p.T, id, lane) : id, p.T);
+        nb = span.y > span.x ? (span.y - 1) / C - span.x / C : 0;
       } else {
-        load_b_nn<D>(mhi, kk, n, lane, b);
-        load_b_nn<D>(mlo, kk, n, lane, c);
+        const int e = (id + 1) * C, seq = bounds_below(p.cu, p.n_seq + 1, e, lane) - 1;
+        span = seq >= 0 && seq < p.n_seq ? seq_span(p.cu, seq, p.T) : make_int2(0, 0);
+        nb = span.y > e && span.x >= e - C ? (span.y - 1) / C - span.x / C : 0;
       }
-      mma16816(acc[n / 8], a, b[0], b[1]);
-      mma16816(acc[n / 8 + 1], a, b[2], b[3]);
-      mma16816(acc[n / 8], a, c[0], c[1]);
-      mma16816(acc[n / 8 + 1], a, c[2], c[3]);
+      if (nb > 0) return true;
     }
+    return false;
   }
-#pragma unroll
-  for (int n = 0; n < D / 8; ++n) {
-    acc[n][0] *= w0;
-    acc[n][1] *= w0;
-    acc[n][2] *= w1;
-    acc[n][3] *= w1;
-  }
-}
+  // first token of the i-th tile, and the edge the walk comes to behind it (edges counted from 0 at token C)
+  __device__ int tile(int i) const { return (rev ? (span.y - 1) / C - i : span.x / C + i) * C; }
+  __device__ int edge(int i) const { return rev ? (span.y - 1) / C - i - 1 : span.x / C + i; }
+};
 
-// acc += (f * a^|i - j| * (X_i . Y_j)) Z_j over the column blocks jb in [jb0, jb1): rows i = r0.. of X, visible pairs
-// j <= i (LOWER) or j >= i
-template <int D, bool LOWER>
-__device__ __forceinline__ void inside_chunk(float (&acc)[D / 8][4], uint32_t x, uint32_t y, uint32_t z, int r0, int jb0,
-                                             int jb1, int lane, float g2, float f) {
-  uint32_t xa[D / 16][4];
-#pragma unroll
-  for (int kk = 0; kk < D / 16; ++kk) load_a<D>(x, r0, kk * 16, lane, xa[kk]);
-  const int i = r0 + (lane >> 2);
+template <int D>
+__global__ void __launch_bounds__(WALK_THREADS, 1)
+gla_walk_kernel(const __grid_constant__ WalkMaps maps, const GlaParams p, const int both) {
+  using L = WalkSmem<D>;
+  constexpr int NS = WALK_STAGES, NW = WALK_BUFS;
+  extern __shared__ uint8_t smem_raw[];
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  const uint32_t k_full = smem_u32(bars), k_empty = smem_u32(bars + NS);
+  const uint32_t w_full = smem_u32(bars + 2 * NS), done = w_full + 8 * NW, t_empty = done + 8 * NW;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NS + 3 * NW);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(k_full + 8 * i, 1);
+      mbar_init(k_empty + 8 * i, 1);
+    }
+    for (int i = 0; i < NW; ++i) {
+      mbar_init(w_full + 8 * i, 8);             // the warps that write it
+      mbar_init(done + 8 * i, 1);               // the products of a tile: weights and accumulator are released by it
+      mbar_init(t_empty + 8 * i, 4);
+    }
+    fence_barrier_init();
+    fence_proxy_async_smem();
+  }
+  if (warp == 13) {
+    tmem_alloc(smem_u32(tmem_slot), 256);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = warp_uniform(*tmem_slot);
+  const uint32_t tiles = smem_u32(smem), ws = tiles + L::OFF_W;
+  uint32_t it = 0;                              // tiles so far: stages and phases
+  bool ok = true;
+
+  if (warp == 12) {
+    const uint32_t leader = elect_one();
+    for (Walk<D> w(p, both, lane); ok && w.next(); )
 #pragma unroll 1
-  for (int jb = jb0; jb < jb1; ++jb) {
-    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      for (int i = 0; i < w.nb; ++i, ++it) {
+        const uint32_t s = it % NS;
+        ok = mbar_wait_warp(k_empty + 8 * s, ((it / NS) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY);
+        if (!ok) break;
+        mbar_expect_tx_warp(leader, k_full + 8 * s, L::TILE + L::V);
+        load_boxes<D, C>(leader, tiles + s * L::TILE, w.rev ? &maps.q : &maps.k, w.h * D, w.tile(i), k_full + 8 * s);
+        tma_load_2d_warp(leader, tiles + L::OFF_V + s * L::V, w.rev ? &maps.d : &maps.v, w.h * D + w.col0, w.tile(i), k_full + 8 * s);
+      }
+    for (uint32_t i = it > NS ? it - NS : 0; i < it; ++i) drain(k_full + 8 * (i % NS), (i / NS) & 1);
+    __syncwarp();
+  } else if (warp >= 13) {
+    const uint32_t leader = elect_one();
+    constexpr uint32_t idesc = make_idesc_bf16(128, 2 * WALK_COLS, true, true);
+    for (Walk<D> w(p, both, lane); ok && w.next(); )
+#pragma unroll 1
+      for (int i = 0; i < w.nb; ++i, ++it) {
+        if (it % 2 != warp - 13u) continue;
+        const uint32_t s = it % NW, ks = it % NS, ph = (it / NW) & 1;
+        ok = mbar_wait_warp(k_full + 8 * ks, (it / NS) & 1, abort_flag, p.status, ST_TIMEOUT_FULL) &&
+             mbar_wait_warp(w_full + 8 * s, ph, abort_flag, p.status, ST_TIMEOUT_FULL) &&
+             mbar_wait_warp(t_empty + 8 * s, ph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY);
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) {
-      uint32_t b[4];
-      load_b_nt<D>(y, jb * 16, kk * 16, lane, b);
-      mma16816(s[0], xa[kk], b[0], b[1]);
-      mma16816(s[1], xa[kk], b[2], b[3]);
-    }
+        for (int kk = 0; kk < C / 16; ++kk)
+          umma_f16_warp(leader, tmem + s * 64, make_smem_desc_sw128(tiles + ks * L::TILE + kk * 2048, C * 128, 1024),
+                        make_smem_desc_sw128(ws + s * L::W + kk * 2048, C * 128, 1024), idesc, kk ? 1u : 0u);
+        umma_commit_warp(leader, k_empty + 8 * ks);
+        umma_commit_warp(leader, done + 8 * s);
+      }
+  } else if (warp >= 4) {
+    const int j = threadIdx.x & 127, half = (threadIdx.x >> 7) - 1;
+    for (Walk<D> w(p, both, lane); ok && w.next(); ) {
+      const float wgt = (w.rev ? p.scale : 1.f) * exp2f(decay2(p, w.h) * (w.rev ? j : C - 1 - j));
+#pragma unroll 1
+      for (int i = 0; i < w.nb; ++i, ++it) {
+        const uint32_t s = it % NW, ks = it % NS;
+        ok = mbar_wait_warp(k_full + 8 * ks, (it / NS) & 1, abort_flag, p.status, ST_TIMEOUT_FULL) &&
+             mbar_wait_warp(done + 8 * s, ((it / NW) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY);
+        if (!ok) break;
+        const int t = w.tile(i) + j;
+        const bool in = t >= w.span.x && t < w.span.y;    // the other tokens of the first and the last tile
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
+        for (int u = 0; u < 2; ++u) {
+          const int c = 2 * half + u;
+          uint32_t x[4], hi[4], lo[4];
+          // what TMA wrote: 64-byte rows, their 16-byte chunks swizzled by pairs of rows
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
+                       : "r"(tiles + L::OFF_V + ks * L::V + j * 64 + ((c ^ ((j >> 1) & 3)) << 4)) : "memory");
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int j = jb * 16 + n * 8 + (lane & 3) * 2 + (e & 1);
-        const int gap = LOWER ? i + (e >> 1) * 8 - j : j - i - (e >> 1) * 8;
-        s[n][e] = gap >= 0 ? s[n][e] * (f * exp2f(g2 * gap)) : 0.f;
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[e]));
+            split2(in ? f.x * wgt : 0.f, in ? f.y * wgt : 0.f, hi[e], lo[e]);
+          }
+          sts16(box_addr(ws + s * L::W, j, c), hi[0], hi[1], hi[2], hi[3]);
+          sts16(box_addr(ws + s * L::W, j, 4 + c), lo[0], lo[1], lo[2], lo[3]);
+        }
+        if (!in && half == 0) zero_row<D>(tiles + ks * L::TILE, j);   // it may be infinite, and meets weights of zero
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(w_full + 8 * s);
       }
     }
-    uint32_t hi[4], lo[4];
-    acc_to_a(s[0], s[1], hi, lo);
+  } else {
+    const uint32_t out = tiles + L::OFF_OUT + warp * L::OUT;
+    for (Walk<D> w(p, both, lane); ok && w.next(); ) {
+      const CUtensorMap* map = w.rev ? &maps.r : &maps.s;
+      const float full = exp2f(decay2(p, w.h) * C);       // between two edges lies a whole tile
+      float st[WALK_COLS];
 #pragma unroll
-    for (int n = 0; n < D; n += 16) {
-      uint32_t b[4];
-      load_b_nn<D>(z, jb * 16, n, lane, b);
-      mma16816(acc[n / 8], hi, b[0], b[1]);
-      mma16816(acc[n / 8 + 1], hi, b[2], b[3]);
-      mma16816(acc[n / 8], lo, b[0], b[1]);
-      mma16816(acc[n / 8 + 1], lo, b[2], b[3]);
+      for (int e = 0; e < WALK_COLS; ++e) st[e] = 0.f;
+#pragma unroll 1
+      for (int i = 0; i < w.nb; ++i, ++it) {
+        const uint32_t s = it % NW;
+        ok = mbar_wait_warp(done + 8 * s, (it / NW) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r[64];
+        tmem_ld_32x32_x64(tmem + (uint32_t(warp * 32) << 16) + s * 64, r);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(t_empty + 8 * s);
+        if (warp * 32 >= D) continue;           // heads of 64
+#pragma unroll
+        for (int e = 0; e < WALK_COLS; ++e)
+          st[e] = fmaf(st[e], full, __uint_as_float(r[e]) + __uint_as_float(r[e + WALK_COLS]));
+        tma_store_wait_read<0>();               // (lane 0's) the tile before has left the staging area
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < WALK_COLS / 8; ++c) {
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) split2(st[8 * c + 2 * u], st[8 * c + 2 * u + 1], hi[u], lo[u]);
+          const uint32_t at = out + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4);
+          sts16(at, hi[0], hi[1], hi[2], hi[3]);
+          sts16(at + L::OUT / 2, lo[0], lo[1], lo[2], lo[3]);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          const int y = (w.edge(i) * p.H + w.h) * 2 * D + warp * 32;
+          tma_store_2d(map, out, w.col0, y);
+          tma_store_2d(map, out + L::OUT / 2, w.col0, y + D);
+          tma_store_commit();
+        }
+      }
     }
+    tma_store_wait<0>();
   }
-}
-
-template <int D>
-__device__ __forceinline__ void zero_acc(float (&acc)[D / 8][4]) {
-#pragma unroll
-  for (int n = 0; n < D / 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-}
-
-// rows r0.. of the result, those below `len`
-template <int D>
-__device__ __forceinline__ void store_rows(const float (&acc)[D / 8][4], __nv_bfloat16* dst, long long stride, int r0, int len,
-                                           int lane) {
-  const int row = r0 + (lane >> 2), col = (lane & 3) * 2;
-#pragma unroll
-  for (int n = 0; n < D / 8; ++n) {
-    if (row < len) *reinterpret_cast<uint32_t*>(dst + row * stride + n * 8 + col) = pack_bf16x2(acc[n][0], acc[n][1]);
-    if (row + 8 < len) *reinterpret_cast<uint32_t*>(dst + (row + 8) * stride + n * 8 + col) = pack_bf16x2(acc[n][2], acc[n][3]);
-  }
-}
-
-// Bound: shared-memory operand reads of the 128-row products (two per MMA term); one CTA per (chunk, head).
-template <int D>
-__global__ void __launch_bounds__(THREADS)
-gla_out_kernel(const GlaParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ ChunkPos slot;
-  constexpr int TILE = C * D * 2;
-  const uint32_t sq = (smem_u32(smem_raw) + 127) & ~127u, sk = sq + TILE, sv = sk + TILE, shi = sv + TILE, slo = shi + D * D * 2;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y;
-  ChunkPos mine{-1, 0, 0, 0, 0};
-  if (warp == 0) mine = find_chunk<C, false>(p.cu, p.n_seq, p.T, blockIdx.x, lane);
-  const ChunkPos pos = broadcast_pos(mine, &slot);
-  if (pos.seq < 0 || pos.boundary0 + pos.index > p.T / C) return;
-  const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
-  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
-  load_tile<D, C, THREADS>(sq, p.q + off, stride, len);
-  load_tile<D, C, THREADS>(sk, p.k + off, stride, len);
-  load_tile<D, C, THREADS>(sv, p.v + off, stride, len);
-  cp_async_commit();
-  if (h == 0) check_bounds(p.cu, p.n_seq, p.T, p.status);
-  if (pos.index > 0) load_state<D>(shi, slo, p.S + ((long long)(pos.boundary0 + pos.index - 1) * p.H + h) * D * D);
-  cp_async_wait<0>();
+  tc_fence_before();
   __syncthreads();
-  const int r0 = warp * 16;
-  if (r0 >= len) return;
-  const float g2 = decay2(p, h);
-  const int i = r0 + (lane >> 2);
-  float acc[D / 8][4];
-  zero_acc<D>(acc);
-  if (pos.index > 0)
-    times_state<D, false>(acc, sq, shi, slo, r0, lane, p.scale * exp2f(g2 * (i + 1)), p.scale * exp2f(g2 * (i + 9)));
-  inside_chunk<D, true>(acc, sq, sk, sv, r0, 0, warp + 1, lane, g2, p.scale);
-  store_rows<D>(acc, p.o + off, stride, r0, len, lane);
+  if (warp == 13) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 256);
+  }
 }
 
-template <int D>
-__global__ void __launch_bounds__(THREADS)
-gla_grad_kernel(const GlaParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ ChunkPos slot;
-  constexpr int TILE = C * D * 2;
-  const uint32_t sq = (smem_u32(smem_raw) + 127) & ~127u, sk = sq + TILE, sv = sk + TILE, sd = sv + TILE;
-  const uint32_t shi = sd + TILE, slo = shi + D * D * 2;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y;
-  ChunkPos mine{-1, 0, 0, 0, 0};
-  if (warp == 0) mine = find_chunk<C, false>(p.cu, p.n_seq, p.T, blockIdx.x, lane);
-  const ChunkPos pos = broadcast_pos(mine, &slot);
-  if (pos.seq < 0 || pos.boundary0 + pos.index > p.T / C) return;
-  const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
-  const bool first = pos.index == 0;
-  const bool last = t + len >= pos.t1 || pos.boundary0 + pos.index >= p.T / C;   // (the latter: overlapping sequences)
-  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
-  load_tile<D, C, THREADS>(sq, p.q + off, stride, len);
-  load_tile<D, C, THREADS>(sk, p.k + off, stride, len);
-  load_tile<D, C, THREADS>(sv, p.v + off, stride, len);
-  load_tile<D, C, THREADS>(sd, p.dout + off, stride, len);
-  cp_async_commit();
-  const long long bnd = ((long long)(pos.boundary0 + pos.index) * p.H + h) * D * D, prev = bnd - (long long)p.H * D * D;
-  if (!first) load_state<D>(shi, slo, p.S + prev);
-  cp_async_wait<0>();
-  __syncthreads();
-  const int r0 = warp * 16, i = r0 + (lane >> 2);
-  const int nblk = (len + 15) / 16;
-  const float g2 = decay2(p, h);
-  float acc[D / 8][4];
-  if (r0 < len) {
-    zero_acc<D>(acc);
-    if (!first)
-      times_state<D, true>(acc, sd, shi, slo, r0, lane, p.scale * exp2f(g2 * (i + 1)), p.scale * exp2f(g2 * (i + 9)));
-    inside_chunk<D, true>(acc, sd, sv, sk, r0, 0, warp + 1, lane, g2, p.scale);
-    store_rows<D>(acc, p.dq + off, stride, r0, len, lane);
-  }
-  if (!last) {
-    __syncthreads();
-    load_state<D>(shi, slo, p.R + bnd);
-    __syncthreads();
-  }
-  if (r0 >= len) return;
-  // a chunk that is not its sequence's last one is full: R decays by a^(C - j) to token j
-  const float w0 = exp2f(g2 * (C - i)), w1 = exp2f(g2 * (C - i - 8));
-  zero_acc<D>(acc);
-  if (!last) times_state<D, true>(acc, sv, shi, slo, r0, lane, w0, w1);
-  inside_chunk<D, false>(acc, sv, sd, sq, r0, warp, nblk, lane, g2, p.scale);
-  store_rows<D>(acc, p.dk + off, stride, r0, len, lane);
-  zero_acc<D>(acc);
-  if (!last) times_state<D, false>(acc, sk, shi, slo, r0, lane, w0, w1);
-  inside_chunk<D, false>(acc, sk, sq, sd, r0, warp, nblk, lane, g2, p.scale);
-  store_rows<D>(acc, p.dv + off, stride, r0, len, lane);
-}
-
-// One chunk of one result, from the state M at its edge (S before it or R behind it) and the pairs inside it:
-//   ROLE       out_i = w_i * (X_i . M) + scale * sum_j a^|i-j| (X_i . Y_j) Z_j
+// ---------------------------------------------------------------------------------------------------- results
+// One result of one tile, from the state M at its edge (S before it or R behind it) and the pairs inside it:
+//   role       out_i = w_i * (X_i . M) + scale * sum_j a^|i-j| (X_i . Y_j) Z_j
 //   O          o  = q S,   (q . k) v       pairs j <= i
 //   DQ         dq = do S^T, (do . v) k     pairs j <= i
 //   DK         dk = v R^T, (v . do) q      pairs j >= i
 //   DV         dv = k R,   (k . q) do      pairs j >= i
-// The state's two terms lie where Y and Z go afterwards, so that three tiles are all a CTA holds and two CTAs share an SM
-// (D = 128: 96 KB each against 160 and 192 above): one computes while the other waits for its tiles.  See `two_per_sm`.
+// Persistent CTAs, two an SM, take these one after the other.  All products run on tcgen05; the state enters as two bf16 terms,
+// the weighted scores X . Y_j return to TMEM as two bf16 terms, the first operand of the last product.  Shared memory holds
+// three tiles: X, then in turn Y and the state's lower term, the upper term and Z.  Warp 8 loads and multiplies:
+//
+//   X Y^T -> scores | X M_hi -> out (loads M_lo over Y, Z over M_hi) | out += X M_lo (loads the next X, Y) | out += P Z
+//
+// Warp 9 finds the next tile's sequences.  Warps 0..7 (thread = row and half of its columns) weight the scores meanwhile, multiply
+// the state's share by w_i before the last product, and write the result out while the next one's first products run.
+//
+// Bound: the waits of that chain, half of them for the state's terms, of which two CTAs overlap: about 12000 cycles a result of
+// 128 x 128 with a state and 5000 without.  One CTA per result (which loaded the state in fp32 and split it itself) took 86 us
+// instead of 46 for the gradients of 4096 tokens, 16 heads of 128.
 enum { O, DQ, DK, DV };
+constexpr int RES_THREADS = 320;
 
-template <int D, int ROLE>
-__device__ __forceinline__ void chunk_result(const GlaParams& p, uint32_t sx, const ChunkPos& pos, int h) {
-  constexpr int TILE = C * D * 2;
-  constexpr bool BACK = ROLE >= DK;
-  const uint32_t sy = sx + TILE, sz = sy + TILE;
-  const __nv_bfloat16* X = ROLE == O ? p.q : ROLE == DQ ? p.dout : ROLE == DK ? p.v : p.k;
-  const __nv_bfloat16* Y = ROLE == O ? p.k : ROLE == DQ ? p.v : ROLE == DK ? p.dout : p.q;
-  const __nv_bfloat16* Z = ROLE == O ? p.v : ROLE == DQ ? p.k : ROLE == DK ? p.q : p.dout;
-  __nv_bfloat16* out = ROLE == O ? p.o : ROLE == DQ ? p.dq : ROLE == DK ? p.dk : p.dv;
-  const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
-  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
-  const int bnd = pos.boundary0 + pos.index;
-  // last chunk of a sequence, or (overlapping sequences) no boundary behind it
-  const bool state = BACK ? t + len < pos.t1 && bnd < p.T / C : pos.index > 0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = warp * 16, i = r0 + (lane >> 2);
-  const float g2 = decay2(p, h);
-  float acc[D / 8][4];
-  zero_acc<D>(acc);
-  load_tile<D, C, THREADS>(sx, X + off, stride, len);
-  cp_async_commit();
-  if (state) {
-    load_state<D>(sy, sz, (BACK ? p.R : p.S) + ((long long)(BACK ? bnd : bnd - 1) * p.H + h) * D * D);
-    cp_async_wait<0>();
-    __syncthreads();
-    // a chunk that is not its sequence's last one is full: R decays by a^(C - i) to token i
-    const float w0 = BACK ? exp2f(g2 * (C - i)) : p.scale * exp2f(g2 * (i + 1));
-    const float w1 = BACK ? exp2f(g2 * (C - i - 8)) : p.scale * exp2f(g2 * (i + 9));
-    if (r0 < len) times_state<D, ROLE == DQ || ROLE == DK>(acc, sx, sy, sz, r0, lane, w0, w1);
-    __syncthreads();
-  }
-  load_tile<D, C, THREADS>(sy, Y + off, stride, len);
-  load_tile<D, C, THREADS>(sz, Z + off, stride, len);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  if (r0 >= len) return;
-  inside_chunk<D, !BACK>(acc, sx, sy, sz, r0, BACK ? warp : 0, BACK ? (len + 15) / 16 : warp + 1, lane, g2, p.scale);
-  store_rows<D>(acc, out + off, stride, r0, len, lane);
-}
-
-// z (gradients): dq, dk, dv
-template <int D, bool GRAD>
-__global__ void __launch_bounds__(THREADS, 2)
-gla_result_kernel(const GlaParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ ChunkPos slot;
+template <int D>
+struct ResultSmem {
+  static constexpr int TILE = C * D * 2;
+  static constexpr int Y = TILE, Z = 2 * TILE;
+  static constexpr int OFF_BAD = 3 * TILE;                  // per column: rows of Z that are not finite there
+  static constexpr int OFF_BAR = OFF_BAD + D * 16;
+  static constexpr int TOTAL = OFF_BAR + 256 + 1024;
   static_assert(D <= C, "a term of the state fits into a tile");
-  const uint32_t sx = (smem_u32(smem_raw) + 127) & ~127u;
-  const int h = blockIdx.y;
-  ChunkPos mine{-1, 0, 0, 0, 0};
-  if (threadIdx.x < 32) mine = find_chunk<C, false>(p.cu, p.n_seq, p.T, blockIdx.x, threadIdx.x);
-  const ChunkPos pos = broadcast_pos(mine, &slot);
-  if (pos.seq < 0 || pos.boundary0 + pos.index > p.T / C) return;
-  if (!GRAD) {
-    if (h == 0) check_bounds(p.cu, p.n_seq, p.T, p.status);
-    chunk_result<D, O>(p, sx, pos, h);
-  } else if (blockIdx.z == 0) {
-    chunk_result<D, DQ>(p, sx, pos, h);
-  } else if (blockIdx.z == 1) {
-    chunk_result<D, DK>(p, sx, pos, h);
+};
+
+struct GlaMaps {
+  CUtensorMap q, k, v, d, s, r;
+};
+
+// What the warps of a CTA need to know of one result of one tile.
+struct ResultItem {
+  int t, len, h, edge, role;                    // first token; tokens (0: no more items); head; the state's edge
+  int state, s0, s1;                            // whether one crosses, and the rows [s0, s1) it reaches
+  uint32_t starts[4];                           // bit r: a sequence starts (or the last one has ended) at row r
+};
+
+// by one warp
+__device__ __forceinline__ ResultItem find_item(const GlaParams& p, int id, int roles, int lane) {
+  ResultItem it{};
+  it.role = roles == 1 ? O : DQ + id % roles;
+  id /= roles;
+  it.h = id % p.H;
+  it.t = id / p.H * C;
+  it.len = min(C, p.T - it.t);
+  auto bound = [&](int i) { return min(max(p.cu[i], 0), p.T) - it.t; };
+  const int n = p.n_seq + 1;
+  bool edge_ends = it.t + C >= p.T;             // no sequence crosses the tile's last edge
+  for (int i0 = bounds_below(p.cu, n, it.t, lane); i0 < n; i0 += 32) {
+    const int r = i0 + lane < n ? bound(i0 + lane) : -1;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) it.starts[w] |= __reduce_or_sync(0xffffffffu, r >= 0 && r >> 5 == w ? 1u << (r & 31) : 0u);
+    edge_ends |= __any_sync(0xffffffffu, r == C);
+    if (__any_sync(0xffffffffu, r >= C)) break;
+  }
+  int first = C, last = 0;
+#pragma unroll
+  for (int w = 3; w >= 0; --w)
+    if (it.starts[w]) first = 32 * w + __ffs(it.starts[w]) - 1;
+#pragma unroll
+  for (int w = 0; w < 4; ++w)
+    if (it.starts[w]) last = 32 * w + 31 - __clz(it.starts[w]);
+  if (it.role >= DK) {
+    it.state = !edge_ends;
+    it.s0 = last;
+    it.s1 = C;
+    it.edge = it.t / C;
   } else {
-    chunk_result<D, DV>(p, sx, pos, h);
+    it.state = it.t > 0 && first > 0;
+    it.s0 = 0;
+    it.s1 = first;
+    it.edge = it.t / C - 1;
   }
+  return it;
 }
 
-// ---------------------------------------------------------------------------------------------------- short sequences
-// Token by token: one CTA of D threads per (sequence, head), thread j keeps column j of the state S [D x D] in registers.  q
-// and k of the current token are staged in shared memory (double buffered) so every thread reads them as broadcasts.
-template <int D>
-__global__ void __launch_bounds__(D)
-gla_token_fwd_kernel(const GlaParams p) {
-  __shared__ float qs[2][D], ks[2][D];
-  const int h = blockIdx.y, j = threadIdx.x;
-  if (h == 0) check_bounds(p.cu, p.n_seq, p.T, p.status);
-  const int2 span = seq_span(p.cu, blockIdx.x, p.T);
-  const float a = __expf(p.decay[h]);
-  const __nv_bfloat16 *__restrict__ q = p.q, *__restrict__ k = p.k, *__restrict__ v = p.v;
-  __nv_bfloat16* __restrict__ o = p.o;
-  float S[D];
-#pragma unroll
-  for (int i = 0; i < D; ++i) S[i] = 0.f;
-  auto stage = [&](int t, int b) {
-    const long long at = ((long long)t * p.H + h) * D + j;
-    qs[b][j] = __bfloat162float(q[at]) * p.scale;
-    ks[b][j] = __bfloat162float(k[at]);
-  };
-  if (span.x < span.y) stage(span.x, 0);
+template <int D, bool GRAD>
+__global__ void __launch_bounds__(RES_THREADS, 2)
+gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const int items) {
+  using L = ResultSmem<D>;
+  constexpr int ROLES = GRAD ? 3 : 1;
+  constexpr uint32_t COL_S = 0, COL_O = 128;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ ResultItem slots[2];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  // every barrier completes once per item: with the item's number comes its phase
+  const uint32_t xy_full = smem_u32(bars), hi_full = xy_full + 8, lo_full = xy_full + 16, z_full = xy_full + 24;
+  const uint32_t s_done = xy_full + 32, hi_done = xy_full + 40, m_done = xy_full + 48, o_done = xy_full + 56;
+  const uint32_t p_full = xy_full + 64, o_read = xy_full + 72;
+  const uint32_t item_full = xy_full + 80, item_read = xy_full + 96;         // two each, by item & 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* bad_item = abort_flag + 1;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    *bad_item = -1;
+    for (int i = 0; i < 8; ++i) mbar_init(xy_full + 8 * i, 1);
+    mbar_init(p_full, 8);
+    mbar_init(o_read, 8);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(item_full + 8 * i, 1);
+      mbar_init(item_read + 8 * i, 9);
+    }
+    fence_barrier_init();
+    fence_proxy_async_smem();
+  }
+  if (warp == 8) {
+    tmem_alloc(smem_u32(tmem_slot), 256);
+    tmem_relinquish();
+  }
+  uint32_t* bad = reinterpret_cast<uint32_t*>(smem + L::OFF_BAD);
+  for (int i = threadIdx.x; i < D * 4; i += RES_THREADS) bad[i] = 0;
+  if (!GRAD) check_bounds(p.cu, p.n_seq, p.T, p.status);
+  tc_fence_before();
   __syncthreads();
-  for (int t = span.x; t < span.y; ++t) {
-    const int b = (t - span.x) & 1;
-    if (t + 1 < span.y) stage(t + 1, b ^ 1);
-    const long long at = ((long long)t * p.H + h) * D + j;
-    const float vj = __bfloat162float(v[at]);
-    float acc = 0.f;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      S[i] = fmaf(S[i], a, ks[b][i] * vj);
-      acc = fmaf(S[i], qs[b][i], acc);
-    }
-    o[at] = __float2bfloat16(acc);
-    __syncthreads();
-  }
-}
+  tc_fence_after();
+  const uint32_t tmem = warp_uniform(*tmem_slot);
+  const uint32_t sx = smem_u32(smem), sy = sx + L::Y, sz = sx + L::Z;
 
-// Backward in three sweeps with no stored states.  Owning rows for dq / dk and columns for dv keeps every reduction inside a
-// thread:
-//   forward, thread = row i of S_t :              dq_t[i] = scale * sum_c S_t[i, c] do_t[c]
-//   reverse, thread = row i of R_t / scale :      dk_t[i] = scale * sum_c (R_t / scale)[i, c] v_t[c]
-//   reverse, thread = column c of R_t / scale :   dv_t[c] = scale * sum_i (R_t / scale)[i, c] k_t[i]
-// Every sweep is  M <- a M + x w^T,  out = scale M z  over one order of the tokens; w and z are shared, x is the thread's own.
-template <int D>
-__global__ void __launch_bounds__(D)
-gla_token_bwd_kernel(const GlaParams p) {
-  __shared__ float ws[D], zs[D];
-  const int h = blockIdx.y, i = threadIdx.x;
-  const int2 span = seq_span(p.cu, blockIdx.x, p.T);
-  const float a = __expf(p.decay[h]);
-  float M[D];
-  auto sweep = [&](bool reverse, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                   const __nv_bfloat16* __restrict__ z, __nv_bfloat16* __restrict__ out) {
+  if (warp == 8) {
+    const uint32_t leader = elect_one();
+    constexpr uint32_t idesc_s = make_idesc_bf16(C, C, false, false), idesc_z = make_idesc_bf16(C, D, false, true);
+    auto next = [&](int n) {
+      ResultItem it{};
+      if (mbar_wait_warp(item_full + 8 * (n & 1), (n >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) it = slots[n & 1];
+      __syncwarp();
+      if (leader) mbar_arrive(item_read + 8 * (n & 1));
+      return it;
+    };
+    auto load_xy = [&](const ResultItem& it) {
+      const CUtensorMap* mx = it.role == O ? &maps.q : it.role == DQ ? &maps.d : it.role == DK ? &maps.v : &maps.k;
+      const CUtensorMap* my = it.role == O ? &maps.k : it.role == DQ ? &maps.v : it.role == DK ? &maps.d : &maps.q;
+      mbar_expect_tx_warp(leader, xy_full, 2 * L::TILE);
+      load_boxes<D, C>(leader, sx, mx, it.h * D, it.t, xy_full);
+      load_boxes<D, C>(leader, sy, my, it.h * D, it.t, xy_full);
+    };
+    auto load_state = [&](const ResultItem& it, int term, uint32_t dst, uint32_t bar) {
+      mbar_expect_tx_warp(leader, bar, D * D * 2);
+      load_boxes<D, D>(leader, dst, it.role >= DK ? &maps.r : &maps.s, 0, ((it.edge * p.H + it.h) * 2 + term) * D, bar);
+    };
+    auto times_state = [&](bool trans, uint32_t m, bool add) {
+      const uint32_t idesc = make_idesc_bf16(C, D, false, !trans);
 #pragma unroll
-    for (int c = 0; c < D; ++c) M[c] = 0.f;
-    for (int n = span.x; n < span.y; ++n) {
-      const long long at = ((long long)(reverse ? span.x + span.y - 1 - n : n) * p.H + h) * D + i;
-      const float xi = __bfloat162float(x[at]);
-      ws[i] = __bfloat162float(w[at]);
-      zs[i] = __bfloat162float(z[at]);
-      __syncthreads();
-      float acc = 0.f;
+      for (int kk = 0; kk < D / 16; ++kk)
+        umma_f16_warp(leader, tmem + COL_O, make_smem_desc_sw128(sx + (kk >> 2) * (C * 128) + (kk & 3) * 32, 16, 1024),
+                      trans ? make_smem_desc_sw128(m + (kk >> 2) * (D * 128) + (kk & 3) * 32, 16, 1024)
+                            : make_smem_desc_sw128(m + kk * 2048, D * 128, 1024),
+                      idesc, add || kk ? 1u : 0u);
+    };
+    auto wait = [&](uint32_t bar, uint32_t ph, int code) {
+      return mbar_wait_warp(bar, ph, abort_flag, p.status, code);
+    };
+    ResultItem it = next(0);
+    if (it.len) load_xy(it);
+    int n = 0;
+    bool ok = true;
+    uint32_t open = it.len ? 1u : 0u, xy_ph = 0;           // loads in flight: bits xy, hi, lo, z
+    for (; it.len && ok; ++n) {
+      const uint32_t ph = n & 1;
+      const bool trans = it.role == DQ || it.role == DK;
+      if (!(ok = wait(xy_full, ph, ST_TIMEOUT_FULL))) break;
+      open &= ~1u;
+      tc_fence_after();
 #pragma unroll
-      for (int c = 0; c < D; ++c) {
-        M[c] = fmaf(M[c], a, xi * ws[c]);
-        acc = fmaf(M[c], zs[c], acc);
+      for (int kk = 0; kk < D / 16; ++kk) {
+        const uint32_t off = (kk >> 2) * (C * 128) + (kk & 3) * 32;
+        umma_f16_warp(leader, tmem + COL_S, make_smem_desc_sw128(sx + off, 16, 1024), make_smem_desc_sw128(sy + off, 16, 1024),
+                      idesc_s, kk ? 1u : 0u);
       }
-      out[at] = __float2bfloat16(acc * p.scale);
-      __syncthreads();
+      umma_commit_warp(leader, s_done);
+      // the last product of the item before has read Z, its result has been taken out of TMEM
+      if (n && !(ok = wait(o_done, ph ^ 1, ST_TIMEOUT_EMPTY))) break;
+      if (it.state) {
+        load_state(it, 0, sz, hi_full);
+        open |= 2u;
+        if (n && !(ok = wait(o_read, ph ^ 1, ST_TIMEOUT_TMEM_EMPTY))) break;
+        if (!(ok = wait(hi_full, ph, ST_TIMEOUT_FULL))) break;
+        open &= ~2u;
+        tc_fence_after();
+        times_state(trans, sz, false);
+        umma_commit_warp(leader, hi_done);
+        if (!(ok = wait(hi_done, ph, ST_TIMEOUT_EMPTY))) break;
+        load_state(it, 1, sy, lo_full);
+        open |= 4u;
+      } else {
+        if (leader) {
+          mbar_arrive(hi_full);
+          mbar_arrive(lo_full);
+        }
+        __syncwarp();
+        umma_commit_warp(leader, hi_done);
+        if (n && !(ok = wait(o_read, ph ^ 1, ST_TIMEOUT_TMEM_EMPTY))) break;
+      }
+      const CUtensorMap* mz = it.role == O ? &maps.v : it.role == DQ ? &maps.k : it.role == DK ? &maps.q : &maps.d;
+      mbar_expect_tx_warp(leader, z_full, L::TILE);
+      load_boxes<D, C>(leader, sz, mz, it.h * D, it.t, z_full);
+      open |= 8u;
+      if (it.state) {
+        if (!(ok = wait(lo_full, ph, ST_TIMEOUT_FULL))) break;
+        open &= ~4u;
+        tc_fence_after();
+        times_state(trans, sy, true);
+      }
+      umma_commit_warp(leader, m_done);
+      const bool state = it.state;
+      const int steps = warp_uniform((it.len + 15) / 16);
+      it = next(n + 1);
+      if (!(ok = wait(m_done, ph, ST_TIMEOUT_EMPTY))) break;
+      if (it.len) {
+        load_xy(it);
+        open |= 1u;
+        xy_ph = ph ^ 1;
+      }
+      if (!(ok = wait(z_full, ph, ST_TIMEOUT_FULL))) break;
+      open &= ~8u;
+      if (!(ok = wait(p_full, ph, ST_TIMEOUT_FULL))) break;
+      tc_fence_after();
+#pragma unroll
+      for (int term = 0; term < 2; ++term)
+#pragma unroll
+        for (int kk = 0; kk < C / 16; ++kk) {
+          if (kk >= steps) break;
+          umma_f16_ts_warp(leader, tmem + COL_O, tmem + COL_S + (kk >> 1) * 32 + term * 16 + (kk & 1) * 8,
+                           make_smem_desc_sw128(sz + kk * 2048, C * 128, 1024), idesc_z, (state || term || kk) ? 1u : 0u);
+        }
+      umma_commit_warp(leader, o_done);
     }
-  };
-  sweep(false, p.k, p.v, p.dout, p.dq);
-  sweep(true, p.q, p.dout, p.v, p.dk);
-  sweep(true, p.dout, p.q, p.k, p.dv);
-}
-
-// A chunk costs about the same however few of its 128 rows a sequence fills, the token kernels cost the same per token.
-// Measured, 8192 tokens, 16 heads, sequences of 8 / 12 / 16 / 32 tokens, us:
-//   heads of 128, forward    chunked 574 / 377 / 283 / 158      token by token 442 / 436 / 430 / 441
-//                            (226 and 134 at 16 and 32 since two CTAs share an SM)
-//                 + backward        1509 / 1004 / 753 / 423                    1520 / 1519 / 1524 / 1571
-//   heads of 64,  forward           183 / 123 / 94 / 57                        93 / 93 / 93 / 95
-//                 + backward        552 / 370 / 283 / 171                      368 / 372 / 375 / 382
-bool by_token(int T, int n_seq) { return (long long)n_seq * 16 > T; }
-
-// One result a CTA and two CTAs an SM, or all results in one CTA.  Heads of 128 only: with 64 several CTAs of either kind share
-// an SM.  There have to be CTAs to share SMs, and the gradients read 9 tiles instead of 4, which pays where the states' products
-// and loads are most of the work, not in sequences of one chunk.  Measured, us, all in one / one a CTA:
-//   heads of 128, 16384 tokens x 32 heads      forward 679 / 548    backward 1482 / 1316
-//   8192 x 16, sequences of 1024                       165 / 144              359 / 332
-//                           200                        157 / 138              331 / 321
-//                           128                         85 / 83               151 / 185
-//                            32                        161 / 134              269 / 327
-//   1000 x 16, one sequence                             34 / 38                58 / 64
-//   heads of 64, 16384 x 32                            241 / 247              505 / 529
-bool two_per_sm(int D, int T, int n_seq, int H, bool grad) {
-  return D == 128 && (long long)(T / C) * H > device_sm_count() && (!grad || (long long)n_seq * C < T);
+    // a wait that gave up: what was loading lands before the CTA goes
+    if (open & 1u) drain(xy_full, xy_ph);
+    if (open & 2u) drain(hi_full, n & 1);
+    if (open & 4u) drain(lo_full, n & 1);
+    if (open & 8u) drain(z_full, n & 1);
+    __syncwarp();
+  } else if (warp == 9) {
+    int id = blockIdx.x;
+    for (int n = 0;; ++n, id += gridDim.x) {
+      const ResultItem it = id < items ? find_item(p, id, ROLES, lane) : ResultItem{};
+      if (!mbar_wait_warp(item_read + 8 * (n & 1), ((n >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+      if (lane == 0) {
+        slots[n & 1] = it;
+        mbar_arrive(item_full + 8 * (n & 1));
+      }
+      __syncwarp();
+      if (it.len == 0) break;
+    }
+  } else {
+    const int q = warp & 3, half = warp >> 2, row = q * 32 + lane;
+    const uint32_t lanes = uint32_t(q * 32) << 16;
+    const uint32_t to = tmem + lanes + COL_O + half * (D / 2), ts = tmem + lanes + COL_S + half * 64;
+    const int blk = half * 2;                   // first of this warp's two blocks of 32 score columns
+    auto wait = [&](uint32_t bar, uint32_t ph, int code) {
+      return mbar_wait_warp(bar, ph, abort_flag, p.status, code);
+    };
+    bool noted = false;                         // this warp's words of `bad` are not zero
+    for (int n = 0;; ++n) {
+      const uint32_t ph = n & 1;
+      if (!wait(item_full + 8 * (n & 1), (n >> 1) & 1, ST_TIMEOUT_FULL)) break;
+      const ResultItem it = slots[n & 1];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(item_read + 8 * (n & 1));
+      if (it.len == 0) break;
+      const bool back = GRAD && it.role >= DK;
+      const float g2 = decay2(p, it.h);
+      // tokens of the row's own sequence that it sees: up to `far` back, or (back) ahead
+      int far;
+      {
+        const uint32_t upto = 0xffffffffu >> (31 - lane);
+        int start = 0, end = it.len;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const uint32_t m = it.starts[w];
+          const uint32_t below = w < q ? m : w == q ? m & upto : 0, above = w > q ? m : w == q ? m & ~upto : 0;
+          if (below) start = 32 * w + 31 - __clz(below);
+          if (above) end = min(end, 32 * w + __ffs(above) - 1);
+        }
+        far = back ? end - 1 - row : row - start;
+      }
+      if (!wait(s_done, ph, ST_TIMEOUT_TMEM_FULL)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {             // 32 scores -> their two terms, in the same columns
+        const int j0 = (blk + b) * 32, sign = back ? 1 : -1, gap0 = sign * (j0 - row);
+        uint32_t hi[16], lo[16];
+        // the columns' gaps are gap0 .. gap0 + 31 or gap0 - 31 .. gap0
+        if (__any_sync(0xffffffffu, back ? gap0 + 31 >= 0 && gap0 <= far : gap0 >= 0 && gap0 - 31 <= far)) {
+          uint32_t r[32];
+          tmem_ld_32x32(ts + b * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            float x[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int gap = gap0 + sign * (e + u);
+              x[u] = gap >= 0 && gap <= far ? __uint_as_float(r[e + u]) * (p.scale * exp2f(g2 * gap)) : 0.f;
+            }
+            split2(x[0], x[1], hi[e >> 1], lo[e >> 1]);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) hi[e] = lo[e] = 0;
+        }
+        tmem_st_32x16(ts + b * 32, hi);
+        tmem_st_32x16(ts + b * 32 + 16, lo);
+      }
+      if (!wait(m_done, ph, ST_TIMEOUT_TMEM_FULL)) break;
+      if (it.state) {
+        const bool reached = row >= it.s0 && row < it.s1;
+        const float w = back ? exp2f(g2 * (C - row)) : p.scale * exp2f(g2 * (row + 1));
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < D / 2; c += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(to + c, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) r[e] = reached ? __float_as_uint(__uint_as_float(r[e]) * w) : 0u;
+          tmem_st_32x32(to + c, r);
+        }
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      // Rows of several sequences meet in the last product, with weights of zero: what is not finite there is taken out of
+      // Z, and noted, so that it stays in its own sequence.
+      const bool several = (it.starts[0] & ~1u) | it.starts[1] | it.starts[2] | it.starts[3];
+      if (several) {
+        if (!wait(z_full, ph, ST_TIMEOUT_FULL)) break;
+        if (noted) {
+          for (int c = lane; c < D / 2; c += 32) bad[(half * (D / 2) + c) * 4 + q] = 0;
+          __syncwarp();
+          noted = false;
+        }
+        bool any = false;
+#pragma unroll 1
+        for (int c = half * (D / 16); c < (half + 1) * (D / 16); ++c) {
+          const uint32_t at = box_addr(sz + (c >> 3) * (C * 128), row, c & 7);
+          uint32_t x[4];
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(at) : "memory");
+          bool here = false;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const uint32_t m = 0x7f80u << (16 * (e & 1));
+            if ((x[e >> 1] & m) == m) {
+              atomicOr(&bad[(c * 8 + e) * 4 + q], 1u << lane);
+              x[e >> 1] &= ~(0xffffu << (16 * (e & 1)));
+              here = true;
+            }
+          }
+          if (here) sts16(at, x[0], x[1], x[2], x[3]);
+          any |= here;
+        }
+        if (any) *bad_item = n;
+        fence_proxy_async_smem();
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      // (p_full: all of the CTA's rows have been looked at)
+      const bool found = several && wait(p_full, ph, ST_TIMEOUT_FULL) && *bad_item == n;
+      if (!wait(o_done, ph, ST_TIMEOUT_TMEM_FULL)) break;
+      tc_fence_after();
+      __nv_bfloat16* out = !GRAD ? p.o : it.role == DQ ? p.dq : it.role == DK ? p.dk : p.dv;
+      __nv_bfloat16* dst = out + ((long long)(it.t + row) * p.H + it.h) * D + half * (D / 2);
+      uint32_t r[D / 2];
+#pragma unroll
+      for (int c = 0; c < D / 2; c += 32) tmem_ld_32x32(to + c, *reinterpret_cast<uint32_t(*)[32]>(r + c));
+      tmem_ld_wait();
+      if (found) {                              // a sum with such a term in it has no value
+        const int j0 = back ? row : row - far, j1 = back ? row + far : row;
+#pragma unroll
+        for (int c = 0; c < D / 2; ++c) {
+          bool seen = false;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            uint32_t m = bad[(half * (D / 2) + c) * 4 + w];
+            if (m == 0) continue;
+            for (; m; m &= m - 1) {
+              const int j = 32 * w + __ffs(m) - 1;
+              seen |= j >= j0 && j <= j1;
+            }
+          }
+          if (seen) r[c] = 0x7fffffffu;
+        }
+        noted = true;
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(o_read);       // and the notes, if any, are read: the next item's Z is loaded behind this
+      if (row < it.len) {
+#pragma unroll
+        for (int c = 0; c < D / 2; c += 16) {
+          uint32_t v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) v[u] = pack_bf16x2(__uint_as_float(r[c + 2 * u]), __uint_as_float(r[c + 2 * u + 1]));
+          stg32(dst + c, v);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 256);
+  }
 }
 
 template <int D>
 int launch_gla(const GlaParams& p, int T, bool grad, cudaStream_t s) {
-  if (by_token(T, p.n_seq)) {
-    const dim3 seqs(p.n_seq, p.H);
-    if (grad) gla_token_bwd_kernel<D><<<seqs, D, 0, s>>>(p);
-    else gla_token_fwd_kernel<D><<<seqs, D, 0, s>>>(p);
-    return (int)cudaGetLastError();
-  }
-  constexpr int B_SMEM = 2 * C * D * 2 + 128, R_SMEM = 3 * C * D * 2 + 128;
-  constexpr int O_SMEM = R_SMEM + 2 * D * D * 2, G_SMEM = O_SMEM + C * D * 2;
+  constexpr int W_SMEM = WalkSmem<D>::TOTAL, R_SMEM = ResultSmem<D>::TOTAL;
   static bool cfg = false;
   cudaError_t e;
   if (!cfg) {
     constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((e = cudaFuncSetAttribute(gla_boundary_kernel<D>, kAttr, B_SMEM)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(gla_out_kernel<D>, kAttr, O_SMEM)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(gla_grad_kernel<D>, kAttr, G_SMEM)) != cudaSuccess)
+    if ((e = cudaFuncSetAttribute(gla_walk_kernel<D>, kAttr, W_SMEM)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gla_result_kernel<D, false>, kAttr, R_SMEM)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gla_result_kernel<D, true>, kAttr, R_SMEM)) != cudaSuccess)
       return (int)e;
-    if constexpr (D == 128)
-      if ((e = cudaFuncSetAttribute(gla_result_kernel<D, false>, kAttr, R_SMEM)) != cudaSuccess ||
-          (e = cudaFuncSetAttribute(gla_result_kernel<D, true>, kAttr, R_SMEM)) != cudaSuccess)
-        return (int)e;
     cfg = true;
   }
-  const int bounds = T / C;                      // a sequence has at most (len - 1) / C boundaries
-  if (bounds > 0) {
-    gla_boundary_kernel<D><<<dim3(bounds, p.H, grad ? 2 : 1), THREADS, B_SMEM, s>>>(p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-    gla_scan_kernel<D><<<dim3(p.n_seq * (D * D / 1024), p.H, grad ? 2 : 1), 256, 0, s>>>(p);
+  const long long width = (long long)p.H * D, edges = (T - 1) / C;
+  GlaMaps m;
+  int rc = 0;
+  if ((rc = make_tmap_2d_bf16(&m.q, p.q, width, T, width, 64, C)) || (rc = make_tmap_2d_bf16(&m.k, p.k, width, T, width, 64, C)) ||
+      (rc = make_tmap_2d_bf16(&m.v, p.v, width, T, width, 64, C)))
+    return rc;
+  m.d = m.s = m.r = m.q;
+  if (grad && (rc = make_tmap_2d_bf16(&m.d, p.dout, width, T, width, 64, C))) return rc;
+  const int sms = device_sm_count();
+  if (edges > 0) {
+    const long long rows = edges * p.H * 2 * D;
+    if ((rc = make_tmap_2d_bf16(&m.s, p.S, D, rows, D, 64, D)) || (grad && (rc = make_tmap_2d_bf16(&m.r, p.R, D, rows, D, 64, D))))
+      return rc;
+    constexpr auto kHalf = CU_TENSOR_MAP_SWIZZLE_64B;
+    WalkMaps w{m.k, m.q, m.q, m.q, m.q, m.q};
+    if ((rc = make_tmap_2d(&w.v, p.v, width, T, width, WALK_COLS, C, 2, kHalf)) ||
+        (rc = make_tmap_2d(&w.s, p.S, D, rows, D, WALK_COLS, 32, 2, kHalf)) ||
+        (grad && (rc = make_tmap_2d(&w.d, p.dout, width, T, width, WALK_COLS, C, 2, kHalf))) ||
+        (grad && (rc = make_tmap_2d(&w.r, p.R, D, rows, D, WALK_COLS, 32, 2, kHalf))))
+      return rc;
+    const long long walks = (edges < p.n_seq ? edges : p.n_seq) * (D / WALK_COLS) * p.H * (grad ? 2 : 1);
+    if (walks > INT_MAX / 2) return -2;
+    gla_walk_kernel<D><<<(int)(walks < sms ? walks : sms), WALK_THREADS, W_SMEM, s>>>(w, p, grad);
     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
   }
-  dim3 grid((T + C - 1) / C + p.n_seq, p.H);   // at least the number of chunks of any packing of T tokens
-  if constexpr (D == 128)
-    if (two_per_sm(D, T, p.n_seq, p.H, grad)) {
-      grid.z = grad ? 3 : 1;
-      if (grad) gla_result_kernel<D, true><<<grid, THREADS, R_SMEM, s>>>(p);
-      else gla_result_kernel<D, false><<<grid, THREADS, R_SMEM, s>>>(p);
-      return (int)cudaGetLastError();
-    }
-  if (grad) gla_grad_kernel<D><<<grid, THREADS, G_SMEM, s>>>(p);
-  else gla_out_kernel<D><<<grid, THREADS, O_SMEM, s>>>(p);
+  const long long items = (edges + 1) * p.H * (grad ? 3 : 1);
+  if (items > INT_MAX / 2) return -2;
+  const int grid = (int)(items < 2 * sms ? items : 2 * sms);
+  if (grad) gla_result_kernel<D, true><<<grid, RES_THREADS, R_SMEM, s>>>(m, p, (int)items);
+  else gla_result_kernel<D, false><<<grid, RES_THREADS, R_SMEM, s>>>(m, p, (int)items);
   return (int)cudaGetLastError();
 }
 
@@ -600,33 +797,33 @@ int run_gla(const GlaParams& p, int T, int D, bool grad, cudaStream_t s) {
 
 extern "C" {
 
-// Rows of the state workspaces: the chunk boundaries a packed batch of T tokens can have at most, none for short sequences.
-int mcb_simple_gla_boundaries(int T, int n_seq) { return by_token(T, n_seq) ? 0 : T / C; }
+// Rows of the state workspaces: the edges between a batch's tiles.
+int mcb_simple_gla_edges(int T) { return T > 0 ? (T - 1) / C : 0; }
 
 // q, k, v, o [T, H, D]; decay [H] fp32 (log-decay per step, <= 0); cu_seqlens [n_seq + 1] int32 from 0 to T;
-// states [boundaries, H, D, D] fp32 workspace.  Boundaries outside the batch are clipped and reported through `status`.
+// states [edges, H, 2, D, D] bf16 workspace.  Boundaries outside the batch are clipped and reported through `status`.
 int mcb_simple_gla_fwd(const void* q, const void* k, const void* v, const float* decay, const int* cu_seqlens, void* o,
-                       float* states, int T, int n_seq, int H, int D, float scale, int* status, void* stream_) {
+                       void* states, int T, int n_seq, int H, int D, float scale, int* status, void* stream_) {
   if (n_seq <= 0 || T <= 0) return 0;
   GlaParams p{};
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
   p.o = (__nv_bfloat16*)o;
-  p.decay = decay; p.cu = cu_seqlens; p.S = states; p.T = T; p.n_seq = n_seq; p.H = H; p.scale = scale;
+  p.decay = decay; p.cu = cu_seqlens; p.S = (__nv_bfloat16*)states; p.T = T; p.n_seq = n_seq; p.H = H; p.scale = scale;
   p.status = status;
   return run_gla(p, T, D, false, reinterpret_cast<cudaStream_t>(stream_));
 }
 
-// states [2, boundaries, H, D, D] fp32 workspace
+// states [2, edges, H, 2, D, D] bf16 workspace
 int mcb_simple_gla_bwd(const void* q, const void* k, const void* v, const void* dout, const float* decay,
-                       const int* cu_seqlens, void* dq, void* dk, void* dv, float* states, int T, int n_seq, int H, int D,
-                       float scale, void* stream_) {
+                       const int* cu_seqlens, void* dq, void* dk, void* dv, void* states, int T, int n_seq, int H, int D,
+                       float scale, int* status, void* stream_) {
   if (n_seq <= 0 || T <= 0) return 0;
   GlaParams p{};
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
   p.dout = (const __nv_bfloat16*)dout;
   p.dq = (__nv_bfloat16*)dq; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
-  p.decay = decay; p.cu = cu_seqlens; p.S = states; p.R = states + (long long)(T / C) * H * D * D;
-  p.T = T; p.n_seq = n_seq; p.H = H; p.scale = scale;
+  p.decay = decay; p.cu = cu_seqlens; p.S = (__nv_bfloat16*)states; p.R = p.S + (long long)((T - 1) / C) * H * 2 * D * D;
+  p.T = T; p.n_seq = n_seq; p.H = H; p.scale = scale; p.status = status;
   return run_gla(p, T, D, true, reinterpret_cast<cudaStream_t>(stream_));
 }
 

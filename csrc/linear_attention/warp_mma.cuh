@@ -149,54 +149,72 @@ __device__ __forceinline__ void check_bounds(const int* __restrict__ cu, int n_s
   }
 }
 
-// One entry of the chunk list of a packed batch: sequence `s` contributes ceil(len / C) chunks and, between them,
-// ceil(len / C) - 1 boundaries.  Called by one warp; finds the sequence that holds item `id` of the list of chunks
-// (BOUNDARY = false) or of boundaries (true).  `seq` is -1 past the end.
+// How many of the first n boundaries lie below `value` (those before 0 count as 0): up to the first that does not; by one warp.
+__device__ __forceinline__ int bounds_below(const int* __restrict__ cu, int n, int value, int lane) {
+  int lo = 0, hi = n;                           // the answer lies in [lo, hi]
+  while (lo < hi) {
+    const int step = (hi - lo + 31) / 32, i = lo + lane * step;
+    const unsigned below = __ballot_sync(0xffffffffu, i < hi && max(cu[min(i, n - 1)], 0) < value);
+    const int c = ~below ? __ffs(~below) - 1 : 32;
+    if (c == 0) break;
+    hi = min(hi, lo + c * step);
+    lo += (c - 1) * step + 1;
+  }
+  return lo;
+}
+// The sequence that comes `rank`-th when the longest are taken first (ties in the batch's order).  n_seq <= 32; by one warp.
+__device__ __forceinline__ int longest_first(const int* __restrict__ cu, int n_seq, int T, int rank, int lane) {
+  const int2 s = seq_span(cu, min(lane, n_seq - 1), T);
+  const int len = lane < n_seq ? s.y - s.x : -1;
+  int before = 0;
+  for (int j = 0; j < n_seq; ++j) {
+    const int other = __shfl_sync(0xffffffffu, len, j);
+    before += other > len || (other == len && j < lane);
+  }
+  return __ffs(__ballot_sync(0xffffffffu, lane < n_seq && before == rank)) - 1;
+}
+
+// One entry of the chunk list of a packed batch: sequence `s` contributes ceil(len / C) chunks.  Called by one warp; finds the
+// sequence that holds chunk `id`.  `seq` is -1 past the end.
 struct ChunkPos {
-  int seq, index, t0, t1, boundary0;   // index inside the sequence; token bounds of the sequence; its first boundary
+  int seq, index, t0, t1;   // index inside the sequence; token bounds of the sequence
 };
 // A lane reads PER sequences at a time.
-template <int C, bool BOUNDARY, int PER>
+template <int C, int PER>
 __device__ __forceinline__ ChunkPos find_chunk_step(const int* __restrict__ cu, int n_seq, int T, int id, int lane) {
-  int done = 0, bdone = 0;
+  int done = 0;
   for (int s0 = 0; s0 < n_seq; s0 += 32 * PER) {
     const int first = s0 + lane * PER;
     int edge[PER + 1];
 #pragma unroll
     for (int u = 0; u <= PER; ++u) edge[u] = cu[min(first + u, n_seq)];
-    int nc[PER], mine = 0, bmine = 0;
+    int nc[PER], mine = 0;
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
       const int a = min(max(edge[u], 0), T), b = min(edge[u + 1], T);
       nc[u] = first + u < n_seq && b > a ? (b - a + C - 1) / C : 0;
-      bmine += max(nc[u] - 1, 0);
-      mine += BOUNDARY ? max(nc[u] - 1, 0) : nc[u];
+      mine += nc[u];
     }
-    int incl = mine, bincl = bmine;
+    int incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(0xffffffffu, incl, o), y = __shfl_up_sync(0xffffffffu, bincl, o);
-      if (lane >= o) {
-        incl += x;
-        bincl += y;
-      }
+      const int x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
     }
     const bool here = id >= done + incl - mine && id < done + incl;
     const unsigned m = __ballot_sync(0xffffffffu, here);
     if (m) {
-      ChunkPos p{-1, id - (done + incl - mine), 0, 0, bdone + bincl - bmine};
+      ChunkPos p{-1, id - (done + incl - mine), 0, 0};
       if (here) {
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
-          const int n = BOUNDARY ? max(nc[u] - 1, 0) : nc[u];
           if (p.seq >= 0) continue;
-          if (p.index < n) {
+          if (p.index < nc[u]) {
             p.seq = first + u;
             p.t0 = min(max(edge[u], 0), T);
             p.t1 = min(edge[u + 1], T);
           } else {
-            p.index -= n;
-            p.boundary0 += max(nc[u] - 1, 0);
+            p.index -= nc[u];
           }
         }
       }
@@ -205,19 +223,16 @@ __device__ __forceinline__ ChunkPos find_chunk_step(const int* __restrict__ cu, 
       p.index = __shfl_sync(0xffffffffu, p.index, w);
       p.t0 = __shfl_sync(0xffffffffu, p.t0, w);
       p.t1 = __shfl_sync(0xffffffffu, p.t1, w);
-      p.boundary0 = __shfl_sync(0xffffffffu, p.boundary0, w);
       return p;
     }
     done += __shfl_sync(0xffffffffu, incl, 31);
-    bdone += __shfl_sync(0xffffffffu, bincl, 31);
   }
-  return ChunkPos{-1, 0, 0, 0, 0};
+  return ChunkPos{-1, 0, 0, 0};
 }
 // With thousands of short sequences the search is a large part of a CTA's life, with a few it is one step either way.
-template <int C, bool BOUNDARY>
+template <int C>
 __device__ __forceinline__ ChunkPos find_chunk(const int* __restrict__ cu, int n_seq, int T, int id, int lane) {
-  return n_seq <= 64 ? find_chunk_step<C, BOUNDARY, 1>(cu, n_seq, T, id, lane)
-                     : find_chunk_step<C, BOUNDARY, 8>(cu, n_seq, T, id, lane);
+  return n_seq <= 64 ? find_chunk_step<C, 1>(cu, n_seq, T, id, lane) : find_chunk_step<C, 8>(cu, n_seq, T, id, lane);
 }
 
 }  // namespace mcb

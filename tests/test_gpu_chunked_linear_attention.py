@@ -373,3 +373,40 @@ def test_simple_gla_one_result_per_block(T, h, cuts):
     parts = [run(slice(0, h // 2)), run(slice(h // 2, h))]
     for got, *want in zip(run(slice(0, h)), *parts):
         assert torch.equal(got, torch.cat(want, dim=1))
+
+
+@pytest.mark.parametrize('T,d,cuts', [(300, 64, [128, 130, 256]), (400, 128, [5, 127, 129, 380]), (129, 64, [128]),
+                                      (1000, 128, list(range(7, 1000, 25))), (520, 64, [0, 384, 384, 500])])
+def test_simple_gla_tiles_shared_by_sequences(T, d, cuts):
+    """Sequences that begin and end anywhere in the tiles of 128 tokens, fewer and more of them than edges between tiles.  What
+    is infinite in one sequence stays there: every other token has the bits it has without it."""
+    from mcore_bridge_b200.ops.gdn import simple_gla
+    (q, k, v, dy), _ = _inputs(T, 2, d, 21)
+    decay = -torch.tensor([0.02, 0.5], device=DEV)
+    cu = torch.tensor([0] + cuts + [T], dtype=torch.int32, device=DEV)
+
+    def run(*tensors):
+        leaves = [t.detach().requires_grad_() for t in tensors[:3]]
+        o = simple_gla(*leaves, decay, cu)
+        return [o.detach(), *torch.autograd.grad(o, leaves, tensors[3])]
+
+    clean = run(q, k, v, dy)
+    wide = [t.double().requires_grad_() for t in (q, k, v)]
+    out = []
+    for s, e in _spans(T, cuts):
+        n = torch.arange(e - s, device=DEV, dtype=torch.float64)
+        gap = n[:, None] - n[None]
+        mix = torch.exp(decay.double()[:, None, None] * gap.clamp(min=0)) * (gap >= 0) * d ** -0.5
+        out.append(torch.einsum('hij,jhd->ihd', torch.einsum('ihd,jhd->hij', wide[0][s:e], wide[1][s:e]) * mix, wide[2][s:e]))
+    ref = torch.cat(out)
+    for a, b in zip(clean, [ref, *torch.autograd.grad(ref, wide, dy.double())]):
+        assert _rel(a, b) < 2 ** -8
+    first, last = max(_spans(T, cuts), key=lambda s: s[1] - s[0])
+    hit = [t.clone() for t in (q, k, v, dy)]
+    for t, value in zip(hit, (float('inf'), float('nan'), -float('inf'), float('inf'))):
+        t[(first + last) // 2, :, 3] = value
+    others = torch.ones(T, dtype=torch.bool, device=DEV)
+    others[first:last] = False
+    for a, b in zip(run(*hit), clean):
+        assert torch.equal(a[others], b[others])
+        assert not a[first:last].isfinite().all()
