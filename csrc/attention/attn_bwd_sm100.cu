@@ -206,9 +206,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* s_full = bars + 11;        // 2
   uint64_t* dp_full = bars + 13;       // 1
   uint64_t* dp_empty = bars + 14;      // 1
-  uint64_t* ds_full = bars + 15;       // 1
-  uint64_t* dq_full = bars + 16;       // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  uint64_t* ds_full = bars + 15;       // 2, by turns: a warp that has nothing to mask may be a block ahead of the others
+  uint64_t* dq_full = bars + 17;       // 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -230,10 +230,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       mbar_init(smem_u32(&v_full[i]), 1);
       mbar_init(smem_u32(&v_empty[i]), 1);
       mbar_init(smem_u32(&s_full[i]), 1);
+      mbar_init(smem_u32(&ds_full[i]), 8);
     }
     mbar_init(smem_u32(dp_full), 1);
     mbar_init(smem_u32(dp_empty), 8);
-    mbar_init(smem_u32(ds_full), 8);
     mbar_init(smem_u32(dq_full), 1);
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -323,7 +323,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (ok && nblk > 1) ok = issue_s(1);
       for (int j = 0; j < nblk && ok; ++j) {
         if (j + 1 < nblk && !issue_dp(j + 1)) { ok = false; break; }
-        if (!mbar_wait_warp(smem_u32(ds_full), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(smem_u32(&ds_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sk = smem_u32(smem + L::OFF_K + (j % 3) * L::TILE);
         const uint32_t ads = tmem + COL_S + (j & 1) * TM;
@@ -382,21 +382,21 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const uint32_t ts = tmem + lane_addr + COL_S + (j & 1) * TM + grp * HALF;
       const uint32_t td = tmem + lane_addr + COL_DP + grp * HALF;
       const int n0 = (kb0 + j) * TM + grp * HALF;
-      const bool full = __all_sync(0xffffffffu, lo <= n0 && n0 + HALF - 1 <= hi);
+      const Seen seen[2] = {seen_keys(lo, hi, n0), seen_keys(lo, hi, n0 + 32)};
       uint32_t pr[HALF];
       if (!mbar_wait(smem_u32(&s_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       tmem_ld_32x32_x64(ts, pr);
       tmem_ld_wait();
 #pragma unroll
-      for (int e = 0; e < HALF; e += 2) {
-        const float2 x = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1])), cc, nl));
-        pr[e] = __float_as_uint(ex2_ftz(x.x));
-        pr[e + 1] = __float_as_uint(ex2_ftz(x.y));
-      }
-      if (!full) {
+      for (int c = 0; c < 2; ++c) {
+        if (seen[c] == Seen::NONE) continue;
 #pragma unroll
-        for (int e = 0; e < HALF; ++e) pr[e] = (unsigned)(n0 + e - lo) <= span ? pr[e] : 0u;
+        for (int e = 32 * c; e < 32 * c + 32; e += 2) {
+          const float2 x = f32x2_split(fma_f32x2(f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1])), cc, nl));
+          pr[e] = __float_as_uint(ex2_ftz(x.x));
+          pr[e + 1] = __float_as_uint(ex2_ftz(x.y));
+        }
       }
       if (!mbar_wait(smem_u32(dp_full), j & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
@@ -408,20 +408,29 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (lane == 0) mbar_arrive(smem_u32(dp_empty));   // dP is in registers: the next dO V^T may start
       uint32_t pk[HALF / 2];
 #pragma unroll
-      for (int e = 0; e < HALF; e += 2) {
-        const uint64_t d2 = add_f32x2(f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1])), nd);
-        float2 x = f32x2_split(mul_f32x2(mul_f32x2(d2, f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1]))), sc));
-        if (!full) {                              // a masked pair contributes zero whatever its dP is
-          x.x = (unsigned)(n0 + e - lo) <= span ? x.x : 0.f;
-          x.y = (unsigned)(n0 + e + 1 - lo) <= span ? x.y : 0.f;
+      for (int c = 0; c < 2; ++c) {
+        if (seen[c] == Seen::NONE) {
+#pragma unroll
+          for (int e = 16 * c; e < 16 * c + 16; ++e) pk[e] = 0;
+          continue;
         }
-        pk[e >> 1] = pack_bf16x2(x.x, x.y);
+        const bool all = seen[c] == Seen::ALL;
+#pragma unroll
+        for (int e = 32 * c; e < 32 * c + 32; e += 2) {
+          const uint64_t d2 = add_f32x2(f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1])), nd);
+          float2 x = f32x2_split(mul_f32x2(mul_f32x2(d2, f32x2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1]))), sc));
+          if (!all) {                             // a masked pair contributes zero whatever its P and dP are
+            x.x = (unsigned)(n0 + e - lo) <= span ? x.x : 0.f;
+            x.y = (unsigned)(n0 + e + 1 - lo) <= span ? x.y : 0.f;
+          }
+          pk[e >> 1] = pack_bf16x2(x.x, x.y);
+        }
       }
       tmem_st_32x32(ts, pk);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(ds_full));
+      if (lane == 0) mbar_arrive(smem_u32(&ds_full[j & 1]));
     }
     __nv_bfloat16* row = p.dq + ((long long)i * p.nq + head) * D + grp * (D / 2);   // each group writes half of the row
     if (nblk <= 0) {
@@ -456,9 +465,9 @@ struct DkvSmem {
   static constexpr int OFF_V = TILE;
   static constexpr int OFF_Q = 2 * TILE;                // 2 stages
   static constexpr int OFF_DO = OFF_Q + 2 * TILE;       // 2 stages
-  static constexpr int OFF_COL = OFF_DO + 2 * TILE;     // 2 buffers: per-query lse / delta / k_lo / k_hi, then the
-                                                        // largest k_lo and the smallest k_hi of the block
-  static constexpr int COL_BYTES = 4 * TM * 4 + 16;
+  static constexpr int OFF_COL = OFF_DO + 2 * TILE;     // 2 buffers: per-query lse / delta / k_lo / k_hi, then of every 32
+                                                        // queries the largest and smallest k_lo, smallest and largest k_hi
+  static constexpr int COL_BYTES = 4 * TM * 4 + 4 * 16;
   static constexpr int OFF_BAR = OFF_COL + 2 * COL_BYTES;
   static constexpr int TOTAL = OFF_BAR + 1024 + 1024;
 };
@@ -519,21 +528,29 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     prefetch_tensormap(&tm_v);
     prefetch_tensormap(&tm_q);
     prefetch_tensormap(&tm_do);
-    if (p.q_lo == nullptr) {
-      // causal self-attention: the last query that can see a key of this tile is the largest i with
-      // k_lo[i] <= last key (k_lo = sequence starts, sorted); the first one is the tile's first key itself
-      const int n_last = min(n0 + TM - 1, p.Tk - 1);
-      int lo = n_last, hi = p.T - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (p.k_lo[mid] <= n_last) lo = mid; else hi = mid - 1;
-      }
+  }
+  __shared__ int s_rng[8];
+  if (p.q_lo != nullptr) {
+    tile_range_partial(p.q_lo, p.q_hi, n0, p.Tk, s_rng);
+  } else if (warp == 2) {
+    // causal self-attention: the last query that can see a key of this tile is the largest i with k_lo[i] <= last key (k_lo =
+    // sequence starts, sorted); the first one is the tile's first key itself.  The lanes look at 32 places at a time: a step
+    // waits for memory, and halving took 12 of them at 4096 tokens before the CTA's first load.
+    const int n_last = min(n0 + TM - 1, p.Tk - 1);
+    int lo = n_last, hi = p.T - 1;                 // the last one lies in [lo, hi]
+    while (lo < hi) {
+      const int step = (hi - lo + 31) / 32, i = min(lo + (lane + 1) * step, hi);
+      const unsigned past = __ballot_sync(0xffffffffu, p.k_lo[i] > n_last);
+      const int c = past ? __ffs(past) - 1 : 32;    // places that still see the key
+      const int from = lo;
+      if (c > 0) lo = min(from + c * step, hi);
+      if (c < 32) hi = min(min(from + (c + 1) * step, hi) - 1, hi);
+    }
+    if (lane == 0) {
       i_end_slot[0] = n0;
       i_end_slot[1] = lo;
     }
   }
-  __shared__ int s_rng[8];
-  if (p.q_lo != nullptr) tile_range_partial(p.q_lo, p.q_hi, n0, p.Tk, s_rng);
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
     tmem_relinquish();
@@ -634,45 +651,53 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       if (ok) umma_commit_warp(leader, smem_u32(out_full));
     } else if (warp == 2) {
       // ---------------------------------------------------------------- per-query values of the coming blocks
+      // A block's values are fetched while the block before it is laid down: their latency is longer than a block's products.
       int h = h_first, qb = 0;
-      for (int it = 0; it < iters; ++it) {
-        const uint32_t b = it & 1, ph = (it >> 1) & 1;
-        float* c_lse = reinterpret_cast<float*>(smem + L::OFF_COL + b * L::COL_BYTES);
-        float* c_delta = c_lse + TM;
-        int* c_lo = reinterpret_cast<int*>(c_delta + TM);
-        int* c_hi = c_lo + TM;
+      float lse[4], dl[4];
+      int klo[4], khi[4];
+      auto fetch = [&]() {
         const int i0 = (qb0 + qb) * TM;
-        float lse[4], dl[4];
-        int klo[4], khi[4], mxlo = 0, mnhi = INT_MAX;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int i = i0 + u * 32 + lane;
           lse[u] = i < p.T ? p.lse[(long long)h * p.T + i] : 0.f;
           dl[u] = i < p.T ? p.delta[(long long)h * p.T + i] : 0.f;
           attn_row_range(p.k_lo, p.k_hi, i, p.T, klo[u], khi[u]);
-          mxlo = max(mxlo, klo[u]);
-          mnhi = min(mnhi, khi[u]);
         }
+        if (++qb == nqb) { qb = 0; ++h; }
+      };
+      if (iters > 0) fetch();
+#pragma unroll 1
+      for (int it = 0; it < iters; ++it) {
+        const uint32_t b = it & 1, ph = (it >> 1) & 1;
+        float* c_lse = reinterpret_cast<float*>(smem + L::OFF_COL + b * L::COL_BYTES);
+        float* c_delta = c_lse + TM;
+        int* c_lo = reinterpret_cast<int*>(c_delta + TM);
+        int* c_hi = c_lo + TM;
+        float x_lse[4], x_dl[4];
+        int x_lo[4], x_hi[4];
 #pragma unroll
-        for (int s = 16; s; s >>= 1) {
-          mxlo = max(mxlo, __shfl_xor_sync(0xffffffffu, mxlo, s));
-          mnhi = min(mnhi, __shfl_xor_sync(0xffffffffu, mnhi, s));
+        for (int u = 0; u < 4; ++u) {
+          x_lse[u] = (lse[u] == -INFINITY) ? 0.f : -lse[u] * LOG2E;    // -inf: such a query sees nothing, masked below
+          x_dl[u] = -dl[u];
+          x_lo[u] = klo[u];
+          x_hi[u] = khi[u];
         }
+        if (it + 1 < iters) fetch();
         if (!mbar_wait(smem_u32(&col_empty[b]), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int c = u * 32 + lane;
-          c_lse[c] = (lse[u] == -INFINITY) ? 0.f : -lse[u] * LOG2E;    // -inf: such a query sees nothing, masked below
-          c_delta[c] = -dl[u];
-          c_lo[c] = klo[u];
-          c_hi[c] = khi[u];
-        }
-        if (lane == 0) {
-          c_hi[TM] = mxlo;
-          c_hi[TM + 1] = mnhi;
+          c_lse[c] = x_lse[u];
+          c_delta[c] = x_dl[u];
+          c_lo[c] = x_lo[u];
+          c_hi[c] = x_hi[u];
+          const bool sees = x_lo[u] <= x_hi[u];
+          const int4 edge = make_int4(__reduce_max_sync(0xffffffffu, x_lo[u]), __reduce_min_sync(0xffffffffu, sees ? x_lo[u] : INT_MAX),
+                                      __reduce_min_sync(0xffffffffu, x_hi[u]), __reduce_max_sync(0xffffffffu, sees ? x_hi[u] : -1));
+          if (lane == 0) reinterpret_cast<int4*>(c_hi + TM)[u] = edge;
         }
         mbar_arrive(smem_u32(&col_full[b]));
-        if (++qb == nqb) { qb = 0; ++h; }
       }
     }
   } else {
@@ -692,27 +717,33 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       const float* c_delta = c_lse + TM;
       const int* c_lo = reinterpret_cast<const int*>(c_delta + TM);
       const int* c_hi = c_lo + TM;
-      const int* c_meta = c_hi + TM - grp * HALF;
+      const int4* c_edge = reinterpret_cast<const int4*>(c_hi + TM - grp * HALF) + 2 * grp;
       if (!mbar_wait(smem_u32(&col_full[b]), (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
       // every query of the block sees this key: largest lower bound <= n <= smallest upper bound
-      const bool full = __all_sync(0xffffffffu, row_ok && c_meta[0] <= n && n <= c_meta[1]);
+      const bool full = __all_sync(0xffffffffu, row_ok && max(c_edge[0].x, c_edge[1].x) <= n && n <= min(c_edge[0].z, c_edge[1].z));
+      uint32_t seen[2] = {0xffffffffu, 0xffffffffu};   // bit e: this key is visible to query e of the half block
+      if (!full) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int4 x = c_edge[c];
+          const Seen some = seen_of(row_ok && x.x <= n && n <= x.z, row_ok && x.y <= n && n <= x.w);
+          if (some == Seen::ALL) continue;
+          seen[c] = 0u;
+          if (some == Seen::NONE) continue;
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            const int4 a = *reinterpret_cast<const int4*>(c_lo + 32 * c + e), z = *reinterpret_cast<const int4*>(c_hi + 32 * c + e);
+            const int aa[4] = {a.x, a.y, a.z, a.w}, zz[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) seen[c] |= (row_ok && aa[u] <= n && n <= zz[u]) ? 1u << (e + u) : 0u;
+          }
+        }
+      }
       if (!mbar_wait(smem_u32(s_full), it & 1, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       uint32_t pr[HALF];
       tmem_ld_32x32_x64(ts, pr);
       tmem_ld_wait();
-      uint32_t seen[2] = {0xffffffffu, 0xffffffffu};   // bit e: this key is visible to query e of the half block
-      if (!full) {
-        seen[0] = seen[1] = 0u;
-#pragma unroll
-        for (int e = 0; e < HALF; e += 4) {
-          const int4 a = *reinterpret_cast<const int4*>(c_lo + e), z = *reinterpret_cast<const int4*>(c_hi + e);
-          const int aa[4] = {a.x, a.y, a.z, a.w}, zz[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            seen[e >> 5] |= (row_ok && aa[u] <= n && n <= zz[u]) ? 1u << ((e + u) & 31) : 0u;
-        }
-      }
 #pragma unroll
       for (int u2 = 0; u2 < 2; ++u2) {
         uint32_t pk[16];

@@ -50,4 +50,20 @@ __device__ __forceinline__ int tile_range_max(const int* s_rng) {
   return max(max(s_rng[4], s_rng[5]), max(s_rng[6], s_rng[7]));
 }
 
+// How much of a 32 x 32 piece of a block (a warp's rows, 32 columns) is visible.  Half of a block on the diagonal, or at the edge of
+// a window, is not, and most of the rest is all visible: only SOME pays for comparisons, and where the arithmetic can branch
+// (dQ) NONE pays for nothing.  us, dQ / dK and dV, per block and per piece: 4095 tokens, 64 / 8 heads of 64, window 128 128 /
+// 138 and 109 / 113; 8192 in five sequences, 32 / 8 of 128 275 / 358 and 256 / 331 (of the latter 10 by the fetch ahead).  In the
+// forward and dK/dV kernels branches around the exponentials cost the blocks without a mask more (5 to 10 %, also as a loop
+// body of their own) than they gave the others.
+enum class Seen : int { NONE, SOME, ALL };
+__device__ __forceinline__ Seen seen_of(bool all, bool any) {
+  const bool a = __all_sync(0xffffffffu, all), b = __any_sync(0xffffffffu, any);
+  return a ? Seen::ALL : b ? Seen::SOME : Seen::NONE;
+}
+// rows with key ranges [lo, hi], keys n0 .. n0 + 31
+__device__ __forceinline__ Seen seen_keys(int lo, int hi, int n0) {
+  return seen_of(lo <= n0 && n0 + 31 <= hi, lo <= n0 + 31 && n0 <= hi);
+}
+
 }  // namespace mcb

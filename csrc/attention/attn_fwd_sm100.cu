@@ -331,11 +331,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       tmem_ld_wait();
       if (!full) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < 4; ++c) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            v[c][e] = (unsigned)(n0 + 32 * c + e - lo) <= span
-                          ? __float_as_uint(__uint_as_float(v[c][e]) * p.scale_log2) : 0xff800000u;
+          for (int e = 0; e < 32; ++e) v[c][e] = __float_as_uint(__uint_as_float(v[c][e]) * p.scale_log2);
+          if (seen_keys(lo, hi, n0 + 32 * c) == Seen::ALL) continue;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[c][e] = (unsigned)(n0 + 32 * c + e - lo) <= span ? v[c][e] : 0xff800000u;
+        }
       }
       float mx;
       {

@@ -101,3 +101,30 @@ def test_probabilities_keep_their_precision_over_many_blocks(T, d):
     rounded = ((p.bfloat16().double() @ vw) / p.sum(-1, keepdim=True)).bfloat16().double()
     # 4000 x 128 (1100 x 256) independent roundings: the two errors agree to far less than half a per cent by chance
     assert (o.transpose(0, 1).double() - ref).norm() <= 1.005 * (rounded - ref).norm()
+
+
+@pytest.mark.parametrize('nq,nkv,d', [(6, 2, 64), (5, 1, 128), (8, 2, 128)])
+@pytest.mark.parametrize('left', [0, 1, 31, 32, 33, 64, 127, 128, 129])
+def test_windows_at_the_edges_of_pieces(nq, nkv, d, left):
+    """The mask is looked at in pieces of 32 x 32: windows that end on, before and behind them; group sizes of 3 and 5, whose dK and
+    dV are summed from as many parts."""
+    from mcore_bridge_b200.ops.attention import attention
+    T, cuts = 420, [0, 33, 160, 420]
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    q, k, v, dy = (torch.randn(T, n, d, generator=gen, device=DEV).bfloat16() for n in (nq, nkv, nkv, nq))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    o = attention(*leaves, torch.tensor(cuts, dtype=torch.int32, device=DEV), 260, window=(left, 0))
+    grads = torch.autograd.grad(o, leaves, dy)
+    i = torch.arange(T, device=DEV)
+    seq = torch.bucketize(i, torch.tensor(cuts[1:], device=DEV), right=True)
+    vis = (seq[:, None] == seq[None]) & (i[None] <= i[:, None]) & (i[None] >= i[:, None] - left)
+    wide = [t.detach().double().requires_grad_() for t in leaves]
+    kw, vw = (t.transpose(0, 1).repeat_interleave(nq // nkv, 0) for t in wide[1:])
+    s = (wide[0].transpose(0, 1) @ kw.transpose(1, 2) * d ** -0.5).masked_fill(~vis[None], float('-inf'))
+    ref = (torch.softmax(s, -1) @ vw).transpose(0, 1)
+    want = torch.autograd.grad(ref, wide, dy.double())
+    # as above: one bf16 rounding of probabilities and result, two more in the gradients (with one visible key dq and dk are zero
+    # but for the rounding of dP - delta, whose terms are sums of d products of size 1)
+    assert (o.double() - ref).norm() < 2 ** -8 * ref.norm()
+    for a, b in zip(grads, want):
+        assert (a.double() - b).norm() < 2 ** -7 * max(b.norm().item(), 2 ** -8 * a.numel() ** 0.5)
