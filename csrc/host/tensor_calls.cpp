@@ -235,8 +235,11 @@ void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor&
            dx.data_ptr(), ptr(dw), 1, ptr(part), rows, H, x2.stride(0), eps, zc, stream());
 }
 
-// How many CTAs share one (key tile, kv head) pair in the dK/dV kernel: enough to put at least about three CTAs on every SM,
-// limited to divisors of the GQA ratio.  MCB200_ATTN_DKV_SPLITS overrides it.
+// How many CTAs share one (key tile, kv head) pair in the dK/dV kernel: the smallest divisor of the GQA ratio that puts about three
+// CTAs on every SM, or the largest there is; a step of more than twice is taken only while SMs are idle.  dK/dV and the sum of
+// the parts, us, whole / in 3, 3, 5 and 3 parts: 3000 tokens, 9 / 3 heads of 128 133 / 63, 8192 in seven sequences, 3 / 1 heads of 64
+// 107 / 48, 777, 5 / 1 of 128 35 / 18; 4096, 24 / 8 of 64 171 / 194 (256 pairs).
+// MCB200_ATTN_DKV_SPLITS overrides it.
 int dkv_splits(ll T, int nq, int nkv) {
   require(nkv > 0, "attention without key heads");
   const int qpg = nq / nkv;
@@ -252,7 +255,11 @@ int dkv_splits(ll T, int nq, int nkv) {
   }
   const ll ctas = (T + 127) / 128 * nkv;
   int s = 1;
-  while (ctas * s < 3ll * mcb_sm_count() && s * 2 <= qpg && qpg % (s * 2) == 0) s *= 2;
+  for (int next = 2; next <= qpg; ++next)
+    if (qpg % next == 0) {
+      if (ctas * s >= (next <= 2 * s ? 3ll : 1ll) * mcb_sm_count()) break;
+      s = next;
+    }
   return s;
 }
 

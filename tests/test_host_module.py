@@ -99,3 +99,6 @@ def test_split_of_the_key_gradient_kernel(monkeypatch):
     monkeypatch.delenv('MCB200_ATTN_DKV_SPLITS')
     with pytest.raises(AssertionError):
         nat.attn_dkv_splits(1000, 8, 0)
+    for tokens, heads, kv_heads, want in [(3000, 9, 3, 3), (777, 5, 1, 5), (2048, 32, 8, 4), (8192, 32, 8, 1), (100, 12, 2, 6),
+                                          (100, 7, 7, 1), (12800, 12, 2, 3), (4096, 24, 8, 1)]:
+        assert nat.attn_dkv_splits(tokens, heads, kv_heads) == want
