@@ -107,7 +107,7 @@ def build_host(verbose: bool = True, force: bool = False) -> Path:
     out = LIB_DIR / host_name()
     stamp = OBJ_DIR / f'{out.name}.sha1'
     h = hashlib.sha1()
-    for src in sorted((CSRC / 'host').glob('*.cpp')):
+    for src in sorted(p for e in ('cpp', 'h') for p in (CSRC / 'host').glob(f'*.{e}')):
         h.update(src.read_bytes())
     if out.exists() and stamp.exists() and stamp.read_text() == h.hexdigest() and not force:
         return out

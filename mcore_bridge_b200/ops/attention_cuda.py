@@ -65,23 +65,6 @@ def _row_starts(seq_start: torch.Tensor, T: int, device, one_each: bool) -> torc
     return (seq_start.expand(T) if n == 1 else seq_start[:T]).contiguous()
 
 
-class _AttnFn(torch.autograd.Function):
-
-    @staticmethod
-    def forward(ctx, q, k, v, seq_start, scale):
-        o, lse, q, k, v = _lib.native().attn_fwd(q, k, v, seq_start, None, None, scale)
-        ctx.save_for_backward(q, k, v, o, lse, seq_start)
-        ctx.scale = scale
-        return o
-
-    @staticmethod
-    def backward(ctx, do):
-        q, k, v, o, lse, seq_start = ctx.saved_tensors
-        dq, dk, dv, _ = _lib.native().attn_bwd(do, q, k, v, o, lse, seq_start, None, None, None, None, False,
-                                              ctx.scale)
-        return dq, dk, dv, None, None
-
-
 def attention(q, k, v, cu_seqlens, max_seqlen, scale, seq_start: Optional[torch.Tensor] = None, window=None,
               sinks: Optional[torch.Tensor] = None):
     """Packed causal self-attention.  ``window = (left, _)`` limits every query to its ``left`` most recent
@@ -94,7 +77,7 @@ def attention(q, k, v, cu_seqlens, max_seqlen, scale, seq_start: Optional[torch.
     left = None if window is None or window[0] is None or int(window[0]) < 0 else int(window[0])
     seq_start = _row_starts(seq_start, T, q.device, left is not None)
     if left is None and sinks is None:
-        return _AttnFn.apply(q, k, v, seq_start, float(scale))
+        return _lib.native().attention(q, k, v, seq_start, None, None, None, None, scale)[0]
     k_lo = seq_start
     if left is not None:
         # still non-decreasing, so the kernels' causal fast paths (k_hi = the query itself) apply unchanged
@@ -110,31 +93,6 @@ def ranges_supported(q, k, v) -> bool:
     d = q.shape[-1]
     return (q.is_cuda and q.dtype == torch.bfloat16 and d in (64, 128) and v.shape[-1] == d and k.shape[-1] == d
             and q.shape[1] % k.shape[1] == 0 and _lib.available())
-
-
-class _AttnRangesFn(torch.autograd.Function):
-    """``o[i] = softmax over keys k_lo[i]..k_hi[i] of q[i] k^T * scale`` applied to ``v``; queries ``[T, nq, d]`` and
-    keys / values ``[Tk, nkv, d]`` may be different token sets.  ``q_lo`` / ``q_hi`` ``[Tk]`` bound, per key, the
-    queries that can see it (they only limit the loops of the dK/dV kernel)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, k_lo, k_hi, q_lo, q_hi, scale, sinks=None):
-        sk = None if sinks is None else sinks.detach().float().contiguous()
-        o, lse, q, k, v = _lib.native().attn_fwd(q, k, v, k_lo, k_hi, sk, scale)
-        ctx.save_for_backward(q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sk)
-        ctx.scale = scale
-        ctx.sink_dtype = None if sinks is None else sinks.dtype
-        ctx.mark_non_differentiable(lse)
-        return o, lse
-
-    @staticmethod
-    def backward(ctx, do, _dlse):
-        q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sk = ctx.saved_tensors
-        dq, dk, dv, dsinks = _lib.native().attn_bwd(do, q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sk,
-                                                    ctx.sink_dtype == torch.bfloat16, ctx.scale)
-        if dsinks is not None:
-            dsinks = dsinks.to(ctx.sink_dtype)
-        return dq, dk, dv, None, None, None, None, None, dsinks
 
 
 def fwd_ranges_raw(q, k, v, k_lo, k_hi, scale: float):
@@ -170,8 +128,12 @@ def bwd_ranges_raw(q, k, v, o, do, lse, delta, k_lo, k_hi, q_lo, q_hi, scale: fl
 
 def attention_ranges(q, k, v, k_lo, k_hi, q_lo, q_hi, scale: Optional[float] = None,
                      sinks: Optional[torch.Tensor] = None):
-    """Returns ``(o [T, nq, d], lse [nq, T])``; all four range tensors are int32 on the device (``k_hi`` / ``q_lo`` /
+    """``o[i] = softmax over keys k_lo[i]..k_hi[i] of q[i] k^T * scale`` applied to ``v``; queries ``[T, nq, d]`` and
+    keys / values ``[Tk, nkv, d]`` may be different token sets.  ``q_lo`` / ``q_hi`` ``[Tk]`` bound, per key, the
+    queries that can see it (they only limit the loops of the dK/dV kernel).
+
+    Returns ``(o [T, nq, d], lse [nq, T])``; all four range tensors are int32 on the device (``k_hi`` / ``q_lo`` /
     ``q_hi`` may all be ``None`` for masks of the causal family: ``k_hi[i] = i`` and a non-decreasing ``k_lo``)."""
     if scale is None:
         scale = 1.0 / math.sqrt(q.shape[-1])
-    return _AttnRangesFn.apply(q, k, v, k_lo, k_hi, q_lo, q_hi, float(scale), sinks)
+    return _lib.native().attention(q, k, v, k_lo, k_hi, q_lo, q_hi, sinks, scale)

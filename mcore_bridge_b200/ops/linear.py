@@ -22,7 +22,7 @@ import torch
 
 from ..parallel import mappings as M
 from ..parallel import state as ps
-from . import gemm
+from . import _lib, gemm
 
 
 @dataclass(frozen=True)
@@ -174,11 +174,20 @@ class _LinearFn(torch.autograd.Function):
         return dx, dw, db, None
 
 
+def _single_rank(x, weight, bias, spec: LinearSpec):
+    """The module whose ``linear`` is the whole function where no collective, no fp8 and no fallback is in it."""
+    if spec.fp8 or not (x.is_cuda and weight.is_cuda and x.dtype == torch.bfloat16) or (bias is not None and not bias.is_cuda) \
+            or (spec.mode and ps.get_world_size(spec.group) > 1):
+        return None
+    return _lib.native_if_enabled()
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            spec: LinearSpec = LinearSpec()) -> torch.Tensor:
     if weight.dtype != x.dtype:
         x = x.to(weight.dtype)
-    y = _LinearFn.apply(x, weight, bias, spec)
+    nat = _single_rank(x, weight, bias, spec)
+    y = _LinearFn.apply(x, weight, bias, spec) if nat is None else nat.linear(x, weight, bias, spec.skip_weight_grad)
     if spec.mode == 'column' and spec.gather_output:
         y = M.gather_from_tensor_model_parallel_region(y, spec.group)
     return y

@@ -18,28 +18,11 @@ def rmsnorm_ref(x: torch.Tensor, w: torch.Tensor, eps: float, zero_centered: boo
     return (y * wf).to(x.dtype)
 
 
-class _RMSNormCuda(torch.autograd.Function):
-
-    @staticmethod
-    def forward(ctx, x, w, eps, zero_centered):
-        y, x2, rstd = _lib.native().rmsnorm_fwd(x, w, eps, zero_centered)
-        ctx.save_for_backward(x2, w, rstd)
-        ctx.eps, ctx.zc, ctx.shape = eps, zero_centered, x.shape
-        return y if x.dim() == 2 else y.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, w, rstd = ctx.saved_tensors
-        # the weight gradient's per-CTA partial rows are summed in a fixed order: it repeats bit for bit
-        dx, dw = _lib.native().rmsnorm_bwd(dy, x2, w, rstd, ctx.eps, ctx.zc, ctx.needs_input_grad[1])
-        return dx.view(ctx.shape), dw, None, None
-
-
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, zero_centered: bool = False) -> torch.Tensor:
     """Normalises the last dimension.  ``x`` may be ``[..., H]`` (per-head norm: pass ``[..., heads, d]``)."""
     if x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 \
             and x.shape[-1] <= 16384 and _lib.available():
-        return _RMSNormCuda.apply(x, w, eps, zero_centered)
+        return _lib.native().rmsnorm(x, w, eps, zero_centered)
     return rmsnorm_ref(x, w, eps, zero_centered)
 
 

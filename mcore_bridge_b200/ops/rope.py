@@ -62,22 +62,6 @@ def qkv_split_norm_rope_ref(qkv, wq, wk, cos, sin, ng, qpg, d, has_gate, interle
     return q.contiguous(), k.contiguous(), v.contiguous(), (gate.contiguous() if gate is not None else None)
 
 
-class _QkvCuda(torch.autograd.Function):
-
-    @staticmethod
-    def forward(ctx, qkv, wq, wk, cos, sin, ng, qpg, d, has_gate, interleaved, eps, zero_centered):
-        meta = (ng, qpg, d, has_gate, interleaved, eps, zero_centered)
-        q, k, v, gate, qkv = _lib.native().qkv_fwd(qkv, wq, wk, cos, sin, *meta)
-        ctx.save_for_backward(qkv, wq, wk, cos, sin)
-        ctx.meta = meta
-        return q, k, v, gate
-
-    @staticmethod
-    def backward(ctx, dq, dk, dv, dgate):
-        dqkv, dwq, dwk = _lib.native().qkv_bwd(dq, dk, dv, dgate, *ctx.saved_tensors, *ctx.meta)
-        return (dqkv, dwq, dwk) + (None,) * 9
-
-
 def qkv_split_norm_rope(qkv: torch.Tensor, wq: Optional[torch.Tensor], wk: Optional[torch.Tensor],
                         cos: Optional[torch.Tensor], sin: Optional[torch.Tensor], num_groups: int,
                         q_per_group: int, head_dim: int, has_gate: bool = False, interleaved: bool = False,
@@ -88,7 +72,7 @@ def qkv_split_norm_rope(qkv: torch.Tensor, wq: Optional[torch.Tensor], wk: Optio
             and (wq is None or wq.dtype == torch.bfloat16)):
         if cos is not None:
             cos, sin = cos.float().contiguous(), sin.float().contiguous()
-        return _QkvCuda.apply(qkv, wq, wk, cos, sin, num_groups, q_per_group, head_dim, has_gate, interleaved, eps,
-                              zero_centered)
+        return _lib.native().qkv(qkv, wq, wk, cos, sin, num_groups, q_per_group, head_dim, has_gate, interleaved, eps,
+                                 zero_centered)
     return qkv_split_norm_rope_ref(qkv, wq, wk, cos, sin, num_groups, q_per_group, head_dim, has_gate, interleaved,
                                    eps, zero_centered)

@@ -1,0 +1,124 @@
+"""The operations whose autograd nodes are native: what torch's machinery expects of a node (shapes, gradients that are not wanted,
+saved-tensor hooks, in-place checks, second passes, `main_grad`), and the transforms they refuse."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV, BF16 = 'cuda', torch.bfloat16
+
+
+def _rand(*shape, seed=1, scale=1.0):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    return (torch.randn(*shape, generator=gen, device=DEV) * scale).to(BF16)
+
+
+def _ops():
+    from mcore_bridge_b200.ops import fused_mlp
+    from mcore_bridge_b200.ops.attention import attention
+    from mcore_bridge_b200.ops.linear import linear
+    from mcore_bridge_b200.ops.norm import rmsnorm
+    from mcore_bridge_b200.ops.rope import qkv_split_norm_rope
+    cu = torch.tensor([0, 30, 70], dtype=torch.int32, device=DEV)
+    return dict(
+        linear=(lambda x, w, b: linear(x, w, b), [_rand(70, 64), _rand(96, 64, seed=2), _rand(96, seed=3)]),
+        linear3=(lambda x, w: linear(x, w), [_rand(2, 35, 64), _rand(96, 64, seed=2)]),
+        rmsnorm=(lambda x, w: rmsnorm(x, w), [_rand(5, 14, 64), _rand(64, seed=2)]),
+        norm_linear=(lambda x, l, w: fused_mlp.norm_linear(x, l, w, 1e-6, False),
+                     [_rand(2, 35, 64), _rand(64, seed=2), _rand(96, 64, seed=3)]),
+        glu_linear=(lambda h, w: fused_mlp.glu_linear(h, w, 0, 0.0, 0.0), [_rand(2, 35, 128), _rand(96, 64, seed=2)]),
+        qkv=(lambda x, a, b: torch.cat([t.reshape(70, -1) for t in qkv_split_norm_rope(x, a, b, None, None, 2, 2, 64)[:3]], -1),
+             [_rand(70, 512), _rand(64, seed=2), _rand(64, seed=3)]),
+        attention=(lambda q, k, v: attention(q, k, v, cu, 40), [_rand(70, 4, 64), _rand(70, 2, 64, seed=2), _rand(70, 2, 64, seed=3)]),
+        sinks=(lambda q, k, v, s: attention(q, k, v, cu, 40, sinks=s),
+               [_rand(70, 4, 64), _rand(70, 2, 64, seed=2), _rand(70, 2, 64, seed=3), _rand(4, seed=4)]))
+
+
+NAMES = ['linear', 'linear3', 'rmsnorm', 'norm_linear', 'glu_linear', 'qkv', 'attention', 'sinks']
+
+
+@pytest.mark.parametrize('name', NAMES)
+def test_a_node_behaves_as_one_of_torch(name):
+    fn, inputs = _ops()[name]
+    leaves = [t.clone().requires_grad_() for t in inputs]
+    y = fn(*leaves)
+    dy = torch.randn_like(y)
+    want = torch.autograd.grad(y, leaves, dy, retain_graph=True)
+    for g, t in zip(want, leaves):
+        assert g.shape == t.shape and g.dtype == t.dtype and g.isfinite().all()
+    for a, b in zip(torch.autograd.grad(y, leaves, dy), want):          # the same bits again, then the graph is gone
+        assert torch.equal(a, b)
+    with pytest.raises(RuntimeError, match='second time'):
+        torch.autograd.grad(y, leaves, dy)
+    with torch.no_grad():
+        assert torch.equal(fn(*leaves), y) and not fn(*leaves).requires_grad
+    # one input at a time wants a gradient: the others' come out as before where they are wanted
+    for i in range(len(inputs)):
+        some = [t.clone().requires_grad_(j == i) for j, t in enumerate(inputs)]
+        assert torch.equal(torch.autograd.grad(fn(*some), [some[i]], dy)[0], want[i])
+    # an expanded gradient, and hooks that replace what is saved
+    packed = []
+
+    def pack(t):
+        packed.append(t)
+        return t.cpu() if t.is_cuda else t
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.to(DEV)):
+        z = fn(*leaves)
+    assert packed
+    for a, b in zip(torch.autograd.grad(z, leaves, dy), want):
+        assert torch.equal(a, b)
+    ones = torch.autograd.grad(fn(*leaves).sum(), leaves)
+    for a, b in zip(ones, torch.autograd.grad(fn(*leaves), leaves, torch.ones_like(dy))):
+        assert torch.equal(a, b)
+    # a saved input that changes in place is noticed
+    last = [t.clone().requires_grad_() for t in inputs]
+    moved = [t * 1 for t in last]
+    z = fn(*moved)
+    with torch.no_grad():
+        for t in moved:
+            t.add_(1)
+    with pytest.raises(RuntimeError, match='inplace'):
+        torch.autograd.grad(z, last, dy)
+
+
+@pytest.mark.parametrize('name', NAMES)
+def test_transforms_are_refused(name):
+    fn, inputs = _ops()[name]
+    with pytest.raises((RuntimeError, NotImplementedError)):
+        torch.func.vmap(lambda t: fn(t, *inputs[1:]))(torch.stack([inputs[0]] * 2))
+    import torch.autograd.forward_ad as fw
+    with fw.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
+        fn(fw.make_dual(inputs[0], torch.ones_like(inputs[0])), *inputs[1:])
+
+
+@pytest.mark.parametrize('name,at', [('linear', 1), ('linear3', 1), ('norm_linear', 2), ('glu_linear', 1)])
+def test_weight_gradients_go_where_the_optimizer_wants_them(name, at):
+    fn, inputs = _ops()[name]
+    leaves = [torch.nn.Parameter(t.clone()) for t in inputs]
+    dy = torch.randn_like(fn(*leaves))
+    want = torch.autograd.grad(fn(*leaves), leaves, dy)
+    w, calls = leaves[at], []
+    w.main_grad = torch.ones(w.shape, device=DEV)
+    w.grad_ready_hook = lambda: calls.append(w.main_grad.clone())
+    fn(*leaves).backward(dy)
+    assert w.grad is None and len(calls) == 1 and torch.equal(calls[0], w.main_grad)
+    # fp32 sum of the product that was rounded to bf16 before: half a unit in the last place of 8 bits
+    assert ((w.main_grad - 1) - want[at].float()).abs().max() <= 2 ** -8 * want[at].float().abs().max() + 1e-5
+    for i, t in enumerate(leaves):
+        assert i == at or torch.equal(t.grad, want[i])
+
+    def broken():
+        raise ValueError('not now')
+
+    w.grad_ready_hook = broken
+    with pytest.raises(ValueError, match='not now'):
+        fn(*leaves).backward(dy)
+
+
+def test_outputs_nobody_uses():
+    from mcore_bridge_b200.ops.rope import qkv_split_norm_rope
+    x = _rand(70, 512).requires_grad_()
+    q, k, v, gate = qkv_split_norm_rope(x, None, None, None, None, 2, 2, 64)
+    assert gate is None
+    dx = torch.autograd.grad(k, x, torch.ones_like(k))[0].view(70, 2, 4, 64)
+    assert (dx[:, :, 2] == 1).all() and (dx[:, :, :2] == 0).all() and (dx[:, :, 3] == 0).all()
