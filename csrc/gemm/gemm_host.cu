@@ -83,27 +83,26 @@ int pick_bn(int M, int N, int groups, int mn_major, int sms) {
   return best;
 }
 
-}  // namespace
-
-extern "C" {
-
-int mcb_sm_count() { return device_sm_count(); }
-
 // Returns 0 on success, a negative code for bad arguments, or a positive cudaError_t.
 //   A: K-major  -> [a_outer rows, a_inner = contraction] with leading dimension lda
 //      MN-major -> [a_outer = contraction rows, a_inner = M] with leading dimension lda
 //   B likewise (rows of a K-major B are the N index).
-int mcb_gemm_bf16(const void* A, long long a_inner, long long a_outer, long long lda, int a_mn,  //
-                  const void* B, long long b_inner, long long b_outer, long long ldb, int b_mn,  //
-                  void* C, long long ldc, long long c_group_stride, int c_fp32, int accumulate,  //
-                  int M, int N, int K, float alpha, const void* bias,                            //
-                  int mode, int num_groups, const int* offsets, int b_group_rows,               //
-                  int* status, int max_sms, int force_bn, void* stream_) {
+//   res      null, or [M, N] bf16 with rows of ldr elements: C = bf16(result) + res (bf16 C, no accumulation, N and both row
+//            strides multiples of 8, both on 16-byte boundaries)
+int gemm_bf16(const void* A, long long a_inner, long long a_outer, long long lda, int a_mn,  //
+              const void* B, long long b_inner, long long b_outer, long long ldb, int b_mn,  //
+              void* C, long long ldc, long long c_group_stride, int c_fp32, int accumulate,  //
+              int M, int N, int K, float alpha, const void* bias, const void* res, long long ldr,  //
+              int mode, int num_groups, const int* offsets, int b_group_rows,               //
+              int* status, int max_sms, int force_bn, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0) return 0;
   if (mode != GEMM_DENSE && (num_groups <= 0 || num_groups > GEMM_MAX_GROUPS || offsets == nullptr)) return -2;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
     return -3;  // TMA needs 16-byte aligned bases and strides
+  if (res && (c_fp32 || accumulate || mode != GEMM_DENSE || K <= 0 || N % 8 || ldc % 8 || ldr % 8 ||
+              (reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(res) & 15)))
+    return -5;
   int sms = device_sm_count();
   if (max_sms > 0 && max_sms < sms) sms = max_sms;
   int groups = (mode == GEMM_GROUPED_K) ? num_groups : 1;
@@ -130,6 +129,7 @@ int mcb_gemm_bf16(const void* A, long long a_inner, long long a_outer, long long
   p.M = M; p.N = N; p.K = K;
   p.C = C; p.ldc = ldc; p.c_group_stride = c_group_stride;
   p.bias = bias; p.c_fp32 = c_fp32; p.alpha = alpha;
+  p.res = reinterpret_cast<const __nv_bfloat16*>(res); p.ldr = ldr;
   // grouped-K (expert weight gradients): many output tiles per unit of math, where reductions would queue at the L2
   p.accumulate = accumulate ? (mode == GEMM_GROUPED_K && c_fp32 ? 2 : 1) : 0;
   p.mode = mode; p.num_groups = num_groups; p.offsets = offsets; p.b_group_rows = b_group_rows;
@@ -148,6 +148,29 @@ int mcb_gemm_bf16(const void* A, long long a_inner, long long a_outer, long long
   else if (bn == 128) e = launch_major<128>(a_mn, b_mn, ta, tb, p, grid, stream);
   else e = launch_major<64>(a_mn, b_mn, ta, tb, p, grid, stream);
   return (int)e;
+}
+
+}  // namespace
+
+extern "C" {
+
+int mcb_sm_count() { return device_sm_count(); }
+
+int mcb_gemm_bf16(const void* A, long long a_inner, long long a_outer, long long lda, int a_mn,  //
+                  const void* B, long long b_inner, long long b_outer, long long ldb, int b_mn,  //
+                  void* C, long long ldc, long long c_group_stride, int c_fp32, int accumulate,  //
+                  int M, int N, int K, float alpha, const void* bias,                            //
+                  int mode, int num_groups, const int* offsets, int b_group_rows,               //
+                  int* status, int max_sms, int force_bn, void* stream) {
+  return gemm_bf16(A, a_inner, a_outer, lda, a_mn, B, b_inner, b_outer, ldb, b_mn, C, ldc, c_group_stride, c_fp32, accumulate, M,
+                   N, K, alpha, bias, nullptr, 0, mode, num_groups, offsets, b_group_rows, status, max_sms, force_bn, stream);
+}
+
+// C[M, N] = res[M, N] + A[M, K] . B[N, K]^T (+ bias), bf16, both operands K-major
+int mcb_gemm_bf16_residual(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, const void* res,
+                           long long ldr, int M, int N, int K, const void* bias, int* status, void* stream) {
+  return gemm_bf16(A, K, M, lda, 0, B, K, N, ldb, 0, C, ldc, 0, 0, 0, M, N, K, 1.f, bias, res, ldr, GEMM_DENSE, 0, nullptr, 0, status,
+                   0, 0, stream);
 }
 
 // Fused language-model head on the GEMM engine: logits = A[M,K] . B[N,K]^T (both K-major) are consumed by the

@@ -59,6 +59,8 @@ struct GemmParams {
   float* ce_tgt;               // EPI_CE_STATS: [M] label logit, written by the tile that holds the label's column
   const float* ce_lse;         // EPI_CE_GRAD: [M] log-sum-exp over the whole vocabulary
   const float* ce_g;           // EPI_CE_GRAD: [M] upstream gradient of each row's loss
+  const __nv_bfloat16* res;    // optional, [M, N] with rows of `ldr` elements: added to the rounded result (the sum rounded again),
+  long long ldr;               // where the result leaves through epilogue_store_bf16
   int* status;          // device status word, 0 = ok
 };
 
@@ -127,9 +129,13 @@ constexpr int EPI_STAGE_BYTES = 4 * EPI_STAGE_WARP;
 // gradients: 4 to 6 k-blocks per tile) were bound by the former: 128 experts x (1536 + 768) x 2048, 256 rows each,
 // 757 -> 466 us.
 // WIDE = 64 columns at a time (4 KiB of shared memory per warp) or 32 (2 KiB, 64 contiguous bytes a row).
+// With `res` (a row is `ldr` elements, 16-byte boundaries as C) C = bf16(bf16(...) + res): the lanes read the 16 bytes they write
+// from there before they wait for the accumulators.  us, the product, with an addition of its own, with `res`: 8192 x 4096 x 4096
+// 174, 204, 188; x 12288 548, 575, 558; 773 x 2048 x 6144 35, 43, 39; 201 x 256 x 256 10.4, 15.5, 10.6.
 template <int BN, int WIDE = 64>
 __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* stage, __nv_bfloat16* C, long long ldc, int row0,
-                                                    int m_limit, int n0, int N, float alpha, const __nv_bfloat16* bias) {
+                                                    int m_limit, int n0, int N, float alpha, const __nv_bfloat16* bias,
+                                                    const __nv_bfloat16* res = nullptr, long long ldr = 0) {
   const int lane = threadIdx.x & 31;
   constexpr int CH = WIDE / 8;                   // 16-byte chunks of a row
   auto at = [&](int row, int j) {                // chunks of a row are permuted so that neither side has bank conflicts
@@ -138,32 +144,50 @@ __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* 
 #pragma unroll 1
   for (int cc = 0; cc < BN; cc += WIDE) {
     if (n0 + cc >= N) break;
+    const int j = lane % CH, col = n0 + cc + 8 * j;
+    uint4 add[CH];
+    if (res) {
+#pragma unroll
+      for (int it = 0; it < CH; ++it) {
+        const int rr = it * (32 / CH) + lane / CH;
+        add[it] = row0 + rr < m_limit && col < N ? *reinterpret_cast<const uint4*>(res + (long long)(row0 + rr) * ldr + col)
+                                                 : make_uint4(0, 0, 0, 0);
+      }
+    }
     uint32_t r[WIDE];
     if constexpr (WIDE == 64) tmem_ld_32x32_x64(tmem_row + cc, r);
     else tmem_ld_32x32(tmem_row + cc, r);
     tmem_ld_wait();
 #pragma unroll
-    for (int j = 0; j < CH; ++j) {
+    for (int c = 0; c < CH; ++c) {
       float v[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]) * alpha;
-      if (bias && n0 + cc + 8 * j < N) {
+      for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * c + e]) * alpha;
+      if (bias && n0 + cc + 8 * c < N) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] += __bfloat162float(bias[n0 + cc + 8 * j + e]);
+        for (int e = 0; e < 8; ++e) v[e] += __bfloat162float(bias[n0 + cc + 8 * c + e]);
       }
       uint4 o;
       o.x = pack_bf16x2(v[0], v[1]);
       o.y = pack_bf16x2(v[2], v[3]);
       o.z = pack_bf16x2(v[4], v[5]);
       o.w = pack_bf16x2(v[6], v[7]);
-      *reinterpret_cast<uint4*>(at(lane, j)) = o;
+      *reinterpret_cast<uint4*>(at(lane, c)) = o;
     }
     __syncwarp();
-    const int j = lane % CH, col = n0 + cc + 8 * j;
 #pragma unroll
     for (int it = 0; it < CH; ++it) {
       const int rr = it * (32 / CH) + lane / CH;
-      const uint4 o = *reinterpret_cast<const uint4*>(at(rr, j));
+      uint4 o = *reinterpret_cast<const uint4*>(at(rr, j));
+      if (res) {
+        __nv_bfloat162 *x = reinterpret_cast<__nv_bfloat162*>(&o);
+        const __nv_bfloat162* y = reinterpret_cast<const __nv_bfloat162*>(&add[it]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __bfloat1622float2(x[e]), g = __bfloat1622float2(y[e]);
+          x[e] = __floats2bfloat162_rn(f.x + g.x, f.y + g.y);
+        }
+      }
       if (row0 + rr < m_limit && col < N) *reinterpret_cast<uint4*>(C + (long long)(row0 + rr) * ldc + col) = o;
     }
     __syncwarp();
@@ -516,7 +540,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         epilogue_store_bf16<BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * BN,
                                 smem + STAGES * L::STAGE_BYTES + L::BAR_BYTES + q * EPI_STAGE_WARP,
                                 reinterpret_cast<__nv_bfloat16*>(p.C) + gbase, p.ldc, c.m0 + q * 32, c.m_limit, c.n0, p.N,
-                                p.alpha, bias);
+                                p.alpha, bias, p.res, p.ldr);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

@@ -208,7 +208,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       if (!p.c_fp32 && !p.accumulate && vec_ok && p.N % 8 == 0) {
         epilogue_store_bf16<PAIR_BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * PAIR_BN,
                                      smem + STAGES * PAIR_STAGE_BYTES + 1024 + q * EPI_STAGE_WARP,
-                                     reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, row - lane, p.M, n0, p.N, p.alpha, bias);
+                                     reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, row - lane, p.M, n0, p.N, p.alpha, bias, p.res, p.ldr);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(acc ? tempty_leader1 : tempty_leader0);

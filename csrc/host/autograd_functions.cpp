@@ -120,21 +120,30 @@ std::vector<int64_t> with_last(const Tensor& x, ll n) {
   return shape;
 }
 Tensor like_input(const Tensor& dx, const std::vector<int64_t>& shape) { return dx.dim() == 2 && shape.size() == 2 ? dx : dx.view(shape); }
-Tensor product(const Tensor& x2, const Tensor& weight, const Tensor& bias, const Tensor& x) {   // in x's leading shape
+// x2 . weight^T (+ bias) (+ residual) in x's leading shape; a residual has that shape too
+Tensor product(const Tensor& x2, const Tensor& weight, const Tensor& bias, const Tensor& x, const Tensor& residual = {}) {
   const Tensor y = at::empty(with_last(x, weight.size(0)), x.options());
+  if (!residual.defined()) {
+    gemm(NT, x2, weight, bias, y);
+    return y;
+  }
+  require(residual.sizes() == y.sizes(), "residual of another shape");
+  const Tensor r2 = residual.dim() == 2 ? residual : residual.reshape({-1, residual.size(-1)});
+  if (gemm_residual(x2, weight, bias, r2, y)) return y;
   gemm(NT, x2, weight, bias, y);
-  return y;
+  return residual.add(y);
 }
 
 // ------------------------------------------------------------------------------------------------ linear
 struct LinearNode : OpNode {
-  bool need_dx, need_dw, bias;
+  bool need_dx, need_dw, bias, residual;
   std::vector<int64_t> shape;
   std::string name() const override { return "McbLinearBackward"; }
   variable_list grads(variable_list& g) override {
     const Tensor x2 = get(0), w = get(1);
     const Tensor dy2 = rows_of(g[0], w.size(0));
-    variable_list r(3);
+    variable_list r(4);
+    if (residual) r[3] = g[0];
     if (need_dx) r[0] = gemm(NN, dy2, w).view(shape);
     if (need_dw) r[1] = weight_grad(w, dy2, x2);
     if (bias) r[2] = dy2.to(at::kFloat).sum(0).to(g[0].scalar_type());
@@ -142,22 +151,24 @@ struct LinearNode : OpNode {
   }
 };
 
-PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {   // x, weight, bias, skip the weight's gradient -> y
-  MCB_BEGIN(4)
+// x, weight, bias, skip the weight's gradient, residual -> y
+PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  MCB_BEGIN(5)
   const Tensor &x = tensor(a[0]), &w = tensor(a[1]);
-  const Tensor bias = optional(a[2]);
-  const bool grad = wants_gradient({x, w, bias});
+  const Tensor bias = optional(a[2]), residual = optional(a[4]);
+  const bool grad = wants_gradient({x, w, bias, residual});
   Tensor y, x2;
   {
     at::NoGradGuard none;
     x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
-    y = product(x2, w, bias, x);
+    y = product(x2, w, bias, x, residual);
   }
   if (grad) {
-    auto node = make_node<LinearNode>({x, w, bias});
+    auto node = make_node<LinearNode>({x, w, bias, residual});
     node->need_dx = x.requires_grad();
     node->need_dw = w.requires_grad() && !truth(a[3]);
     node->bias = bias.defined();
+    node->residual = residual.defined();
     node->shape = x.sizes().vec();
     node->save({x2, w});
     torch::autograd::set_history(y, node);
@@ -175,7 +186,7 @@ struct NormNode : OpNode {
   variable_list grads(variable_list& g) override {
     const Tensor x2 = get(0), w = get(1), rstd = get(2);
     Tensor dx, dw;
-    norm_bwd(g[0].reshape({x2.size(0), x2.size(1)}).contiguous(), x2, w, rstd, eps, zc, false, need_dw, dx, dw);
+    norm_bwd(g[0].reshape({x2.size(0), x2.size(1)}).contiguous(), x2, w, rstd, eps, zc, false, need_dw, {}, dx, dw);
     return {like_input(dx, shape), dw};
   }
 };
@@ -212,15 +223,19 @@ struct NormLinearNode : OpNode {
   std::string name() const override { return "McbNormLinearBackward"; }
   variable_list grads(variable_list& g) override {
     const Tensor x2 = get(0), ln_w = get(1), rstd = get(2), w = get(3);
+    if (!g[0].defined()) return {g[1], {}, {}};
     const Tensor dy2 = rows_of(g[0], w.size(0)), dxn = gemm(NN, dy2, w);
+    const Tensor dkept = g.size() > 1 && g[1].defined() ? g[1].reshape({x2.size(0), x2.size(1)}).contiguous() : Tensor();
     Tensor dx, dlw;
-    norm_bwd(dxn, x2, ln_w, rstd, eps, zc, need_dw, true, dx, dlw);   // dxn becomes the normalised input
+    norm_bwd(dxn, x2, ln_w, rstd, eps, zc, need_dw, true, dkept, dx, dlw);   // dxn becomes the normalised input
     return {like_input(dx, shape), dlw, need_dw ? weight_grad(w, dy2, dxn) : Tensor()};
   }
 };
 
-PyObject* norm_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {   // x, norm weight, weight, eps, zc -> y
-  MCB_BEGIN(5)
+// x, norm weight, weight, eps, zc, keep -> y, or with `keep` y and x again: what uses x from there sends its gradient through this
+// node, whose kernel adds it to the norm's
+PyObject* norm_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  MCB_BEGIN(6)
   const Tensor &x = tensor(a[0]), &ln_w = tensor(a[1]), &w = tensor(a[2]);
   const float eps = real(a[3]);
   const bool zc = truth(a[4]), grad = wants_gradient({x, ln_w, w});
@@ -240,15 +255,24 @@ PyObject* norm_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {   // x, nor
     node->shape = x.sizes().vec();
     node->save({x2, ln_w, rstd, w});
     torch::autograd::set_history(y, node);
+    if (truth(a[5])) {
+      Tensor kept;
+      {
+        at::AutoDispatchBelowADInplaceOrView plain;
+        kept = x.detach();
+      }
+      torch::autograd::set_history(kept, node);
+      return tuple({y, kept});
+    }
   }
-  return THPVariable_Wrap(y);
+  return truth(a[5]) ? tuple({y, x}) : THPVariable_Wrap(y);
   MCB_END
 }
 
 // ------------------------------------------------------------------------------------------------ gated activation + linear
 struct GluLinearNode : OpNode {
   GluArgs args;
-  bool need_dw;
+  bool need_dw, residual;
   std::vector<int64_t> shape;
   std::string name() const override { return "McbGluLinearBackward"; }
   variable_list grads(variable_list& g) override {
@@ -256,25 +280,27 @@ struct GluLinearNode : OpNode {
     const Tensor dy2 = rows_of(g[0], w.size(0)), da = gemm(NN, dy2, w);
     Tensor none;
     const Tensor dh = glu_rows_bwd(da, h2, {}, args, need_dw, none);  // da becomes the activation
-    return {like_input(dh, shape), need_dw ? weight_grad(w, dy2, da) : Tensor()};
+    return {like_input(dh, shape), need_dw ? weight_grad(w, dy2, da) : Tensor(), residual ? g[0] : Tensor()};
   }
 };
 
-PyObject* glu_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {   // h, weight, kind, clamp, offset -> y
-  MCB_BEGIN(5)
+PyObject* glu_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {   // h, weight, kind, clamp, offset, residual -> y
+  MCB_BEGIN(6)
   const Tensor &h = tensor(a[0]), &w = tensor(a[1]);
+  const Tensor residual = optional(a[5]);
   const GluArgs args{static_cast<int>(integer(a[2])), real(a[3]), real(a[4])};
-  const bool grad = wants_gradient({h, w});
+  const bool grad = wants_gradient({h, w, residual});
   Tensor y, h2;
   {
     at::NoGradGuard none;
     h2 = rows_of(h, h.size(-1));
-    y = product(glu_rows_fwd(h2, {}, args), w, {}, h);
+    y = product(glu_rows_fwd(h2, {}, args), w, {}, h, residual);
   }
   if (grad) {
-    auto node = make_node<GluLinearNode>({h, w});
+    auto node = make_node<GluLinearNode>({h, w, residual});
     node->args = args;
     node->need_dw = w.requires_grad();
+    node->residual = residual.defined();
     node->shape = h.sizes().vec();
     node->save({h2, w});
     torch::autograd::set_history(y, node);

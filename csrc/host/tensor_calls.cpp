@@ -145,6 +145,25 @@ Tensor gemm(int layout, const Tensor& a_, const Tensor& b_, const Tensor& bias_,
   return c;
 }
 
+bool gemm_residual(const Tensor& a_, const Tensor& b_, const Tensor& bias_, const Tensor& res, const Tensor& y) {
+  const ll M = a_.size(0), K = a_.size(1), N = b_.size(0);
+  auto aligned = [](const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
+  if (M == 0 || K == 0 || N % 8 || res.dim() != 2 || res.scalar_type() != at::kBFloat16 || res.stride(1) != 1 || res.stride(0) % 8 ||
+      !aligned(res) || !aligned(y))
+    return false;
+  const Tensor a = tma_rows(a_), b = tma_rows(b_);
+  operand(a, at::kBFloat16, M * K, a, "GEMM operands: bf16 on one device");
+  operand(b, at::kBFloat16, N * K, a, "GEMM operands: bf16 on one device");
+  require(b.size(1) == K, "GEMM operands whose contraction sizes differ");
+  require(res.size(0) == M && res.size(1) == N && res.device() == a.device(), "residual of another shape");
+  require(!bias_.defined() || (bias_.numel() == N && bias_.device() == a.device()), "GEMM bias: one for every column");
+  Tensor bias = bias_;
+  if (bias.defined()) bias = bias.to(at::kBFloat16).contiguous();
+  launch("mcb_gemm_bf16_residual", mcb_gemm_bf16_residual, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), y.data_ptr(), N,
+         res.data_ptr(), res.stride(0), M, N, K, ptr(bias), status_of(a), stream());
+  return true;
+}
+
 void norm_fwd(const Tensor& x2, const Tensor& w, float eps, bool zc, const Tensor& y, Tensor& rstd) {
   const ll rows = x2.size(0), H = x2.size(1);
   operand(x2, at::kBFloat16, 0, x2, "norm input: bf16");
@@ -155,11 +174,13 @@ void norm_fwd(const Tensor& x2, const Tensor& w, float eps, bool zc, const Tenso
 }
 
 void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor& rstd, float eps, bool zc, bool over,
-              bool need_dw, Tensor& dx, Tensor& dw) {
+              bool need_dw, const Tensor& dres_, Tensor& dx, Tensor& dw) {
   const ll rows = x2.size(0), H = x2.size(1);
+  const Tensor dres = H <= 8192 ? dres_ : Tensor();   // a wider row's kernel has no registers for it
   operand(dy, at::kBFloat16, rows * H, x2, "norm gradient: bf16 of the input's size");
   operand(w, at::kBFloat16, H, x2, "norm weight: bf16, one for every column");
   operand(rstd, at::kFloat, rows, x2, "norm: an fp32 for every row");
+  operand(dres, at::kBFloat16, rows * H, x2, "gradient of the residual: bf16 of the input's size");
   dx = at::empty({rows, H}, x2.options());
   Tensor part;
   if (need_dw) {
@@ -167,11 +188,12 @@ void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor&
     part = at::empty({mcb_rmsnorm_bwd_partial_rows(rows, static_cast<int>(H)), H}, x2.options().dtype(at::kFloat));
   }
   if (over)
-    launch("mcb_rmsnorm_bwd_det", mcb_rmsnorm_bwd_det_y, dy.data_ptr(), x2.data_ptr(), w.data_ptr(), rstd.data_ptr(), nullptr,
+    launch("mcb_rmsnorm_bwd_det", mcb_rmsnorm_bwd_det_y, dy.data_ptr(), x2.data_ptr(), w.data_ptr(), rstd.data_ptr(), ptr(dres),
            dx.data_ptr(), ptr(dw), need_dw, ptr(part), rows, H, x2.stride(0), eps, zc, stream());
   else
-    launch("mcb_rmsnorm_bwd_det", mcb_rmsnorm_bwd_det, dy.data_ptr(), x2.data_ptr(), w.data_ptr(), rstd.data_ptr(), nullptr,
+    launch("mcb_rmsnorm_bwd_det", mcb_rmsnorm_bwd_det, dy.data_ptr(), x2.data_ptr(), w.data_ptr(), rstd.data_ptr(), ptr(dres),
            dx.data_ptr(), ptr(dw), need_dw, ptr(part), rows, H, x2.stride(0), eps, zc, stream());
+  if (dres_.defined() && !dres.defined()) dx = dx.add(dres_);
 }
 
 // How many CTAs share one (key tile, kv head) pair in the dK/dV kernel: the smallest divisor of the GQA ratio that puts about three
@@ -346,7 +368,7 @@ PyObject* rmsnorm_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {       // dy
   const Tensor& x2 = tensor(a[1]);
   const Tensor dy = tensor(a[0]).reshape({x2.size(0), x2.size(1)}).contiguous();
   Tensor dx, dw;
-  norm_bwd(dy, x2, tensor(a[2]), tensor(a[3]), real(a[4]), truth(a[5]), false, truth(a[6]), dx, dw);
+  norm_bwd(dy, x2, tensor(a[2]), tensor(a[3]), real(a[4]), truth(a[5]), false, truth(a[6]), {}, dx, dw);
   return tuple({dx, dw});
   MCB_END
 }
@@ -367,7 +389,7 @@ PyObject* norm_linear_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor &x2 = tensor(a[1]), &w = tensor(a[4]);
   const Tensor dy2 = rows_of(tensor(a[0]), w.size(0)), dxn = gemm(NN, dy2, w);
   Tensor dx, dlw;
-  norm_bwd(dxn, x2, tensor(a[2]), tensor(a[3]), real(a[5]), truth(a[6]), truth(a[7]), true, dx, dlw);
+  norm_bwd(dxn, x2, tensor(a[2]), tensor(a[3]), real(a[5]), truth(a[6]), truth(a[7]), true, {}, dx, dlw);
   return tuple({dx, dlw, dy2, truth(a[7]) ? dxn : Tensor()});
   MCB_END
 }

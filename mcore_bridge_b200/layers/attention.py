@@ -123,10 +123,15 @@ class SelfAttention(nn.Module):
         self.use_rope = use_rope and config.position_embedding_type in ('rope', 'mrope')
         self.rope_key = rope_key
 
-    def forward(self, x: torch.Tensor, ctx: ForwardContext) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, ctx: ForwardContext, residual: bool = False) -> torch.Tensor:
+        """``residual``: ``x`` is added to the result."""
         cfg = self.config
+        lin = self.linear_qkv
         with nvtx_range('qkv'):
-            qkv = self.linear_qkv(x)                              # [T, local packed qkv]
+            if residual and isinstance(lin, LayerNormColumnParallelLinear):
+                qkv, x = lin.with_input(x)                        # [T, local packed qkv]
+            else:
+                qkv = lin(x)
         qpg = self.qpg
         if self.kv_rep > 1:
             from ..parallel import mappings as M
@@ -170,4 +175,7 @@ class SelfAttention(nn.Module):
         if gate is not None:
             o = o * torch.sigmoid(gate.reshape(o.shape[0], -1).float()).to(o.dtype)
         with nvtx_range('linear_proj'):
-            return self.linear_proj(o)
+            proj = self.linear_proj
+            if not residual:
+                return proj(o)
+            return proj.add_to(x, o) if isinstance(proj, RowParallelLinear) else x + proj(o)

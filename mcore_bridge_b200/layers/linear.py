@@ -26,6 +26,12 @@ def _set_tp_attrs(p: nn.Parameter, is_parallel: bool, dim: int, is_expert: bool 
     p.is_expert = is_expert
 
 
+def is_plain(module: nn.Module, cls) -> bool:
+    """A module whose call is its class's ``forward`` and nothing else: what a caller may fuse into another operation."""
+    return (type(module) is cls and 'forward' not in module.__dict__
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks))
+
+
 class _LinearBase(nn.Module):
 
     def _group(self, is_expert: bool) -> str:
@@ -120,6 +126,16 @@ class LayerNormColumnParallelLinear(ColumnParallelLinear):
         if self._lean(x):
             from ..ops import fused_mlp
             return fused_mlp.norm_linear(x, self.layer_norm_weight, self.weight, self.eps, self.zero_centered)
+        return self._unfused(x)
+
+    def with_input(self, x):
+        """``(self(x), x)``, ``x`` in a form whose gradient joins the norm's inside its backward kernel where that is possible."""
+        if is_plain(self, LayerNormColumnParallelLinear) and self._lean(x):
+            from ..ops import fused_mlp
+            return fused_mlp.norm_linear(x, self.layer_norm_weight, self.weight, self.eps, self.zero_centered, True)
+        return self(x), x
+
+    def _unfused(self, x):
         xn = self.norm(x)
         y = linear(xn, self.weight, self.bias, self.spec)
         if self.return_layernorm_output:
@@ -158,6 +174,12 @@ class RowParallelLinear(_LinearBase):
 
     def forward(self, x):
         return linear(x, self.weight, self.bias, self.spec)
+
+    def add_to(self, residual, x):
+        """``residual + self(x)``"""
+        if is_plain(self, RowParallelLinear):
+            return linear(x, self.weight, self.bias, self.spec, residual)
+        return residual + self(x)
 
     def extra_repr(self):
         return (f'in={self.input_size_per_partition} (of {self.input_size}), out={self.output_size}, '

@@ -25,10 +25,14 @@ class MLP(nn.Module):
                     prm.partition_stride = 2
         self.kind = 'swiglu' if config.swiglu else ('quick_geglu' if config.quick_geglu else 'geglu_tanh')
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, residual: bool = False) -> torch.Tensor:
+        """``residual``: ``x`` is added to the result."""
         cfg = self.config
-        h = self.linear_fc1(x)
-        fc2 = self.linear_fc2
+        fc1, fc2 = self.linear_fc1, self.linear_fc2
+        if residual and isinstance(fc1, LayerNormColumnParallelLinear):
+            h, x = fc1.with_input(x)
+        else:
+            h = fc1(x)
         # the fused block does not call fc2 as a module: with hooks on it, which want its input or output, it is called
         if cfg.gated_linear_unit and type(fc2) is RowParallelLinear and fc2.bias is None and not fc2.spec.fp8 \
                 and getattr(cfg, 'lean_activations', True) and not (fc2._forward_hooks or fc2._forward_pre_hooks):
@@ -37,9 +41,11 @@ class MLP(nn.Module):
             if ps.get_world_size(fc2.group) == 1 and fused_mlp.usable(h, fc2.weight) and (h.shape[-1] // 2) % 8 == 0:
                 from ..ops.activation import KINDS
                 return fused_mlp.glu_linear(h, fc2.weight, KINDS[self.kind], cfg.activation_func_clamp_value or 0.0,
-                                            cfg.glu_linear_offset)
+                                            cfg.glu_linear_offset, x if residual else None)
         if cfg.gated_linear_unit:
             h = glu(h, self.kind, None, cfg.activation_func_clamp_value or 0.0, cfg.glu_linear_offset)
         else:
             h = cfg.activation_func(h)
-        return self.linear_fc2(h)
+        if not residual:
+            return fc2(h)
+        return fc2.add_to(x, h) if isinstance(fc2, RowParallelLinear) else x + fc2(h)

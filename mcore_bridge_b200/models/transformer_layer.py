@@ -20,6 +20,7 @@ from torch import nn
 
 from ..layers.attention import SelfAttention
 from ..layers.context import ForwardContext
+from ..layers.linear import is_plain
 from ..layers.mlp import MLP
 from ..layers.moe import MoELayer
 from ..layers.norm import Norm
@@ -86,6 +87,9 @@ class TransformerLayer(nn.Module):
             hidden, post, res = hc.pre(streams)
         x = hidden if self.input_layernorm is None else self.input_layernorm(hidden)
         with nvtx_range('attention'):
+            if hc is None and self.input_layernorm is None and not self.config.post_sublayer_layernorm \
+                    and is_plain(self.self_attention, SelfAttention):
+                return self.self_attention(x, ctx, True)         # the residual is added where the projection is formed
             out = self.self_attention(x, ctx)
         if self.config.post_sublayer_layernorm:
             out = self.self_attention.post_self_attn_layernorm(out)
@@ -103,6 +107,8 @@ class TransformerLayer(nn.Module):
         with nvtx_range('moe' if self.is_moe else 'mlp'):
             if self.is_moe:
                 out = self.mlp(x, ctx.padding_mask, ctx.seg_ids, ctx.num_seqs, ctx.input_ids)
+            elif hc is None and self.pre_mlp_layernorm is None and not cfg.post_sublayer_layernorm and is_plain(self.mlp, MLP):
+                return self.mlp(x, True)
             else:
                 out = self.mlp(x)
         if cfg.post_sublayer_layernorm:

@@ -21,9 +21,12 @@ def usable(x: torch.Tensor, weight: torch.Tensor) -> bool:
             and x.shape[-1] % 8 == 0)
 
 
-def norm_linear(x, ln_w, weight, eps, zero_centered):
-    return _lib.native().norm_linear(x, ln_w, weight, eps, zero_centered)
+def norm_linear(x, ln_w, weight, eps, zero_centered, keep: bool = False):
+    """With ``keep`` returns ``x`` as well: a residual taken from there has its gradient added to the norm's by the norm's
+    backward kernel."""
+    return _lib.native().norm_linear(x, ln_w, weight, eps, zero_centered, keep)
 
 
-def glu_linear(h, weight, kind: int, clamp: float, offset: float):
-    return _lib.native().glu_linear(h, weight, kind, clamp or 0.0, offset)
+def glu_linear(h, weight, kind: int, clamp: float, offset: float, residual=None):
+    """``residual`` (of the result's shape) is added in the product's epilogue."""
+    return _lib.native().glu_linear(h, weight, kind, clamp or 0.0, offset, residual)

@@ -183,11 +183,14 @@ def _single_rank(x, weight, bias, spec: LinearSpec):
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
-           spec: LinearSpec = LinearSpec()) -> torch.Tensor:
+           spec: LinearSpec = LinearSpec(), residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``residual`` (of the result's shape) is added to the result."""
     if weight.dtype != x.dtype:
         x = x.to(weight.dtype)
     nat = _single_rank(x, weight, bias, spec)
-    y = _LinearFn.apply(x, weight, bias, spec) if nat is None else nat.linear(x, weight, bias, spec.skip_weight_grad)
+    if nat is not None and (residual is None or (residual.is_cuda and residual.dtype == x.dtype)):
+        return nat.linear(x, weight, bias, spec.skip_weight_grad, residual)
+    y = _LinearFn.apply(x, weight, bias, spec)
     if spec.mode == 'column' and spec.gather_output:
         y = M.gather_from_tensor_model_parallel_region(y, spec.group)
-    return y
+    return y if residual is None else residual + y

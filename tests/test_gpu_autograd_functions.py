@@ -122,3 +122,55 @@ def test_outputs_nobody_uses():
     assert gate is None
     dx = torch.autograd.grad(k, x, torch.ones_like(k))[0].view(70, 2, 4, 64)
     assert (dx[:, :, 2] == 1).all() and (dx[:, :, :2] == 0).all() and (dx[:, :, 3] == 0).all()
+
+
+@pytest.mark.parametrize('shape,n,k', [((70,), 96, 64), ((2, 35), 104, 64), ((300,), 512, 128), ((1, 129), 264, 72)])
+def test_residuals_are_added_as_by_an_addition(shape, n, k):
+    """The same bits as a sum of its own, in the product's epilogue (also where the kernel does not take the residual: 104 columns,
+    off their boundary) and in the norm's backward pass."""
+    from mcore_bridge_b200.ops import fused_mlp
+    from mcore_bridge_b200.ops.linear import linear
+    x, h, w, v, ln = (_rand(*s, seed=i) for i, s in enumerate([(*shape, k), (*shape, 2 * k), (n, k), (k, k), (k,)]))
+    bias, res = _rand(n, seed=7), _rand(*shape, n, seed=8) if n != 104 else _rand(*shape, n + 1, seed=8)[..., 1:]
+    dy = _rand(*shape, n, seed=9)
+    for first, fused, apart in [
+            (x, lambda x, w, b, r: linear(x, w, b, residual=r), lambda x, w, b, r: r + linear(x, w, b)),
+            (h, lambda h, w, b, r: fused_mlp.glu_linear(h, w, 0, 0.0, 0.0, r),
+             lambda h, w, b, r: r + fused_mlp.glu_linear(h, w, 0, 0.0, 0.0))]:
+        leaves = [t.detach().requires_grad_() for t in (first, w, bias, res)]
+        a, b = fused(*leaves), apart(*leaves)
+        assert torch.equal(a, b)
+        for g, e in zip(torch.autograd.grad(a, leaves, dy, allow_unused=True), torch.autograd.grad(b, leaves, dy, allow_unused=True)):
+            assert (g is None and e is None) or torch.equal(g, e)
+        with torch.no_grad():
+            assert torch.equal(fused(*leaves), a)
+
+    leaves = [t.clone().requires_grad_() for t in (x, ln, v)]
+    dk = _rand(*shape, k, seed=10)
+
+    def block(keep):
+        if keep:
+            y, kept = fused_mlp.norm_linear(*leaves, 1e-6, False, True)
+        else:
+            y, kept = fused_mlp.norm_linear(*leaves, 1e-6, False), leaves[0]
+        return y, kept
+
+    y, kept = block(True)
+    assert torch.equal(kept, x) and torch.equal(y, block(False)[0])
+    got = torch.autograd.grad(block(True), leaves, [dk, dk])
+    want = torch.autograd.grad(block(False), leaves, [dk, dk])
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    assert torch.equal(torch.autograd.grad(block(True)[1], leaves[0], dk)[0], dk)     # the residual alone
+    assert torch.equal(torch.autograd.grad(block(True)[0], leaves[0], dk)[0], torch.autograd.grad(block(False)[0], leaves[0], dk)[0])
+
+
+def test_residual_of_a_wide_row():
+    """More columns than the norm's backward kernel has registers for: the gradients are added behind it."""
+    from mcore_bridge_b200.ops import fused_mlp
+    x, ln, v = _rand(5, 8200, seed=1), _rand(8200, seed=2), _rand(64, 8200, seed=3, scale=0.01)
+    leaves = [t.requires_grad_() for t in (x, ln, v)]
+    dy, dk = _rand(5, 64, seed=4), _rand(5, 8200, seed=5)
+    got = torch.autograd.grad(fused_mlp.norm_linear(*leaves, 1e-6, False, True), leaves, [dy, dk])
+    want = torch.autograd.grad(fused_mlp.norm_linear(*leaves, 1e-6, False), leaves, dy)
+    assert torch.equal(got[0], want[0] + dk) and torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
