@@ -481,6 +481,51 @@ PyObject* attn_window_starts(PyObject*, PyObject* const* a, Py_ssize_t n) {   //
   MCB_END
 }
 
+PyObject* seq_starts(PyObject*, PyObject* const* a, Py_ssize_t n) {          // boundaries, tokens -> first token of each one's sequence
+  MCB_BEGIN(2)
+  const Tensor cu = tensor(a[0]).contiguous();
+  const ll T = integer(a[1]);
+  require(cu.scalar_type() == at::kInt || cu.scalar_type() == at::kLong, "sequence boundaries: int32 or int64");
+  const Tensor out = at::empty({T}, cu.options().dtype(at::kInt));
+  launch("mcb_seq_starts", mcb_seq_starts, cu.data_ptr(), cu.scalar_type() == at::kLong, cu.numel(), out.data_ptr(), T, stream());
+  return THPVariable_Wrap(out);
+  MCB_END
+}
+
+PyObject* rope_tables(PyObject*, PyObject* const* a, Py_ssize_t n) {         // positions, inverse frequencies, scale -> cos, sin
+  MCB_BEGIN(3)
+  const Tensor pos = tensor(a[0]).contiguous(), inv = tensor(a[1]).contiguous();
+  require(pos.scalar_type() == at::kInt || pos.scalar_type() == at::kLong, "positions: int32 or int64");
+  operand(inv, at::kFloat, 0, pos, "inverse frequencies: fp32 on the positions' device");
+  const ll T = pos.numel(), R = inv.numel();
+  const Tensor cos = at::empty({T, R}, inv.options()), sin = at::empty({T, R}, inv.options());
+  launch("mcb_rope_tables", mcb_rope_tables, pos.data_ptr(), pos.scalar_type() == at::kLong, inv.data_ptr(), real(a[2]),
+         cos.data_ptr(), sin.data_ptr(), T, R, stream());
+  return tuple({cos, sin});
+  MCB_END
+}
+
+PyObject* ce_combine(PyObject*, PyObject* const* a, Py_ssize_t n) {          // statistics of every row's tiles -> max, sum
+  MCB_BEGIN(1)
+  const Tensor& part = tensor(a[0]);
+  require(part.dim() == 3 && part.size(2) == 2 && part.scalar_type() == at::kFloat && part.is_contiguous(),
+          "statistics: fp32 pairs of every tile of every row");
+  const Tensor m = at::empty({part.size(0)}, part.options()), s = at::empty({part.size(0)}, part.options());
+  launch("mcb_ce_combine", mcb_ce_combine, part.data_ptr(), m.data_ptr(), s.data_ptr(), part.size(0), part.size(1), stream());
+  return tuple({m, s});
+  MCB_END
+}
+
+PyObject* ce_loss(PyObject*, PyObject* const* a, Py_ssize_t n) {             // max, sum, label logits -> log-sum-exp, loss
+  MCB_BEGIN(3)
+  const Tensor m = tensor(a[0]).contiguous(), s = tensor(a[1]).contiguous(), tgt = tensor(a[2]).contiguous();
+  for (const Tensor& t : {m, s, tgt}) operand(t, at::kFloat, m.numel(), m, "statistics: an fp32 for every row");
+  const Tensor lse = at::empty_like(m), loss = at::empty_like(m);
+  launch("mcb_ce_loss", mcb_ce_loss, m.data_ptr(), s.data_ptr(), tgt.data_ptr(), lse.data_ptr(), loss.data_ptr(), m.numel(), stream());
+  return tuple({lse, loss});
+  MCB_END
+}
+
 PyObject* attn_dkv_splits(PyObject*, PyObject* const* a, Py_ssize_t n) {      // keys, query heads, kv heads
   MCB_BEGIN(3)
   return PyLong_FromLong(dkv_splits(integer(a[0]), static_cast<int>(integer(a[1])), static_cast<int>(integer(a[2]))));
@@ -551,6 +596,10 @@ PyMethodDef methods[] = {MCB_FAST(init),
                          MCB_FAST(attn_bwd),
                          MCB_FAST(attn_window_starts),
                          MCB_FAST(attn_dkv_splits),
+                         MCB_FAST(seq_starts),
+                         MCB_FAST(rope_tables),
+                         MCB_FAST(ce_combine),
+                         MCB_FAST(ce_loss),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_mcb200_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

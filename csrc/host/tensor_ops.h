@@ -45,6 +45,10 @@ typedef long long ll;
                                float, float*, int, int*, void*))                                                        \
   X(mcb_attn_sink_grad, int, (const float*, const float*, const float*, void*, int, int, int, void*))                   \
   X(mcb_attn_window_starts, int, (const int*, int*, int, int, void*))                                                   \
+  X(mcb_seq_starts, int, (const void*, int, int, int*, ll, void*))                                                      \
+  X(mcb_rope_tables, int, (const void*, int, const float*, float, float*, float*, ll, int, void*))                      \
+  X(mcb_ce_combine, int, (const float*, float*, float*, ll, int, void*))                                                \
+  X(mcb_ce_loss, int, (const float*, const float*, const float*, float*, float*, ll, void*))                            \
   X(mcb_sm_count, int, ())
 
 #define MCB_EXTERN(name, ret, args) extern ret(*name) args;

@@ -15,6 +15,8 @@ from typing import Optional, Tuple
 
 import torch
 
+from ..ops import _lib
+
 
 def _rope_type(rope_scaling: Optional[dict]) -> str:
     if not rope_scaling:
@@ -190,6 +192,9 @@ class RotaryEmbedding(torch.nn.Module):
         else:
             if position_ids.dim() == 2:
                 position_ids = position_ids[0]
+            if position_ids.is_cuda and inv.device == position_ids.device and position_ids.dtype in (torch.int32, torch.int64) \
+                    and position_ids.dim() == 1 and _lib.cuda_enabled():
+                return _lib.native().rope_tables(position_ids, inv, self.attention_scaling)
             freqs = position_ids.float()[:, None] * inv[None, :]
         cos, sin = freqs.cos(), freqs.sin()
         if self.attention_scaling != 1.0:

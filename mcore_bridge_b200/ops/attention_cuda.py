@@ -44,6 +44,9 @@ def seq_start_from_cu(cu_seqlens: Optional[torch.Tensor], T: int, device) -> tor
     """``[T]`` int32: index of the first token of the packed sequence each token belongs to."""
     if cu_seqlens is None:
         return torch.zeros(T, dtype=torch.int32, device=device)
+    if cu_seqlens.is_cuda and cu_seqlens.device == torch.device(device) and cu_seqlens.numel() >= 2 \
+            and cu_seqlens.dtype in (torch.int32, torch.int64) and cu_seqlens.dim() == 1 and _lib.cuda_enabled():
+        return _lib.native().seq_starts(cu_seqlens, T)
     cu = cu_seqlens.to(device=device, dtype=torch.int64)
     seg = torch.searchsorted(cu[1:].contiguous(), torch.arange(T, device=device), right=True)
     return cu[:-1][seg.clamp(max=cu.numel() - 2)].to(torch.int32)

@@ -233,10 +233,7 @@ def _head_stats(h2, weight, lab, vocab_start, logits=None):
                                      None, None, _lib.ptr(logits), _ll(vl), _int(0),
                                      _lib.ptr(_lib.status_word(h2.device)), _lib.stream_ptr())
     _lib.check_rc(rc, 'mcb_gemm_ce_bf16')
-    m_t, s_t = part[..., 0], part[..., 1]
-    m = m_t.max(dim=1).values
-    s = (s_t * torch.exp(m_t - m[:, None])).sum(1)
-    return m, s, tgt
+    return *_lib.native().ce_combine(part), tgt
 
 
 def _head_dlogits(h2, weight, lab, vocab_start, lse, g):
@@ -306,10 +303,14 @@ class _FusedLinearCE(torch.autograd.Function):
             if logits is not None:
                 ctx.kept = _Kept(logits)
             m, s, tgt = _head_stats(h2, weight, lab, r * vl, logits)
-            lse_all, tgt = _combine(m, s, tgt, group_name, group)
+            if group is None and m.is_cuda:
+                lse_all, loss = _lib.native().ce_loss(m, s, tgt)
+            else:
+                lse_all, tgt = _combine(m, s, tgt, group_name, group)
+                loss = lse_all - tgt
             ctx.save_for_backward(h2, weight, lab, lse_all)
             ctx.meta = (group_name, chunk, r * vl, h.shape, labels.shape)
-            return (lse_all - tgt).view(labels.shape)
+            return loss.view(labels.shape)
         loss = torch.empty(T, dtype=torch.float32, device=h.device)
         lse_all = torch.empty(T, dtype=torch.float32, device=h.device)
         ldt = torch.float32
