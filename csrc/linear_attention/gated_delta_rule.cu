@@ -33,12 +33,16 @@
 // as far off as those of an fp32 torch evaluation (0.0017, their own rounding), dg and dbeta by 1.4e-7 .. 5.4e-7, torch by
 // 2.8e-7 .. 3.8e-5.  Two terms throughout and decays from an fp32 sum gave 4.5e-6 .. 7.8e-5.
 //
-// In the scans a warp owns 16 columns of v and keeps S^T (16 x d) in its accumulators: the accumulators of every product
-// are the first operand of the next one, so the warps of a CTA share the loaded tiles and never exchange values.  Bound:
-// the chain of MMAs per chunk (forward about 500, backward 900 and 800); the next chunk's tiles are copied meanwhile.
-// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.27 ms (prep 0.09, scan 0.17), backward 1.04 ms (scan
-// 0.30, scan_bwd 0.36, grad 0.39); with two terms throughout they took 0.22 and 0.72.  The batched torch evaluation of the
-// rule was most of a 29.5 ms block.
+// In the scans four warps own 16 columns of v, with S^T (16 x d) in their accumulators: the accumulators of every product are the
+// first operand of the next one.  Bound: the latency of what a chunk does one after the other (a warp issues every tenth cycle, the
+// MMAs, forward about 500 a strip, backward 900 and 800, take 40 to 48 % of the time); the next chunk's tiles are copied
+// meanwhile.  With one warp for a strip, which passes nothing on and forms every term itself, us, before / now, scan, the
+// backward pass's scan and scan_bwd: 4096 tokens in three sequences, 32 heads of 128 171, 297, 358 / 147, 239, 263; in 64
+// sequences 176, 308, 431 / 173, 285, 317; 8192 in one, 16 heads 636, 1120, 1338 / 562, 910, 1007.  Two warps a strip: 173, 276,
+// 307 (of the first).  No change from starting the strips apart, slower with the operands of M and P fetched before the
+// strip's barrier (162, 335, 367: registers).
+// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.24 ms (prep 0.09), backward 0.88 ms (grad 0.38).  The batched
+// torch evaluation of the rule was most of a 29.5 ms block.
 #include "../common/host_utils.cuh"
 #include "warp_mma.cuh"
 
@@ -47,7 +51,8 @@ using namespace mcb;
 namespace {
 
 constexpr int C = 64;           // tokens of a chunk
-constexpr int THREADS = 128;    // 4 warps, 16 rows (tokens, or columns of v) each
+constexpr int THREADS = 128;    // 4 warps, 16 tokens each
+constexpr int ST = 512;         // scans: 4 strips of 16 columns of v, 4 warps each
 constexpr int CC = C * C;       // elements of a chunk's square matrices
 constexpr int SQ = CC * 2;      // bytes of one of their bf16 terms
 constexpr int MP = 3;           // terms kept of M and P
@@ -82,9 +87,6 @@ __device__ __forceinline__ ChunkPos locate(const GdrParams& p, ChunkPos* slot) {
 }
 
 // 64 x 64 bf16 matrix (contiguous) -> tile
-__device__ __forceinline__ void load_square(uint32_t tile, const __nv_bfloat16* src) {
-  for (int id = threadIdx.x; id < C * 8; id += THREADS) cp_async16(tile_addr<64>(tile, id >> 3, (id & 7) * 8), src + id * 8, 16);
-}
 // exp of a sum of two floats, the second far smaller
 __device__ __forceinline__ float exp_pair(float hi, float lo) {
   const float e = expf(hi);
@@ -221,30 +223,53 @@ gdr_prep_kernel(const GdrParams p) {
 }
 
 // ---------------------------------------------------------------------------------------------------- scans
-// shared-memory stage of a scan: k, q, 64-column slices of v and of do (X / Z), NT terms of M and P, the last rows of gb
+// Shared memory of a scan: two stages of k, q, 64-column slices of v and of do (X / Z), the last rows of gb and NT terms of M and P
+// (the ten 16 x 16 blocks on and below the diagonal); what the four warps of a strip pass on to each other.
+constexpr int SQB = 10 * 512;
 template <int D, int NT, bool WITH_DO>
 struct ScanSmem {
-  static constexpr int K = 0, Q = C * D * 2, X = 2 * C * D * 2, Z = X + SQ, M = Z + (WITH_DO ? SQ : 0);
-  static constexpr int P = M + NT * SQ, G = P + NT * SQ;
-  static constexpr int STAGE = G + 4 * C * 4;
-  static constexpr int TOTAL = 2 * STAGE + 128;
+  static constexpr int K = 0, Q = C * D * 2, X = 2 * C * D * 2, Z = X + SQ, G = Z + (WITH_DO ? SQ : 0);
+  static constexpr int M = G + 4 * C * 4, P = M + NT * SQB, STAGE = P + NT * SQB;
+  static constexpr int SHARE = 2 * STAGE;
+  static constexpr int PART = 4 * NT * 512, STRIP = 2 * PART;        // 16 x 64 as second operands; S^T takes both parts
+  static constexpr int BARS = SHARE + 4 * STRIP;
+  static constexpr int TOTAL = BARS + 64 + 128;
+  static_assert(D / 16 * NT * 512 <= 2 * PART && TOTAL + 64 <= 232448, "shared memory");
 };
 
+// 16 x 16 blocks of 512 bytes; the two halves of a row change places every four rows, so that eight rows of a half lie in
+// distinct banks
+__device__ __forceinline__ uint32_t block_addr(uint32_t tile, int bi, int bj, int r, int half) {
+  return tile + (bi * (bi + 1) / 2 + bj) * 512 + r * 32 + ((half ^ ((r >> 2) & 1)) << 4);
+}
+__device__ __forceinline__ void load_square(uint32_t tile, const __nv_bfloat16* src) {
+  for (int id = threadIdx.x; id < 320; id += ST) {
+    const int blk = id >> 5, bi = blk >= 6 ? 3 : blk >= 3 ? 2 : blk >= 1 ? 1 : 0, bj = blk - bi * (bi + 1) / 2, rr = (id >> 1) & 15, half = id & 1;
+    cp_async16(block_addr(tile, bi, bj, rr, half), src + (bi * 16 + rr) * C + bj * 16 + half * 8, 16);
+  }
+}
+
+// arrives when this thread's copies so far have landed
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+// by all threads; the mbarriers `full` (tiles) and full + 16 (M and P) have a count of ST
 template <int D, int NT, bool WITH_DO>
-__device__ __forceinline__ void load_stage(uint32_t st, const GdrParams& p, int t, int len, int h, int col0, long long ch) {
+__device__ __forceinline__ void load_stage(uint32_t st, uint32_t full, const GdrParams& p, int t, int len, int h, int col0, long long ch) {
   using L = ScanSmem<D, NT, WITH_DO>;
   const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
-  load_tile<D, C, THREADS>(st + L::K, p.k + off, stride, len);
-  load_tile<D, C, THREADS>(st + L::Q, p.q + off, stride, len);
-  load_tile<64, C, THREADS>(st + L::X, p.v + off + col0, stride, len);
-  if (WITH_DO) load_tile<64, C, THREADS>(st + L::Z, p.dout + off + col0, stride, len);
+  load_tile<D, C, ST>(st + L::K, p.k + off, stride, len);
+  load_tile<D, C, ST>(st + L::Q, p.q + off, stride, len);
+  load_tile<64, C, ST>(st + L::X, p.v + off + col0, stride, len);
+  if (WITH_DO) load_tile<64, C, ST>(st + L::Z, p.dout + off + col0, stride, len);
+  if (threadIdx.x < 64) cp_async16(st + L::G + threadIdx.x * 16, p.gb + (ch * G_ROWS + G_BETA) * C + threadIdx.x * 4, 16);
+  cp_async_arrive(full);
 #pragma unroll
   for (int m = 0; m < NT; ++m) {
-    load_square(st + L::M + m * SQ, p.mp + (ch * 2 * MP + m) * CC);
-    load_square(st + L::P + m * SQ, p.mp + (ch * 2 * MP + MP + m) * CC);
+    load_square(st + L::M + m * SQB, p.mp + (ch * 2 * MP + m) * CC);
+    load_square(st + L::P + m * SQB, p.mp + (ch * 2 * MP + MP + m) * CC);
   }
-  if (threadIdx.x < 64) cp_async16(st + L::G + threadIdx.x * 16, p.gb + (ch * G_ROWS + G_BETA) * C + threadIdx.x * 4, 16);
-  cp_async_commit();
+  cp_async_arrive(full + 16);
 }
 
 struct ScanPos {
@@ -328,306 +353,368 @@ __device__ __forceinline__ void join(float (&a)[N][4], const float (&b)[N][4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) a[n][e] += b[n][e];
 }
-// NT terms of two neighbouring 8-column blocks of a 64 x 64 matrix, as the B operand of X M^T (TRANS) or X M
+// NT terms of block (bi, bj) of M or P, as the B operand of X M^T (TRANS) or X M
 template <int NT, bool TRANS>
-__device__ __forceinline__ void load_square_b(uint32_t tile, int n0, int k0, int lane, uint32_t (&b)[NT][4]) {
+__device__ __forceinline__ void load_square_b(uint32_t tile, int bi, int bj, int lane, uint32_t (&b)[NT][4]) {
 #pragma unroll
   for (int m = 0; m < NT; ++m) {
-    if (TRANS) load_b_nt<64>(tile + m * SQ, n0, k0, lane, b[m]);
-    else load_b_nn<64>(tile + m * SQ, k0, n0, lane, b[m]);
+    if (TRANS) ldsm4(block_addr(tile + m * SQB, bi, bj, ((lane >> 4) << 3) + (lane & 7), (lane >> 3) & 1), b[m]);
+    else ldsm4_t(block_addr(tile + m * SQB, bi, bj, (((lane >> 3) & 1) << 3) + (lane & 7), lane >> 4), b[m]);
   }
 }
 
-// x [8][4] holds (16 columns of v) x (64 tokens), `tile` bf16 rows of the same tokens and columns: the dot product of every
-// token over these columns -> dst[64]
-__device__ __forceinline__ void token_dots(const float (&x)[8][4], uint32_t tile, float* dst, int warp, int lane) {
-#pragma unroll
-  for (int n = 0; n < 8; n += 2) {
-    uint32_t a[4];
-    load_a_t<64>(tile, warp * 16, n * 8, lane, a);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u]));
-      const float2 y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u + 1]));
-      float d0 = fmaf(x[n + u][0], y0.x, x[n + u][2] * y1.x), d1 = fmaf(x[n + u][1], y0.y, x[n + u][3] * y1.y);
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-        d1 += __shfl_xor_sync(0xffffffffu, d1, o);
+// The four strips of a CTA do not wait for each other: their chunks are shifted against each other by up to half a chunk, so that the
+// tensor-core products of one strip meet the arithmetic and the waits of others on each scheduler (a warp of every strip).  A stage
+// is loaded by all threads, in the middle of the chunk before it and once all strips are done with the chunk that was in it.
+struct ScanRing {
+  uint32_t full, empty;                         // mbarriers of the first stage; + 8 of the second; + 16 (full) of M and P
+  volatile int* abort_flag;
+  int* status;
+  __device__ __forceinline__ void init(uint32_t bars, volatile int* flag, int* st) {
+    full = bars;
+    empty = bars + 32;
+    abort_flag = flag;
+    status = st;
+    if (threadIdx.x == 0) {
+      *flag = 0;
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(full + 8 * i, ST);
+        mbar_init(full + 16 + 8 * i, ST);
+        mbar_init(empty + 8 * i, ST / 32);
       }
-      if (lane < 4) *reinterpret_cast<float2*>(dst + (n + u) * 8 + lane * 2) = make_float2(d0, d1);
+      fence_barrier_init();
     }
+    __syncthreads();
+  }
+  // a wait that gives up reports it and the walk goes on, with what is there, to its end: the barriers of a strip stay whole
+  __device__ __forceinline__ void wait_full(int i) { mbar_wait_warp(full + 8 * (i & 1), (i >> 1) & 1, abort_flag, status, ST_TIMEOUT_FULL); }
+  __device__ __forceinline__ void wait_squares(int i) {
+    mbar_wait_warp(full + 16 + 8 * (i & 1), (i >> 1) & 1, abort_flag, status, ST_TIMEOUT_FULL);
+  }
+  __device__ __forceinline__ void wait_empty(int i) {          // until stage i & 1 is free for the i-th chunk
+    if (i >= 2) mbar_wait_warp(empty + 8 * (i & 1), ((i >> 1) & 1) ^ 1, abort_flag, status, ST_TIMEOUT_EMPTY);
+  }
+  __device__ __forceinline__ void done(int i, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty + 8 * (i & 1));
+  }
+};
+
+// Four warps share a strip of 16 columns of v: each has 16 of a chunk's tokens as columns of the token products and a quarter of
+// the d columns of the state.  What all of them need as the second operand of the next product goes through shared memory as the
+// terms it enters in, formed once; a lane reads what the same lane of another warp wrote.
+__device__ __forceinline__ void strip_sync(int strip) { asm volatile("bar.sync %0, 128;" ::"r"(1 + strip) : "memory"); }
+template <int NT>
+__device__ __forceinline__ void share(uint32_t at, int kk, const uint32_t (&a)[NT][4]) {          // `at` includes the lane
+#pragma unroll
+  for (int m = 0; m < NT; ++m)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + (kk * NT + m) * 512), "r"(a[m][0]), "r"(a[m][1]), "r"(a[m][2]),
+                 "r"(a[m][3]) : "memory");
+}
+template <int NT>
+__device__ __forceinline__ void shared_terms(uint32_t at, int kk, uint32_t (&a)[NT][4]) {
+#pragma unroll
+  for (int m = 0; m < NT; ++m)
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(a[m][0]), "=r"(a[m][1]), "=r"(a[m][2]), "=r"(a[m][3])
+                 : "r"(at + (kk * NT + m) * 512) : "memory");
+}
+template <int NT, int N>
+__device__ __forceinline__ void share_state(uint32_t at, int quarter, const float (&S)[N][4]) {
+#pragma unroll
+  for (int n = 0; n < N; n += 2) {
+    uint32_t a[NT][4];
+    acc_to_terms<NT>(S[n], S[n + 1], a);
+    share<NT>(at, (quarter * N + n) / 2, a);
   }
 }
 
-// accumulators (16 rows x 8 N columns) -> two bf16 planes with `ld` columns
-template <int N>
-__device__ __forceinline__ void store_terms(const float (&a)[N][4], __nv_bfloat16* dst, long long plane, int ld, int row, int lane) {
-  const int col = (lane & 3) * 2;
+// x [2][4] holds (16 columns of v) x (16 tokens), `tile` bf16 rows of the same tokens and columns: the dot product of every token
+// over these columns -> dst[64]
+__device__ __forceinline__ void token_dots(const float (&x)[2][4], uint32_t tile, float* dst, int strip, int tok0, int lane) {
+  uint32_t a[4];
+  load_a_t<64>(tile, strip * 16, tok0, lane, a);
 #pragma unroll
-  for (int n = 0; n < N; ++n) {
+  for (int u = 0; u < 2; ++u) {
+    const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u]));
+    const float2 y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u + 1]));
+    float d0 = fmaf(x[u][0], y0.x, x[u][2] * y1.x), d1 = fmaf(x[u][1], y0.y, x[u][3] * y1.y);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      d0 += __shfl_xor_sync(0xffffffffu, d0, o);
+      d1 += __shfl_xor_sync(0xffffffffu, d1, o);
+    }
+    if (lane < 4) *reinterpret_cast<float2*>(dst + tok0 + u * 8 + lane * 2) = make_float2(d0, d1);
+  }
+}
+
+// accumulators (16 rows x 16 tokens) -> two bf16 planes with 64 columns
+__device__ __forceinline__ void store_terms(const float (&a)[2][4], __nv_bfloat16* dst, long long plane, int row, int tok0, int lane) {
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       uint32_t hi, lo;
       split2(a[n][2 * r], a[n][2 * r + 1], hi, lo);
-      __nv_bfloat16* at = dst + (long long)(row + 8 * r) * ld + n * 8 + col;
+      __nv_bfloat16* at = dst + (long long)(row + 8 * r) * C + tok0 + n * 8 + (lane & 3) * 2;
       *reinterpret_cast<uint32_t*>(at) = hi;
       *reinterpret_cast<uint32_t*>(at + plane) = lo;
     }
   }
 }
 
-// x [8][4] holds (16 columns of v) x (64 tokens): written as bf16 rows of tokens through the warp's columns of `tile`
-__device__ __forceinline__ void store_transposed(const float (&x)[8][4], uint32_t tile, __nv_bfloat16* dst, long long stride, int len,
-                                                 int warp, int lane) {
+// x [2][4] holds (16 columns of v) x (16 tokens): written as bf16 rows of tokens through the warp's part of `tile`
+__device__ __forceinline__ void store_transposed(const float (&x)[2][4], uint32_t tile, __nv_bfloat16* dst, long long stride, int len,
+                                                 int strip, int tok0, int lane) {
   __syncwarp();
-#pragma unroll
-  for (int n = 0; n < 8; n += 2) {
-    const int tok = n * 8 + ((lane >> 4) << 3) + (lane & 7), col = warp * 16 + (((lane >> 3) & 1) << 3);
-    stsm4_t(tile_addr<64>(tile, tok, col), pack_bf16x2(x[n][0], x[n][1]), pack_bf16x2(x[n][2], x[n][3]),
-            pack_bf16x2(x[n + 1][0], x[n + 1][1]), pack_bf16x2(x[n + 1][2], x[n + 1][3]));
-  }
+  stsm4_t(tile_addr<64>(tile, tok0 + ((lane >> 4) << 3) + (lane & 7), strip * 16 + (((lane >> 3) & 1) << 3)),
+          pack_bf16x2(x[0][0], x[0][1]), pack_bf16x2(x[0][2], x[0][3]), pack_bf16x2(x[1][0], x[1][1]), pack_bf16x2(x[1][2], x[1][3]));
   __syncwarp();
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int tok = u * 16 + (lane >> 1), col = warp * 16 + (lane & 1) * 8;
-    uint4 v;
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "r"(tile_addr<64>(tile, tok, col)) : "memory");
-    if (tok < len) *reinterpret_cast<uint4*>(dst + (long long)tok * stride + col) = v;
-  }
+  const int tok = tok0 + (lane >> 1), col = strip * 16 + (lane & 1) * 8;
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(tile_addr<64>(tile, tok, col)) : "memory");
+  if (tok < len) *reinterpret_cast<uint4*>(dst + (long long)tok * stride + col) = v;
 }
 
 // SAVE: keep S, V and E of every chunk for the backward pass and form do . O of every token; else the outputs
 template <int D, bool SAVE>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(ST, 1)
 gdr_scan_kernel(const GdrParams p) {
-  constexpr int NT = SAVE ? 3 : 2;
+  constexpr int NT = SAVE ? 3 : 2, NB = D / 32;  // NB: 8-column blocks of a quarter of the state
   using L = ScanSmem<D, NT, SAVE>;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ int slot;
+  __shared__ int slot, flag;
   const uint32_t base = (smem_u32(smem_raw) + 127) & ~127u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, strip = warp_uniform(threadIdx.x >> 7), quarter = (warp_uniform(threadIdx.x >> 5) + strip) & 3;
   const ScanPos s = scan_pos<D>(p, &slot);
   if (s.n == 0) return;
   const long long stride = (long long)p.H * D;
-  const int row = s.col0 + warp * 16 + (lane >> 2);
-  float St[D / 8][4];
+  const int row = s.col0 + strip * 16 + (lane >> 2), tok0 = quarter * 16;
+  const uint32_t part0 = base + L::SHARE + strip * L::STRIP + lane * 16, part1 = part0 + L::PART;   // S in both; X, what V adds to S; V
+  float St[NB][4];
   zero(St);
-  load_stage<D, NT, SAVE>(base, p, s.t0, min(C, s.len), s.h, s.col0, (long long)s.chunk0 * p.H + s.h);
+  ScanRing ring;
+  ring.init(base + L::BARS, &flag, p.status);
+  auto load = [&](int c) {
+    if (c >= s.n) return;
+    ring.wait_empty(c);
+    load_stage<D, NT, SAVE>(base + (c & 1) * L::STAGE, ring.full + 8 * (c & 1), p, s.t0 + c * C, min(C, s.len - c * C), s.h, s.col0,
+                            (long long)(s.chunk0 + c) * p.H + s.h);
+  };
+  load(0);
   for (int c = 0; c < s.n; ++c) {
     const uint32_t st = base + (c & 1) * L::STAGE;
     const int t = s.t0 + c * C, len = min(C, s.len - c * C);
     const long long ch = (long long)(s.chunk0 + c) * p.H + s.h;
-    if (c + 1 < s.n) {
-      load_stage<D, NT, SAVE>(base + ((c + 1) & 1) * L::STAGE, p, t + C, min(C, s.len - (c + 1) * C), s.h, s.col0, ch + p.H);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    if (SAVE) store_f32(St, p.S + ch * D * D, D, row, lane);
-    float X[8][4] = {}, O[8][4] = {}, Xl[8][4] = {}, Ol[8][4] = {};
+    ring.wait_full(c);
+    if (c > 0) strip_sync(strip);               // S
+    if (SAVE) store_f32(St, p.S + ch * D * D + quarter * (D / 4), D, row, lane);
+    float X[2][4] = {}, O[2][4] = {}, Xl[2][4] = {}, Ol[2][4] = {};
     if (c > 0) {                                // the state is zero before the first chunk
 #pragma unroll
       for (int kk = 0; kk < D / 16; ++kk) {
-        uint32_t a[NT][4];
-        acc_to_terms<NT>(St[2 * kk], St[2 * kk + 1], a);
+        uint32_t a[NT][4], b[4], d[4];
+        shared_terms<NT>(part0, kk, a);
+        load_b_nt<D>(st + L::K, tok0, kk * 16, lane, b);
+        load_b_nt<D>(st + L::Q, tok0, kk * 16, lane, d);
 #pragma unroll
-        for (int n = 0; n < 8; n += 2) {
-          uint32_t b[4], d[4];
-          load_b_nt<D>(st + L::K, n * 8, kk * 16, lane, b);
-          load_b_nt<D>(st + L::Q, n * 8, kk * 16, lane, d);
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            mma_exact<NT>(X[n + u], Xl[n + u], a, b[2 * u], b[2 * u + 1]);
-            mma_exact<NT>(O[n + u], Ol[n + u], a, d[2 * u], d[2 * u + 1]);
-          }
+        for (int u = 0; u < 2; ++u) {
+          mma_exact<NT>(X[u], Xl[u], a, b[2 * u], b[2 * u + 1]);
+          mma_exact<NT>(O[u], Ol[u], a, d[2 * u], d[2 * u + 1]);
         }
       }
       join(X, Xl);
       join(O, Ol);
     }
     // V (as -E so far) = -exp(G) k S, X = v - exp(G) k S; columns = tokens
-    const uint32_t sb = st + L::G + (lane & 3) * 8, se = sb + C * 4, sr = se + C * 4, sp = sr + C * 4;   // rows of gb
+    const uint32_t sb = st + L::G + (tok0 + (lane & 3) * 2) * 4, se = sb + C * 4, sr = se + C * 4, sp = sr + C * 4;   // rows of gb
     const float el = lds1(st + L::G + (2 * C - 1) * 4);
-    float V[8][4], Vl[8][4] = {};
-#pragma unroll
-    for (int n = 0; n < 8; n += 2) {
+    float V[2][4], Vl[2][4] = {};
+    float2 vv[2][2];
+    {
       uint32_t a[4];
-      load_a_t<64>(st + L::X, warp * 16, n * 8, lane, a);
+      load_a_t<64>(st + L::X, strip * 16, tok0, lane, a);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const float2 e = lds2(se + (n + u) * 32);
-        const float2 v0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u]));
-        const float2 v1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u + 1]));
-        float (&x)[4] = X[n + u], (&o)[4] = O[n + u];
-        float (&y)[4] = V[n + u];
+        const float2 e = lds2(se + u * 32);
+        vv[u][0] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u]));
+        vv[u][1] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u + 1]));
+        float (&x)[4] = X[u], (&o)[4] = O[u], (&y)[4] = V[u];
         y[0] = -e.x * x[0];
         y[1] = -e.y * x[1];
         y[2] = -e.x * x[2];
         y[3] = -e.y * x[3];
-        x[0] = v0.x + y[0];
-        x[1] = v0.y + y[1];
-        x[2] = v1.x + y[2];
-        x[3] = v1.y + y[3];
+        x[0] = vv[u][0].x + y[0];
+        x[1] = vv[u][0].y + y[1];
+        x[2] = vv[u][1].x + y[2];
+        x[3] = vv[u][1].y + y[3];
         o[0] *= p.scale * e.x;
         o[1] *= p.scale * e.y;
         o[2] *= p.scale * e.x;
         o[3] *= p.scale * e.y;
       }
     }
+    strip_sync(strip);                          // all have read S
+    {
+      uint32_t a[NT][4];
+      acc_to_terms<NT>(X[0], X[1], a);
+      share<NT>(part0, quarter, a);
+    }
+    strip_sync(strip);
+    ring.wait_squares(c);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
-      uint32_t a[NT][4];
-      acc_to_terms<NT>(X[2 * kk], X[2 * kk + 1], a);
-#pragma unroll
-      for (int n = 2 * kk; n < 8; n += 2) {     // M is lower triangular
-        uint32_t b[NT][4];
-        load_square_b<NT, true>(st + L::M, n * 8, kk * 16, lane, b);
-        mma_terms<NT>(V[n], Vl[n], a, b, 0);
-        mma_terms<NT>(V[n + 1], Vl[n + 1], a, b, 1);
-      }
+      if (kk > quarter) break;                  // M is lower triangular
+      uint32_t a[NT][4], b[NT][4];
+      shared_terms<NT>(part0, kk, a);
+      load_square_b<NT, true>(st + L::M, quarter, kk, lane, b);
+      mma_terms<NT>(V[0], Vl[0], a, b, 0);
+      mma_terms<NT>(V[1], Vl[1], a, b, 1);
     }
     join(V, Vl);
+    load(c + 1);
     if (SAVE) {
-      float4* e = reinterpret_cast<float4*>(p.E + (ch * (D / 16) + (s.col0 >> 4) + warp) * (16 * C)) + lane;
+      float4* e = reinterpret_cast<float4*>(p.E + (ch * (D / 16) + (s.col0 >> 4) + strip) * (16 * C)) + lane;
 #pragma unroll
-      for (int n = 0; n < 8; ++n) e[n * 32] = make_float4(-V[n][0], -V[n][1], -V[n][2], -V[n][3]);
+      for (int n = 0; n < 2; ++n) e[(2 * quarter + n) * 32] = make_float4(-V[n][0], -V[n][1], -V[n][2], -V[n][3]);
     }
-#pragma unroll
-    for (int n = 0; n < 8; n += 2) {
-      uint32_t a[4];
-      load_a_t<64>(st + L::X, warp * 16, n * 8, lane, a);
+    {
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const float2 b = lds2(sb + (n + u) * 32);
-        const float2 v0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u]));
-        const float2 v1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[2 * u + 1]));
-        float (&x)[4] = V[n + u];
-        x[0] = b.x * (v0.x + x[0]);
-        x[1] = b.y * (v0.y + x[1]);
-        x[2] = b.x * (v1.x + x[2]);
-        x[3] = b.y * (v1.y + x[3]);
+        const float2 b = lds2(sb + u * 32);
+        float (&x)[4] = V[u];
+        x[0] = b.x * (vv[u][0].x + x[0]);
+        x[1] = b.y * (vv[u][0].y + x[1]);
+        x[2] = b.x * (vv[u][1].x + x[2]);
+        x[3] = b.y * (vv[u][1].y + x[3]);
       }
+      uint32_t a[NT][4];
+      acc_to_terms<NT>(V[0], V[1], a);
+      share<NT>(part1, quarter, a);
     }
-    if (SAVE) store_terms<8>(V, p.V + ch * 2 * D * C, (long long)D * C, C, row, lane);
+    strip_sync(strip);                          // V; and all have read X
+    if (c + 1 < s.n) {
+      float W[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float2 w = lds2(sr + u * 32);
+        W[u][0] = V[u][0] * w.x;
+        W[u][1] = V[u][1] * w.y;
+        W[u][2] = V[u][2] * w.x;
+        W[u][3] = V[u][3] * w.y;
+      }
+      uint32_t a[NT][4];
+      acc_to_terms<NT>(W[0], W[1], a);
+      share<NT>(part0, quarter, a);
+    }
+    if (SAVE) store_terms(V, p.V + ch * 2 * D * C, (long long)D * C, row, tok0, lane);
     zero(Ol);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
-      uint32_t a[NT][4];
-      acc_to_terms<NT>(V[2 * kk], V[2 * kk + 1], a);
-#pragma unroll
-      for (int n = 2 * kk; n < 8; n += 2) {     // P is lower triangular
-        uint32_t b[NT][4];
-        load_square_b<NT, true>(st + L::P, n * 8, kk * 16, lane, b);
-        mma_terms<NT>(O[n], Ol[n], a, b, 0);
-        mma_terms<NT>(O[n + 1], Ol[n + 1], a, b, 1);
-      }
+      if (kk > quarter) break;                  // P is lower triangular
+      uint32_t a[NT][4], b[NT][4];
+      shared_terms<NT>(part1, kk, a);
+      load_square_b<NT, true>(st + L::P, quarter, kk, lane, b);
+      mma_terms<NT>(O[0], Ol[0], a, b, 0);
+      mma_terms<NT>(O[1], Ol[1], a, b, 1);
     }
     join(O, Ol);
     if (SAVE) {
-      token_dots(O, st + L::Z, p.oo + (ch * (D / 16) + (s.col0 >> 4) + warp) * C, warp, lane);
+      token_dots(O, st + L::Z, p.oo + (ch * (D / 16) + (s.col0 >> 4) + strip) * C, strip, tok0, lane);
     } else {
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
+      for (int n = 0; n < 2; ++n) {
         const float2 d = lds2(sp + n * 32);
         O[n][0] = fmaf(d.x, V[n][0], O[n][0]);
         O[n][1] = fmaf(d.y, V[n][1], O[n][1]);
         O[n][2] = fmaf(d.x, V[n][2], O[n][2]);
         O[n][3] = fmaf(d.y, V[n][3], O[n][3]);
       }
-      store_transposed(O, st + L::X, p.o + ((long long)t * p.H + s.h) * D + s.col0, stride, len, warp, lane);
+      store_transposed(O, st + L::X, p.o + ((long long)t * p.H + s.h) * D + s.col0, stride, len, strip, tok0, lane);
     }
     if (c + 1 < s.n) {
-      uint32_t a[4][NT][4];
+      strip_sync(strip);
+      float U[NB][4] = {}, Ul[NB][4] = {};      // what the chunk adds is summed apart: many chunks meet in the state
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        const float2 w = lds2(sr + n * 32);
-        V[n][0] *= w.x;
-        V[n][1] *= w.y;
-        V[n][2] *= w.x;
-        V[n][3] *= w.y;
-      }
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t a[NT][4];
+        shared_terms<NT>(part0, kk, a);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) acc_to_terms<NT>(V[2 * kk], V[2 * kk + 1], a[kk]);
-#pragma unroll
-      for (int n = 0; n < D / 8; n += 2) {      // what the chunk adds is summed apart: many chunks meet in the state
-        float U[2][4] = {}, Ul[2][4] = {};
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
+        for (int n = 0; n < NB; n += 2) {
           uint32_t b[4];
-          load_b_nn<D>(st + L::K, kk * 16, n * 8, lane, b);
-          mma_exact<NT>(U[0], Ul[0], a[kk], b[0], b[1]);
-          mma_exact<NT>(U[1], Ul[1], a[kk], b[2], b[3]);
+          load_b_nn<D>(st + L::K, kk * 16, quarter * (D / 4) + n * 8, lane, b);
+          mma_exact<NT>(U[n], Ul[n], a, b[0], b[1]);
+          mma_exact<NT>(U[n + 1], Ul[n + 1], a, b[2], b[3]);
         }
-        join(U, Ul);
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) St[n + u][e] = fmaf(St[n + u][e], el, U[u][e]);
       }
+      join(U, Ul);
+#pragma unroll
+      for (int n = 0; n < NB; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) St[n][e] = fmaf(St[n][e], el, U[n][e]);
+      ring.done(c, lane);
+      strip_sync(strip);                        // all have read V and what it adds
+      share_state<NT>(part0, quarter, St);
     }
-    __syncthreads();                            // the stage is free for the copies of the chunk after the next
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");   // nothing to wait for, unless a wait gave up
 }
 
 template <int D>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(ST, 1)
 gdr_scan_bwd_kernel(const GdrParams p) {
-  constexpr int NT = 3;
+  constexpr int NT = 3, NB = D / 32;
   using L = ScanSmem<D, NT, true>;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ int slot;
+  __shared__ int slot, flag;
   const uint32_t base = (smem_u32(smem_raw) + 127) & ~127u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, strip = warp_uniform(threadIdx.x >> 7), quarter = (warp_uniform(threadIdx.x >> 5) + strip) & 3;
   const ScanPos s = scan_pos<D>(p, &slot);
   if (s.n == 0) return;
   const long long stride = (long long)p.H * D;
-  const int row = s.col0 + warp * 16 + (lane >> 2);
-  const uint32_t mine = base + 2 * L::STAGE + warp * (16 * C * 4) + lane * 16;
-  float dSt[D / 8][4];
+  const int row = s.col0 + strip * 16 + (lane >> 2), tok0 = quarter * 16;
+  const uint32_t part0 = base + L::SHARE + strip * L::STRIP + lane * 16, part1 = part0 + L::PART;   // dS in both; beta (F + p do), do; B
+  float dSt[NB][4];
   zero(dSt);
   const int lastc = s.n - 1;
-  load_stage<D, NT, true>(base, p, s.t0 + lastc * C, s.len - lastc * C, s.h, s.col0, (long long)(s.chunk0 + lastc) * p.H + s.h);
+  ScanRing ring;
+  ring.init(base + L::BARS, &flag, p.status);
+  auto load = [&](int it) {
+    const int c = lastc - it;
+    if (c < 0) return;
+    ring.wait_empty(it);
+    load_stage<D, NT, true>(base + (it & 1) * L::STAGE, ring.full + 8 * (it & 1), p, s.t0 + c * C, min(C, s.len - c * C), s.h, s.col0,
+                            (long long)(s.chunk0 + c) * p.H + s.h);
+  };
+  load(0);
   for (int it = 0; it < s.n; ++it) {
     const int c = lastc - it;
     const uint32_t st = base + (it & 1) * L::STAGE;
     const int t = s.t0 + c * C, len = min(C, s.len - c * C);
     const long long ch = (long long)(s.chunk0 + c) * p.H + s.h;
-    const long long part = ch * (D / 16) + (s.col0 >> 4) + warp;
+    const long long part = ch * (D / 16) + (s.col0 >> 4) + strip;
+    float4 Ev[2];
 #pragma unroll
-    for (int n = 0; n < 8; ++n)                 // every lane copies what it will read itself
-      cp_async16(mine + n * 512, p.E + part * (16 * C) + (n * 32 + lane) * 4, 16);
-    cp_async_commit();
-    if (c > 0) {
-      load_stage<D, NT, true>(base + ((it + 1) & 1) * L::STAGE, p, t - C, C, s.h, s.col0, ch - p.H);
-      cp_async_wait<2>();
-    } else {
-      cp_async_wait<1>();
-    }
-    __syncthreads();
-    store_f32(dSt, p.dS + ch * D * D, D, row, lane);
-    const uint32_t sb = st + L::G + (lane & 3) * 8, se = sb + C * 4, sr = se + C * 4, sp = sr + C * 4;   // rows of gb
+    for (int n = 0; n < 2; ++n) Ev[n] = reinterpret_cast<const float4*>(p.E + part * (16 * C))[(2 * quarter + n) * 32 + lane];
+    ring.wait_full(it);
+    if (it > 0) strip_sync(strip);              // dS
+    store_f32(dSt, p.dS + ch * D * D + quarter * (D / 4), D, row, lane);
+    const uint32_t sb = st + L::G + (tok0 + (lane & 3) * 2) * 4, se = sb + C * 4, sr = se + C * 4, sp = sr + C * 4;   // rows of gb
     const float el = lds1(st + L::G + (2 * C - 1) * 4);
-    float dV[8][4] = {}, lo[8][4] = {};
+    float dV[2][4] = {}, lo[2][4] = {};
     if (it > 0) {                               // nothing flows into the sequence's last state
 #pragma unroll
       for (int kk = 0; kk < D / 16; ++kk) {
-        uint32_t a[NT][4];
-        acc_to_terms<NT>(dSt[2 * kk], dSt[2 * kk + 1], a);
-#pragma unroll
-        for (int n = 0; n < 8; n += 2) {
-          uint32_t b[4];
-          load_b_nt<D>(st + L::K, n * 8, kk * 16, lane, b);
-          mma_exact<NT>(dV[n], lo[n], a, b[0], b[1]);
-          mma_exact<NT>(dV[n + 1], lo[n + 1], a, b[2], b[3]);
-        }
+        uint32_t a[NT][4], b[4];
+        shared_terms<NT>(part0, kk, a);
+        load_b_nt<D>(st + L::K, tok0, kk * 16, lane, b);
+        mma_exact<NT>(dV[0], lo[0], a, b[0], b[1]);
+        mma_exact<NT>(dV[1], lo[1], a, b[2], b[3]);
       }
       join(dV, lo);
       zero(lo);
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
+      for (int n = 0; n < 2; ++n) {
         const float2 w = lds2(sr + n * 32);
         dV[n][0] *= w.x;
         dV[n][1] *= w.y;
@@ -635,130 +722,133 @@ gdr_scan_bwd_kernel(const GdrParams p) {
         dV[n][3] *= w.y;
       }
     }
+    strip_sync(strip);                          // all have read dS
+    ring.wait_squares(it);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
-      uint32_t da[4];                           // do^T: rows = columns of v, contraction = tokens
-      load_a_t<64>(st + L::Z, warp * 16, kk * 16, lane, da);
+      if (kk < quarter) continue;               // rows i of P from column block j <= i
+      uint32_t da[4], b[NT][4];                 // do^T: rows = columns of v, contraction = tokens
+      load_a_t<64>(st + L::Z, strip * 16, kk * 16, lane, da);
+      load_square_b<NT, false>(st + L::P, kk, quarter, lane, b);
 #pragma unroll
-      for (int n = 0; n <= 2 * kk; n += 2) {    // rows i of P from column block j <= i
-        uint32_t b[NT][4];
-        load_square_b<NT, false>(st + L::P, n * 8, kk * 16, lane, b);
+      for (int u = 0; u < 2; ++u) {
+        mma16816(dV[u], da, b[0][2 * u], b[0][2 * u + 1]);
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          mma16816(dV[n + u], da, b[0][2 * u], b[0][2 * u + 1]);
-#pragma unroll
-          for (int m = 1; m < NT; ++m) mma16816(lo[n + u], da, b[m][2 * u], b[m][2 * u + 1]);
-        }
+        for (int m = 1; m < NT; ++m) mma16816(lo[u], da, b[m][2 * u], b[m][2 * u + 1]);
       }
     }
     join(dV, lo);
     zero(lo);
-    float B[8][4] = {};
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {            // M^T (beta (F + p do))
-      uint32_t da[4], a[NT][4];
-      load_a_t<64>(st + L::Z, warp * 16, kk * 16, lane, da);
+    uint32_t da[4];
+    load_a_t<64>(st + L::Z, strip * 16, tok0, lane, da);
+    {
+      uint32_t a[NT][4];                        // beta (F + p do); registers 2u, 2u + 1: tokens of the lower / upper half of the slice
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const float2 b = lds2(sb + (2 * kk + u) * 32), d = lds2(sp + (2 * kk + u) * 32);
+        const float2 b = lds2(sb + u * 32), d = lds2(sp + u * 32);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&da[2 * u + r]));
-          split_terms<NT>(nonzero(b.x) * fmaf(d.x, x.x, dV[2 * kk + u][2 * r]),
-                          nonzero(b.y) * fmaf(d.y, x.y, dV[2 * kk + u][2 * r + 1]), a, 2 * u + r);
+          split_terms<NT>(nonzero(b.x) * fmaf(d.x, x.x, dV[u][2 * r]), nonzero(b.y) * fmaf(d.y, x.y, dV[u][2 * r + 1]), a, 2 * u + r);
         }
       }
+      share<NT>(part0, quarter, a);
+    }
+    strip_sync(strip);
+    float B[2][4] = {};
 #pragma unroll
-      for (int n = 0; n <= 2 * kk; n += 2) {
-        uint32_t b[NT][4];
-        load_square_b<NT, false>(st + L::M, n * 8, kk * 16, lane, b);
-        mma_terms<NT>(B[n], lo[n], a, b, 0);
-        mma_terms<NT>(B[n + 1], lo[n + 1], a, b, 1);
-      }
+    for (int kk = 0; kk < 4; ++kk) {            // M^T (beta (F + p do))
+      if (kk < quarter) continue;
+      uint32_t a[NT][4], b[NT][4];
+      shared_terms<NT>(part0, kk, a);
+      load_square_b<NT, false>(st + L::M, kk, quarter, lane, b);
+      mma_terms<NT>(B[0], lo[0], a, b, 0);
+      mma_terms<NT>(B[1], lo[1], a, b, 1);
     }
     join(B, lo);
-    if (c > 0) cp_async_wait<1>();              // E (the next stage may still be on its way)
-    else cp_async_wait<0>();
+    load(it + 1);
     float *nn = p.nn + part * C, *yy = p.yy + part * C;
+    uint32_t va[4], ab[NT][4];                  // ab: -exp(G) B
+    load_a_t<64>(st + L::X, strip * 16, tok0, lane, va);
 #pragma unroll
-    for (int n = 0; n < 8; n += 2) {
-      uint32_t da[4], va[4];
-      load_a_t<64>(st + L::Z, warp * 16, n * 8, lane, da);
-      load_a_t<64>(st + L::X, warp * 16, n * 8, lane, va);
+    for (int u = 0; u < 2; ++u) {
+      const float2 b = lds2(sb + u * 32), d = lds2(sp + u * 32), eg = lds2(se + u * 32);
+      const float E[4] = {Ev[u].x, Ev[u].y, Ev[u].z, Ev[u].w};
+      float dn[2] = {0.f, 0.f}, dy[2] = {0.f, 0.f};
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const float2 b = lds2(sb + (n + u) * 32), d = lds2(sp + (n + u) * 32);
-        float E[4];
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(E[0]), "=f"(E[1]), "=f"(E[2]), "=f"(E[3])
-                     : "r"(mine + (n + u) * 512) : "memory");
-        float dn[2] = {0.f, 0.f}, dy[2] = {0.f, 0.f};
+      for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 x2 = *reinterpret_cast<const __nv_bfloat162*>(&da[2 * u + (e >> 1)]);
+        const __nv_bfloat162 v2 = *reinterpret_cast<const __nv_bfloat162*>(&va[2 * u + (e >> 1)]);
+        const float x = e & 1 ? __high2float(x2) : __low2float(x2), v = e & 1 ? __high2float(v2) : __low2float(v2);
+        const float be = e & 1 ? b.y : b.x, W = v - E[e];
+        const float N = dV[u][e] + B[u][e] / nonzero(be), Y = fmaf(e & 1 ? d.y : d.x, x, N);
+        dn[e & 1] += be * fmaf(W, N, Y * E[e]);
+        dy[e & 1] = fmaf(Y, W, dy[e & 1]);
+        B[u][e] = be * Y;
+      }
+      split_terms<NT>(-eg.x * B[u][0], -eg.y * B[u][1], ab, 2 * u);
+      split_terms<NT>(-eg.x * B[u][2], -eg.y * B[u][3], ab, 2 * u + 1);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const __nv_bfloat162 x2 = *reinterpret_cast<const __nv_bfloat162*>(&da[2 * u + (e >> 1)]);
-          const __nv_bfloat162 v2 = *reinterpret_cast<const __nv_bfloat162*>(&va[2 * u + (e >> 1)]);
-          const float x = e & 1 ? __high2float(x2) : __low2float(x2), v = e & 1 ? __high2float(v2) : __low2float(v2);
-          const float be = e & 1 ? b.y : b.x, W = v - E[e];
-          const float N = dV[n + u][e] + B[n + u][e] / nonzero(be), Y = fmaf(e & 1 ? d.y : d.x, x, N);
-          dn[e & 1] += be * fmaf(W, N, Y * E[e]);
-          dy[e & 1] = fmaf(Y, W, dy[e & 1]);
-          B[n + u][e] = be * Y;
-        }
+      for (int o = 4; o < 32; o <<= 1) {
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            dn[r] += __shfl_xor_sync(0xffffffffu, dn[r], o);
-            dy[r] += __shfl_xor_sync(0xffffffffu, dy[r], o);
-          }
-        }
-        if (lane < 4) {
-          *reinterpret_cast<float2*>(nn + (n + u) * 8 + lane * 2) = make_float2(dn[0], dn[1]);
-          *reinterpret_cast<float2*>(yy + (n + u) * 8 + lane * 2) = make_float2(dy[0], dy[1]);
+        for (int r = 0; r < 2; ++r) {
+          dn[r] += __shfl_xor_sync(0xffffffffu, dn[r], o);
+          dy[r] += __shfl_xor_sync(0xffffffffu, dy[r], o);
         }
       }
+      if (lane < 4) {
+        *reinterpret_cast<float2*>(nn + tok0 + u * 8 + lane * 2) = make_float2(dn[0], dn[1]);
+        *reinterpret_cast<float2*>(yy + tok0 + u * 8 + lane * 2) = make_float2(dy[0], dy[1]);
+      }
     }
-    store_terms<8>(B, p.B + ch * 2 * D * C, (long long)D * C, C, row, lane);
-    store_transposed(B, st + L::X, p.dv + ((long long)t * p.H + s.h) * D + s.col0, stride, len, warp, lane);
+    share<NT>(part1, quarter, ab);
+    store_terms(B, p.B + ch * 2 * D * C, (long long)D * C, row, tok0, lane);
+    store_transposed(B, st + L::X, p.dv + ((long long)t * p.H + s.h) * D + s.col0, stride, len, strip, tok0, lane);
     if (c > 0) {
-      uint32_t aq[4][NT][4], ak[4][NT][4];      // scale exp(G) do^T and -exp(G) B^T
+      strip_sync(strip);                        // all have read beta (F + p do)
+      {
+        uint32_t q[NT][4];                      // scale exp(G) do
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        uint32_t da[4];
-        load_a_t<64>(st + L::Z, warp * 16, kk * 16, lane, da);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {           // registers 2u, 2u + 1: tokens of the lower / upper half of the slice
-          const float2 e = lds2(se + (2 * kk + u) * 32);
+        for (int u = 0; u < 2; ++u) {
+          const float2 e = lds2(se + u * 32);
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&da[2 * u + r]));
-            split_terms<NT>(x.x * (p.scale * e.x), x.y * (p.scale * e.y), aq[kk], 2 * u + r);
-            split_terms<NT>(-e.x * B[2 * kk + u][2 * r], -e.y * B[2 * kk + u][2 * r + 1], ak[kk], 2 * u + r);
+            split_terms<NT>(x.x * (p.scale * e.x), x.y * (p.scale * e.y), q, 2 * u + r);
           }
         }
+        share<NT>(part0, quarter, q);
       }
+      strip_sync(strip);
+      float U[NB][4] = {}, Ul[NB][4] = {};
 #pragma unroll
-      for (int n = 0; n < D / 8; n += 2) {
-        float U[2][4] = {}, Ul[2][4] = {};
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t aq[NT][4], ak[NT][4];
+        shared_terms<NT>(part0, kk, aq);
+        shared_terms<NT>(part1, kk, ak);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
+        for (int n = 0; n < NB; n += 2) {
           uint32_t b[4], d[4];
-          load_b_nn<D>(st + L::Q, kk * 16, n * 8, lane, b);
-          load_b_nn<D>(st + L::K, kk * 16, n * 8, lane, d);
+          load_b_nn<D>(st + L::Q, kk * 16, quarter * (D / 4) + n * 8, lane, b);
+          load_b_nn<D>(st + L::K, kk * 16, quarter * (D / 4) + n * 8, lane, d);
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            mma_exact<NT>(U[u], Ul[u], aq[kk], b[2 * u], b[2 * u + 1]);
-            mma_exact<NT>(U[u], Ul[u], ak[kk], d[2 * u], d[2 * u + 1]);
+            mma_exact<NT>(U[n + u], Ul[n + u], aq, b[2 * u], b[2 * u + 1]);
+            mma_exact<NT>(U[n + u], Ul[n + u], ak, d[2 * u], d[2 * u + 1]);
           }
         }
-        join(U, Ul);
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) dSt[n + u][e] = fmaf(dSt[n + u][e], el, U[u][e]);
       }
+      join(U, Ul);
+#pragma unroll
+      for (int n = 0; n < NB; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) dSt[n][e] = fmaf(dSt[n][e], el, U[n][e]);
+      ring.done(it, lane);
+      strip_sync(strip);                        // all have read both parts
+      share_state<NT>(part0, quarter, dSt);
     }
-    __syncthreads();
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");   // nothing to wait for, unless a wait gave up
 }
 
 // ---------------------------------------------------------------------------------------------------- grad
@@ -1039,14 +1129,13 @@ template <int D>
 int launch_gdr(const GdrParams& p, int T, bool grad, cudaStream_t s) {
   constexpr int PREP = PREP_TILES<D> + C * (C + 4) * 4 + 128;
   constexpr int FWD = ScanSmem<D, 2, false>::TOTAL, SAVE = ScanSmem<D, 3, true>::TOTAL;
-  constexpr int BWD = SAVE + 64 * C * 4;         // and E
   static bool cfg = false;
   cudaError_t e;
   if (!cfg) {
     if ((e = cudaFuncSetAttribute(gdr_prep_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, PREP)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(gdr_scan_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(gdr_scan_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAVE)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(gdr_scan_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(gdr_scan_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAVE)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(gdr_grad_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, GradSmem<D>::TOTAL)) != cudaSuccess)
       return (int)e;
     cfg = true;
@@ -1056,12 +1145,12 @@ int launch_gdr(const GdrParams& p, int T, bool grad, cudaStream_t s) {
   if (!grad) {
     gdr_prep_kernel<D><<<chunks, THREADS, PREP, s>>>(p);
     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-    gdr_scan_kernel<D, false><<<scans, THREADS, FWD, s>>>(p);
+    gdr_scan_kernel<D, false><<<scans, ST, FWD, s>>>(p);
     return (int)cudaGetLastError();
   }
-  gdr_scan_kernel<D, true><<<scans, THREADS, SAVE, s>>>(p);
+  gdr_scan_kernel<D, true><<<scans, ST, SAVE, s>>>(p);
   if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-  gdr_scan_bwd_kernel<D><<<scans, THREADS, BWD, s>>>(p);
+  gdr_scan_bwd_kernel<D><<<scans, ST, SAVE, s>>>(p);
   if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
   gdr_grad_kernel<D><<<chunks, GT, GradSmem<D>::TOTAL, s>>>(p);
   return (int)cudaGetLastError();
