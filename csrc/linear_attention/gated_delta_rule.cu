@@ -41,7 +41,7 @@
 // sequences 176, 308, 431 / 173, 285, 317; 8192 in one, 16 heads 636, 1120, 1338 / 562, 910, 1007.  Two warps a strip: 173, 276,
 // 307 (of the first).  No change from starting the strips apart, slower with the operands of M and P fetched before the
 // strip's barrier (162, 335, 367: registers).
-// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.24 ms (prep 0.09), backward 0.88 ms (grad 0.38).  The batched
+// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.24 ms (prep 0.09), backward 0.79 ms (grad 0.29).  The batched
 // torch evaluation of the rule was most of a 29.5 ms block.
 #include "../common/host_utils.cuh"
 #include "warp_mma.cuh"
@@ -852,13 +852,21 @@ gdr_scan_bwd_kernel(const GdrParams p) {
 }
 
 // ---------------------------------------------------------------------------------------------------- grad
-// dq, dk, dg, dbeta of one chunk.  Rows = tokens; two warps share 16 of them, each with half of the d columns of dq and dk
-// (both form the 16 x 16 blocks of dP and dL: a fifth more MMAs, yet 387 -> 363 us against one warp per 16 rows, whose
-// chains waited for themselves; what bounds it is the rate of the warp-level MMAs and the unoverlapped load of 320 KB a
-// chunk).  S^T and dS'^T pass through shared memory 32 columns per half at a time; everything else the chunk needs is
-// resident.  V, B and the states enter as two bf16 terms: dq and dk are rounded to bf16.  dg and dbeta are put together from
-// the scans' dot products and <S', dS'>, in fp32.
-constexpr int GT = 256;
+// dq, dk, dg, dbeta of one chunk.  Rows = tokens, 16 to a warp:
+//
+//   F = do S^T   E = B S^T   H = V dS'^T   dP = scale (do V^T) D   dA = -(B V^T) D  (on and below / below the diagonal)
+//   dq = scale exp(G) F + dP k      dk = exp(G_last - G) H - exp(G) E + dA k + dP^T q + dA^T k
+//
+// dP and dA are formed first, each 16 x 16 block once, and kept as two terms in shared memory, where they are read as they are and
+// transposed.  Then four warps share 16 tokens: two halves of the d columns, 32 columns at a time, and for each one warp for
+// F, E and dq and one for H and dk, which takes E from the other.  S^T and dS'^T are read 32 columns per half at a time,
+// the first while dP and dA are formed; everything else the chunk needs is resident.  V, B and the states enter as two bf16 terms: dq
+// and dk are rounded to bf16.  dg and dbeta are put together from the scans' dot products and <S', dS'>, in fp32.
+// Bound: 6200 warp-level MMAs a chunk (6.6 us) and 320 KB.
+// With two warps to 16 tokens, each forming the blocks of dP and dA it needs in both orientations (8600 MMAs), us, before / now: 4096
+// tokens, 32 heads of 128 381 / 293, in 64 sequences 500 / 383; of 64 134 / 131.  What is left is the phases of a lone CTA
+// (the MMAs take a third of the time): states on their way to the L2 a wave of CTAs ahead gave 1 to 4 %, and cost 2 % at 64.
+constexpr int GT = 512;
 
 template <int D>
 struct GradSmem {
@@ -867,7 +875,10 @@ struct GradSmem {
   static constexpr int VT = 3 * TILE, YT = 5 * TILE;                        // V^T, B^T: two terms of [D][64] each
   static constexpr int ST = 7 * TILE;                                       // per half: S^T, dS'^T, two terms of [D][32] each
   static constexpr int STRIP = D * 32 * 2;
-  static constexpr int TOTAL = ST + 2 * 4 * STRIP + 128;
+  static constexpr int DP = ST + 2 * 4 * STRIP, DA = DP + 2 * SQ;           // two terms of [64][64] each
+  static constexpr int E = DA + 2 * SQ;                                     // 8 warps: 16 x 32 fp32
+  static constexpr int TOTAL = E + 8 * 2048 + 128;
+  static_assert(TOTAL + 1024 <= 232448, "shared memory");
 };
 
 // four neighbouring columns of a tile, as two bf16 terms
@@ -881,34 +892,133 @@ __device__ __forceinline__ void put4(uint32_t hi, uint32_t lo, int r, int c, con
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(tile_addr<D>(lo, r, c & ~7) + off), "r"(b[0]), "r"(b[1]) : "memory");
 }
 
-// Columns col0 .. col0 + 31 of S and dS' of this chunk -> tiles; returns this thread's share of <S', dS'> (`next`: S' of this
-// chunk, null behind the sequence's last one, whose dS' is zero).  128 threads.
+// 32 columns per half of S and dS' of this chunk, and of S' (null behind the sequence's last chunk, whose dS' is zero)
 template <int D>
-__device__ __forceinline__ float load_strips(uint32_t st, const float* S, const float* dS, const float* next, int col0) {
-  float dot = 0.f;
-#pragma unroll 4
-  for (int id = threadIdx.x & 127; id < D * 8; id += 128) {
-    const int r = id >> 3, c = (id & 7) * 4;
-    const long long at = (long long)r * D + col0 + c;
-    const float4 x = *reinterpret_cast<const float4*>(S + at), y = *reinterpret_cast<const float4*>(dS + at);
-    const float4 z = next ? *reinterpret_cast<const float4*>(next + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-    put4<32>(st, st + GradSmem<D>::STRIP, r, c, x);
-    put4<32>(st + 2 * GradSmem<D>::STRIP, st + 3 * GradSmem<D>::STRIP, r, c, y);
-    dot += (y.x * z.x + y.y * z.y) + (y.z * z.z + y.w * z.w);
+struct Strips {
+  static constexpr int N = D * 16 / GT;
+  float4 x[N], y[N], z[N];
+  __device__ __forceinline__ void at(int i, int& half, int& r, int& c) const {
+    const int id = threadIdx.x + i * GT;
+    half = id / (D * 8);
+    r = (id >> 3) % D;
+    c = (id & 7) * 4;
   }
-  return dot;
+  __device__ __forceinline__ void fetch(const float* S, const float* dS, const float* next, int w) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      int half, r, c;
+      at(i, half, r, c);
+      const long long o = (long long)r * D + half * (D / 2) + w * 32 + c;
+      x[i] = *reinterpret_cast<const float4*>(S + o);
+      y[i] = *reinterpret_cast<const float4*>(dS + o);
+      z[i] = next ? *reinterpret_cast<const float4*>(next + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  // -> tiles; returns this thread's share of <S', dS'>
+  __device__ __forceinline__ float put(uint32_t tiles) const {
+    constexpr int STRIP = GradSmem<D>::STRIP;
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      int half, r, c;
+      at(i, half, r, c);
+      const uint32_t st = tiles + half * 4 * STRIP;
+      put4<32>(st, st + STRIP, r, c, x[i]);
+      put4<32>(st + 2 * STRIP, st + 3 * STRIP, r, c, y[i]);
+      dot += (y[i].x * z[i].x + y[i].y * z[i].y) + (y[i].z * z[i].z + y[i].w * z[i].w);
+    }
+    return dot;
+  }
+};
+
+// block (rb, cb) of dP (B false) or dA -> two terms of its tile
+template <int D, bool B>
+__device__ __forceinline__ void pair_block(uint32_t base, int rb, int cb, const float* s_gh, const float* s_gl, float scale, int lane) {
+  using L = GradSmem<D>;
+  float d[2][4] = {};
+#pragma unroll 2
+  for (int kk = 0; kk < D; kk += 16) {
+    uint32_t vh[4], vl[4];
+    load_b_nn<64>(base + L::VT, kk, cb * 16, lane, vh);
+    load_b_nn<64>(base + L::VT + L::TILE, kk, cb * 16, lane, vl);
+    if (B) {
+      uint32_t yh[4], yl[4];
+      load_a_t<64>(base + L::YT, rb * 16, kk, lane, yh);
+      load_a_t<64>(base + L::YT + L::TILE, rb * 16, kk, lane, yl);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(d[u], yh, vh[2 * u], vh[2 * u + 1]);
+        mma16816(d[u], yl, vh[2 * u], vh[2 * u + 1]);
+        mma16816(d[u], yh, vl[2 * u], vl[2 * u + 1]);
+      }
+    } else {
+      uint32_t a[4];
+      load_a<D>(base + L::DO, rb * 16, kk, lane, a);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(d[u], a, vh[2 * u], vh[2 * u + 1]);
+        mma16816(d[u], a, vl[2 * u], vl[2 * u + 1]);
+      }
+    }
+  }
+  const uint32_t tile = base + (B ? L::DA : L::DP);
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = rb * 16 + (lane >> 2) + 8 * r, j = cb * 16 + n * 8 + (lane & 3) * 2;
+      float x[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const bool in = B ? j + e < i : j + e <= i;
+        const float D_ = in ? expf((s_gh[i] - s_gh[j + e]) + (s_gl[i] - s_gl[j + e])) : 0.f;
+        x[e] = B ? (in ? -d[n][2 * r + e] * D_ : 0.f) : d[n][2 * r + e] * (scale * D_);
+      }
+      uint32_t hi, lo;
+      split2(x[0], x[1], hi, lo);
+      const uint32_t at = tile_addr<64>(tile, i, j & ~7) + (lane & 3) * 4;
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(hi) : "memory");
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + SQ), "r"(lo) : "memory");
+    }
+}
+
+// out += X Y for 16 rows r0 of X (two terms of [64][64], TRANS: its transpose) and 32 columns c0 of the token tile Y, over the
+// 16 x 16 blocks k0 .. k1 - 1
+template <int D, bool TRANS>
+__device__ __forceinline__ void add_pairs(float (&out)[4][4], uint32_t x, uint32_t y, int r0, int c0, int k0, int k1, int lane) {
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    uint32_t xh[4], xl[4];
+    if (TRANS) {
+      load_a_t<64>(x, r0, k * 16, lane, xh);
+      load_a_t<64>(x + SQ, r0, k * 16, lane, xl);
+    } else {
+      load_a<64>(x, r0, k * 16, lane, xh);
+      load_a<64>(x + SQ, r0, k * 16, lane, xl);
+    }
+#pragma unroll
+    for (int n = 0; n < 4; n += 2) {
+      uint32_t b[4];
+      load_b_nn<D>(y, k * 16, c0 + n * 8, lane, b);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma16816(out[n + u], xh, b[2 * u], b[2 * u + 1]);
+        mma16816(out[n + u], xl, b[2 * u], b[2 * u + 1]);
+      }
+    }
+  }
 }
 
 template <int D>
-__global__ void __launch_bounds__(GT)
+__global__ void __launch_bounds__(GT, 1)
 gdr_grad_kernel(const GdrParams p) {
   using L = GradSmem<D>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ ChunkPos slot;
   __shared__ float s_gh[C], s_gl[C], s_red[GT / 32];
-  constexpr int NW = D / 64, NT = D / 16;      // strips and 8-column blocks of a half
+  constexpr int NW = D / 64;                   // strips of a half
   const uint32_t base = (smem_u32(smem_raw) + 127) & ~127u;
-  const int warp = (threadIdx.x >> 5) & 3, half = threadIdx.x >> 7, lane = threadIdx.x & 31, h = blockIdx.y;
+  const int lane = threadIdx.x & 31, id = warp_uniform(threadIdx.x >> 5), warp = id & 3, half = (id >> 2) & 1, h = blockIdx.y;
   const ChunkPos pos = locate(p, &slot);
   if (pos.seq < 0) return;
   const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
@@ -917,8 +1027,8 @@ gdr_grad_kernel(const GdrParams p) {
   load_tile<D, C, GT>(base + L::Q, p.q + off, stride, len);
   load_tile<D, C, GT>(base + L::K, p.k + off, stride, len);
   load_tile<D, C, GT>(base + L::DO, p.dout + off, stride, len);
-  for (int id = threadIdx.x; id < 4 * D * 8; id += GT) {
-    const int m = id / (D * 8), r = (id / 8) % D, c = (id & 7) * 8;
+  for (int i = threadIdx.x; i < 4 * D * 8; i += GT) {
+    const int m = i / (D * 8), r = (i / 8) % D, c = (i & 7) * 8;
     const __nv_bfloat16* src = (m < 2 ? p.V : p.B) + ch * 2 * D * C + (m & 1) * D * C + r * C + c;
     cp_async16(tile_addr<64>(base + L::VT + m * L::TILE, r, c), src, 16);
   }
@@ -931,164 +1041,116 @@ gdr_grad_kernel(const GdrParams p) {
   const float *S = p.S + ch * D * D, *dS = p.dS + ch * D * D;
   const bool more = t + C < pos.t1 && blockIdx.x + 1 < gridDim.x;   // (the latter: overlapping sequences)
   const float* next = more ? S + (long long)p.H * D * D : nullptr;
-  const int c0 = half * (D / 2);               // first column of this warp's half
-  const uint32_t st = base + L::ST + half * 4 * L::STRIP;
+  Strips<D> strips;
+  strips.fetch(S, dS, next, 0);
   const int r0 = warp * 16, i = r0 + (lane >> 2), c2 = (lane & 3) * 2;
-  float dq[NT][4], dk[NT][4], tot = 0.f;
   const float eg[2] = {gb[G_EXP * C + i], gb[G_EXP * C + i + 8]}, el[2] = {gb[G_REST * C + i], gb[G_REST * C + i + 8]};
+  cp_async_wait<0>();
+  __syncthreads();
+  {
+    // ten blocks of dA (48 MMAs) and ten of dP (32): one of dA, or one or two of dP to a warp
+    auto row_of = [](int b) { return b >= 6 ? 3 : b >= 3 ? 2 : b >= 1 ? 1 : 0; };
+    if (id < 10) {
+      const int rb = row_of(id);
+      pair_block<D, true>(base, rb, id - rb * (rb + 1) / 2, s_gh, s_gl, p.scale, lane);
+    } else {
+#pragma unroll 1
+      for (int b = id - 10; b < 10; b += 6) {
+        const int rb = row_of(b);
+        pair_block<D, false>(base, rb, b - rb * (rb + 1) / 2, s_gh, s_gl, p.scale, lane);
+      }
+    }
+  }
+  float tot = strips.put(base + L::ST);
+  __syncthreads();
+  const uint32_t st = base + L::ST + half * 4 * L::STRIP, ex = base + L::E + (id & 7) * 2048 + lane * 16;
 #pragma unroll
   for (int w = 0; w < NW; ++w) {
-    tot += load_strips<D>(st, S, dS, next, c0 + w * 32);
-    cp_async_wait<0>();
-    __syncthreads();
-    float F[4][4] = {}, E[4][4] = {}, Hh[4][4] = {};
+    if (w + 1 < NW) strips.fetch(S, dS, next, w + 1);
+    const int c0 = half * (D / 2) + w * 32;
+    float out[4][4] = {};
+    __nv_bfloat16* dst;
+    if (id < 8) {
+      float E[4][4] = {};
 #pragma unroll 1
-    for (int kk = 0; kk < D; kk += 16) {        // contraction over the columns of v
-      uint32_t a[4], yh[4], yl[4], vh[4], vl[4];
-      load_a<D>(base + L::DO, r0, kk, lane, a);
-      load_a_t<64>(base + L::YT, r0, kk, lane, yh);
-      load_a_t<64>(base + L::YT + L::TILE, r0, kk, lane, yl);
-      load_a_t<64>(base + L::VT, r0, kk, lane, vh);
-      load_a_t<64>(base + L::VT + L::TILE, r0, kk, lane, vl);
+      for (int kk = 0; kk < D; kk += 16) {      // contraction over the columns of v
+        uint32_t a[4], yh[4], yl[4];
+        load_a<D>(base + L::DO, r0, kk, lane, a);
+        load_a_t<64>(base + L::YT, r0, kk, lane, yh);
+        load_a_t<64>(base + L::YT + L::TILE, r0, kk, lane, yl);
 #pragma unroll
-      for (int n = 0; n < 4; n += 2) {
-        uint32_t b[4], d[4];
-        load_b_nn<32>(st, kk, n * 8, lane, b);
-        load_b_nn<32>(st + L::STRIP, kk, n * 8, lane, d);
+        for (int n = 0; n < 4; n += 2) {
+          uint32_t b[4], d[4];
+          load_b_nn<32>(st, kk, n * 8, lane, b);
+          load_b_nn<32>(st + L::STRIP, kk, n * 8, lane, d);
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          mma16816(F[n + u], a, b[2 * u], b[2 * u + 1]);
-          mma16816(E[n + u], yh, b[2 * u], b[2 * u + 1]);
-          mma16816(F[n + u], a, d[2 * u], d[2 * u + 1]);
-          mma16816(E[n + u], yl, b[2 * u], b[2 * u + 1]);
-          mma16816(E[n + u], yh, d[2 * u], d[2 * u + 1]);
-        }
-        load_b_nn<32>(st + 2 * L::STRIP, kk, n * 8, lane, b);
-        load_b_nn<32>(st + 3 * L::STRIP, kk, n * 8, lane, d);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          mma16816(Hh[n + u], vh, b[2 * u], b[2 * u + 1]);
-          mma16816(Hh[n + u], vl, b[2 * u], b[2 * u + 1]);
-          mma16816(Hh[n + u], vh, d[2 * u], d[2 * u + 1]);
+          for (int u = 0; u < 2; ++u) {
+            mma16816(out[n + u], a, b[2 * u], b[2 * u + 1]);
+            mma16816(E[n + u], yh, b[2 * u], b[2 * u + 1]);
+            mma16816(out[n + u], a, d[2 * u], d[2 * u + 1]);
+            mma16816(E[n + u], yl, b[2 * u], b[2 * u + 1]);
+            mma16816(E[n + u], yh, d[2 * u], d[2 * u + 1]);
+          }
         }
       }
-    }
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
+      for (int n = 0; n < 4; ++n) {
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ex + n * 512), "f"(E[n][0]), "f"(E[n][1]), "f"(E[n][2]),
+                     "f"(E[n][3]) : "memory");
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        dq[w * 4 + n][e] = p.scale * eg[e >> 1] * F[n][e];
-        dk[w * 4 + n][e] = el[e >> 1] * Hh[n][e] - eg[e >> 1] * E[n][e];
+        for (int e = 0; e < 4; ++e) out[n][e] *= p.scale * eg[e >> 1];
       }
-    }
-    __syncthreads();
-  }
-  const float gh[2] = {s_gh[i], s_gh[i + 8]}, gl[2] = {s_gl[i], s_gl[i + 8]};
-  // rows i, columns j <= i
+      add_pairs<D, false>(out, base + L::DP, base + L::K, r0, c0, 0, warp + 1, lane);
+      dst = p.dq;
+    } else {
 #pragma unroll 1
-  for (int jb = 0; jb <= warp; ++jb) {
-    float dP[2][4] = {}, dA[2][4] = {};
-#pragma unroll 1
-    for (int kk = 0; kk < D; kk += 16) {
-      uint32_t a[4], yh[4], yl[4], b[4], d[4];
-      load_a<D>(base + L::DO, r0, kk, lane, a);
-      load_a_t<64>(base + L::YT, r0, kk, lane, yh);
-      load_a_t<64>(base + L::YT + L::TILE, r0, kk, lane, yl);
-      load_b_nn<64>(base + L::VT, kk, jb * 16, lane, b);
-      load_b_nn<64>(base + L::VT + L::TILE, kk, jb * 16, lane, d);
+      for (int kk = 0; kk < D; kk += 16) {
+        uint32_t vh[4], vl[4];
+        load_a_t<64>(base + L::VT, r0, kk, lane, vh);
+        load_a_t<64>(base + L::VT + L::TILE, r0, kk, lane, vl);
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        mma16816(dP[u], a, b[2 * u], b[2 * u + 1]);
-        mma16816(dA[u], yh, b[2 * u], b[2 * u + 1]);
-        mma16816(dP[u], a, d[2 * u], d[2 * u + 1]);
-        mma16816(dA[u], yl, b[2 * u], b[2 * u + 1]);
-        mma16816(dA[u], yh, d[2 * u], d[2 * u + 1]);
+        for (int n = 0; n < 4; n += 2) {
+          uint32_t b[4], d[4];
+          load_b_nn<32>(st + 2 * L::STRIP, kk, n * 8, lane, b);
+          load_b_nn<32>(st + 3 * L::STRIP, kk, n * 8, lane, d);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            mma16816(out[n + u], vh, b[2 * u], b[2 * u + 1]);
+            mma16816(out[n + u], vl, b[2 * u], b[2 * u + 1]);
+            mma16816(out[n + u], vh, d[2 * u], d[2 * u + 1]);
+          }
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) out[n][e] *= el[e >> 1];
+      add_pairs<D, false>(out, base + L::DA, base + L::K, r0, c0, 0, warp + 1, lane);
+      add_pairs<D, true>(out, base + L::DP, base + L::Q, r0, c0, warp, 4, lane);
+      add_pairs<D, true>(out, base + L::DA, base + L::K, r0, c0, warp, 4, lane);
+      dst = p.dk;
+    }
+    __syncthreads();                            // E is there; the strips have been read
+    if (id >= 8) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        float E[4];
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(E[0]), "=f"(E[1]), "=f"(E[2]), "=f"(E[3]) : "r"(ex + n * 512) : "memory");
+#pragma unroll
+        for (int e = 0; e < 4; ++e) out[n][e] = fmaf(-eg[e >> 1], E[e], out[n][e]);
       }
     }
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
+    for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = e >> 1, ii = i + 8 * r, jj = jb * 16 + n * 8 + c2 + (e & 1);
-        const float D_ = jj <= ii ? expf((gh[r] - s_gh[jj]) + (gl[r] - s_gl[jj])) : 0.f;
-        dP[n][e] *= p.scale * D_;                                   // d(q k^T)_ij
-        dA[n][e] = jj < ii ? -dA[n][e] * D_ : 0.f;                  // d(k k^T)_ij
-      }
-    uint32_t xh[4], xl[4], yh[4], yl[4];
-    acc_to_a(dP[0], dP[1], xh, xl);
-    acc_to_a(dA[0], dA[1], yh, yl);
-#pragma unroll
-    for (int n = 0; n < NT; n += 2) {
-      uint32_t b[4];
-      load_b_nn<D>(base + L::K, jb * 16, c0 + n * 8, lane, b);
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        mma16816(dq[n + u], xh, b[2 * u], b[2 * u + 1]);
-        mma16816(dk[n + u], yh, b[2 * u], b[2 * u + 1]);
-        mma16816(dq[n + u], xl, b[2 * u], b[2 * u + 1]);
-        mma16816(dk[n + u], yl, b[2 * u], b[2 * u + 1]);
-      }
-    }
-  }
-  // the same pairs seen from their column: rows j (this warp's tokens), columns i >= j
-#pragma unroll 1
-  for (int ib = warp; ib < 4; ++ib) {
-    float dP[2][4] = {}, dA[2][4] = {};
-#pragma unroll 1
-    for (int kk = 0; kk < D; kk += 16) {
-      uint32_t vh[4], vl[4], b[4], d[4];
-      load_a_t<64>(base + L::VT, r0, kk, lane, vh);
-      load_a_t<64>(base + L::VT + L::TILE, r0, kk, lane, vl);
-      load_b_nt<D>(base + L::DO, ib * 16, kk, lane, b);
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        mma16816(dP[u], vh, b[2 * u], b[2 * u + 1]);
-        mma16816(dP[u], vl, b[2 * u], b[2 * u + 1]);
-      }
-      load_b_nn<64>(base + L::YT, kk, ib * 16, lane, b);
-      load_b_nn<64>(base + L::YT + L::TILE, kk, ib * 16, lane, d);
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        mma16816(dA[u], vh, b[2 * u], b[2 * u + 1]);
-        mma16816(dA[u], vl, b[2 * u], b[2 * u + 1]);
-        mma16816(dA[u], vh, d[2 * u], d[2 * u + 1]);
-      }
-    }
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = e >> 1, jj = i + 8 * r, ii = ib * 16 + n * 8 + c2 + (e & 1);
-        const float D_ = jj <= ii ? expf((s_gh[ii] - gh[r]) + (s_gl[ii] - gl[r])) : 0.f;
-        dP[n][e] *= p.scale * D_;
-        dA[n][e] = jj < ii ? -dA[n][e] * D_ : 0.f;
-      }
-    uint32_t xh[4], xl[4], yh[4], yl[4];
-    acc_to_a(dP[0], dP[1], xh, xl);
-    acc_to_a(dA[0], dA[1], yh, yl);
-#pragma unroll
-    for (int n = 0; n < NT; n += 2) {
-      uint32_t b[4], d[4];
-      load_b_nn<D>(base + L::Q, ib * 16, c0 + n * 8, lane, b);
-      load_b_nn<D>(base + L::K, ib * 16, c0 + n * 8, lane, d);
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        mma16816(dk[n + u], xh, b[2 * u], b[2 * u + 1]);
-        mma16816(dk[n + u], xl, b[2 * u], b[2 * u + 1]);
-        mma16816(dk[n + u], yh, d[2 * u], d[2 * u + 1]);
-        mma16816(dk[n + u], yl, d[2 * u], d[2 * u + 1]);
-      }
+      for (int r = 0; r < 2; ++r)
+        if (i + 8 * r < len)
+          *reinterpret_cast<uint32_t*>(dst + off + (i + 8 * r) * stride + c0 + n * 8 + c2) = pack_bf16x2(out[n][2 * r], out[n][2 * r + 1]);
+    if (w + 1 < NW) {
+      tot += strips.put(base + L::ST);
+      __syncthreads();
     }
   }
-#pragma unroll
-  for (int n = 0; n < NT; ++n)
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-      if (i + 8 * r < len) {
-        const long long at = off + (i + 8 * r) * stride + c0 + n * 8 + c2;
-        *reinterpret_cast<uint32_t*>(p.dq + at) = pack_bf16x2(dq[n][2 * r], dq[n][2 * r + 1]);
-        *reinterpret_cast<uint32_t*>(p.dk + at) = pack_bf16x2(dk[n][2 * r], dk[n][2 * r + 1]);
-      }
 #pragma unroll
   for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   if (lane == 0) s_red[threadIdx.x >> 5] = tot;
