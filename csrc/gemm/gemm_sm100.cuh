@@ -20,6 +20,7 @@
 // 225 / 204, 64-wide 528 / 380 / 271, CTA pairs 185 / 171 / 171; 776 x 2048 x 12288 63 / 46 / 42, with B MN-major 63 / 53 / 39;
 // 512 x 512 x 4096 both MN-major 23 / 21 / 13.
 #pragma once
+#include <type_traits>
 #include "../common/ce_math.cuh"
 #include "../common/ptx.cuh"
 
@@ -132,7 +133,8 @@ constexpr int EPI_STAGE_BYTES = 4 * EPI_STAGE_WARP;
 // With `res` (a row is `ldr` elements, 16-byte boundaries as C) C = bf16(bf16(...) + res): the lanes read the 16 bytes they write
 // from there before they wait for the accumulators.  us, the product, with an addition of its own, with `res`: 8192 x 4096 x 4096
 // 174, 204, 188; x 12288 548, 575, 558; 773 x 2048 x 6144 35, 43, 39; 201 x 256 x 256 10.4, 15.5, 10.6.
-template <int BN, int WIDE = 64>
+// (RES: as a run-time question it cost the products without one up to 12 %, the expert weight gradients above 480 -> 538 us.)
+template <int BN, int WIDE = 64, bool RES = false>
 __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* stage, __nv_bfloat16* C, long long ldc, int row0,
                                                     int m_limit, int n0, int N, float alpha, const __nv_bfloat16* bias,
                                                     const __nv_bfloat16* res = nullptr, long long ldr = 0) {
@@ -145,8 +147,8 @@ __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* 
   for (int cc = 0; cc < BN; cc += WIDE) {
     if (n0 + cc >= N) break;
     const int j = lane % CH, col = n0 + cc + 8 * j;
-    uint4 add[CH];
-    if (res) {
+    uint4 add[RES ? CH : 1];
+    if constexpr (RES) {
 #pragma unroll
       for (int it = 0; it < CH; ++it) {
         const int rr = it * (32 / CH) + lane / CH;
@@ -179,7 +181,7 @@ __device__ __forceinline__ void epilogue_store_bf16(uint32_t tmem_row, uint8_t* 
     for (int it = 0; it < CH; ++it) {
       const int rr = it * (32 / CH) + lane / CH;
       uint4 o = *reinterpret_cast<const uint4*>(at(rr, j));
-      if (res) {
+      if constexpr (RES) {
         __nv_bfloat162 *x = reinterpret_cast<__nv_bfloat162*>(&o);
         const __nv_bfloat162* y = reinterpret_cast<const __nv_bfloat162*>(&add[it]);
 #pragma unroll
@@ -357,6 +359,7 @@ template <int BN, bool A_MN, bool B_MN, int EPI = EPI_NONE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                        const GemmParams p) {
+  constexpr bool MAY_ADD = !A_MN && !B_MN && EPI == EPI_NONE;   // the host gives `res` to these only
   using L = GemmSmem<BN>;
   constexpr int STAGES = L::STAGES;
   constexpr uint32_t TMEM_COLS = (2 * BN < 32) ? 32 : 2 * BN;  // two accumulators
@@ -537,10 +540,13 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
       if (!p.c_fp32 && !p.accumulate && vec_ok && has_acc && p.N % 8 == 0) {
         const long long gbase = p.mode == GEMM_GROUPED_K ? (long long)c.group * p.c_group_stride : 0ll;
-        epilogue_store_bf16<BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * BN,
-                                smem + STAGES * L::STAGE_BYTES + L::BAR_BYTES + q * EPI_STAGE_WARP,
-                                reinterpret_cast<__nv_bfloat16*>(p.C) + gbase, p.ldc, c.m0 + q * 32, c.m_limit, c.n0, p.N,
-                                p.alpha, bias, p.res, p.ldr);
+        auto store = [&](auto with_res) {
+          epilogue_store_bf16<BN, 64, decltype(with_res)::value>(
+              tmem_base + (uint32_t(q * 32) << 16) + acc * BN, smem + STAGES * L::STAGE_BYTES + L::BAR_BYTES + q * EPI_STAGE_WARP,
+              reinterpret_cast<__nv_bfloat16*>(p.C) + gbase, p.ldc, c.m0 + q * 32, c.m_limit, c.n0, p.N, p.alpha, bias, p.res, p.ldr);
+        };
+        if (MAY_ADD && p.res) store(std::true_type{});
+        else store(std::false_type{});
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

@@ -32,6 +32,7 @@ template <bool A_MN, bool B_MN, int EPI = EPI_NONE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const GemmParams p) {
+  constexpr bool MAY_ADD = !A_MN && !B_MN && EPI == EPI_NONE;   // the host gives `res` to these only
   constexpr int STAGES = PAIR_STAGES;
   constexpr uint32_t TMEM_COLS = 2 * PAIR_BN;  // two accumulators of 256 columns
   extern __shared__ uint8_t smem_raw[];
@@ -206,9 +207,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
       const bool vec_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
       if (!p.c_fp32 && !p.accumulate && vec_ok && p.N % 8 == 0) {
-        epilogue_store_bf16<PAIR_BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * PAIR_BN,
-                                     smem + STAGES * PAIR_STAGE_BYTES + 1024 + q * EPI_STAGE_WARP,
-                                     reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, row - lane, p.M, n0, p.N, p.alpha, bias, p.res, p.ldr);
+        auto store = [&](auto with_res) {
+          epilogue_store_bf16<PAIR_BN, 64, decltype(with_res)::value>(
+              tmem_base + (uint32_t(q * 32) << 16) + acc * PAIR_BN, smem + STAGES * PAIR_STAGE_BYTES + 1024 + q * EPI_STAGE_WARP,
+              reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, row - lane, p.M, n0, p.N, p.alpha, bias, p.res, p.ldr);
+        };
+        if (MAY_ADD && p.res) store(std::true_type{});
+        else store(std::false_type{});
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(acc ? tempty_leader1 : tempty_leader0);
