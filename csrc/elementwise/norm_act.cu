@@ -138,11 +138,15 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
 }
 
 // `y` (optional, may be `dy`: a thread reads its part of dy first) receives the forward's result, x * rstd * w_eff, which
-// costs a write here and a read, a write and a launch as a forward pass of its own: 8192 x 4096 82 instead of 70 + 34 us.
-// `dres` (RES) is added to the rounded gradient, to the bits of a sum of its own: 8192 x 4096 101 us instead of 93 and 130 with
-// the sum, 1024 x 256 14.6 instead of 13.6 and 17.8.  Rows of more than 8192 have no registers for it and are added to.
-template <int VPT, bool RES>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* dy, __nv_bfloat16* y,
+// costs a write here and a read, a write and a launch as a forward pass of its own: 8192 x 4096 56 instead of 52 + 34 us.
+// `dres` (RES) is added to the rounded gradient, to the bits of a sum of its own: 8192 x 4096 73 us with y, 56 without it
+// and 36 for a sum of its own.  Rows of more than 8192 have no registers for it and are added to.
+// RING: a CTA that has more than one pair of rows copies the next pair to shared memory (each thread what it will read itself)
+// while it works on one; two CTAs or one on an SM, as registers allow, otherwise leave the memory idle between their loads.
+// us, registers only (VPT 2: one of the two CTAs resident) / now: 8192 x 4096 79 / 52, with y 87 / 56, with dres 88 / 69, with both
+// 95 / 73 (4.6 TB/s); 16384 x 1024 69 / 44; 4096 x 8192 64 / 58.  One pair a CTA, and H > 8192: as before.
+template <int VPT, bool RES, bool RING>
+__global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1) rmsnorm_bwd_kernel(const __nv_bfloat16* dy, __nv_bfloat16* y,
                                    const __nv_bfloat16* __restrict__ x,
                                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
@@ -167,19 +171,46 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* d
       }
     }
   }
-  for (long long row0 = 2LL * blockIdx.x; row0 < rows; row0 += 2LL * gridDim.x) {
+  constexpr int NQ = RES ? 3 : 2;
+  extern __shared__ __align__(16) uint8_t ring[];              // [2 stages][NQ][2 rows][nvec] vectors
+  uint4* const own = reinterpret_cast<uint4*>(ring) + threadIdx.x;
+  auto slot = [&](int stage, int q, int r, int i) { return own + ((stage * NQ + q) * 2 + r) * nvec + i * (int)blockDim.x; };
+  auto source = [&](int q, long long row) {
+    return reinterpret_cast<const uint4*>(q == 0 ? x + row * ldx : (q == 1 ? dy : dres) + row * (long long)H) + threadIdx.x;
+  };
+  auto copy = [&](long long row0, int stage) {
+    if (row0 < rows) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          const uint4* src = source(q, min(row0 + r, rows - 1));
+#pragma unroll
+          for (int i = 0; i < VPT; ++i)
+            if ((int)threadIdx.x + i * (int)blockDim.x < nvec)
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(slot(stage, q, r, i))), "l"(src + i * blockDim.x) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if constexpr (RING) copy(2LL * blockIdx.x, 0);
+  int stage = 0;
+  for (long long row0 = 2LL * blockIdx.x; row0 < rows; row0 += 2LL * gridDim.x, stage ^= 1) {
     const bool two = row0 + 1 < rows;
     uint4 xr[2][VPT], gr[2][VPT], dr[2][RES ? VPT : 1];
+    if constexpr (RING) {
+      copy(row0 + 2LL * gridDim.x, stage ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const long long row = row0 + ((r == 1 && two) ? 1 : 0);
 #pragma unroll
       for (int i = 0; i < VPT; ++i) {
-        const int vi = threadIdx.x + i * blockDim.x;
-        if (vi < nvec) {
-          xr[r][i] = reinterpret_cast<const uint4*>(x + row * ldx)[vi];
-          gr[r][i] = reinterpret_cast<const uint4*>(dy + row * (long long)H)[vi];
-          if constexpr (RES) dr[r][i] = reinterpret_cast<const uint4*>(dres + row * (long long)H)[vi];
+        if ((int)threadIdx.x + i * (int)blockDim.x < nvec) {
+          xr[r][i] = RING ? *slot(stage, 0, r, i) : source(0, row)[i * blockDim.x];
+          gr[r][i] = RING ? *slot(stage, 1, r, i) : source(1, row)[i * blockDim.x];
+          if constexpr (RES) dr[r][i] = RING ? *slot(stage, 2, r, i) : source(2, row)[i * blockDim.x];
         }
       }
     }
@@ -224,8 +255,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* d
         if (vi < nvec) {
           float xv[8], gv[8], o[8];
           bf16x8 a, b;
-          a.raw = xr[r][i];
-          b.raw = gr[r][i];
+          a.raw = RING ? *slot(stage, 0, r, i) : xr[r][i];
+          b.raw = RING ? *slot(stage, 1, r, i) : gr[r][i];
           a.unpack(xv);
           b.unpack(gv);
           if (y) {
@@ -245,7 +276,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* d
           if constexpr (RES) {
             float s[8];
             bf16x8 rr;
-            rr.raw = dr[r][i];
+            rr.raw = RING ? *slot(stage, 2, r, i) : dr[r][i];
             rr.unpack(s);
             ov.unpack(o);
 #pragma unroll
@@ -305,43 +336,64 @@ __device__ __forceinline__ float act_grad(float g, int kind) {
   return 0.5f * (1.f + t) + 0.5f * g * (1.f - t * t) * k0 * (1.f + 3.f * k1 * g * g);
 }
 
-__global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ in, const float* __restrict__ probs,
-                               __nv_bfloat16* __restrict__ out, long long rows, int F, long long ld_in, int kind,
-                               float clamp, float offset) {
-  const int nvec = F / 8;
-  const long long total = rows * nvec;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long row = i / nvec;
-    const int vi = (int)(i - row * nvec);
-    bf16x8 g, u;
-    g.raw = reinterpret_cast<const uint4*>(in + row * ld_in)[vi];
-    u.raw = reinterpret_cast<const uint4*>(in + row * ld_in + F)[vi];
-    float gf[8], uf[8], o[8];
-    g.unpack(gf);
-    u.unpack(uf);
-    const float pr = probs ? probs[row] : 1.f;
+// Eight values of the forward result.  KIND and CLAMP are compile-time: as arguments they cost as many instructions as the
+// arithmetic, which took as long as the memory did.
+template <int KIND, bool CLAMP>
+__device__ __forceinline__ uint4 glu_fwd8(const uint4& graw, const uint4& uraw, float pr, float clamp, float offset) {
+  bf16x8 g, u;
+  g.raw = graw;
+  u.raw = uraw;
+  float gf[8], uf[8], o[8];
+  g.unpack(gf);
+  u.unpack(uf);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float gg = gf[j], uu = uf[j];
-      if (clamp > 0.f) {
-        gg = fminf(gg, clamp);
-        uu = fminf(fmaxf(uu, -clamp), clamp);
-      }
-      o[j] = act_fwd(gg, kind) * (uu + offset) * pr;
+  for (int j = 0; j < 8; ++j) {
+    float gg = gf[j], uu = uf[j];
+    if (CLAMP) {
+      gg = fminf(gg, clamp);
+      uu = fminf(fmaxf(uu, -clamp), clamp);
     }
-    bf16x8 ov;
-    ov.pack(o);
-    reinterpret_cast<uint4*>(out + row * (long long)F)[vi] = ov.raw;
+    o[j] = act_fwd(gg, KIND) * (uu + offset) * pr;
+  }
+  bf16x8 ov;
+  ov.pack(o);
+  return ov.raw;
+}
+
+// The row of a thread's next vector follows from the last one's, without a division.  All 64 warps of an SM resident: two vectors
+// in flight a thread and 40 warps were 3 to 12 % slower.  us, a
+// division a vector and everything an argument / now: 8192 x 12288 108 / 104 (5.8 TB/s), 16384 x 1536 32.8 / 30.7.
+template <int KIND, bool CLAMP>
+__global__ void __launch_bounds__(256, 8) glu_fwd_kernel(const __nv_bfloat16* __restrict__ in, const float* __restrict__ probs,
+                               __nv_bfloat16* __restrict__ out, long long rows, int F, long long ld_in, float clamp, float offset) {
+  const int nvec = F / 8;
+  const long long step = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long step_row = step / nvec;
+  const int step_v = (int)(step - step_row * nvec);
+  long long row = first / nvec;
+  int vi = (int)(first - row * nvec);
+  while (row < rows) {
+    const uint4* src = reinterpret_cast<const uint4*>(in + row * ld_in);
+    const uint4 g = src[vi], u = src[nvec + vi];
+    reinterpret_cast<uint4*>(out + row * (long long)F)[vi] = glu_fwd8<KIND, CLAMP>(g, u, probs ? probs[row] : 1.f, clamp, offset);
+    row += step_row;
+    vi += step_v;
+    if (vi >= nvec) {
+      vi -= nvec;
+      ++row;
+    }
   }
 }
 
 // din[rows, 2F] from dout[rows, F]; optional dprobs[row] = sum_j dout * act(g) * (u+offset); `act` (optional, may be `dout`: a
 // thread reads its part of it first) receives the forward's result, for one write instead of a forward pass over `in`.
-__global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ in, const float* __restrict__ probs,
+template <int KIND, bool CLAMP>
+__global__ void __launch_bounds__(256) glu_bwd_kernel(const __nv_bfloat16* __restrict__ in, const float* __restrict__ probs,
                                const __nv_bfloat16* dout, __nv_bfloat16* act, __nv_bfloat16* __restrict__ din,
-                               float* __restrict__ dprobs, long long rows, int F, long long ld_in, int kind,
-                               float clamp, float offset) {
-  // one warp per row, so the dprobs reduction stays inside a warp; without dprobs gridDim.y warps share a row
+                               float* __restrict__ dprobs, long long rows, int F, long long ld_in, float clamp, float offset) {
+  // one warp per row, so the dprobs reduction stays inside a warp; without dprobs gridDim.y warps share a row.  Two vectors a lane
+  // are in flight together.  us, one vector and everything an argument / now: 8192 x 12288 219 / 164 (6.1 TB/s), with `act` 244 / 197,
+  // 16384 x 1536 61 / 47, 773 x 6144 18 / 14; quick-GEGLU with probs, which needs more registers, 242 / 236.
   const int nvec = F / 8;
   const int per = (nvec + (int)gridDim.y * 32 - 1) / ((int)gridDim.y * 32) * 32;
   const int v0 = blockIdx.y * per, v1 = min(nvec, v0 + per);
@@ -351,41 +403,54 @@ __global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ in, const float
   for (long long row = warp_global; row < rows; row += nwarps) {
     const float pr = probs ? probs[row] : 1.f;
     float dp = 0.f;
-    for (int vi = v0 + lane; vi < v1; vi += 32) {
-      bf16x8 g, u, d;
-      g.raw = reinterpret_cast<const uint4*>(in + row * ld_in)[vi];
-      u.raw = reinterpret_cast<const uint4*>(in + row * ld_in + F)[vi];
-      d.raw = reinterpret_cast<const uint4*>(dout + row * (long long)F)[vi];
-      float gf[8], uf[8], df[8], dg[8], du[8], y[8];
-      g.unpack(gf);
-      u.unpack(uf);
-      d.unpack(df);
+    const uint4 *pg = reinterpret_cast<const uint4*>(in + row * ld_in), *pu = reinterpret_cast<const uint4*>(in + row * ld_in + F);
+    const uint4* pd = reinterpret_cast<const uint4*>(dout + row * (long long)F);
+    for (int vi = v0 + lane; vi < v1; vi += 64) {
+      bf16x8 g[2], u[2], d[2];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float gg = gf[j], uu = uf[j];
-        bool g_pass = true, u_pass = true;
-        if (clamp > 0.f) {
-          g_pass = gg <= clamp;
-          u_pass = (uu >= -clamp) && (uu <= clamp);
-          gg = fminf(gg, clamp);
-          uu = fminf(fmaxf(uu, -clamp), clamp);
+      for (int k = 0; k < 2; ++k) {
+        const int at = vi + 32 * k;
+        if (k == 0 || at < v1) {
+          g[k].raw = pg[at];
+          u[k].raw = pu[at];
+          d[k].raw = pd[at];
         }
-        const float a = act_fwd(gg, kind);
-        y[j] = a * (uu + offset) * pr;
-        dp += df[j] * a * (uu + offset);
-        dg[j] = g_pass ? df[j] * pr * (uu + offset) * act_grad(gg, kind) : 0.f;
-        du[j] = u_pass ? df[j] * pr * a : 0.f;
       }
-      bf16x8 og, ou;
-      og.pack(dg);
-      ou.pack(du);
-      if (act) {
-        bf16x8 oy;
-        oy.pack(y);
-        reinterpret_cast<uint4*>(act + row * (long long)F)[vi] = oy.raw;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int at = vi + 32 * k;
+        if (k > 0 && at >= v1) break;
+        float gf[8], uf[8], df[8], dg[8], du[8], y[8];
+        g[k].unpack(gf);
+        u[k].unpack(uf);
+        d[k].unpack(df);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float gg = gf[j], uu = uf[j];
+          bool g_pass = true, u_pass = true;
+          if (CLAMP) {
+            g_pass = gg <= clamp;
+            u_pass = (uu >= -clamp) && (uu <= clamp);
+            gg = fminf(gg, clamp);
+            uu = fminf(fmaxf(uu, -clamp), clamp);
+          }
+          const float a = act_fwd(gg, KIND);
+          y[j] = a * (uu + offset) * pr;
+          dp += df[j] * a * (uu + offset);
+          dg[j] = g_pass ? df[j] * pr * (uu + offset) * act_grad(gg, KIND) : 0.f;
+          du[j] = u_pass ? df[j] * pr * a : 0.f;
+        }
+        bf16x8 og, ou;
+        og.pack(dg);
+        ou.pack(du);
+        if (act) {
+          bf16x8 oy;
+          oy.pack(y);
+          reinterpret_cast<uint4*>(act + row * (long long)F)[at] = oy.raw;
+        }
+        reinterpret_cast<uint4*>(din + row * (long long)(2 * F))[at] = og.raw;
+        reinterpret_cast<uint4*>(din + row * (long long)(2 * F) + F)[at] = ou.raw;
       }
-      reinterpret_cast<uint4*>(din + row * (long long)(2 * F))[vi] = og.raw;
-      reinterpret_cast<uint4*>(din + row * (long long)(2 * F) + F)[vi] = ou.raw;
     }
     if (dprobs) {
       dp = warp_sum(dp);
@@ -393,6 +458,22 @@ __global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ in, const float
     }
   }
 }
+
+// calls f<KIND, CLAMP>
+#define MCB_GLU_KINDS(kind, clamp, F)      \
+  do {                                     \
+    const bool c_ = (clamp) > 0.f;         \
+    if ((kind) == 0) {                     \
+      if (c_) F(0, true);                  \
+      else F(0, false);                    \
+    } else if ((kind) == 1) {              \
+      if (c_) F(1, true);                  \
+      else F(1, false);                    \
+    } else {                               \
+      if (c_) F(2, true);                  \
+      else F(2, false);                    \
+    }                                      \
+  } while (0)
 
 int pick_threads(int H, int* vpt) {
   const int nvec = H / 8;
@@ -443,21 +524,33 @@ static int rmsnorm_bwd_launch(const void* dy, void* y, const void* x, const void
   if (!dw_any) partials = nullptr;
   if (dw_bf16 && !partials) return -3;
   if (dres && vpt > 4) return -4;
-#define LAUNCH(V, R)                                                                                                 \
-  rmsnorm_bwd_kernel<V, R><<<(int)grid, threads, 0, s>>>((const __nv_bfloat16*)dy, (__nv_bfloat16*)y,                    \
-                                                      (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,      \
-                                                      (__nv_bfloat16*)dx, dw, partials, rows, H, ldx, eps,            \
-                                                      zero_centered)
-  if (dres) {
-    if (vpt <= 1) LAUNCH(1, true);
-    else if (vpt <= 2) LAUNCH(2, true);
-    else LAUNCH(4, true);
-  } else {
-    if (vpt <= 1) LAUNCH(1, false);
-    else if (vpt <= 2) LAUNCH(2, false);
-    else if (vpt <= 4) LAUNCH(4, false);
-    else LAUNCH(8, false);
-  }
+  const bool ring = pairs > grid && vpt <= 4;
+#define LAUNCH(V, R, P)                                                                                              \
+  do {                                                                                                               \
+    const int smem = P ? 2 * (R ? 3 : 2) * 2 * H * 2 : 0;                                                            \
+    static bool cfg = false;                                                                                         \
+    if (P && !cfg) {                                                                                                 \
+      const cudaError_t e = cudaFuncSetAttribute(rmsnorm_bwd_kernel<V, R, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                                 2 * (R ? 3 : 2) * 2 * 2048 * V * 2);                                \
+      if (e != cudaSuccess) return (int)e;                                                                           \
+      cfg = true;                                                                                                    \
+    }                                                                                                                \
+    rmsnorm_bwd_kernel<V, R, P><<<(int)grid, threads, smem, s>>>(                                                     \
+        (const __nv_bfloat16*)dy, (__nv_bfloat16*)y, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,          \
+        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw, partials, rows, H, ldx, eps, zero_centered);             \
+  } while (0)
+#define LAUNCH_V(V)                     \
+  do {                                  \
+    if (dres && ring) LAUNCH(V, true, true);   \
+    else if (dres) LAUNCH(V, true, false);     \
+    else if (ring) LAUNCH(V, false, true);     \
+    else LAUNCH(V, false, false);              \
+  } while (0)
+  if (vpt <= 1) LAUNCH_V(1);
+  else if (vpt <= 2) LAUNCH_V(2);
+  else if (vpt <= 4) LAUNCH_V(4);
+  else LAUNCH(8, false, false);
+#undef LAUNCH_V
 #undef LAUNCH
   if (partials && dw_bf16)
     launch_reduce_partials<__nv_bfloat16>(partials, (int)grid, H, reinterpret_cast<__nv_bfloat16*>(dw_any), nullptr, H, s);
@@ -510,9 +603,11 @@ int mcb_glu_fwd(const void* in, const float* probs, void* out, long long rows, i
   long long total = rows * (F / 8);
   long long blocks = (total + 255) / 256;
   long long cap = (long long)device_sm_count() * 8;
-  glu_fwd_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, s>>>((const __nv_bfloat16*)in, probs,
-                                                                     (__nv_bfloat16*)out, rows, F, ld_in, kind, clamp,
-                                                                     offset);
+#define LAUNCH(K, C)                                                                                                     \
+  glu_fwd_kernel<K, C><<<(int)(blocks < cap ? blocks : cap), 256, 0, s>>>((const __nv_bfloat16*)in, probs, (__nv_bfloat16*)out, rows, \
+                                                                          F, ld_in, clamp, offset)
+  MCB_GLU_KINDS(kind, clamp, LAUNCH);
+#undef LAUNCH
   return (int)cudaGetLastError();
 }
 
@@ -531,8 +626,11 @@ static int glu_bwd_launch(const void* in, const float* probs, const void* dout, 
     parts = want < most ? want : most;
   }
   const dim3 grid((unsigned)(blocks < cap ? blocks : cap), (unsigned)parts);
-  glu_bwd_kernel<<<grid, 256, 0, s>>>((const __nv_bfloat16*)in, probs, (const __nv_bfloat16*)dout, (__nv_bfloat16*)act,
-                                      (__nv_bfloat16*)din, dprobs, rows, F, ld_in, kind, clamp, offset);
+#define LAUNCH(K, C)                                                                                                     \
+  glu_bwd_kernel<K, C><<<grid, 256, 0, s>>>((const __nv_bfloat16*)in, probs, (const __nv_bfloat16*)dout, (__nv_bfloat16*)act, \
+                                            (__nv_bfloat16*)din, dprobs, rows, F, ld_in, clamp, offset)
+  MCB_GLU_KINDS(kind, clamp, LAUNCH);
+#undef LAUNCH
   return (int)cudaGetLastError();
 }
 

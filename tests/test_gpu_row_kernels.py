@@ -1,0 +1,65 @@
+"""Row-wise kernels at the edges of how they walk: one vector, a pair of heads or of rows at a time, with the next in flight."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = 'cuda'
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+
+def _rand(*shape, seed=0):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    return torch.randn(*shape, generator=gen, device=DEV).bfloat16()
+
+
+@pytest.mark.parametrize('rows,F', [(1, 8), (3, 264), (33, 256), (700, 104), (5, 8192)])
+@pytest.mark.parametrize('kind,clamp,offset', [('swiglu', 0.0, 0.0), ('quick_geglu', 2.0, 1.0), ('geglu_tanh', 0.0, 0.0)])
+def test_gated_activation(rows, F, kind, clamp, offset):
+    from mcore_bridge_b200.ops.activation import glu, glu_ref
+    x, dy = _rand(rows, 2 * F), _rand(rows, F, seed=1)
+    probs = torch.rand(rows, device=DEV)
+    for pr in (None, probs):
+        leaves = [t.clone().requires_grad_() for t in (x, pr) if t is not None]
+        got = torch.autograd.grad(glu(leaves[0], kind, leaves[1] if pr is not None else None, clamp, offset), leaves, dy)
+        out = glu(x, kind, pr, clamp, offset)
+        wide = [t.detach().double().requires_grad_() for t in leaves]
+        ref = glu_ref(wide[0], kind, wide[1] if pr is not None else None, clamp, offset)
+        want = torch.autograd.grad(ref, wide, dy.double())
+        # rounded once; fp32: sums of F products, and the hardware's tanh, within 2^-11, enters g (1 + tanh) / 2
+        tanh = 2 ** -12 * (x[:, :F] * x[:, F:] * dy).double().abs().sum(-1).norm() if kind == 'geglu_tanh' else 0.0
+        for a, b in zip([out, *got], [ref, *want]):
+            assert _rel(a, b) < (2 ** -8 if a.dtype == torch.bfloat16 else 2 ** -17 + tanh / b.norm())
+
+
+@pytest.mark.parametrize('rows,H', [(593, 104), (1190, 2048), (601, 4096), (300, 8192), (1201, 1024)])
+def test_norm_backward_with_the_next_rows_in_flight(rows, H):
+    # more rows than the grid takes at once: every row has the bits it has alone, with and without the residual's gradient
+    from mcore_bridge_b200.ops import _lib
+    lib, ptr, ll = _lib.lib(), lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr()), ctypes.c_longlong
+    x, dy, res, w = _rand(rows, H), _rand(rows, H, seed=1), _rand(rows, H, seed=2), _rand(H, seed=3)
+    rstd = torch.rsqrt(x.float().pow(2).mean(-1) + 1e-6)
+
+    def backward(first, last, res, with_y):
+        n = last - first
+        part = torch.empty(lib.mcb_rmsnorm_bwd_partial_rows(ll(n), H), H, device=DEV)
+        d, dx, dw = dy[first:last].clone(), torch.empty(n, H, device=DEV, dtype=torch.bfloat16), torch.empty(H, device=DEV).bfloat16()
+        f = lib.mcb_rmsnorm_bwd_det_y if with_y else lib.mcb_rmsnorm_bwd_det
+        assert f(ptr(d), ptr(x[first:]), ptr(w), ptr(rstd[first:]), ptr(None if res is None else res[first:]), ptr(dx), ptr(dw), 1, ptr(part),
+                 ll(n), H, ll(H), ctypes.c_float(1e-6), 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        return dx, dw, d
+
+    dx, dw, _ = backward(0, rows, None, False)
+    for first, last in ((0, 1), (0, 100), (rows - 101, rows)):
+        assert torch.equal(backward(first, last, None, False)[0], dx[first:last])
+    dxr, dwr, y = backward(0, rows, res, True)
+    assert torch.equal(dxr, dx + res) and torch.equal(dwr, dw)
+    assert _rel(y, x.double() * rstd.double()[:, None] * w.double()) < 2 ** -8
+    wide = x.double().requires_grad_(), w.double().requires_grad_()
+    ref = wide[0] * torch.rsqrt(wide[0].pow(2).mean(-1, keepdim=True) + 1e-6) * wide[1]
+    for a, b in zip((dx, dw), torch.autograd.grad(ref, wide, dy.double())):
+        assert _rel(a, b) < 2 ** -8
