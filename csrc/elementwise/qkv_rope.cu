@@ -8,6 +8,7 @@
 //   for each of `ng` groups: [ qpg query heads (each optionally followed by its gate head) | k | v ], head size d.
 // cos/sin are per-token tables [T, rot/2] fp32, so positions, packing, context-parallel chunking,
 // MRoPE sections and attention scaling are all decided by whoever builds the table.
+#include <initializer_list>
 #include "../common/partials.cuh"
 #include "../common/host_utils.cuh"
 #include "../common/ptx.cuh"
@@ -18,6 +19,7 @@ namespace {
 
 constexpr int MAX_D = 256;
 constexpr int WARPS = 8;
+constexpr int FWD_CTAS = 4, BWD_CTAS = 3;   // CTAs an SM holds of the fast kernels
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -276,58 +278,142 @@ qkv_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __res
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Fast path for head size 128 with rotate-half RoPE over the whole head (the Qwen3 / Llama layout): a lane holds
-// elements {2l, 2l+1} and their rotation partners {64+2l, 65+2l}, so the head never leaves registers.
-__device__ __forceinline__ float2 ld_bf2(const __nv_bfloat16* p) {
-  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+// Fast path for head size 128 with rotate-half RoPE over the whole head (the Qwen3 / Llama layout): 16 lanes to a head, a lane holds
+// elements 4l .. 4l + 3 and their rotation partners 64 + 4l .. , so the head never leaves registers.  A warp has one pair of heads
+// and walks the tokens: what the heads are is found out once, and the next token's are loaded while it works on one.
+// us, forward and backward, before (a warp to a head, 4 bytes a lane, heads of a token in turn) / now: 8192 tokens, 32 + 8 + 8 heads
+// with norms 72, 114 / 51, 93, without 63, 75 / 51, 60; 16384, 40 + 8 + 8 131, 160 / 102, 126.  With one CTA an SM more (spills)
+// 63, 134, with one less 57, 99; two pairs in flight (spills) 78, 179.
+// WIDE: all tensors start on 8-byte boundaries.
+template <bool WIDE>
+__device__ __forceinline__ uint2 ld_bf4(const __nv_bfloat16* p) {
+  if (WIDE) return *reinterpret_cast<const uint2*>(p);
+  return make_uint2(reinterpret_cast<const uint32_t*>(p)[0], reinterpret_cast<const uint32_t*>(p)[1]);
+}
+template <bool WIDE>
+__device__ __forceinline__ void st_bf4(__nv_bfloat16* p, uint2 v) {
+  if (WIDE) {
+    *reinterpret_cast<uint2*>(p) = v;
+  } else {
+    reinterpret_cast<uint32_t*>(p)[0] = v.x;
+    reinterpret_cast<uint32_t*>(p)[1] = v.y;
+  }
+}
+__device__ __forceinline__ void unpack4(uint2 v, float (&f)[4]) {
+  const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+  const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+  f[0] = x.x;
+  f[1] = x.y;
+  f[2] = y.x;
+  f[3] = y.y;
+}
+__device__ __forceinline__ uint2 pack4(const float (&f)[4]) { return make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3])); }
+// the sum over a head's 16 lanes of x + y
+__device__ __forceinline__ float head_sum(float x, float y) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    x += __shfl_xor_sync(0xffffffffu, x, o);
+    y += __shfl_xor_sync(0xffffffffu, y, o);
+  }
+  return x + y;
+}
+// The head of a half of a warp, and the warp's walk over the tokens: first one and step.
+struct HeadWalk {
+  int at, slot, kind, head;                       // slot -1: no head
+  long long t, step;
+  __device__ __forceinline__ HeadWalk(const QkvLayout& L) {
+    const int slots = L.ng * (L.qpg * (1 + L.gate) + 2), pairs = (slots + 1) / 2;
+    const int id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;   // the host sees that
+    at = (threadIdx.x & 15) * 4;                                                                          // warps >= pairs
+    slot = 2 * (id % pairs) + ((threadIdx.x >> 4) & 1);
+    t = id / pairs;
+    step = warps / pairs;
+    if (t >= step) t = 1ll << 62;                 // the remainder of the warps
+    kind = head = 0;
+    if (slot < slots) decode_slot(L, slot, kind, head);
+    else slot = -1;
+  }
+};
+__device__ __forceinline__ void head_weights(const QkvLayout& L, const __nv_bfloat16* w, int at, float (&a)[4], float (&b)[4]) {
+  unpack4(ld_bf4<false>(w + at), a);
+  unpack4(ld_bf4<false>(w + at + 64), b);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    a[e] += L.zero_centered ? 1.f : 0.f;
+    b[e] += L.zero_centered ? 1.f : 0.f;
+  }
+}
+__device__ __forceinline__ void ld_angles(const float* __restrict__ tab, float (&f)[4]) {
+  const float2 x = reinterpret_cast<const float2*>(tab)[0], y = reinterpret_cast<const float2*>(tab)[1];
+  f[0] = x.x;
+  f[1] = x.y;
+  f[2] = y.x;
+  f[3] = y.y;
 }
 
-__global__ void __launch_bounds__(WARPS * 32)
+template <bool WIDE>
+__global__ void __launch_bounds__(WARPS * 32, FWD_CTAS)
 qkv_fwd_fast_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ wq,
                     const __nv_bfloat16* __restrict__ wk, const float* __restrict__ cosb,
                     const float* __restrict__ sinb, __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ k,
                     __nv_bfloat16* __restrict__ v, __nv_bfloat16* __restrict__ gate, long long T, QkvLayout L) {
   constexpr int D = 128;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slots = L.ng * (L.qpg * (1 + L.gate) + 2);
-  const int nq = L.ng * L.qpg;
-  const float wbase = L.zero_centered ? 1.f : 0.f;
-  float2 wqa = make_float2(1.f, 1.f), wqb = wqa, wka = wqa, wkb = wqa;
-  if (L.norm) {
-    wqa = ld_bf2(wq + 2 * lane); wqb = ld_bf2(wq + 64 + 2 * lane);
-    wka = ld_bf2(wk + 2 * lane); wkb = ld_bf2(wk + 64 + 2 * lane);
-    wqa.x += wbase; wqa.y += wbase; wqb.x += wbase; wqb.y += wbase;
-    wka.x += wbase; wka.y += wbase; wkb.x += wbase; wkb.y += wbase;
-  }
-  for (long long t = blockIdx.x; t < T; t += gridDim.x) {
-    const float2 c = *reinterpret_cast<const float2*>(cosb + t * 64 + 2 * lane);
-    const float2 sn = *reinterpret_cast<const float2*>(sinb + t * 64 + 2 * lane);
-    for (int slot = warp; slot < slots; slot += WARPS) {
-      int kind, head;
-      decode_slot(L, slot, kind, head);
-      const __nv_bfloat16* src = qkv + t * L.ld + (long long)slot * D;
-      __nv_bfloat16* dst = kind == 0 ? q + (t * nq + head) * D
-                           : kind == 1 ? gate + (t * nq + head) * D
-                           : kind == 2 ? k + (t * L.ng + head) * D
-                                       : v + (t * L.ng + head) * D;
-      if (kind == 1 || kind == 3) {
-        *reinterpret_cast<uint2*>(dst + 4 * lane) = *reinterpret_cast<const uint2*>(src + 4 * lane);
-        continue;
+  const HeadWalk h(L);
+  const int nq = L.ng * L.qpg, heads = h.kind < 2 ? nq : L.ng;
+  const bool rot = h.kind == 0 || h.kind == 2, live = h.slot >= 0;
+  float wa[4] = {}, wb[4] = {};
+  const __nv_bfloat16* src = qkv + (live ? h.slot : 0) * D + h.at;
+  __nv_bfloat16* dst = (h.kind == 0 ? q : h.kind == 1 ? gate : h.kind == 2 ? k : v) + (long long)h.head * D + h.at;
+  uint2 ra, rb;
+  float c[4], sn[4];
+  auto fetch = [&](long long t) {
+    ra = rb = make_uint2(0, 0);
+    if (t >= T) return;
+    ra = ld_bf4<WIDE>(src + t * L.ld);
+    rb = ld_bf4<WIDE>(src + t * L.ld + 64);
+    ld_angles(cosb + t * 64 + h.at, c);
+    ld_angles(sinb + t * 64 + h.at, sn);
+  };
+  fetch(h.t);
+  if (L.norm) head_weights(L, h.kind == 0 ? wq : wk, h.at, wa, wb);
+  for (long long t = h.t; t < T; t += h.step) {
+    float a[4], b[4], x[4], y[4], cc[4], ss_[4];
+    uint2 oa = ra, ob = rb;
+    unpack4(ra, a);
+    unpack4(rb, b);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      cc[e] = c[e];
+      ss_[e] = sn[e];
+    }
+    fetch(t + h.step);
+    if (L.norm) {
+      const float ss = head_sum(a[0] * a[0] + a[1] * a[1] + b[0] * b[0] + b[1] * b[1], a[2] * a[2] + a[3] * a[3] + b[2] * b[2] + b[3] * b[3]);
+      const float rstd = rsqrtf(ss * (1.f / D) + L.eps);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        a[e] *= rstd * wa[e];
+        b[e] *= rstd * wb[e];
       }
-      float2 a = ld_bf2(src + 2 * lane), b = ld_bf2(src + 64 + 2 * lane);
-      if (L.norm) {
-        const float ss = warp_sum(a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y);
-        const float rstd = rsqrtf(ss * (1.f / D) + L.eps);
-        const float2 wa = kind == 0 ? wqa : wka, wb = kind == 0 ? wqb : wkb;
-        a.x *= rstd * wa.x; a.y *= rstd * wa.y; b.x *= rstd * wb.x; b.y *= rstd * wb.y;
+    }
+    if (rot) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        x[e] = fmaf(a[e], cc[e], -__fmul_rn(b[e], ss_[e]));
+        y[e] = fmaf(a[e], ss_[e], __fmul_rn(b[e], cc[e]));
       }
-      *reinterpret_cast<uint32_t*>(dst + 2 * lane) = pack_bf16x2(a.x * c.x - b.x * sn.x, a.y * c.y - b.y * sn.y);
-      *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = pack_bf16x2(b.x * c.x + a.x * sn.x, b.y * c.y + a.y * sn.y);
+      oa = pack4(x);
+      ob = pack4(y);
+    }
+    if (live) {
+      st_bf4<WIDE>(dst + t * heads * D, oa);
+      st_bf4<WIDE>(dst + t * heads * D + 64, ob);
     }
   }
 }
 
-__global__ void __launch_bounds__(WARPS * 32)
+template <bool WIDE>
+__global__ void __launch_bounds__(WARPS * 32, BWD_CTAS)
 qkv_bwd_fast_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ wq,
                     const __nv_bfloat16* __restrict__ wk, const float* __restrict__ cosb,
                     const float* __restrict__ sinb, const __nv_bfloat16* __restrict__ dq,
@@ -336,75 +422,83 @@ qkv_bwd_fast_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
                     float* __restrict__ dwq, float* __restrict__ dwk, float* __restrict__ partials, long long T,
                     QkvLayout L) {
   constexpr int D = 128;
-  __shared__ float sdw[WARPS][2][D];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slots = L.ng * (L.qpg * (1 + L.gate) + 2);
-  const int nq = L.ng * L.qpg;
-  for (int i = threadIdx.x; i < WARPS * 2 * D; i += blockDim.x) (&sdw[0][0][0])[i] = 0.f;
-  __syncthreads();
-  const float wbase = L.zero_centered ? 1.f : 0.f;
-  float2 wqa = make_float2(1.f, 1.f), wqb = wqa, wka = wqa, wkb = wqa;
-  if (L.norm) {
-    wqa = ld_bf2(wq + 2 * lane); wqb = ld_bf2(wq + 64 + 2 * lane);
-    wka = ld_bf2(wk + 2 * lane); wkb = ld_bf2(wk + 64 + 2 * lane);
-    wqa.x += wbase; wqa.y += wbase; wqb.x += wbase; wqb.y += wbase;
-    wka.x += wbase; wka.y += wbase; wkb.x += wbase; wkb.y += wbase;
-  }
-  float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-  for (long long t = blockIdx.x; t < T; t += gridDim.x) {
-    const float2 c = *reinterpret_cast<const float2*>(cosb + t * 64 + 2 * lane);
-    const float2 sn = *reinterpret_cast<const float2*>(sinb + t * 64 + 2 * lane);
-    for (int slot = warp; slot < slots; slot += WARPS) {
-      int kind, head;
-      decode_slot(L, slot, kind, head);
-      const __nv_bfloat16* src = qkv + t * L.ld + (long long)slot * D;
-      __nv_bfloat16* dst = dqkv + t * L.ld + (long long)slot * D;
-      const __nv_bfloat16* gsrc = kind == 0 ? dq + (t * nq + head) * D
-                                  : kind == 1 ? (dgate ? dgate + (t * nq + head) * D : nullptr)
-                                  : kind == 2 ? dk + (t * L.ng + head) * D
-                                              : dv + (t * L.ng + head) * D;
-      if (kind == 1 || kind == 3) {
-        *reinterpret_cast<uint2*>(dst + 4 * lane) =
-            gsrc ? *reinterpret_cast<const uint2*>(gsrc + 4 * lane) : make_uint2(0, 0);
-        continue;
-      }
-      const float2 ga = ld_bf2(gsrc + 2 * lane), gb = ld_bf2(gsrc + 64 + 2 * lane);
-      // transpose of the rotation
-      float2 na = make_float2(ga.x * c.x + gb.x * sn.x, ga.y * c.y + gb.y * sn.y);
-      float2 nb = make_float2(gb.x * c.x - ga.x * sn.x, gb.y * c.y - ga.y * sn.y);
-      if (L.norm) {
-        const float2 xa = ld_bf2(src + 2 * lane), xb = ld_bf2(src + 64 + 2 * lane);
-        const float2 wa = kind == 0 ? wqa : wka, wb = kind == 0 ? wqb : wkb;
-        float ss = xa.x * xa.x + xa.y * xa.y + xb.x * xb.x + xb.y * xb.y;
-        float dot = na.x * wa.x * xa.x + na.y * wa.y * xa.y + nb.x * wb.x * xb.x + nb.y * wb.y * xb.y;
-        ss = warp_sum(ss);
-        dot = warp_sum(dot);
-        const float rstd = rsqrtf(ss * (1.f / D) + L.eps);
-        const float c3 = dot * rstd * rstd * rstd * (1.f / D);
-        const float d0 = na.x * xa.x * rstd, d1 = na.y * xa.y * rstd, d2 = nb.x * xb.x * rstd, d3 = nb.y * xb.y * rstd;
-        if (kind == 0) { acc[0][0] += d0; acc[0][1] += d1; acc[0][2] += d2; acc[0][3] += d3; }
-        else { acc[1][0] += d0; acc[1][1] += d1; acc[1][2] += d2; acc[1][3] += d3; }
-        na.x = na.x * wa.x * rstd - xa.x * c3; na.y = na.y * wa.y * rstd - xa.y * c3;
-        nb.x = nb.x * wb.x * rstd - xb.x * c3; nb.y = nb.y * wb.y * rstd - xb.y * c3;
-      }
-      *reinterpret_cast<uint32_t*>(dst + 2 * lane) = pack_bf16x2(na.x, na.y);
-      *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = pack_bf16x2(nb.x, nb.y);
+  __shared__ float sdw[WARPS * 2][D];
+  __shared__ int kinds[WARPS * 2];
+  const HeadWalk h(L);
+  const int nq = L.ng * L.qpg, heads = h.kind < 2 ? nq : L.ng;
+  const bool rot = h.kind == 0 || h.kind == 2, live = h.slot >= 0;
+  float wa[4] = {}, wb[4] = {}, acc[8] = {};
+  const __nv_bfloat16* src = qkv + (live ? h.slot : 0) * D + h.at;
+  const __nv_bfloat16* gsrc = h.kind == 0 ? dq : h.kind == 1 ? dgate : h.kind == 2 ? dk : dv;
+  const bool given = gsrc != nullptr;
+  gsrc += (long long)h.head * D + h.at;
+  __nv_bfloat16* dst = dqkv + (live ? h.slot : 0) * D + h.at;
+  uint2 ga, gb, xa, xb;
+  float c[4], sn[4];
+  auto fetch = [&](long long t) {
+    ga = gb = xa = xb = make_uint2(0, 0);
+    if (t >= T) return;
+    if (given) {
+      ga = ld_bf4<WIDE>(gsrc + t * heads * D);
+      gb = ld_bf4<WIDE>(gsrc + t * heads * D + 64);
     }
-  }
-  if (L.norm) {
+    if (L.norm && rot) {
+      xa = ld_bf4<WIDE>(src + t * L.ld);
+      xb = ld_bf4<WIDE>(src + t * L.ld + 64);
+    }
+    ld_angles(cosb + t * 64 + h.at, c);
+    ld_angles(sinb + t * 64 + h.at, sn);
+  };
+  fetch(h.t);
+  if (L.norm) head_weights(L, h.kind == 0 ? wq : wk, h.at, wa, wb);
+  for (long long t = h.t; t < T; t += h.step) {
+    // transpose of the rotation
+    float a[4], b[4], x[4], y[4], na[4], nb[4];
+    uint2 oa = ga, ob = gb;
+    unpack4(ga, a);
+    unpack4(gb, b);
+    unpack4(xa, x);
+    unpack4(xb, y);
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
-      sdw[warp][a][2 * lane] = acc[a][0];
-      sdw[warp][a][2 * lane + 1] = acc[a][1];
-      sdw[warp][a][64 + 2 * lane] = acc[a][2];
-      sdw[warp][a][65 + 2 * lane] = acc[a][3];
+    for (int e = 0; e < 4; ++e) {
+      na[e] = a[e] * c[e] + b[e] * sn[e];
+      nb[e] = b[e] * c[e] - a[e] * sn[e];
     }
+    fetch(t + h.step);
+    if (L.norm) {
+      const float ss = head_sum(x[0] * x[0] + x[1] * x[1] + y[0] * y[0] + y[1] * y[1], x[2] * x[2] + x[3] * x[3] + y[2] * y[2] + y[3] * y[3]);
+      const float dot = head_sum(na[0] * wa[0] * x[0] + na[1] * wa[1] * x[1] + nb[0] * wb[0] * y[0] + nb[1] * wb[1] * y[1],
+                                 na[2] * wa[2] * x[2] + na[3] * wa[3] * x[3] + nb[2] * wb[2] * y[2] + nb[3] * wb[3] * y[3]);
+      const float rstd = rsqrtf(ss * (1.f / D) + L.eps);
+      const float c3 = dot * rstd * rstd * rstd * (1.f / D);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc[e] += na[e] * x[e] * rstd;
+        acc[4 + e] += nb[e] * y[e] * rstd;
+        na[e] = na[e] * wa[e] * rstd - x[e] * c3;
+        nb[e] = nb[e] * wb[e] * rstd - y[e] * c3;
+      }
+    }
+    if (rot) {
+      oa = pack4(na);
+      ob = pack4(nb);
+    }
+    if (live) {
+      st_bf4<WIDE>(dst + t * L.ld, oa);
+      st_bf4<WIDE>(dst + t * L.ld + 64, ob);
+    }
+  }
+  if (L.norm) {
+    const int half = threadIdx.x >> 4;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sdw[half][h.at + (e & 3) + (e >> 2) * 64] = acc[e];
+    if ((threadIdx.x & 15) == 0) kinds[half] = live ? h.kind : 3;
     __syncthreads();
     for (int i = threadIdx.x; i < D; i += blockDim.x) {
       float a = 0.f, b = 0.f;
-      for (int w = 0; w < WARPS; ++w) {
-        a += sdw[w][0][i];
-        b += sdw[w][1][i];
+      for (int w = 0; w < WARPS * 2; ++w) {
+        if (kinds[w] == 0) a += sdw[w][i];
+        if (kinds[w] == 2) b += sdw[w][i];
       }
       if (partials) {
         partials[((long long)blockIdx.x * 2) * D + i] = a;
@@ -415,6 +509,19 @@ qkv_bwd_fast_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
       }
     }
   }
+}
+
+// CTAs of the fast kernels, 0 where a warp for every pair of heads is more than there are
+int fast_grid(const QkvLayout& L, long long T, int ctas_per_sm) {
+  const long long pairs = (L.ng * (L.qpg * (1LL + L.gate) + 2) + 1) / 2, cap = (long long)device_sm_count() * ctas_per_sm;
+  if (pairs > cap * WARPS) return 0;
+  const long long blocks = (T * pairs + WARPS - 1) / WARPS;
+  return (int)(blocks < cap ? blocks : cap);
+}
+bool on_8_bytes(std::initializer_list<const void*> ps) {
+  uintptr_t bits = 0;
+  for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
+  return bits % 8 == 0;
 }
 
 }  // namespace
@@ -430,8 +537,10 @@ int mcb_qkv_split_norm_rope_fwd(const void* qkv, const void* wq, const void* wk,
   QkvLayout L{ng, qpg, d, has_gate, rot, interleaved, norm, zero_centered, eps, ld};
   long long blocks = T;
   long long cap = (long long)device_sm_count() * 16;
-  if (d == 128 && rot == 128 && !interleaved) {
-    qkv_fwd_fast_kernel<<<(int)(blocks < cap ? blocks : cap), WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(
+  const int fast = d == 128 && rot == 128 && !interleaved ? fast_grid(L, T, FWD_CTAS) : 0;
+  if (fast > 0) {
+    auto* kernel = on_8_bytes({qkv, q, k, v, gate}) ? qkv_fwd_fast_kernel<true> : qkv_fwd_fast_kernel<false>;
+    kernel<<<fast, WARPS * 32, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(
         (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, cosb, sinb, (__nv_bfloat16*)q,
         (__nv_bfloat16*)k, (__nv_bfloat16*)v, (__nv_bfloat16*)gate, T, L);
     return (int)cudaGetLastError();
@@ -442,10 +551,9 @@ int mcb_qkv_split_norm_rope_fwd(const void* qkv, const void* wq, const void* wk,
   return (int)cudaGetLastError();
 }
 
-// CTAs the backward kernels launch for T tokens = rows of `partials` ([rows, 2, d] fp32) the caller provides
+// CTAs the backward kernels launch for T tokens at most = rows of `partials` ([rows, 2, d] fp32) the caller provides
 int mcb_qkv_bwd_partial_rows(long long T) {
-  const long long cap = (long long)device_sm_count() * 8;
-  return (int)(T < cap ? T : cap);
+  return T > 0 ? device_sm_count() * 8 : 0;
 }
 
 // dwq / dwk: fp32 [d], accumulated into (caller zeroes or carries them across micro-batches), or, with `dw_bf16` (needs
@@ -460,13 +568,16 @@ int mcb_qkv_split_norm_rope_bwd(const void* qkv, const void* wq, const void* wk,
   if (d > MAX_D || d % 8 || rot > d || (rot & 1) || ld % 8) return -1;
   QkvLayout L{ng, qpg, d, has_gate, rot, interleaved, norm, zero_centered, eps, ld};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  const int grid = mcb_qkv_bwd_partial_rows(T);
+  int grid = (int)min(T, (long long)mcb_qkv_bwd_partial_rows(T));
   if (!norm) partials = nullptr;
   if (norm && dw_bf16 && !partials) return -3;
   float* dwq = dw_bf16 ? nullptr : reinterpret_cast<float*>(dwq_any);
   float* dwk = dw_bf16 ? nullptr : reinterpret_cast<float*>(dwk_any);
-  if (d == 128 && rot == 128 && !interleaved) {
-    qkv_bwd_fast_kernel<<<grid, WARPS * 32, 0, s>>>(
+  const int fast = d == 128 && rot == 128 && !interleaved ? fast_grid(L, T, BWD_CTAS) : 0;
+  if (fast > 0) {
+    grid = fast;
+    auto* kernel = on_8_bytes({qkv, dq, dk, dv, dgate, dqkv}) ? qkv_bwd_fast_kernel<true> : qkv_bwd_fast_kernel<false>;
+    kernel<<<grid, WARPS * 32, 0, s>>>(
         (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, cosb, sinb,
         (const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, (const __nv_bfloat16*)dgate,
         (__nv_bfloat16*)dqkv, dwq, dwk, partials, T, L);

@@ -63,3 +63,34 @@ def test_norm_backward_with_the_next_rows_in_flight(rows, H):
     ref = wide[0] * torch.rsqrt(wide[0].pow(2).mean(-1, keepdim=True) + 1e-6) * wide[1]
     for a, b in zip((dx, dw), torch.autograd.grad(ref, wide, dy.double())):
         assert _rel(a, b) < 2 ** -8
+
+
+@pytest.mark.parametrize('T,ng,qpg,gate', [(1, 1, 1, False), (2, 16, 3, False), (333, 1, 2, True), (7, 300, 1, False), (2500, 3, 1, False)])
+@pytest.mark.parametrize('norm', [False, True])
+def test_heads_of_128(T, ng, qpg, gate, norm):
+    from mcore_bridge_b200.ops.rope import qkv_split_norm_rope, qkv_split_norm_rope_ref
+    W = ng * (qpg * (2 if gate else 1) + 2) * 128
+    cos, sin = torch.rand(T, 64, device=DEV), torch.rand(T, 64, device=DEV)
+    buf = _rand(T * W + 2)
+    ws = [_rand(128, seed=s) for s in (1, 2)] if norm else [None, None]
+
+    def run(qkv, f, ws):
+        leaves = [t.requires_grad_() for t in (qkv, *ws) if t is not None]
+        outs = [t for t in f(qkv, ws[0], ws[1], cos.to(qkv.dtype), sin.to(qkv.dtype), ng, qpg, 128, gate, False, 1e-6, False) if t is not None]
+        gen = torch.Generator(device=DEV).manual_seed(5)
+        seeds = [torch.randn(t.shape, generator=gen, device=DEV).bfloat16().to(t.dtype) for t in outs]
+        return outs + list(torch.autograd.grad(outs, leaves, seeds))
+
+    def single(qkv, wq, wk, cos, sin, *rest):
+        return qkv_split_norm_rope(qkv, wq, wk, cos.float(), sin.float(), *rest)
+
+    qkv = buf[:T * W].view(T, W)
+    got = run(qkv.detach().clone(), single, [None if w is None else w.clone() for w in ws])
+    cos, sin = cos.double(), sin.double()
+    want = run(qkv.double(), qkv_split_norm_rope_ref, [None if w is None else w.double() for w in ws])
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 2 ** -8                                      # rounded once
+    cos, sin = cos.float(), sin.float()
+    buf[2:] = buf[:-2].clone()                                           # four bytes from any wider boundary
+    for a, b in zip(run(buf[2:].view(T, W).detach(), single, ws), got):
+        assert torch.equal(a, b)
