@@ -76,8 +76,7 @@ class _RouterGateFn(torch.autograd.Function):
         x, w = ctx.saved_tensors
         E = w.shape[0]
         if dl.dtype == torch.float32:
-            hi = dl.to(torch.bfloat16)
-            d2 = torch.cat([hi, (dl - hi.float()).to(torch.bfloat16)], dim=1)      # [T, 2E]
+            d2 = moe_ops.split_terms(dl)                                           # [T, 2E]
             w2 = torch.cat([w, w], dim=0)                                          # [2E, H]
         else:
             d2, w2 = dl.contiguous(), w
@@ -85,9 +84,7 @@ class _RouterGateFn(torch.autograd.Function):
         dw = None
         if ctx.needs_input_grad[1]:
             dw = gemm.mm_tn(d2, x, out_dtype=torch.float32)                         # [2E or E, H]
-            if dw.shape[0] != E:
-                dw = dw[:E] + dw[E:]
-            dw = dw.to(w.dtype)
+            dw = dw.to(w.dtype) if dw.shape[0] == E else moe_ops.add_halves(dw)
         return dx, dw, None
 
 
@@ -468,11 +465,16 @@ class MoELayer(nn.Module):
                 with torch.no_grad():
                     r.local_tokens_per_expert += counts.float()
             coeff = cfg.moe_aux_loss_coeff
-            if self.training and coeff and lb in ('aux_loss', 'global_aux_loss'):
+            group = 'tp_dp_cp' if lb == 'global_aux_loss' else ('tp_cp' if cfg.sequence_parallel or
+                                                                cfg.context_parallel_size > 1 else None)
+            if self.training and coeff and lb in ('aux_loss', 'global_aux_loss') and valid is None and T > 0 and \
+                    (group is None or ps.get_world_size(group) == 1):
+                aux, value = moe_ops.RouterAuxLoss.apply(score_sum, counts, T, r.topk, float(coeff))
+                probs = moe_ops.MoEAuxLossAutoScaler.apply(probs, aux)
+                _track('load_balancing_loss', value)
+            elif self.training and coeff and lb in ('aux_loss', 'global_aux_loss'):
                 ntok = torch.full((), float(T), device=x.device) if valid is None else valid.sum().float()
                 cnt = counts.float()
-                group = 'tp_dp_cp' if lb == 'global_aux_loss' else ('tp_cp' if cfg.sequence_parallel or
-                                                                    cfg.context_parallel_size > 1 else None)
                 ntok_all = ntok
                 if group is not None and ps.get_world_size(group) > 1:
                     packed = torch.cat([cnt, ntok.view(1)])

@@ -84,6 +84,15 @@ class ExchangeBuffers:
         _lib.check_rc(rc, 'mcb_moe_sort')
 
 
+    def publish_rows(self, parity: int, x: torch.Tensor):
+        """Where each rank finds its sources' rows ``[T, H]``: a copy in the published region, or, when this rank is its
+        only source and ``x`` can be read as it is, ``x`` itself."""
+        if self.world == 1 and x.is_contiguous() and x.dtype == torch.bfloat16 and x.data_ptr() % 16 == 0:
+            return _arr([x.data_ptr()])
+        self.view('x', parity, (self.T, self.H), torch.bfloat16).copy_(x)
+        return self.ptrs('x', parity)
+
+
 class _ExchangeAllocation:
     """Published/received buffers of one direction (forward or backward), laid out for up to ``T_alloc`` tokens."""
 
@@ -247,7 +256,8 @@ class _RouterFn(torch.autograd.Function):
         ctx.save_for_backward(scores, idx_saved, valid)
         ctx.meta = (k, sigmoid, renorm, scaling)
         ctx.mark_non_differentiable(idx_saved)
-        return probs_out.clone(), idx_saved, score_sum
+        ctx.mark_dirty(probs_out)
+        return probs_out, idx_saved, score_sum
 
     @staticmethod
     def backward(ctx, dprobs, _didx, dscore_sum):
@@ -404,9 +414,10 @@ def _weight_grad_grouped(weight, dy, x, offsets):
     return gemm.grouped_mm_tn(dy, x, offsets, out_dtype=weight.dtype)
 
 
-def _pull_gemm(b: ExchangeBuffers, par: int, mode: int, st: 'DispatchState', El: int, rows_region: str, weight,
+def _pull_gemm(b: ExchangeBuffers, par: int, mode: int, st: 'DispatchState', El: int, rows, weight,
                b_mn: bool, xp, row_probs, out):
-    """Launches the fused pull + grouped GEMM kernel on ``b``'s published regions of parity ``par``."""
+    """Launches the fused pull + grouped GEMM kernel on ``b``'s published regions of parity ``par`` and the rows at ``rows``
+    (``publish_rows``)."""
     T, H, k, E = b.T, b.H, b.k, b.E
     G, d1, d2 = weight.shape
     w2 = weight.view(G * d1, d2)
@@ -416,7 +427,7 @@ def _pull_gemm(b: ExchangeBuffers, par: int, mode: int, st: 'DispatchState', El:
         N, b_inner, b_outer, group_rows = d1, d2, G * d1, d1
     fwd = mode == 0
     rc = _lib.lib().mcb_moe_pull_gemm(
-        b.ptrs(rows_region, par), b.ptrs('order', par) if fwd else None, b.ptrs('eoff', par) if fwd else None,
+        rows, b.ptrs('order', par) if fwd else None, b.ptrs('eoff', par) if fwd else None,
         b.ptrs('probs', par) if fwd else None, b.ptrs('sent', par) if fwd else None, _int(b.world), _int(b.rank),
         _int(T), _int(k), _int(E), _int(El), _int(H), _int(N), _int(b.cap), _int(mode), _lib.ptr(st.seg_off),
         _lib.ptr(st.row_src), _lib.ptr(row_probs), _lib.ptr(xp), _lib.ptr(b.blk_flags), _u(b.next_pull_epoch()),
@@ -492,7 +503,7 @@ class _DispatchFc1Fn(torch.autograd.Function):
         b = st.fwd
         T, H, k = b.T, b.H, b.k
         par, epoch = st.parity, b.epoch
-        b.view('x', par, (T, H), torch.bfloat16).copy_(x)
+        rows = b.publish_rows(par, x)
         b.view('probs', par, (T, k), torch.float32).copy_(probs.float())
         b.sort_routing(par)                   # idx and counts were published by the router
         b.signal(F_READY, epoch)
@@ -501,7 +512,7 @@ class _DispatchFc1Fn(torch.autograd.Function):
         xp = torch.empty((b.cap, H), dtype=torch.bfloat16, device=dev)
         h = torch.empty((b.cap, w1.shape[1]), dtype=torch.bfloat16, device=dev)
         row_probs = torch.empty(b.cap, dtype=torch.float32, device=dev)
-        _pull_gemm(b, par, 0, st, El, 'x', w1, False, xp, row_probs, h)
+        _pull_gemm(b, par, 0, st, El, rows, w1, False, xp, row_probs, h)
         ctx.save_for_backward(xp, w1)
         ctx.st, ctx.El, ctx.pdtype = st, El, probs.dtype
         return h, row_probs
@@ -591,12 +602,12 @@ class _Fc2CombineFn(torch.autograd.Function):
         T, H = b.T, b.H
         epoch = b.next_epoch()
         par = epoch & 1
-        b.view('x', par, (T, H), torch.bfloat16).copy_(dout)
+        rows = b.publish_rows(par, dout)
         b.signal(F_READY, epoch)
         b.wait(F_READY, epoch)
         dy = torch.empty((b.cap, H), dtype=torch.bfloat16, device=dout.device)
         da = torch.empty_like(a)
-        _pull_gemm(b, par, 1, st, El, 'x', w2, True, dy, None, da)
+        _pull_gemm(b, par, 1, st, El, rows, w2, True, dy, None, da)
         dw2 = _weight_grad_grouped(w2, dy, a, st.seg_off) if ctx.needs_input_grad[1] else None
         return da, dw2, None, None
 

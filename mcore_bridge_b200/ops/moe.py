@@ -10,9 +10,12 @@
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional, Tuple
 
 import torch
+
+from . import _lib
 
 PAD = 128
 
@@ -128,11 +131,63 @@ class MoEAuxLossAutoScaler(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_output):
         (aux,) = ctx.saved_tensors
-        return grad_output, torch.ones_like(aux) * MoEAuxLossAutoScaler.main_loss_backward_scale
+        return grad_output, torch.full_like(aux, MoEAuxLossAutoScaler.main_loss_backward_scale)
 
     @staticmethod
     def set_loss_scale(scale: float):
         MoEAuxLossAutoScaler.main_loss_backward_scale = float(scale)
+
+
+class RouterAuxLoss(torch.autograd.Function):
+    """``aux_loss`` from the router kernel's statistics (``score_sum`` fp32 and ``counts`` int32, ``[E]``) of ``tokens`` tokens,
+    and the same divided by ``coeff`` for the log, in one launch each way."""
+
+    @staticmethod
+    def forward(ctx, score_sum, counts, tokens, topk, coeff):
+        E = score_sum.shape[0]
+        out = torch.empty(E + 2, dtype=torch.float32, device=score_sum.device)
+        c = coeff * E
+        rc = _lib.lib().mcb_router_aux(_lib.ptr(counts), _lib.ptr(score_sum), _lib.ptr(out[2:]), _lib.ptr(out), ctypes.c_int(E),
+                                       ctypes.c_float(tokens), ctypes.c_int(topk), ctypes.c_float(c), ctypes.c_float(coeff),
+                                       _lib.stream_ptr())
+        _lib.check_rc(rc, 'mcb_router_aux')
+        aux, value, frac = out[0], out[1], out[2:]
+        ctx.save_for_backward(frac)
+        ctx.meta = (float(tokens), c)
+        ctx.mark_non_differentiable(value)
+        return aux, value
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, g, _dvalue):
+        (frac,) = ctx.saved_tensors
+        tokens, c = ctx.meta
+        g = g.float().contiguous()
+        out = torch.empty_like(frac)
+        rc = _lib.lib().mcb_router_aux_bwd(_lib.ptr(g), _lib.ptr(frac), _lib.ptr(out), ctypes.c_int(frac.numel()),
+                                           ctypes.c_float(tokens), ctypes.c_float(c), _lib.stream_ptr())
+        _lib.check_rc(rc, 'mcb_router_aux_bwd')
+        return out, None, None, None, None
+
+
+def split_terms(x: torch.Tensor) -> torch.Tensor:
+    """fp32 ``[T, E]`` -> bf16 ``[T, 2E]``: the value rounded, and the rounding error rounded."""
+    T, E = x.shape
+    x = x.contiguous()
+    if x.data_ptr() % 16:
+        x = x.clone()
+    out = torch.empty((T, 2 * E), dtype=torch.bfloat16, device=x.device)
+    _lib.check_rc(_lib.lib().mcb_split_terms(_lib.ptr(x), _lib.ptr(out), ctypes.c_longlong(T), ctypes.c_int(E), _lib.stream_ptr()),
+                  'mcb_split_terms')
+    return out
+
+
+def add_halves(x: torch.Tensor) -> torch.Tensor:
+    """fp32 ``[2E, H]`` -> bf16 ``[E, H]``: the sum of the two halves."""
+    out = torch.empty((x.shape[0] // 2, *x.shape[1:]), dtype=torch.bfloat16, device=x.device)
+    _lib.check_rc(_lib.lib().mcb_add_halves(_lib.ptr(x), _lib.ptr(out), ctypes.c_longlong(out.numel()), _lib.stream_ptr()),
+                  'mcb_add_halves')
+    return out
 
 
 def z_loss(logits: torch.Tensor, coeff: float) -> torch.Tensor:
