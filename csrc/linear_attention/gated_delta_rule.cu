@@ -37,11 +37,12 @@
 // first operand of the next one.  Bound: the latency of what a chunk does one after the other (a warp issues every tenth cycle, the
 // MMAs, forward about 500 a strip, backward 900 and 800, take 40 to 48 % of the time); the next chunk's tiles are copied
 // meanwhile.  With one warp for a strip, which passes nothing on and forms every term itself, us, before / now, scan, the
-// backward pass's scan and scan_bwd: 4096 tokens in three sequences, 32 heads of 128 171, 297, 358 / 147, 239, 263; in 64
-// sequences 176, 308, 431 / 173, 285, 317; 8192 in one, 16 heads 636, 1120, 1338 / 562, 910, 1007.  Two warps a strip: 173, 276,
+// backward pass's scan and scan_bwd: 4096 tokens in three sequences, 32 heads of 128 171, 297, 358 / 133, 216, 254; in 64
+// sequences 176, 308, 431 / 159, 260, 297; 8192 in one, 16 heads 636, 1120, 1338 / 504, 821, 959.  Two warps a strip: 173, 276,
 // 307 (of the first).  No change from starting the strips apart, slower with the operands of M and P fetched before the
-// strip's barrier (162, 335, 367: registers).
-// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.24 ms (prep 0.09), backward 0.79 ms (grad 0.29).  The batched
+// strip's barrier (162, 335, 367: registers) and with 8 + 8 tokens a warp, for which M and P have as many blocks in each (145,
+// 231, 274: more instructions).
+// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.22 ms (prep 0.08), backward 0.76 ms (grad 0.29).  The batched
 // torch evaluation of the rule was most of a 29.5 ms block.
 #include "../common/host_utils.cuh"
 #include "warp_mma.cuh"
@@ -60,6 +61,13 @@ constexpr int MP = 3;           // terms kept of M and P
 // rows of `gb`: G as a sum of two floats, beta, exp(G), exp(G_last - G), the diagonal p
 enum { G_HI, G_LO, G_BETA, G_EXP, G_REST, G_DIAG, G_ROWS };
 
+// M and P are kept as the ten 16 x 16 blocks on and below the diagonal, 512 bytes each; the two halves of a row change places every
+// four rows, so that in shared memory, where they are copied as they are, eight rows of a half lie in distinct banks.
+constexpr int SQB = 10 * 512;   // bytes of one term
+__device__ __forceinline__ int block_off(int bi, int bj, int r, int half) {
+  return (bi * (bi + 1) / 2 + bj) * 512 + r * 32 + ((half ^ ((r >> 2) & 1)) << 4);
+}
+
 struct GdrParams {
   const __nv_bfloat16 *q, *k, *v, *dout;   // [T, H, D]
   const float *g, *beta;                   // [T, H]
@@ -67,7 +75,7 @@ struct GdrParams {
   __nv_bfloat16 *o, *dq, *dk, *dv;
   float *dg, *dbeta;                       // [T, H]
   // per chunk and head, chunks numbered through the packed batch:
-  __nv_bfloat16* mp;                       // [2 MP, 64, 64]: M and P, MP terms each
+  __nv_bfloat16* mp;                       // [2 MP, 64, 64], of each a part: M and P, MP terms each, one behind the other
   float* gb;                               // [G_ROWS, 64] (beta 0 past the end of the sequence)
   float *S, *dS;                           // [D, D]: S^T and dS'^T
   __nv_bfloat16 *V, *B;                    // [2, D, 64]: V^T and B^T, two terms
@@ -183,7 +191,9 @@ gdr_prep_kernel(const GdrParams p) {
         uint32_t t[MP][4];
         split_terms<MP>(pv[0], pv[1], t, 0);
 #pragma unroll
-        for (int m = 0; m < MP; ++m) *reinterpret_cast<uint32_t*>(mp + (MP + m) * CC + (i + 8 * r) * C + j) = t[m][0];
+        for (int m = 0; m < MP; ++m)
+          if (jb <= warp)
+            *reinterpret_cast<uint32_t*>(mp + MP * CC + (m * SQB + block_off(warp, jb, (lane >> 2) + 8 * r, n)) / 2 + (lane & 3) * 2) = t[m][0];
       }
     }
   }
@@ -218,14 +228,15 @@ gdr_prep_kernel(const GdrParams p) {
   __syncthreads();
   for (int id = threadIdx.x; id < MP * C * 8; id += THREADS) {
     const int m = id >> 9, r = (id >> 3) & 63, c = (id & 7) * 8;
-    *reinterpret_cast<uint4*>(mp + m * CC + r * C + c) = *reinterpret_cast<const uint4*>(sm + m * C * 72 + r * 72 + c);
+    if ((c >> 4) <= (r >> 4))
+      *reinterpret_cast<uint4*>(mp + (m * SQB + block_off(r >> 4, c >> 4, r & 15, (c >> 3) & 1)) / 2) =
+          *reinterpret_cast<const uint4*>(sm + m * C * 72 + r * 72 + c);
   }
 }
 
 // ---------------------------------------------------------------------------------------------------- scans
-// Shared memory of a scan: two stages of k, q, 64-column slices of v and of do (X / Z), the last rows of gb and NT terms of M and P
-// (the ten 16 x 16 blocks on and below the diagonal); what the four warps of a strip pass on to each other.
-constexpr int SQB = 10 * 512;
+// Shared memory of a scan: two stages of k, q, 64-column slices of v and of do (X / Z), the last rows of gb and NT terms of M and P;
+// what the four warps of a strip pass on to each other.
 template <int D, int NT, bool WITH_DO>
 struct ScanSmem {
   static constexpr int K = 0, Q = C * D * 2, X = 2 * C * D * 2, Z = X + SQ, G = Z + (WITH_DO ? SQ : 0);
@@ -237,40 +248,54 @@ struct ScanSmem {
   static_assert(D / 16 * NT * 512 <= 2 * PART && TOTAL + 64 <= 232448, "shared memory");
 };
 
-// 16 x 16 blocks of 512 bytes; the two halves of a row change places every four rows, so that eight rows of a half lie in
-// distinct banks
-__device__ __forceinline__ uint32_t block_addr(uint32_t tile, int bi, int bj, int r, int half) {
-  return tile + (bi * (bi + 1) / 2 + bj) * 512 + r * 32 + ((half ^ ((r >> 2) & 1)) << 4);
-}
-__device__ __forceinline__ void load_square(uint32_t tile, const __nv_bfloat16* src) {
-  for (int id = threadIdx.x; id < 320; id += ST) {
-    const int blk = id >> 5, bi = blk >= 6 ? 3 : blk >= 3 ? 2 : blk >= 1 ? 1 : 0, bj = blk - bi * (bi + 1) / 2, rr = (id >> 1) & 15, half = id & 1;
-    cp_async16(block_addr(tile, bi, bj, rr, half), src + (bi * 16 + rr) * C + bj * 16 + half * 8, 16);
-  }
-}
-
 // arrives when this thread's copies so far have landed
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
-// by all threads; the mbarriers `full` (tiles) and full + 16 (M and P) have a count of ST
+// A thread's part of the copies of a chunk, found once: with the addresses formed for each chunk they took 1400 of the 8000 cycles
+// a chunk spends on its way through a warp.
 template <int D, int NT, bool WITH_DO>
-__device__ __forceinline__ void load_stage(uint32_t st, uint32_t full, const GdrParams& p, int t, int len, int h, int col0, long long ch) {
+struct StageLoad {
   using L = ScanSmem<D, NT, WITH_DO>;
-  const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
-  load_tile<D, C, ST>(st + L::K, p.k + off, stride, len);
-  load_tile<D, C, ST>(st + L::Q, p.q + off, stride, len);
-  load_tile<64, C, ST>(st + L::X, p.v + off + col0, stride, len);
-  if (WITH_DO) load_tile<64, C, ST>(st + L::Z, p.dout + off + col0, stride, len);
-  if (threadIdx.x < 64) cp_async16(st + L::G + threadIdx.x * 16, p.gb + (ch * G_ROWS + G_BETA) * C + threadIdx.x * 4, 16);
-  cp_async_arrive(full);
-#pragma unroll
-  for (int m = 0; m < NT; ++m) {
-    load_square(st + L::M + m * SQB, p.mp + (ch * 2 * MP + m) * CC);
-    load_square(st + L::P + m * SQB, p.mp + (ch * 2 * MP + MP + m) * CC);
+  static constexpr int N = D * C / 8 / ST;      // 16-byte pieces of q or k
+  static constexpr int ROWS = ST / (D / 8);     // rows between two of them
+  uint32_t off, at, xoff, xat;                  // of the first piece: elements from the chunk's first, bytes in the tile
+  int row, xrow;
+  __device__ __forceinline__ StageLoad(const GdrParams& p) {
+    const uint32_t stride = p.H * D;
+    row = threadIdx.x / (D / 8);
+    off = row * stride + threadIdx.x % (D / 8) * 8;
+    at = tile_addr<D>(0, row, threadIdx.x % (D / 8) * 8);
+    xrow = threadIdx.x >> 3;
+    xoff = xrow * stride + (threadIdx.x & 7) * 8;
+    xat = tile_addr<64>(0, xrow, (threadIdx.x & 7) * 8);
   }
-  cp_async_arrive(full + 16);
-}
+  // by all threads; the mbarriers `full` (tiles, gb) and full + 16 (M and P) have counts of ST + 1 and 1
+  __device__ __forceinline__ void operator()(uint32_t st, uint32_t full, const GdrParams& p, int t, int len, int h, int col0, long long ch) const {
+    static_assert(ROWS % 8 == 0, "the same place in the swizzle");
+    if (threadIdx.x == 0) {
+      mbar_expect_tx(full, 4 * C * 4);
+      bulk_load_1d(st + L::G, p.gb + (ch * G_ROWS + G_BETA) * C, 4 * C * 4, full);
+      mbar_expect_tx(full + 16, 2 * NT * SQB);
+      bulk_load_1d(st + L::M, p.mp + ch * 2 * MP * CC, NT * SQB, full + 16);
+      bulk_load_1d(st + L::P, p.mp + (ch * 2 * MP + MP) * CC, NT * SQB, full + 16);
+    }
+    const long long first = ((long long)t * p.H + h) * D;
+    const __nv_bfloat16 *k = p.k + first, *q = p.q + first;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const bool in = row + i * ROWS < len;
+      const uint32_t o = in ? off + i * ROWS * (uint32_t)(p.H * D) : 0;
+      cp_async16(st + L::K + at + i * ROWS * D * 2, k + o, in ? 16 : 0);
+      cp_async16(st + L::Q + at + i * ROWS * D * 2, q + o, in ? 16 : 0);
+    }
+    const bool in = xrow < len;
+    const uint32_t o = (in ? xoff : 0) + col0;
+    cp_async16(st + L::X + xat, p.v + first + o, in ? 16 : 0);
+    if (WITH_DO) cp_async16(st + L::Z + xat, p.dout + first + o, in ? 16 : 0);
+    cp_async_arrive(full);
+  }
+};
 
 struct ScanPos {
   int t0, len, chunk0, n, h, col0;   // the sequence; its first chunk and their number; head; first column of v
@@ -358,8 +383,8 @@ template <int NT, bool TRANS>
 __device__ __forceinline__ void load_square_b(uint32_t tile, int bi, int bj, int lane, uint32_t (&b)[NT][4]) {
 #pragma unroll
   for (int m = 0; m < NT; ++m) {
-    if (TRANS) ldsm4(block_addr(tile + m * SQB, bi, bj, ((lane >> 4) << 3) + (lane & 7), (lane >> 3) & 1), b[m]);
-    else ldsm4_t(block_addr(tile + m * SQB, bi, bj, (((lane >> 3) & 1) << 3) + (lane & 7), lane >> 4), b[m]);
+    if (TRANS) ldsm4(tile + m * SQB + block_off(bi, bj, ((lane >> 4) << 3) + (lane & 7), (lane >> 3) & 1), b[m]);
+    else ldsm4_t(tile + m * SQB + block_off(bi, bj, (((lane >> 3) & 1) << 3) + (lane & 7), lane >> 4), b[m]);
   }
 }
 
@@ -378,8 +403,8 @@ struct ScanRing {
     if (threadIdx.x == 0) {
       *flag = 0;
       for (int i = 0; i < 2; ++i) {
-        mbar_init(full + 8 * i, ST);
-        mbar_init(full + 16 + 8 * i, ST);
+        mbar_init(full + 8 * i, ST + 1);
+        mbar_init(full + 16 + 8 * i, 1);
         mbar_init(empty + 8 * i, ST / 32);
       }
       fence_barrier_init();
@@ -495,10 +520,11 @@ gdr_scan_kernel(const GdrParams p) {
   zero(St);
   ScanRing ring;
   ring.init(base + L::BARS, &flag, p.status);
+  const StageLoad<D, NT, SAVE> copy(p);
   auto load = [&](int c) {
     if (c >= s.n) return;
     ring.wait_empty(c);
-    load_stage<D, NT, SAVE>(base + (c & 1) * L::STAGE, ring.full + 8 * (c & 1), p, s.t0 + c * C, min(C, s.len - c * C), s.h, s.col0,
+    copy(base + (c & 1) * L::STAGE, ring.full + 8 * (c & 1), p, s.t0 + c * C, min(C, s.len - c * C), s.h, s.col0,
                             (long long)(s.chunk0 + c) * p.H + s.h);
   };
   load(0);
@@ -679,11 +705,12 @@ gdr_scan_bwd_kernel(const GdrParams p) {
   const int lastc = s.n - 1;
   ScanRing ring;
   ring.init(base + L::BARS, &flag, p.status);
+  const StageLoad<D, NT, true> copy(p);
   auto load = [&](int it) {
     const int c = lastc - it;
     if (c < 0) return;
     ring.wait_empty(it);
-    load_stage<D, NT, true>(base + (it & 1) * L::STAGE, ring.full + 8 * (it & 1), p, s.t0 + c * C, min(C, s.len - c * C), s.h, s.col0,
+    copy(base + (it & 1) * L::STAGE, ring.full + 8 * (it & 1), p, s.t0 + c * C, min(C, s.len - c * C), s.h, s.col0,
                             (long long)(s.chunk0 + c) * p.H + s.h);
   };
   load(0);
