@@ -37,12 +37,12 @@
 // first operand of the next one.  Bound: the latency of what a chunk does one after the other (a warp issues every tenth cycle, the
 // MMAs, forward about 500 a strip, backward 900 and 800, take 40 to 48 % of the time); the next chunk's tiles are copied
 // meanwhile.  With one warp for a strip, which passes nothing on and forms every term itself, us, before / now, scan, the
-// backward pass's scan and scan_bwd: 4096 tokens in three sequences, 32 heads of 128 171, 297, 358 / 133, 216, 254; in 64
-// sequences 176, 308, 431 / 159, 260, 297; 8192 in one, 16 heads 636, 1120, 1338 / 504, 821, 959.  Two warps a strip: 173, 276,
+// backward pass's scan and scan_bwd: 4096 tokens in three sequences, 32 heads of 128 171, 297, 358 / 133, 213, 233; in 64
+// sequences 176, 308, 431 / 159, 257, 289; 8192 in one, 16 heads 636, 1120, 1338 / 504, 809, 897.  Two warps a strip: 173, 276,
 // 307 (of the first).  No change from starting the strips apart, slower with the operands of M and P fetched before the
 // strip's barrier (162, 335, 367: registers) and with 8 + 8 tokens a warp, for which M and P have as many blocks in each (145,
 // 231, 274: more instructions).
-// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.22 ms (prep 0.08), backward 0.76 ms (grad 0.29).  The batched
+// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.22 ms (prep 0.08), backward 0.72 ms (grad 0.28).  The batched
 // torch evaluation of the rule was most of a 29.5 ms block.
 #include "../common/host_utils.cuh"
 #include "warp_mma.cuh"
@@ -78,7 +78,7 @@ struct GdrParams {
   __nv_bfloat16* mp;                       // [2 MP, 64, 64], of each a part: M and P, MP terms each, one behind the other
   float* gb;                               // [G_ROWS, 64] (beta 0 past the end of the sequence)
   float *S, *dS;                           // [D, D]: S^T and dS'^T
-  __nv_bfloat16 *V, *B;                    // [2, D, 64]: V^T and B^T, two terms
+  __nv_bfloat16 *V, *B;                    // [2, D, 64]: V^T and B^T, two terms, as tiles in shared memory
   float* E;                                // [D / 16, 8, 32, 4]: E^T as the accumulators of the scans hold it
   float *oo, *nn, *yy;                     // [D / 16, 64]: do . O, V . N + B . E and dbeta over 16 columns of v
   int T, n_seq, H;
@@ -472,7 +472,7 @@ __device__ __forceinline__ void token_dots(const float (&x)[2][4], uint32_t tile
   }
 }
 
-// accumulators (16 rows x 16 tokens) -> two bf16 planes with 64 columns
+// accumulators (16 rows x 16 tokens) -> two bf16 planes with 64 columns, 16-byte chunks where tile_addr<64> has them
 __device__ __forceinline__ void store_terms(const float (&a)[2][4], __nv_bfloat16* dst, long long plane, int row, int tok0, int lane) {
 #pragma unroll
   for (int n = 0; n < 2; ++n) {
@@ -480,7 +480,7 @@ __device__ __forceinline__ void store_terms(const float (&a)[2][4], __nv_bfloat1
     for (int r = 0; r < 2; ++r) {
       uint32_t hi, lo;
       split2(a[n][2 * r], a[n][2 * r + 1], hi, lo);
-      __nv_bfloat16* at = dst + (long long)(row + 8 * r) * C + tok0 + n * 8 + (lane & 3) * 2;
+      __nv_bfloat16* at = dst + tile_addr<64>(0, row + 8 * r, tok0 + n * 8) / 2 + (lane & 3) * 2;
       *reinterpret_cast<uint32_t*>(at) = hi;
       *reinterpret_cast<uint32_t*>(at + plane) = lo;
     }
@@ -891,7 +891,7 @@ gdr_scan_bwd_kernel(const GdrParams p) {
 // and dk are rounded to bf16.  dg and dbeta are put together from the scans' dot products and <S', dS'>, in fp32.
 // Bound: 6200 warp-level MMAs a chunk (6.6 us) and 320 KB.
 // With two warps to 16 tokens, each forming the blocks of dP and dA it needs in both orientations (8600 MMAs), us, before / now: 4096
-// tokens, 32 heads of 128 381 / 293, in 64 sequences 500 / 383; of 64 134 / 131.  What is left is the phases of a lone CTA
+// tokens, 32 heads of 128 381 / 275, in 64 sequences 500 / 362; of 64 134 / 128.  What is left is the phases of a lone CTA
 // (the MMAs take a third of the time): states on their way to the L2 a wave of CTAs ahead gave 1 to 4 %, and cost 2 % at 64.
 constexpr int GT = 512;
 
@@ -963,7 +963,7 @@ template <int D, bool B>
 __device__ __forceinline__ void pair_block(uint32_t base, int rb, int cb, const float* s_gh, const float* s_gl, float scale, int lane) {
   using L = GradSmem<D>;
   float d[2][4] = {};
-#pragma unroll 2
+#pragma unroll
   for (int kk = 0; kk < D; kk += 16) {
     uint32_t vh[4], vl[4];
     load_b_nn<64>(base + L::VT, kk, cb * 16, lane, vh);
@@ -1043,6 +1043,8 @@ gdr_grad_kernel(const GdrParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ ChunkPos slot;
   __shared__ float s_gh[C], s_gl[C], s_red[GT / 32];
+  __shared__ __align__(8) uint64_t vb_full;
+  __shared__ int flag;
   constexpr int NW = D / 64;                   // strips of a half
   const uint32_t base = (smem_u32(smem_raw) + 127) & ~127u;
   const int lane = threadIdx.x & 31, id = warp_uniform(threadIdx.x >> 5), warp = id & 3, half = (id >> 2) & 1, h = blockIdx.y;
@@ -1051,13 +1053,26 @@ gdr_grad_kernel(const GdrParams p) {
   const int t = pos.t0 + pos.index * C, len = min(C, pos.t1 - t);
   const long long stride = (long long)p.H * D, off = ((long long)t * p.H + h) * D;
   const long long ch = (long long)blockIdx.x * p.H + h;
-  load_tile<D, C, GT>(base + L::Q, p.q + off, stride, len);
-  load_tile<D, C, GT>(base + L::K, p.k + off, stride, len);
-  load_tile<D, C, GT>(base + L::DO, p.dout + off, stride, len);
-  for (int i = threadIdx.x; i < 4 * D * 8; i += GT) {
-    const int m = i / (D * 8), r = (i / 8) % D, c = (i & 7) * 8;
-    const __nv_bfloat16* src = (m < 2 ? p.V : p.B) + ch * 2 * D * C + (m & 1) * D * C + r * C + c;
-    cp_async16(tile_addr<64>(base + L::VT + m * L::TILE, r, c), src, 16);
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&vb_full), 1);
+    fence_barrier_init();
+    mbar_expect_tx(smem_u32(&vb_full), 4 * L::TILE);
+    bulk_load_1d(base + L::VT, p.V + ch * 2 * D * C, 2 * L::TILE, smem_u32(&vb_full));
+    bulk_load_1d(base + L::YT, p.B + ch * 2 * D * C, 2 * L::TILE, smem_u32(&vb_full));
+  }
+  {
+    constexpr int PIECES = D / 8, ROWS = GT / PIECES;
+    const int row = threadIdx.x / PIECES, c = threadIdx.x % PIECES * 8;
+    const uint32_t to = tile_addr<D>(base, row, c), from = row * (uint32_t)stride + c;
+    static_assert(ROWS % 8 == 0, "the same place in the swizzle");
+#pragma unroll
+    for (int u = 0; u < C / ROWS; ++u) {
+      const bool in = row + u * ROWS < len;
+      const uint32_t o = in ? from + u * ROWS * (uint32_t)stride : 0;
+      cp_async16(to + L::Q + u * ROWS * D * 2, p.q + off + o, in ? 16 : 0);
+      cp_async16(to + L::K + u * ROWS * D * 2, p.k + off + o, in ? 16 : 0);
+      cp_async16(to + L::DO + u * ROWS * D * 2, p.dout + off + o, in ? 16 : 0);
+    }
   }
   cp_async_commit();
   const float* gb = p.gb + ch * G_ROWS * C;
@@ -1072,8 +1087,10 @@ gdr_grad_kernel(const GdrParams p) {
   strips.fetch(S, dS, next, 0);
   const int r0 = warp * 16, i = r0 + (lane >> 2), c2 = (lane & 3) * 2;
   const float eg[2] = {gb[G_EXP * C + i], gb[G_EXP * C + i + 8]}, el[2] = {gb[G_REST * C + i], gb[G_REST * C + i + 8]};
+  if (threadIdx.x == 0) flag = 0;
   cp_async_wait<0>();
-  __syncthreads();
+  __syncthreads();                             // (the mbarrier too)
+  mbar_wait_warp(smem_u32(&vb_full), 0, &flag, p.status, ST_TIMEOUT_FULL);   // gives up only with the device in trouble
   {
     // ten blocks of dA (48 MMAs) and ten of dP (32): one of dA, or one or two of dP to a warp
     auto row_of = [](int b) { return b >= 6 ? 3 : b >= 3 ? 2 : b >= 1 ? 1 : 0; };
