@@ -353,11 +353,11 @@ struct CombineArgs {
   const float* scalar_ptrs[MAX_WORLD]; // optional per-row scalar on the owner (e.g. d(prob))
 };
 
-// The sums of moe_combine_kernel below, in the same order, for 4 to 8 rows a token: all of them are found first, then one 16-byte piece
+// The sums of moe_combine_kernel below, in the same order, for 4 to 8 rows a token: a lane finds each of them, then one 16-byte piece
 // of each is in flight per lane; blockIdx.y takes runs of 32 pieces, which gives few tokens more warps.  Bound: the reads.  us, the
-// kernel below / this one: 4096 tokens x 8 rows of 2048 61 / 41 (3.7 TB/s), 1024 x 8 53 / 16, 64 x 8 49 / 8, 1000 x 6 43 / 14, 8192 x 4
-// of 2880 92 / 74; it has too little in flight with fewer rows: 8192 x 2 of 4096 68 / 74, 16384 x 1 of 5120 80 / 147.  Two pieces a
-// lane measured the same or slower (43, 16, 10, 14, 78).
+// kernel below / all lanes finding all rows / this one: 4096 tokens x 8 rows of 2048 61 / 41 / 35 (4.3 TB/s), 1024 x 8 53 / 16 / 14,
+// 64 x 8 49 / 8 / 8, 1000 x 6 43 / 14 / 12, 8192 x 4 of 2880 92 / 74 / 57; it has too little in flight with fewer rows: 8192 x 2 of
+// 4096 68 below and 74 here, 16384 x 1 of 5120 80 and 147.  Two pieces a lane measured the same or slower (43, 16, 10, 14, 78).
 __global__ void __launch_bounds__(256)
 moe_combine8_kernel(CombineArgs a, const int* __restrict__ idx, const int* __restrict__ sent_row,
                     __nv_bfloat16* __restrict__ out, float* __restrict__ scalar_out) {
@@ -365,16 +365,14 @@ moe_combine8_kernel(CombineArgs a, const int* __restrict__ idx, const int* __res
   const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= a.T) return;
   const int nvec = a.H / 8, v = blockIdx.y * 32 + lane;
+  unsigned long long mine = 0;                  // lane kk finds the kk-th row
+  if (lane < a.k) {
+    const int row = sent_row[t * a.k + lane], owner = a.world > 1 ? idx[t * a.k + lane] / a.El : 0;
+    if (row >= 0) mine = reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(a.y_ptrs[owner]) + (long long)row * a.H);
+  }
   const uint4* src[8];
 #pragma unroll
-  for (int kk = 0; kk < 8; ++kk) {
-    src[kk] = nullptr;
-    if (kk < a.k) {
-      const int e = idx[t * a.k + kk], row = sent_row[t * a.k + kk];
-      if (row >= 0)
-        src[kk] = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.y_ptrs[e / a.El]) + (long long)row * a.H);
-    }
-  }
+  for (int kk = 0; kk < 8; ++kk) src[kk] = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, mine, kk));
   uint4 raw[8];
 #pragma unroll
   for (int kk = 0; kk < 8; ++kk) raw[kk] = src[kk] && v < nvec ? src[kk][v] : make_uint4(0, 0, 0, 0);
@@ -399,9 +397,8 @@ moe_combine8_kernel(CombineArgs a, const int* __restrict__ idx, const int* __res
     reinterpret_cast<uint4*>(out + t * a.H)[v] = o;
   }
   if (scalar_out && blockIdx.y == 0 && lane < a.k) {
-    const int e = idx[t * a.k + lane];
-    const int row = sent_row[t * a.k + lane];
-    scalar_out[t * a.k + lane] = (row >= 0 && a.scalar_ptrs[e / a.El]) ? a.scalar_ptrs[e / a.El][row] : 0.f;
+    const int row = sent_row[t * a.k + lane], owner = a.world > 1 ? idx[t * a.k + lane] / a.El : 0;
+    scalar_out[t * a.k + lane] = (row >= 0 && a.scalar_ptrs[owner]) ? a.scalar_ptrs[owner][row] : 0.f;
   }
 }
 
