@@ -65,6 +65,19 @@ def test_norm_backward_with_the_next_rows_in_flight(rows, H):
         assert _rel(a, b) < 2 ** -8
 
 
+@pytest.mark.parametrize('rows,H', [(1, 8), (9500, 136), (20000, 256), (2500, 264), (1300, 4096), (1200, 8192)])
+@pytest.mark.parametrize('zero_centered', [False, True])
+def test_norm_forward_with_the_next_row_in_flight(rows, H, zero_centered):
+    from mcore_bridge_b200.ops.norm import rmsnorm
+    x, w = _rand(rows, H), _rand(H, seed=3)
+    y = rmsnorm(x, w, 1e-6, zero_centered)
+    wide = x.double()
+    ref = wide * torch.rsqrt(wide.pow(2).mean(-1, keepdim=True) + 1e-6) * (w.double() + (1 if zero_centered else 0))
+    assert _rel(y, ref) < 2 ** -8                                        # rounded once
+    for rows_of in (slice(0, 1), slice(rows - 3, rows)):                 # every row has the bits it has alone
+        assert torch.equal(rmsnorm(x[rows_of], w, 1e-6, zero_centered), y[rows_of])
+
+
 @pytest.mark.parametrize('T,ng,qpg,gate', [(1, 1, 1, False), (2, 16, 3, False), (333, 1, 2, True), (7, 300, 1, False), (2500, 3, 1, False)])
 @pytest.mark.parametrize('norm', [False, True])
 def test_heads_of_128(T, ng, qpg, gate, norm):
