@@ -6,6 +6,7 @@
 //
 // Packed sequences are described by `seq_start[t]` (index of the first token of t's sequence), as in the attention
 // kernels: no host synchronisation, histories never cross a sequence boundary.
+#include <initializer_list>
 #include "../common/host_utils.cuh"
 #include "../common/ptx.cuh"
 
@@ -176,79 +177,152 @@ __global__ void conv1d_silu_bwd_kernel(const __nv_bfloat16* __restrict__ x, cons
 }
 
 // ------------------------------------------------------------------------------------------ gated RMSNorm
-// rows x D (D = 64, 128 or 256): one warp per row.  y = x * rstd * w * silu(z)
-template <int D>
-__global__ void gated_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ z,
-                                         const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                         float* __restrict__ rstd, long long rows, float eps) {
-  constexpr int PER = D / 32;
-  const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  float xv[PER], zv[PER];
-  float ss = 0.f;
+// rows x D (D = 64, 128 or 256), D / 8 lanes to a row, eight columns a lane; the warp's next rows are loaded while it works on these.
+// y = x * rstd * w * silu(z).  WIDE: all tensors start on 16-byte boundaries.  us, a warp to a row, two bytes a lane / now, forward and
+// backward: 131072 x 128 31, 47 / 25, 39, x 64 22, 35 / 16, 23; 65536 x 256 31, 47 / 25, 39.
+template <bool WIDE>
+__device__ __forceinline__ uint4 row8(const __nv_bfloat16* p) {
+  if (WIDE) return *reinterpret_cast<const uint4*>(p);
+  uint32_t v[4];
+  const uint16_t* h = reinterpret_cast<const uint16_t*>(p);
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    xv[i] = __bfloat162float(x[row * D + lane + 32 * i]);
-    zv[i] = __bfloat162float(z[row * D + lane + 32 * i]);
-    ss += xv[i] * xv[i];
-  }
-  ss = wsum(ss);
-  const float r = rsqrtf(ss / D + eps);
+  for (int i = 0; i < 4; ++i) v[i] = h[2 * i] | (uint32_t)h[2 * i + 1] << 16;
+  return make_uint4(v[0], v[1], v[2], v[3]);
+}
+template <bool WIDE>
+__device__ __forceinline__ void put_row8(__nv_bfloat16* p, const float (&f)[8]) {
+  if (WIDE) {
+    store8(p, f);
+  } else {
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    // the normalised value is rounded to bf16 before the weight multiply, as the module it replaces does
-    const float n = __bfloat162float(__float2bfloat16(xv[i] * r));
-    const float wv = __bfloat162float(w[lane + 32 * i]);
-    y[row * D + lane + 32 * i] = __float2bfloat16(wv * n * zv[i] * sigmoidf_(zv[i]));
+    for (int i = 0; i < 8; ++i) p[i] = __float2bfloat16(f[i]);
   }
-  if (lane == 0) rstd[row] = r;
+}
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[i]));
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+template <int LANES>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+  for (int o = LANES / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-template <int D>
-__global__ void gated_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ z,
-                                         const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ dy,
-                                         const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
-                                         __nv_bfloat16* __restrict__ dz, float* __restrict__ dw, long long rows) {
-  constexpr int PER = D / 32;
+template <int D, bool WIDE>
+__global__ void __launch_bounds__(256, 5)
+gated_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ z, const __nv_bfloat16* __restrict__ w,
+                         __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, long long rows, float eps) {
+  constexpr int LANES = D / 8, PER = 32 / LANES;            // rows of a warp
+  const int lane = threadIdx.x & 31, c0 = lane % LANES * 8;
+  const long long step = (((long long)gridDim.x * blockDim.x) >> 5) * PER;
+  long long first = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * PER;   // of the warp
+  float wv[8];
+  unpack8(row8<WIDE>(w + c0), wv);
+  uint4 xr, zr;
+  auto fetch = [&](long long row) {
+    xr = zr = make_uint4(0, 0, 0, 0);
+    if (row >= rows) return;
+    xr = row8<WIDE>(x + row * D + c0);
+    zr = row8<WIDE>(z + row * D + c0);
+  };
+  fetch(first + lane / LANES);
+  for (; first < rows; first += step) {
+    const long long row = first + lane / LANES;
+    float xv[8], zv[8], o[8], ss = 0.f;
+    unpack8(xr, xv);
+    unpack8(zr, zv);
+    fetch(row + step);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += xv[i] * xv[i];
+    const float r = rsqrtf(group_sum<LANES>(ss) / D + eps);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      // the normalised value is rounded to bf16 before the weight multiply, as the module it replaces does
+      const float n = __bfloat162float(__float2bfloat16(xv[i] * r));
+      o[i] = wv[i] * n * zv[i] * sigmoidf_(zv[i]);
+    }
+    if (row < rows) {
+      put_row8<WIDE>(y + row * D + c0, o);
+      if (c0 == 0) rstd[row] = r;
+    }
+  }
+}
+
+template <int D, bool WIDE>
+__global__ void __launch_bounds__(256)
+gated_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ z, const __nv_bfloat16* __restrict__ w,
+                         const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
+                         __nv_bfloat16* __restrict__ dz, float* __restrict__ dw, long long rows) {
+  constexpr int LANES = D / 8, PER = 32 / LANES;
   __shared__ float dws[D];
   for (int i = threadIdx.x; i < D; i += blockDim.x) dws[i] = 0.f;
   __syncthreads();
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  float dwl[PER];
+  const int lane = threadIdx.x & 31, c0 = lane % LANES * 8;
+  const long long step = (((long long)gridDim.x * blockDim.x) >> 5) * PER;
+  long long first = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * PER;
+  float wv[8], dwl[8] = {};
+  unpack8(row8<WIDE>(w + c0), wv);
+  uint4 xr, zr, gr;
+  float rr = 0.f;
+  auto fetch = [&](long long row) {
+    xr = zr = gr = make_uint4(0, 0, 0, 0);
+    if (row >= rows) return;
+    xr = row8<WIDE>(x + row * D + c0);
+    zr = row8<WIDE>(z + row * D + c0);
+    gr = row8<WIDE>(dy + row * D + c0);
+    rr = rstd[row];
+  };
+  fetch(first + lane / LANES);
+  for (; first < rows; first += step) {
+    const long long row = first + lane / LANES;
+    const float r = rr;
+    float xv[8], zv[8], gv[8], gz[8], dn[8], dot = 0.f;
+    unpack8(xr, xv);
+    unpack8(zr, zv);
+    unpack8(gr, gv);
+    fetch(row + step);
 #pragma unroll
-  for (int i = 0; i < PER; ++i) dwl[i] = 0.f;
-  for (long long row = (long long)blockIdx.x * nw + wib; row < rows; row += (long long)gridDim.x * nw) {
-    const float r = rstd[row];
-    float xv[PER], gz[PER], dn[PER];
-    float dot = 0.f;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int c = lane + 32 * i;
-      xv[i] = __bfloat162float(x[row * D + c]);
-      const float zv = __bfloat162float(z[row * D + c]);
-      const float g = __bfloat162float(dy[row * D + c]);
-      const float wv = __bfloat162float(w[c]);
-      const float s = sigmoidf_(zv);
+    for (int i = 0; i < 8; ++i) {
+      const float s = sigmoidf_(zv[i]);
       const float n = xv[i] * r;
-      gz[i] = g * wv * n * s * (1.f + zv * (1.f - s));     // d/dz of silu(z)
-      dn[i] = g * wv * zv * s;                             // gradient w.r.t. the normalised value
-      dwl[i] += g * n * zv * s;
+      gz[i] = gv[i] * wv[i] * n * s * (1.f + zv[i] * (1.f - s));     // d/dz of silu(z)
+      dn[i] = gv[i] * wv[i] * zv[i] * s;                             // gradient w.r.t. the normalised value
+      dwl[i] += gv[i] * n * zv[i] * s;
       dot += dn[i] * xv[i];
     }
-    dot = wsum(dot);
-    const float k = dot * r * r * r / D;
+    const float k = group_sum<LANES>(dot) * r * r * r / D;
+    if (row < rows) {
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int c = lane + 32 * i;
-      dx[row * D + c] = __float2bfloat16(dn[i] * r - xv[i] * k);
-      dz[row * D + c] = __float2bfloat16(gz[i]);
+      for (int i = 0; i < 8; ++i) dn[i] = dn[i] * r - xv[i] * k;
+      put_row8<WIDE>(dx + row * D + c0, dn);
+      put_row8<WIDE>(dz + row * D + c0, gz);
     }
   }
 #pragma unroll
-  for (int i = 0; i < PER; ++i) atomicAdd(&dws[lane + 32 * i], dwl[i]);
+  for (int i = 0; i < 8; ++i) {
+#pragma unroll
+    for (int o = LANES; o < 32; o <<= 1) dwl[i] += __shfl_xor_sync(0xffffffffu, dwl[i], o);
+    if (lane < LANES) atomicAdd(&dws[c0 + i], dwl[i]);
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < D; i += blockDim.x) atomicAdd(&dw[i], dws[i]);
+}
+
+bool on_16_bytes(std::initializer_list<const void*> ps) {
+  uintptr_t bits = 0;
+  for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
+  return bits % 16 == 0;
+}
+// CTAs for warps of `rows_of_warp` rows, no more than what an SM holds
+unsigned row_grid(long long rows, int rows_of_warp, int ctas_per_sm) {
+  const long long want = (rows + 8 * rows_of_warp - 1) / (8 * rows_of_warp), cap = (long long)ctas_per_sm * device_sm_count();
+  return (unsigned)(want < cap ? want : cap);
 }
 
 }  // namespace
@@ -299,10 +373,11 @@ int mcb_gated_rmsnorm_fwd(const void* x, const void* z, const void* w, void* y, 
                           float eps, void* stream_) {
   if (rows == 0) return 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  const unsigned grid = (unsigned)((rows + 7) / 8);
+  const bool wide = on_16_bytes({x, z, w, y});
 #define MCB_GN_FWD(D_)                                                                                               \
-  gated_rmsnorm_fwd_kernel<D_><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)z,                 \
-                                                    (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rstd, rows, eps)
+  (wide ? gated_rmsnorm_fwd_kernel<D_, true> : gated_rmsnorm_fwd_kernel<D_, false>)                                  \
+      <<<row_grid(rows, 256 / D_, 5), 256, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)z, (const __nv_bfloat16*)w,   \
+                                                   (__nv_bfloat16*)y, rstd, rows, eps)
   if (D == 128) MCB_GN_FWD(128);
   else if (D == 64) MCB_GN_FWD(64);
   else if (D == 256) MCB_GN_FWD(256);
@@ -316,12 +391,11 @@ int mcb_gated_rmsnorm_bwd(const void* x, const void* z, const void* w, const voi
                           void* dz, float* dw, long long rows, int D, void* stream_) {
   if (rows == 0) return 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  const long long want = (rows + 7) / 8;
-  const unsigned grid = (unsigned)(want < 4LL * device_sm_count() ? want : 4LL * device_sm_count());
+  const bool wide = on_16_bytes({x, z, w, dy, dx, dz});
 #define MCB_GN_BWD(D_)                                                                                               \
-  gated_rmsnorm_bwd_kernel<D_><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)z,                 \
-                                                    (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, rstd,          \
-                                                    (__nv_bfloat16*)dx, (__nv_bfloat16*)dz, dw, rows)
+  (wide ? gated_rmsnorm_bwd_kernel<D_, true> : gated_rmsnorm_bwd_kernel<D_, false>)                                  \
+      <<<row_grid(rows, 256 / D_, 3), 256, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)z, (const __nv_bfloat16*)w,   \
+                                                   (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx, (__nv_bfloat16*)dz, dw, rows)
   if (D == 128) MCB_GN_BWD(128);
   else if (D == 64) MCB_GN_BWD(64);
   else if (D == 256) MCB_GN_BWD(256);

@@ -107,3 +107,23 @@ def test_heads_of_128(T, ng, qpg, gate, norm):
     buf[2:] = buf[:-2].clone()                                           # four bytes from any wider boundary
     for a, b in zip(run(buf[2:].view(T, W).detach(), single, ws), got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize('rows,D', [(1, 128), (77, 64), (9001, 128), (5, 256), (3001, 256), (20001, 64)])
+def test_gated_norm(rows, D):
+    from mcore_bridge_b200.ops import gdn
+    x, z, dy, w = _rand(rows, D), _rand(rows, D, seed=1), _rand(rows, D, seed=2), _rand(D, seed=3)
+
+    def run(x, z, w, dy):
+        leaves = [t.detach().requires_grad_() for t in (x, z, w)]
+        y = gdn.gated_rmsnorm(*leaves, 1e-6)
+        return [y, *torch.autograd.grad(y, leaves, dy)]
+
+    wide = [t.double().requires_grad_() for t in (x, z, w)]
+    ref = wide[0] * torch.rsqrt(wide[0].pow(2).mean(-1, keepdim=True) + 1e-6) * wide[2] * torch.nn.functional.silu(wide[1])
+    got = run(x, z, w, dy)
+    for a, b in zip(got, [ref, *torch.autograd.grad(ref, wide, dy.double())]):
+        assert _rel(a, b) < 2 ** -7                                      # rounded once, and the normalised value before it
+    odd = [torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(t.shape) for t in (x, z, w, dy)]      # two bytes from a wider boundary
+    for i, (a, b) in enumerate(zip(run(*odd), got)):
+        assert torch.equal(a, b) or (i == 3 and _rel(a, b) < 2 ** -8)    # the weight's gradient is summed with atomics
