@@ -42,7 +42,7 @@
 // 307 (of the first).  No change from starting the strips apart, slower with the operands of M and P fetched before the
 // strip's barrier (162, 335, 367: registers) and with 8 + 8 tokens a warp, for which M and P have as many blocks in each (145,
 // 231, 274: more instructions).
-// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.22 ms (prep 0.08), backward 0.72 ms (grad 0.28).  The batched
+// Measured, 4096 tokens in three sequences, 32 heads of 128: forward 0.19 ms (prep 0.06), backward 0.72 ms (grad 0.28).  The batched
 // torch evaluation of the rule was most of a 29.5 ms block.
 #include "../common/host_utils.cuh"
 #include "warp_mma.cuh"
@@ -105,7 +105,7 @@ __device__ __forceinline__ float nonzero(float b) { return fabsf(b) < 0x1p-40f ?
 
 // ---------------------------------------------------------------------------------------------------- prep
 template <int D>
-constexpr int PREP_TILES = 2 * C * D * 2 > MP * C * 72 * 2 ? 2 * C * D * 2 : MP * C * 72 * 2;   // q and k, later M's terms
+constexpr int PREP_TILES = 2 * C * D * 2 > C * (C + 4) * 4 ? 2 * C * D * 2 : C * (C + 4) * 4;   // q and k, later I + M
 
 template <int D>
 __global__ void __launch_bounds__(THREADS)
@@ -198,39 +198,90 @@ gdr_prep_kernel(const GdrParams p) {
     }
   }
   __syncthreads();
-  // I + M = (I + L beta)^-1, one column a thread by forward substitution (rows are shared-memory broadcasts); the columns meet as
-  // bf16 terms in the q / k tiles, which nothing reads any more
-  __nv_bfloat16* sm = reinterpret_cast<__nv_bfloat16*>(smem_raw + (sq - smem_u32(smem_raw)));  // [MP][64][72]
-  if (threadIdx.x < C) {
-    const int j = threadIdx.x;
-    float x[C];
+  // I + M = (I + A)^-1 in blocks of 16: X_ii by forward substitution, a block to a warp, then X_ij = -X_ii sum_k A_ik X_kj row block by
+  // row block.  A warp has four columns of every block column, so that nothing but its own results goes into its next ones.
+  // X takes the place of the q / k tiles, which nothing reads any more.  A column to a thread, 64 rows one after the other, was 25000 of
+  // the kernel's 43000 cycles: 4096 tokens, 32 heads of 128 84 -> 61 us, of 64 75 -> 47, 200 tokens, 4 heads 16 -> 11.
+  float* sX = reinterpret_cast<float*>(smem_raw + (sq - smem_u32(smem_raw)));  // [64][LDA]
+  if (lane < 16) {
+    const float* A = sA + r0 * LDA + r0;
+    float x[16];
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      float s0 = r == j ? 1.f : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    for (int r = 0; r < 16; ++r) {
+      float s0 = r == lane ? 1.f : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
       for (int c = 0; c < r; c += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(sA + r * LDA + c);
+        const float4 a = *reinterpret_cast<const float4*>(A + r * LDA + c);
         s0 = fmaf(-a.x, x[c], s0);
         if (c + 1 < r) s1 = fmaf(-a.y, x[c + 1], s1);
         if (c + 2 < r) s2 = fmaf(-a.z, x[c + 2], s2);
         if (c + 3 < r) s3 = fmaf(-a.w, x[c + 3], s3);
       }
       x[r] = (s0 + s1) + (s2 + s3);
-      float rest = r == j ? 0.f : x[r];
-#pragma unroll
-      for (int m = 0; m < MP; ++m) {
-        const __nv_bfloat16 t = __float2bfloat16(rest);
-        sm[m * C * 72 + r * 72 + j] = t;
-        rest -= __bfloat162float(t);
-      }
+      sX[(r0 + r) * LDA + r0 + lane] = x[r];
     }
   }
   __syncthreads();
-  for (int id = threadIdx.x; id < MP * C * 8; id += THREADS) {
-    const int m = id >> 9, r = (id >> 3) & 63, c = (id & 7) * 8;
-    if ((c >> 4) <= (r >> 4))
-      *reinterpret_cast<uint4*>(mp + (m * SQB + block_off(r >> 4, c >> 4, r & 15, (c >> 3) & 1)) / 2) =
-          *reinterpret_cast<const uint4*>(sm + m * C * 72 + r * 72 + c);
+  {
+    const int row = lane >> 1, col = warp * 4 + (lane & 1) * 2;
+    // out += a[row][0 .. 15] x[0 .. 15][col, col + 1]
+    auto block = [&](float2& out, const float* a, const float* x) {
+#pragma unroll
+      for (int t = 0; t < 16; t += 4) {
+        const float4 f = *reinterpret_cast<const float4*>(a + row * LDA + t);
+        const float w[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float2 g = *reinterpret_cast<const float2*>(x + (t + u) * LDA + col);
+          out.x = fmaf(w[u], g.x, out.x);
+          out.y = fmaf(w[u], g.y, out.y);
+        }
+      }
+    };
+#pragma unroll
+    for (int ib = 1; ib < 4; ++ib) {
+      float2 y[3];
+#pragma unroll
+      for (int jb = 0; jb < ib; ++jb) {
+        float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int kb = jb; kb < ib; ++kb) block(sum, sA + ib * 16 * LDA + kb * 16, sX + kb * 16 * LDA + jb * 16);
+        *reinterpret_cast<float2*>(sX + (ib * 16 + row) * LDA + jb * 16 + col) = sum;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int jb = 0; jb < ib; ++jb) {
+        y[jb] = make_float2(0.f, 0.f);
+        block(y[jb], sX + ib * 16 * LDA + ib * 16, sX + ib * 16 * LDA + jb * 16);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int jb = 0; jb < ib; ++jb) *reinterpret_cast<float2*>(sX + (ib * 16 + row) * LDA + jb * 16 + col) = make_float2(-y[jb].x, -y[jb].y);
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (int id = threadIdx.x; id < C * 8; id += THREADS) {
+    const int r = id >> 3, c = (id & 7) * 8;
+    if ((c >> 4) > (r >> 4)) continue;
+    const float4 u = *reinterpret_cast<const float4*>(sX + r * LDA + c), v = *reinterpret_cast<const float4*>(sX + r * LDA + c + 4);
+    float rest[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (c + e == r) rest[e] = 0.f;
+#pragma unroll
+    for (int m = 0; m < MP; ++m) {
+      uint32_t t[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 h2 = __floats2bfloat162_rn(rest[2 * e], rest[2 * e + 1]);
+        t[e] = *reinterpret_cast<const uint32_t*>(&h2);
+        const float2 f = __bfloat1622float2(h2);
+        rest[2 * e] -= f.x;
+        rest[2 * e + 1] -= f.y;
+      }
+      *reinterpret_cast<uint4*>(mp + (m * SQB + block_off(r >> 4, c >> 4, r & 15, (c >> 3) & 1)) / 2) = make_uint4(t[0], t[1], t[2], t[3]);
+    }
   }
 }
 
