@@ -136,7 +136,9 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_narrow_kernel(const __nv_bflo
   bf16x8 t, next;
   t.raw = in ? reinterpret_cast<const uint4*>(w)[lane] : make_uint4(0, 0, 0, 0);
   t.unpack(wf);
-  auto fetch = [&](long long row) { next.raw = in && row < rows ? reinterpret_cast<const uint4*>(x + row * ldx)[lane] : make_uint4(0, 0, 0, 0); };
+  auto fetch = [&](long long row) {
+    next.raw = in && row < rows ? reinterpret_cast<const uint4*>(x + row * ldx)[lane] : make_uint4(0, 0, 0, 0);
+  };
   long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   fetch(row);
   for (; row < rows; row += step) {
@@ -235,7 +237,9 @@ __global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1) rmsnorm_bwd_kernel(cons
 #pragma unroll
           for (int i = 0; i < VPT; ++i)
             if ((int)threadIdx.x + i * (int)blockDim.x < nvec)
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(slot(stage, q, r, i))), "l"(src + i * blockDim.x) : "memory");
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(slot(stage, q, r, i))),
+                           "l"(src + i * blockDim.x)
+                           : "memory");
         }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -541,8 +545,8 @@ int mcb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, void* y, v
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
   if (H <= 256 && !res_in) {
     const long long blocks = (rows + 7) / 8, cap = (long long)device_sm_count() * 8;
-    rmsnorm_fwd_narrow_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y,
-                                                                              rstd, rows, H, ldx, eps, zero_centered);
+    rmsnorm_fwd_narrow_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, s>>>(
+        (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rstd, rows, H, ldx, eps, zero_centered);
     return (int)cudaGetLastError();
   }
   int vpt, threads = pick_threads(H, &vpt);

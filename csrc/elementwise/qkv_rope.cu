@@ -388,7 +388,8 @@ qkv_fwd_fast_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
     }
     fetch(t + h.step);
     if (L.norm) {
-      const float ss = head_sum(a[0] * a[0] + a[1] * a[1] + b[0] * b[0] + b[1] * b[1], a[2] * a[2] + a[3] * a[3] + b[2] * b[2] + b[3] * b[3]);
+      const float ss = head_sum(a[0] * a[0] + a[1] * a[1] + b[0] * b[0] + b[1] * b[1],
+                                a[2] * a[2] + a[3] * a[3] + b[2] * b[2] + b[3] * b[3]);
       const float rstd = rsqrtf(ss * (1.f / D) + L.eps);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -466,7 +467,8 @@ qkv_bwd_fast_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
     }
     fetch(t + h.step);
     if (L.norm) {
-      const float ss = head_sum(x[0] * x[0] + x[1] * x[1] + y[0] * y[0] + y[1] * y[1], x[2] * x[2] + x[3] * x[3] + y[2] * y[2] + y[3] * y[3]);
+      const float ss = head_sum(x[0] * x[0] + x[1] * x[1] + y[0] * y[0] + y[1] * y[1],
+                                x[2] * x[2] + x[3] * x[3] + y[2] * y[2] + y[3] * y[3]);
       const float dot = head_sum(na[0] * wa[0] * x[0] + na[1] * wa[1] * x[1] + nb[0] * wb[0] * y[0] + nb[1] * wb[1] * y[1],
                                  na[2] * wa[2] * x[2] + na[3] * wa[3] * x[3] + nb[2] * wb[2] * y[2] + nb[3] * wb[3] * y[3]);
       const float rstd = rsqrtf(ss * (1.f / D) + L.eps);

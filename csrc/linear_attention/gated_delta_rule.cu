@@ -193,7 +193,8 @@ gdr_prep_kernel(const GdrParams p) {
 #pragma unroll
         for (int m = 0; m < MP; ++m)
           if (jb <= warp)
-            *reinterpret_cast<uint32_t*>(mp + MP * CC + (m * SQB + block_off(warp, jb, (lane >> 2) + 8 * r, n)) / 2 + (lane & 3) * 2) = t[m][0];
+            *reinterpret_cast<uint32_t*>(mp + MP * CC + (m * SQB + block_off(warp, jb, (lane >> 2) + 8 * r, n)) / 2 +
+                                         (lane & 3) * 2) = t[m][0];
       }
     }
   }
@@ -256,7 +257,8 @@ gdr_prep_kernel(const GdrParams p) {
       }
       __syncwarp();
 #pragma unroll
-      for (int jb = 0; jb < ib; ++jb) *reinterpret_cast<float2*>(sX + (ib * 16 + row) * LDA + jb * 16 + col) = make_float2(-y[jb].x, -y[jb].y);
+      for (int jb = 0; jb < ib; ++jb)
+        *reinterpret_cast<float2*>(sX + (ib * 16 + row) * LDA + jb * 16 + col) = make_float2(-y[jb].x, -y[jb].y);
       __syncwarp();
     }
   }
@@ -322,7 +324,8 @@ struct StageLoad {
     xat = tile_addr<64>(0, xrow, (threadIdx.x & 7) * 8);
   }
   // by all threads; the mbarriers `full` (tiles, gb) and full + 16 (M and P) have counts of ST + 1 and 1
-  __device__ __forceinline__ void operator()(uint32_t st, uint32_t full, const GdrParams& p, int t, int len, int h, int col0, long long ch) const {
+  __device__ __forceinline__ void operator()(uint32_t st, uint32_t full, const GdrParams& p, int t, int len, int h, int col0,
+                                             long long ch) const {
     static_assert(ROWS % 8 == 0, "the same place in the swizzle");
     if (threadIdx.x == 0) {
       mbar_expect_tx(full, 4 * C * 4);
@@ -463,7 +466,9 @@ struct ScanRing {
     __syncthreads();
   }
   // a wait that gives up reports it and the walk goes on, with what is there, to its end: the barriers of a strip stay whole
-  __device__ __forceinline__ void wait_full(int i) { mbar_wait_warp(full + 8 * (i & 1), (i >> 1) & 1, abort_flag, status, ST_TIMEOUT_FULL); }
+  __device__ __forceinline__ void wait_full(int i) {
+    mbar_wait_warp(full + 8 * (i & 1), (i >> 1) & 1, abort_flag, status, ST_TIMEOUT_FULL);
+  }
   __device__ __forceinline__ void wait_squares(int i) {
     mbar_wait_warp(full + 16 + 8 * (i & 1), (i >> 1) & 1, abort_flag, status, ST_TIMEOUT_FULL);
   }
@@ -1230,7 +1235,8 @@ gdr_grad_kernel(const GdrParams p) {
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
         float E[4];
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(E[0]), "=f"(E[1]), "=f"(E[2]), "=f"(E[3]) : "r"(ex + n * 512) : "memory");
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(E[0]), "=f"(E[1]), "=f"(E[2]), "=f"(E[3])
+                     : "r"(ex + n * 512) : "memory");
 #pragma unroll
         for (int e = 0; e < 4; ++e) out[n][e] = fmaf(-eg[e >> 1], E[e], out[n][e]);
       }

@@ -368,7 +368,8 @@ moe_combine8_kernel(CombineArgs a, const int* __restrict__ idx, const int* __res
   unsigned long long mine = 0;                  // lane kk finds the kk-th row
   if (lane < a.k) {
     const int row = sent_row[t * a.k + lane], owner = a.world > 1 ? idx[t * a.k + lane] / a.El : 0;
-    if (row >= 0) mine = reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(a.y_ptrs[owner]) + (long long)row * a.H);
+    if (row >= 0)
+      mine = reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(a.y_ptrs[owner]) + (long long)row * a.H);
   }
   const uint4* src[8];
 #pragma unroll

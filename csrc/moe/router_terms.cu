@@ -33,8 +33,8 @@ router_aux_kernel(const int* __restrict__ counts, const float* __restrict__ scor
   }
 }
 
-__global__ void router_aux_bwd_kernel(const float* __restrict__ g, const float* __restrict__ frac, float* __restrict__ out, int E, float tokens,
-                                      float c) {
+__global__ void router_aux_bwd_kernel(const float* __restrict__ g, const float* __restrict__ frac, float* __restrict__ out, int E,
+                                      float tokens, float c) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < E) out[e] = (g[0] * c * frac[e]) / tokens;
 }

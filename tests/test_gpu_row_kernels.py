@@ -47,10 +47,10 @@ def test_norm_backward_with_the_next_rows_in_flight(rows, H):
     def backward(first, last, res, with_y):
         n = last - first
         part = torch.empty(lib.mcb_rmsnorm_bwd_partial_rows(ll(n), H), H, device=DEV)
-        d, dx, dw = dy[first:last].clone(), torch.empty(n, H, device=DEV, dtype=torch.bfloat16), torch.empty(H, device=DEV).bfloat16()
+        d, dx, dw = dy[first:last].clone(), torch.empty_like(dy[first:last]), torch.empty_like(w)
         f = lib.mcb_rmsnorm_bwd_det_y if with_y else lib.mcb_rmsnorm_bwd_det
-        assert f(ptr(d), ptr(x[first:]), ptr(w), ptr(rstd[first:]), ptr(None if res is None else res[first:]), ptr(dx), ptr(dw), 1, ptr(part),
-                 ll(n), H, ll(H), ctypes.c_float(1e-6), 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        assert f(ptr(d), ptr(x[first:]), ptr(w), ptr(rstd[first:]), ptr(None if res is None else res[first:]), ptr(dx), ptr(dw),
+                 1, ptr(part), ll(n), H, ll(H), ctypes.c_float(1e-6), 0, _lib.stream_ptr()) == 0
         return dx, dw, d
 
     dx, dw, _ = backward(0, rows, None, False)
@@ -89,7 +89,8 @@ def test_heads_of_128(T, ng, qpg, gate, norm):
 
     def run(qkv, f, ws):
         leaves = [t.requires_grad_() for t in (qkv, *ws) if t is not None]
-        outs = [t for t in f(qkv, ws[0], ws[1], cos.to(qkv.dtype), sin.to(qkv.dtype), ng, qpg, 128, gate, False, 1e-6, False) if t is not None]
+        outs = f(qkv, ws[0], ws[1], cos.to(qkv.dtype), sin.to(qkv.dtype), ng, qpg, 128, gate, False, 1e-6, False)
+        outs = [t for t in outs if t is not None]
         gen = torch.Generator(device=DEV).manual_seed(5)
         seeds = [torch.randn(t.shape, generator=gen, device=DEV).bfloat16().to(t.dtype) for t in outs]
         return outs + list(torch.autograd.grad(outs, leaves, seeds))
