@@ -353,11 +353,12 @@ struct CombineArgs {
   const float* scalar_ptrs[MAX_WORLD]; // optional per-row scalar on the owner (e.g. d(prob))
 };
 
-// The sums of moe_combine_kernel below, in the same order, for 4 to 8 rows a token: a lane finds each of them, then one 16-byte piece
+// The sums of moe_combine_kernel below, in the same order, for 2 to 8 rows a token: a lane finds each of them, then one 16-byte piece
 // of each is in flight per lane; blockIdx.y takes runs of 32 pieces, which gives few tokens more warps.  Bound: the reads.  us, the
 // kernel below / all lanes finding all rows / this one: 4096 tokens x 8 rows of 2048 61 / 41 / 35 (4.3 TB/s), 1024 x 8 53 / 16 / 14,
-// 64 x 8 49 / 8 / 8, 1000 x 6 43 / 14 / 12, 8192 x 4 of 2880 92 / 74 / 57; it has too little in flight with fewer rows: 8192 x 2 of
-// 4096 68 below and 74 here, 16384 x 1 of 5120 80 and 147.  Two pieces a lane measured the same or slower (43, 16, 10, 14, 78).
+// 64 x 8 49 / 8 / 8, 1000 x 6 43 / 14 / 12, 8192 x 4 of 2880 92 / 74 / 57, 4096 x 3 of 2048 30 / - / 22, 8192 x 2 of 4096 67 / 74 / 59,
+// 300 x 2 of 2048 18 / - / 8.  With one row a token there is too little in flight: 16384 x 1 of 5120 80 below and 127 here.  Two
+// pieces a lane measured the same or slower (43, 16, 10, 14, 78).
 __global__ void __launch_bounds__(256)
 moe_combine8_kernel(CombineArgs a, const int* __restrict__ idx, const int* __restrict__ sent_row,
                     __nv_bfloat16* __restrict__ out, float* __restrict__ scalar_out) {
@@ -581,7 +582,7 @@ int mcb_moe_combine(const void* const* y_ptrs, const float* const* scalar_ptrs, 
     a.scalar_ptrs[i] = scalar_ptrs ? scalar_ptrs[i] : nullptr;
   }
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  if (k >= 4 && k <= 8)
+  if (k >= 2 && k <= 8)
     moe_combine8_kernel<<<dim3((unsigned)((T + 7) / 8), (unsigned)((H / 8 + 31) / 32)), 256, 0, s>>>(a, idx, sent_row,
                                                                                                     (__nv_bfloat16*)out, scalar_out);
   else

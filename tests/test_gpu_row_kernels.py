@@ -128,3 +128,22 @@ def test_gated_norm(rows, D):
     odd = [torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(t.shape) for t in (x, z, w, dy)]      # two bytes from a wider boundary
     for i, (a, b) in enumerate(zip(run(*odd), got)):
         assert torch.equal(a, b) or (i == 3 and _rel(a, b) < 2 ** -8)    # the weight's gradient is summed with atomics
+
+
+@pytest.mark.parametrize('T,k,H', [(1, 1, 8), (100, 2, 264), (7, 3, 2048), (33, 5, 512), (300, 8, 520), (9, 9, 256)])
+def test_combined_rows(T, k, H):
+    from mcore_bridge_b200.ops import _lib
+    rows = T * k
+    y, idx = _rand(rows, H), torch.zeros(T, k, dtype=torch.int32, device=DEV)
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    sent = torch.randperm(rows, generator=gen, device=DEV).view(T, k).int()
+    sent[torch.rand(T, k, generator=gen, device=DEV) < 0.1] = -1                         # entries that were not sent
+    scalars, out, probs = torch.rand(rows, device=DEV), torch.empty(T, H, device=DEV).bfloat16(), torch.empty(T, k, device=DEV)
+    tables = [(ctypes.c_void_p * 1)(t.data_ptr()) for t in (y, scalars)]
+    assert _lib.lib().mcb_moe_combine(*tables, *map(ctypes.c_int, (1, T, k, 4, H)), _lib.ptr(idx), _lib.ptr(sent), _lib.ptr(out),
+                                      _lib.ptr(probs), _lib.stream_ptr()) == 0
+    want = torch.zeros(T, H, device=DEV)
+    for j in range(k):
+        want += torch.where(sent[:, j, None] >= 0, y[sent[:, j].clamp(min=0).long()].float(), 0.0)
+    assert torch.equal(out, want.bfloat16())
+    assert torch.equal(probs, torch.where(sent >= 0, scalars[sent.clamp(min=0).long()], 0.0))
