@@ -10,17 +10,17 @@
 // launches: `walk` forms the states at the edges, `result` computes every tile and result independently.  States are fp32
 // sums, kept as two bf16 terms (64 KB per edge and head at d = 128; 128-token tiles keep that traffic at half of the
 // inputs') and enter the products as these; weights and weighted scores are split the same way: against fp64 the bf16
-// results are off by 0.00166, their own rounding, as token by token in fp32.
+// results are off by 0.00166, their own rounding.  Batches of fewer than 16 tokens a sequence are evaluated token by token in fp32
+// (by_token).
 //
-// Measured, us, inputs not in the L2, heads of 128 (64): against kernels with warp-level MMAs on chunks of one sequence each (states
-// by one kernel for all chunks and a prefix sum) and token-by-token kernels below 16 tokens a sequence
+// Measured, us, inputs not in the L2, heads of 128 (64), against kernels with warp-level MMAs on chunks of one sequence each (states
+// by one kernel for all chunks and a prefix sum)
 //                                          forward before    now         backward before   now
 //   4096 tokens, sequences of 2926 and 1170, 16 heads    87 (48)   52 (42)       183 (79)    83 (56)
 //   16384 in one, 32 heads                              544 (234) 241 (161)     1318 (495)  482 (273)
 //   8192 in sequences of 1024, 16 heads                 144 (62)   79 (46)       331 (130)  130 (85)
 //                        128                             83 (44)   62 (40)       148 (83)   105 (71)
 //                         16                            226 (101)  73 (44)       470 (194)  132 (83)
-//                          8                            457 (115)  71 (44)      1084 (270)  132 (83)
 //   8192 in one, 4 heads (the chain of `walk`)           64 (44)   62 (58)       114 (62)    73 (67)
 //
 // Packed sequences are described by cu_seqlens on the device; nothing waits for the host.
@@ -741,8 +741,97 @@ gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const
   }
 }
 
+// ---------------------------------------------------------------------------------------------------- short sequences
+// Token by token: one CTA of D threads per (sequence, head), thread j keeps column j of the state S [D x D] in registers.  q
+// and k of the current token are staged in shared memory (double buffered) so every thread reads them as broadcasts.
+template <int D>
+__global__ void __launch_bounds__(D)
+gla_token_fwd_kernel(const GlaParams p) {
+  __shared__ float qs[2][D], ks[2][D];
+  const int h = blockIdx.y, j = threadIdx.x;
+  if (h == 0) check_bounds(p.cu, p.n_seq, p.T, p.status);
+  const int2 span = seq_span(p.cu, blockIdx.x, p.T);
+  const float a = __expf(p.decay[h]);
+  const __nv_bfloat16 *__restrict__ q = p.q, *__restrict__ k = p.k, *__restrict__ v = p.v;
+  __nv_bfloat16* __restrict__ o = p.o;
+  float S[D];
+#pragma unroll
+  for (int i = 0; i < D; ++i) S[i] = 0.f;
+  auto stage = [&](int t, int b) {
+    const long long at = ((long long)t * p.H + h) * D + j;
+    qs[b][j] = __bfloat162float(q[at]) * p.scale;
+    ks[b][j] = __bfloat162float(k[at]);
+  };
+  if (span.x < span.y) stage(span.x, 0);
+  __syncthreads();
+  for (int t = span.x; t < span.y; ++t) {
+    const int b = (t - span.x) & 1;
+    if (t + 1 < span.y) stage(t + 1, b ^ 1);
+    const long long at = ((long long)t * p.H + h) * D + j;
+    const float vj = __bfloat162float(v[at]);
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      S[i] = fmaf(S[i], a, ks[b][i] * vj);
+      acc = fmaf(S[i], qs[b][i], acc);
+    }
+    o[at] = __float2bfloat16(acc);
+    __syncthreads();
+  }
+}
+
+// Backward in three sweeps with no stored states.  Owning rows for dq / dk and columns for dv keeps every reduction inside a
+// thread:
+//   forward, thread = row i of S_t :              dq_t[i] = scale * sum_c S_t[i, c] do_t[c]
+//   reverse, thread = row i of R_t / scale :      dk_t[i] = scale * sum_c (R_t / scale)[i, c] v_t[c]
+//   reverse, thread = column c of R_t / scale :   dv_t[c] = scale * sum_i (R_t / scale)[i, c] k_t[i]
+// Every sweep is  M <- a M + x w^T,  out = scale M z  over one order of the tokens; w and z are shared, x is the thread's own.
+template <int D>
+__global__ void __launch_bounds__(D)
+gla_token_bwd_kernel(const GlaParams p) {
+  __shared__ float ws[D], zs[D];
+  const int h = blockIdx.y, i = threadIdx.x;
+  const int2 span = seq_span(p.cu, blockIdx.x, p.T);
+  const float a = __expf(p.decay[h]);
+  float M[D];
+  auto sweep = [&](bool reverse, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                   const __nv_bfloat16* __restrict__ z, __nv_bfloat16* __restrict__ out) {
+#pragma unroll
+    for (int c = 0; c < D; ++c) M[c] = 0.f;
+    for (int n = span.x; n < span.y; ++n) {
+      const long long at = ((long long)(reverse ? span.x + span.y - 1 - n : n) * p.H + h) * D + i;
+      const float xi = __bfloat162float(x[at]);
+      ws[i] = __bfloat162float(w[at]);
+      zs[i] = __bfloat162float(z[at]);
+      __syncthreads();
+      float acc = 0.f;
+#pragma unroll
+      for (int c = 0; c < D; ++c) {
+        M[c] = fmaf(M[c], a, xi * ws[c]);
+        acc = fmaf(M[c], zs[c], acc);
+      }
+      out[at] = __float2bfloat16(acc * p.scale);
+      __syncthreads();
+    }
+  };
+  sweep(false, p.k, p.v, p.dout, p.dq);
+  sweep(true, p.q, p.dout, p.v, p.dk);
+  sweep(true, p.dout, p.q, p.k, p.dv);
+}
+
+// Batches of fewer than 16 tokens a sequence on average: fp32 throughout, where the tiles' weights, values and states are sums of two
+// bf16 terms.  A result there is a sum of a few products, and those 16 bits show: of 2048 tokens in sequences of 12, 4 heads, 0.0002 of
+// the results are not the exact ones' nearest bf16 values, by tiles 0.0017 (long sequences: 0.0025 either way).
+bool by_token(int T, int n_seq) { return (long long)n_seq * 16 > T; }
+
 template <int D>
 int launch_gla(const GlaParams& p, int T, bool grad, cudaStream_t s) {
+  if (by_token(T, p.n_seq)) {
+    const dim3 seqs(p.n_seq, p.H);
+    if (grad) gla_token_bwd_kernel<D><<<seqs, D, 0, s>>>(p);
+    else gla_token_fwd_kernel<D><<<seqs, D, 0, s>>>(p);
+    return (int)cudaGetLastError();
+  }
   constexpr int W_SMEM = WalkSmem<D>::TOTAL, R_SMEM = ResultSmem<D>::TOTAL;
   static bool cfg = false;
   cudaError_t e;
@@ -797,8 +886,8 @@ int run_gla(const GlaParams& p, int T, int D, bool grad, cudaStream_t s) {
 
 extern "C" {
 
-// Rows of the state workspaces: the edges between a batch's tiles.
-int mcb_simple_gla_edges(int T) { return T > 0 ? (T - 1) / C : 0; }
+// Rows of the state workspaces: the edges between a batch's tiles, none for short sequences.
+int mcb_simple_gla_edges(int T, int n_seq) { return T <= 0 || by_token(T, n_seq) ? 0 : (T - 1) / C; }
 
 // q, k, v, o [T, H, D]; decay [H] fp32 (log-decay per step, <= 0); cu_seqlens [n_seq + 1] int32 from 0 to T;
 // states [edges, H, 2, D, D] bf16 workspace.  Boundaries outside the batch are clipped and reported through `status`.

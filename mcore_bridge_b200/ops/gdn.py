@@ -338,7 +338,7 @@ class _SimpleGlaFn(torch.autograd.Function):
         o = torch.empty_like(v)
         n_seq = max(cu_seqlens.numel() - 1, 0)
         lib = _lib.lib()
-        states = torch.empty((lib.mcb_simple_gla_edges(T), h, 2, dk, dv), dtype=q.dtype, device=q.device)
+        states = torch.empty((lib.mcb_simple_gla_edges(T, n_seq), h, 2, dk, dv), dtype=q.dtype, device=q.device)
         rc = lib.mcb_simple_gla_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(decay), _lib.ptr(cu_seqlens),
                                     _lib.ptr(o), _lib.ptr(states), ctypes.c_int(T), ctypes.c_int(n_seq),
                                     ctypes.c_int(h), ctypes.c_int(dk), ctypes.c_float(scale),
@@ -360,7 +360,7 @@ class _SimpleGlaFn(torch.autograd.Function):
         lib = _lib.lib()
         # the forward's states are formed again: keeping them would add half of the layer's q / k / v / o
         n_seq = max(cu.numel() - 1, 0)
-        states = torch.empty((2, lib.mcb_simple_gla_edges(T), h, 2, dk, dk), dtype=q.dtype, device=q.device)
+        states = torch.empty((2, lib.mcb_simple_gla_edges(T, n_seq), h, 2, dk, dk), dtype=q.dtype, device=q.device)
         rc = lib.mcb_simple_gla_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(do), _lib.ptr(decay), _lib.ptr(cu),
                                     _lib.ptr(dq), _lib.ptr(dk_), _lib.ptr(dv), _lib.ptr(states), ctypes.c_int(T),
                                     ctypes.c_int(n_seq), ctypes.c_int(h), ctypes.c_int(dk), ctypes.c_float(ctx.scale),
@@ -537,7 +537,8 @@ def chunk_gated_delta_rule(q, k, v, g, beta, cu_seqlens=None, scale: Optional[fl
 
 
 def simple_gla(q, k, v, decay, cu_seqlens=None, scale: Optional[float] = None) -> torch.Tensor:
-    """Dispatches to the CUDA kernels (bf16, square 64 / 128 state) or the torch restatement."""
+    """Dispatches to the CUDA kernels (bf16, square 64 / 128 state; in tiles, or token by token for short sequences) or
+    the torch restatement."""
     T, h, dk = q.shape
     scale = dk**-0.5 if scale is None else scale
     if _cuda_ok(q, k, v) and dk == v.shape[-1] and dk in (64, 128):

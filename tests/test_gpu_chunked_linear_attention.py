@@ -410,3 +410,29 @@ def test_simple_gla_tiles_shared_by_sequences(T, d, cuts):
     for a, b in zip(run(*hit), clean):
         assert torch.equal(a[others], b[others])
         assert not a[first:last].isfinite().all()
+
+
+@pytest.mark.parametrize('T,d,lengths', [(64, 64, [13]), (2048, 128, [12]), (2047, 64, [8, 3, 17]), (1000, 128, [15])])
+def test_simple_gla_short_sequences_in_full_fp32_precision(T, d, lengths):
+    """fp32 sums of d products are off by about 2^-25 sqrt(d) < 2^-21 of themselves, bf16 results 2^-8 .. 2^-7 apart: they are the
+    exact ones' nearest but for 2^-12 of them.  Operands of 16 bits would move eight times as many."""
+    from mcore_bridge_b200.ops.gdn import simple_gla
+    ends, n, h = [0], 0, 32
+    while ends[-1] < T:
+        ends.append(min(T, ends[-1] + lengths[n % len(lengths)]))
+        n += 1
+    (q, k, v, dy), _ = _inputs(T, h, d, 31)
+    decay = -(2.0 ** (-8.0 * torch.arange(1, h + 1, device=DEV) / h))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    o = simple_gla(*leaves, decay, torch.tensor(ends, dtype=torch.int32, device=DEV))
+    grads = torch.autograd.grad(o, leaves, dy)
+    wide = [t.detach().double().requires_grad_() for t in leaves]
+    out = []
+    for s, e in zip(ends[:-1], ends[1:]):
+        n = torch.arange(e - s, device=DEV, dtype=torch.float64)
+        gap = n[:, None] - n[None]
+        mix = torch.exp(decay.double()[:, None, None] * gap.clamp(min=0)) * (gap >= 0) * d ** -0.5
+        out.append(torch.einsum('hij,jhd->ihd', torch.einsum('ihd,jhd->hij', wide[0][s:e], wide[1][s:e]) * mix, wide[2][s:e]))
+    ref = torch.cat(out)
+    for a, b in zip([o, *grads], [ref, *torch.autograd.grad(ref, wide, dy.double())]):
+        assert (a != b.bfloat16()).double().mean() < 2 ** -11
