@@ -63,6 +63,9 @@ __device__ __forceinline__ uint32_t box_addr(uint32_t box, int row, int chunk) {
 __device__ __forceinline__ void sts16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+__device__ __forceinline__ void lds16(uint32_t addr, uint32_t (&x)[4]) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(addr) : "memory");
+}
 // one whole 32-byte sector
 __device__ __forceinline__ void stg32(void* p, const uint32_t (&v)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
@@ -256,8 +259,7 @@ gla_walk_kernel(const __grid_constant__ WalkMaps maps, const GlaParams p, const 
           const int c = 2 * half + u;
           uint32_t x[4], hi[4], lo[4];
           // what TMA wrote: 64-byte rows, their 16-byte chunks swizzled by pairs of rows
-          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
-                       : "r"(tiles + L::OFF_V + ks * L::V + j * 64 + ((c ^ ((j >> 1) & 3)) << 4)) : "memory");
+          lds16(tiles + L::OFF_V + ks * L::V + j * 64 + ((c ^ ((j >> 1) & 3)) << 4), x);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[e]));
@@ -340,7 +342,7 @@ gla_walk_kernel(const __grid_constant__ WalkMaps maps, const GlaParams p, const 
 //
 //   X Y^T -> scores | X M_hi -> out (loads M_lo over Y, Z over M_hi) | out += X M_lo (loads the next X, Y) | out += P Z
 //
-// Warp 9 finds the next tile's sequences.  Warps 0..7 (thread = row and half of its columns) weight the scores meanwhile, multiply
+// Warp 9 finds the next tile's sequences and looks for what is not finite in Z.  Warps 0..7 (thread = row and half of its columns) weight the scores meanwhile, multiply
 // the state's share by w_i before the last product, and write the result out while the next one's first products run.
 //
 // Bound: the waits of that chain, half of them for the state's terms, of which two CTAs overlap: about 12000 cycles a result of
@@ -409,6 +411,48 @@ __device__ __forceinline__ ResultItem find_item(const GlaParams& p, int id, int 
   return it;
 }
 
+// All rows meet all of Z in the last product, most of them with weights of zero: what is not finite there is taken out of Z, and
+// noted, so that it stays with the rows that see it.  By warp 9, which has time: us, gradients, only where several sequences share
+// the tile / by the warps of the rows / by warp 9, 16384 in one, 32 heads of 128 287 / 317 / 304, 4096 in two, 16 heads 45.6 / 47.7 /
+// 46.3, 8192 in sequences of 16 88 / 67 / 69.
+template <int D>
+__device__ __forceinline__ bool all_finite(uint32_t z, int lane) {
+  // x * 0 is zero for what is finite, and NaN is what stays in a sum
+  __nv_bfloat162 sum[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) sum[e] = __float2bfloat162_rn(0.f);
+  for (int b = 0; b < D / 64; ++b)
+#pragma unroll 4
+    for (int c = 0; c < C / 4; ++c) {           // a quarter of a warp to a row
+      uint32_t x[4];
+      lds16(box_addr(z + b * C * 128, 4 * c + (lane >> 3), lane & 7), x);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sum[e] = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&x[e]), __float2bfloat162_rn(0.f), sum[e]);
+    }
+  const __nv_bfloat162 s = __hadd2(__hadd2(sum[0], sum[1]), __hadd2(sum[2], sum[3]));
+  return !__any_sync(0xffffffffu, __hisnan(__low2bfloat16(s)) || __hisnan(__high2bfloat16(s)));
+}
+// bad[column][q]: bit r, row 32 q + r is not finite there
+template <int D>
+__device__ __forceinline__ void take_out(uint32_t z, uint32_t* bad, int lane) {
+#pragma unroll 1
+  for (int i = 0; i < 4 * (D / 8); ++i) {
+    const int q = i & 3, c = i >> 2;
+    const uint32_t at = box_addr(z + (c >> 3) * (C * 128), 32 * q + lane, c & 7);
+    uint32_t x[4];
+    lds16(at, x);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const uint32_t m = 0x7f80u << (16 * (e & 1));
+      const bool out = (x[e >> 1] & m) == m;
+      const uint32_t rows = __ballot_sync(0xffffffffu, out);
+      if (lane == 0) bad[(c * 8 + e) * 4 + q] = rows;
+      if (out) x[e >> 1] &= ~(0xffffu << (16 * (e & 1)));
+    }
+    sts16(at, x[0], x[1], x[2], x[3]);
+  }
+}
+
 template <int D, bool GRAD>
 __global__ void __launch_bounds__(RES_THREADS, 2)
 gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const int items) {
@@ -432,7 +476,7 @@ gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const
     *abort_flag = 0;
     *bad_item = -1;
     for (int i = 0; i < 8; ++i) mbar_init(xy_full + 8 * i, 1);
-    mbar_init(p_full, 8);
+    mbar_init(p_full, 9);
     mbar_init(o_read, 8);
     for (int i = 0; i < 2; ++i) {
       mbar_init(item_full + 8 * i, 1);
@@ -446,7 +490,6 @@ gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const
     tmem_relinquish();
   }
   uint32_t* bad = reinterpret_cast<uint32_t*>(smem + L::OFF_BAD);
-  for (int i = threadIdx.x; i < D * 4; i += RES_THREADS) bad[i] = 0;
   if (!GRAD) check_bounds(p.cu, p.n_seq, p.T, p.status);
   tc_fence_before();
   __syncthreads();
@@ -569,16 +612,30 @@ gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const
     if (open & 8u) drain(z_full, n & 1);
     __syncwarp();
   } else if (warp == 9) {
-    int id = blockIdx.x;
-    for (int n = 0;; ++n, id += gridDim.x) {
-      const ResultItem it = id < items ? find_item(p, id, ROLES, lane) : ResultItem{};
-      if (!mbar_wait_warp(item_read + 8 * (n & 1), ((n >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+    auto publish = [&](int n, const ResultItem& it) {
+      if (!mbar_wait_warp(item_read + 8 * (n & 1), ((n >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) return false;
       if (lane == 0) {
         slots[n & 1] = it;
         mbar_arrive(item_full + 8 * (n & 1));
       }
       __syncwarp();
-      if (it.len == 0) break;
+      return true;
+    };
+    int id = blockIdx.x;
+    ResultItem it = find_item(p, id, ROLES, lane);
+    bool ok = publish(0, it);
+    for (int n = 0; ok && it.len; ++n) {
+      id += gridDim.x;
+      it = id < items ? find_item(p, id, ROLES, lane) : ResultItem{};
+      ok = publish(n + 1, it) && mbar_wait_warp(z_full, n & 1, abort_flag, p.status, ST_TIMEOUT_FULL);
+      if (!ok) break;
+      if (!all_finite<D>(sz, lane)) {
+        take_out<D>(sz, bad, lane);
+        *bad_item = n;
+        fence_proxy_async_smem();
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
     }
   } else {
     const int q = warp & 3, half = warp >> 2, row = q * 32 + lane;
@@ -588,7 +645,6 @@ gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const
     auto wait = [&](uint32_t bar, uint32_t ph, int code) {
       return mbar_wait_warp(bar, ph, abort_flag, p.status, code);
     };
-    bool noted = false;                         // this warp's words of `bad` are not zero
     for (int n = 0;; ++n) {
       const uint32_t ph = n & 1;
       if (!wait(item_full + 8 * (n & 1), (n >> 1) & 1, ST_TIMEOUT_FULL)) break;
@@ -657,43 +713,10 @@ gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const
       }
       tmem_st_wait();
       tc_fence_before();
-      // Rows of several sequences meet in the last product, with weights of zero: what is not finite there is taken out of
-      // Z, and noted, so that it stays in its own sequence.
-      const bool several = (it.starts[0] & ~1u) | it.starts[1] | it.starts[2] | it.starts[3];
-      if (several) {
-        if (!wait(z_full, ph, ST_TIMEOUT_FULL)) break;
-        if (noted) {
-          for (int c = lane; c < D / 2; c += 32) bad[(half * (D / 2) + c) * 4 + q] = 0;
-          __syncwarp();
-          noted = false;
-        }
-        bool any = false;
-#pragma unroll 1
-        for (int c = half * (D / 16); c < (half + 1) * (D / 16); ++c) {
-          const uint32_t at = box_addr(sz + (c >> 3) * (C * 128), row, c & 7);
-          uint32_t x[4];
-          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(at) : "memory");
-          bool here = false;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const uint32_t m = 0x7f80u << (16 * (e & 1));
-            if ((x[e >> 1] & m) == m) {
-              atomicOr(&bad[(c * 8 + e) * 4 + q], 1u << lane);
-              x[e >> 1] &= ~(0xffffu << (16 * (e & 1)));
-              here = true;
-            }
-          }
-          if (here) sts16(at, x[0], x[1], x[2], x[3]);
-          any |= here;
-        }
-        if (any) *bad_item = n;
-        fence_proxy_async_smem();
-      }
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
-      // (p_full: all of the CTA's rows have been looked at)
-      const bool found = several && wait(p_full, ph, ST_TIMEOUT_FULL) && *bad_item == n;
-      if (!wait(o_done, ph, ST_TIMEOUT_TMEM_FULL)) break;
+      if (!wait(o_done, ph, ST_TIMEOUT_TMEM_FULL) || !wait(p_full, ph, ST_TIMEOUT_FULL)) break;
+      const bool found = *bad_item == n;        // (p_full: warp 9 has looked)
       tc_fence_after();
       __nv_bfloat16* out = !GRAD ? p.o : it.role == DQ ? p.dq : it.role == DK ? p.dk : p.dv;
       __nv_bfloat16* dst = out + ((long long)(it.t + row) * p.H + it.h) * D + half * (D / 2);
@@ -717,7 +740,6 @@ gla_result_kernel(const __grid_constant__ GlaMaps maps, const GlaParams p, const
           }
           if (seen) r[c] = 0x7fffffffu;
         }
-        noted = true;
       }
       tc_fence_before();
       __syncwarp();

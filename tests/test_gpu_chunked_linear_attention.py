@@ -436,3 +436,42 @@ def test_simple_gla_short_sequences_in_full_fp32_precision(T, d, lengths):
     ref = torch.cat(out)
     for a, b in zip([o, *grads], [ref, *torch.autograd.grad(ref, wide, dy.double())]):
         assert (a != b.bfloat16()).double().mean() < 2 ** -11
+
+
+@pytest.mark.parametrize('T,d,cuts,at', [(40, 64, [], 17), (128, 128, [], 100), (300, 64, [], 130), (400, 128, [128], 250),
+                                         (64, 128, list(range(8, 64, 8)), 21), (300, 64, [20], 290)])
+def test_simple_gla_what_is_not_finite_stays_with_the_tokens_that_see_it(T, d, cuts, at):
+    """One infinite channel of one token: the other results of its sequence have the bits they have without it."""
+    from mcore_bridge_b200.ops.gdn import simple_gla
+    tensors, _ = _inputs(T, 2, d, 23)
+    decay = -torch.tensor([0.02, 0.001], device=DEV)
+    cu = torch.tensor([0] + cuts + [T], dtype=torch.int32, device=DEV)
+
+    def run(tensors):
+        leaves = [t.detach().requires_grad_() for t in tensors[:3]]
+        o = simple_gla(*leaves, decay, cu)
+        return [o.detach(), *torch.autograd.grad(o, leaves, tensors[3])]
+
+    clean = run(tensors)
+    first, last = next(s for s in _spans(T, cuts) if s[0] <= at < s[1])
+    t, c = torch.arange(T, device=DEV), 3
+    own, later, earlier = t == at, (t >= at) & (t < last), (t <= at) & (t >= first)
+    channel = torch.zeros(d, dtype=torch.bool, device=DEV)
+    channel[c] = True
+    none, row = torch.zeros(T, d, dtype=torch.bool, device=DEV), torch.ones(d, dtype=torch.bool, device=DEV)
+
+    def where(rows, columns):
+        return rows[:, None] & columns[None]
+
+    # of q, k, v and dy: the parts of o, dq, dk and dv it enters
+    reach = [(where(own, row), none, where(earlier, channel), where(earlier, row)),
+             (where(later, row), where(later, channel), none, where(own, row)),
+             (where(later, channel), where(later, row), where(own, row), none),
+             (none, where(own, row), where(earlier, row), where(earlier, channel))]
+    for i, value in enumerate((float('inf'), float('nan'), -float('inf'), float('inf'))):
+        hit = [x.clone() for x in tensors]
+        hit[i][at, :, c] = value
+        for a, b, r in zip(run(hit), clean, reach[i]):
+            r = r[:, None].expand(a.shape)
+            assert torch.equal(a[~r], b[~r])
+            assert not a[r].isfinite().any()
