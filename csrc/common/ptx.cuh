@@ -99,6 +99,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// The loads that signal `bar` have landed (or 0.2 s have passed): nothing may write into a CTA that is gone
+__device__ __forceinline__ void drain(uint32_t bar, uint32_t parity) {
+  const uint64_t t0 = globaltimer_ns();
+  while (!mbar_try_wait(bar, parity))
+    if (globaltimer_ns() - t0 > 200000000ull) break;
+}
+
 // ---------------------------------------------------------------- issuing with a whole warp
 // A tcgen05 instruction takes its descriptors and addresses from uniform registers.  Inside `if (lane == 0)` they are
 // computed per thread and moved over one by one, about 85 cycles for each MMA where the tensor core needs 64 for

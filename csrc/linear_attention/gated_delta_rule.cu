@@ -449,6 +449,8 @@ struct ScanRing {
   uint32_t full, empty;                         // mbarriers of the first stage; + 8 of the second; + 16 (full) of M and P
   volatile int* abort_flag;
   int* status;
+  int loads = 0;                                // of chunks, by this warp
+  bool ok = true;                               // of this warp's waits so far
   __device__ __forceinline__ void init(uint32_t bars, volatile int* flag, int* st) {
     full = bars;
     empty = bars + 32;
@@ -465,15 +467,27 @@ struct ScanRing {
     }
     __syncthreads();
   }
-  // a wait that gives up reports it and the walk goes on, with what is there, to its end: the barriers of a strip stay whole
-  __device__ __forceinline__ void wait_full(int i) {
-    mbar_wait_warp(full + 8 * (i & 1), (i >> 1) & 1, abort_flag, status, ST_TIMEOUT_FULL);
+  // A wait that gives up reports it and the walk goes on to its end, with what is there, so that the barriers of a strip stay whole;
+  // the warp waits for nothing and loads nothing any more.
+  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, int code) {
+    if (ok) ok = mbar_wait_warp(bar, parity, abort_flag, status, code);
   }
-  __device__ __forceinline__ void wait_squares(int i) {
-    mbar_wait_warp(full + 16 + 8 * (i & 1), (i >> 1) & 1, abort_flag, status, ST_TIMEOUT_FULL);
+  __device__ __forceinline__ void wait_full(int i) { wait(full + 8 * (i & 1), (i >> 1) & 1, ST_TIMEOUT_FULL); }
+  __device__ __forceinline__ void wait_squares(int i) { wait(full + 16 + 8 * (i & 1), (i >> 1) & 1, ST_TIMEOUT_FULL); }
+  __device__ __forceinline__ bool wait_empty(int i) {          // until stage i & 1 is free for the i-th chunk
+    if (i >= 2) wait(empty + 8 * (i & 1), ((i >> 1) & 1) ^ 1, ST_TIMEOUT_EMPTY);
+    loads += ok;
+    return ok;
   }
-  __device__ __forceinline__ void wait_empty(int i) {          // until stage i & 1 is free for the i-th chunk
-    if (i >= 2) mbar_wait_warp(empty + 8 * (i & 1), ((i >> 1) & 1) ^ 1, abort_flag, status, ST_TIMEOUT_EMPTY);
+  // At the end of the walk.  A warp that has seen everything land has nothing to wait for; nothing lands in a CTA that is gone.
+  __device__ __forceinline__ void finish() {
+    if (ok) return;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (threadIdx.x >= 32) return;              // the first warp issues the bulk copies
+    for (int i = max(loads - 2, 0); i < loads; ++i) {
+      drain(full + 8 * (i & 1), (i >> 1) & 1);
+      drain(full + 16 + 8 * (i & 1), (i >> 1) & 1);
+    }
   }
   __device__ __forceinline__ void done(int i, int lane) {
     __syncwarp();
@@ -578,8 +592,7 @@ gdr_scan_kernel(const GdrParams p) {
   ring.init(base + L::BARS, &flag, p.status);
   const StageLoad<D, NT, SAVE> copy(p);
   auto load = [&](int c) {
-    if (c >= s.n) return;
-    ring.wait_empty(c);
+    if (c >= s.n || !ring.wait_empty(c)) return;
     copy(base + (c & 1) * L::STAGE, ring.full + 8 * (c & 1), p, s.t0 + c * C, min(C, s.len - c * C), s.h, s.col0,
                             (long long)(s.chunk0 + c) * p.H + s.h);
   };
@@ -739,7 +752,7 @@ gdr_scan_kernel(const GdrParams p) {
       share_state<NT>(part0, quarter, St);
     }
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");   // nothing to wait for, unless a wait gave up
+  ring.finish();
 }
 
 template <int D>
@@ -764,8 +777,7 @@ gdr_scan_bwd_kernel(const GdrParams p) {
   const StageLoad<D, NT, true> copy(p);
   auto load = [&](int it) {
     const int c = lastc - it;
-    if (c < 0) return;
-    ring.wait_empty(it);
+    if (c < 0 || !ring.wait_empty(it)) return;
     copy(base + (it & 1) * L::STAGE, ring.full + 8 * (it & 1), p, s.t0 + c * C, min(C, s.len - c * C), s.h, s.col0,
                             (long long)(s.chunk0 + c) * p.H + s.h);
   };
@@ -931,7 +943,7 @@ gdr_scan_bwd_kernel(const GdrParams p) {
       share_state<NT>(part0, quarter, dSt);
     }
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");   // nothing to wait for, unless a wait gave up
+  ring.finish();
 }
 
 // ---------------------------------------------------------------------------------------------------- grad
@@ -1146,7 +1158,7 @@ gdr_grad_kernel(const GdrParams p) {
   if (threadIdx.x == 0) flag = 0;
   cp_async_wait<0>();
   __syncthreads();                             // (the mbarrier too)
-  mbar_wait_warp(smem_u32(&vb_full), 0, &flag, p.status, ST_TIMEOUT_FULL);   // gives up only with the device in trouble
+  const bool landed = mbar_wait_warp(smem_u32(&vb_full), 0, &flag, p.status, ST_TIMEOUT_FULL);   // if not, it is reported
   {
     // ten blocks of dA (48 MMAs) and ten of dP (32): one of dA, or one or two of dP to a warp
     auto row_of = [](int b) { return b >= 6 ? 3 : b >= 3 ? 2 : b >= 1 ? 1 : 0; };
@@ -1285,6 +1297,7 @@ gdr_grad_kernel(const GdrParams p) {
     const long long at = (long long)(t + 2 * lane) * p.H + h;
     if (2 * lane < len) p.dg[at] = (float)run;
     if (2 * lane + 1 < len) p.dg[at + p.H] = (float)(run - x[0]);
+    if (!landed) drain(smem_u32(&vb_full), 0);
   }
 }
 
@@ -1357,7 +1370,7 @@ int mcb_gdr_fwd(const void* q, const void* k, const void* v, const float* g, con
 int mcb_gdr_bwd(const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu_seqlens,
                 const void* dout, void* dq, void* dk, void* dv, float* dg, float* dbeta, void* mp, float* gb,
                 float* states, void* values, float* predictions, float* dots, int T, int n_seq, int H, int D, float scale,
-                void* stream_) {
+                int* status, void* stream_) {
   if (n_seq <= 0 || T <= 0) return 0;
   GdrParams p = common(q, k, v, g, beta, cu_seqlens, mp, gb, T, n_seq, H, scale);
   const long long n = (long long)mcb_gdr_chunks(T, n_seq) * H;
@@ -1367,6 +1380,7 @@ int mcb_gdr_bwd(const void* q, const void* k, const void* v, const float* g, con
   p.V = (__nv_bfloat16*)values; p.B = p.V + n * 2 * D * C;
   p.E = predictions;
   p.oo = dots; p.nn = p.oo + n * (D / 16) * C; p.yy = p.nn + n * (D / 16) * C;
+  p.status = status;
   return run_gdr(p, T, D, true, reinterpret_cast<cudaStream_t>(stream_));
 }
 

@@ -87,12 +87,6 @@ __device__ __forceinline__ void load_boxes(uint32_t leader, uint32_t tile, const
 #pragma unroll
   for (int b = 0; b < D / 64; ++b) tma_load_2d_warp(leader, tile + b * ROWS * 128, map, x + b * 64, y, bar);
 }
-// the loads that signal `bar` have landed (or 0.2 s have passed): nothing may write into a CTA that is gone
-__device__ __forceinline__ void drain(uint32_t bar, uint32_t parity) {
-  const uint64_t t0 = globaltimer_ns();
-  while (!mbar_try_wait(bar, parity))
-    if (globaltimer_ns() - t0 > 200000000ull) break;
-}
 
 // ---------------------------------------------------------------------------------------------------- states
 // States at the edges between tiles: S behind the tokens before an edge, R of those behind it, of the sequence that crosses it,

@@ -418,7 +418,7 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
                              _lib.ptr(do), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(dg), _lib.ptr(dbeta),
                              _lib.ptr(mp), _lib.ptr(gb), _lib.ptr(states), _lib.ptr(values), _lib.ptr(preds),
                              _lib.ptr(dots), ctypes.c_int(T), ctypes.c_int(n_seq), ctypes.c_int(h), ctypes.c_int(d),
-                             ctypes.c_float(ctx.scale), _lib.stream_ptr())
+                             ctypes.c_float(ctx.scale), _lib.ptr(_lib.status_word(q.device)), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_gdr_bwd')
         return dq, dk, dv, dg, dbeta, None, None, None
 

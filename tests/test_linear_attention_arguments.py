@@ -81,3 +81,18 @@ def test_kernels_only_see_aligned_tensors(monkeypatch, op):
     assert len(calls) == 2
     for pointers in calls.values():
         assert all(p % 16 == 0 for p in pointers)
+
+
+@pytest.mark.parametrize('op', ['gla', 'rule'])
+def test_kernels_that_wait_know_where_to_report(monkeypatch, op):
+    """A wait that gives up is reported through the device's status word, in both directions."""
+    rec, status = _Recorder(), torch.zeros(16, dtype=torch.int32)
+    monkeypatch.setattr(gdn, '_cuda_ok', lambda *ts: True)
+    monkeypatch.setattr(_lib, 'lib', lambda: rec)
+    monkeypatch.setattr(_lib, 'stream_ptr', lambda: ctypes.c_void_p(0))
+    monkeypatch.setattr(_lib, 'status_word', lambda device=None: status)
+    q, k, v, g, beta = (t.requires_grad_() for t in _tensors())
+    o = gdn.simple_gla(q, k, v, -torch.rand(H)) if op == 'gla' else gdn.chunk_gated_delta_rule(q, k, v, g, beta)
+    torch.autograd.grad(o, (q, k, v), torch.ones_like(o))
+    calls = {n: p for n, p in rec.pointers.items() if n.endswith(('_fwd', '_bwd'))}
+    assert len(calls) == 2 and all(status.data_ptr() in p for p in calls.values())
