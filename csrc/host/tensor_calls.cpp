@@ -273,8 +273,10 @@ Qkv qkv_split(const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tenso
   return r;
 }
 
-void qkv_join(Qkv dr, const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin, const QkvArgs& g,
+void qkv_join(Qkv dr, const Tensor& qkv_, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin, const QkvArgs& g,
               Tensor& dqkv, Tensor& dwq, Tensor& dwk) {
+  // the kernels write the gradient with the strides they read qkv by: columns of a wider tensor are copied first
+  const Tensor qkv = qkv_.contiguous();
   const ll T = qkv.size(0), d = g.d;
   const bool norm = wq.defined();
   check_qkv(qkv, wq, wk, cos, sin, g);

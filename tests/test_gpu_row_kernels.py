@@ -147,3 +147,20 @@ def test_combined_rows(T, k, H):
         want += torch.where(sent[:, j, None] >= 0, y[sent[:, j].clamp(min=0).long()].float(), 0.0)
     assert torch.equal(out, want.bfloat16())
     assert torch.equal(probs, torch.where(sent >= 0, scalars[sent.clamp(min=0).long()], 0.0))
+
+
+@pytest.mark.parametrize('T,ng,qpg,d,gate', [(1, 2, 2, 128, False), (333, 2, 4, 128, True), (70, 3, 2, 64, False)])
+def test_heads_in_columns_of_a_wider_tensor(T, ng, qpg, d, gate):
+    """The gradient of such columns is dense: the bits of a contiguous copy's, and of nothing beside it."""
+    from mcore_bridge_b200.ops.rope import qkv_split_norm_rope
+    W = ng * (qpg * (2 if gate else 1) + 2) * d
+    wide, ws = _rand(T, W + 40), [_rand(d, seed=s) for s in (1, 2)]
+    cos, sin = torch.rand(T, d // 2, device=DEV), torch.rand(T, d // 2, device=DEV)
+
+    def run(qkv):
+        leaves = [qkv.detach().requires_grad_(), *(w.clone().requires_grad_() for w in ws)]
+        outs = [t for t in qkv_split_norm_rope(*leaves, cos, sin, ng, qpg, d, gate, False, 1e-6, False) if t is not None]
+        return outs + list(torch.autograd.grad(outs, leaves, [_rand(*t.shape, seed=5) for t in outs]))
+
+    for a, b in zip(run(wide[:, :W]), run(wide[:, :W].clone())):
+        assert a.shape == b.shape and torch.equal(a, b)
