@@ -120,7 +120,8 @@ std::vector<int64_t> with_last(const Tensor& x, ll n) {
   return shape;
 }
 Tensor like_input(const Tensor& dx, const std::vector<int64_t>& shape) { return dx.dim() == 2 && shape.size() == 2 ? dx : dx.view(shape); }
-// x2 . weight^T (+ bias) (+ residual) in x's leading shape; a residual has that shape too
+// x2 . weight^T (+ bias) (+ residual) in x's leading shape; a residual has that shape too.  One of another type is added as torch
+// adds it, in the wider of the two.
 Tensor product(const Tensor& x2, const Tensor& weight, const Tensor& bias, const Tensor& x, const Tensor& residual = {}) {
   const Tensor y = at::empty(with_last(x, weight.size(0)), x.options());
   if (!residual.defined()) {
@@ -141,12 +142,12 @@ struct LinearNode : OpNode {
   std::string name() const override { return "McbLinearBackward"; }
   variable_list grads(variable_list& g) override {
     const Tensor x2 = get(0), w = get(1);
-    const Tensor dy2 = rows_of(g[0], w.size(0));
+    const Tensor dy2 = rows_of(g[0].to(w.scalar_type()), w.size(0));   // a residual may have made the result wider
     variable_list r(4);
     if (residual) r[3] = g[0];
     if (need_dx) r[0] = gemm(NN, dy2, w).view(shape);
     if (need_dw) r[1] = weight_grad(w, dy2, x2);
-    if (bias) r[2] = dy2.to(at::kFloat).sum(0).to(g[0].scalar_type());
+    if (bias) r[2] = dy2.to(at::kFloat).sum(0).to(dy2.scalar_type());
     return r;
   }
 };
@@ -277,7 +278,7 @@ struct GluLinearNode : OpNode {
   std::string name() const override { return "McbGluLinearBackward"; }
   variable_list grads(variable_list& g) override {
     const Tensor h2 = get(0), w = get(1);
-    const Tensor dy2 = rows_of(g[0], w.size(0)), da = gemm(NN, dy2, w);
+    const Tensor dy2 = rows_of(g[0].to(w.scalar_type()), w.size(0)), da = gemm(NN, dy2, w);
     Tensor none;
     const Tensor dh = glu_rows_bwd(da, h2, {}, args, need_dw, none);  // da becomes the activation
     return {like_input(dh, shape), need_dw ? weight_grad(w, dy2, da) : Tensor(), residual ? g[0] : Tensor()};

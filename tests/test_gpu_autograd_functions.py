@@ -174,3 +174,38 @@ def test_residual_of_a_wide_row():
     got = torch.autograd.grad(fused_mlp.norm_linear(*leaves, 1e-6, False, True), leaves, [dy, dk])
     want = torch.autograd.grad(fused_mlp.norm_linear(*leaves, 1e-6, False), leaves, dy)
     assert torch.equal(got[0], want[0] + dk) and torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+
+
+@pytest.mark.parametrize('name', ['linear', 'glu_linear'])
+@pytest.mark.parametrize('shape', [(70,), (2, 35)])
+def test_a_residual_of_another_type(name, shape):
+    """An fp32 residual under bf16 operands: fp32 results, and gradients as of an addition."""
+    from mcore_bridge_b200.ops import _lib, fused_mlp
+    x, w, res = _rand(*shape, 128), _rand(96, 128 if name == 'linear' else 64, seed=2), _rand(*shape, 96, seed=3).float()
+    nat = _lib.native()
+
+    def op(x, w, r):
+        return nat.linear(x, w, None, False, r) if name == 'linear' else fused_mlp.glu_linear(x, w, 0, 0.0, 0.0, r)
+
+    leaves = [t.requires_grad_() for t in (x, w, res)]
+    a, b = op(*leaves), res + op(x, w, None)
+    assert a.dtype == torch.float32 and torch.equal(a, b)
+    dy = torch.randn_like(a)
+    for g, e in zip(torch.autograd.grad(a, leaves, dy), torch.autograd.grad(b, leaves, dy)):
+        assert g.dtype == e.dtype and torch.equal(g, e)
+
+
+def test_a_feed_forward_block_under_an_fp32_residual_stream():
+    from mcore_bridge_b200.layers.mlp import MLP
+    from mcore_bridge_b200.train.presets import model_config
+    with torch.device(DEV):
+        mlp = MLP(model_config('qwen3_tiny', bf16=True), fuse_input_norm=True)
+    for i, p in enumerate(mlp.parameters()):
+        with torch.no_grad():
+            p.copy_(_rand(*p.shape, seed=i, scale=0.02))
+    x = _rand(50, mlp.config.hidden_size).float().requires_grad_()
+    leaves, dy = [x, *mlp.parameters()], torch.randn(50, mlp.config.hidden_size, device=DEV)
+    a, b = mlp(x, True), x + mlp(x)
+    assert a.dtype == torch.float32 and torch.equal(a, b)
+    for g, e in zip(torch.autograd.grad(a, leaves, dy), torch.autograd.grad(b, leaves, dy)):
+        assert g.dtype == e.dtype and torch.equal(g, e)
