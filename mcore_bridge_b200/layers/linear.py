@@ -29,7 +29,13 @@ def _set_tp_attrs(p: nn.Parameter, is_parallel: bool, dim: int, is_expert: bool 
 def is_plain(module: nn.Module, cls) -> bool:
     """A module whose call is its class's ``forward`` and nothing else: what a caller may fuse into another operation."""
     return (type(module) is cls and 'forward' not in module.__dict__
-            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks))
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+            and not any(_GLOBAL_HOOKS))
+
+
+# hooks on every module of the process: the dictionaries that torch's registration functions fill
+_GLOBAL_HOOKS = tuple(getattr(nn.modules.module, f'_global_{kind}_hooks')
+                      for kind in ('forward', 'forward_pre', 'backward', 'backward_pre'))
 
 
 class _LinearBase(nn.Module):

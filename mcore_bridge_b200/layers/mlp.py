@@ -5,7 +5,7 @@ import torch
 from torch import nn
 
 from ..ops.activation import glu
-from .linear import ColumnParallelLinear, LayerNormColumnParallelLinear, RowParallelLinear
+from .linear import ColumnParallelLinear, LayerNormColumnParallelLinear, RowParallelLinear, is_plain
 
 
 class MLP(nn.Module):
@@ -34,8 +34,8 @@ class MLP(nn.Module):
         else:
             h = fc1(x)
         # the fused block does not call fc2 as a module: with hooks on it, which want its input or output, it is called
-        if cfg.gated_linear_unit and type(fc2) is RowParallelLinear and fc2.bias is None and not fc2.spec.fp8 \
-                and getattr(cfg, 'lean_activations', True) and not (fc2._forward_hooks or fc2._forward_pre_hooks):
+        if cfg.gated_linear_unit and is_plain(fc2, RowParallelLinear) and fc2.bias is None and not fc2.spec.fp8 \
+                and getattr(cfg, 'lean_activations', True):
             from ..parallel import state as ps
             from ..ops import fused_mlp
             if ps.get_world_size(fc2.group) == 1 and fused_mlp.usable(h, fc2.weight) and (h.shape[-1] // 2) % 8 == 0:
