@@ -18,7 +18,7 @@ from ..ops.rope import qkv_split_norm_rope
 from ..parallel import state as ps
 from ..utils.profiling import nvtx_range
 from .context import ForwardContext, layer_cp_comm_type
-from .linear import ColumnParallelLinear, LayerNormColumnParallelLinear, RowParallelLinear
+from .linear import ColumnParallelLinear, LayerNormColumnParallelLinear, RowParallelLinear, fusable
 from .norm import Norm
 
 
@@ -73,6 +73,7 @@ class _ShardedChannelNorm(nn.Module):
         return y.to(x.dtype)
 
 
+@fusable
 class SelfAttention(nn.Module):
 
     def __init__(self, config, layer_number: int, fuse_input_norm: bool = True, use_rope: bool = True,

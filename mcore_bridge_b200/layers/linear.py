@@ -26,9 +26,19 @@ def _set_tp_attrs(p: nn.Parameter, is_parallel: bool, dim: int, is_expert: bool 
     p.is_expert = is_expert
 
 
+_FORWARDS = {}
+
+
+def fusable(cls):
+    """Class decorator: a module of this class may be fused into its caller's operation, see :func:`is_plain`."""
+    _FORWARDS[cls] = cls.forward
+    return cls
+
+
 def is_plain(module: nn.Module, cls) -> bool:
-    """A module whose call is its class's ``forward`` and nothing else: what a caller may fuse into another operation."""
-    return (type(module) is cls and 'forward' not in module.__dict__
+    """A module whose call is the ``forward`` that ``cls`` was written with and nothing else: what a caller may fuse into another
+    operation."""
+    return (type(module) is cls and cls.forward is _FORWARDS[cls] and 'forward' not in module.__dict__
             and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
             and not any(_GLOBAL_HOOKS))
 
@@ -87,6 +97,7 @@ class ColumnParallelLinear(_LinearBase):
                 f'bias={self.bias is not None}, sp={self.sequence_parallel}')
 
 
+@fusable
 class LayerNormColumnParallelLinear(ColumnParallelLinear):
     """Norm folded into the following column-parallel linear (``layer_norm_weight``).
 
@@ -149,6 +160,7 @@ class LayerNormColumnParallelLinear(ColumnParallelLinear):
         return y
 
 
+@fusable
 class RowParallelLinear(_LinearBase):
     """``y = x W^T + b`` with ``W [out, in/tp]``; output reduce-scattered (SP) or all-reduced."""
 

@@ -5,9 +5,10 @@ import torch
 from torch import nn
 
 from ..ops.activation import glu
-from .linear import ColumnParallelLinear, LayerNormColumnParallelLinear, RowParallelLinear, is_plain
+from .linear import ColumnParallelLinear, LayerNormColumnParallelLinear, RowParallelLinear, fusable, is_plain
 
 
+@fusable
 class MLP(nn.Module):
 
     def __init__(self, config, ffn_hidden_size: int = None, fuse_input_norm: bool = True):

@@ -62,3 +62,19 @@ def test_global_backward_hooks_see_every_module():
     finally:
         handle.remove()
     assert sorted(n for n in seen if n in SEEN_BY) == sorted(SEEN_BY)
+
+
+@pytest.mark.parametrize('cls,name', [(SelfAttention, 'self_attention'), (MLP, 'mlp'), (RowParallelLinear, 'linear_proj'),
+                                      (LayerNormColumnParallelLinear, 'linear_qkv')])
+def test_a_forward_put_in_the_class_is_called(monkeypatch, cls, name):
+    layer, x, ctx = _layer()
+    want, names, seen, own = layer(x, ctx), _names(layer), [], cls.forward
+
+    def forward(self, x, *ctx):                  # as the class's own before it took a residual
+        assert len(ctx) <= (cls is SelfAttention)
+        seen.append(names[self])
+        return own(self, x, *ctx)
+
+    monkeypatch.setattr(cls, 'forward', forward)
+    assert torch.equal(layer(x, ctx), want)
+    assert name in seen
