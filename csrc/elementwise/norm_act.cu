@@ -188,8 +188,9 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
 
 // `y` (optional, may be `dy`: a thread reads its part of dy first) receives the forward's result, x * rstd * w_eff, which
 // costs a write here and a read, a write and a launch as a forward pass of its own: 8192 x 4096 56 instead of 52 + 34 us.
-// `dres` (RES) is added to the rounded gradient, to the bits of a sum of its own: 8192 x 4096 73 us with y, 56 without it
-// and 36 for a sum of its own.  Rows of more than 8192 have no registers for it and are added to.
+// `dres` (RES) is added to the gradient before it is rounded, or (`apart`) to the rounded one, to the bits of a sum of its own: 8192 x
+// 4096 73 us with y, 56 without it and 36 for a sum of its own.  In rows of more than 8192, which fill the registers, it is
+// loaded where it is added.
 // RING: a CTA that has more than one pair of rows copies the next pair to shared memory (each thread what it will read itself)
 // while it works on one; two CTAs or one on an SM, as registers allow, otherwise leave the memory idle between their loads.
 // us, registers only (VPT 2: one of the two CTAs resident) / now: 8192 x 4096 79 / 52, with y 87 / 56, with dres 88 / 69, with both
@@ -200,7 +201,7 @@ __global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1) rmsnorm_bwd_kernel(cons
                                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                                    float* __restrict__ dw, float* __restrict__ partials, long long rows, int H,
-                                   long long ldx, float eps, int zero_centered) {
+                                   long long ldx, float eps, int zero_centered, int apart) {
   __shared__ float red[66];
   const int nvec = H / 8;
   float dwacc[VPT][8];
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1) rmsnorm_bwd_kernel(cons
     }
   }
   constexpr int NQ = RES ? 3 : 2;
+  constexpr bool AHEAD = RES && VPT <= 4;                      // dres is loaded with dy and x
   extern __shared__ __align__(16) uint8_t ring[];              // [2 stages][NQ][2 rows][nvec] vectors
   uint4* const own = reinterpret_cast<uint4*>(ring) + threadIdx.x;
   auto slot = [&](int stage, int q, int r, int i) { return own + ((stage * NQ + q) * 2 + r) * nvec + i * (int)blockDim.x; };
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1) rmsnorm_bwd_kernel(cons
   int stage = 0;
   for (long long row0 = 2LL * blockIdx.x; row0 < rows; row0 += 2LL * gridDim.x, stage ^= 1) {
     const bool two = row0 + 1 < rows;
-    uint4 xr[2][VPT], gr[2][VPT], dr[2][RES ? VPT : 1];
+    uint4 xr[2][VPT], gr[2][VPT], dr[2][AHEAD ? VPT : 1];
     if constexpr (RING) {
       copy(row0 + 2LL * gridDim.x, stage ^ 1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1) rmsnorm_bwd_kernel(cons
         if ((int)threadIdx.x + i * (int)blockDim.x < nvec) {
           xr[r][i] = RING ? *slot(stage, 0, r, i) : source(0, row)[i * blockDim.x];
           gr[r][i] = RING ? *slot(stage, 1, r, i) : source(1, row)[i * blockDim.x];
-          if constexpr (RES) dr[r][i] = RING ? *slot(stage, 2, r, i) : source(2, row)[i * blockDim.x];
+          if constexpr (AHEAD) dr[r][i] = RING ? *slot(stage, 2, r, i) : source(2, row)[i * blockDim.x];
         }
       }
     }
@@ -323,17 +325,20 @@ __global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1) rmsnorm_bwd_kernel(cons
             dwacc[i][j] += gv[j] * xv[j] * rstd[r];
           }
           bf16x8 ov;
-          ov.pack(o);
           if constexpr (RES) {
             float s[8];
             bf16x8 rr;
-            rr.raw = RING ? *slot(stage, 2, r, i) : dr[r][i];
+            if constexpr (AHEAD) rr.raw = RING ? *slot(stage, 2, r, i) : dr[r][i];
+            else rr.raw = source(2, row)[i * blockDim.x];
             rr.unpack(s);
-            ov.unpack(o);
+            if (apart) {
+              ov.pack(o);
+              ov.unpack(o);
+            }
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j] += s[j];
-            ov.pack(o);
           }
+          ov.pack(o);
           reinterpret_cast<uint4*>(dx + row * (long long)H)[vi] = ov.raw;
         }
       }
@@ -564,8 +569,8 @@ int mcb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, void* y, v
   return (int)cudaGetLastError();
 }
 
-static int rmsnorm_bwd_launch(const void* dy, void* y, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                              void* dw_any, int dw_bf16, float* partials, long long rows, int H, long long ldx, float eps,
+static int rmsnorm_bwd_launch(const void* dy, void* y, const void* x, const void* w, const float* rstd, const void* dres, int apart,
+                              void* dx, void* dw_any, int dw_bf16, float* partials, long long rows, int H, long long ldx, float eps,
                               int zero_centered, cudaStream_t s) {
   float* dw = dw_bf16 ? nullptr : reinterpret_cast<float*>(dw_any);
   if (rows == 0) return 0;
@@ -580,7 +585,6 @@ static int rmsnorm_bwd_launch(const void* dy, void* y, const void* x, const void
   long long grid = pairs < cap ? pairs : cap;
   if (!dw_any) partials = nullptr;
   if (dw_bf16 && !partials) return -3;
-  if (dres && vpt > 4) return -4;
   const bool ring = pairs > grid && vpt <= 4;
 #define LAUNCH(V, R, P)                                                                                              \
   do {                                                                                                               \
@@ -594,7 +598,7 @@ static int rmsnorm_bwd_launch(const void* dy, void* y, const void* x, const void
     }                                                                                                                \
     rmsnorm_bwd_kernel<V, R, P><<<(int)grid, threads, smem, s>>>(                                                     \
         (const __nv_bfloat16*)dy, (__nv_bfloat16*)y, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,          \
-        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw, partials, rows, H, ldx, eps, zero_centered);             \
+        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw, partials, rows, H, ldx, eps, zero_centered, apart);      \
   } while (0)
 #define LAUNCH_V(V)                     \
   do {                                  \
@@ -606,6 +610,7 @@ static int rmsnorm_bwd_launch(const void* dy, void* y, const void* x, const void
   if (vpt <= 1) LAUNCH_V(1);
   else if (vpt <= 2) LAUNCH_V(2);
   else if (vpt <= 4) LAUNCH_V(4);
+  else if (dres) LAUNCH(8, true, false);
   else LAUNCH(8, false, false);
 #undef LAUNCH_V
 #undef LAUNCH
@@ -617,10 +622,10 @@ static int rmsnorm_bwd_launch(const void* dy, void* y, const void* x, const void
 }
 
 // dw (fp32, [H]) is accumulated into (with atomics: the sum order varies from run to run); pass nullptr to skip.
-// dres (optional, H <= 8192) is added to dx (residual branch).
+// dres (optional) is added to dx (residual branch), in fp32.
 int mcb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                     float* dw, long long rows, int H, long long ldx, float eps, int zero_centered, void* stream_) {
-  return rmsnorm_bwd_launch(dy, nullptr, x, w, rstd, dres, dx, dw, 0, nullptr, rows, H, ldx, eps, zero_centered,
+  return rmsnorm_bwd_launch(dy, nullptr, x, w, rstd, dres, 0, dx, dw, 0, nullptr, rows, H, ldx, eps, zero_centered,
                             reinterpret_cast<cudaStream_t>(stream_));
 }
 
@@ -640,15 +645,23 @@ int mcb_rmsnorm_bwd_partial_rows(long long rows, int H) {
 int mcb_rmsnorm_bwd_det(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                         void* dw, int dw_bf16, float* partials, long long rows, int H, long long ldx, float eps,
                         int zero_centered, void* stream_) {
-  return rmsnorm_bwd_launch(dy, nullptr, x, w, rstd, dres, dx, dw, dw_bf16, partials, rows, H, ldx, eps, zero_centered,
+  return rmsnorm_bwd_launch(dy, nullptr, x, w, rstd, dres, 0, dx, dw, dw_bf16, partials, rows, H, ldx, eps, zero_centered,
                             reinterpret_cast<cudaStream_t>(stream_));
 }
 
-// mcb_rmsnorm_bwd_det with the forward's result recomputed on the way: it replaces dy.  rstd as kept by the forward.
+// mcb_rmsnorm_bwd_det with dres added to the rounded dx, as by an addition of its own.
+int mcb_rmsnorm_bwd_det_add(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
+                            void* dw, int dw_bf16, float* partials, long long rows, int H, long long ldx, float eps,
+                            int zero_centered, void* stream_) {
+  return rmsnorm_bwd_launch(dy, nullptr, x, w, rstd, dres, 1, dx, dw, dw_bf16, partials, rows, H, ldx, eps, zero_centered,
+                            reinterpret_cast<cudaStream_t>(stream_));
+}
+
+// mcb_rmsnorm_bwd_det_add with the forward's result recomputed on the way: it replaces dy.  rstd as kept by the forward.
 int mcb_rmsnorm_bwd_det_y(void* dy_y, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                           void* dw, int dw_bf16, float* partials, long long rows, int H, long long ldx, float eps,
                           int zero_centered, void* stream_) {
-  return rmsnorm_bwd_launch(dy_y, dy_y, x, w, rstd, dres, dx, dw, dw_bf16, partials, rows, H, ldx, eps, zero_centered,
+  return rmsnorm_bwd_launch(dy_y, dy_y, x, w, rstd, dres, 1, dx, dw, dw_bf16, partials, rows, H, ldx, eps, zero_centered,
                             reinterpret_cast<cudaStream_t>(stream_));
 }
 

@@ -176,7 +176,8 @@ void norm_fwd(const Tensor& x2, const Tensor& w, float eps, bool zc, const Tenso
 void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor& rstd, float eps, bool zc, bool over,
               bool need_dw, const Tensor& dres_, Tensor& dx, Tensor& dw) {
   const ll rows = x2.size(0), H = x2.size(1);
-  const Tensor dres = H <= 8192 ? dres_ : Tensor();   // a wider row's kernel has no registers for it
+  // a wider row's kernel has no registers for it: 3000 x 12288 189 us, 114 without it and an addition of 221 MB
+  const Tensor dres = H <= 8192 ? dres_ : Tensor();
   operand(dy, at::kBFloat16, rows * H, x2, "norm gradient: bf16 of the input's size");
   operand(w, at::kBFloat16, H, x2, "norm weight: bf16, one for every column");
   operand(rstd, at::kFloat, rows, x2, "norm: an fp32 for every row");
@@ -191,7 +192,7 @@ void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor&
     launch("mcb_rmsnorm_bwd_det", mcb_rmsnorm_bwd_det_y, dy.data_ptr(), x2.data_ptr(), w.data_ptr(), rstd.data_ptr(), ptr(dres),
            dx.data_ptr(), ptr(dw), need_dw, ptr(part), rows, H, x2.stride(0), eps, zc, stream());
   else
-    launch("mcb_rmsnorm_bwd_det", mcb_rmsnorm_bwd_det, dy.data_ptr(), x2.data_ptr(), w.data_ptr(), rstd.data_ptr(), ptr(dres),
+    launch("mcb_rmsnorm_bwd_det", mcb_rmsnorm_bwd_det_add, dy.data_ptr(), x2.data_ptr(), w.data_ptr(), rstd.data_ptr(), ptr(dres),
            dx.data_ptr(), ptr(dw), need_dw, ptr(part), rows, H, x2.stride(0), eps, zc, stream());
   if (dres_.defined() && !dres.defined()) dx = dx.add(dres_);
 }

@@ -24,7 +24,7 @@ typedef long long ll;
   X(mcb_gemm_bf16_residual, int, (const void*, ll, const void*, ll, void*, ll, const void*, ll, int, int, int, const void*,   \
                                   int*, void*))                                                                         \
   X(mcb_rmsnorm_fwd, int, (const void*, const void*, const void*, void*, void*, float*, ll, int, ll, float, int, void*))  \
-  X(mcb_rmsnorm_bwd_det, int, (const void*, const void*, const void*, const float*, const void*, void*, void*, int, float*,   \
+  X(mcb_rmsnorm_bwd_det_add, int, (const void*, const void*, const void*, const float*, const void*, void*, void*, int, float*,   \
                                ll, int, ll, float, int, void*))                                                         \
   X(mcb_rmsnorm_bwd_det_y, int, (void*, const void*, const void*, const float*, const void*, void*, void*, int, float*, ll,   \
                                  int, ll, float, int, void*))                                                           \
@@ -108,7 +108,7 @@ enum Layout { NT = 0, NN = 1, TN = 2 };
 Tensor gemm(int layout, const Tensor& a, const Tensor& b, const Tensor& bias = {}, const Tensor& out = {}, bool fp32 = false,
             bool accumulate = false, float alpha = 1.f, int max_sms = 0, int force_bn = 0);
 void norm_fwd(const Tensor& x2, const Tensor& w, float eps, bool zc, const Tensor& y, Tensor& rstd);
-// `over` replaces dy with the norm's result; `dres` (optional, [rows, H]) is added to dx
+// `over` replaces dy with the norm's result; `dres` (optional, [rows, H]) is added to the rounded dx
 void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor& rstd, float eps, bool zc, bool over, bool need_dw,
               const Tensor& dres, Tensor& dx, Tensor& dw);
 // y = res + a . b^T (+ bias) in the kernel's epilogue; false where the kernel does not take the operands

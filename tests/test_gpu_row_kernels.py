@@ -164,3 +164,25 @@ def test_heads_in_columns_of_a_wider_tensor(T, ng, qpg, d, gate):
 
     for a, b in zip(run(wide[:, :W]), run(wide[:, :W].clone())):
         assert a.shape == b.shape and torch.equal(a, b)
+
+
+@pytest.mark.parametrize('rows,H', [(5, 104), (700, 2048), (3, 8192), (7, 8200), (300, 16384)])
+def test_norm_backward_adds_a_residual_gradient_once_rounded(rows, H):
+    from mcore_bridge_b200.ops import _lib
+    lib, ptr, ll = _lib.lib(), lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr()), ctypes.c_longlong
+    x, dy, w = _rand(rows, H), _rand(rows, H, seed=1), _rand(H, seed=3)
+    wide = x.double()
+    r = torch.rsqrt(wide.pow(2).mean(-1, keepdim=True) + 1e-6)
+    g, xh = dy.double() * w.double(), wide * r
+    dx = r * (g - xh * (g * xh).mean(-1, keepdim=True))
+    res = (_rand(rows, H, seed=2) * 2 ** -6 - dx).bfloat16()           # the sum is small beside its two terms
+    part = torch.empty(lib.mcb_rmsnorm_bwd_partial_rows(ll(rows), H), H, device=DEV)
+    dw, acc = torch.empty_like(w), torch.zeros(H, device=DEV)
+    for f, extra in ((lib.mcb_rmsnorm_bwd_det, (ptr(dw), 1, ptr(part))), (lib.mcb_rmsnorm_bwd, (ptr(acc),))):
+        out = torch.empty_like(x)
+        assert f(ptr(dy), ptr(x), ptr(w), None, ptr(res), ptr(out), *extra, ll(rows), H, ll(H), ctypes.c_float(1e-6), 0,
+                 _lib.stream_ptr()) == 0
+        # half a unit of the last of the result's 8 bits, 2^-8 of it at most, and fp32 arithmetic on terms of the size of g and of xh
+        # times the mean: sums of up to 16384 terms over 256 chains, some 20 roundings of 2^-24 for the mean
+        size = r * (g.abs() + xh.abs() * (g * xh).abs().mean(-1, keepdim=True))
+        assert ((out.double() - (dx + res.double())).abs() <= 2 ** -8 * (dx + res.double()).abs() + 2 ** -18 * size).all()
