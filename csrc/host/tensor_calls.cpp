@@ -8,6 +8,7 @@
 
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
 
 #include <cstdlib>
 #include <cstring>
@@ -489,6 +490,7 @@ PyObject* seq_starts(PyObject*, PyObject* const* a, Py_ssize_t n) {          // 
   const Tensor cu = tensor(a[0]).contiguous();
   const ll T = integer(a[1]);
   require(cu.scalar_type() == at::kInt || cu.scalar_type() == at::kLong, "sequence boundaries: int32 or int64");
+  const c10::cuda::OptionalCUDAGuard here(at::device_of(cu));   // as a tensor operation: on the tensor's device
   const Tensor out = at::empty({T}, cu.options().dtype(at::kInt));
   launch("mcb_seq_starts", mcb_seq_starts, cu.data_ptr(), cu.scalar_type() == at::kLong, cu.numel(), out.data_ptr(), T, stream());
   return THPVariable_Wrap(out);
@@ -500,6 +502,7 @@ PyObject* rope_tables(PyObject*, PyObject* const* a, Py_ssize_t n) {         // 
   const Tensor pos = tensor(a[0]).contiguous(), inv = tensor(a[1]).contiguous();
   require(pos.scalar_type() == at::kInt || pos.scalar_type() == at::kLong, "positions: int32 or int64");
   operand(inv, at::kFloat, 0, pos, "inverse frequencies: fp32 on the positions' device");
+  const c10::cuda::OptionalCUDAGuard here(at::device_of(pos));
   const ll T = pos.numel(), R = inv.numel();
   const Tensor cos = at::empty({T, R}, inv.options()), sin = at::empty({T, R}, inv.options());
   launch("mcb_rope_tables", mcb_rope_tables, pos.data_ptr(), pos.scalar_type() == at::kLong, inv.data_ptr(), real(a[2]),

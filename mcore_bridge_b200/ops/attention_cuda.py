@@ -40,11 +40,18 @@ def supported(q, k, v, causal, window, sinks, softcap) -> bool:
     return unsupported_reason(q, k, v, causal, window, sinks, softcap) is None and _lib.available()
 
 
+def _here(t: torch.Tensor, device) -> bool:
+    """Whether a CUDA tensor is on ``device``, where ``cuda`` is the current one."""
+    device = torch.device(device)
+    index = torch.cuda.current_device() if device.type == 'cuda' and device.index is None else device.index
+    return device.type == 'cuda' and t.device.index == index
+
+
 def seq_start_from_cu(cu_seqlens: Optional[torch.Tensor], T: int, device) -> torch.Tensor:
     """``[T]`` int32: index of the first token of the packed sequence each token belongs to."""
     if cu_seqlens is None:
         return torch.zeros(T, dtype=torch.int32, device=device)
-    if cu_seqlens.is_cuda and cu_seqlens.device == torch.device(device) and cu_seqlens.numel() >= 2 \
+    if cu_seqlens.is_cuda and _here(cu_seqlens, device) and cu_seqlens.numel() >= 2 \
             and cu_seqlens.dtype in (torch.int32, torch.int64) and cu_seqlens.dim() == 1 and _lib.cuda_enabled():
         return _lib.native().seq_starts(cu_seqlens, T)
     cu = cu_seqlens.to(device=device, dtype=torch.int64)

@@ -10,11 +10,14 @@ DEV = 'cuda'
 @pytest.mark.parametrize('cu,T', [([0, 1], 1), ([0, 5, 5, 9], 9), ([0, 300], 300), ([0, 100, 257], 300), ([3, 10], 12),
                                   (list(range(0, 2001, 2)), 2000), ([0, 0, 0, 7], 7)])
 def test_sequence_starts(cu, T, dtype):
+    from mcore_bridge_b200.ops import _lib
     from mcore_bridge_b200.ops.attention_cuda import seq_start_from_cu
     host = torch.tensor(cu)
     seg = torch.searchsorted(host[1:].contiguous(), torch.arange(T), right=True)
     want = host[:-1][seg.clamp(max=len(cu) - 2)].int()
+    before = _lib.LAUNCHES
     got = seq_start_from_cu(host.to(DEV, dtype), T, DEV)
+    assert _lib.LAUNCHES == before + 1
     assert got.dtype == torch.int32 and torch.equal(got.cpu(), want)
     wide = torch.stack([host, host], 1).to(DEV, dtype)[:, 0]             # strided
     assert torch.equal(seq_start_from_cu(wide, T, DEV).cpu(), want)
@@ -50,3 +53,17 @@ def test_head_statistics(rows, tiles):
     # fp32 sums of up to 594 positive terms in 32 chains: a few units in the last place
     assert ((lse.double() - want).abs()[ok] <= 2 ** -21 * want.abs().clamp(min=1)[ok]).all()
     assert torch.equal(loss[ok], (lse - tgt)[ok])
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason='needs 2 GPUs')
+def test_tables_of_another_device_than_the_current():
+    from mcore_bridge_b200.ops import _lib
+    from mcore_bridge_b200.ops.attention_cuda import seq_start_from_cu
+    cu = torch.tensor([0, 100, 257], dtype=torch.int32, device='cuda:1')
+    got = seq_start_from_cu(cu, 300, 'cuda:1')
+    assert got.device == cu.device and got.tolist() == [0] * 100 + [100] * 200
+    assert seq_start_from_cu(cu, 300, 'cuda').device == torch.device('cuda', torch.cuda.current_device())
+    pos, inv = torch.arange(50, device='cuda:1'), torch.rand(8, device='cuda:1')
+    cos, sin = _lib.native().rope_tables(pos, inv, 1.0)
+    freqs = pos.float()[:, None] * inv[None]
+    assert torch.equal(cos, freqs.cos()) and torch.equal(sin, freqs.sin())
