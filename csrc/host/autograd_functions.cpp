@@ -376,6 +376,9 @@ PyObject* attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     k = k_.contiguous();
     v = v_.contiguous();
     if (sinks_.defined()) sinks = sinks_.detach().to(at::kFloat).contiguous();
+    if (grad)                                    // the backward pass's, before anything runs
+      for (const Tensor& t : {q_lo, q_hi})
+        operand(t, at::kInt, k.size(0), q, "first and last queries: an int32 for every key, on the keys' device");
     attn_forward(q, k, v, k_lo, k_hi, sinks, scale, o, lse);
   }
   if (grad) {

@@ -353,69 +353,6 @@ PyObject* mm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 GluArgs glu_args(PyObject* const* a) { return {static_cast<int>(integer(a[0])), real(a[1]), real(a[2])}; }
-QkvArgs qkv_args(PyObject* const* a) {   // ng, qpg, d, has_gate, interleaved, eps, zc
-  return {integer(a[0]), integer(a[1]), integer(a[2]), truth(a[3]), truth(a[4]), real(a[5]), truth(a[6])};
-}
-
-PyObject* rmsnorm_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {       // x, w, eps, zc -> y, x2, rstd
-  MCB_BEGIN(4)
-  const Tensor& x = tensor(a[0]);
-  const Tensor x2 = rows_of(x, x.size(-1)), y = at::empty_like(x2, at::MemoryFormat::Contiguous);
-  Tensor rstd;
-  norm_fwd(x2, tensor(a[1]), real(a[2]), truth(a[3]), y, rstd);
-  return tuple({y, x2, rstd});
-  MCB_END
-}
-
-PyObject* rmsnorm_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {       // dy, x2, w, rstd, eps, zc, need_dw -> dx, dw
-  MCB_BEGIN(7)
-  const Tensor& x2 = tensor(a[1]);
-  const Tensor dy = tensor(a[0]).reshape({x2.size(0), x2.size(1)}).contiguous();
-  Tensor dx, dw;
-  norm_bwd(dy, x2, tensor(a[2]), tensor(a[3]), real(a[4]), truth(a[5]), false, truth(a[6]), {}, dx, dw);
-  return tuple({dx, dw});
-  MCB_END
-}
-
-PyObject* norm_linear_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {   // x, norm weight, weight, eps, zc -> y, x2, rstd
-  MCB_BEGIN(5)
-  const Tensor& x = tensor(a[0]);
-  const Tensor x2 = rows_of(x, x.size(-1)), xn = at::empty_like(x2, at::MemoryFormat::Contiguous);
-  Tensor rstd;
-  norm_fwd(x2, tensor(a[1]), real(a[3]), truth(a[4]), xn, rstd);
-  return tuple({gemm(NT, xn, tensor(a[2])), x2, rstd});
-  MCB_END
-}
-
-// dy, x2, norm weight, rstd, weight, eps, zc, need_dw -> dx, d norm weight, dy2, normalised input (with need_dw)
-PyObject* norm_linear_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  MCB_BEGIN(8)
-  const Tensor &x2 = tensor(a[1]), &w = tensor(a[4]);
-  const Tensor dy2 = rows_of(tensor(a[0]), w.size(0)), dxn = gemm(NN, dy2, w);
-  Tensor dx, dlw;
-  norm_bwd(dxn, x2, tensor(a[2]), tensor(a[3]), real(a[5]), truth(a[6]), truth(a[7]), true, {}, dx, dlw);
-  return tuple({dx, dlw, dy2, truth(a[7]) ? dxn : Tensor()});
-  MCB_END
-}
-
-PyObject* glu_linear_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {    // h, weight, kind, clamp, offset -> y, h2
-  MCB_BEGIN(5)
-  const Tensor& h = tensor(a[0]);
-  const Tensor h2 = rows_of(h, h.size(-1));
-  return tuple({gemm(NT, glu_rows_fwd(h2, {}, glu_args(a + 2)), tensor(a[1])), h2});
-  MCB_END
-}
-
-// dy, h2, weight, kind, clamp, offset, need_dw -> dh, dy2, activation (with need_dw)
-PyObject* glu_linear_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  MCB_BEGIN(7)
-  const Tensor &h2 = tensor(a[1]), &w = tensor(a[2]);
-  const Tensor dy2 = rows_of(tensor(a[0]), w.size(0)), da = gemm(NN, dy2, w);
-  Tensor none;
-  const Tensor dh = glu_rows_bwd(da, h2, {}, glu_args(a + 3), truth(a[6]), none);
-  return tuple({dh, dy2, truth(a[6]) ? da : Tensor()});
-  MCB_END
-}
 
 PyObject* glu_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {           // x, probs, kind, clamp, offset -> y, x2
   MCB_BEGIN(5)
@@ -432,45 +369,6 @@ PyObject* glu_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {           // dy
   Tensor dp;
   const Tensor dx = glu_rows_bwd(dy, x2, optional(a[2]), glu_args(a + 3), false, dp);
   return tuple({dx, dp});
-  MCB_END
-}
-
-// qkv, wq, wk, cos, sin, ng, qpg, d, has_gate, interleaved, eps, zc -> q, k, v, gate, qkv
-PyObject* qkv_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  MCB_BEGIN(12)
-  const Tensor& qkv_ = tensor(a[0]);
-  const Tensor qkv = qkv_.stride(-1) == 1 ? qkv_ : qkv_.contiguous();
-  const Qkv r = qkv_split(qkv, optional(a[1]), optional(a[2]), optional(a[3]), optional(a[4]), qkv_args(a + 5));
-  return tuple({r.q, r.k, r.v, r.gate, qkv});
-  MCB_END
-}
-
-// dq, dk, dv, dgate, qkv, wq, wk, cos, sin, ng, qpg, d, has_gate, interleaved, eps, zc -> dqkv, dwq, dwk
-PyObject* qkv_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  MCB_BEGIN(16)
-  Tensor dqkv, dwq, dwk;
-  qkv_join({optional(a[0]), optional(a[1]), optional(a[2]), optional(a[3])}, tensor(a[4]), optional(a[5]), optional(a[6]),
-           optional(a[7]), optional(a[8]), qkv_args(a + 9), dqkv, dwq, dwk);
-  return tuple({dqkv, dwq, dwk});
-  MCB_END
-}
-
-// q, k, v, k_lo, k_hi, sinks, scale -> o, lse, q, k, v (contiguous)
-PyObject* attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  MCB_BEGIN(7)
-  const Tensor q = tensor(a[0]).contiguous(), k = tensor(a[1]).contiguous(), v = tensor(a[2]).contiguous();
-  Tensor o, lse;
-  attn_forward(q, k, v, tensor(a[3]), optional(a[4]), optional(a[5]), real(a[6]), o, lse);
-  return tuple({o, lse, q, k, v});
-  MCB_END
-}
-
-// do, q, k, v, o, lse, k_lo, k_hi, q_lo, q_hi, sinks, bf16 sinks, scale -> dq, dk, dv, dsinks
-PyObject* attn_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  MCB_BEGIN(13)
-  const AttnGrads g = attn_backward(tensor(a[0]), tensor(a[1]), tensor(a[2]), tensor(a[3]), tensor(a[4]), tensor(a[5]), tensor(a[6]),
-                                    optional(a[7]), optional(a[8]), optional(a[9]), optional(a[10]), truth(a[11]), real(a[12]));
-  return tuple({g.dq, g.dk, g.dv, g.dsinks});
   MCB_END
 }
 
@@ -588,18 +486,8 @@ PyMethodDef methods[] = {MCB_FAST(init),
                          {"raw_stream", raw_stream, METH_NOARGS, nullptr},
                          MCB_FAST(memory),
                          MCB_FAST(mm),
-                         MCB_FAST(rmsnorm_fwd),
-                         MCB_FAST(rmsnorm_bwd),
-                         MCB_FAST(norm_linear_fwd),
-                         MCB_FAST(norm_linear_bwd),
-                         MCB_FAST(glu_linear_fwd),
-                         MCB_FAST(glu_linear_bwd),
                          MCB_FAST(glu_fwd),
                          MCB_FAST(glu_bwd),
-                         MCB_FAST(qkv_fwd),
-                         MCB_FAST(qkv_bwd),
-                         MCB_FAST(attn_fwd),
-                         MCB_FAST(attn_bwd),
                          MCB_FAST(attn_window_starts),
                          MCB_FAST(attn_dkv_splits),
                          MCB_FAST(seq_starts),

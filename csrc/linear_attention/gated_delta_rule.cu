@@ -94,7 +94,6 @@ __device__ __forceinline__ ChunkPos locate(const GdrParams& p, ChunkPos* slot) {
   return *slot;
 }
 
-// 64 x 64 bf16 matrix (contiguous) -> tile
 // exp of a sum of two floats, the second far smaller
 __device__ __forceinline__ float exp_pair(float hi, float lo) {
   const float e = expf(hi);

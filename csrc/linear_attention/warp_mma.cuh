@@ -106,14 +106,6 @@ __device__ __forceinline__ void mma_terms(float (&c)[4], float (&lo)[4], const u
     for (int i = 0; i <= o; ++i) mma16816(lo, a[i], b[o - i][2 * u], b[o - i][2 * u + 1]);
 }
 
-// accumulators of two neighbouring 16 x 8 blocks -> the A operand of the next product, as two terms
-__device__ __forceinline__ void acc_to_a(const float (&c0)[4], const float (&c1)[4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-  split2(c0[0], c0[1], hi[0], lo[0]);
-  split2(c0[2], c0[3], hi[1], lo[1]);
-  split2(c1[0], c1[1], hi[2], lo[2]);
-  split2(c1[2], c1[3], hi[3], lo[3]);
-}
-
 // 16-byte asynchronous copy; `bytes` 0 writes zeros instead of reading
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");

@@ -45,16 +45,16 @@ def test_attention_refuses_other_starts(start, window):
 @pytest.mark.parametrize('bad', REFUSED)
 def test_ranges_are_checked_before_the_launch(bad):
     nat, q, good = _lib.native(), torch.zeros(T, 2, 64, dtype=torch.bfloat16), torch.zeros(T, dtype=torch.int32)
-    lse = torch.zeros(2, T)
     before = _lib.LAUNCHES
     for ranges in [(bad, None), (good, bad)]:
         with pytest.raises(AssertionError):
-            nat.attn_fwd(q, q, q, *ranges, None, 1.0)
+            nat.attention(q, q, q, *ranges, None, None, None, 1.0)
     with pytest.raises(AssertionError):
-        nat.attn_fwd(q, q, q, good, None, torch.zeros(1), 1.0)               # two heads
+        nat.attention(q, q, q, good, None, None, None, torch.zeros(1), 1.0)  # two heads
+    leaf = q.clone().requires_grad_()
     for ranges in [(bad, None, None, None), (good, bad, good, good), (good, good, bad, good), (good, good, good, bad)]:
         with pytest.raises(AssertionError):
-            nat.attn_bwd(q, q, q, q, q, lse, *ranges, None, False, 1.0)
+            nat.attention(leaf, q, q, *ranges, None, 1.0)
     assert _lib.LAUNCHES == before
 
 

@@ -37,17 +37,24 @@ def _bf(*shape):
     lambda n: n.mm(0, _bf(8, 8), _bf(8, 8), None, torch.zeros(8, 8, device=META), False, False, 1.0, 0, 0),
     lambda n: n.mm(0, _bf(8, 8), _bf(8, 8), torch.zeros(7), None, False, False, 1.0, 0, 0),               # a bias too short
     lambda n: n.mm(2, _bf(8, 8), _bf(8, 8), None, _bf(2, 4, 8), False, False, 1.0, 0, 0),                  # a gradient of 3 axes
-    lambda n: n.rmsnorm_fwd(_bf(4, 16), torch.zeros(16), 1e-6, False),
-    lambda n: n.rmsnorm_fwd(_bf(4, 16), _bf(8), 1e-6, False),
-    lambda n: n.rmsnorm_bwd(_bf(4, 16), _bf(4, 16), _bf(16), torch.zeros(3), 1e-6, False, True),
-    lambda n: n.norm_linear_fwd(_bf(4, 16), _bf(16).to(META), _bf(8, 16), 1e-6, False),
+    lambda n: n.rmsnorm(_bf(4, 16), torch.zeros(16), 1e-6, False),
+    lambda n: n.rmsnorm(_bf(4, 16), _bf(8), 1e-6, False),
+    lambda n: n.rmsnorm(torch.zeros(4, 16), _bf(16), 1e-6, False),
+    lambda n: n.linear(_bf(4, 16), torch.zeros(8, 16), None, False, None),
+    lambda n: n.linear(_bf(4, 16), _bf(8, 8), None, False, None),
+    lambda n: n.linear(_bf(4, 16), _bf(8, 16), torch.zeros(7), False, None),
+    lambda n: n.linear(_bf(4, 16), _bf(8, 16), None, False, _bf(4, 16)),                                   # a residual of another shape
+    lambda n: n.linear(_bf(4, 16), _bf(8, 16), None, False, _bf(4, 8).to(META)),
+    lambda n: n.norm_linear(_bf(4, 16), _bf(16).to(META), _bf(8, 16), 1e-6, False, False),
     lambda n: n.glu_fwd(torch.zeros(4, 16), None, 0, 0.0, 0.0),
     lambda n: n.glu_fwd(_bf(4, 16), torch.zeros(3), 0, 0.0, 0.0),
-    lambda n: n.glu_linear_fwd(torch.zeros(4, 16), _bf(8, 8), 0, 0.0, 0.0),
-    lambda n: n.qkv_fwd(_bf(4, 31), None, None, None, None, 1, 2, 8, False, False, 1e-6, False),           # 4 heads of 8
-    lambda n: n.qkv_fwd(_bf(4, 32), _bf(8), _bf(4), None, None, 1, 2, 8, False, False, 1e-6, False),
-    lambda n: n.qkv_fwd(_bf(4, 32), None, None, torch.zeros(4, 4), torch.zeros(3, 4), 1, 2, 8, False, False, 1e-6, False),
-    lambda n: n.attn_fwd(_bf(4, 2, 64), _bf(4, 2, 64), torch.zeros(4, 2, 64), torch.zeros(4, dtype=torch.int32), None, None, 1.0),
+    lambda n: n.glu_bwd(_bf(4, 8), _bf(4, 16), torch.zeros(3), 0, 0.0, 0.0),
+    lambda n: n.glu_linear(torch.zeros(4, 16), _bf(8, 8), 0, 0.0, 0.0, None),
+    lambda n: n.qkv(_bf(4, 31), None, None, None, None, 1, 2, 8, False, False, 1e-6, False),               # 4 heads of 8
+    lambda n: n.qkv(_bf(4, 32), _bf(8), _bf(4), None, None, 1, 2, 8, False, False, 1e-6, False),
+    lambda n: n.qkv(_bf(4, 32), None, None, torch.zeros(4, 4), torch.zeros(3, 4), 1, 2, 8, False, False, 1e-6, False),
+    lambda n: n.attention(_bf(4, 2, 64), _bf(4, 2, 64), torch.zeros(4, 2, 64), torch.zeros(4, dtype=torch.int32), None, None, None,
+                          None, 1.0),
 ])
 def test_operands_the_kernels_would_misread_are_refused(call):
     before = _lib.LAUNCHES
