@@ -54,8 +54,7 @@ namespace {
 constexpr int C = 64;           // tokens of a chunk
 constexpr int THREADS = 128;    // 4 warps, 16 tokens each
 constexpr int ST = 512;         // scans: 4 strips of 16 columns of v, 4 warps each
-constexpr int CC = C * C;       // elements of a chunk's square matrices
-constexpr int SQ = CC * 2;      // bytes of one of their bf16 terms
+constexpr int SQ = C * C * 2;   // bytes of one bf16 term of a chunk's square matrices
 constexpr int MP = 3;           // terms kept of M and P
 
 // rows of `gb`: G as a sum of two floats, beta, exp(G), exp(G_last - G), the diagonal p
@@ -64,6 +63,7 @@ enum { G_HI, G_LO, G_BETA, G_EXP, G_REST, G_DIAG, G_ROWS };
 // M and P are kept as the ten 16 x 16 blocks on and below the diagonal, 512 bytes each; the two halves of a row change places every
 // four rows, so that in shared memory, where they are copied as they are, eight rows of a half lie in distinct banks.
 constexpr int SQB = 10 * 512;   // bytes of one term
+constexpr int MPE = MP * SQB / 2;   // elements of all terms of M, or of P
 __device__ __forceinline__ int block_off(int bi, int bj, int r, int half) {
   return (bi * (bi + 1) / 2 + bj) * 512 + r * 32 + ((half ^ ((r >> 2) & 1)) << 4);
 }
@@ -75,7 +75,7 @@ struct GdrParams {
   __nv_bfloat16 *o, *dq, *dk, *dv;
   float *dg, *dbeta;                       // [T, H]
   // per chunk and head, chunks numbered through the packed batch:
-  __nv_bfloat16* mp;                       // [2 MP, 64, 64], of each a part: M and P, MP terms each, one behind the other
+  __nv_bfloat16* mp;                       // [2, MP, 10, 16, 16]: blocks of M and P
   float* gb;                               // [G_ROWS, 64] (beta 0 past the end of the sequence)
   float *S, *dS;                           // [D, D]: S^T and dS'^T
   __nv_bfloat16 *V, *B;                    // [2, D, 64]: V^T and B^T, two terms, as tiles in shared memory
@@ -155,7 +155,7 @@ gdr_prep_kernel(const GdrParams p) {
   cp_async_wait<0>();
   __syncthreads();
   const int r0 = warp * 16, i = r0 + (lane >> 2);
-  __nv_bfloat16* mp = p.mp + ch * 2 * MP * CC;
+  __nv_bfloat16* mp = p.mp + ch * 2 * MPE;
   const float gh[2] = {s_gh[i], s_gh[i + 8]}, gl[2] = {s_gl[i], s_gl[i + 8]};
   for (int jb = 0; jb < 4; ++jb) {
     float kk2[2][4] = {}, qk2[2][4] = {};
@@ -192,7 +192,7 @@ gdr_prep_kernel(const GdrParams p) {
 #pragma unroll
         for (int m = 0; m < MP; ++m)
           if (jb <= warp)
-            *reinterpret_cast<uint32_t*>(mp + MP * CC + (m * SQB + block_off(warp, jb, (lane >> 2) + 8 * r, n)) / 2 +
+            *reinterpret_cast<uint32_t*>(mp + MPE + (m * SQB + block_off(warp, jb, (lane >> 2) + 8 * r, n)) / 2 +
                                          (lane & 3) * 2) = t[m][0];
       }
     }
@@ -330,8 +330,8 @@ struct StageLoad {
       mbar_expect_tx(full, 4 * C * 4);
       bulk_load_1d(st + L::G, p.gb + (ch * G_ROWS + G_BETA) * C, 4 * C * 4, full);
       mbar_expect_tx(full + 16, 2 * NT * SQB);
-      bulk_load_1d(st + L::M, p.mp + ch * 2 * MP * CC, NT * SQB, full + 16);
-      bulk_load_1d(st + L::P, p.mp + (ch * 2 * MP + MP) * CC, NT * SQB, full + 16);
+      bulk_load_1d(st + L::M, p.mp + ch * 2 * MPE, NT * SQB, full + 16);
+      bulk_load_1d(st + L::P, p.mp + (ch * 2 + 1) * MPE, NT * SQB, full + 16);
     }
     const long long first = ((long long)t * p.H + h) * D;
     const __nv_bfloat16 *k = p.k + first, *q = p.q + first;
@@ -1353,7 +1353,7 @@ extern "C" {
 int mcb_gdr_chunks(int T, int n_seq) { return T / C + n_seq; }
 
 // q, k, v, o [T, H, D] bf16; g, beta [T, H] fp32; cu_seqlens [n_seq + 1] int32 from 0 to T.  Workspaces, per chunk and
-// head: mp [6, 64, 64] bf16, gb [6, 64] fp32; the backward pass reads them again.  Boundaries outside the batch are clipped
+// head: mp [2, 3, 10, 16, 16] bf16, gb [6, 64] fp32; the backward pass reads them again.  Boundaries outside the batch are clipped
 // and reported through `status`.
 int mcb_gdr_fwd(const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu_seqlens, void* o,
                 void* mp, float* gb, int T, int n_seq, int H, int D, float scale, int* status, void* stream_) {

@@ -371,7 +371,7 @@ class _SimpleGlaFn(torch.autograd.Function):
 
 class _GatedDeltaRuleFn(torch.autograd.Function):
     """``csrc/linear_attention/gated_delta_rule.cu``; kept for the backward pass: the inputs and, per chunk and head,
-    the two 64 x 64 matrices ``prep`` forms (three bf16 terms each: as much as q, k and v at a head size of 128)."""
+    the lower triangles of the two 64 x 64 matrices ``prep`` forms, in blocks of 16 and three bf16 terms each."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, cu, scale, covered):
@@ -383,7 +383,7 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
         n_seq = max(cu.numel() - 1, 0)
         o = torch.empty_like(v) if covered else torch.zeros_like(v)
         n = lib.mcb_gdr_chunks(T, n_seq) * h
-        mp = torch.empty((n, 6, 64, 64), dtype=torch.bfloat16, device=q.device)
+        mp = torch.empty((n, 2, 3, 10, 16, 16), dtype=torch.bfloat16, device=q.device)
         gb = torch.empty((n, 6, 64), dtype=torch.float32, device=q.device)
         rc = lib.mcb_gdr_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(g), _lib.ptr(beta), _lib.ptr(cu),
                              _lib.ptr(o), _lib.ptr(mp), _lib.ptr(gb), ctypes.c_int(T), ctypes.c_int(n_seq),

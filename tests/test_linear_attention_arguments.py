@@ -96,3 +96,18 @@ def test_kernels_that_wait_know_where_to_report(monkeypatch, op):
     torch.autograd.grad(o, (q, k, v), torch.ones_like(o))
     calls = {n: p for n, p in rec.pointers.items() if n.endswith(('_fwd', '_bwd'))}
     assert len(calls) == 2 and all(status.data_ptr() in p for p in calls.values())
+
+
+def test_what_the_delta_rule_keeps(monkeypatch):
+    """Of a chunk's two triangular 64 x 64 matrices, in three terms, the ten 16 x 16 blocks on and below the diagonal."""
+    monkeypatch.setattr(gdn, '_cuda_ok', lambda *ts: True)
+    monkeypatch.setattr(_lib, 'lib', lambda: _Recorder())
+    monkeypatch.setattr(_lib, 'stream_ptr', lambda: ctypes.c_void_p(0))
+    monkeypatch.setattr(_lib, 'status_word', lambda device=None: torch.zeros(16, dtype=torch.int32))
+    inputs = [t.requires_grad_() for t in _tensors()]
+    kept = {}
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.setdefault(t.data_ptr(), t), lambda t: t):
+        gdn.chunk_gated_delta_rule(*inputs)
+    own = sum(t.numel() * t.element_size() for p, t in kept.items() if p not in {x.data_ptr() for x in inputs})
+    chunks = 4 * H                               # _Recorder's, of every head
+    assert own <= chunks * (6 * 10 * 256 * 2 + 6 * 64 * 4) + 64
