@@ -200,7 +200,7 @@ PyObject* rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {   // x, weight,
   Tensor y, x2, rstd;
   {
     at::NoGradGuard none;
-    x2 = rows_of(x, x.size(-1));
+    x2 = aligned(rows_of(x, x.size(-1)));
     y = at::empty(x.sizes(), x.options());
     norm_fwd(x2, w, eps, zc, y, rstd);
   }
@@ -243,7 +243,7 @@ PyObject* norm_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor y, x2, rstd;
   {
     at::NoGradGuard none;
-    x2 = rows_of(x, x.size(-1));
+    x2 = aligned(rows_of(x, x.size(-1)));
     const Tensor xn = at::empty_like(x2, at::MemoryFormat::Contiguous);
     norm_fwd(x2, ln_w, eps, zc, xn, rstd);
     y = product(xn, w, {}, x);
@@ -294,7 +294,7 @@ PyObject* glu_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {   // h, weig
   Tensor y, h2;
   {
     at::NoGradGuard none;
-    h2 = rows_of(h, h.size(-1));
+    h2 = aligned(rows_of(h, h.size(-1)));
     y = product(glu_rows_fwd(h2, {}, args), w, {}, h, residual);
   }
   if (grad) {
@@ -333,7 +333,7 @@ PyObject* qkv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor x2;
   {
     at::NoGradGuard none;
-    x2 = x.stride(-1) == 1 ? x : x.contiguous();
+    x2 = aligned(x.stride(-1) == 1 ? x : x.contiguous(), qkv_boundary(args, cos));
     r = qkv_split(x2, wq, wk, cos, sin, args);
   }
   if (grad) {

@@ -148,9 +148,9 @@ Tensor gemm(int layout, const Tensor& a_, const Tensor& b_, const Tensor& bias_,
 
 bool gemm_residual(const Tensor& a_, const Tensor& b_, const Tensor& bias_, const Tensor& res, const Tensor& y) {
   const ll M = a_.size(0), K = a_.size(1), N = b_.size(0);
-  auto aligned = [](const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
+  auto starts = [](const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
   if (M == 0 || K == 0 || N % 8 || res.dim() != 2 || res.scalar_type() != at::kBFloat16 || res.stride(1) != 1 || res.stride(0) % 8 ||
-      !aligned(res) || !aligned(y))
+      !starts(res) || !starts(y))
     return false;
   const Tensor a = tma_rows(a_), b = tma_rows(b_);
   operand(a, at::kBFloat16, M * K, a, "GEMM operands: bf16 on one device");
@@ -165,8 +165,9 @@ bool gemm_residual(const Tensor& a_, const Tensor& b_, const Tensor& bias_, cons
   return true;
 }
 
-void norm_fwd(const Tensor& x2, const Tensor& w, float eps, bool zc, const Tensor& y, Tensor& rstd) {
+void norm_fwd(const Tensor& x2, const Tensor& w_, float eps, bool zc, const Tensor& y, Tensor& rstd) {
   const ll rows = x2.size(0), H = x2.size(1);
+  const Tensor w = aligned(w_);
   operand(x2, at::kBFloat16, 0, x2, "norm input: bf16");
   operand(w, at::kBFloat16, H, x2, "norm weight: bf16, one for every column");
   rstd = at::empty({rows}, x2.options().dtype(at::kFloat));
@@ -174,11 +175,12 @@ void norm_fwd(const Tensor& x2, const Tensor& w, float eps, bool zc, const Tenso
          rows, H, x2.stride(0), eps, zc, stream());
 }
 
-void norm_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, const Tensor& rstd, float eps, bool zc, bool over,
+void norm_bwd(const Tensor& dy_, const Tensor& x2, const Tensor& w_, const Tensor& rstd, float eps, bool zc, bool over,
               bool need_dw, const Tensor& dres_, Tensor& dx, Tensor& dw) {
   const ll rows = x2.size(0), H = x2.size(1);
+  const Tensor dy = over ? dy_ : aligned(dy_), w = aligned(w_);   // what is replaced is a product's result
   // a wider row's kernel has no registers for it: 3000 x 12288 189 us, 114 without it and an addition of 221 MB
-  const Tensor dres = H <= 8192 ? dres_ : Tensor();
+  const Tensor dres = H <= 8192 ? aligned(dres_) : Tensor();
   operand(dy, at::kBFloat16, rows * H, x2, "norm gradient: bf16 of the input's size");
   operand(w, at::kBFloat16, H, x2, "norm weight: bf16, one for every column");
   operand(rstd, at::kFloat, rows, x2, "norm: an fp32 for every row");
@@ -261,8 +263,9 @@ static void check_qkv(const Tensor& qkv, const Tensor& wq, const Tensor& wk, con
   operand(sin, at::kFloat, T * (cos.defined() ? cos.size(-1) : 0), qkv, "sines: fp32, a row for every token");
 }
 
-Qkv qkv_split(const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin, const QkvArgs& g) {
-  check_qkv(qkv, wq, wk, cos, sin, g);
+Qkv qkv_split(const Tensor& qkv, const Tensor& wq_, const Tensor& wk_, const Tensor& cos_, const Tensor& sin_, const QkvArgs& g) {
+  check_qkv(qkv, wq_, wk_, cos_, sin_, g);
+  const Tensor wq = aligned(wq_, 4), wk = aligned(wk_, 4), cos = aligned(cos_, 8), sin = aligned(sin_, 8);
   const ll T = qkv.size(0), d = g.d;
   Qkv r;
   r.q = at::empty({T, g.ng * g.qpg, d}, qkv.options());
@@ -275,14 +278,18 @@ Qkv qkv_split(const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tenso
   return r;
 }
 
-void qkv_join(Qkv dr, const Tensor& qkv_, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin, const QkvArgs& g,
+void qkv_join(Qkv dr, const Tensor& qkv_, const Tensor& wq_, const Tensor& wk_, const Tensor& cos_, const Tensor& sin_, const QkvArgs& g,
               Tensor& dqkv, Tensor& dwq, Tensor& dwk) {
   // the kernels write the gradient with the strides they read qkv by: columns of a wider tensor are copied first
   const Tensor qkv = qkv_.contiguous();
   const ll T = qkv.size(0), d = g.d;
+  check_qkv(qkv, wq_, wk_, cos_, sin_, g);
+  const Tensor wq = aligned(wq_, 4), wk = aligned(wk_, 4), cos = aligned(cos_, 8), sin = aligned(sin_, 8);
   const bool norm = wq.defined();
-  check_qkv(qkv, wq, wk, cos, sin, g);
-  auto grad = [&](const Tensor& t, ll heads) { return t.defined() ? t.contiguous() : at::zeros({T, heads, d}, qkv.options()); };
+  const int bytes = qkv_boundary(g, cos);
+  auto grad = [&](const Tensor& t, ll heads) {
+    return t.defined() ? aligned(t.contiguous(), bytes) : at::zeros({T, heads, d}, qkv.options());
+  };
   const Tensor dq = grad(dr.q, g.ng * g.qpg), dk = grad(dr.k, g.ng), dv = grad(dr.v, g.ng);
   const Tensor dgate = g.gated ? grad(dr.gate, g.ng * g.qpg) : Tensor();
   dqkv = at::empty_like(qkv);
@@ -357,7 +364,7 @@ GluArgs glu_args(PyObject* const* a) { return {static_cast<int>(integer(a[0])), 
 PyObject* glu_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {           // x, probs, kind, clamp, offset -> y, x2
   MCB_BEGIN(5)
   const Tensor& x = tensor(a[0]);
-  const Tensor x2 = rows_of(x, x.size(-1));
+  const Tensor x2 = aligned(rows_of(x, x.size(-1)));
   return tuple({glu_rows_fwd(x2, optional(a[1]), glu_args(a + 2)), x2});
   MCB_END
 }
@@ -365,7 +372,7 @@ PyObject* glu_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {           // x,
 PyObject* glu_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {           // dy, x2, probs, kind, clamp, offset -> dx, dprobs
   MCB_BEGIN(6)
   const Tensor& x2 = tensor(a[1]);
-  const Tensor dy = tensor(a[0]).reshape({x2.size(0), x2.size(1) / 2}).contiguous();
+  const Tensor dy = aligned(tensor(a[0]).reshape({x2.size(0), x2.size(1) / 2}).contiguous());
   Tensor dp;
   const Tensor dx = glu_rows_bwd(dy, x2, optional(a[2]), glu_args(a + 3), false, dp);
   return tuple({dx, dp});

@@ -71,6 +71,10 @@ int* status_of(const Tensor& t);
 inline void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 Tensor rows_of(const Tensor& t, ll width);   // [rows, width] with a contiguous last dimension
+// What a kernel reads `bytes` at a time: a tensor that does not start on such a boundary is copied.
+inline Tensor aligned(const Tensor& t, int bytes = 16) {
+  return t.defined() && reinterpret_cast<uintptr_t>(t.data_ptr()) % bytes ? t.clone(at::MemoryFormat::Contiguous) : t;
+}
 // An operand a kernel reads at least n elements of one type from, beside `like`; an undefined one is left out.
 void operand(const Tensor& t, at::ScalarType type, ll n, const Tensor& like, const char* what);
 // What a kernel reads one int32 of per query or key from.
@@ -129,6 +133,11 @@ struct QkvArgs {
 struct Qkv {
   Tensor q, k, v, gate;
 };
+// The boundary its kernels want qkv and the gradients on: heads of 128 have one that reads 4 bytes where it has to.
+inline int qkv_boundary(const QkvArgs& g, const Tensor& cos) {
+  const ll pairs = (g.ng * (g.qpg * (g.gated ? 2 : 1) + 2) + 1) / 2;
+  return g.d == 128 && cos.defined() && cos.size(-1) == 64 && !g.interleaved && pairs <= 24ll * mcb_sm_count() ? 4 : 16;
+}
 Qkv qkv_split(const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin, const QkvArgs& g);
 // undefined gradients count as zero
 void qkv_join(Qkv d, const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin, const QkvArgs& g,

@@ -260,7 +260,7 @@ class _ConvFn(torch.autograd.Function):
 
         from . import _lib
         T, C = x.shape
-        x, w = x.contiguous(), weight.contiguous()
+        x, w = _aligned(x), _aligned(weight)
         y = torch.empty_like(x)
         rc = _lib.lib().mcb_conv1d_silu_fwd(_lib.ptr(x), _lib.ptr(w), _lib.ptr(seq_start), _lib.ptr(y), ctypes.c_int(T),
                                             ctypes.c_int(C), ctypes.c_int(w.shape[1]), ctypes.c_int(int(act)),
@@ -277,7 +277,7 @@ class _ConvFn(torch.autograd.Function):
         from . import _lib
         x, w, seq_start = ctx.saved_tensors
         T, C = x.shape
-        dy = dy.contiguous()
+        dy = _aligned(dy)
         dx = torch.empty_like(x)
         dw = torch.zeros(w.shape, dtype=torch.float32, device=x.device)
         rc = _lib.lib().mcb_conv1d_silu_bwd(_lib.ptr(x), _lib.ptr(w), _lib.ptr(dy), _lib.ptr(seq_start), _lib.ptr(dx),

@@ -186,3 +186,37 @@ def test_norm_backward_adds_a_residual_gradient_once_rounded(rows, H):
         # times the mean: sums of up to 16384 terms over 256 chains, some 20 roundings of 2^-24 for the mean
         size = r * (g.abs() + xh.abs() * (g * xh).abs().mean(-1, keepdim=True))
         assert ((out.double() - (dx + res.double())).abs() <= 2 ** -8 * (dx + res.double()).abs() + 2 ** -18 * size).all()
+
+
+def _odd(t):
+    """The same values, contiguous, two bytes behind a 16-byte boundary."""
+    return torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(t.shape)
+
+
+@pytest.mark.parametrize('name', ['rmsnorm', 'norm_linear', 'glu', 'glu_linear', 'heads of 64', 'heads of 128', 'conv'])
+def test_tensors_off_a_16_byte_boundary_give_the_same_bits(name):
+    from mcore_bridge_b200.ops import fused_mlp, gdn
+    from mcore_bridge_b200.ops.activation import glu
+    from mcore_bridge_b200.ops.norm import rmsnorm
+    from mcore_bridge_b200.ops.rope import qkv_split_norm_rope
+    d = 128 if name == 'heads of 128' else 64
+    cos, sin = torch.rand(50, d // 2, device=DEV), torch.rand(50, d // 2, device=DEV)
+    x, w = _rand(50, 256), _rand(96, 256, seed=2)
+    # inputs, and whether they and the results' gradients may lie anywhere: products read neither weights nor gradients that do
+    fn, inputs, odd, odd_grads = {
+        'rmsnorm': (rmsnorm, [x, _rand(256, seed=1)], (1, 1), (1,)),
+        'norm_linear': (lambda x, l, w: fused_mlp.norm_linear(x, l, w, 1e-6, False, True), [x, _rand(256, seed=1), w], (1, 1, 0), (0, 1)),
+        'glu': (glu, [x], (1,), (1,)),
+        'glu_linear': (lambda h, w: fused_mlp.glu_linear(h, w, 0, 0.0, 0.0), [_rand(50, 512), w], (1, 0), (0,)),
+        'conv': (lambda x, w: gdn.causal_conv1d_silu(x, w), [x, _rand(256, 4, seed=1)], (1, 1), (1,)),
+    }.get(name) or (lambda x, a, b: qkv_split_norm_rope(x, a, b, cos, sin, 2, 2, d)[:3],
+                    [_rand(50, 8 * d), _rand(d, seed=1), _rand(d, seed=2)], (1, 1, 1), (1, 1, 1))
+
+    def run(lay):
+        leaves = [(lay if o else torch.clone)(t).detach().requires_grad_() for t, o in zip(inputs, odd)]
+        y = fn(*leaves)
+        y = [y] if torch.is_tensor(y) else list(y)
+        return y + list(torch.autograd.grad(y, leaves, [(lay if o else torch.clone)(_rand(*t.shape, seed=9)) for t, o in zip(y, odd_grads)]))
+
+    for i, (a, b) in enumerate(zip(run(torch.clone), run(_odd))):
+        assert torch.equal(a, b) or (name == 'conv' and i == 2 and _rel(a, b) < 2 ** -7)   # summed with atomics
