@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace mcb {
 
 inline int device_sm_count() {
@@ -18,6 +20,17 @@ inline int device_sm_count() {
     cached[dev] = n > 0 ? n : 148;
   }
   return cached[dev];
+}
+
+// Dynamic shared memory beyond 48 KB, which a kernel may use only after it was asked for on the device.  `done` is the kernel's.
+template <class K>
+inline cudaError_t allow_smem(K kernel, int bytes, std::atomic<bool> (&done)[64]) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (dev < 64 && done[dev])) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev < 64) done[dev] = true;
+  return e;
 }
 
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

@@ -589,12 +589,10 @@ static int rmsnorm_bwd_launch(const void* dy, void* y, const void* x, const void
 #define LAUNCH(V, R, P)                                                                                              \
   do {                                                                                                               \
     const int smem = P ? 2 * (R ? 3 : 2) * 2 * H * 2 : 0;                                                            \
-    static bool cfg = false;                                                                                         \
-    if (P && !cfg) {                                                                                                 \
-      const cudaError_t e = cudaFuncSetAttribute(rmsnorm_bwd_kernel<V, R, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                                 2 * (R ? 3 : 2) * 2 * 2048 * V * 2);                                \
+    static std::atomic<bool> allowed[64];                                                                            \
+    if (P) {                                                                                                         \
+      const cudaError_t e = allow_smem(rmsnorm_bwd_kernel<V, R, P>, 2 * (R ? 3 : 2) * 2 * 2048 * V * 2, allowed);    \
       if (e != cudaSuccess) return (int)e;                                                                           \
-      cfg = true;                                                                                                    \
     }                                                                                                                \
     rmsnorm_bwd_kernel<V, R, P><<<(int)grid, threads, smem, s>>>(                                                     \
         (const __nv_bfloat16*)dy, (__nv_bfloat16*)y, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,          \

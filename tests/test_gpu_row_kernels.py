@@ -65,6 +65,18 @@ def test_norm_backward_with_the_next_rows_in_flight(rows, H):
         assert _rel(a, b) < 2 ** -8
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason='needs 2 GPUs')
+def test_norm_backward_on_one_device_after_the_other():
+    from mcore_bridge_b200.ops.norm import rmsnorm
+    grads = []
+    for index in (0, 1):
+        with torch.cuda.device(index):
+            x, w = (t.to(index).requires_grad_() for t in (_rand(1190, 2048), _rand(2048, seed=3)))
+            grads.append(torch.autograd.grad(rmsnorm(x, w), [x, w], _rand(1190, 2048, seed=1).to(index)))
+    for a, b in zip(*grads):
+        assert torch.equal(a.cpu(), b.cpu())
+
+
 @pytest.mark.parametrize('rows,H', [(1, 8), (9500, 136), (20000, 256), (2500, 264), (1300, 4096), (1200, 8192)])
 @pytest.mark.parametrize('zero_centered', [False, True])
 def test_norm_forward_with_the_next_row_in_flight(rows, H, zero_centered):
