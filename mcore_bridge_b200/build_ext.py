@@ -30,8 +30,8 @@ NVCC_FLAGS = [
 ]
 # sources whose fp32 results are computed with the full-precision math functions and divisions (denormals are flushed in
 # them as everywhere else)
-PRECISE_SOURCES = {'attention/attn_sink_grad.cu', 'elementwise/ce_combine.cu', 'elementwise/token_tables.cu', 'linear_attention/gdn_inputs.cu',
-                   'linear_attention/gated_delta_rule.cu', 'moe/router_terms.cu'}
+PRECISE_SOURCES = {'attention/attn_sink_grad.cu', 'elementwise/ce_combine.cu', 'elementwise/token_tables.cu',
+                   'linear_attention/gdn_inputs.cu', 'linear_attention/gated_delta_rule.cu', 'moe/router_terms.cu'}
 
 
 def _flags(src: Path) -> list[str]:

@@ -36,16 +36,17 @@ def fusable(cls):
 
 
 def is_plain(module: nn.Module, cls) -> bool:
-    """A module whose call is the ``forward`` that ``cls`` was written with and nothing else: what a caller may fuse into another
-    operation."""
-    return (type(module) is cls and cls.forward is _FORWARDS[cls] and 'forward' not in module.__dict__
-            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
-            and not any(_GLOBAL_HOOKS))
+    """A module whose call is the ``forward`` that ``cls`` was written with and nothing else: what a caller may fuse into
+    another operation."""
+    own = module.__dict__
+    return (type(module) is cls and cls.forward is _FORWARDS[cls] and 'forward' not in own
+            and not (own['_forward_hooks'] or own['_forward_pre_hooks'] or own['_backward_hooks']
+                     or own['_backward_pre_hooks'] or _FORWARD or _FORWARD_PRE or _BACKWARD or _BACKWARD_PRE))
 
 
 # hooks on every module of the process: the dictionaries that torch's registration functions fill
-_GLOBAL_HOOKS = tuple(getattr(nn.modules.module, f'_global_{kind}_hooks')
-                      for kind in ('forward', 'forward_pre', 'backward', 'backward_pre'))
+_FORWARD, _FORWARD_PRE, _BACKWARD, _BACKWARD_PRE = (getattr(nn.modules.module, f'_global_{kind}_hooks') for kind in (
+    'forward', 'forward_pre', 'backward', 'backward_pre'))
 
 
 class _LinearBase(nn.Module):
@@ -146,7 +147,8 @@ class LayerNormColumnParallelLinear(ColumnParallelLinear):
         return self._unfused(x)
 
     def with_input(self, x):
-        """``(self(x), x)``, ``x`` in a form whose gradient joins the norm's inside its backward kernel where that is possible."""
+        """``(self(x), x)``, ``x`` in a form whose gradient joins the norm's inside its backward kernel where that is
+        possible."""
         if is_plain(self, LayerNormColumnParallelLinear) and self._lean(x):
             from ..ops import fused_mlp
             return fused_mlp.norm_linear(x, self.layer_norm_weight, self.weight, self.eps, self.zero_centered, True)

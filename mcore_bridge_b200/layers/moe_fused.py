@@ -416,8 +416,8 @@ def _weight_grad_grouped(weight, dy, x, offsets):
 
 def _pull_gemm(b: ExchangeBuffers, par: int, mode: int, st: 'DispatchState', El: int, rows, weight,
                b_mn: bool, xp, row_probs, out):
-    """Launches the fused pull + grouped GEMM kernel on ``b``'s published regions of parity ``par`` and the rows at ``rows``
-    (``publish_rows``)."""
+    """Launches the fused pull + grouped GEMM kernel on ``b``'s published regions of parity ``par`` and the rows at
+    ``rows`` (``publish_rows``)."""
     T, H, k, E = b.T, b.H, b.k, b.E
     G, d1, d2 = weight.shape
     w2 = weight.view(G * d1, d2)

@@ -192,8 +192,8 @@ class RotaryEmbedding(torch.nn.Module):
         else:
             if position_ids.dim() == 2:
                 position_ids = position_ids[0]
-            if position_ids.is_cuda and inv.device == position_ids.device and position_ids.dtype in (torch.int32, torch.int64) \
-                    and position_ids.dim() == 1 and _lib.cuda_enabled():
+            if position_ids.is_cuda and inv.device == position_ids.device and position_ids.dim() == 1 \
+                    and position_ids.dtype in (torch.int32, torch.int64) and _lib.cuda_enabled():
                 return _lib.native().rope_tables(position_ids, inv, self.attention_scaling)
             freqs = position_ids.float()[:, None] * inv[None, :]
         cos, sin = freqs.cos(), freqs.sin()

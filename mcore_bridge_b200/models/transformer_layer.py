@@ -107,7 +107,8 @@ class TransformerLayer(nn.Module):
         with nvtx_range('moe' if self.is_moe else 'mlp'):
             if self.is_moe:
                 out = self.mlp(x, ctx.padding_mask, ctx.seg_ids, ctx.num_seqs, ctx.input_ids)
-            elif hc is None and self.pre_mlp_layernorm is None and not cfg.post_sublayer_layernorm and is_plain(self.mlp, MLP):
+            elif hc is None and self.pre_mlp_layernorm is None and not cfg.post_sublayer_layernorm \
+                    and is_plain(self.mlp, MLP):
                 return self.mlp(x, True)
             else:
                 out = self.mlp(x)

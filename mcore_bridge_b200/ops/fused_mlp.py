@@ -22,8 +22,8 @@ def usable(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 
 def norm_linear(x, ln_w, weight, eps, zero_centered, keep: bool = False):
-    """With ``keep`` returns ``x`` as well: a residual taken from there has its gradient added to the norm's by the norm's
-    backward kernel."""
+    """With ``keep`` returns ``x`` as well: a residual taken from there has its gradient added to the norm's by the
+    norm's backward kernel."""
     return _lib.native().norm_linear(x, ln_w, weight, eps, zero_centered, keep)
 
 

@@ -176,8 +176,8 @@ class _LinearFn(torch.autograd.Function):
 
 def _single_rank(x, weight, bias, spec: LinearSpec):
     """The module whose ``linear`` is the whole function where no collective, no fp8 and no fallback is in it."""
-    if spec.fp8 or not (x.is_cuda and weight.is_cuda and x.dtype == torch.bfloat16) or (bias is not None and not bias.is_cuda) \
-            or (spec.mode and ps.get_world_size(spec.group) > 1):
+    if spec.fp8 or not (x.is_cuda and weight.is_cuda and x.dtype == torch.bfloat16) \
+            or (bias is not None and not bias.is_cuda) or (spec.mode and ps.get_world_size(spec.group) > 1):
         return None
     return _lib.native_if_enabled()
 

@@ -139,17 +139,17 @@ class MoEAuxLossAutoScaler(torch.autograd.Function):
 
 
 class RouterAuxLoss(torch.autograd.Function):
-    """``aux_loss`` from the router kernel's statistics (``score_sum`` fp32 and ``counts`` int32, ``[E]``) of ``tokens`` tokens,
-    and the same divided by ``coeff`` for the log, in one launch each way."""
+    """``aux_loss`` from the router kernel's statistics (``score_sum`` fp32 and ``counts`` int32, ``[E]``) of ``tokens``
+    tokens, and the same divided by ``coeff`` for the log, in one launch each way."""
 
     @staticmethod
     def forward(ctx, score_sum, counts, tokens, topk, coeff):
         E = score_sum.shape[0]
         out = torch.empty(E + 2, dtype=torch.float32, device=score_sum.device)
         c = coeff * E
-        rc = _lib.lib().mcb_router_aux(_lib.ptr(counts), _lib.ptr(score_sum), _lib.ptr(out[2:]), _lib.ptr(out), ctypes.c_int(E),
-                                       ctypes.c_float(tokens), ctypes.c_int(topk), ctypes.c_float(c), ctypes.c_float(coeff),
-                                       _lib.stream_ptr())
+        rc = _lib.lib().mcb_router_aux(_lib.ptr(counts), _lib.ptr(score_sum), _lib.ptr(out[2:]), _lib.ptr(out),
+                                       ctypes.c_int(E), ctypes.c_float(tokens), ctypes.c_int(topk), ctypes.c_float(c),
+                                       ctypes.c_float(coeff), _lib.stream_ptr())
         _lib.check_rc(rc, 'mcb_router_aux')
         aux, value, frac = out[0], out[1], out[2:]
         ctx.save_for_backward(frac)
@@ -177,16 +177,17 @@ def split_terms(x: torch.Tensor) -> torch.Tensor:
     if x.data_ptr() % 16:
         x = x.clone()
     out = torch.empty((T, 2 * E), dtype=torch.bfloat16, device=x.device)
-    _lib.check_rc(_lib.lib().mcb_split_terms(_lib.ptr(x), _lib.ptr(out), ctypes.c_longlong(T), ctypes.c_int(E), _lib.stream_ptr()),
-                  'mcb_split_terms')
+    rc = _lib.lib().mcb_split_terms(_lib.ptr(x), _lib.ptr(out), ctypes.c_longlong(T), ctypes.c_int(E),
+                                    _lib.stream_ptr())
+    _lib.check_rc(rc, 'mcb_split_terms')
     return out
 
 
 def add_halves(x: torch.Tensor) -> torch.Tensor:
     """fp32 ``[2E, H]`` -> bf16 ``[E, H]``: the sum of the two halves."""
     out = torch.empty((x.shape[0] // 2, *x.shape[1:]), dtype=torch.bfloat16, device=x.device)
-    _lib.check_rc(_lib.lib().mcb_add_halves(_lib.ptr(x), _lib.ptr(out), ctypes.c_longlong(out.numel()), _lib.stream_ptr()),
-                  'mcb_add_halves')
+    rc = _lib.lib().mcb_add_halves(_lib.ptr(x), _lib.ptr(out), ctypes.c_longlong(out.numel()), _lib.stream_ptr())
+    _lib.check_rc(rc, 'mcb_add_halves')
     return out
 
 
