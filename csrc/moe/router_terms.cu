@@ -10,7 +10,8 @@ using namespace mcb;
 
 namespace {
 
-// out = {c sum_e frac_e score_sum_e / tokens, that / coeff},  frac_e = counts_e / (tokens k)
+// out = {c sum_e frac_e score_sum_e / tokens, that / coeff},  frac_e = counts_e / (tokens k); the sum in another order than a tensor
+// operation's, the gradient with its bits
 __global__ void __launch_bounds__(256)
 router_aux_kernel(const int* __restrict__ counts, const float* __restrict__ score_sum, float* __restrict__ frac, float* __restrict__ out,
                   int E, float tokens, float copies, float c, float coeff) {
